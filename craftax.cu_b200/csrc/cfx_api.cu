@@ -41,9 +41,9 @@ struct cfx_policy {
     float* params = nullptr;        // fp32 arena (device)
     float* gates_t = nullptr;       // strict path: transposed gate matrices
     float* state = nullptr;         // [L][n][H]
-    float* scratch_h[2] = {nullptr, nullptr};  // strict path layer ping-pong
+    float* scratch_h[2] = {nullptr, nullptr};  // fp32 mode: layer ping-pong
     float* logits_scratch = nullptr;           // [n][A+1] when the caller passes none
-    unsigned long long* step_ctr = nullptr;
+    unsigned long long* step_ctr = nullptr;   // {step counter, finished blocks of the fp32 sampler}
     cudaStream_t stream = nullptr;
     FusedPlan* fused = nullptr;
     int last_launches = 0;
@@ -78,8 +78,17 @@ static int policy_refresh_mirrors(cfx_policy* p, cudaStream_t st) {
     return CFX_OK;
 }
 
+// What only the fp32 mode needs: two activation buffers [H][n] and room for the logits.
+static int policy_ensure_fp32(cfx_policy* p) {
+    for (int i = 0; i < 2; i++)
+        if (!p->scratch_h[i]) CFX_CUDA(cudaMalloc((void**)&p->scratch_h[i], (size_t)p->H * p->n * sizeof(float)));
+    if (!p->logits_scratch)
+        CFX_CUDA(cudaMalloc((void**)&p->logits_scratch, (size_t)p->n * (p->A + 1) * sizeof(float)));
+    return CFX_OK;
+}
+
 static int policy_ensure_fused(cfx_policy* p) {
-    if (p->precision == CFX_PREC_FP32) return CFX_OK;
+    if (p->precision == CFX_PREC_FP32) return policy_ensure_fp32(p);
     if (!fused_supported(p->H, p->L, p->A, p->precision, p->game)) {
         set_error("precision %d is not built for hidden=%d layers=%d actions=%d", p->precision,
                   p->H, p->L, p->A);
@@ -175,16 +184,13 @@ static int policy_create(cfx_policy** out, int device, int num_envs, int hidden,
     CFX_TRY_ALLOC(p->params, p->param_count * sizeof(float));
     CFX_TRY_ALLOC(p->gates_t, (size_t)layers * 3 * hidden * hidden * sizeof(float));
     CFX_TRY_ALLOC(p->state, (size_t)layers * hn * sizeof(float));
-    CFX_TRY_ALLOC(p->scratch_h[0], hn * sizeof(float));
-    CFX_TRY_ALLOC(p->scratch_h[1], hn * sizeof(float));
-    CFX_TRY_ALLOC(p->logits_scratch, (size_t)num_envs * (num_actions + 1) * sizeof(float));
-    CFX_TRY_ALLOC(p->step_ctr, sizeof(unsigned long long));
+    CFX_TRY_ALLOC(p->step_ctr, 2 * sizeof(unsigned long long));
 #undef CFX_TRY_ALLOC
     cudaError_t e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail(cuda_fail(e, "cudaStreamCreateWithFlags", __FILE__, __LINE__));
     e = cudaMemsetAsync(p->params, 0, p->param_count * sizeof(float), p->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(p->state, 0, (size_t)layers * hn * sizeof(float), p->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p->step_ctr, 0, sizeof(unsigned long long), p->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->step_ctr, 0, 2 * sizeof(unsigned long long), p->stream);
     if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__));
     rc = policy_ensure_fused(p);
     if (rc) return fail(rc);
@@ -345,6 +351,11 @@ int cfx_policy_set_precision(cfx_policy* p, int precision) {
     const int old = p->precision;
     p->precision = precision;
     if (precision == CFX_PREC_FP32) {
+        int rc = policy_ensure_fp32(p);
+        if (rc) {
+            p->precision = old;
+            return rc;
+        }
         if (p->fused) {
             fused_destroy(p->fused);
             p->fused = nullptr;
@@ -438,6 +449,7 @@ static int forward_range(cfx_policy* p, const cfx_forward_io* io, void* stream, 
         a.seed = io->seed;
         a.env_offset = io->env_offset;
         a.step_ctr = p->step_ctr;
+        a.bump_step = io->bump_step ? 1 : 0;
         rc = strict_forward(a, st, &launches);
     } else {
         CFX_REQUIRE(p->fused != nullptr, "cfx_policy_forward: fused plan missing");
@@ -462,11 +474,6 @@ static int forward_range(cfx_policy* p, const cfx_forward_io* io, void* stream, 
         rc = fused_forward(p->fused, a, st, &launches);
     }
     if (rc) return rc;
-    if (io->bump_step && p->precision == CFX_PREC_FP32) {
-        rc = launch_bump(p->step_ctr, st);
-        if (rc) return rc;
-        launches++;
-    }
     p->last_launches = launches;
     return CFX_OK;
 }
@@ -633,7 +640,7 @@ int cfx_sample_actions(int device, const float* logits, int ld, int num_actions,
     CFX_REQUIRE(num_actions >= 2 && num_actions <= kMaxActions && ld >= num_actions,
                 "cfx_sample_actions: num_actions=%d ld=%d", num_actions, ld);
     CFX_GUARD(device);
-    return launch_sample(logits, ld, num_actions, uniforms, 0, 0, nullptr, n, nullptr, actions,
+    return launch_sample(logits, ld, num_actions, uniforms, 0, 0, nullptr, 0, n, nullptr, actions,
                          logprobs, nullptr, (cudaStream_t)stream);
 }
 

@@ -34,6 +34,7 @@
 #include <cuda_fp16.h>
 
 #include "cfx_common.cuh"
+#include "cfx_f32x2.cuh"
 #include "cfx_fused.h"
 #include "cfx_sampler.cuh"
 #include "cfx_tmap.h"
@@ -387,32 +388,8 @@ __device__ __forceinline__ float tanh_fast(float x) {
     return y;
 }
 
-// Two units at once with the packed fp32 instructions of sm_100 (`fma.rn.f32x2` and friends:
-// two results per issue slot, the same roundings as the scalar forms).  The cell phase is
-// bound by instruction issue and latency (two worker warps per scheduler), not by the FMA pipe.
-__device__ __forceinline__ uint64_t f2pack(float a, float b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2unpack(uint64_t v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2mul(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t f2sub(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t f2fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
+// Two units at once with the packed fp32 instructions: the cell phase is bound by instruction
+// issue and latency (two worker warps per scheduler), not by the FMA pipe.
 // hzh, hzg, hzp: zh/2, zg/2, zp/2 of two units
 __device__ __forceinline__ void mingru_cell_pair(float hzh0, float hzh1, float hzg0, float hzg1, float hzp0,
                                                  float hzp1, float st0, float st1, float x0, float x1,

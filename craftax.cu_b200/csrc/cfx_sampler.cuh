@@ -47,19 +47,22 @@ __device__ __forceinline__ int sample_action(const float (&logits)[A], float u, 
     return action;
 }
 
-// Runtime-A variant for the stand-alone sampler entry point.
-__device__ __forceinline__ int sample_action_dyn(const float* logits, int A, float u, float* logprob) {
-    float m = logits[0];
-    for (int a = 1; a < A; a++) m = fmaxf(m, logits[a]);
+// The same with a runtime A, for the stand-alone sampler: the maximum m and p[a] = expf(l[a] - m)
+// are given.
+__device__ __forceinline__ int pick_action(const float* l, const float* p, int A, float m, float u, float* logprob) {
     float total = 0.0f;
-    for (int a = 0; a < A; a++) total += expf(logits[a] - m);
-    float target = u * total, cum = 0.0f;
-    int action = A - 1;
-    for (int a = 0; a < A; a++) {
-        cum += expf(logits[a] - m);
-        if (target <= cum) { action = a; break; }
+#pragma unroll 8
+    for (int a = 0; a < A; a++) total += p[a];
+    const float target = u * total;
+    float cum = 0.0f;
+    int action = -1;
+#pragma unroll 8
+    for (int a = 0; a < A; a++) {   // no early exit: the reads stay ahead of the sum
+        cum += p[a];
+        if (action < 0 && target <= cum) action = a;
     }
-    *logprob = logits[action] - m - logf(total);
+    if (action < 0) action = A - 1;
+    *logprob = l[action] - m - logf(total);
     return action;
 }
 

@@ -12,6 +12,7 @@
 #include <atomic>
 
 #include "cfx_common.cuh"
+#include "cfx_f32x2.cuh"
 #include "cfx_sampler.cuh"
 #include "cfx_strict.h"
 
@@ -37,48 +38,204 @@ __global__ void k_expand(const uint8_t* __restrict__ rec, float* __restrict__ ou
     out[idx] = x;
 }
 
-// ---------------------------------------------------------------- encoder
-// h_enc[e][k] = b_enc[k] + sum_f x[e][f] * W_enc[f][k], ascending f.
-// Block = H threads (one per unit) x ENC_ENVS envs; the records of the tile are
-// expanded chunk-wise into shared memory as fp32, transposed to [f][e] so the
-// inner loop reads x by broadcast and W_enc rows coalesced.
-constexpr int ENC_ENVS = 32;
-constexpr int ENC_FCHUNK = 64;
-
-__global__ void k_encoder_fp32(const uint8_t* __restrict__ rec, const float* __restrict__ W_enc,
-                               const float* __restrict__ b_enc, float* __restrict__ h_out,
-                               int n, int H) {
-    __shared__ float xs[ENC_FCHUNK][ENC_ENVS + 1];
-    const int e0 = blockIdx.x * ENC_ENVS;
-    const int k = threadIdx.x;  // unit
-    float acc[ENC_ENVS];
-    const float b = b_enc[k];
+// ---------------------------------------------------------------- tiling of the fp32 layers
+// The encoder and the MinGRU layers are fp32 matrix products whose sums run in ascending input
+// order, so nothing may be split along the inputs; the work is split over (env, unit) tiles.  They
+// are bound by the FMA pipe (128 lanes per clock and SM), and a thread that loads an operand for few FMAs by
+// shared-memory reads instead (a cycle per operand register and warp, broadcast or not).  In a layer a lane
+// owns TM envs x 4 units, all three gates, a warp 4 TM envs x 32 units (lane = 8 groups of units x 4
+// groups of envs), and a block is WM x WU such warps.  Activations travel between the kernels transposed,
+// [H][n], so that both operands of a k step are contiguous in shared memory; two units at a time go
+// through the packed FMA (`fma.rn.f32x2`, the rounding of fmaf), which leaves issue slots for
+// the operand reads.
+// (The doubled input of a pair is made with register moves: stored doubled it costs 8 more operand
+// registers from shared memory a k step, and the layer kernel went from 52 to 59 us at 4,096 envs.)
+template <int TM> struct Frag {   // the TM inputs of a lane, each doubled for the packed FMA
+    uint64_t v[TM];
+    __device__ __forceinline__ void load(const float* x) {
+        if constexpr (TM >= 4) {
 #pragma unroll
-    for (int e = 0; e < ENC_ENVS; e++) acc[e] = b;
-    for (int f0 = 0; f0 < kObs; f0 += ENC_FCHUNK) {
-        const int fc = min(ENC_FCHUNK, kObs - f0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < ENC_ENVS * ENC_FCHUNK; i += blockDim.x) {
-            int e = i / ENC_FCHUNK, f = i % ENC_FCHUNK;
-            float x = 0.0f;
-            if (f < fc && e0 + e < n) {
-                const uint8_t* r = rec + (size_t)(e0 + e) * kRec;
-                int ff = f0 + f;
-                x = ff < kMap ? (float)r[ff]
-                              : *reinterpret_cast<const float*>(r + kMap + 4 * (ff - kMap));
+            for (int q = 0; q < TM / 4; q++) {
+                const float4 f = *reinterpret_cast<const float4*>(x + 4 * q);
+                v[4 * q] = f2pack(f.x, f.x); v[4 * q + 1] = f2pack(f.y, f.y);
+                v[4 * q + 2] = f2pack(f.z, f.z); v[4 * q + 3] = f2pack(f.w, f.w);
             }
-            xs[f][e] = x;
-        }
-        __syncthreads();
-        for (int f = 0; f < fc; f++) {
-            const float w = W_enc[(size_t)(f0 + f) * H + k];
-#pragma unroll
-            for (int e = 0; e < ENC_ENVS; e++) acc[e] = fmaf(xs[f][e], w, acc[e]);
+        } else {
+            v[0] = f2pack(x[0], x[0]);
         }
     }
+};
+// TM consecutive floats of a [H][n] row
+template <int TM> __device__ __forceinline__ void load_envs(const float* p, float (&v)[TM]) {
+    if constexpr (TM >= 4) {
 #pragma unroll
-    for (int e = 0; e < ENC_ENVS; e++)
-        if (e0 + e < n) h_out[(size_t)(e0 + e) * H + k] = acc[e];
+        for (int q = 0; q < TM / 4; q++) {
+            const float4 f = *reinterpret_cast<const float4*>(p + 4 * q);
+            v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
+        }
+    } else {
+        v[0] = p[0];
+    }
+}
+template <int TM> __device__ __forceinline__ void store_envs(float* p, const float (&v)[TM]) {
+    if constexpr (TM >= 4) {
+#pragma unroll
+        for (int q = 0; q < TM / 4; q++)
+            *reinterpret_cast<float4*>(p + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+        p[0] = v[0];
+    }
+}
+// 16 bytes global -> shared in flight (zeros where `on` is false); a source that is only 4-byte
+// aligned goes as four words
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool on, bool aligned) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (aligned) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * i), "l"(src + i), "r"(on ? 4 : 0) : "memory");
+    }
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// The kernels of a forward are launched with programmatic stream serialisation and wait here until the
+// results of the kernel in front are in memory.  None lets the next one start early
+// (griddepcontrol.launch_dependents): its blocks would fill the SMs that this kernel's last blocks leave
+// free and pile up there (4,096 envs: 227 us against 178 for a forward).
+__device__ __forceinline__ void wait_for_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ---------------------------------------------------------------- encoder
+// h_enc[k][e] = b_enc[k] + sum_f x[e][f] * W_enc[f][k], ascending f.  A lane owns TM envs x G groups of 4
+// units, the groups 32 units apart.  Few warps of such tiles fall to an SM scheduler (one at 4,096 envs,
+// hidden 256), so everything but the sums is taken out of them: four warps of a block fill the stages (record words ->
+// fp32, transposed; W_enc rows by asynchronous copies), four multiply, and named barriers hand the
+// stages over.  4,096 envs, hidden 256: 52 us, against 63 us with every warp doing both, and 78 us
+// with the features kept as bytes and converted by the lanes that multiply.
+constexpr int kEncK = 32, kEncStages = 3;
+template <int TM, int G> struct Enc {
+    static constexpr int BM = 16 * TM, BU = 32 * G, XS = BM + 4;       // envs, units, row stride of x
+    static constexpr int kStage = kEncK * (XS + BU);                   // floats
+    static constexpr int kSmem = kEncStages * kStage * (int)sizeof(float);
+};
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+template <int TM, int G>
+__global__ void __launch_bounds__(256, 2)
+k_encoder_fp32(const uint8_t* __restrict__ rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc,
+                  float* __restrict__ h_out, int n, int H, int w_aligned) {
+    constexpr int BM = Enc<TM, G>::BM, BU = Enc<TM, G>::BU, XS = Enc<TM, G>::XS, K = kEncK, kStage = Enc<TM, G>::kStage;
+    constexpr int kChunks = (kObs + K - 1) / K, FULL = 1, EMPTY = FULL + kEncStages;   // barrier ids
+    extern __shared__ __align__(16) float sm[];   // per stage: x [K][XS], w [K][BU]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int e0 = blockIdx.x * BM, u0 = blockIdx.y * BU;
+    wait_for_previous_kernel();
+    if (warp >= 4) {
+        const int tid = threadIdx.x - 128;
+        // a task is one record word (four features of an env): lanes = 16 envs x 2 words
+        constexpr int TASKS = BM * (K / 4) / 128;
+        uint32_t raw[TASKS][4];   // one word = four map features, or four raw floats in the tail
+        auto slot = [&](int i, int& e, int& w) {
+            const int idx = i * 128 + tid;
+            e = idx % 16 + 16 * ((idx / 32) % (BM / 16));
+            w = (idx % 32) / 16 + 2 * (idx / (2 * BM));
+        };
+        auto fetch = [&](int f0) {
+#pragma unroll
+            for (int i = 0; i < TASKS; i++) {
+                int e, w;
+                slot(i, e, w);
+                const uint8_t* r = rec + (size_t)(e0 + e) * kRec;
+                const int f = f0 + 4 * w;
+                const bool on = e0 + e < n;
+                raw[i][0] = on && f < kMap ? *reinterpret_cast<const uint32_t*>(r + f) : 0u;   // (792 is a multiple of 4)
+                raw[i][1] = raw[i][2] = raw[i][3] = 0u;
+                if (on && f >= kMap) {
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (f + q < kObs) raw[i][q] = *reinterpret_cast<const uint32_t*>(r + kMap + 4 * (f + q - kMap));
+                }
+            }
+        };
+        fetch(0);
+        for (int c = 0; c < kChunks; c++) {
+            const int s = c % kEncStages, f0 = c * K;
+            float* x = sm + s * kStage;
+            float* w = x + K * XS;
+            if (c >= kEncStages) bar_sync(EMPTY + s, 256);
+            for (int i = tid; i < K * (BU / 4); i += 128) {
+                const int k = i / (BU / 4), col = 4 * (i % (BU / 4));
+                if (f0 + k < kObs) copy16(w + k * BU + col, W_enc + (size_t)(f0 + k) * H + u0 + col, true, w_aligned != 0);
+            }
+            copy_commit();
+#pragma unroll
+            for (int i = 0; i < TASKS; i++) {
+                int e, wd;
+                slot(i, e, wd);
+                const bool map = f0 + 4 * wd < kMap;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    x[(4 * wd + q) * XS + e] = map ? (float)((raw[i][0] >> (8 * q)) & 0xFFu) : __uint_as_float(raw[i][q]);
+            }
+            if (c + 1 < kChunks) fetch(f0 + K);
+            copy_wait<0>();
+            bar_arrive(FULL + s, 256);
+        }
+        return;
+    }
+    const int el = warp * 4 * TM + (lane >> 3) * TM, ul = (lane & 7) * 4;
+    uint64_t z[G][TM][2];
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+        const float* b = b_enc + u0 + ul + 32 * g;
+#pragma unroll
+        for (int e = 0; e < TM; e++) { z[g][e][0] = f2pack(b[0], b[1]); z[g][e][1] = f2pack(b[2], b[3]); }
+    }
+    for (int c = 0; c < kChunks; c++) {
+        const int s = c % kEncStages;
+        const float* xp = sm + s * kStage + el;
+        const float* wp = sm + s * kStage + K * XS + ul;
+        bar_sync(FULL + s, 256);
+        auto step = [&](int k) {
+            Frag<TM> x;
+            x.load(xp + k * XS);
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                const float4 w = *reinterpret_cast<const float4*>(wp + k * BU + 32 * g);
+                const uint64_t w01 = f2pack(w.x, w.y), w23 = f2pack(w.z, w.w);
+#pragma unroll
+                for (int e = 0; e < TM; e++) {
+                    z[g][e][0] = f2fma(x.v[e], w01, z[g][e][0]);
+                    z[g][e][1] = f2fma(x.v[e], w23, z[g][e][1]);
+                }
+            }
+        };
+        if (c + 1 < kChunks) {
+#pragma unroll 16
+            for (int k = 0; k < K; k++) step(k);
+        } else {
+            for (int k = 0; k < kObs - c * K; k++) step(k);
+        }
+        if (c + kEncStages < kChunks) bar_arrive(EMPTY + s, 256);
+    }
+    if (e0 + el < n) {
+#pragma unroll
+        for (int i = 0; i < 4 * G; i++) {
+            const int g = i >> 2, u = i & 3;
+            float h[TM];
+#pragma unroll
+            for (int e = 0; e < TM; e++) {
+                float lo, hi;
+                f2unpack(z[g][e][u >> 1], lo, hi);
+                h[e] = (u & 1) ? hi : lo;
+            }
+            store_envs<TM>(h_out + (size_t)(u0 + ul + 32 * g + u) * n + e0 + el, h);
+        }
+    }
 }
 
 // ---------------------------------------------------------------- classic game
@@ -116,6 +273,7 @@ __global__ void k_classic_encoder_fp32(const uint8_t* __restrict__ rec, const fl
     __shared__ uint8_t rs[kClassicRec];
     const int e = blockIdx.x;
     const int k = threadIdx.x;
+    wait_for_previous_kernel();
     for (int i = threadIdx.x; i < kClassicRec; i += blockDim.x) rs[i] = rec[(size_t)e * kClassicRec + i];
     __syncthreads();
     const float* Wk = W_enc + k;
@@ -141,7 +299,7 @@ __global__ void k_classic_encoder_fp32(const uint8_t* __restrict__ rec, const fl
     hv = fmaf(light, Wk[(size_t)f * H], hv);
     f++;
     hv = fmaf(sleeping ? 1.0f : 0.0f, Wk[(size_t)f * H], hv);
-    h_out[(size_t)e * H + k] = hv;
+    h_out[(size_t)k * n + e] = hv;   // [H][n]; the scattered words meet in L2 (a record gathers 100 rows of W_enc)
 }
 
 // r_done int8 flags of the classic rollout (main_classic.cu:436-443) -> the float flags the
@@ -152,105 +310,252 @@ __global__ void k_done_to_terminals(const int8_t* __restrict__ done, float* __re
 }
 
 // ---------------------------------------------------------------- MinGRU layer
-// One layer: gate dots (ascending j, fmaf) + cell (k_mingru_epi_fwd,
-// craftax_full.cu:9350-9395).  Wt is the layer's gate matrix transposed to
-// [H][3H] so that unit-indexed threads read it coalesced.
-constexpr int GRU_ENVS = 16;
-
+// One layer: gate dots (ascending j, fmaf) + cell (k_mingru_epi_fwd, craftax_full.cu:9350-9395).
+// Wt is the layer's gate matrix transposed to [H][3H]; x_in and h_out are [H][n].  K chunks of 32,
+// two buffers (chunks of 16 with three: 155 against 152 us a forward at 4,096 envs, 970 against 944 us at 8,192 envs with
+// hidden 512, depth 3); the k loop has to be unrolled well (by 4: 170 us).  Bound by the FMA pipe: 66 % of its peak at
+// hidden 512; one thread per unit with 16 envs, before, 20 %.
 __device__ __forceinline__ float sigmoid_ref(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float mingru_g_ref(float x) { return x >= 0.0f ? x + 0.5f : sigmoid_ref(x); }
 
-__global__ void k_mingru_fp32(const float* __restrict__ x_in, const float* __restrict__ Wt,
-                              float* __restrict__ state, const float* __restrict__ prev_terminals,
-                              float* __restrict__ h_out, float* __restrict__ r_state, int r_bf16,
-                              int n, int H) {
-    extern __shared__ float xs[];  // [GRU_ENVS][H]
-    const int e0 = blockIdx.x * GRU_ENVS;
-    const int k = threadIdx.x;
-    for (int i = threadIdx.x; i < GRU_ENVS * H; i += blockDim.x) {
-        int e = i / H;
-        xs[i] = (e0 + e < n) ? x_in[(size_t)e0 * H + i] : 0.0f;
+constexpr int kGruK = 32, kGruStages = 2;
+template <int TM, int WM, int WU> constexpr int gru_stage_floats() { return kGruK * (4 * TM * WM + 3 * 32 * WU); }
+
+template <int TM, int WM, int WU>
+__global__ void __launch_bounds__(32 * WM * WU, 3)
+k_mingru_fp32(const float* __restrict__ x_in, const float* __restrict__ Wt, float* __restrict__ state,
+              const float* __restrict__ prev_terminals, float* __restrict__ h_out, float* __restrict__ r_state,
+              int r_bf16, int n, int H, int s_aligned) {
+    constexpr int T = 32 * WM * WU, BM = 4 * TM * WM, BU = 32 * WU;
+    extern __shared__ __align__(16) float sm[];   // per stage: x [kGruK][BM][2], w [kGruK][3][BU]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int e0 = blockIdx.x * BM, u0 = blockIdx.y * BU;
+    const int el = (warp % WM) * 4 * TM + (lane >> 3) * TM, ul = (warp / WM) * 32 + (lane & 7) * 4;
+    const bool live = e0 + el < n;
+    wait_for_previous_kernel();
+
+    auto copy_chunk = [&](int c) {
+        float* x = sm + (c % kGruStages) * gru_stage_floats<TM, WM, WU>();
+        float* w = x + kGruK * BM;
+        for (int i = tid; i < kGruK * (BM / 4); i += T) {
+            const int k = i / (BM / 4), e = 4 * (i % (BM / 4));
+            copy16(x + k * BM + e, x_in + (size_t)(c * kGruK + k) * n + e0 + e, e0 + e < n, true);
+        }
+        for (int i = tid; i < kGruK * 3 * (BU / 4); i += T) {
+            const int k = i / (3 * (BU / 4)), r = i % (3 * (BU / 4)), g = r / (BU / 4), u = 4 * (r % (BU / 4));
+            copy16(w + (k * 3 + g) * BU + u, Wt + (size_t)(c * kGruK + k) * 3 * H + g * H + u0 + u, true, true);
+        }
+    };
+    const int chunks = H / kGruK;
+#pragma unroll
+    for (int c = 0; c < kGruStages - 1; c++) {
+        if (c < chunks) copy_chunk(c);
+        copy_commit();
     }
-    __syncthreads();
-    float zh[GRU_ENVS], zg[GRU_ENVS], zp[GRU_ENVS];
+    uint64_t z[3][TM][2];
 #pragma unroll
-    for (int e = 0; e < GRU_ENVS; e++) zh[e] = zg[e] = zp[e] = 0.0f;
-    for (int j = 0; j < H; j++) {
-        const float* wr = Wt + (size_t)j * 3 * H;
-        const float wh = wr[k], wg = wr[H + k], wp = wr[2 * H + k];
+    for (int g = 0; g < 3; g++)
 #pragma unroll
-        for (int e = 0; e < GRU_ENVS; e++) {
-            const float xv = xs[e * H + j];
-            zh[e] = fmaf(wh, xv, zh[e]);
-            zg[e] = fmaf(wg, xv, zg[e]);
-            zp[e] = fmaf(wp, xv, zp[e]);
+        for (int e = 0; e < TM; e++) z[g][e][0] = z[g][e][1] = 0ull;
+    for (int c = 0; c < chunks; c++) {
+        copy_wait<kGruStages - 2>();
+        __syncthreads();   // chunk c is complete, and everybody is done with chunk c - 1
+        if (c + kGruStages - 1 < chunks) copy_chunk(c + kGruStages - 1);
+        copy_commit();
+        const float* x = sm + (c % kGruStages) * gru_stage_floats<TM, WM, WU>() + el;
+        const float* w = sm + (c % kGruStages) * gru_stage_floats<TM, WM, WU>() + kGruK * BM + ul;
+#pragma unroll 16
+        for (int k = 0; k < kGruK; k++) {
+            Frag<TM> xv;
+            xv.load(x + k * BM);
+#pragma unroll
+            for (int g = 0; g < 3; g++) {
+                const float4 wv = *reinterpret_cast<const float4*>(w + (k * 3 + g) * BU);
+                const uint64_t w01 = f2pack(wv.x, wv.y), w23 = f2pack(wv.z, wv.w);
+#pragma unroll
+                for (int e = 0; e < TM; e++) {
+                    z[g][e][0] = f2fma(w01, xv.v[e], z[g][e][0]);
+                    z[g][e][1] = f2fma(w23, xv.v[e], z[g][e][1]);
+                }
+            }
+        }
+    }
+    if (!live) return;
+    // this lane's TM x 4 states and terminal flags
+    float st[TM][4];
+#pragma unroll
+    for (int e = 0; e < TM; e++) {
+        const size_t o = (size_t)(e0 + el + e) * H + u0 + ul;
+        st[e][0] = st[e][1] = st[e][2] = st[e][3] = 0.0f;
+        if (!(prev_terminals != nullptr && prev_terminals[e0 + el + e] != 0.0f)) {
+            if (s_aligned) {
+                const float4 f = *reinterpret_cast<const float4*>(state + o);
+                st[e][0] = f.x; st[e][1] = f.y; st[e][2] = f.z; st[e][3] = f.w;
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; u++) st[e][u] = state[o + u];
+            }
+        }
+    }
+    if (r_state != nullptr) {   // the post-zero state inputs
+#pragma unroll
+        for (int e = 0; e < TM; e++) {
+            const size_t o = (size_t)(e0 + el + e) * H + u0 + ul;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o + u] = __float2bfloat16(st[e][u]);
+                else r_state[o + u] = st[e][u];
+            }
         }
     }
 #pragma unroll
-    for (int e = 0; e < GRU_ENVS; e++) {
-        if (e0 + e >= n) break;
-        const size_t o = (size_t)(e0 + e) * H + k;
-        float st = state[o];
-        if (prev_terminals != nullptr && prev_terminals[e0 + e] != 0.0f) st = 0.0f;
-        if (r_state != nullptr) {
-            if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o] = __float2bfloat16(st);
-            else r_state[o] = st;
+    for (int u = 0; u < 4; u++) {
+        float x[TM], h[TM];
+        load_envs<TM>(x_in + (size_t)(u0 + ul + u) * n + e0 + el, x);
+#pragma unroll
+        for (int e = 0; e < TM; e++) {
+            float lo, hi;
+            f2unpack(z[0][e][u >> 1], lo, hi);
+            const float zh = (u & 1) ? hi : lo;
+            f2unpack(z[1][e][u >> 1], lo, hi);
+            const float zg = (u & 1) ? hi : lo;
+            f2unpack(z[2][e][u >> 1], lo, hi);
+            const float zp = (u & 1) ? hi : lo;
+            const float s = st[e][u];
+            const float out = s + sigmoid_ref(zg) * (mingru_g_ref(zh) - s);
+            const float p = sigmoid_ref(zp);
+            h[e] = p * out + (1.0f - p) * x[e];
+            st[e][u] = out;
         }
-        const float out = st + sigmoid_ref(zg[e]) * (mingru_g_ref(zh[e]) - st);
-        const float p = sigmoid_ref(zp[e]);
-        h_out[o] = p * out + (1.0f - p) * xs[e * H + k];
-        state[o] = out;
+        store_envs<TM>(h_out + (size_t)(u0 + ul + u) * n + e0 + el, h);
+    }
+#pragma unroll
+    for (int e = 0; e < TM; e++) {
+        const size_t o = (size_t)(e0 + el + e) * H + u0 + ul;
+        if (s_aligned) {
+            *reinterpret_cast<float4*>(state + o) = make_float4(st[e][0], st[e][1], st[e][2], st[e][3]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; u++) state[o + u] = st[e][u];
+        }
     }
 }
 
 // ---------------------------------------------------------------- heads
-// logits_av[e][a] = bias[a] + sum_j W_av[a][j] * h[e][j] (ascending j); row A
-// is the value head.  Accumulator starts at the bias as in the scalar
-// reference (craftax_full.cu:9838-9845).
-constexpr int HEAD_ENVS = 8;
+// logits_av[e][a] = bias[a] + sum_j W_av[a][j] * h[j][e] (ascending j); row A is the value head.
+// Accumulator starts at the bias as in the scalar reference (craftax_full.cu:9838-9845).  A block
+// takes 32 envs; a lane owns 2 envs x 3 rows, a warp 16 envs x 12 rows.  The 32 columns of h and the head
+// matrix are staged in shared memory with every load in flight at once.
+constexpr int kHeadEnvs = 32, kHeadRows = 12, kHeadLaneRows = 3;
+constexpr int head_row_groups(int A) { return (A + 1 + kHeadRows - 1) / kHeadRows; }
+constexpr int head_threads(int A) { return 64 * head_row_groups(A); }
+constexpr size_t head_smem(int H, int A) {
+    return ((size_t)kHeadEnvs * H + (size_t)head_row_groups(A) * kHeadRows * (H + 4)) * sizeof(float);
+}
 
-__global__ void k_heads_fp32(const float* __restrict__ h, const float* __restrict__ W_a,
-                             const float* __restrict__ b_a, const float* __restrict__ W_v,
-                             const float* __restrict__ b_v, float* __restrict__ logits_av,
-                             int n, int H, int A) {
-    extern __shared__ float hs[];  // [HEAD_ENVS][H]
-    const int e0 = blockIdx.x * HEAD_ENVS;
-    for (int i = threadIdx.x; i < HEAD_ENVS * H; i += blockDim.x) {
-        int e = i / H;
-        hs[i] = (e0 + e < n) ? h[(size_t)e0 * H + i] : 0.0f;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < HEAD_ENVS * (A + 1); i += blockDim.x) {
-        const int e = i / (A + 1), a = i % (A + 1);
-        if (e0 + e >= n) continue;
+__global__ void __launch_bounds__(384) k_heads_fp32(const float* __restrict__ h, const float* __restrict__ W_a,
+                                                    const float* __restrict__ b_a, const float* __restrict__ W_v,
+                                                    const float* __restrict__ b_v, float* __restrict__ logits_av,
+                                                    int n, int H, int A) {
+    extern __shared__ __align__(16) float hs[];   // h [H][32], then W [rows][H + 4]
+    float* wsh = hs + kHeadEnvs * H;
+    const int tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, lane = tid & 31;
+    const int e0 = blockIdx.x * kHeadEnvs, WS = H + 4;
+    wait_for_previous_kernel();
+    for (int i = tid; i < H * (kHeadEnvs / 4); i += T)
+        copy16(hs + 4 * i, h + (size_t)(i / (kHeadEnvs / 4)) * n + e0 + 4 * (i % (kHeadEnvs / 4)), true, true);
+    for (int a = warp; a < A + 1; a += T / 32) {
         const float* w = a < A ? W_a + (size_t)a * H : W_v;
-        float z = a < A ? b_a[a] : b_v[0];
-        const float* hv = hs + e * H;
-        for (int j = 0; j < H; j++) z = fmaf(w[j], hv[j], z);
-        logits_av[(size_t)(e0 + e) * (A + 1) + a] = z;
+        const bool al = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+        for (int j = 4 * lane; j < H; j += 128) copy16(wsh + a * WS + j, w + j, true, al);
     }
+    copy_commit();
+    const int a0 = (warp >> 1) * kHeadRows + (lane >> 3) * kHeadLaneRows, el = 16 * (warp & 1) + 2 * (lane & 7);
+    float z[kHeadLaneRows][2];
+#pragma unroll
+    for (int r = 0; r < kHeadLaneRows; r++)
+        z[r][0] = z[r][1] = a0 + r < A ? b_a[a0 + r] : b_v[0];
+    copy_wait<0>();
+    __syncthreads();
+#pragma unroll 4
+    for (int j = 0; j < H; j += 4) {
+        float w[kHeadLaneRows][4];
+#pragma unroll
+        for (int r = 0; r < kHeadLaneRows; r++) {
+            const float4 v = *reinterpret_cast<const float4*>(wsh + (a0 + r) * WS + j);
+            w[r][0] = v.x; w[r][1] = v.y; w[r][2] = v.z; w[r][3] = v.w;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float2 x = *reinterpret_cast<const float2*>(hs + (j + q) * kHeadEnvs + el);
+#pragma unroll
+            for (int r = 0; r < kHeadLaneRows; r++) {
+                z[r][0] = fmaf(w[r][q], x.x, z[r][0]);
+                z[r][1] = fmaf(w[r][q], x.y, z[r][1]);
+            }
+        }
+    }
+    __syncthreads();   // the h columns are used up: the logits take their place
+#pragma unroll
+    for (int r = 0; r < kHeadLaneRows; r++)
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+            if (a0 + r < A + 1) hs[(el + e) * (A + 1) + a0 + r] = z[r][e];
+    __syncthreads();
+    for (int i = tid; i < kHeadEnvs * (A + 1); i += T) logits_av[(size_t)e0 * (A + 1) + i] = hs[i];
 }
 
 // ---------------------------------------------------------------- sampler
-// One thread per env (k_value_sample, craftax_full.cu:9714-9741); logits
-// already carry their biases.
-__global__ void k_sample(const float* __restrict__ logits, int ld, int A,
-                         const float* __restrict__ uniforms, uint64_t seed, uint64_t env_offset,
-                         const unsigned long long* __restrict__ step_ctr, int n,
-                         float* __restrict__ env_actions, int32_t* __restrict__ actions,
-                         float* __restrict__ logprobs, float* __restrict__ values) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    const float* l = logits + (size_t)e * ld;
-    float u;
-    if (uniforms != nullptr) u = uniforms[e];
-    else u = philox_uniform(seed, env_offset + (uint64_t)e, step_ctr ? *step_ctr : 0ULL);
-    float lp;
-    const int a = sample_action_dyn(l, A, u, &lp);
-    if (env_actions) env_actions[e] = (float)a;
-    if (actions) actions[e] = a;
-    if (logprobs) logprobs[e] = lp;
-    if (values) values[e] = l[A];
+// k_value_sample (craftax_full.cu:9714-9741); logits already carry their biases.  A block of 128
+// threads takes 32 envs: the rows come in coalesced, four threads of an env take its maximum and its
+// exponentials (both independent of order), one thread adds them up in the reference's order.
+// `ctr` (optional): device step counter {offset, blocks finished}; with `bump` the last block raises it.
+constexpr int kSampleEnvs = 32, kSampleThreads = 128;
+
+__global__ void __launch_bounds__(kSampleThreads)
+k_sample(const float* __restrict__ logits, int ld, int A, const float* __restrict__ uniforms, uint64_t seed,
+         uint64_t env_offset, unsigned long long* ctr, int bump, int n, float* __restrict__ env_actions,
+         int32_t* __restrict__ actions, float* __restrict__ logprobs, float* __restrict__ values) {
+    __shared__ float l[kSampleEnvs][kMaxActions + 2], p[kSampleEnvs][kMaxActions + 2];   // odd row length
+    const int tid = threadIdx.x, e0 = blockIdx.x * kSampleEnvs;
+    const int cols = values != nullptr ? A + 1 : A;
+    wait_for_previous_kernel();
+    const int envs = min(kSampleEnvs, n - e0);
+    for (int i = tid; i < envs * cols; i += kSampleThreads)
+        l[i / cols][i % cols] = logits[(size_t)(e0 + i / cols) * ld + i % cols];
+    const int e = tid >> 2, part = tid & 3;   // env and quarter of its actions
+    float u = 0.0f;
+    if (part == 0 && e < envs)
+        u = uniforms != nullptr ? uniforms[e0 + e]
+                                : philox_uniform(seed, env_offset + (uint64_t)(e0 + e), ctr ? *ctr : 0ULL);
+    __syncthreads();
+    float m = -INFINITY;
+    if (e < envs)
+        for (int a = part; a < A; a += 4) m = fmaxf(m, l[e][a]);
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if (e < envs)
+        for (int a = part; a < A; a += 4) p[e][a] = expf(l[e][a] - m);
+    __syncwarp();
+    if (part == 0 && e < envs) {
+        float lp;
+        const int a = pick_action(l[e], p[e], A, m, u, &lp);
+        const int env = e0 + e;
+        if (env_actions) env_actions[env] = (float)a;
+        if (actions) actions[env] = a;
+        if (logprobs) logprobs[env] = lp;
+        if (values) values[env] = l[e][A];
+    }
+    if (bump) {
+        __syncthreads();   // this block has read the counter
+        if (tid == 0) {
+            __threadfence();
+            if (atomicAdd(ctr + 1, 1ULL) == gridDim.x - 1) {
+                ctr[0] += 1ULL;
+                ctr[1] = 0ULL;
+            }
+        }
+    }
 }
 
 __global__ void k_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, float* u) {
@@ -280,6 +585,24 @@ __global__ void k_init_uniform(float* w, int count, float bound, uint64_t seed, 
 }
 
 // ---------------------------------------------------------------- launchers
+// Launch with programmatic stream serialisation (see wait_for_previous_kernel): the launch and the
+// start-up of a kernel run under the kernel in front of it.
+template <typename... P, typename... Args>
+static int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CFX_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return CFX_OK;
+}
+
 int launch_expand(const uint8_t* rec, float* out, int n, cudaStream_t st) {
     size_t total = (size_t)n * kObs;
     k_expand<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(rec, out, n);
@@ -300,13 +623,11 @@ int launch_done_to_terminals(const int8_t* done, float* out, int n, cudaStream_t
 }
 
 int launch_sample(const float* logits, int ld, int A, const float* u, uint64_t seed,
-                  uint64_t env_offset, const unsigned long long* step_ctr, int n,
+                  uint64_t env_offset, unsigned long long* step_ctr, int bump, int n,
                   float* env_actions, int32_t* actions, float* logprobs, float* values,
                   cudaStream_t st) {
-    k_sample<<<(n + 127) / 128, 128, 0, st>>>(logits, ld, A, u, seed, env_offset, step_ctr, n,
-                                              env_actions, actions, logprobs, values);
-    CFX_CUDA(cudaGetLastError());
-    return CFX_OK;
+    return launch_chained(k_sample, dim3((n + kSampleEnvs - 1) / kSampleEnvs), kSampleThreads, 0, st, logits, ld, A, u,
+                          seed, env_offset, step_ctr, bump, n, env_actions, actions, logprobs, values);
 }
 
 int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, float* u, cudaStream_t st) {
@@ -334,41 +655,84 @@ int launch_init_uniform(float* w, int count, float bound, uint64_t seed, int sub
     return CFX_OK;
 }
 
-// Full strict forward.  scratch_h: two [n][H] fp32 buffers; logits_av [n][A+1].
+// Tiles by the number q of warps that 8 envs x 4 units a lane would give (the GPU has 592 SM schedulers).
+// A layer takes 8 envs a lane from q = 1,024 (4,096 envs at hidden 256: 152 us a forward, 154 with 4; at 3,072 envs
+// 152 against 134), 4 below, and 1 under 96, where even the 4-env tiles leave schedulers without a warp
+// (256 envs: 55 against 71 us; 512 envs: 77 against 72).
+static int strict_tile(long long q) { return q >= 1024 ? 8 : (q >= 96 ? 4 : 1); }
+// The encoder has a third of a layer's units: envs x groups of 4 units a lane, 1 x 1, 4 x 1, 4 x 2 and 8 x 2 (2,048 envs
+// at hidden 256, q = 512: 102, 97 and 113 us a forward with the last three; 1,024 envs: 73, 80 and 94).
+static int strict_encoder_tile(long long q) { return q >= 640 ? 82 : (q >= 400 ? 42 : (q >= 96 ? 41 : 11)); }
+
+template <int TM, int G>
+static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, cudaStream_t st) {
+    using E = Enc<TM, G>;
+    if (E::kSmem > 48 * 1024)
+        CFX_CUDA(cudaFuncSetAttribute(k_encoder_fp32<TM, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, E::kSmem));
+    return launch_chained(k_encoder_fp32<TM, G>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
+                          a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], a.n, a.H,
+                          ((uintptr_t)(a.params + o.w_enc) & 15) == 0);
+}
+
+template <int TM, int WM, int WU>
+static int strict_layers(const StrictArgs& a, const ArenaLayout& o, cudaStream_t st, int* cnt) {
+    const int H = a.H, n = a.n;
+    constexpr int BM = 4 * TM * WM, BU = 32 * WU, T = 32 * WM * WU;
+    constexpr int smem = kGruStages * gru_stage_floats<TM, WM, WU>() * (int)sizeof(float);
+    if (smem > 48 * 1024)
+        CFX_CUDA(cudaFuncSetAttribute(k_mingru_fp32<TM, WM, WU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const dim3 grid((n + BM - 1) / BM, H / BU);
+    int rc;
+    const int s_aligned = ((uintptr_t)a.state & 15) == 0;
+    for (int l = 0; l < a.L; l++) {
+        float* r = a.r_state ? reinterpret_cast<float*>(reinterpret_cast<char*>(a.r_state) +
+                                                        (size_t)l * n * H * (a.r_state_bf16 ? 2 : 4))
+                             : nullptr;
+        rc = launch_chained(k_mingru_fp32<TM, WM, WU>, grid, T, smem, st, a.scratch_h[l & 1],
+                            a.gates_t + (size_t)l * 3 * H * H, a.state + (size_t)l * n * H, a.prev_terminals,
+                            a.scratch_h[(l + 1) & 1], r, a.r_state_bf16, n, H, s_aligned);
+        if (rc) return rc;
+    }
+    *cnt += a.L;
+    return CFX_OK;
+}
+
+// Full strict forward.  scratch_h: two [H][n] fp32 buffers; logits_av [n][A+1].
 int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     const int H = a.H, L = a.L, A = a.A, n = a.n;
     const ArenaLayout o = ArenaLayout::make(H, L, A, a.game == CFX_GAME_CLASSIC ? kClassicObs : kObs);
-    int cnt = 0;
-    if (a.game == CFX_GAME_CLASSIC)
-        k_classic_encoder_fp32<<<n, H, 0, st>>>(a.records, a.params + o.w_enc, a.params + o.b_enc,
-                                                a.scratch_h[0], n, H);
-    else
-        k_encoder_fp32<<<(n + ENC_ENVS - 1) / ENC_ENVS, H, 0, st>>>(
-            a.records, a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], n, H);
-    cnt++;
-    const float* x = a.scratch_h[0];
-    for (int l = 0; l < L; l++) {
-        float* out = a.scratch_h[(l + 1) & 1];
-        k_mingru_fp32<<<(n + GRU_ENVS - 1) / GRU_ENVS, H, GRU_ENVS * H * sizeof(float), st>>>(
-            x, a.gates_t + (size_t)l * 3 * H * H, a.state + (size_t)l * n * H, a.prev_terminals,
-            out,
-            a.r_state ? reinterpret_cast<float*>(reinterpret_cast<char*>(a.r_state) +
-                                                 (size_t)l * n * H * (a.r_state_bf16 ? 2 : 4))
-                      : nullptr,
-            a.r_state_bf16, n, H);
-        cnt++;
-        x = out;
+    int cnt = 0, rc;
+    const long long q = (long long)n * H / 1024;
+    if (a.game == CFX_GAME_CLASSIC) {
+        rc = launch_chained(k_classic_encoder_fp32, dim3(n), H, 0, st, a.records, a.params + o.w_enc, a.params + o.b_enc,
+                            a.scratch_h[0], n, H);
+    } else {
+        const int te = strict_encoder_tile(q);
+        if (te == 11) rc = strict_encoder<1, 1>(a, o, st);
+        else if (te == 41 || H % 64 != 0) rc = strict_encoder<4, 1>(a, o, st);
+        else rc = te == 42 ? strict_encoder<4, 2>(a, o, st) : strict_encoder<8, 2>(a, o, st);
     }
-    k_heads_fp32<<<(n + HEAD_ENVS - 1) / HEAD_ENVS, 128, HEAD_ENVS * H * sizeof(float), st>>>(
-        x, a.params + o.w_a, a.params + o.b_a, a.params + o.w_v, a.params + o.b_v,
-        a.logits_av, n, H, A);
+    if (rc) return rc;
     cnt++;
-    k_sample<<<(n + 127) / 128, 128, 0, st>>>(a.logits_av, A + 1, A, a.uniforms, a.seed,
-                                              a.env_offset, a.step_ctr, n, a.env_actions,
-                                              a.actions, a.logprobs, a.values);
-    cnt++;
-    CFX_CUDA(cudaGetLastError());
-    if (launches) *launches = cnt;
+    // a hidden size that is an odd multiple of 32 has the warps of a block side by side along the envs
+    const int tm = strict_tile(q);
+    if (H % 64 == 0)
+        rc = tm == 8 ? strict_layers<8, 2, 2>(a, o, st, &cnt) : tm == 4 ? strict_layers<4, 2, 2>(a, o, st, &cnt)
+                                                              : strict_layers<1, 2, 2>(a, o, st, &cnt);
+    else
+        rc = tm == 8 ? strict_layers<8, 4, 1>(a, o, st, &cnt) : tm == 4 ? strict_layers<4, 4, 1>(a, o, st, &cnt)
+                                                              : strict_layers<1, 4, 1>(a, o, st, &cnt);
+    if (rc) return rc;
+    const size_t hsmem = head_smem(H, A);
+    if (hsmem > 48 * 1024)
+        CFX_CUDA(cudaFuncSetAttribute(k_heads_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+    rc = launch_chained(k_heads_fp32, dim3(n / kHeadEnvs), head_threads(A), hsmem, st, a.scratch_h[L & 1],
+                        a.params + o.w_a, a.params + o.b_a, a.params + o.w_v, a.params + o.b_v, a.logits_av, n, H, A);
+    if (rc) return rc;
+    rc = launch_sample(a.logits_av, A + 1, A, a.uniforms, a.seed, a.env_offset, a.step_ctr, a.bump_step, n,
+                       a.env_actions, a.actions, a.logprobs, a.values, st);
+    if (rc) return rc;
+    if (launches) *launches = cnt + 2;
     return CFX_OK;
 }
 
@@ -469,6 +833,6 @@ extern "C" int cfx_strict_forward_static(int device, const float* params, int hi
     a.values = io->values;
     a.seed = io->seed;
     a.env_offset = io->env_offset;
-    a.step_ctr = reinterpret_cast<const unsigned long long*>(step_ctr);
+    a.step_ctr = reinterpret_cast<unsigned long long*>(const_cast<uint64_t*>(step_ctr));   // read only: no bump
     return strict_forward(a, st, nullptr);
 }

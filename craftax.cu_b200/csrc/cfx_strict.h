@@ -14,7 +14,7 @@ struct StrictArgs {
     const float* prev_terminals;
     const float* uniforms;
     float* state;           // [L][n][H]
-    float* scratch_h[2];    // [n][H] each
+    float* scratch_h[2];    // [H][n] each, 16-byte aligned
     float* logits_av;       // [n][A+1]
     float* r_state;
     int r_state_bf16 = 0;   // r_state holds bf16 instead of fp32
@@ -23,7 +23,8 @@ struct StrictArgs {
     float* logprobs;
     float* values;
     uint64_t seed, env_offset;
-    const unsigned long long* step_ctr;
+    unsigned long long* step_ctr;   // {Philox offset, blocks finished (bump_step)}
+    int bump_step = 0;      // raise the offset after the forward
 };
 
 int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches);
@@ -31,7 +32,7 @@ int launch_expand(const uint8_t* rec, float* out, int n, cudaStream_t st);
 int launch_classic_expand(const uint8_t* rec, float* out, int n, cudaStream_t st);
 int launch_done_to_terminals(const int8_t* done, float* out, int n, cudaStream_t st);
 int launch_sample(const float* logits, int ld, int A, const float* u, uint64_t seed,
-                  uint64_t env_offset, const unsigned long long* step_ctr, int n,
+                  uint64_t env_offset, unsigned long long* step_ctr, int bump, int n,
                   float* env_actions, int32_t* actions, float* logprobs, float* values,
                   cudaStream_t st);
 int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, float* u, cudaStream_t st);

@@ -1,0 +1,66 @@
+"""Every tile shape of the fp32 layer kernels against the CPU oracle, at batch sizes that end inside
+a tile, and the allocation-free variant on arrays that are only 4-byte aligned."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+A = 43
+
+
+def _inputs(oracle, n, H, L):
+    rng = np.random.default_rng(n + H)
+    return (oracle.synthetic_records(n, seed=4), oracle.init_weights(H, L, A, seed=5, scheme="uniform"),
+            rng.normal(0, 1, (L, n, H)).astype(np.float32), (rng.random(n) < 0.3).astype(np.float32),
+            rng.random(n, dtype=np.float32))
+
+
+def _close(got, want):
+    # both sides sum in the same order; they differ in expf and its neighbours (2 ulp each), which
+    # the layers pass on: 3e-5 of the largest value, as for the other shapes of this mode
+    assert np.abs(got - want).max() < 3e-5 * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("n,H,L", [(32, 32, 1),       # 1 env a lane, one unit tile
+                                   (416, 256, 1),     # 4 envs a lane (warps of q = 104)
+                                   (1632, 256, 2),    # encoder 4 x 2
+                                   (2592, 256, 1),    # encoder 8 x 2, ragged
+                                   (4128, 256, 2),    # 8 envs a lane, ragged
+                                   (1056, 96, 2), (11040, 96, 1)])   # warps along the envs
+def test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L):
+    rec, params, state, prev_t, u = _inputs(oracle, n, H, L)
+    pol = cfx.Policy(n, H, L, A, "fp32")
+    pol.set_weights(params)
+    pol.set_state(state)
+    pol.step = 7
+    d = pol.forward_host(rec, prev_t, u, want_r_state=True, bump_step=True)
+    st = state.copy()
+    lav, rs = oracle.forward(params, rec, prev_t, st, H, L, A, want_r_state=True)
+    _close(d["logits_av"], lav)
+    _close(pol.get_state(), st)
+    assert np.array_equal(d["r_state"], rs)
+    assert pol.step == 8     # raised by the sampler's last block
+    a, lp = oracle.sample(d["logits_av"][:, :A], u)
+    assert (d["actions"] != a).sum() <= 1    # a boundary of the distribution within rounding of its uniform
+    same = d["actions"] == a
+    assert np.abs(d["logprobs"][same] - lp[same]).max() < 1e-5
+    pol.close()
+
+
+def test_static_forward_takes_arrays_of_any_word_alignment(cfx, gpu, oracle):
+    n, H, L = 96, 256, 2
+    rec, params, state, prev_t, u = _inputs(oracle, n, H, L)
+
+    def shifted(a):   # device copy that starts 4 bytes past an aligned address
+        return cfx.DeviceBuffer.from_host(np.concatenate([np.zeros(1, np.float32), a.ravel()]))
+    d_par, d_st = shifted(params), shifted(state)
+    d_rec, d_pt, d_u = (cfx.DeviceBuffer.from_host(x) for x in (rec, prev_t, u))
+    d_act, d_lav = cfx.DeviceBuffer((n,), np.int32), cfx.DeviceBuffer((n, A + 1), np.float32)
+    io = cfx.ForwardIO(d_rec.ptr, d_pt.ptr, d_u.ptr, None, d_act.ptr, None, None, d_lav.ptr, None, 0, 0, 0, 0)
+    cfx.check(cfx.lib().cfx_strict_forward_static(0, d_par.ptr + 4, H, L, A, n, d_st.ptr + 4, C.byref(io), None, None))
+    cfx.check(cfx.lib().cfx_stream_sync(0, None))
+    st = state.copy()
+    lav = oracle.forward(params, rec, prev_t, st, H, L, A)
+    _close(d_lav.download(), lav)
+    _close(d_st.download()[1:].reshape(st.shape), st)
