@@ -77,4 +77,29 @@ struct DeviceGuard {
         }                                                                                \
     } while (0)
 
+// Kernels launched with programmatic stream serialisation: the launch and the start-up of a kernel run
+// under the kernel in front of it in the stream, and it waits here until the results of that kernel are in
+// memory.  Nothing that another kernel may have written is read before.  The small kernels do not
+// let the next one start early (griddepcontrol.launch_dependents): its blocks would fill the SMs that this
+// kernel's last blocks leave free and pile up there (fp32 forward, 4,096 envs: 227 us against 178).
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... Args>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CFX_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return CFX_OK;
+}
+#endif
+
 }  // namespace cfx

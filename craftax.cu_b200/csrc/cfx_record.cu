@@ -3,36 +3,40 @@
 //
 // The reference gives every env a warp and lets lane 0 walk the mob slots and compute the 51
 // tail scalars; every one of its ~110 scalar loads then fetches 4 bytes of a sector on its own,
-// one after the other.  Here a block of four warps owns 32 consecutive envs and works in two
-// phases:
-//   1. lane per env: the ~50 SoA fields and the 14 mob slots of the player's level (type, mask,
-//      position, light at the position) are loaded by lane e for env e, so that a warp's loads
-//      of a field are one 128-byte line and all loads of a lane are independent; each warp takes
-//      a quarter of the fields; they leave the 51 tail floats, the visible mobs (an earlier slot
-//      of a class that a later slot covers is dropped) and (level, top, left) in shared memory;
-//   2. warp per env (8 envs per warp, the next env's loads in flight while one is stored): the
-//      99 view cells, 8 bytes each from three byte maps, go out as coalesced 8-byte stores,
-//      then one lane per visible mob stores its byte, then the tail goes out as coalesced
-//      4-byte stores from shared memory.
+// one after the other.  Here a block of eight warps owns 32 consecutive envs:
+//   1. the view of an env is 9 rows of 11 bytes, 48 bytes apart: at most 410 contiguous bytes of each of
+//      three map planes.  Every warp starts asynchronous 16-byte copies of its four envs' spans to shared
+//      memory, all twelve in flight;
+//   2. meanwhile, lane per env: the ~50 SoA fields and the 14 mob slots of the player's level are loaded
+//      by lane e for env e, so that a warp's loads of a field are one 128-byte line, each warp an eighth
+//      of them, all of a lane's in flight; they leave the 51 tail floats and the mobs (an earlier
+//      slot of a class that a later slot covers is dropped) in shared memory;
+//   3. warp per env: a lane makes four cells of a view row from the spans in registers, the four records
+//      are put together where the spans were, and go out as one bulk copy (1,992 blocks of 16 bytes a
+//      block) or, where an env is skipped, as coalesced words.
+// Before: a byte load per cell and map, two half-used store instructions per 32 cells, the fields one DRAM
+// latency after the other (see ld_now), a read of the light map per mob behind them.  65,536 envs with 62 KB of maps
+// each: 54.7 -> 49 us (16,384 envs: 24.9 -> 14.9 us); 182 MB of DRAM traffic instead of 204, bound by
+// the scattered pieces: 3.7 TB/s whatever the mix, and the time adds up over writes, spans and fields.
 // The bytes are the reference's: the same predicates, the same "last slot of a class wins a
 // cell" order, the same float expressions (sqrtf(x) * 0.1f, x * 0.1f, x * 0.5f, x * 0.25f; no
-// fused multiply-add can form).  HBM traffic per env: 996 B written, 27 map sectors (9 rows of
-// 11 bytes in three maps) and ~100 SoA words read.
+// fused multiply-add can form).
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <type_traits>
 
 #include "cfx_common.cuh"
 
 namespace cfx {
 namespace record {
 
-constexpr int kRows = 9, kCols = 11, kCells = kRows * kCols;   // view around the player
+constexpr int kRows = 9, kCols = 11;   // view around the player
 constexpr int kMapSize = 48, kLevels = 9, kMobTypes = 8, kClasses = 5, kSlots = 3;
 constexpr int kMobs = kClasses * kSlots;                       // slot 2 of class 2 is never used
 constexpr int kLit = 12;                                       // light_map > 12 = visible
 constexpr int kKilledToClear = 8;
-constexpr int kBlockEnvs = 32, kBlockThreads = 128;
+constexpr int kBlockEnvs = 32, kBlockThreads = 256;
 
 struct Params {
     cfx_env_view v;
@@ -43,11 +47,17 @@ struct Params {
     const int* count_dev;
     int n;
 };
+constexpr int kSpan = 416, kPlanes = 3;   // 8 rows x 48 + 11 bytes, plus 15 to the boundary before: 410
+constexpr int kWarps = kBlockThreads / 32, kOwn = kBlockEnvs / kWarps;   // envs whose records a warp writes
+constexpr int kPlaneBytes = kMapSize * kMapSize, kRecWords = kRec / 4, kMapWords = kMap / 4;
 struct Shared {
     float tail[kBlockEnvs][kTail];       // odd row length: conflict-free thread-per-env writes
     uint32_t mobs[kBlockEnvs][kMobs];
-    int32_t level[kBlockEnvs], top[kBlockEnvs], left[kBlockEnvs], env[kBlockEnvs];   // env < 0: nothing to write
+    // per warp the spans of its four envs (light, block, item; words before and after are read, and masked), and in their
+    // place, once they are in registers, its four records as they go out
+    __align__(16) uint8_t span[kWarps][kOwn][kPlanes][kSpan];
 };
+static_assert(kOwn * kRec % 16 == 0 && kRec <= kPlanes * kSpan, "a warp's records are whole 16-byte words");
 
 // craftax_wg_jax_index (:1963-1975): negative indices wrap once, then clamp
 __device__ __forceinline__ int jax_index(int i, int size) {
@@ -55,190 +65,444 @@ __device__ __forceinline__ int jax_index(int i, int size) {
     if (i < 0) return 0;
     return i >= size ? size - 1 : i;
 }
+// Loads that are issued where they stand.  A plain load through a pointer of the view may alias the shared memory
+// that is written in between, so the compiler keeps load, conversion and store of every field in order, one DRAM
+// latency a field; a read-only load it sinks to its use, with the same effect.  Every loop below
+// therefore loads all its fields first.
+__device__ __forceinline__ uint32_t ld_bits(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int32_t ld_now(const int32_t* p) { return (int32_t)ld_bits(reinterpret_cast<const uint32_t*>(p)); }
+__device__ __forceinline__ uint32_t ld_now(const uint32_t* p) { return ld_bits(p); }
+__device__ __forceinline__ float ld_now(const float* p) { return __uint_as_float(ld_bits(reinterpret_cast<const uint32_t*>(p))); }
+__device__ __forceinline__ uint8_t ld_now(const uint8_t* p) {
+    uint16_t v;
+    asm volatile("ld.global.nc.u8 %0, [%1];" : "=h"(v) : "l"(p));
+    return (uint8_t)v;
+}
+__device__ __forceinline__ int8_t ld_now(const int8_t* p) { return (int8_t)ld_now(reinterpret_cast<const uint8_t*>(p)); }
+__device__ __forceinline__ int16_t ld_now(const int16_t* p) {
+    int16_t v;
+    asm volatile("ld.global.nc.s16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
 template <typename T>
 __device__ __forceinline__ T soa(const T* f, int elem, int n, int e) {
-    return f[(size_t)elem * (size_t)n + (size_t)e];
+    return ld_now(f + ((size_t)elem * (size_t)n + (size_t)e));
 }
 // flat index of (class, level, slot) in the mob fields (CFM, :715)
 __device__ __forceinline__ int mob_index(int c, int level, int i) { return (c * kLevels + level) * kSlots + i; }
 
-// phase 1: everything of env e that does not depend on the cell.  Lane t of EVERY warp of the
-// block works on env t of the block; warp `part` takes a quarter of the work:
-//   part 0: tail scalars 0-25        part 1: tail scalars 26-49
-//   part 2: mob classes 0-2 + the boss flag (tail scalar 50)        part 3: mob classes 3-4
-__device__ __forceinline__ void gather_env(const cfx_env_view& V, int e, int t, int part, Shared& S) {
+// a mob inside the view and on the map: valid | cell << 8 | channel << 4 | value
+__device__ __forceinline__ uint32_t pack_mob(int c, int type_id, bool mask, int mr, int mc, int top, int left) {
+    const int lr = mr - top, lc = mc - left;
+    const bool on = type_id >= 0 && type_id < kMobTypes && mask && lr >= 0 && lr < kRows && lc >= 0 && lc < kCols &&
+                    mr >= 0 && mr < kMapSize && mc >= 0 && mc < kMapSize;
+    return on ? 0x80000000u | (uint32_t)(lr * kCols + lc) << 8 | (uint32_t)(3 + c) << 4 | (uint32_t)(type_id + 1) : 0u;
+}
+__device__ __forceinline__ bool same_cell(uint32_t a, uint32_t b) {
+    return (a & b & 0x80000000u) && ((a ^ b) & 0xFF00u) == 0;
+}
+
+// the slots of mob class C; true if one of them is alive
+template <int C>
+__device__ __forceinline__ bool gather_mobs(const cfx_env_view& V, int e, int mob_level, int top, int left, uint32_t* mobs) {
+    constexpr int kN = C == 2 ? 2 : kSlots;   // slot 2 of class 2 is never used
     const int n = V.num_envs;
-    const int level = soa(V.player_level, 0, n, e);
-    float* o = S.tail[t];
-    int k = 0;
-    auto sq10 = [&](const int32_t* f, int i) { o[k++] = sqrtf((float)soa(f, i, n, e)) * (1.0f / 10.0f); };
-    auto mul = [&](const int32_t* f, int i, float m) { o[k++] = (float)soa(f, i, n, e) * m; };
-    auto flag = [&](bool b) { o[k++] = b ? 1.0f : 0.0f; };
-    // the 51 scalars in the order of craftax_encode_scalar_observation_tail_at (:2429-2487)
-    if (part == 0) {
-        sq10(V.inv_wood, 0); sq10(V.inv_stone, 0); sq10(V.inv_coal, 0); sq10(V.inv_iron, 0);
-        sq10(V.inv_diamond, 0); sq10(V.inv_sapphire, 0); sq10(V.inv_ruby, 0); sq10(V.inv_sapling, 0);
-        sq10(V.inv_torches, 0); sq10(V.inv_arrows, 0);
-        mul(V.inv_books, 0, 1.0f / 2.0f);
-        mul(V.inv_pickaxe, 0, 1.0f / 4.0f);
-        mul(V.inv_sword, 0, 1.0f / 4.0f);
-        o[k++] = (float)soa(V.sword_enchantment, 0, n, e);
-        o[k++] = (float)soa(V.bow_enchantment, 0, n, e);
-        o[k++] = (float)soa(V.inv_bow, 0, n, e);
+    int32_t type[kN], row[kN], col[kN];
+    uint8_t on[kN];
 #pragma unroll
-        for (int i = 0; i < 6; i++) sq10(V.inv_potions, i);
-        o[k++] = soa(V.player_health, 0, n, e) * (1.0f / 10.0f);
-        mul(V.player_food, 0, 1.0f / 10.0f); mul(V.player_drink, 0, 1.0f / 10.0f);
-        mul(V.player_energy, 0, 1.0f / 10.0f);   // scalar 25
-        return;
+    for (int i = 0; i < kN; i++) on[i] = soa(V.mob_mask, mob_index(C, mob_level, i), n, e);
+    // the rest of a slot only where a mob is alive: an env on another level than its neighbours reads a
+    // 64-byte burst for every word
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+        const int idx = mob_index(C, mob_level, i);
+        type[i] = row[i] = col[i] = -1;
+        if (on[i] != 0) {
+            type[i] = soa(V.mob_type_id, idx, n, e);
+            row[i] = soa(V.mob_position, idx * 2, n, e);
+            col[i] = soa(V.mob_position, idx * 2 + 1, n, e);
+        }
     }
-    if (part == 1) {
-        k = 26;
-        mul(V.player_mana, 0, 1.0f / 10.0f);
-        mul(V.player_xp, 0, 1.0f / 10.0f); mul(V.player_dexterity, 0, 1.0f / 10.0f);
-        mul(V.player_strength, 0, 1.0f / 10.0f); mul(V.player_intelligence, 0, 1.0f / 10.0f);
+    bool alive = false;
+    uint32_t pk[kSlots] = {0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+        alive = alive || on[i] != 0;
+        pk[i] = pack_mob(C, type[i], on[i] != 0, row[i], col[i], top, left);
+    }
+    // "last slot wins": a later slot of the class on the same cell replaces an earlier one
+    // (:9222-9231); the earlier one is dropped here, so the stores of phase 3 need no order
+#pragma unroll
+    for (int i = 0; i < kN - 1; i++)
+#pragma unroll
+        for (int i2 = i + 1; i2 < kN; i2++)
+            if (same_cell(pk[i], pk[i2])) pk[i] = 0;
+#pragma unroll
+    for (int i = 0; i < kSlots; i++) mobs[C * kSlots + i] = pk[i];
+    return alive;
+}
+
+// phase 2: everything of env e that does not depend on the cell.  Lane t of EVERY warp of the
+// block works on env t of the block; warp `part` takes an eighth of the loads.  The 51 scalars are in
+// the order of craftax_encode_scalar_observation_tail_at (:2429-2487).
+__device__ __forceinline__ void gather_env(const cfx_env_view& V, int e, int t, int part, int level, int top, int left,
+                                           Shared& S) {
+    const int n = V.num_envs;
+    float* o = S.tail[t];
+    // mobs of the player's level inside the view and on the map (:9195-9236).  Whether the cell is lit is
+    // looked up in the span when the record is put together: two slots on one cell are both lit or
+    // both not, so the order of dropping does not depend on it.
+    const int mob_level = jax_index(level, kLevels);
+    auto mobs = [&](auto... c) { return (gather_mobs<decltype(c)::value>(V, e, mob_level, top, left, S.mobs[t]) | ...); };
+    if (part == 0) {
+        const int32_t* const counts[10] = {V.inv_wood, V.inv_stone, V.inv_coal, V.inv_iron, V.inv_diamond, V.inv_sapphire,
+                                           V.inv_ruby, V.inv_sapling, V.inv_torches, V.inv_arrows};
+        int32_t a[10];
+#pragma unroll
+        for (int i = 0; i < 10; i++) a[i] = soa(counts[i], 0, n, e);
+        const int32_t books = soa(V.inv_books, 0, n, e), pickaxe = soa(V.inv_pickaxe, 0, n, e);
+#pragma unroll
+        for (int i = 0; i < 10; i++) o[i] = sqrtf((float)a[i]) * (1.0f / 10.0f);
+        o[10] = (float)books * (1.0f / 2.0f);
+        o[11] = (float)pickaxe * (1.0f / 4.0f);
+    } else if (part == 1) {
+        const int32_t sword = soa(V.inv_sword, 0, n, e);
+        const int32_t b[3] = {soa(V.sword_enchantment, 0, n, e), soa(V.bow_enchantment, 0, n, e), soa(V.inv_bow, 0, n, e)};
+        int32_t p[6];
+#pragma unroll
+        for (int i = 0; i < 6; i++) p[i] = soa(V.inv_potions, i, n, e);
+        const float health = soa(V.player_health, 0, n, e);
+        o[12] = (float)sword * (1.0f / 4.0f);
+#pragma unroll
+        for (int i = 0; i < 3; i++) o[13 + i] = (float)b[i];
+#pragma unroll
+        for (int i = 0; i < 6; i++) o[16 + i] = sqrtf((float)p[i]) * (1.0f / 10.0f);
+        o[22] = health * (1.0f / 10.0f);
+    } else if (part == 2) {
+        const int32_t* const tenths[8] = {V.player_food, V.player_drink, V.player_energy, V.player_mana, V.player_xp,
+                                          V.player_dexterity, V.player_strength, V.player_intelligence};
+        int32_t a[8], arm[4];
+#pragma unroll
+        for (int i = 0; i < 8; i++) a[i] = soa(tenths[i], 0, n, e);
         const int direction_index = soa(V.player_direction, 0, n, e) - 1;
 #pragma unroll
-        for (int i = 0; i < 4; i++) flag(i == direction_index);
+        for (int i = 0; i < 4; i++) arm[i] = soa(V.inv_armour, i, n, e);
 #pragma unroll
-        for (int i = 0; i < 4; i++) mul(V.inv_armour, i, 1.0f / 2.0f);
+        for (int i = 0; i < 8; i++) o[23 + i] = (float)a[i] * (1.0f / 10.0f);
 #pragma unroll
-        for (int i = 0; i < 4; i++) o[k++] = (float)soa(V.armour_enchantments, i, n, e);
-        o[k++] = soa(V.light_level, 0, n, e);
-        flag(soa(V.is_sleeping, 0, n, e) != 0);
-        flag(soa(V.is_resting, 0, n, e) != 0);
-        flag(soa(V.learned_spells, 0, n, e) != 0);
-        flag(soa(V.learned_spells, 1, n, e) != 0);
-        mul(V.player_level, 0, 1.0f / 10.0f);
-        flag((unsigned)level < (unsigned)kLevels && soa(V.monsters_killed, level, n, e) >= kKilledToClear);   // scalar 49
-        return;
-    }
-    // visible mobs of the player's level, class-major, slot-minor (:9195-9236):
-    // packed = valid | cell << 8 | channel << 4 | value
-    const int mob_level = jax_index(level, kLevels);
-    const int top = soa(V.player_position, 0, n, e) - kRows / 2;
-    const int left = soa(V.player_position, 1, n, e) - kCols / 2;
-    const uint8_t* light = V.state_base + (size_t)e * V.state_stride + V.light_map_offset +
-                           (size_t)mob_level * kMapSize * kMapSize;
-    const int c0 = part == 2 ? 0 : 3, c1 = part == 2 ? 3 : kClasses;
-    bool melee_or_ranged = false;
-    for (int c = c0; c < c1; c++) {
-        uint32_t pk[kSlots];
+        for (int i = 0; i < 4; i++) o[31 + i] = i == direction_index ? 1.0f : 0.0f;
 #pragma unroll
-        for (int i = 0; i < kSlots; i++) {
-            pk[i] = 0;
-            if (i < (c == 2 ? 2 : 3)) {
-                const int idx = mob_index(c, mob_level, i);
-                const int type_id = soa(V.mob_type_id, idx, n, e);
-                const bool mask = soa(V.mob_mask, idx, n, e) != 0;
-                if (c == 0 || c == 2) melee_or_ranged = melee_or_ranged || mask;
-                const int mr = soa(V.mob_position, idx * 2, n, e), mc = soa(V.mob_position, idx * 2 + 1, n, e);
-                const int lr = mr - top, lc = mc - left;
-                if (type_id >= 0 && type_id < kMobTypes && mask && lr >= 0 && lr < kRows && lc >= 0 && lc < kCols &&
-                    mr >= 0 && mr < kMapSize && mc >= 0 && mc < kMapSize && light[mr * kMapSize + mc] > kLit)
-                    pk[i] = 0x80000000u | (uint32_t)(lr * kCols + lc) << 8 | (uint32_t)(3 + c) << 4 |
-                            (uint32_t)(type_id + 1);
-            }
-        }
-        // "last slot wins": a later slot of the class on the same cell replaces an earlier one
-        // (:9222-9231); the earlier one is dropped here, so the stores of phase 2 need no order
+        for (int i = 0; i < 4; i++) o[35 + i] = (float)arm[i] * (1.0f / 2.0f);
+    } else if (part == 3) {
+        int32_t ench[4];
 #pragma unroll
-        for (int i = 0; i < kSlots - 1; i++)
+        for (int i = 0; i < 4; i++) ench[i] = soa(V.armour_enchantments, i, n, e);
+        const float light = soa(V.light_level, 0, n, e);
+        const uint8_t f[4] = {soa(V.is_sleeping, 0, n, e), soa(V.is_resting, 0, n, e), soa(V.learned_spells, 0, n, e),
+                              soa(V.learned_spells, 1, n, e)};
+        const bool level_ok = (unsigned)level < (unsigned)kLevels;
+        const int killed = soa(V.monsters_killed, level_ok ? level : 0, n, e);
 #pragma unroll
-            for (int i2 = i + 1; i2 < kSlots; i2++)
-                if ((pk[i] & pk[i2] & 0x80000000u) && ((pk[i] ^ pk[i2]) & 0xFF00u) == 0) pk[i] = 0;
+        for (int i = 0; i < 4; i++) o[39 + i] = (float)ench[i];
+        o[43] = light;
 #pragma unroll
-        for (int i = 0; i < kSlots; i++) S.mobs[t][c * kSlots + i] = pk[i];
-    }
-    if (part == 2) {
+        for (int i = 0; i < 4; i++) o[44 + i] = f[i] != 0 ? 1.0f : 0.0f;
+        o[48] = (float)level * (1.0f / 10.0f);
+        o[49] = level_ok && killed >= kKilledToClear ? 1.0f : 0.0f;
+    } else if (part == 4) {
+        const int32_t boss = soa(V.boss_timesteps_to_spawn_this_round, 0, n, e);
+        const bool melee_or_ranged = mobs(std::integral_constant<int, 0>(), std::integral_constant<int, 2>());
         // craftax_wg_is_boss_vulnerable (:1988-2003): no melee and no ranged mob alive on the level
-        o[kTail - 1] = !melee_or_ranged && soa(V.boss_timesteps_to_spawn_this_round, 0, n, e) <= 0 ? 1.0f : 0.0f;
+        o[50] = !melee_or_ranged && boss <= 0 ? 1.0f : 0.0f;
+    } else if (part == 5) {
+        mobs(std::integral_constant<int, 1>());
+    } else if (part == 6) {
+        mobs(std::integral_constant<int, 3>());
     } else {
-        S.level[t] = level; S.top[t] = top; S.left[t] = left;
+        mobs(std::integral_constant<int, 4>());
     }
 }
 
-// phase 2: the cells of one env.  The three byte loads per cell of all four rounds are issued
-// at once (load_cells); the caller holds them in registers while it stores the previous env.
-struct Cells { uint32_t l[4], b[4], it[4]; };
-__device__ __forceinline__ void load_cells(const cfx_env_view& V, const Shared& S, int t, int lane, Cells& c) {
-    const int e = S.env[t];
-    if (e < 0) return;
-    const int level = S.level[t], top = S.top[t], left = S.left[t];
-    const uint8_t* blk = V.state_base + (size_t)e * V.state_stride + (size_t)level * kMapSize * kMapSize;
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int cell = lane + 32 * r;
-        const int wr = top + cell / kCols, wc = left + cell % kCols;
-        // (a level outside [0, 9) never comes out of the env; the reference would read outside
-        // its maps there, here such an env gets unlit cells)
-        const bool in = cell < kCells && wr >= 0 && wr < kMapSize && wc >= 0 && wc < kMapSize &&
-                        (unsigned)level < (unsigned)kLevels;
-        const int o = in ? wr * kMapSize + wc : 0;
-        c.l[r] = in ? blk[V.light_map_offset + o] : 0u;
-        c.b[r] = in ? blk[V.map_offset + o] : 0u;
-        c.it[r] = in ? blk[V.item_map_offset + o] : 0u;
+// What the copies and the assembly of one env need, two words: the rows and columns of the view that are on the map are
+// contiguous in a plane from `first` (aligned down to what the copies move at a time, `grain` bytes).
+struct View {
+    uint32_t where;   // first | (top + 32) << 12 | (left + 32) << 19 | level in [0, 9) << 26
+    uint32_t plane;   // bytes to copy | level's plane << 16
+    __device__ __forceinline__ int first() const { return where & 0xFFF; }
+    __device__ __forceinline__ int top() const { return (int)(where >> 12 & 127u) - 32; }
+    __device__ __forceinline__ int left() const { return (int)(where >> 19 & 127u) - 32; }
+    __device__ __forceinline__ bool level_ok() const { return where >> 26; }
+    __device__ __forceinline__ int bytes() const { return plane & 0xFFFF; }
+    __device__ __forceinline__ int level() const { return plane >> 16; }
+};
+__device__ __forceinline__ View make_view(int level, int top, int left, int grain) {
+    top = min(max(top, -32), 64);      // (a view that is off the map stays off it)
+    left = min(max(left, -32), 64);
+    const int r0 = max(top, 0), r1 = min(top + kRows, kMapSize) - 1, c0 = max(left, 0), c1 = min(left + kCols, kMapSize) - 1;
+    int first = 0, bytes = 0;
+    if (r0 <= r1 && c0 <= c1) {
+        first = (r0 * kMapSize + c0) & ~(grain - 1);
+        bytes = r1 * kMapSize + c1 + 1 - first;
     }
+    View v;
+    v.where = (uint32_t)first | (uint32_t)(top + 32) << 12 | (uint32_t)(left + 32) << 19 |
+              ((unsigned)level < (unsigned)kLevels ? 1u << 26 : 0u);
+    v.plane = (uint32_t)bytes | (uint32_t)jax_index(level, kLevels) << 16;
+    return v;
 }
-// map cells: 8 bytes each {block, item + 1, lit, five mob classes}  (:9241-9269), then the tail
-__device__ __forceinline__ void store_env(const Params& P, const Shared& S, int t, int lane, const Cells& c) {
-    const int e = S.env[t];
-    if (e < 0) return;
-    uint8_t* rec = P.records + (size_t)e * kRec;
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int cell = lane + 32 * r;
-        if (cell < kCells) {
-            const uint32_t w0 = c.l[r] > (uint32_t)kLit ? (c.b[r] | ((c.it[r] + 1u) & 0xFFu) << 8 | 1u << 16) : 0u;
-            uint32_t* dst = reinterpret_cast<uint32_t*>(rec + (size_t)cell * 8);   // 4-byte aligned (996 = 4 x 249)
-            dst[0] = w0;
-            dst[1] = 0u;
+// Starts the copies of one env's three spans (light, block, item) into `dst`.  A plane is 2,304 bytes, so 16-byte
+// pieces (4-byte pieces) stay inside it where the planes are aligned to 16 (4) bytes.
+__device__ __forceinline__ void copy_spans(const cfx_env_view& V, int e, View v, int grain, int lane, uint8_t (*dst)[kSpan]) {
+    const uint8_t* q = V.state_base + (size_t)e * V.state_stride + (v.level() * kPlaneBytes + v.first());
+    auto plane = [&](const uint8_t* src, uint8_t* d) {
+        const uint32_t ds = (uint32_t)__cvta_generic_to_shared(d);
+        if (grain == 16) {
+            const int o = 16 * lane;
+            if (o < v.bytes()) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ds + o), "l"(src + o) : "memory");
+        } else if (grain == 4) {
+            for (int o = 4 * lane; o < v.bytes(); o += 128)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(ds + o), "l"(src + o) : "memory");
+        } else {
+            for (int o = lane; o < v.bytes(); o += 32) d[o] = ld_now(src + o);
         }
-    }
-    __syncwarp();   // the mob bytes land on cells other lanes have just written
-    if (lane < kMobs) {
-        const uint32_t pk = S.mobs[t][lane];
-        if (pk & 0x80000000u) rec[(size_t)((pk >> 8) & 0xFFu) * 8 + ((pk >> 4) & 0xFu)] = (uint8_t)(pk & 0xFu);
-    }
-    for (int j = lane; j < kTail; j += 32) *reinterpret_cast<float*>(rec + kMap + 4 * j) = S.tail[t][j];
+    };
+    plane(q + V.light_map_offset, dst[0]);
+    plane(q + V.map_offset, dst[1]);
+    plane(q + V.item_map_offset, dst[2]);
 }
-// warp `warp` writes envs warp, warp + 4, ... of the block, loading one env ahead
-__device__ __forceinline__ void write_envs(const Params& P, const Shared& S, int warp, int lane) {
-    constexpr int kWarps = kBlockThreads / 32;
-    Cells cur, nxt;
-    load_cells(P.v, S, warp, lane, cur);
-    for (int k = warp; k < kBlockEnvs; k += kWarps) {
-        if (k + kWarps < kBlockEnvs) load_cells(P.v, S, k + kWarps, lane, nxt);
-        store_env(P, S, k, lane, cur);
-        if (k + kWarps < kBlockEnvs) cur = nxt;
-    }
+__device__ __forceinline__ void wait_spans() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+}
+__device__ __forceinline__ int copy_grain(const cfx_env_view& V) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(V.state_base) | V.state_stride | V.map_offset | V.item_map_offset | V.light_map_offset;
+    return (a & 15) == 0 ? 16 : ((a & 3) == 0 ? 4 : 1);
 }
 
-__global__ void __launch_bounds__(kBlockThreads) k_record_rows(const __grid_constant__ Params P) {
-    __shared__ Shared S;   // 9 KB
+// phase 3: the map cells of an env's record from its spans, 8 bytes each {block, item + 1, lit, five mob
+// classes} (:9241-9269).  A lane takes four cells of a row, bytes side by side in the spans.
+__device__ __forceinline__ uint32_t span_word(const uint8_t* span, int o) {   // bytes o .. o + 3
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(span + (o & ~3));
+    return __funnelshift_r(w[0], w[1], 8 * (o & 3));
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {   // (__byte_perm drops the sign bit of a selector)
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+}
+__device__ __forceinline__ uint32_t low_bytes(int k) { return k <= 0 ? 0u : (k >= 4 ? ~0u : (1u << 8 * k) - 1u); }
+struct Cells { uint32_t w[4]; };   // first words of this lane's cells; the second ones hold mobs only
+constexpr int kGroups = (kCols + 3) / 4;
+static_assert(kRows * kGroups <= 32, "a lane a group");
+__device__ __forceinline__ Cells make_cells(View v, int lane, const uint8_t (*span)[kSpan]) {
+    const int dr = lane / kGroups, g = lane % kGroups, row = v.top() + dr, col = v.left() + 4 * g;
+    Cells c = {{0u, 0u, 0u, 0u}};
+    // (a level outside [0, 9) never comes out of the env; the reference would read outside
+    // its maps there, here such an env gets unlit cells)
+    if (dr >= kRows || (unsigned)row >= (unsigned)kMapSize || v.bytes() == 0 || !v.level_ok()) return c;
+    const int o = row * kMapSize + col - v.first();
+    const uint32_t in = low_bytes(min(kMapSize - col, kCols - 4 * g)) & ~low_bytes(-col);
+    const uint32_t lit = __vcmpgtu4(span_word(span[0], o), kLit * 0x01010101u) & in;
+    const uint32_t b = span_word(span[1], o) & lit, it = __vadd4(span_word(span[2], o), 0x01010101u) & lit;
+    const uint32_t one = lit & 0x01010101u, lo = __byte_perm(b, it, 0x5140), hi = __byte_perm(b, it, 0x7362);
+    c.w[0] = prmt(lo, one, 0xC410);   // {block, item, lit, 0}: selector 8 + i repeats the sign of byte i, here 0
+    c.w[1] = prmt(lo, one, 0xD532);
+    c.w[2] = prmt(hi, one, 0xE610);
+    c.w[3] = prmt(hi, one, 0xF732);
+    return c;
+}
+__device__ __forceinline__ void put_cells(const Cells& c, int lane, uint32_t* rec) {
+    const int dr = lane / kGroups, g = lane % kGroups;
+    if (dr >= kRows) return;
+    uint32_t* d = rec + 2 * (dr * kCols + 4 * g);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (4 * g + i < kCols) { d[2 * i] = c.w[i]; d[2 * i + 1] = 0u; }
+}
+// a mob whose cell is lit, or 0 (the mobs of a level are those of the light plane that was copied), and its byte
+__device__ __forceinline__ uint32_t lit_mob(View v, uint32_t pk, const uint8_t (*span)[kSpan]) {
+    if (!(pk & 0x80000000u)) return 0u;
+    const int cell = (pk >> 8) & 0xFFu;
+    return span[0][(v.top() + cell / kCols) * kMapSize + v.left() + cell % kCols - v.first()] > kLit ? pk : 0u;
+}
+__device__ __forceinline__ void put_mob(uint32_t pk, uint32_t* rec) {
+    if (pk) reinterpret_cast<uint8_t*>(rec)[((pk >> 8) & 0xFFu) * 8 + ((pk >> 4) & 0xFu)] = (uint8_t)(pk & 0xFu);
+}
+__device__ __forceinline__ void store_record(uint8_t* records, int e, int lane, const uint32_t* rec) {
+    uint32_t* dst = reinterpret_cast<uint32_t*>(records + (size_t)e * kRec);   // 4-byte aligned (996 = 4 x 249)
+#pragma unroll
+    for (int w = lane; w < kRecWords; w += 32) dst[w] = rec[w];
+}
+
+__global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_constant__ Params P) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    Shared& S = *reinterpret_cast<Shared*>(smem);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int e = blockIdx.x * kBlockEnvs + lane;
-    const bool live = e < P.n && (P.skip == nullptr || P.skip[e] == 0);
-    if (live) gather_env(P.v, e, lane, warp, S);
-    if (warp == 0) S.env[lane] = live ? e : -1;
+    const int e0 = blockIdx.x * kBlockEnvs, e = e0 + lane;
+    const int n = P.v.num_envs, grain = copy_grain(P.v);
+    wait_for_previous_kernel();
+    const bool live = e < P.n && (P.skip == nullptr || ld_now(P.skip + e) == 0);
+    int level = 0, top = 0, left = 0;
+    if (live) {
+        level = soa(P.v.player_level, 0, n, e);
+        top = soa(P.v.player_position, 0, n, e) - kRows / 2;
+        left = soa(P.v.player_position, 1, n, e) - kCols / 2;
+    }
+    const View mine = make_view(level, top, left, grain);
+    const uint32_t todo = __ballot_sync(0xffffffffu, live) >> (kOwn * warp) & ((1u << kOwn) - 1u);
+    View v[kOwn];   // of this warp's envs, kOwn * warp + k of the block
+#pragma unroll
+    for (int k = 0; k < kOwn; k++) {
+        v[k].where = __shfl_sync(0xffffffffu, mine.where, kOwn * warp + k);
+        v[k].plane = __shfl_sync(0xffffffffu, mine.plane, kOwn * warp + k);
+        if (todo >> k & 1u) copy_spans(P.v, e0 + kOwn * warp + k, v[k], grain, lane, S.span[warp][k]);
+    }
+    if (live) gather_env(P.v, e, lane, warp, level, top, left, S);
+    wait_spans();
     __syncthreads();
-    write_envs(P, S, warp, lane);
+    Cells cells[kOwn];
+    uint32_t mob[kOwn / 2];   // two envs at a time, 16 lanes each
+#pragma unroll
+    for (int k = 0; k < kOwn; k++) cells[k] = make_cells(v[k], lane, S.span[warp][k]);
+#pragma unroll
+    for (int k = 0; k < kOwn; k += 2) {
+        const int h = k + (lane >> 4);
+        mob[k / 2] = 0u;
+        if ((todo >> h & 1u) && (lane & 15) < kMobs)
+            mob[k / 2] = lit_mob(lane < 16 ? v[k] : v[k + 1], S.mobs[kOwn * warp + h][lane & 15], S.span[warp][h]);
+    }
+    __syncwarp();   // the spans are in registers
+    uint32_t* rec = reinterpret_cast<uint32_t*>(S.span[warp]);   // [kOwn][kRecWords]
+#pragma unroll
+    for (int k = 0; k < kOwn; k++) {
+        put_cells(cells[k], lane, rec + k * kRecWords);
+        for (int j = lane; j < kTail; j += 32) rec[k * kRecWords + kMapWords + j] = __float_as_uint(S.tail[kOwn * warp + k][j]);
+    }
+    __syncwarp();   // the mob bytes land on cells other lanes have written
+#pragma unroll
+    for (int k = 0; k < kOwn; k += 2) put_mob(mob[k / 2], rec + (k + (lane >> 4)) * kRecWords);
+    __syncwarp();
+    if (todo == (1u << kOwn) - 1u && (reinterpret_cast<uintptr_t>(P.records) & 15) == 0) {
+        // the warp's records in one bulk copy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(P.records + (size_t)(e0 + kOwn * warp) * kRec),
+                         "r"((uint32_t)__cvta_generic_to_shared(rec)), "r"(kOwn * kRec) : "memory");
+            asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
+    } else {
+        for (int k = 0; k < kOwn; k++)
+            if (todo >> k & 1u) store_record(P.records, e0 + kOwn * warp + k, lane, rec + k * kRecWords);
+    }
 }
 
-// the envs named by a device-side list (first int32 of every entry), 32 entries per block pass
-__global__ void __launch_bounds__(kBlockThreads) k_record_rows_list(const __grid_constant__ Params P) {
-    __shared__ Shared S;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+// ------------------------------------------------------------------ list of envs
+// The envs named by a device-side list (first int32 of every entry): a few that are being reset, anywhere in
+// the batch, so what counts is the chain of dependent loads and not coalescing.  A warp takes an
+// env: entry -> every scalar, the level and the position, all lanes at once -> mobs and map spans -> record.  About 250
+// entries of 65,536 envs: 26 us with a block for 32 entries, now 9.9.
+// The fields of the tail by position: which field pointer of the view, which element, how it is scaled.
+enum Scale : uint8_t { S_SQRT10, S_10, S_2, S_4, S_INT, S_F10, S_FLOAT, S_FLAG, S_DIR, S_KILLED, S_BOSS };
+struct TailField { uint8_t field, elem, scale; };
+#define CFX_FIELD(name) (uint8_t)((offsetof(cfx_env_view, name) - offsetof(cfx_env_view, player_position)) / sizeof(void*))
+// the 51 scalars in the order of craftax_encode_scalar_observation_tail_at (:2429-2487)
+__device__ const TailField kTailFields[kTail] = {
+    {CFX_FIELD(inv_wood), 0, S_SQRT10}, {CFX_FIELD(inv_stone), 0, S_SQRT10}, {CFX_FIELD(inv_coal), 0, S_SQRT10},
+    {CFX_FIELD(inv_iron), 0, S_SQRT10}, {CFX_FIELD(inv_diamond), 0, S_SQRT10}, {CFX_FIELD(inv_sapphire), 0, S_SQRT10},
+    {CFX_FIELD(inv_ruby), 0, S_SQRT10}, {CFX_FIELD(inv_sapling), 0, S_SQRT10}, {CFX_FIELD(inv_torches), 0, S_SQRT10},
+    {CFX_FIELD(inv_arrows), 0, S_SQRT10}, {CFX_FIELD(inv_books), 0, S_2}, {CFX_FIELD(inv_pickaxe), 0, S_4},
+    {CFX_FIELD(inv_sword), 0, S_4}, {CFX_FIELD(sword_enchantment), 0, S_INT}, {CFX_FIELD(bow_enchantment), 0, S_INT},
+    {CFX_FIELD(inv_bow), 0, S_INT}, {CFX_FIELD(inv_potions), 0, S_SQRT10}, {CFX_FIELD(inv_potions), 1, S_SQRT10},
+    {CFX_FIELD(inv_potions), 2, S_SQRT10}, {CFX_FIELD(inv_potions), 3, S_SQRT10}, {CFX_FIELD(inv_potions), 4, S_SQRT10},
+    {CFX_FIELD(inv_potions), 5, S_SQRT10}, {CFX_FIELD(player_health), 0, S_F10}, {CFX_FIELD(player_food), 0, S_10},
+    {CFX_FIELD(player_drink), 0, S_10}, {CFX_FIELD(player_energy), 0, S_10}, {CFX_FIELD(player_mana), 0, S_10},
+    {CFX_FIELD(player_xp), 0, S_10}, {CFX_FIELD(player_dexterity), 0, S_10}, {CFX_FIELD(player_strength), 0, S_10},
+    {CFX_FIELD(player_intelligence), 0, S_10}, {CFX_FIELD(player_direction), 1, S_DIR}, {CFX_FIELD(player_direction), 2, S_DIR},
+    {CFX_FIELD(player_direction), 3, S_DIR}, {CFX_FIELD(player_direction), 4, S_DIR}, {CFX_FIELD(inv_armour), 0, S_2},
+    {CFX_FIELD(inv_armour), 1, S_2}, {CFX_FIELD(inv_armour), 2, S_2}, {CFX_FIELD(inv_armour), 3, S_2},
+    {CFX_FIELD(armour_enchantments), 0, S_INT}, {CFX_FIELD(armour_enchantments), 1, S_INT},
+    {CFX_FIELD(armour_enchantments), 2, S_INT}, {CFX_FIELD(armour_enchantments), 3, S_INT},
+    {CFX_FIELD(light_level), 0, S_FLOAT}, {CFX_FIELD(is_sleeping), 0, S_FLAG}, {CFX_FIELD(is_resting), 0, S_FLAG},
+    {CFX_FIELD(learned_spells), 0, S_FLAG}, {CFX_FIELD(learned_spells), 1, S_FLAG}, {CFX_FIELD(player_level), 0, S_10},
+    {CFX_FIELD(monsters_killed), 0, S_KILLED}, {CFX_FIELD(boss_timesteps_to_spawn_this_round), 0, S_BOSS}};
+
+// the raw bits of tail scalar f (S_KILLED is read by its own lane later, when the level is known)
+__device__ __forceinline__ uint32_t tail_raw(const cfx_env_view& V, const TailField& f, int e) {
+    const void* base = (&reinterpret_cast<const void* const&>(V.player_position))[f.field];
+    const size_t elem = f.scale == S_DIR ? 0 : f.elem, i = elem * (size_t)V.num_envs + (size_t)e;
+    if (f.scale == S_KILLED) return 0u;
+    return f.scale == S_FLAG ? (uint32_t)ld_now(reinterpret_cast<const uint8_t*>(base) + i) : ld_now(reinterpret_cast<const uint32_t*>(base) + i);
+}
+__device__ __forceinline__ float tail_value(const TailField& f, uint32_t raw, bool killed, bool mob_alive) {
+    const float v = (float)(int32_t)raw;
+    switch (f.scale) {
+        case S_SQRT10: return sqrtf(v) * (1.0f / 10.0f);
+        case S_10: return v * (1.0f / 10.0f);
+        case S_2: return v * (1.0f / 2.0f);
+        case S_4: return v * (1.0f / 4.0f);
+        case S_INT: return v;
+        case S_F10: return __uint_as_float(raw) * (1.0f / 10.0f);
+        case S_FLOAT: return __uint_as_float(raw);
+        case S_FLAG: return raw != 0 ? 1.0f : 0.0f;
+        case S_DIR: return (int32_t)raw == f.elem ? 1.0f : 0.0f;
+        case S_KILLED: return killed ? 1.0f : 0.0f;
+        default: return !mob_alive && (int32_t)raw <= 0 ? 1.0f : 0.0f;
+    }
+}
+
+struct ListShared {
+    uint32_t rec[kRecWords + 3];
+    __align__(16) uint8_t span[kPlanes][kSpan];
+};
+static_assert(sizeof(ListShared) % 16 == 0, "alignment");
+constexpr int kListThreads = 128, kListWarps = kListThreads / 32;
+
+__global__ void __launch_bounds__(kListThreads) k_record_rows_list(const __grid_constant__ Params P) {
+    __shared__ ListShared LS[kListWarps];
+    const cfx_env_view& V = P.v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = V.num_envs, grain = copy_grain(V);
+    ListShared& S = LS[warp];
+    const TailField f0 = kTailFields[lane], f1 = kTailFields[min(lane + 32, kTail - 1)];
+    wait_for_previous_kernel();
     const int count = *P.count_dev;
-    for (int base = blockIdx.x * kBlockEnvs; base < count; base += (int)gridDim.x * kBlockEnvs) {
-        int e = -1;
-        if (base + lane < count) e = *reinterpret_cast<const int32_t*>(P.list + (size_t)(base + lane) * P.list_stride);
-        const bool live = e >= 0 && e < P.v.num_envs;
-        if (live) gather_env(P.v, e, lane, warp, S);
-        if (warp == 0) S.env[lane] = live ? e : -1;
-        __syncthreads();
-        write_envs(P, S, warp, lane);
-        __syncthreads();
+    const int stride = (int)gridDim.x * kListWarps;
+    for (int i = (int)blockIdx.x * kListWarps + warp; i < count; i += stride) {
+        const int e = *reinterpret_cast<const int32_t*>(P.list + (size_t)i * P.list_stride);
+        if (e < 0 || e >= n) continue;
+        const int level = soa(V.player_level, 0, n, e);
+        const int top = soa(V.player_position, 0, n, e) - kRows / 2, left = soa(V.player_position, 1, n, e) - kCols / 2;
+        const uint32_t raw0 = tail_raw(V, f0, e), raw1 = lane + 32 < kTail ? tail_raw(V, f1, e) : 0u;
+        const View v = make_view(level, top, left, grain);
+        copy_spans(V, e, v, grain, lane, S.span);
+        const bool killed = (unsigned)level < (unsigned)kLevels && soa(V.monsters_killed, level, n, e) >= kKilledToClear;
+        // lane 3 c + i: slot i of mob class c
+        const int c = lane / kSlots, slot = lane % kSlots;
+        uint32_t pk = 0;
+        bool mask = false;
+        if (lane < kMobs && slot < (c == 2 ? 2 : 3)) {
+            const int idx = mob_index(c, jax_index(level, kLevels), slot);
+            mask = soa(V.mob_mask, idx, n, e) != 0;
+            pk = pack_mob(c, soa(V.mob_type_id, idx, n, e), mask, soa(V.mob_position, idx * 2, n, e),
+                          soa(V.mob_position, idx * 2 + 1, n, e), top, left);
+        }
+        const bool alive = __any_sync(0xffffffffu, mask && (c == 0 || c == 2));
+        const uint32_t next1 = __shfl_down_sync(0xffffffffu, pk, 1), next2 = __shfl_down_sync(0xffffffffu, pk, 2);
+        if ((slot < 2 && same_cell(pk, next1)) || (slot < 1 && same_cell(pk, next2))) pk = 0;   // a later slot covers it
+        float* tail = reinterpret_cast<float*>(S.rec + kMapWords);
+        tail[lane] = tail_value(f0, raw0, killed, alive);
+        if (lane + 32 < kTail) tail[lane + 32] = tail_value(f1, raw1, killed, alive);
+        wait_spans();
+        put_cells(make_cells(v, lane, S.span), lane, S.rec);
+        __syncwarp();
+        put_mob(lit_mob(v, pk, S.span), S.rec);
+        __syncwarp();
+        store_record(P.records, e, lane, S.rec);
+        __syncwarp();
     }
 }
 
@@ -259,7 +523,7 @@ static int make_params(const char* who, const cfx_env_view* view, uint8_t* recor
     return CFX_OK;
 }
 
-static_assert(sizeof(Shared) <= 48 * 1024, "static shared memory");
+static_assert(4 * (sizeof(Shared) + 1024) <= 228 * 1024, "four blocks an SM");
 static_assert(offsetof(cfx_env_view, mob_type_id) - offsetof(cfx_env_view, player_position) == 39 * sizeof(void*),
               "the field pointers of cfx_env_view are contiguous (make_params walks them)");
 
@@ -268,72 +532,116 @@ static_assert(offsetof(cfx_env_view, mob_type_id) - offsetof(cfx_env_view, playe
 // record_obs_kernel (craftax_classic.cu:1884-1890) gives every env a thread that writes its 148
 // bytes one by one: 148 store instructions per warp, each touching 32 different records.  Here a
 // block gathers the records of 128 consecutive envs in shared memory, thread per env (the SoA
-// loads of a warp are contiguous), and writes the 18,944 contiguous bytes out as coalesced words.
+// loads of a warp are contiguous), and writes the 18,944 contiguous bytes out as coalesced 16-byte
+// words.  The nine cells of a view row are nibbles of at most five bytes, so of two aligned words of the map: 14
+// loads a thread for the view, all in flight at once, where a load per cell made 63 (each touching
+// 32 sectors a warp), and the record's words are put together in registers (row length 37 words: no bank conflicts).
+// 262,144 envs: 103 -> 42 us.
 constexpr int kClRows = 7, kClCols = 9, kClCells = kClRows * kClCols, kClMap = 64, kClRowBytes = 32;
-constexpr int kClInv = 12, kClOutOfBounds = 1, kClBlockEnvs = 128;
-static_assert(2 * kClCells + kClInv + 6 + 4 == kClassicRec, "classic record layout");
+constexpr int kClInv = 12, kClOutOfBounds = 1, kClBlockEnvs = 128, kClWords = kClassicRec / 4;
+static_assert(2 * kClCells + kClInv + 6 + 4 == kClassicRec && kClassicRec % 4 == 0, "classic record layout");
+
+// bytes of a record put together in order, word by word; positions are compile-time constants once unrolled
+struct ClassicWords {
+    uint32_t w[kClWords];
+    __device__ __forceinline__ void put(int pos, uint32_t v, int bytes) {   // v < 2^(8 bytes)
+        w[pos / 4] |= v << (8 * (pos % 4));
+        if (pos % 4 + bytes > 4) w[pos / 4 + 1] |= v >> (32 - 8 * (pos % 4));
+    }
+};
 
 __global__ void __launch_bounds__(kClBlockEnvs) k_classic_record_rows(const __grid_constant__ cfx_classic_env_view V,
                                                                      uint8_t* __restrict__ records, int n_envs) {
-    __shared__ __align__(16) uint8_t srec[kClBlockEnvs * kClassicRec];
+    __shared__ __align__(16) uint32_t srec[kClBlockEnvs * kClWords];
     const int t = threadIdx.x;
     const int e0 = blockIdx.x * kClBlockEnvs, e = e0 + t;
     const int n = V.num_envs;
+    wait_for_previous_kernel();
     if (e < n_envs) {
-        uint8_t* o = srec + t * kClassicRec;
-        const int pr = V.player_r[e], pc = V.player_c[e];
+        const int pr = soa(V.player_r, 0, n, e), pc = soa(V.player_c, 0, n, e);
         const uint8_t* map = V.map_packed + (size_t)e * V.map_stride;
-        // view rows: blocks (a nibble per map column; 1 outside the map), mob bytes cleared  (:1061-1100)
+        // view rows: blocks (a nibble per map column; 1 outside the map)  (:1061-1100)
+        const int o = (pc - 4) >> 1, wi = o >> 2;   // first byte and word of the view's columns in a map row
+        const bool aligned = ((reinterpret_cast<uintptr_t>(V.map_packed) | V.map_stride) & 3) == 0;
+        auto word = [&](int mr, int i) -> uint32_t {
+            if (mr < 0 || mr >= kClMap || i < 0 || i >= kClRowBytes / 4) return 0u;
+            const uint8_t* q = map + mr * kClRowBytes + 4 * i;
+            if (aligned) return ld_now(reinterpret_cast<const uint32_t*>(q));
+            return ld_now(q) | (uint32_t)ld_now(q + 1) << 8 | (uint32_t)ld_now(q + 2) << 16 | (uint32_t)ld_now(q + 3) << 24;
+        };
+        uint32_t m0[kClRows], m1[kClRows];
 #pragma unroll
         for (int r = 0; r < kClRows; r++) {
-            const int mr = pr - 3 + r;
-            const bool row_in = mr >= 0 && mr < kClMap;
-#pragma unroll
-            for (int c = 0; c < kClCols; c++) {
-                const int mc = pc - 4 + c;
-                uint8_t blk = kClOutOfBounds;
-                if (row_in && mc >= 0 && mc < kClMap) {
-                    const uint8_t b = map[mr * kClRowBytes + (mc >> 1)];
-                    blk = (mc & 1) ? (b >> 4) : (b & 0x0F);
-                }
-                o[r * kClCols + c] = blk;
-                o[kClCells + r * kClCols + c] = 0;
-            }
+            m0[r] = word(pr - 3 + r, wi);
+            m1[r] = word(pr - 3 + r, wi + 1);
         }
-        // mobs inside the view set their bit  (:1102-1125)
-        auto stamp = [&](const int16_t* rr, const int16_t* cc, const uint8_t* mask, int slots, uint8_t bit) {
-            for (int i = 0; i < slots; i++) {
-                if (!mask[(size_t)i * n + e]) continue;
-                const int dr = rr[(size_t)i * n + e] - pr, dc = cc[(size_t)i * n + e] - pc;
-                if (dr < -3 || dr > 3 || dc < -4 || dc > 4) continue;
-                o[kClCells + (dr + 3) * kClCols + (dc + 4)] |= bit;
-            }
-        };
-        stamp(V.zombie_r, V.zombie_c, V.zombie_mask, 3, 1);
-        stamp(V.cow_r, V.cow_c, V.cow_mask, 3, 2);
-        stamp(V.skel_r, V.skel_c, V.skel_mask, 2, 4);
-        stamp(V.arrow_r, V.arrow_c, V.arrow_mask, 3, 8);
-        // inventory, intrinsics, direction, sleeping, light  (:1590-1603)
-        int idx = 2 * kClCells;
+        int8_t inv[kClInv];
 #pragma unroll
-        for (int i = 0; i < kClInv; i++) o[idx++] = (uint8_t)V.inv[(size_t)i * n + e];
-        o[idx++] = (uint8_t)V.health[e];
-        o[idx++] = (uint8_t)V.food[e];
-        o[idx++] = (uint8_t)V.drink[e];
-        o[idx++] = (uint8_t)V.energy[e];
-        o[idx++] = (uint8_t)V.player_dir[e];
-        o[idx++] = V.is_sleeping[e] ? 1 : 0;
-        const uint32_t light = __float_as_uint(V.light_level[e]);
-        o[idx++] = (uint8_t)light; o[idx++] = (uint8_t)(light >> 8);
-        o[idx++] = (uint8_t)(light >> 16); o[idx++] = (uint8_t)(light >> 24);
+        for (int i = 0; i < kClInv; i++) inv[i] = soa(V.inv, i, n, e);
+        const int8_t intr[5] = {soa(V.health, 0, n, e), soa(V.food, 0, n, e), soa(V.drink, 0, n, e), soa(V.energy, 0, n, e),
+                                soa(V.player_dir, 0, n, e)};
+        const uint8_t sleeping = soa(V.is_sleeping, 0, n, e);
+        const float light = soa(V.light_level, 0, n, e);
+        constexpr int kMobsCl = 11;
+        const int16_t* const mob_r[4] = {V.zombie_r, V.cow_r, V.skel_r, V.arrow_r};
+        const int16_t* const mob_c[4] = {V.zombie_c, V.cow_c, V.skel_c, V.arrow_c};
+        const uint8_t* const mob_m[4] = {V.zombie_mask, V.cow_mask, V.skel_mask, V.arrow_mask};
+        constexpr int kKind[kMobsCl] = {0, 0, 0, 1, 1, 1, 2, 2, 3, 3, 3}, kSlot[kMobsCl] = {0, 1, 2, 0, 1, 2, 0, 1, 0, 1, 2};
+        int16_t mr[kMobsCl], mc[kMobsCl];
+        uint8_t on[kMobsCl];
+#pragma unroll
+        for (int i = 0; i < kMobsCl; i++) {
+            on[i] = soa(mob_m[kKind[i]], kSlot[i], n, e);
+            mr[i] = soa(mob_r[kKind[i]], kSlot[i], n, e);
+            mc[i] = soa(mob_c[kKind[i]], kSlot[i], n, e);
+        }
+        ClassicWords R;
+#pragma unroll
+        for (int i = 0; i < kClWords; i++) R.w[i] = 0u;
+        // inventory, intrinsics, direction, sleeping, light  (:1590-1603)
+        constexpr int kTailPos = 2 * kClCells;
+#pragma unroll
+        for (int i = 0; i < kClInv; i++) R.put(kTailPos + i, (uint8_t)inv[i], 1);
+#pragma unroll
+        for (int i = 0; i < 5; i++) R.put(kTailPos + kClInv + i, (uint8_t)intr[i], 1);
+        R.put(kTailPos + kClInv + 5, sleeping ? 1u : 0u, 1);
+        R.put(kTailPos + kClInv + 6, __float_as_uint(light), 4);
+        // columns of the view that lie on the map, a nibble each
+        uint64_t in = 0;
+#pragma unroll
+        for (int c = 0; c < kClCols; c++)
+            if (pc - 4 + c >= 0 && pc - 4 + c < kClMap) in |= 15ull << (4 * c);
+        const int shift = 8 * (o & 3) + 4 * (pc & 1);
+#pragma unroll
+        for (int r = 0; r < kClRows; r++) {
+            const bool row_in = pr - 3 + r >= 0 && pr - 3 + r < kClMap;
+            const uint64_t keep = row_in ? in : 0ull;
+            const uint64_t v = (((uint64_t)m1[r] << 32 | m0[r]) >> shift & keep) |
+                               (0x111111111ull * kClOutOfBounds & ~keep);
+            const uint32_t lo = (uint32_t)v, even = lo & 0x0F0F0F0Fu, odd = lo >> 4 & 0x0F0F0F0Fu;
+            R.put(r * kClCols, __byte_perm(even, odd, 0x5140), 4);
+            R.put(r * kClCols + 4, __byte_perm(even, odd, 0x7362), 4);
+            R.put(r * kClCols + 8, (uint32_t)(v >> 32) & 15u, 1);
+        }
+#pragma unroll
+        for (int i = 0; i < kClWords; i++) srec[t * kClWords + i] = R.w[i];
+        // mobs inside the view set their bit  (:1102-1125)
+        uint8_t* mobs = reinterpret_cast<uint8_t*>(srec + t * kClWords) + kClCells;
+#pragma unroll
+        for (int i = 0; i < kMobsCl; i++) {
+            const int dr = mr[i] - pr + 3, dc = mc[i] - pc + 4;
+            if (on[i] != 0 && (unsigned)dr < (unsigned)kClRows && (unsigned)dc < (unsigned)kClCols)
+                mobs[dr * kClCols + dc] |= (uint8_t)(1 << kKind[i]);
+        }
     }
     __syncthreads();
     // the block's records are contiguous in global memory: 37 words per env
-    const int envs = min(kClBlockEnvs, n_envs - e0);
-    const int words = envs * (kClassicRec / 4);
+    const int words = min(kClBlockEnvs, n_envs - e0) * kClWords;
     uint32_t* dst = reinterpret_cast<uint32_t*>(records + (size_t)e0 * kClassicRec);
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(srec);
-    for (int w = t; w < words; w += kClBlockEnvs) dst[w] = src[w];
+    const int quads = (reinterpret_cast<uintptr_t>(records) & 15) == 0 ? words / 4 : 0;
+    for (int q = t; q < quads; q += kClBlockEnvs)
+        reinterpret_cast<uint4*>(dst)[q] = reinterpret_cast<const uint4*>(srec)[q];
+    for (int w = 4 * quads + t; w < words; w += kClBlockEnvs) dst[w] = srec[w];
 }
 
 }  // namespace record
@@ -351,9 +659,8 @@ extern "C" int cfx_record_obs(int device, const cfx_env_view* view, uint8_t* rec
     P.n = n;
     P.skip = skip;
     const unsigned blocks = (unsigned)((n + record::kBlockEnvs - 1) / record::kBlockEnvs);
-    record::k_record_rows<<<blocks, record::kBlockThreads, 0, (cudaStream_t)stream>>>(P);
-    CFX_CUDA(cudaGetLastError());
-    return CFX_OK;
+    CFX_CUDA(cudaFuncSetAttribute(record::k_record_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(record::Shared)));
+    return launch_chained(record::k_record_rows, dim3(blocks), record::kBlockThreads, sizeof(record::Shared), (cudaStream_t)stream, P);
 }
 
 extern "C" int cfx_record_obs_list(int device, const cfx_env_view* view, uint8_t* records, const void* list,
@@ -367,13 +674,11 @@ extern "C" int cfx_record_obs_list(int device, const cfx_env_view* view, uint8_t
     P.list = (const uint8_t*)list;
     P.list_stride = list_stride;
     P.count_dev = count_dev;
-    // the count is on the device: a fixed grid walks the list (the reference uses at most
-    // 128 blocks of 8 warps for its list pass, :11941)
-    int blocks = (view->num_envs + record::kBlockEnvs - 1) / record::kBlockEnvs;
+    // the count is on the device: a fixed grid of at most four blocks an SM walks the list, a warp an entry
+    // (the reference uses at most 128 blocks of 8 warps for its list pass, :11941)
+    int blocks = (view->num_envs + record::kListWarps - 1) / record::kListWarps;
     if (blocks > 592) blocks = 592;
-    record::k_record_rows_list<<<blocks, record::kBlockThreads, 0, (cudaStream_t)stream>>>(P);
-    CFX_CUDA(cudaGetLastError());
-    return CFX_OK;
+    return launch_chained(record::k_record_rows_list, dim3((unsigned)blocks), record::kListThreads, 0, (cudaStream_t)stream, P);
 }
 
 extern "C" int cfx_classic_record_obs(int device, const cfx_classic_env_view* view, uint8_t* records, int n,
@@ -391,7 +696,5 @@ extern "C" int cfx_classic_record_obs(int device, const cfx_classic_env_view* vi
         CFX_REQUIRE(*q != nullptr, "cfx_classic_record_obs: field pointer %d of the view is NULL", (int)(q - first));
     CFX_GUARD(device);
     const unsigned blocks = (unsigned)((n + record::kClBlockEnvs - 1) / record::kClBlockEnvs);
-    record::k_classic_record_rows<<<blocks, record::kClBlockEnvs, 0, (cudaStream_t)stream>>>(*view, records, n);
-    CFX_CUDA(cudaGetLastError());
-    return CFX_OK;
+    return launch_chained(record::k_classic_record_rows, dim3(blocks), record::kClBlockEnvs, 0, (cudaStream_t)stream, *view, records, n);
 }

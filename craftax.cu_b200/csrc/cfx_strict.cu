@@ -100,13 +100,6 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool on, bo
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// The kernels of a forward are launched with programmatic stream serialisation and wait here until the
-// results of the kernel in front are in memory.  None lets the next one start early
-// (griddepcontrol.launch_dependents): its blocks would fill the SMs that this kernel's last blocks leave
-// free and pile up there (4,096 envs: 227 us against 178 for a forward).
-__device__ __forceinline__ void wait_for_previous_kernel() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 
 // ---------------------------------------------------------------- encoder
 // h_enc[k][e] = b_enc[k] + sum_f x[e][f] * W_enc[f][k], ascending f.  A lane owns TM envs x G groups of 4
@@ -585,24 +578,6 @@ __global__ void k_init_uniform(float* w, int count, float bound, uint64_t seed, 
 }
 
 // ---------------------------------------------------------------- launchers
-// Launch with programmatic stream serialisation (see wait_for_previous_kernel): the launch and the
-// start-up of a kernel run under the kernel in front of it.
-template <typename... P, typename... Args>
-static int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    CFX_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
-    return CFX_OK;
-}
-
 int launch_expand(const uint8_t* rec, float* out, int n, cudaStream_t st) {
     size_t total = (size_t)n * kObs;
     k_expand<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(rec, out, n);
