@@ -31,6 +31,9 @@
 // a ring come free in the order they were filled, and several lanes of one warp, each in its own
 // loop, serve their slots far more slowly than one thread serves them all.
 #include "cfx_fused_common.cuh"
+#include "cfx_fused_split.h"
+
+#include <algorithm>
 
 namespace cfx {
 namespace fused {
@@ -1107,7 +1110,7 @@ k_policy_fused(const __grid_constant__ Params P) {
     // read the counter (in its sampler threads) before it got here.
     if (tid == 0 && P.bump_step) {
         __threadfence();
-        if (atomicAdd(P.done_ctr, 1u) == gridDim.x - 1) {
+        if (atomicAdd(P.done_ctr, 1u) == P.done_blocks - 1) {
             *P.step_ctr += 1ULL;
             *P.done_ctr = 0u;
         }
@@ -1160,10 +1163,12 @@ struct FusedPlan {
     float* state = nullptr;
     const float* params = nullptr;
     CUtensorMap state_map[fused::kMaxLayers];
+    CUtensorMap quad_map[fused::kMaxLayers];   // the same with boxes of 32 rows
     CUtensorMap w_map[3];          // pair mode: operand image regions (encoder, gates, heads)
     int sm_count = 0;
     int pair = 0;        // 1: launch as clusters of two CTAs (cta_group::2 MMAs)
     int max_pairs = 0;   // co-resident clusters of two
+    int max_split[2] = {0, 0};   // co-resident clusters of four and of two CTAs that share a tile
 };
 
 bool fused_supported(int H, int L, int A, int precision, int game) {
@@ -1231,9 +1236,11 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
         return cuda_fail(e, "fused_create alloc", __FILE__, __LINE__);
     }
     for (int l = 0; l < L; l++) {
-        if (!make_tmap_2d(&p->state_map[l], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                          state + (size_t)l * n * H, (uint64_t)n, (uint64_t)H, (uint64_t)H * 4,
-                          fused::kTile, fused::kHalfUnits, CU_TENSOR_MAP_SWIZZLE_128B)) {
+        auto map = [&](CUtensorMap* m, int rows) {
+            return make_tmap_2d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, state + (size_t)l * n * H, (uint64_t)n, (uint64_t)H,
+                                (uint64_t)H * 4, rows, fused::kHalfUnits, CU_TENSOR_MAP_SWIZZLE_128B);
+        };
+        if (!map(&p->state_map[l], fused::kTile) || !map(&p->quad_map[l], 32)) {
             fused_destroy(p);
             set_error("fused_create: cuTensorMapEncodeTiled failed for the state");
             return CFX_ERR_CUDA;
@@ -1292,6 +1299,10 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
                 return CFX_ERR_CUDA;
             }
             base += rows[r] * 128;
+        }
+        for (int i = 0; i < 2; i++) {   // (the small-batch form reads the pairs' operand image)
+            int rc = fused::split_prepare(precision, game, H, i == 0 ? 4 : 2, p->sm_count, &p->max_split[i]);
+            if (rc) { fused_destroy(p); return rc; }
         }
     }
     *out = p;
@@ -1375,6 +1386,19 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     P.off_b_enc = o.b_enc;
     P.off_b_a = o.b_a;
     P.off_b_v = o.b_v;
+    if (launches) *launches = 1;
+    // Small batches: a tile is shared by four (two) CTAs as long as every tile then has its SMs at once, and is as
+    // short as that allows (cfx_fused_split.cu)
+    const int rows = std::min(p->n, P.num_tiles * fused::kTile) - P.tile_begin * fused::kTile;
+    for (int i = 0; i < 2; i++)
+        for (int tr = 32; tr <= fused::kTile; tr *= 2) {
+            const int tiles = (rows + tr - 1) / tr, S = i == 0 ? 4 : 2;
+            if (tiles > p->max_split[i]) continue;
+            for (int l = 0; l < p->L; l++) P.state_map[l] = p->quad_map[l];
+            P.tile_rows = tr;
+            P.done_blocks = (uint32_t)(tiles * (tr / 32));
+            return fused::split_launch(p->precision, p->game, p->H, S, tiles, P, st);
+        }
     int smem = 0;
     const void* kern = fused_kernel(p->precision, p->pair, p->game, p->H, &smem);
     void* kargs[1] = {(void*)&P};
@@ -1397,9 +1421,8 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
         P.num_tiles_loop = P.num_tiles;
         cfg.gridDim = dim3((unsigned)(range_tiles < p->sm_count ? range_tiles : p->sm_count));
     }
+    P.done_blocks = cfg.gridDim.x;
     CFX_CUDA(cudaLaunchKernelExC(&cfg, kern, kargs));
-    CFX_CUDA(cudaGetLastError());
-    if (launches) *launches = 1;
     return CFX_OK;
 }
 

@@ -106,10 +106,12 @@ struct Params {
     unsigned long long* step_ctr;        // device step counter (Philox offset); see bump_step
     uint32_t* status;
     uint32_t* done_ctr;                  // blocks that have finished this launch (bump_step)
+    uint32_t done_blocks;                // how many there are (small-batch form: warps that need the counter)
     int bump_step;
     uint64_t seed, env_offset;
     int n, L, num_tiles;  // num_tiles: end of the tile range of this launch (exclusive)
     int tile_begin;       // first tile of this launch (a launch may cover a slice of the envs)
+    int tile_rows;        // small-batch form: rows of a tile
     int rec_bytes;        // bytes of one record (996 full game, 148 classic)
     int num_tiles_loop;   // trip bound of the tile loops: num_tiles, rounded up to even for CTA pairs
     size_t off_b_enc, off_b_a, off_b_v;
@@ -304,16 +306,10 @@ __device__ __forceinline__ void expand_classic(const uint8_t* rp, int kc, uint32
 }
 
 // ------------------------------------------------------------------ outputs of an env
-// Head accumulator row + biases (bias[a] for action a, bias[kA] for the value) -> logits_av, sampled
-// action, log-probability, value.
-template <int GAME, int N>
-__device__ __forceinline__ void write_outputs(const Params& P, int env, const uint32_t (&hv)[N], const float* bias, float u) {
+template <int GAME, int A>
+__device__ __forceinline__ void write_logits(const Params& P, int env, const float (&logits)[A], float value) {
     constexpr int kA = Gm<GAME>::kA;
-    static_assert(N > kA, "columns");
-    float logits[kA];
-#pragma unroll
-    for (int a = 0; a < kA; a++) logits[a] = __uint_as_float(hv[a]) + bias[a];
-    const float value = __uint_as_float(hv[kA]) + bias[kA];
+    static_assert(A == kA, "actions");
     if constexpr ((kA + 1) % 8 != 4) {
         static_assert((kA + 1) % 2 == 0, "rows are 8-byte aligned");
         float* dst = P.logits_av + (size_t)env * (kA + 1);
@@ -351,12 +347,27 @@ __device__ __forceinline__ void write_outputs(const Params& P, int env, const ui
             st_global_v8(dst + 8 * q + (odd ? 4 : 0), v8);
         }
     }
-    float lp;
-    const int act = sample_action<kA>(logits, u, &lp);
+}
+__device__ __forceinline__ void write_action(const Params& P, int env, int act, float lp, float value) {
     if (P.env_actions) P.env_actions[env] = (float)act;
     P.actions[env] = act;
     if (P.logprobs) P.logprobs[env] = lp;
     if (P.values) P.values[env] = value;
+}
+// Head accumulator row + biases (bias[a] for action a, bias[kA] for the value) -> logits_av, sampled
+// action, log-probability, value.
+template <int GAME, int N>
+__device__ __forceinline__ void write_outputs(const Params& P, int env, const uint32_t (&hv)[N], const float* bias, float u) {
+    constexpr int kA = Gm<GAME>::kA;
+    static_assert(N > kA, "columns");
+    float logits[kA];
+#pragma unroll
+    for (int a = 0; a < kA; a++) logits[a] = __uint_as_float(hv[a]) + bias[a];
+    const float value = __uint_as_float(hv[kA]) + bias[kA];
+    write_logits<GAME>(P, env, logits, value);
+    float lp;
+    const int act = sample_action<kA>(logits, u, &lp);
+    write_action(P, env, act, lp, value);
 }
 
 }  // namespace fused

@@ -1,0 +1,666 @@
+// Fused policy forward for batches that leave SMs idle when every 128-env tile has one SM (or pair of
+// SMs) of its own: a tile is given to a cluster of S CTAs (2 or 4), each of which owns 1/S of the hidden
+// units.  What a small batch costs is one tile's chain of dependent steps; here the chain is
+// shorter: a CTA multiplies 64 NS instead of 256 encoder columns, one gate slice (NS = 1) instead of four a
+// layer, and sixteen worker warps share the expansion and the cell where the one-SM kernel
+// (cfx_fused.cu) has eight.
+//
+//   records   the tile's records are contiguous: four bulk copies of 32 rows into shared memory.  A row is an odd
+//             number of words, so thread-per-row reads have no bank conflicts.  (Tensor boxes of 80 bytes a
+//             row, as in cfx_fused.cu, cost more than the rest of the encoder here.)  Every CTA of
+//             the cluster expands the whole record into tensor memory, chunk kc by warpgroup kc % 4
+//   encoder   A from tensor memory, N = 64 NS own units
+//   layers    A from shared memory: the layer's input as K blocks of 64 units (128-byte swizzled operand
+//             tiles, 16 KB).  A CTA writes its own K blocks and copies them to the other CTAs (bulk
+//             copies shared memory -> shared memory of the cluster, counted on the receiver's
+//             barrier), a quadrant of 32 rows = 4 KB at a time, as soon as its four warps are done
+//   state     boxes of 128 rows x 32 units by tensor copies, updated in place and written back (a thread's own
+//             64 bytes of a row, read and written by the threads, kept the load/store unit busy for 4,000 cycles a
+//             layer and with it every barrier operation of the SM)
+//   heads     in every CTA, over all rows; the quadrants of rows are sampled in different CTAs
+// The cluster works on one tile and exits, so every barrier but those of the rings is used once or once a
+// layer.  The products of a row are accumulated in the order of cfx_fused.cu: same bits.
+// The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
+// records.  The one input buffer is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
+// which a CTA's commit signals in all of them).
+// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 14.4, 1,024 25.7 -> 16.4,
+// 2,368 26 -> 19.9, 8,192 26.9 -> 22.8; classic h256x3, 1,024 envs 35.7 -> 23.4.  Bound by the chain: of 26,000 cycles
+// at 1,024 envs the records take 1,400, the encoder 7,000 (54 MMAs at the ~105 cycles one takes to issue), a layer 6,500 (exchange
+// 1,900, MMAs 1,800, cell 2,700: 48 tanh for each of the four warps of an SM scheduler), heads and sampler 4,500.
+#include "cfx_fused_split.h"
+
+#include <type_traits>
+
+namespace cfx {
+namespace fused {
+namespace split {
+
+constexpr int kWorkerWarp0 = 4, kWorkerWarps = 16, kThreads = (kWorkerWarp0 + kWorkerWarps) * 32;
+constexpr int kWarpUnits = 16;                       // units of a 64-unit slice that one worker warp handles
+constexpr int kABlock = kTile * 128;                 // K block of the layer input: [128 rows][64 K]
+constexpr int kWSlots = 4, kWSlot = kGateBlockBytes; // weight ring: one gate K block (24 KB) a slot
+constexpr int kASlots = 12;                          // operand chunks in tensor memory; a multiple of the warpgroups
+constexpr int kSSlots = 4, kSBox = kTile * 128, kQuadBox = 32 * 128;   // state ring: 128 rows x 32 units a slot, copied 32 rows at a time
+constexpr uint32_t kColAexp = 0, kColAcc = 384, kColHead = 448;
+__host__ __device__ constexpr uint32_t col_gate(int j) { return 192u * (uint32_t)j; }   // over the operand chunks, done by then
+
+template <int GAME, int HID, int S> struct Cfg {
+    static constexpr int kKB = HID / 64;                        // K blocks of a layer's input
+    static constexpr int kNS = HID / 64 / S;                    // gate slices of a CTA
+    static constexpr int kUnits = 64 * kNS;                     // hidden units of a CTA
+    static constexpr int kEncTile = kUnits * 128;               // its rows of one encoder weight block
+    static constexpr int kEncPerItem = kNS == 1 ? 3 : 1;        // encoder blocks of one ring slot
+    static constexpr int kEncItems = (Gm<GAME>::kEncBlocks + kEncPerItem - 1) / kEncPerItem;
+    static constexpr int kHeadHalf = Gm<GAME>::kHeadPair / 2 * 128;   // half of the head rows, one K block
+    static constexpr int kHeadItems = kKB / 2;                  // two K blocks of the heads a slot
+    static constexpr int kRowBytes = Gm<GAME>::kRecBytes, kQuadBytes = 32 * kRowBytes;
+    static constexpr int kBoxes = 2 * kNS;                      // state boxes of a layer
+    static constexpr int kOffS = kKB * kABlock, kASBytes = kOffS + kSSlots * kSBox;   // layer input, state; first the records
+    static constexpr int kOffW = (kASBytes > 4 * kQuadBytes ? kASBytes : 4 * kQuadBytes + 1023) / 1024 * 1024;
+    static constexpr int kOffBias = kOffW + kWSlots * kWSlot;
+    static constexpr int kOffBars = kOffBias + (kUnits + kHeadMax) * 4;
+    static_assert(kNS >= 1 && kNS <= 2 && kUnits * S == HID && kEncTile * kEncPerItem <= kWSlot &&
+                      4 * kHeadHalf <= kWSlot && kQuadBytes % 16 == 0 &&
+                      kRowBytes % 8 == 4, "shapes");
+};
+
+enum Bar {
+    W_FULL = 0, W_EMPTY = W_FULL + kWSlots, REC_FULL = W_EMPTY + kWSlots, REC_FREE = REC_FULL + 4,
+    AEXP_FULL = REC_FREE + 1, AEXP_EMPTY = AEXP_FULL + kASlots, ACC_FULL = AEXP_EMPTY + kASlots,
+    S_FULL = ACC_FULL + 1, ST_READY = S_FULL + kSSlots, MMA_DONE = ST_READY + kSSlots,
+    QUAD = MMA_DONE + 1, G_FULL = QUAD + 8,   // QUAD: [slice][quadrant]
+    H_FULL = G_FULL + 2, A_KB = H_FULL + 1,   // A_KB: [layer input][K block]
+    NUM_BARS = A_KB + (kMaxLayers + 1) * 4
+};
+template <int GAME, int HID, int S> constexpr int smem_bytes() {
+    return Cfg<GAME, HID, S>::kOffBars + NUM_BARS * 8 + 16 + 1024;   // misc, alignment slack
+}
+static_assert(smem_bytes<CFX_GAME_FULL, 256, 2>() <= 232448 && smem_bytes<CFX_GAME_FULL, 128, 2>() <= 232448, "shared memory");
+
+constexpr uint32_t kSite = 0x40;   // wait-site codes: kSite + barrier
+
+struct Smem {
+    uint8_t* base;
+    int off_bars;
+    __device__ __forceinline__ uint32_t bar(int i) const { return smem_u32(base + off_bars + i * 8); }
+    __device__ __forceinline__ uint32_t* tmem_base() const { return reinterpret_cast<uint32_t*>(base + off_bars + NUM_BARS * 8); }
+    __device__ __forceinline__ volatile uint32_t* abort_flag() const { return tmem_base() + 1; }
+};
+#define CFX_SWAIT(barid, parity) \
+    if (!mbar_wait<false>(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return
+#define CFX_SWAIT_SPIN(barid, parity)                                               \
+    if (!mbar_test_wait(sm.bar(barid), (parity)) &&                                 \
+        !mbar_wait_spin(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) \
+    return
+
+// shared memory of this CTA -> shared memory of another CTA of the cluster, counted on a barrier there
+__device__ __forceinline__ void bulk_s2s(uint32_t dst_cluster, uint32_t src, uint32_t bytes, uint32_t bar_cluster) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_cluster),
+        "r"(src), "r"(bytes), "r"(bar_cluster)
+        : "memory");
+}
+
+// the cluster barrier without memory ordering (with it the arrival waits for the stores of the outputs)
+__device__ __forceinline__ void cluster_sync_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+// arrives on the barrier in every CTA of the cluster when all MMAs issued so far are done
+template <int S>
+__device__ __forceinline__ void mma_commit_all(uint32_t bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"((uint16_t)((1u << S) - 1u))
+        : "memory");
+}
+
+// ------------------------------------------------------------------ weights
+// The operand image is the one the CTA pairs of cfx_fused.cu use: stages of two blocks, every block in two halves of
+// rows.  A CTA's rows of an encoder block are contiguous in it, a gate K block is two pieces.
+template <int GAME, int HID, int S>
+__device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, uint32_t rank) {
+    using C = Cfg<GAME, HID, S>;
+    constexpr int kSlices = HID / 64, kHalf = HID / 2;
+    constexpr size_t enc_b = enc_bytes<GAME, HID>();
+    const int gates = P.L * C::kNS * C::kKB, items = C::kEncItems + gates + C::kHeadItems;
+    const uint32_t ring = smem_u32(sm.base + C::kOffW);
+    for (int i = 0; i < items; i++) {
+        const int slot = i % kWSlots;
+        if (i >= kWSlots) CFX_SWAIT(W_EMPTY + slot, ((i / kWSlots) - 1) & 1);
+        const uint32_t dst = ring + slot * kWSlot, full = sm.bar(W_FULL + slot);
+        if (i < C::kEncItems) {
+            const int blocks = min(C::kEncPerItem, Gm<GAME>::kEncBlocks - i * C::kEncPerItem), u0 = C::kUnits * (int)rank;
+            mbar_arrive_expect_tx(full, blocks * C::kEncTile);
+            for (int b = 0; b < blocks; b++) {
+                const int blk = i * C::kEncPerItem + b;
+                const size_t off = (size_t)(blk / 2) * Hd<HID>::kEncCopyBytes +
+                                   (size_t)((u0 / kHalf) * 2 + (blk & 1)) * (kHalf * 128) + (size_t)(u0 % kHalf) * 128;
+                bulk_g2s(dst + b * C::kEncTile, P.image + off, C::kEncTile, full);
+            }
+        } else if (i < C::kEncItems + gates) {
+            const int g = i - C::kEncItems, kb = g % C::kKB, j = g / C::kKB % C::kNS, l = g / (C::kKB * C::kNS);
+            const int stage = (l * kSlices + (int)rank * C::kNS + j) * (C::kKB / 2) + kb / 2;
+            const uint8_t* src = P.image + enc_b + (size_t)stage * kGateStageBytes + (size_t)(kb & 1) * (kGateBlockBytes / 2);
+            mbar_arrive_expect_tx(full, kGateBlockBytes);
+            bulk_g2s(dst, src, kGateBlockBytes / 2, full);
+            bulk_g2s(dst + kGateBlockBytes / 2, src + kGateBlockBytes, kGateBlockBytes / 2, full);
+        } else {
+            const int h = i - C::kEncItems - gates;
+            const uint8_t* src = P.image + enc_b + (size_t)P.L * kSlices * C::kKB * kGateBlockBytes;
+            mbar_arrive_expect_tx(full, 4 * C::kHeadHalf);
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+#pragma unroll
+                for (int half = 0; half < 2; half++)
+                    bulk_g2s(dst + (2 * b + half) * C::kHeadHalf, src + (size_t)(half * C::kKB + 2 * h + b) * C::kHeadHalf, C::kHeadHalf, full);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ MMA
+// One thread issues every MMA.  There is one tile, so every ring position is a compile-time constant and every
+// descriptor one addition away from two bases: an MMA whose descriptor is computed takes ~150 cycles to issue, and
+// 54 of them were two thirds of the encoder.  The barriers of the next step are probed before the
+// current step's MMAs (CFX_PROBE), so that a probe's round trip runs under their issue.
+#define CFX_SPROBE(name, barid, parity) CFX_PROBE(name, sm.bar(barid), (uint32_t)(parity))
+#define CFX_SWAIT_PROBED(name, barid, parity)                                                               \
+    {                                                                                                       \
+        uint32_t ready_;                                                                                    \
+        CFX_PROBE_READ(name, ready_);                                                                       \
+        if (ready_ == 0 && !mbar_wait_spin(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return; \
+    }
+template <typename T16, int GAME, int HID, int S>
+__device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32_t tmem, uint32_t rank) {
+    using C = Cfg<GAME, HID, S>;
+    constexpr uint32_t fmt = Op16<T16>::kFmt;
+    constexpr uint32_t idesc_enc = make_idesc(fmt, kTile, C::kUnits), idesc_gate = make_idesc(fmt, kTile, 3 * kSliceUnits),
+                       idesc_head = make_idesc(fmt, kTile, Gm<GAME>::kHeadSingle);
+    constexpr int kChunks = Gm<GAME>::kEncChunks, kGateItems = C::kNS * C::kKB;
+    static_assert(kGateItems % kWSlots == 0 || kWSlots % kGateItems == 0, "a layer's first ring slot");
+    const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
+    // ---- encoder
+    CFX_SPROBE(cfx_p_b, W_FULL, 0);
+    CFX_SPROBE(cfx_p_a, AEXP_FULL, 0);
+#pragma unroll
+    for (int kc = 0; kc < kChunks; kc++) {
+        // block of 64 K columns, first of its 16-byte K pieces, K steps (see expand_full), last chunk of its block
+        const bool full = GAME == CFX_GAME_FULL;
+        const int blk = full && kc >= 12 ? (kc < 14 ? 12 : 13) : kc, first = full && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0;
+        const int ks = full ? full_ksteps(kc) : (kc == kChunks - 1 ? 1 : 4);
+        const bool starts = !(full && (kc == 13 || kc == 15)), ends = !(full && (kc == 12 || kc == 14));
+        const int item = blk / C::kEncPerItem, slot = item % kWSlots, as = kc % kASlots;
+        if (starts && blk % C::kEncPerItem == 0) {
+            CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, (item / kWSlots) & 1);
+            CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
+        }
+        CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + as, (kc / kASlots) & 1);
+        if (kc + 1 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + (kc + 1) % kASlots, ((kc + 1) / kASlots) & 1);
+        tc_fence_after_sync();
+        const uint64_t bd = wdesc + (uint64_t)(((slot * kWSlot + blk % C::kEncPerItem * C::kEncTile) >> 4) + first);
+        const uint32_t a = tmem + kColAexp + as * 32;
+#pragma unroll
+        for (int k = 0; k < ks; k++) mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+        if (kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
+        if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
+        if (ends && ((blk + 1) % C::kEncPerItem == 0 || kc == kChunks - 1)) mma_commit(sm.bar(W_EMPTY + slot));
+    }
+    // ---- layers and heads (a loop over the layers: straight-line code for all of them would be fetched cold)
+    uint32_t wpar = 0;   // parity bit of every ring slot
+#pragma unroll
+    for (int i = 0; i < C::kEncItems; i++) wpar ^= 1u << (i % kWSlots);
+    // the ring slot of a layer's first item: the same for every layer where its items are whole rounds of the ring
+    auto first_slot = [&](int l) { return kGateItems % kWSlots == 0 ? C::kEncItems % kWSlots : (C::kEncItems + l * kGateItems) % kWSlots; };
+#pragma unroll 1
+    for (int l = 0; l < P.L; l++) {
+        const int slot0 = first_slot(l);
+        CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
+        // this CTA's own K blocks first: the gate columns are free when its cells have read them
+#pragma unroll
+        for (int j = 0; j < C::kNS; j++) CFX_SWAIT_SPIN(A_KB + 4 * l + (int)rank * C::kNS + j, 0);
+#pragma unroll
+        for (int j = 0; j < C::kNS; j++) {
+#pragma unroll
+            for (int kb = 0; kb < C::kKB; kb++) {
+                const int slot = (slot0 + j * C::kKB + kb) % kWSlots, slot1 = (slot + 1) % kWSlots;
+                if (j == 0) {
+                    CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * l + kb, 0);
+                    if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * l + kb + 1, 0);
+                }
+                CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, wpar >> slot & 1u);
+                wpar ^= 1u << slot;
+                CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
+                tc_fence_after_sync();
+                const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++)
+                    mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
+                if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL + j));
+                if (j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
+                mma_commit(sm.bar(W_EMPTY + slot));
+            }
+        }
+    }
+    const int slot0 = first_slot(P.L);
+    CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L, 0);
+#pragma unroll
+    for (int kb = 0; kb < C::kKB; kb++) {
+        const int slot = (slot0 + kb / 2) % kWSlots, slot1 = (slot + 1) % kWSlots;
+        CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * P.L + kb, 0);
+        if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L + kb + 1, 0);
+        if (kb % 2 == 0) {
+            CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, wpar >> slot & 1u);
+            CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
+        }
+        tc_fence_after_sync();
+        const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
+#pragma unroll
+        for (int ks = 0; ks < 4; ks++)
+            mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+    }
+    mma_commit(sm.bar(H_FULL));
+}
+
+// ------------------------------------------------------------------ state
+// One thread: box b of the tile (layer b / kBoxes, 32 units of all rows) uses slot b % kSSlots; a slot is loaded again when
+// the box before has been read out of it.
+template <int GAME, int HID, int S>
+__device__ __forceinline__ void role_state(const Smem& sm, const Params& P, int row0, uint32_t rank) {
+    using C = Cfg<GAME, HID, S>;
+    const int boxes = P.L * C::kBoxes;
+    const int quads = P.tile_rows / 32;
+    auto slot_at = [&](int b) { return smem_u32(sm.base + C::kOffS + (b % kSSlots) * kSBox); };
+    auto unit = [&](int b) { return (int)rank * C::kUnits + (b % C::kBoxes) * 32; };
+    auto load = [&](int b) {
+        mbar_arrive_expect_tx(sm.bar(S_FULL + b % kSSlots), quads * kQuadBox);
+        for (int q = 0; q < quads; q++)
+            tensor_g2s_2d(slot_at(b) + q * kQuadBox, &P.state_map[b / C::kBoxes], unit(b), row0 + 32 * q, sm.bar(S_FULL + b % kSSlots));
+    };
+    CFX_SWAIT(REC_FREE, 0);
+    for (int b = 0; b < kSSlots && b < boxes; b++) load(b);
+    for (int b = 0; b < boxes; b++) {
+        CFX_SWAIT(ST_READY + b % kSSlots, (b / kSSlots) & 1);
+        for (int q = 0; q < quads; q++) tensor_s2g_2d(&P.state_map[b / C::kBoxes], slot_at(b) + q * kQuadBox, unit(b), row0 + 32 * q);
+        bulk_commit_group();
+        if (b + kSSlots < boxes) {
+            bulk_wait_group_read<0>();
+            load(b + kSSlots);
+        }
+    }
+    bulk_wait_group<0>();
+}
+
+// ------------------------------------------------------------------ workers
+// Sixteen warps: warp (quadrant, wg) owns TMEM lanes [32 quadrant, + 32) = those rows of the tile, converts
+// chunks wg, wg + 4, ... and handles units [16 wg, 16 wg + 16) of every slice of the CTA.
+template <typename T16, int GAME, int HID, int S>
+__device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
+                                            uint32_t rank) {
+    using Op = Op16<T16>;
+    using C = Cfg<GAME, HID, S>;
+    constexpr int kChunks = Gm<GAME>::kEncChunks, kA = Gm<GAME>::kA;
+    const int quadrant = warp & 3, wg = (warp - kWorkerWarp0) >> 2, row = quadrant * 32 + lane;
+    const uint32_t lane_base = tmem + ((uint32_t)(quadrant * 32) << 16);
+    const int env = row0 + row, quads = P.tile_rows / 32;
+    if (quadrant >= quads) return;   // (rows that nobody reads)
+    const bool valid = env < P.n;   // of a quadrant all rows or none (n is a multiple of 32)
+    const float* bias = reinterpret_cast<const float*>(sm.base + C::kOffBias);
+    const bool samples = quadrant * min(S, quads) / quads == (int)rank;   // this CTA samples the quadrant's rows
+    const unsigned long long step0 = samples && wg == 0 && P.uniforms == nullptr ? *P.step_ctr : 0ull;
+    const bool zero_state = valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
+    if (valid && lane < P.L * C::kNS) {   // this warp's rows of the state, on their way to L2 while the records are expanded
+        const float* q = P.state + ((size_t)(lane / C::kNS) * P.n + env - lane) * HID + ((int)rank * C::kNS + lane % C::kNS) * kSliceUnits;
+        for (int r = wg; r < 32; r += 4) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(q + (size_t)r * HID));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(q + (size_t)r * HID + 32));
+        }
+    }
+
+    // ---- expand
+    const uint8_t* rec = sm.base + row * C::kRowBytes;
+    if (valid) CFX_SWAIT(REC_FULL + quadrant, 0);
+    // a chunk is handed over after the next one is converted: the stores of the one drain meanwhile
+    auto hand_over = [&](int kc) {
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + kc % kASlots));
+    };
+    for (int kc = wg; kc < kChunks; kc += 4) {
+        const int as = kc % kASlots;
+        uint32_t regs[32];
+        if (valid) {
+            if constexpr (GAME == CFX_GAME_CLASSIC) expand_classic<Op>(rec, kc, regs);
+            else expand_full<Op>(rec + 64 * kc, kc, regs);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 32; q++) regs[q] = 0u;
+        }
+        if (kc >= 8) hand_over(kc - 4);
+        if (kc >= kASlots) {
+            CFX_SWAIT(AEXP_EMPTY + as, ((kc / kASlots) - 1) & 1);
+            tc_fence_after_sync();
+        }
+        uint32_t lo[16], hi[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) { lo[q] = regs[q]; hi[q] = regs[16 + q]; }
+        tmem_st16(lane_base + kColAexp + as * 32, lo);
+        tmem_st16(lane_base + kColAexp + as * 32 + 16, hi);
+        if (kc < 4) hand_over(kc);   // (the first one at once: the MMA thread waits for it)
+    }
+    hand_over(wg + (kChunks - 1 - wg) / 4 * 4);
+    __syncwarp();
+    if (lane < S) mbar_arrive_cluster(map_to_cta(sm.bar(REC_FREE), (uint32_t)lane));
+    // The last of the warps that need the step counter raises it, once all have read it (here, where the encoder's MMAs are
+    // waited for; at the kernel's end it was a microsecond of the step)
+    float u = 0.0f;
+    if (samples && wg == 0) {
+        if (valid)
+            u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
+        __syncwarp();
+        if (lane == 0 && P.bump_step) {
+            __threadfence();
+            if (atomicAdd(P.done_ctr, 1u) == P.done_blocks - 1) {
+                *P.step_ctr += 1ULL;
+                *P.done_ctr = 0u;
+            }
+        }
+    }
+
+    // Hands this thread's 16 units of layer input l, slice j, on: into the own K block, and, once the quadrant's four
+    // warps have done so, to the other CTAs.  One warp of the quadrant issues the copies.
+    // (A barrier a slice: a warp may be one slice ahead of another, but not one layer.)
+    auto send = [&](int l, int j, const uint32_t (&h)[8]) {
+        const uint32_t kb = rank * C::kNS + j, block = kb * kABlock;
+        uint8_t* r = sm.base + block + (row >> 3) * 1024 + (row & 7) * 128;
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            *reinterpret_cast<uint4*>(r + (((2 * wg + q) ^ (row & 7)) << 4)) = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+        tc_fence_before_sync();
+        fence_proxy_async_smem();
+        __syncwarp();
+        bool ok = true;
+        if (lane == 0) {
+            mbar_arrive(sm.bar(QUAD + 4 * j + quadrant));
+            if (wg == quadrant) {
+                ok = mbar_wait<false>(sm.bar(QUAD + 4 * j + quadrant), l & 1, sm.abort_flag(), kSite + QUAD);
+                if (ok) {
+                    const uint32_t src = smem_u32(sm.base) + block + quadrant * (kABlock / 4), bar = sm.bar(A_KB + 4 * l + (int)kb);
+                    mbar_arrive(bar);
+#pragma unroll
+                    for (uint32_t d = 1; d < (uint32_t)S; d++) {
+                        const uint32_t peer = (rank + d) % (uint32_t)S;
+                        bulk_s2s(map_to_cta(src, peer), src, kABlock / 4, map_to_cta(bar, peer));
+                    }
+                }
+            }
+        }
+        return __all_sync(0xffffffffu, ok);
+    };
+
+    // ---- encoder output + bias -> layer-0 input
+    uint32_t x[C::kNS][8];   // this thread's units of the layer input, packed: operand and the cell's blend input
+    CFX_SWAIT(ACC_FULL, 0);
+    tc_fence_after_sync();
+#pragma unroll
+    for (int j = 0; j < C::kNS; j++) {
+        uint32_t acc[16];
+        tmem_ld16(lane_base + kColAcc + kSliceUnits * j + kWarpUnits * wg, acc);
+        tmem_wait_ld();
+        const float* b = bias + kSliceUnits * j + kWarpUnits * wg;
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            x[j][q] = Op::pack(__uint_as_float(acc[2 * q]) + b[2 * q], __uint_as_float(acc[2 * q + 1]) + b[2 * q + 1]);
+    }
+    CFX_SWAIT(REC_FREE, 0);
+#pragma unroll
+    for (int j = 0; j < C::kNS; j++)
+        if (!send(0, j, x[j])) return;
+
+    // ---- layers
+    for (int l = 0; l < P.L; l++) {
+#pragma unroll
+        for (int j = 0; j < C::kNS; j++) {
+            CFX_SWAIT(G_FULL + j, l & 1);
+            tc_fence_after_sync();
+            uint32_t zh[16], zg[16], zp[16];
+            tmem_ld16(lane_base + col_gate(j) + kWarpUnits * wg, zh);
+            tmem_ld16(lane_base + col_gate(j) + kSliceUnits + kWarpUnits * wg, zg);
+            tmem_ld16(lane_base + col_gate(j) + 2 * kSliceUnits + kWarpUnits * wg, zp);
+            tmem_wait_ld();
+            const int box = l * C::kBoxes + 2 * j + (wg >> 1), slot = box % kSSlots;
+            CFX_SWAIT(S_FULL + slot, (box / kSSlots) & 1);
+            uint8_t* sp = sm.base + C::kOffS + slot * kSBox + (row >> 3) * 1024 + (row & 7) * 128;
+            auto piece = [&](int q) { return reinterpret_cast<float4*>(sp + (((4 * (wg & 1) + q) ^ (row & 7)) << 4)); };
+            float st[kWarpUnits];
+#pragma unroll
+            for (int q = 0; q < kWarpUnits / 4; q++) {
+                float4 v = *piece(q);
+                if (zero_state) v = make_float4(0.f, 0.f, 0.f, 0.f);
+                st[4 * q] = v.x; st[4 * q + 1] = v.y; st[4 * q + 2] = v.z; st[4 * q + 3] = v.w;
+            }
+            // optional BPTT record of the post-zero input state (craftax_full.cu:9370-9375)
+            if (P.r_state != nullptr && valid) {
+                const size_t at = ((size_t)l * P.n + env) * HID + ((int)rank * C::kNS + j) * kSliceUnits + wg * kWarpUnits;
+                if (P.r_state_bf16) {
+#pragma unroll
+                    for (int q = 0; q < kWarpUnits / 8; q++) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int i = 0; i < 4; i++) w[i] = Op16<__nv_bfloat16>::pack(st[8 * q + 2 * i], st[8 * q + 2 * i + 1]);
+                        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(P.r_state) + at + 8 * q) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kWarpUnits / 4; q++)
+                        *reinterpret_cast<float4*>(P.r_state + at + 4 * q) = make_float4(st[4 * q], st[4 * q + 1], st[4 * q + 2], st[4 * q + 3]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kWarpUnits / 4; q++) {
+#pragma unroll
+                for (int i = 4 * q; i < 4 * q + 4; i += 2) {
+                    const float2 xv = Op::unpack(x[j][i / 2]);
+                    float o0, o1, h0, h1;
+                    mingru_cell_pair(__uint_as_float(zh[i]), __uint_as_float(zh[i + 1]), __uint_as_float(zg[i]), __uint_as_float(zg[i + 1]),
+                                     __uint_as_float(zp[i]), __uint_as_float(zp[i + 1]), st[i], st[i + 1], xv.x, xv.y, o0, o1, h0, h1);
+                    st[i] = o0; st[i + 1] = o1;
+                    x[j][i / 2] = Op::pack(h0, h1);
+                }
+                *piece(q) = make_float4(st[4 * q], st[4 * q + 1], st[4 * q + 2], st[4 * q + 3]);
+            }
+            if (j == 0) CFX_SWAIT(MMA_DONE, l & 1);
+            if (!send(l + 1, j, x[j])) return;
+            if (lane == 0) mbar_arrive(sm.bar(ST_READY + slot));   // (send fenced the box as well)
+        }
+    }
+
+    // ---- heads + sampler: the quadrant's four warps take a quarter of the exponentials each, then the first one draws
+    if (samples) {
+        constexpr int kHeadCols = (kA + 1 + 15) / 16 * 16, kPart = (kA + 3) / 4;
+        CFX_SWAIT(H_FULL, 0);
+        tc_fence_after_sync();
+        uint32_t hv[kHeadCols];
+#pragma unroll
+        for (int b = 0; b < kHeadCols / 16; b++) {
+            uint32_t t[16];
+            tmem_ld16(lane_base + kColHead + 16 * b, t);
+#pragma unroll
+            for (int q = 0; q < 16; q++) hv[16 * b + q] = t[q];
+        }
+        tmem_wait_ld();
+        const float* hb = bias + C::kUnits;
+        float* p = reinterpret_cast<float*>(sm.base + C::kOffW) + row;   // [action][row]: all weights are used up
+        float logits[kA];
+#pragma unroll
+        for (int a = 0; a < kA; a++) logits[a] = __uint_as_float(hv[a]) + hb[a];
+        const float value = __uint_as_float(hv[kA]) + hb[kA];
+        float m = logits[0];
+#pragma unroll
+        for (int a = 1; a < kA; a++) m = fmaxf(m, logits[a]);
+#pragma unroll
+        for (int a = 0; a < kA; a++)
+            if (a / kPart == wg) p[a * kTile] = expf(logits[a] - m);
+        if (wg == 1 && valid) write_logits<GAME>(P, env, logits, value);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + quadrant) : "memory");
+        if (wg == 0 && valid) {
+            float pr[kA];
+#pragma unroll
+            for (int a = 0; a < kA; a++) pr[a] = p[a * kTile];
+            float lp;
+            const int act = draw_action<kA>(logits, pr, m, u, &lp);
+            write_action(P, env, act, lp, value);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ kernel
+template <typename T16, int GAME, int HID, int S>
+__global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_constant__ Params P) {
+    using C = Cfg<GAME, HID, S>;
+    constexpr int kA = Gm<GAME>::kA;
+    CFX_PROBE_DECL(cfx_p_a);
+    CFX_PROBE_DECL(cfx_p_b);
+    extern __shared__ uint8_t smem_raw[];
+    Smem sm;
+    sm.base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    sm.off_bars = C::kOffBars;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_ctarank();
+    const int row0 = P.tile_begin * kTile + (int)blockIdx.x / S * P.tile_rows, quads = P.tile_rows / 32;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp == 0) {   // a lane sets a barrier up
+        for (int i = lane; i < NUM_BARS; i += 32) {
+            uint32_t arrivals = 1, bytes = 0;
+            if (i == REC_FREE) arrivals = S * 4 * quads;
+            else if (i >= AEXP_FULL && i < AEXP_FULL + kASlots) arrivals = quads;
+            else if (i == ACC_FULL) arrivals = 2;                          // the MMAs, and the biases are in place
+            else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = 2 * quads;
+            else if (i == MMA_DONE) arrivals = S;
+            else if (i >= QUAD && i < QUAD + 8) arrivals = 4;
+            else if (i >= A_KB) {
+                const int kb = (i - A_KB) % 4;
+                if (kb / C::kNS == (int)rank) arrivals = quads;
+                else if (kb < C::kKB) bytes = quads * (kABlock / 4);       // a block of another CTA, counted by its bytes
+            }
+            mbar_init(sm.bar(i), arrivals);
+            fence_mbar_init();
+            if (bytes) mbar_arrive_expect_tx(sm.bar(i), bytes);
+        }
+        if (lane == 0) *sm.abort_flag() = 0;
+    }
+    if (warp == 3 && lane == 0)
+        for (int l = 0; l < P.L; l++) prefetch_tensormap(&P.state_map[l]);
+    if (warp == 1) {
+        tmem_alloc(smem_u32(sm.tmem_base()), 512);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    cluster_sync_all();   // the other CTAs' barriers are initialised before anybody copies to them
+    tc_fence_after_sync();
+    const uint32_t tmem = *sm.tmem_base();
+
+    // The operand image and the biases are only ever written by calls that wait for the device, so they may be
+    // read while the kernel in front still runs; everything else waits for it.
+    if (warp == 0) {
+        if (lane == 0) role_weights<GAME, HID, S>(sm, P, rank);
+    } else if (warp == 1) {
+        if (lane == 0) role_mma<T16, GAME, HID, S>(sm, P, tmem, rank);
+    } else if (warp == 2) {
+        // the tile's records, 32 rows a copy
+        wait_for_previous_kernel();
+        if (lane < quads && row0 + 32 * lane < P.n) {
+            mbar_arrive_expect_tx(sm.bar(REC_FULL + lane), C::kQuadBytes);
+            bulk_g2s(smem_u32(sm.base + lane * C::kQuadBytes), P.records + ((size_t)row0 + 32 * lane) * C::kRowBytes,
+                     C::kQuadBytes, sm.bar(REC_FULL + lane));
+        }
+        for (int i = lane; i < C::kUnits + kA + 1; i += 32) {
+            const int a = i - C::kUnits;
+            reinterpret_cast<float*>(sm.base + C::kOffBias)[i] =
+                P.params[a < 0 ? P.off_b_enc + C::kUnits * rank + i : (a < kA ? P.off_b_a + a : P.off_b_v)];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sm.bar(ACC_FULL));
+    } else if (warp == 3) {
+        wait_for_previous_kernel();
+        if (lane == 0) role_state<GAME, HID, S>(sm, P, row0, rank);
+    } else {
+        wait_for_previous_kernel();
+        role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
+    }
+
+    // common exit, also after a timed-out wait: no CTA leaves while another may still copy to it
+    __syncwarp();
+    tc_fence_before_sync();
+    cluster_sync_relaxed();
+    const uint32_t aborted = *sm.abort_flag();
+    if (aborted != 0) {
+        if (tid == 0) atomicCAS(P.status, 0u, aborted | ((uint32_t)blockIdx.x << 8));
+        for (int i = 0; i < 64; i++) __nanosleep(1000);   // time for copies in flight
+        __syncthreads();
+    }
+    if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+static const void* kernel(int precision, int game, int H, int S, int* smem) {
+    const bool h = precision == CFX_PREC_F16;
+#define CFX_SPLIT(G, HID, SS)                                               \
+    do {                                                                    \
+        *smem = smem_bytes<G, HID, SS>();                                   \
+        return h ? (const void*)k_policy_split<__half, G, HID, SS>          \
+                 : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS>;  \
+    } while (0)
+    if (game == CFX_GAME_CLASSIC) {
+        if (S == 4) CFX_SPLIT(CFX_GAME_CLASSIC, 256, 4);
+        CFX_SPLIT(CFX_GAME_CLASSIC, 256, 2);
+    }
+    if (H == 128) CFX_SPLIT(CFX_GAME_FULL, 128, 2);
+    if (S == 4) CFX_SPLIT(CFX_GAME_FULL, 256, 4);
+    CFX_SPLIT(CFX_GAME_FULL, 256, 2);
+#undef CFX_SPLIT
+}
+
+static cudaLaunchConfig_t config(cudaLaunchAttribute (&at)[2], int blocks, int S, int smem, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see wait_for_previous_kernel
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+
+}  // namespace split
+
+int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_clusters) {
+    *max_clusters = 0;
+    if (H / 64 / S < 1) return CFX_OK;
+    int smem = 0;
+    const void* k = split::kernel(precision, game, H, S, &smem);
+    CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaLaunchAttribute at[2];
+    cudaLaunchConfig_t cfg = split::config(at, sm_count / S * S, S, smem, nullptr);
+    cfg.numAttrs = 1;
+    int nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, k, &cfg) == cudaSuccess) *max_clusters = nc;
+    else cudaGetLastError();
+    return CFX_OK;
+}
+
+int split_launch(int precision, int game, int H, int S, int tiles, const Params& P, cudaStream_t st) {
+    int smem = 0;
+    const void* k = split::kernel(precision, game, H, S, &smem);
+    cudaLaunchAttribute at[2];
+    cudaLaunchConfig_t cfg = split::config(at, tiles * S, S, smem, st);
+    void* args[1] = {(void*)&P};
+    CFX_CUDA(cudaLaunchKernelExC(&cfg, k, args));
+    return CFX_OK;
+}
+
+}  // namespace fused
+}  // namespace cfx

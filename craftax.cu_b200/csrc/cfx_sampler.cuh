@@ -17,19 +17,12 @@ __device__ __forceinline__ float philox_uniform(uint64_t seed, uint64_t env, uin
 // cf_nn_sample_action (craftax_full.cu:9147-9165): running max, p = expf(l - m)
 // summed in ascending action order, first action whose running sum reaches
 // u * total (default A - 1), logprob = l - m - logf(total).  A is a template
-// parameter so that p[] stays in registers.
+// parameter so that p[] stays in registers (draw_action takes the maximum and the exponentials as given).
 template <int A>
-__device__ __forceinline__ int sample_action(const float (&logits)[A], float u, float* logprob) {
-    float m = logits[0];
-#pragma unroll
-    for (int a = 1; a < A; a++) m = fmaxf(m, logits[a]);
-    float p[A];
+__device__ __forceinline__ int draw_action(const float (&logits)[A], const float (&p)[A], float m, float u, float* logprob) {
     float total = 0.0f;
 #pragma unroll
-    for (int a = 0; a < A; a++) {
-        p[a] = expf(logits[a] - m);
-        total += p[a];
-    }
+    for (int a = 0; a < A; a++) total += p[a];
     float target = u * total, cum = 0.0f;
     int action = A - 1;
     float la = logits[A - 1];
@@ -45,6 +38,16 @@ __device__ __forceinline__ int sample_action(const float (&logits)[A], float u, 
     }
     *logprob = la - m - logf(total);
     return action;
+}
+template <int A>
+__device__ __forceinline__ int sample_action(const float (&logits)[A], float u, float* logprob) {
+    float m = logits[0];
+#pragma unroll
+    for (int a = 1; a < A; a++) m = fmaxf(m, logits[a]);
+    float p[A];
+#pragma unroll
+    for (int a = 0; a < A; a++) p[a] = expf(logits[a] - m);
+    return draw_action<A>(logits, p, m, u, logprob);
 }
 
 // The same with a runtime A, for the stand-alone sampler: the maximum m and p[a] = expf(l[a] - m)
