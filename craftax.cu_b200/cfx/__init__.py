@@ -363,20 +363,20 @@ class Policy:
         rec = np.ascontiguousarray(records, np.uint8)
         assert rec.size == n * self.rec_bytes
         o = out if out is not None else {}
-        o.setdefault("env_actions", np.empty(n, np.float32))
-        o.setdefault("actions", np.empty(n, np.int32))
-        o.setdefault("logprobs", np.empty(n, np.float32))
-        o.setdefault("values", np.empty(n, np.float32))
+        want = [("env_actions", n, np.float32), ("actions", n, np.int32), ("logprobs", n, np.float32),
+                ("values", n, np.float32)]
         if want_logits:
-            o.setdefault("logits_av", np.empty((n, A + 1), np.float32))
+            want.append(("logits_av", (n, A + 1), np.float32))
         if want_r_state:
-            o.setdefault("r_state", np.empty((self.L, n, self.H),
-                                             np.uint16 if want_r_state == "bf16" else np.float32))
+            want.append(("r_state", (self.L, n, self.H), np.uint16 if want_r_state == "bf16" else np.float32))
+        for name, shape, dtype in want:
+            if name not in o:
+                o[name] = np.empty(shape, dtype)
         pt = None if prev_terminals is None else np.ascontiguousarray(prev_terminals, np.float32)
         u = None if uniforms is None else np.ascontiguousarray(uniforms, np.float32)
 
-        def hp(a):
-            return None if a is None else a.ctypes.data
+        def hp(a):   # (as `a.ctypes.data`, a third of its time)
+            return None if a is None else a.__array_interface__["data"][0]
         io = ForwardIO(hp(rec), hp(pt), hp(u), hp(o["env_actions"]), hp(o["actions"]),
                        hp(o["logprobs"]), hp(o["values"]), hp(o.get("logits_av")),
                        hp(o.get("r_state")), seed, env_offset, 1 if bump_step else 0,

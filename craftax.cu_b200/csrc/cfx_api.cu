@@ -29,7 +29,8 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
 using namespace cfx;
 
 constexpr int kHostSlicesMax = 8;
-constexpr size_t kHostSliceEnvs = 32768;   // smallest slice of the pipelined host-buffer forward
+constexpr size_t kHostSliceEnvs = 32768;   // a slice of the pipelined host-buffer forward for this many envs, from two on
+constexpr size_t kHostSmallEnvs = 8192;    // batches whose per-env arrays the kernel reads and writes in host memory
 
 // The handle: role of CuPolicy (craftax_full.cu:11758-11796).
 struct cfx_policy {
@@ -57,10 +58,12 @@ struct cfx_policy {
     float* st_values = nullptr;
     float* st_logits = nullptr;
     float* st_r_state = nullptr;
-    // cfx_policy_forward_host: copy stream and per-slice events of the pipelined upload
-    cudaStream_t copy_stream = nullptr;
-    cudaEvent_t slice_ready[kHostSlicesMax] = {};
+    // cfx_policy_forward_host: streams of the pipelined upload and read-back, events per slice; page-locked memory for
+    // what a small batch's kernel reads and writes in place
+    cudaStream_t copy_stream = nullptr, out_stream = nullptr;
+    cudaEvent_t slice_ready[kHostSlicesMax] = {}, slice_done[kHostSlicesMax] = {};
     cudaEvent_t host_fence = nullptr;
+    uint8_t* host_io = nullptr;
 };
 
 static void free_dev(void* p) {
@@ -68,18 +71,14 @@ static void free_dev(void* p) {
 }
 
 static int policy_refresh_mirrors(cfx_policy* p, cudaStream_t st) {
+    if (p->precision != CFX_PREC_FP32) return fused_refresh(p->fused, p->params, st);
     const ArenaLayout o = ArenaLayout::make(p->H, p->L, p->A, p->obs);
-    int rc = launch_transpose_gates(p->params + o.w_gru, p->gates_t, p->H, p->L, st);
-    if (rc) return rc;
-    if (p->fused) {
-        rc = fused_refresh(p->fused, p->params, st);
-        if (rc) return rc;
-    }
-    return CFX_OK;
+    return launch_transpose_gates(p->params + o.w_gru, p->gates_t, p->H, p->L, st);
 }
 
-// What only the fp32 mode needs: two activation buffers [H][n] and room for the logits.
+// What only the fp32 mode needs: the transposed gate matrices, two activation buffers [H][n] and room for the logits.
 static int policy_ensure_fp32(cfx_policy* p) {
+    if (!p->gates_t) CFX_CUDA(cudaMalloc((void**)&p->gates_t, (size_t)p->L * 3 * p->H * p->H * sizeof(float)));
     for (int i = 0; i < 2; i++)
         if (!p->scratch_h[i]) CFX_CUDA(cudaMalloc((void**)&p->scratch_h[i], (size_t)p->H * p->n * sizeof(float)));
     if (!p->logits_scratch)
@@ -182,7 +181,6 @@ static int policy_create(cfx_policy** out, int device, int num_envs, int hidden,
         if (_e != cudaSuccess) return fail(cuda_fail(_e, "cudaMalloc " #ptr, __FILE__, __LINE__)); \
     } while (0)
     CFX_TRY_ALLOC(p->params, p->param_count * sizeof(float));
-    CFX_TRY_ALLOC(p->gates_t, (size_t)layers * 3 * hidden * hidden * sizeof(float));
     CFX_TRY_ALLOC(p->state, (size_t)layers * hn * sizeof(float));
     CFX_TRY_ALLOC(p->step_ctr, 2 * sizeof(unsigned long long));
 #undef CFX_TRY_ALLOC
@@ -223,10 +221,14 @@ int cfx_policy_destroy(cfx_policy* p) {
     free_dev(p->st_values);
     free_dev(p->st_logits);
     free_dev(p->st_r_state);
-    for (int i = 0; i < kHostSlicesMax; i++)
+    for (int i = 0; i < kHostSlicesMax; i++) {
         if (p->slice_ready[i]) cudaEventDestroy(p->slice_ready[i]);
+        if (p->slice_done[i]) cudaEventDestroy(p->slice_done[i]);
+    }
     if (p->host_fence) cudaEventDestroy(p->host_fence);
     if (p->copy_stream) cudaStreamDestroy(p->copy_stream);
+    if (p->out_stream) cudaStreamDestroy(p->out_stream);
+    if (p->host_io) cudaFreeHost(p->host_io);
     if (p->stream) cudaStreamDestroy(p->stream);
     delete p;
     return CFX_OK;
@@ -360,6 +362,9 @@ int cfx_policy_set_precision(cfx_policy* p, int precision) {
             fused_destroy(p->fused);
             p->fused = nullptr;
         }
+        rc = policy_refresh_mirrors(p, p->stream);
+        if (rc) return rc;
+        CFX_CUDA(cudaStreamSynchronize(p->stream));
         return CFX_OK;
     }
     int rc = policy_ensure_fused(p);
@@ -484,21 +489,13 @@ int cfx_policy_forward(cfx_policy* p, const cfx_forward_io* io, void* stream) {
 
 }  // extern "C"
 
+static int check_status(cfx_policy* p);
+
 extern "C" int cfx_policy_check(cfx_policy* p, void* stream) {
     CFX_REQUIRE(p, "cfx_policy_check: NULL handle");
     CFX_GUARD(p->device);
-    cudaStream_t st = stream ? (cudaStream_t)stream : p->stream;
-    CFX_CUDA(cudaStreamSynchronize(st));
-    if (p->fused) {
-        unsigned status = 0;
-        int rc = fused_check_status(p->fused, st, &status);
-        if (rc) return rc;
-        if (status) {
-            set_error("device-side wait timed out: site %u, block %u", status & 0xFF, status >> 8);
-            return CFX_ERR_DEVICE_TIMEOUT;
-        }
-    }
-    return CFX_OK;
+    CFX_CUDA(cudaStreamSynchronize(stream ? (cudaStream_t)stream : p->stream));
+    return check_status(p);
 }
 
 extern "C" int cfx_selftest_wait_timeout(int device, unsigned limit_ms) {
@@ -523,6 +520,81 @@ static int ensure_staging(T** slot, size_t count) {
     return CFX_OK;
 }
 
+static int check_status(cfx_policy* p) {
+    const unsigned status = p->fused ? fused_take_status(p->fused) : 0u;
+    if (status == 0) return CFX_OK;
+    set_error("device-side wait timed out: site %u, block %u", status & 0xFF, status >> 8);
+    return CFX_ERR_DEVICE_TIMEOUT;
+}
+
+// The device's address of page-locked host memory, or NULL.
+static void* device_address(const void* host) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+}
+
+// Small batches, fused kernel: what such a step costs is calls and round trips, not bytes.  Flags, uniforms and the four
+// per-env outputs are read and written by the kernel in page-locked host memory of the handle (a few KB, copied
+// from and to the caller's arrays here).  The smallest batches' records are fetched by a kernel, which saves the
+// hand-over between a copy engine and the SMs, and their logits are written in place: to the caller's array where it
+// is page-locked, else by way of the handle's.  Beyond, a copy moves them faster than the SMs do over PCIe.
+// us a call, with a copy for each array and for the status word before -> now: 32 envs 82 -> 42, 1,024 envs 108 -> 68,
+// 4,096 envs 178 -> 150 (512 envs: 58 with the records fetched by the kernel, 55 copied).
+constexpr size_t kHostFetchEnvs = 256, kHostLogitsEnvs = 2048, kHostLogitsCopyEnvs = 256;
+static int forward_host_small(cfx_policy* p, const cfx_forward_io* h, cfx_forward_io* d) {
+    cudaStream_t st = p->stream;
+    const size_t n = (size_t)p->n, row = (size_t)(p->A + 1) * 4;
+    if (!p->host_io)
+        CFX_CUDA(cudaHostAlloc((void**)&p->host_io, 6 * n * 4 + (n <= kHostLogitsCopyEnvs ? n * row : 0),
+                               cudaHostAllocPortable | cudaHostAllocMapped));
+    auto part = [&](int i) { return p->host_io + (size_t)i * n * 4; };   // n is a multiple of 32: 128-byte aligned
+    auto in = [&](const float* src, int i) -> const float* {
+        if (!src) return nullptr;
+        memcpy(part(i), src, n * 4);
+        return (const float*)part(i);
+    };
+    d->prev_terminals = in(h->prev_terminals, 0);
+    d->uniforms = in(h->uniforms, 1);
+    d->env_actions = h->env_actions ? (float*)part(2) : nullptr;
+    d->actions = (int32_t*)part(3);
+    d->logprobs = h->logprobs ? (float*)part(4) : nullptr;
+    d->values = h->values ? (float*)part(5) : nullptr;
+    void* logits = h->logits_av && n <= kHostLogitsEnvs ? device_address(h->logits_av) : nullptr;
+    if (logits && ((uintptr_t)logits & 15) != 0) logits = nullptr;
+    const bool staged = h->logits_av && !logits && n <= kHostLogitsCopyEnvs;
+    if (staged) logits = part(6);
+    if (logits) d->logits_av = (float*)logits;
+    const size_t bytes = n * (size_t)p->rec_bytes;
+    const void* rec = n <= kHostFetchEnvs ? device_address(h->records) : nullptr;
+    int rc;
+    if (rec && ((uintptr_t)rec & 15) == 0) {
+        if ((rc = launch_fetch(rec, p->st_records, bytes, st))) return rc;
+    } else {
+        CFX_CUDA(cudaMemcpyAsync(p->st_records, h->records, bytes, cudaMemcpyHostToDevice, st));
+    }
+    if ((rc = cfx_policy_forward(p, d, st))) return rc;
+    if (h->logits_av && !logits)
+        CFX_CUDA(cudaMemcpyAsync(h->logits_av, p->st_logits, n * row, cudaMemcpyDeviceToHost, st));
+    if (h->r_state)
+        CFX_CUDA(cudaMemcpyAsync(h->r_state, p->st_r_state, (size_t)p->L * n * p->H * (h->r_state_bf16 ? 2 : 4),
+                                 cudaMemcpyDeviceToHost, st));
+    CFX_CUDA(cudaStreamSynchronize(st));
+    if ((rc = check_status(p))) return rc;
+    auto out = [&](void* dst, int i, size_t bytes_out) {
+        if (dst) memcpy(dst, part(i), bytes_out);
+    };
+    out(h->env_actions, 2, n * 4);
+    out(h->actions, 3, n * 4);
+    out(h->logprobs, 4, n * 4);
+    out(h->values, 5, n * 4);
+    if (staged) out(h->logits_av, 6, n * row);
+    return CFX_OK;
+}
+
 extern "C" {
 
 int cfx_policy_forward_host(cfx_policy* p, const cfx_forward_io* h) {
@@ -531,72 +603,93 @@ int cfx_policy_forward_host(cfx_policy* p, const cfx_forward_io* h) {
     CFX_GUARD(p->device);
     cudaStream_t st = p->stream;
     const size_t n = (size_t)p->n;
-    // r_state staging in floats: bf16 records take half
-    const size_t lav = n * (size_t)(p->A + 1), rs = (size_t)p->L * n * p->H / (h->r_state_bf16 ? 2 : 1);
+    const bool fused = p->precision != CFX_PREC_FP32, small = fused && n < kHostSmallEnvs;
+    const size_t lav = (size_t)(p->A + 1);
     int rc;
     if ((rc = ensure_staging(&p->st_records, n * (size_t)p->rec_bytes))) return rc;
+    if (h->logits_av && (rc = ensure_staging(&p->st_logits, n * lav))) return rc;
+    if (h->r_state && (rc = ensure_staging(&p->st_r_state, (size_t)p->L * n * p->H))) return rc;
+    cfx_forward_io d = *h;
+    d.records = p->st_records;
+    d.logits_av = h->logits_av ? p->st_logits : nullptr;
+    d.r_state = h->r_state ? p->st_r_state : nullptr;
+    if (small) return forward_host_small(p, h, &d);
+
     if ((rc = ensure_staging(&p->st_actions, n))) return rc;
     if (h->prev_terminals && (rc = ensure_staging(&p->st_terminals, n))) return rc;
     if (h->uniforms && (rc = ensure_staging(&p->st_uniforms, n))) return rc;
     if (h->env_actions && (rc = ensure_staging(&p->st_env_actions, n))) return rc;
     if (h->logprobs && (rc = ensure_staging(&p->st_logprobs, n))) return rc;
     if (h->values && (rc = ensure_staging(&p->st_values, n))) return rc;
-    if (h->logits_av && (rc = ensure_staging(&p->st_logits, lav))) return rc;
-    if (h->r_state && (rc = ensure_staging(&p->st_r_state, (size_t)p->L * n * p->H))) return rc;
-
-    cfx_forward_io d = *h;
-    d.records = p->st_records;
     d.prev_terminals = h->prev_terminals ? p->st_terminals : nullptr;
     d.uniforms = h->uniforms ? p->st_uniforms : nullptr;
     d.env_actions = h->env_actions ? p->st_env_actions : nullptr;
     d.actions = p->st_actions;
     d.logprobs = h->logprobs ? p->st_logprobs : nullptr;
     d.values = h->values ? p->st_values : nullptr;
-    d.logits_av = h->logits_av ? p->st_logits : nullptr;
-    d.r_state = h->r_state ? p->st_r_state : nullptr;
-
-    // The record upload dominates a host-buffer step (996 bytes per env over PCIe against
-    // ~1.6 ns of kernel time).  With the fused kernel and a large batch the records go up in
-    // slices on a copy stream and the kernel runs slice by slice behind them (a launch takes a
-    // tile range), so that only the last slice's kernel is not hidden under the upload.
-    const int tiles = (int)((n + 127) / 128);
-    int slices = 1;
-    if (p->precision != CFX_PREC_FP32) {
-        slices = (int)(n / kHostSliceEnvs);
-        slices = slices < 1 ? 1 : (slices > kHostSlicesMax ? kHostSlicesMax : slices);
-    }
-    if (slices == 1) {
-        CFX_CUDA(cudaMemcpyAsync(p->st_records, h->records, n * (size_t)p->rec_bytes, cudaMemcpyHostToDevice, st));
+    auto inputs = [&](cudaStream_t s) {
+        cudaError_t e = cudaSuccess;
         if (h->prev_terminals)
-            CFX_CUDA(cudaMemcpyAsync(p->st_terminals, h->prev_terminals, n * sizeof(float),
-                                     cudaMemcpyHostToDevice, st));
-        if (h->uniforms)
-            CFX_CUDA(cudaMemcpyAsync(p->st_uniforms, h->uniforms, n * sizeof(float),
-                                     cudaMemcpyHostToDevice, st));
+            e = cudaMemcpyAsync(p->st_terminals, h->prev_terminals, n * sizeof(float), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess && h->uniforms)
+            e = cudaMemcpyAsync(p->st_uniforms, h->uniforms, n * sizeof(float), cudaMemcpyHostToDevice, s);
+        return e;
+    };
+    // the outputs of envs [e0, e1)
+    auto outputs = [&](size_t e0, size_t e1, cudaStream_t s) {
+        auto one = [&](void* dst, const void* src, size_t words) {
+            if (!dst) return cudaSuccess;
+            return cudaMemcpyAsync((uint8_t*)dst + e0 * words * 4, (const uint8_t*)src + e0 * words * 4, (e1 - e0) * words * 4,
+                                   cudaMemcpyDeviceToHost, s);
+        };
+        cudaError_t e = one(h->logits_av, p->st_logits, lav);
+        if (e == cudaSuccess) e = one(h->actions, p->st_actions, 1);
+        if (e == cudaSuccess) e = one(h->env_actions, p->st_env_actions, 1);
+        if (e == cudaSuccess) e = one(h->logprobs, p->st_logprobs, 1);
+        if (e == cudaSuccess) e = one(h->values, p->st_values, 1);
+        return e;
+    };
+    cudaStream_t last = st;   // the stream whose end is the end of the call
+    if (!fused || n < 2 * kHostSliceEnvs) {
+        CFX_CUDA(cudaMemcpyAsync(p->st_records, h->records, n * (size_t)p->rec_bytes, cudaMemcpyHostToDevice, st));
+        CFX_CUDA(inputs(st));
         rc = cfx_policy_forward(p, &d, st);
         if (rc) return rc;
+        CFX_CUDA(outputs(0, n, st));
     } else {
+        // The record upload dominates a host-buffer step (996 bytes per env over PCIe against 192 bytes of outputs the other
+        // way and ~1.6 ns of kernel time).  The records go up in slices on a stream of their own, the kernel runs slice by
+        // slice behind them (a launch takes a tile range) and the outputs of a slice go down on a third stream, so
+        // that only the last slice's kernel and outputs are not hidden under the upload.  The slices shrink: a slice's kernel
+        // and outputs take a third of its upload, so that each is done when the next, smaller one has arrived.
+        // 65,536 envs: 1,533 us with two equal slices and the outputs at the end, 1,357 us now (the upload alone 1,180).
+        int slices = (int)(n / kHostSliceEnvs);
+        slices = slices > kHostSlicesMax ? kHostSlicesMax : slices;
         if (!p->copy_stream) {
             CFX_CUDA(cudaStreamCreateWithFlags(&p->copy_stream, cudaStreamNonBlocking));
+            CFX_CUDA(cudaStreamCreateWithFlags(&p->out_stream, cudaStreamNonBlocking));
             CFX_CUDA(cudaEventCreateWithFlags(&p->host_fence, cudaEventDisableTiming));
-            for (int i = 0; i < kHostSlicesMax; i++)
+            for (int i = 0; i < kHostSlicesMax; i++) {
                 CFX_CUDA(cudaEventCreateWithFlags(&p->slice_ready[i], cudaEventDisableTiming));
+                CFX_CUDA(cudaEventCreateWithFlags(&p->slice_done[i], cudaEventDisableTiming));
+            }
         }
         cudaStream_t cs = p->copy_stream;
         // the staging buffers may still be read by work queued earlier on the handle's stream
         CFX_CUDA(cudaEventRecord(p->host_fence, st));
         CFX_CUDA(cudaStreamWaitEvent(cs, p->host_fence, 0));
-        if (h->prev_terminals)
-            CFX_CUDA(cudaMemcpyAsync(p->st_terminals, h->prev_terminals, n * sizeof(float),
-                                     cudaMemcpyHostToDevice, cs));
-        if (h->uniforms)
-            CFX_CUDA(cudaMemcpyAsync(p->st_uniforms, h->uniforms, n * sizeof(float),
-                                     cudaMemcpyHostToDevice, cs));
-        int per = (tiles + slices - 1) / slices;
-        per += per & 1;   // slices start at even tiles (CTA pairs)
+        CFX_CUDA(inputs(cs));
+        // what is left after slice k: from the whole batch down to the last slice in equal ratios
+        const double end = (double)n / 5 < 16384 ? (double)n / 5 : 16384.0, ratio = pow(end / (double)n, 1.0 / (slices - 1));
+        const int tiles = (int)((n + 127) / 128);
+        double left = (double)n;
         int launches = 0;
-        for (int k = 0, t0 = 0; t0 < tiles; k++, t0 += per) {
-            const int t1 = t0 + per < tiles ? t0 + per : tiles;
+        for (int k = 0, t0 = 0; t0 < tiles; k++) {
+            left *= ratio;
+            int t1 = k == slices - 1 ? tiles : (int)(((double)n - left) / 128);
+            t1 += t1 & 1;   // slices start at even tiles (CTA pairs)
+            t1 = t1 < t0 + 2 ? t0 + 2 : t1;
+            t1 = t1 > tiles ? tiles : t1;
             const size_t e0 = (size_t)t0 * 128, e1 = (size_t)t1 * 128 < n ? (size_t)t1 * 128 : n;
             CFX_CUDA(cudaMemcpyAsync(p->st_records + e0 * p->rec_bytes, h->records + e0 * p->rec_bytes,
                                      (e1 - e0) * (size_t)p->rec_bytes, cudaMemcpyHostToDevice, cs));
@@ -607,21 +700,19 @@ int cfx_policy_forward_host(cfx_policy* p, const cfx_forward_io* h) {
             rc = forward_range(p, &dk, st, t0, t1);
             if (rc) return rc;
             launches += p->last_launches;
+            CFX_CUDA(cudaEventRecord(p->slice_done[k], st));
+            CFX_CUDA(cudaStreamWaitEvent(p->out_stream, p->slice_done[k], 0));
+            CFX_CUDA(outputs(e0, e1, p->out_stream));
+            t0 = t1;
         }
         p->last_launches = launches;
+        last = p->out_stream;
     }
-    CFX_CUDA(cudaMemcpyAsync(h->actions, p->st_actions, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    if (h->env_actions)
-        CFX_CUDA(cudaMemcpyAsync(h->env_actions, p->st_env_actions, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (h->logprobs)
-        CFX_CUDA(cudaMemcpyAsync(h->logprobs, p->st_logprobs, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (h->values)
-        CFX_CUDA(cudaMemcpyAsync(h->values, p->st_values, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (h->logits_av)
-        CFX_CUDA(cudaMemcpyAsync(h->logits_av, p->st_logits, lav * sizeof(float), cudaMemcpyDeviceToHost, st));
     if (h->r_state)
-        CFX_CUDA(cudaMemcpyAsync(h->r_state, p->st_r_state, rs * sizeof(float), cudaMemcpyDeviceToHost, st));
-    return cfx_policy_check(p, st);
+        CFX_CUDA(cudaMemcpyAsync(h->r_state, p->st_r_state, (size_t)p->L * n * p->H * (h->r_state_bf16 ? 2 : 4),
+                                 cudaMemcpyDeviceToHost, last));
+    CFX_CUDA(cudaStreamSynchronize(last));
+    return check_status(p);
 }
 
 // ------------------------------------------------------------------ stand-alone stages

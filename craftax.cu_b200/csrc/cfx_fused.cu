@@ -1096,7 +1096,7 @@ k_policy_fused(const __grid_constant__ Params P) {
     else __syncthreads();
     const uint32_t aborted = *sm.abort_flag();
     if (aborted != 0) {
-        if (tid == 0) atomicCAS(P.status, 0u, aborted | ((uint32_t)blockIdx.x << 8));
+        if (tid == 0) *reinterpret_cast<volatile uint32_t*>(P.status) = aborted | ((uint32_t)blockIdx.x << 8);
         // give copies that are still in flight time to land before shared memory is released
         for (int i = 0; i < 64; i++) __nanosleep(1000);
         __syncthreads();
@@ -1159,7 +1159,8 @@ struct FusedPlan {
     int device, n, H, L, A, precision;
     int game = CFX_GAME_FULL;
     uint8_t* image = nullptr;
-    uint32_t* status = nullptr;    // [0] status word, [1] finished-block counter
+    uint32_t* status = nullptr;    // status word, in page-locked host memory: the host reads it without a copy
+    uint32_t* done_ctr = nullptr;  // finished-block counter
     float* state = nullptr;
     const float* params = nullptr;
     CUtensorMap state_map[fused::kMaxLayers];
@@ -1217,20 +1218,24 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
         set_error("fused kernel: unsupported shape/precision");
         return CFX_ERR_UNSUPPORTED;
     }
-    cudaDeviceProp prop;
-    CFX_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10) {
-        set_error("fused kernel needs an sm_100 GPU (found sm_%d%d)", prop.major, prop.minor);
+    int major = 0, minor = 0, sm_count = 0;
+    CFX_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    CFX_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    CFX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+    if (major != 10) {
+        set_error("fused kernel needs an sm_100 GPU (found sm_%d%d)", major, minor);
         return CFX_ERR_UNSUPPORTED;
     }
     FusedPlan* p = new FusedPlan();
     p->device = device; p->n = n; p->H = H; p->L = L; p->A = A; p->precision = precision;
     p->game = game;
     p->state = state;
-    p->sm_count = prop.multiProcessorCount;
+    p->sm_count = sm_count;
     cudaError_t e = cudaMalloc((void**)&p->image, fused_image_bytes(game, H, L));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&p->status, 2 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(p->status, 0, 2 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&p->done_ctr, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(p->done_ctr, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&p->status, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e == cudaSuccess) *p->status = 0;
     if (e != cudaSuccess) {
         fused_destroy(p);
         return cuda_fail(e, "fused_create alloc", __FILE__, __LINE__);
@@ -1366,7 +1371,7 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     P.r_state_bf16 = a.r_state_bf16;
     P.step_ctr = a.step_ctr;
     P.status = p->status;
-    P.done_ctr = p->status + 1;
+    P.done_ctr = p->done_ctr;
     P.bump_step = a.bump_step;
     P.seed = a.seed;
     P.env_offset = a.env_offset;
@@ -1426,20 +1431,18 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     return CFX_OK;
 }
 
-int fused_check_status(FusedPlan* p, cudaStream_t st, unsigned* status) {
-    uint32_t v = 0;
-    CFX_CUDA(cudaMemcpyAsync(&v, p->status, sizeof(v), cudaMemcpyDeviceToHost, st));
-    CFX_CUDA(cudaStreamSynchronize(st));
-    if (v != 0) CFX_CUDA(cudaMemsetAsync(p->status, 0, sizeof(v), st));
-    if (status) *status = v;
-    return CFX_OK;
+unsigned fused_take_status(FusedPlan* p) {
+    volatile uint32_t* word = p->status;
+    const uint32_t v = *word;
+    if (v != 0) *word = 0;
+    return v;
 }
-
 
 void fused_destroy(FusedPlan* p) {
     if (!p) return;
     if (p->image) cudaFree(p->image);
-    if (p->status) cudaFree(p->status);
+    if (p->status) cudaFreeHost(p->status);
+    if (p->done_ctr) cudaFree(p->done_ctr);
     delete p;
 }
 

@@ -34,8 +34,8 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
 // Rebuilds the operand mirrors from the fp32 arena (device pointer).
 int fused_refresh(FusedPlan* plan, const float* params, cudaStream_t st);
 int fused_forward(FusedPlan* plan, const FusedArgs& a, cudaStream_t st, int* launches);
-// Reads and clears the device status word (non-zero = a bounded wait gave up).
-int fused_check_status(FusedPlan* plan, cudaStream_t st, unsigned* status);
+// Reads and clears the status word (non-zero = a bounded wait gave up); the stream has been waited for.
+unsigned fused_take_status(FusedPlan* plan);
 void fused_destroy(FusedPlan* plan);
 
 int fused_selftest_wait_timeout(unsigned limit_ms, unsigned* status_out);

@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     cluster_sync_relaxed();
     const uint32_t aborted = *sm.abort_flag();
     if (aborted != 0) {
-        if (tid == 0) atomicCAS(P.status, 0u, aborted | ((uint32_t)blockIdx.x << 8));
+        if (tid == 0) *reinterpret_cast<volatile uint32_t*>(P.status) = aborted | ((uint32_t)blockIdx.x << 8);
         for (int i = 0; i < 64; i++) __nanosleep(1000);   // time for copies in flight
         __syncthreads();
     }

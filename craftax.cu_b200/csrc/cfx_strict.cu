@@ -556,6 +556,12 @@ __global__ void k_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, in
     if (e < n) u[e] = philox_uniform(seed, env_offset + (uint64_t)e, step);
 }
 
+__global__ void k_fetch(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t count) {
+    wait_for_previous_kernel();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) dst[i] = src[i];
+}
+
 __global__ void k_bump(unsigned long long* ctr) { *ctr += 1ULL; }
 
 // Gate matrices transposed for the strict layer kernel: Wt[l][j][r] = W[l][r][j].
@@ -609,6 +615,11 @@ int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, fl
     k_uniforms<<<(n + 255) / 256, 256, 0, st>>>(seed, env_offset, step, n, u);
     CFX_CUDA(cudaGetLastError());
     return CFX_OK;
+}
+
+int launch_fetch(const void* host, void* dst, size_t bytes, cudaStream_t st) {
+    const size_t count = bytes / 16;
+    return launch_chained(k_fetch, dim3((unsigned)((count + 127) / 128)), 128, 0, st, (const uint4*)host, (uint4*)dst, count);
 }
 
 int launch_bump(unsigned long long* ctr, cudaStream_t st) {

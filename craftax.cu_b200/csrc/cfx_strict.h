@@ -36,6 +36,8 @@ int launch_sample(const float* logits, int ld, int A, const float* u, uint64_t s
                   float* env_actions, int32_t* actions, float* logprobs, float* values,
                   cudaStream_t st);
 int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, float* u, cudaStream_t st);
+// copies `bytes` (a multiple of 16) from page-locked host memory, both 16-byte aligned
+int launch_fetch(const void* host, void* dst, size_t bytes, cudaStream_t st);
 int launch_bump(unsigned long long* ctr, cudaStream_t st);
 int launch_transpose_gates(const float* W, float* Wt, int H, int L, cudaStream_t st);
 int launch_init_uniform(float* w, int count, float bound, uint64_t seed, int subseq, cudaStream_t st);
