@@ -455,6 +455,7 @@ static int forward_range(cfx_policy* p, const cfx_forward_io* io, void* stream, 
         a.env_offset = io->env_offset;
         a.step_ctr = p->step_ctr;
         a.bump_step = io->bump_step ? 1 : 0;
+        a.weights_ready = 1;
         rc = strict_forward(a, st, &launches);
     } else {
         CFX_REQUIRE(p->fused != nullptr, "cfx_policy_forward: fused plan missing");

@@ -1057,10 +1057,10 @@ k_policy_fused(const __grid_constant__ Params P) {
         prefetch_tensormap(&P.rec_map);
         for (int l = 0; l < P.L; l++) prefetch_tensormap(&P.state_map[l]);
     }
-    // Everything above is this launch's own; from here on memory is read that the kernel in front in the
-    // stream may have written.  The next kernel may start its own set-up as soon as SMs come free.
-    wait_for_previous_kernel();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // The next kernel may start its own set-up as soon as SMs come free.  The operand image and the biases are only
+    // ever written by calls that wait for the device, so they may be read while the kernel in front in the stream
+    // still runs; the roles that touch anything else wait for it.
+    launch_next_kernel();
     for (int i = tid; i < kH + kHeadMax; i += kThreads) {
         float v = 0.0f;
         if (i < kH) v = P.params[P.off_b_enc + i];
@@ -1081,10 +1081,13 @@ k_policy_fused(const __grid_constant__ Params P) {
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) role_mma<T16, PAIR, GAME, HID>(sm, P, tmem);
     } else if (warp == 2) {
+        wait_for_previous_kernel();
         if (lane == 0) role_loads<PAIR, GAME, HID>(sm, P);
     } else if (warp == 3) {
+        wait_for_previous_kernel();
         if (lane == 0) role_stores<PAIR, GAME, HID>(sm, P);
     } else {
+        wait_for_previous_kernel();
         role_worker<T16, PAIR, GAME, HID>(sm, P, tmem, warp, lane, bar0_cta0);
     }
 

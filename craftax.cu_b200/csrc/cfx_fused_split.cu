@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_ctarank();
     const int row0 = P.tile_begin * kTile + (int)blockIdx.x / S * P.tile_rows, quads = P.tile_rows / 32;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    launch_next_kernel();
     if (warp == 0) {   // a lane sets a barrier up
         for (int i = lane; i < NUM_BARS; i += 32) {
             uint32_t arrivals = 1, bytes = 0;

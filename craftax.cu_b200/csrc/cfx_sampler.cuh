@@ -50,23 +50,4 @@ __device__ __forceinline__ int sample_action(const float (&logits)[A], float u, 
     return draw_action<A>(logits, p, m, u, logprob);
 }
 
-// The same with a runtime A, for the stand-alone sampler: the maximum m and p[a] = expf(l[a] - m)
-// are given.
-__device__ __forceinline__ int pick_action(const float* l, const float* p, int A, float m, float u, float* logprob) {
-    float total = 0.0f;
-#pragma unroll 8
-    for (int a = 0; a < A; a++) total += p[a];
-    const float target = u * total;
-    float cum = 0.0f;
-    int action = -1;
-#pragma unroll 8
-    for (int a = 0; a < A; a++) {   // no early exit: the reads stay ahead of the sum
-        cum += p[a];
-        if (action < 0 && target <= cum) action = a;
-    }
-    if (action < 0) action = A - 1;
-    *logprob = l[action] - m - logf(total);
-    return action;
-}
-
 }  // namespace cfx

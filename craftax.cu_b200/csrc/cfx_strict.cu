@@ -44,8 +44,9 @@ __global__ void k_expand(const uint8_t* __restrict__ rec, float* __restrict__ ou
 // are bound by the FMA pipe (128 lanes per clock and SM), and a thread that loads an operand for few FMAs by
 // shared-memory reads instead (a cycle per operand register and warp, broadcast or not).  In a layer a lane
 // owns TM envs x 4 units, all three gates, a warp 4 TM envs x 32 units (lane = 8 groups of units x 4
-// groups of envs), and a block is WM x WU such warps.  Activations travel between the kernels transposed,
-// [H][n], so that both operands of a k step are contiguous in shared memory; two units at a time go
+// groups of envs), and a block is WM x WU such warps.  Activations travel between the kernels in tiles of
+// 32 envs, [n / 32][H][32], and the gate matrices in tiles of 64 (32) units, so that a chunk of k steps is one contiguous
+// piece for the copies and both operands of a k step are contiguous in shared memory; two units at a time go
 // through the packed FMA (`fma.rn.f32x2`, the rounding of fmaf), which leaves issue slots for
 // the operand reads.
 // (The doubled input of a pair is made with register moves: stored doubled it costs 8 more operand
@@ -65,7 +66,7 @@ template <int TM> struct Frag {   // the TM inputs of a lane, each doubled for t
         }
     }
 };
-// TM consecutive floats of a [H][n] row
+// TM consecutive envs of a unit
 template <int TM> __device__ __forceinline__ void load_envs(const float* p, float (&v)[TM]) {
     if constexpr (TM >= 4) {
 #pragma unroll
@@ -101,18 +102,30 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool on, bo
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// `early` of the kernels: start the next kernel at once; the weights may be read before the kernel in front has
+// ended (those of a handle are only ever written by calls that wait for the device)
+constexpr int kLaunchNext = 1, kWeightsReady = 2;
+
+// element (unit k, env e) of the activations
+__host__ __device__ __forceinline__ size_t act_at(size_t e, int k, int H) { return ((e >> 5) * (size_t)H + (size_t)k) * 32 + (e & 31); }
+
 // ---------------------------------------------------------------- encoder
 // h_enc[k][e] = b_enc[k] + sum_f x[e][f] * W_enc[f][k], ascending f.  A lane owns TM envs x G groups of 4
 // units, the groups 32 units apart.  Few warps of such tiles fall to an SM scheduler (one at 4,096 envs,
 // hidden 256), so everything but the sums is taken out of them: four warps of a block fill the stages (record words ->
 // fp32, transposed; W_enc rows by asynchronous copies), four multiply, and named barriers hand the
 // stages over.  4,096 envs, hidden 256: 52 us, against 63 us with every warp doing both, and 78 us
-// with the features kept as bytes and converted by the lanes that multiply.
-constexpr int kEncK = 32, kEncStages = 3;
+// with the features kept as bytes and converted by the lanes that multiply.  A small batch is bound by the latency of these
+// loads: record words are fetched three chunks ahead, W_enc rows S - 2 chunks, and the 51 raw floats of the tail are copied
+// at the start by the warps that multiply (32 envs: 25 us with one chunk ahead, @@ now).
+constexpr int kEncK = 32, kEncAhead = 3;
+constexpr int kMapChunks = (kMap + kEncK - 1) / kEncK, kEncChunks = kMapChunks + (kTail + kEncK - 1) / kEncK;   // 25 of record bytes, 2 of the tail
+static_assert(kEncChunks % kEncAhead == 0, "the chunk loop is unrolled by the words in flight");
 template <int TM, int G> struct Enc {
     static constexpr int BM = 16 * TM, BU = 32 * G, XS = BM + 4;       // envs, units, row stride of x
+    static constexpr int S = TM == 1 ? 6 : (TM == 4 ? 4 : 3);          // stages
     static constexpr int kStage = kEncK * (XS + BU);                   // floats
-    static constexpr int kSmem = kEncStages * kStage * (int)sizeof(float);
+    static constexpr int kSmem = (S * kStage + kTail * XS) * (int)sizeof(float);
 };
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
@@ -120,66 +133,84 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("
 template <int TM, int G>
 __global__ void __launch_bounds__(256, 2)
 k_encoder_fp32(const uint8_t* __restrict__ rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc,
-                  float* __restrict__ h_out, int n, int H, int w_aligned) {
-    constexpr int BM = Enc<TM, G>::BM, BU = Enc<TM, G>::BU, XS = Enc<TM, G>::XS, K = kEncK, kStage = Enc<TM, G>::kStage;
-    constexpr int kChunks = (kObs + K - 1) / K, FULL = 1, EMPTY = FULL + kEncStages;   // barrier ids
-    extern __shared__ __align__(16) float sm[];   // per stage: x [K][XS], w [K][BU]
+               float* __restrict__ h_out, int n, int H, int w_aligned, int early) {
+    using E = Enc<TM, G>;
+    constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = kEncK, S = E::S, D = S - 2;
+    constexpr int FULL = 1, EMPTY = FULL + S, TAIL = 15;   // barrier ids
+    extern __shared__ __align__(16) float sm[];   // per stage: x [K][XS], w [K][BU]; then the tail [kTail][XS]
+    float* tail = sm + S * E::kStage;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e0 = blockIdx.x * BM, u0 = blockIdx.y * BU;
-    wait_for_previous_kernel();
+    if (early & kLaunchNext) launch_next_kernel();
     if (warp >= 4) {
         const int tid = threadIdx.x - 128;
+        // rows of W_enc that chunk c needs, and the first of them
+        auto copy_w = [&](int c) {
+            const int f0 = c < kMapChunks ? c * K : kMap + (c - kMapChunks) * K;
+            const int rows = c < kMapChunks ? min(K, kMap - c * K) : min(K, kObs - f0);
+            float* w = sm + (c % S) * E::kStage + K * XS;
+            for (int i = tid; i < rows * (BU / 4); i += 128) {
+                const int k = i / (BU / 4), col = 4 * (i % (BU / 4));
+                copy16(w + k * BU + col, W_enc + (size_t)(f0 + k) * H + u0 + col, true, w_aligned != 0);
+            }
+        };
+        if (!(early & kWeightsReady)) wait_for_previous_kernel();
+#pragma unroll
+        for (int c = 0; c < D; c++) { copy_w(c); copy_commit(); }
+        wait_for_previous_kernel();
         // a task is one record word (four features of an env): lanes = 16 envs x 2 words
         constexpr int TASKS = BM * (K / 4) / 128;
-        uint32_t raw[TASKS][4];   // one word = four map features, or four raw floats in the tail
         auto slot = [&](int i, int& e, int& w) {
             const int idx = i * 128 + tid;
             e = idx % 16 + 16 * ((idx / 32) % (BM / 16));
             w = (idx % 32) / 16 + 2 * (idx / (2 * BM));
         };
-        auto fetch = [&](int f0) {
+        uint32_t raw[kEncAhead][TASKS];
+        auto fetch = [&](int c, uint32_t (&r)[TASKS]) {
 #pragma unroll
             for (int i = 0; i < TASKS; i++) {
                 int e, w;
                 slot(i, e, w);
-                const uint8_t* r = rec + (size_t)(e0 + e) * kRec;
-                const int f = f0 + 4 * w;
-                const bool on = e0 + e < n;
-                raw[i][0] = on && f < kMap ? *reinterpret_cast<const uint32_t*>(r + f) : 0u;   // (792 is a multiple of 4)
-                raw[i][1] = raw[i][2] = raw[i][3] = 0u;
-                if (on && f >= kMap) {
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if (f + q < kObs) raw[i][q] = *reinterpret_cast<const uint32_t*>(r + kMap + 4 * (f + q - kMap));
-                }
+                const int f = c * K + 4 * w;   // (792 is a multiple of 4)
+                r[i] = f < kMap && e0 + e < n ? *reinterpret_cast<const uint32_t*>(rec + (size_t)(e0 + e) * kRec + f) : 0u;
             }
         };
-        fetch(0);
-        for (int c = 0; c < kChunks; c++) {
-            const int s = c % kEncStages, f0 = c * K;
-            float* x = sm + s * kStage;
-            float* w = x + K * XS;
-            if (c >= kEncStages) bar_sync(EMPTY + s, 256);
-            for (int i = tid; i < K * (BU / 4); i += 128) {
-                const int k = i / (BU / 4), col = 4 * (i % (BU / 4));
-                if (f0 + k < kObs) copy16(w + k * BU + col, W_enc + (size_t)(f0 + k) * H + u0 + col, true, w_aligned != 0);
-            }
-            copy_commit();
 #pragma unroll
-            for (int i = 0; i < TASKS; i++) {
-                int e, wd;
-                slot(i, e, wd);
-                const bool map = f0 + 4 * wd < kMap;
+        for (int c = 0; c < kEncAhead; c++) fetch(c, raw[c]);
+        for (int c0 = 0; c0 < kEncChunks; c0 += kEncAhead) {
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    x[(4 * wd + q) * XS + e] = map ? (float)((raw[i][0] >> (8 * q)) & 0xFFu) : __uint_as_float(raw[i][q]);
+            for (int q = 0; q < kEncAhead; q++) {
+                const int c = c0 + q, s = c % S;
+                if (c + D < kEncChunks) {
+                    if (c + D >= S) bar_sync(EMPTY + (c + D) % S, 256);
+                    copy_w(c + D);
+                }
+                copy_commit();
+                if (c < kMapChunks) {
+                    float* x = sm + s * E::kStage;
+#pragma unroll
+                    for (int i = 0; i < TASKS; i++) {
+                        int e, wd;
+                        slot(i, e, wd);
+#pragma unroll
+                        for (int b = 0; b < 4; b++) x[(4 * wd + b) * XS + e] = (float)((raw[q][i] >> (8 * b)) & 0xFFu);
+                    }
+                    fetch(c + kEncAhead, raw[q]);
+                }
+                copy_wait<D>();
+                bar_arrive(FULL + s, 256);
             }
-            if (c + 1 < kChunks) fetch(f0 + K);
-            copy_wait<0>();
-            bar_arrive(FULL + s, 256);
         }
         return;
     }
+    wait_for_previous_kernel();
+    for (int i = threadIdx.x; i < BM * kTail; i += 128) {
+        const int e = i / kTail, j = i % kTail;
+        const bool on = e0 + e < n;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(tail + j * XS + e)),
+                     "l"(rec + (size_t)(on ? e0 + e : e0) * kRec + kMap + 4 * j), "r"(on ? 4 : 0) : "memory");
+    }
+    copy_commit();
     const int el = warp * 4 * TM + (lane >> 3) * TM, ul = (lane & 7) * 4;
     uint64_t z[G][TM][2];
 #pragma unroll
@@ -188,32 +219,41 @@ k_encoder_fp32(const uint8_t* __restrict__ rec, const float* __restrict__ W_enc,
 #pragma unroll
         for (int e = 0; e < TM; e++) { z[g][e][0] = f2pack(b[0], b[1]); z[g][e][1] = f2pack(b[2], b[3]); }
     }
-    for (int c = 0; c < kChunks; c++) {
-        const int s = c % kEncStages;
-        const float* xp = sm + s * kStage + el;
-        const float* wp = sm + s * kStage + K * XS + ul;
-        bar_sync(FULL + s, 256);
-        auto step = [&](int k) {
-            Frag<TM> x;
-            x.load(xp + k * XS);
+    auto step = [&](const float* xp, const float* wp) {
+        Frag<TM> x;
+        x.load(xp);
 #pragma unroll
-            for (int g = 0; g < G; g++) {
-                const float4 w = *reinterpret_cast<const float4*>(wp + k * BU + 32 * g);
-                const uint64_t w01 = f2pack(w.x, w.y), w23 = f2pack(w.z, w.w);
+        for (int g = 0; g < G; g++) {
+            const float4 w = *reinterpret_cast<const float4*>(wp + 32 * g);
+            const uint64_t w01 = f2pack(w.x, w.y), w23 = f2pack(w.z, w.w);
 #pragma unroll
-                for (int e = 0; e < TM; e++) {
-                    z[g][e][0] = f2fma(x.v[e], w01, z[g][e][0]);
-                    z[g][e][1] = f2fma(x.v[e], w23, z[g][e][1]);
-                }
+            for (int e = 0; e < TM; e++) {
+                z[g][e][0] = f2fma(x.v[e], w01, z[g][e][0]);
+                z[g][e][1] = f2fma(x.v[e], w23, z[g][e][1]);
             }
-        };
-        if (c + 1 < kChunks) {
-#pragma unroll 16
-            for (int k = 0; k < K; k++) step(k);
-        } else {
-            for (int k = 0; k < kObs - c * K; k++) step(k);
         }
-        if (c + kEncStages < kChunks) bar_arrive(EMPTY + s, 256);
+    };
+    for (int c = 0; c < kEncChunks; c++) {
+        const int s = c % S;
+        const float* wp = sm + s * E::kStage + K * XS + ul;
+        if (c == kMapChunks) {
+            copy_wait<0>();
+            bar_sync(TAIL, 128);
+        }
+        const float* xp = (c < kMapChunks ? sm + s * E::kStage : tail + (c - kMapChunks) * K * XS) + el;
+        const int rows = c < kMapChunks ? min(K, kMap - c * K) : min(K, kTail - (c - kMapChunks) * K);
+        bar_sync(FULL + s, 256);
+        if (rows == K) {
+#pragma unroll 16
+            for (int k = 0; k < K; k++) step(xp + k * XS, wp + k * BU);
+        } else {
+            int k = 0;
+            for (; k + 8 <= rows; k += 8)
+#pragma unroll
+                for (int i = 0; i < 8; i++) step(xp + (k + i) * XS, wp + (k + i) * BU);
+            for (; k < rows; k++) step(xp + k * XS, wp + k * BU);
+        }
+        if (c + S < kEncChunks) bar_arrive(EMPTY + s, 256);
     }
     if (e0 + el < n) {
 #pragma unroll
@@ -226,7 +266,7 @@ k_encoder_fp32(const uint8_t* __restrict__ rec, const float* __restrict__ W_enc,
                 f2unpack(z[g][e][u >> 1], lo, hi);
                 h[e] = (u & 1) ? hi : lo;
             }
-            store_envs<TM>(h_out + (size_t)(u0 + ul + 32 * g + u) * n + e0 + el, h);
+            store_envs<TM>(h_out + act_at(e0 + el, u0 + ul + 32 * g + u, H), h);
         }
     }
 }
@@ -292,7 +332,7 @@ __global__ void k_classic_encoder_fp32(const uint8_t* __restrict__ rec, const fl
     hv = fmaf(light, Wk[(size_t)f * H], hv);
     f++;
     hv = fmaf(sleeping ? 1.0f : 0.0f, Wk[(size_t)f * H], hv);
-    h_out[(size_t)k * n + e] = hv;   // [H][n]; the scattered words meet in L2 (a record gathers 100 rows of W_enc)
+    h_out[act_at(e, k, H)] = hv;   // the scattered words meet in L2 (a record gathers 100 rows of W_enc)
 }
 
 // r_done int8 flags of the classic rollout (main_classic.cu:436-443) -> the float flags the
@@ -304,63 +344,81 @@ __global__ void k_done_to_terminals(const int8_t* __restrict__ done, float* __re
 
 // ---------------------------------------------------------------- MinGRU layer
 // One layer: gate dots (ascending j, fmaf) + cell (k_mingru_epi_fwd, craftax_full.cu:9350-9395).
-// Wt is the layer's gate matrix transposed to [H][3H]; x_in and h_out are [H][n].  K chunks of 32,
-// two buffers (chunks of 16 with three: 155 against 152 us a forward at 4,096 envs, 970 against 944 us at 8,192 envs with
-// hidden 512, depth 3); the k loop has to be unrolled well (by 4: 170 us).  Bound by the FMA pipe: 66 % of its peak at
-// hidden 512; one thread per unit with 16 envs, before, 20 %.
+// Wt is the layer's gate matrix as k_transpose_gates lays it out, x_in and h_out activations.  K chunks of 32; ST buffers:
+// two where several blocks share an SM, more for small batches, which wait for the loads (chunks of 16 with three: 155 against
+// 152 us a forward at 4,096 envs, 970 against 944 us at 8,192 envs with hidden 512, depth 3); the k loop has to be unrolled
+// well (by 4: 170 us).  Bound by the FMA pipe: 66 % of its peak at hidden 512; one thread per unit with 16 envs, before, 20 %.
 __device__ __forceinline__ float sigmoid_ref(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float mingru_g_ref(float x) { return x >= 0.0f ? x + 0.5f : sigmoid_ref(x); }
 
-constexpr int kGruK = 32, kGruStages = 2;
+constexpr int kGruK = 32;
 template <int TM, int WM, int WU> constexpr int gru_stage_floats() { return kGruK * (4 * TM * WM + 3 * 32 * WU); }
 
-template <int TM, int WM, int WU>
+template <int TM, int WM, int WU, int ST>
 __global__ void __launch_bounds__(32 * WM * WU, 3)
 k_mingru_fp32(const float* __restrict__ x_in, const float* __restrict__ Wt, float* __restrict__ state,
               const float* __restrict__ prev_terminals, float* __restrict__ h_out, float* __restrict__ r_state,
-              int r_bf16, int n, int H, int s_aligned) {
-    constexpr int T = 32 * WM * WU, BM = 4 * TM * WM, BU = 32 * WU;
-    extern __shared__ __align__(16) float sm[];   // per stage: x [kGruK][BM][2], w [kGruK][3][BU]
+              int r_bf16, int n, int H, int s_aligned, int early) {
+    constexpr int T = 32 * WM * WU, BM = 4 * TM * WM, BU = 32 * WU, kStage = gru_stage_floats<TM, WM, WU>();
+    constexpr int EB = BM < 32 ? BM : 32;         // envs of an activation tile that a block takes
+    extern __shared__ __align__(16) float sm[];   // per stage: x [BM / EB][kGruK][EB], w [kGruK][3][BU]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int e0 = blockIdx.x * BM, u0 = blockIdx.y * BU;
     const int el = (warp % WM) * 4 * TM + (lane >> 3) * TM, ul = (warp / WM) * 32 + (lane & 7) * 4;
     const bool live = e0 + el < n;
-    wait_for_previous_kernel();
-
-    auto copy_chunk = [&](int c) {
-        float* x = sm + (c % kGruStages) * gru_stage_floats<TM, WM, WU>();
-        float* w = x + kGruK * BM;
-        for (int i = tid; i < kGruK * (BM / 4); i += T) {
-            const int k = i / (BM / 4), e = 4 * (i % (BM / 4));
-            copy16(x + k * BM + e, x_in + (size_t)(c * kGruK + k) * n + e0 + e, e0 + e < n, true);
-        }
-        for (int i = tid; i < kGruK * 3 * (BU / 4); i += T) {
-            const int k = i / (3 * (BU / 4)), r = i % (3 * (BU / 4)), g = r / (BU / 4), u = 4 * (r % (BU / 4));
-            copy16(w + (k * 3 + g) * BU + u, Wt + (size_t)(c * kGruK + k) * 3 * H + g * H + u0 + u, true, true);
+    const float* wsrc = Wt + (size_t)u0 * 3 * H;
+    auto copy_w = [&](int c) {
+        float* w = sm + (c % ST) * kStage + kGruK * BM;
+        const float* src = wsrc + (size_t)c * kGruK * 3 * BU;
+#pragma unroll 4
+        for (int i = 4 * tid; i < kGruK * 3 * BU; i += 4 * T) copy16(w + i, src + i, true, true);
+    };
+    auto copy_x = [&](int c) {
+        float* x = sm + (c % ST) * kStage;
+#pragma unroll
+        for (int t = 0; t < BM / EB; t++) {
+            const bool on = e0 + t * EB < n;
+            const float* src = x_in + act_at(on ? e0 + t * EB : e0, c * kGruK, H);
+            for (int i = tid; i < kGruK * (EB / 4); i += T)
+                copy16(x + t * kGruK * EB + 4 * i, src + (i / (EB / 4)) * 32 + 4 * (i % (EB / 4)), on, true);
         }
     };
+    if (early & kLaunchNext) launch_next_kernel();
     const int chunks = H / kGruK;
+    if (!(early & kWeightsReady)) wait_for_previous_kernel();
 #pragma unroll
-    for (int c = 0; c < kGruStages - 1; c++) {
-        if (c < chunks) copy_chunk(c);
+    for (int c = 0; c < ST - 1; c++)
+        if (c < chunks) copy_w(c);
+    wait_for_previous_kernel();
+#pragma unroll
+    for (int c = 0; c < ST - 1; c++) {
+        if (c < chunks) copy_x(c);
         copy_commit();
     }
+    if (live)   // this lane's states, on their way to L2 while the sums run
+#pragma unroll
+        for (int e = 0; e < TM; e++)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(state + (size_t)(e0 + el + e) * H + u0 + ul));
     uint64_t z[3][TM][2];
 #pragma unroll
     for (int g = 0; g < 3; g++)
 #pragma unroll
         for (int e = 0; e < TM; e++) z[g][e][0] = z[g][e][1] = 0ull;
+    const float* xl = sm + (el / EB) * kGruK * EB + el % EB;
     for (int c = 0; c < chunks; c++) {
-        copy_wait<kGruStages - 2>();
+        copy_wait<ST - 2>();
         __syncthreads();   // chunk c is complete, and everybody is done with chunk c - 1
-        if (c + kGruStages - 1 < chunks) copy_chunk(c + kGruStages - 1);
+        if (c + ST - 1 < chunks) {
+            copy_w(c + ST - 1);
+            copy_x(c + ST - 1);
+        }
         copy_commit();
-        const float* x = sm + (c % kGruStages) * gru_stage_floats<TM, WM, WU>() + el;
-        const float* w = sm + (c % kGruStages) * gru_stage_floats<TM, WM, WU>() + kGruK * BM + ul;
+        const float* x = xl + (c % ST) * kStage;
+        const float* w = sm + (c % ST) * kStage + kGruK * BM + ul;
 #pragma unroll 16
         for (int k = 0; k < kGruK; k++) {
             Frag<TM> xv;
-            xv.load(x + k * BM);
+            xv.load(x + k * EB);
 #pragma unroll
             for (int g = 0; g < 3; g++) {
                 const float4 wv = *reinterpret_cast<const float4*>(w + (k * 3 + g) * BU);
@@ -404,7 +462,7 @@ k_mingru_fp32(const float* __restrict__ x_in, const float* __restrict__ Wt, floa
 #pragma unroll
     for (int u = 0; u < 4; u++) {
         float x[TM], h[TM];
-        load_envs<TM>(x_in + (size_t)(u0 + ul + u) * n + e0 + el, x);
+        load_envs<TM>(x_in + act_at(e0 + el, u0 + ul + u, H), x);
 #pragma unroll
         for (int e = 0; e < TM; e++) {
             float lo, hi;
@@ -420,7 +478,7 @@ k_mingru_fp32(const float* __restrict__ x_in, const float* __restrict__ Wt, floa
             h[e] = p * out + (1.0f - p) * x[e];
             st[e][u] = out;
         }
-        store_envs<TM>(h_out + (size_t)(u0 + ul + u) * n + e0 + el, h);
+        store_envs<TM>(h_out + act_at(e0 + el, u0 + ul + u, H), h);
     }
 #pragma unroll
     for (int e = 0; e < TM; e++) {
@@ -449,19 +507,21 @@ constexpr size_t head_smem(int H, int A) {
 __global__ void __launch_bounds__(384) k_heads_fp32(const float* __restrict__ h, const float* __restrict__ W_a,
                                                     const float* __restrict__ b_a, const float* __restrict__ W_v,
                                                     const float* __restrict__ b_v, float* __restrict__ logits_av,
-                                                    int n, int H, int A) {
+                                                    int n, int H, int A, int early) {
     extern __shared__ __align__(16) float hs[];   // h [H][32], then W [rows][H + 4]
     float* wsh = hs + kHeadEnvs * H;
     const int tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, lane = tid & 31;
     const int e0 = blockIdx.x * kHeadEnvs, WS = H + 4;
-    wait_for_previous_kernel();
-    for (int i = tid; i < H * (kHeadEnvs / 4); i += T)
-        copy16(hs + 4 * i, h + (size_t)(i / (kHeadEnvs / 4)) * n + e0 + 4 * (i % (kHeadEnvs / 4)), true, true);
+    if (early & kLaunchNext) launch_next_kernel();
+    if (!(early & kWeightsReady)) wait_for_previous_kernel();
     for (int a = warp; a < A + 1; a += T / 32) {
         const float* w = a < A ? W_a + (size_t)a * H : W_v;
         const bool al = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
         for (int j = 4 * lane; j < H; j += 128) copy16(wsh + a * WS + j, w + j, true, al);
     }
+    wait_for_previous_kernel();
+    const float* hsrc = h + (size_t)e0 * H;   // 32 envs are one tile
+    for (int i = 4 * tid; i < H * kHeadEnvs; i += 4 * T) copy16(hs + i, hsrc + i, true, true);
     copy_commit();
     const int a0 = (warp >> 1) * kHeadRows + (lane >> 3) * kHeadLaneRows, el = 16 * (warp & 1) + 2 * (lane & 7);
     float z[kHeadLaneRows][2];
@@ -502,52 +562,74 @@ __global__ void __launch_bounds__(384) k_heads_fp32(const float* __restrict__ h,
 // k_value_sample (craftax_full.cu:9714-9741); logits already carry their biases.  A block of 128
 // threads takes 32 envs: the rows come in coalesced, four threads of an env take its maximum and its
 // exponentials (both independent of order), one thread adds them up in the reference's order.
-// `ctr` (optional): device step counter {offset, blocks finished}; with `bump` the last block raises it.
+// The running sums are kept, so that the search for the first one that reaches the target is parallel too.
+// `ctr` (optional): device step counter {offset, blocks finished}; with `bump` the last block that has read it raises it.
 constexpr int kSampleEnvs = 32, kSampleThreads = 128;
 
 __global__ void __launch_bounds__(kSampleThreads)
 k_sample(const float* __restrict__ logits, int ld, int A, const float* __restrict__ uniforms, uint64_t seed,
          uint64_t env_offset, unsigned long long* ctr, int bump, int n, float* __restrict__ env_actions,
-         int32_t* __restrict__ actions, float* __restrict__ logprobs, float* __restrict__ values) {
-    __shared__ float l[kSampleEnvs][kMaxActions + 2], p[kSampleEnvs][kMaxActions + 2];   // odd row length
+         int32_t* __restrict__ actions, float* __restrict__ logprobs, float* __restrict__ values, int early) {
+    __shared__ float l[kSampleEnvs][kMaxActions + 2], p[kSampleEnvs + 1][kMaxActions + 2];   // odd row length
     const int tid = threadIdx.x, e0 = blockIdx.x * kSampleEnvs;
     const int cols = values != nullptr ? A + 1 : A;
+    if (early & kLaunchNext) launch_next_kernel();
     wait_for_previous_kernel();
     const int envs = min(kSampleEnvs, n - e0);
     for (int i = tid; i < envs * cols; i += kSampleThreads)
         l[i / cols][i % cols] = logits[(size_t)(e0 + i / cols) * ld + i % cols];
     const int e = tid >> 2, part = tid & 3;   // env and quarter of its actions
+    const unsigned mates = 0xFu << (tid & 28);
     float u = 0.0f;
     if (part == 0 && e < envs)
         u = uniforms != nullptr ? uniforms[e0 + e]
                                 : philox_uniform(seed, env_offset + (uint64_t)(e0 + e), ctr ? *ctr : 0ULL);
-    __syncthreads();
-    float m = -INFINITY;
-    if (e < envs)
-        for (int a = part; a < A; a += 4) m = fmaxf(m, l[e][a]);
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    if (e < envs)
-        for (int a = part; a < A; a += 4) p[e][a] = expf(l[e][a] - m);
-    __syncwarp();
-    if (part == 0 && e < envs) {
-        float lp;
-        const int a = pick_action(l[e], p[e], A, m, u, &lp);
-        const int env = e0 + e;
-        if (env_actions) env_actions[env] = (float)a;
-        if (actions) actions[env] = a;
-        if (logprobs) logprobs[env] = lp;
-        if (values) values[env] = l[e][A];
+    __syncthreads();   // the rows are here, and this block has read the counter
+    if (bump && tid == kSampleThreads - 1) {
+        if (gridDim.x > 1) __threadfence();
+        if (gridDim.x == 1 || atomicAdd(ctr + 1, 1ULL) == gridDim.x - 1) {
+            ctr[0] += 1ULL;
+            ctr[1] = 0ULL;
+        }
     }
-    if (bump) {
-        __syncthreads();   // this block has read the counter
-        if (tid == 0) {
-            __threadfence();
-            if (atomicAdd(ctr + 1, 1ULL) == gridDim.x - 1) {
-                ctr[0] += 1ULL;
-                ctr[1] = 0ULL;
+    if (e >= envs) return;   // (all four threads of an env)
+    float m = -INFINITY;
+#pragma unroll 4
+    for (int a = part; a < A; a += 4) m = fmaxf(m, l[e][a]);
+    m = fmaxf(m, __shfl_xor_sync(mates, m, 1));
+    m = fmaxf(m, __shfl_xor_sync(mates, m, 2));
+#pragma unroll 4
+    for (int a = part; a < A; a += 4) p[e][a] = expf(l[e][a] - m);
+    __syncwarp(mates);
+    float total = 0.0f;
+    if (part == 0) {
+        for (int a = 0; a < A; a += 8) {   // (loads of a batch before its stores)
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = p[e][a + i];   // beyond A: room in the row's neighbours, not used
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (a + i >= A) break;
+                total += v[i];
+                p[e][a + i] = total;
             }
         }
+    }
+    __syncwarp(mates);
+    total = __shfl_sync(mates, total, tid & 28);
+    u = __shfl_sync(mates, u, tid & 28);
+    const float target = u * total;
+    int action = A - 1;
+    for (int a = part; a < A; a += 4)
+        if (target <= p[e][a]) { action = a; break; }
+    action = min(action, __shfl_xor_sync(mates, action, 1));
+    action = min(action, __shfl_xor_sync(mates, action, 2));
+    if (part == 0) {
+        const int env = e0 + e;
+        if (env_actions) env_actions[env] = (float)action;
+        if (actions) actions[env] = action;
+        if (logprobs) logprobs[env] = l[e][action] - m - logf(total);
+        if (values) values[env] = l[e][A];
     }
 }
 
@@ -564,13 +646,15 @@ __global__ void k_fetch(const uint4* __restrict__ src, uint4* __restrict__ dst, 
 
 __global__ void k_bump(unsigned long long* ctr) { *ctr += 1ULL; }
 
-// Gate matrices transposed for the strict layer kernel: Wt[l][j][r] = W[l][r][j].
+// Gate matrices for the fp32 layer kernel: Wt[l][unit tile][j][gate][unit of the tile] = W[l][gate H + unit][j], tiles of 64
+// units, or of 32 where the hidden size is an odd multiple of it.
 __global__ void k_transpose_gates(const float* __restrict__ W, float* __restrict__ Wt, int H, int L) {
     size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t per = (size_t)3 * H * H;
     if (idx >= per * L) return;
-    size_t l = idx / per, r = (idx % per) / H, j = idx % H;
-    Wt[l * per + j * 3 * H + r] = W[idx];
+    const size_t l = idx / per, r = (idx % per) / H, j = idx % H;
+    const int U = H % 64 == 0 ? 64 : 32, g = (int)(r / H), u = (int)(r % H);
+    Wt[l * per + (size_t)(u / U) * 3 * H * U + (j * 3 + g) * U + u % U] = W[idx];
 }
 
 // Reference initialiser: U(+-bound) from Philox(seed, subsequence, index)
@@ -606,9 +690,9 @@ int launch_done_to_terminals(const int8_t* done, float* out, int n, cudaStream_t
 int launch_sample(const float* logits, int ld, int A, const float* u, uint64_t seed,
                   uint64_t env_offset, unsigned long long* step_ctr, int bump, int n,
                   float* env_actions, int32_t* actions, float* logprobs, float* values,
-                  cudaStream_t st) {
+                  cudaStream_t st, int early) {
     return launch_chained(k_sample, dim3((n + kSampleEnvs - 1) / kSampleEnvs), kSampleThreads, 0, st, logits, ld, A, u,
-                          seed, env_offset, step_ctr, bump, n, env_actions, actions, logprobs, values);
+                          seed, env_offset, step_ctr, bump, n, env_actions, actions, logprobs, values, early);
 }
 
 int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, float* u, cudaStream_t st) {
@@ -650,75 +734,88 @@ static int strict_tile(long long q) { return q >= 1024 ? 8 : (q >= 96 ? 4 : 1); 
 // at hidden 256, q = 512: 102, 97 and 113 us a forward with the last three; 1,024 envs: 73, 80 and 94).
 static int strict_encoder_tile(long long q) { return q >= 640 ? 82 : (q >= 400 ? 42 : (q >= 96 ? 41 : 11)); }
 
-template <int TM, int G>
-static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, cudaStream_t st) {
-    using E = Enc<TM, G>;
-    if (E::kSmem > 48 * 1024)
-        CFX_CUDA(cudaFuncSetAttribute(k_encoder_fp32<TM, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, E::kSmem));
-    return launch_chained(k_encoder_fp32<TM, G>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
-                          a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], a.n, a.H,
-                          ((uintptr_t)(a.params + o.w_enc) & 15) == 0);
+// A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per device
+template <auto kernel>
+static int allow_smem(int smem) {
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> done[kMaxDevices];   // the largest size allowed so far
+    int dev = 0;
+    CFX_CUDA(cudaGetDevice(&dev));
+    if (dev < kMaxDevices && done[dev].load(std::memory_order_relaxed) >= smem) return CFX_OK;
+    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (dev < kMaxDevices) done[dev].store(smem, std::memory_order_relaxed);
+    return CFX_OK;
 }
 
-template <int TM, int WM, int WU>
-static int strict_layers(const StrictArgs& a, const ArenaLayout& o, cudaStream_t st, int* cnt) {
+template <int TM, int G>
+static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, int early, cudaStream_t st) {
+    using E = Enc<TM, G>;
+    int rc = allow_smem<k_encoder_fp32<TM, G>>(E::kSmem);
+    if (rc) return rc;
+    return launch_chained(k_encoder_fp32<TM, G>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
+                          a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], a.n, a.H,
+                          ((uintptr_t)(a.params + o.w_enc) & 15) == 0, early);
+}
+
+template <int TM, int WM, int WU, int ST>
+static int strict_layers(const StrictArgs& a, int early, cudaStream_t st) {
     const int H = a.H, n = a.n;
     constexpr int BM = 4 * TM * WM, BU = 32 * WU, T = 32 * WM * WU;
-    constexpr int smem = kGruStages * gru_stage_floats<TM, WM, WU>() * (int)sizeof(float);
-    if (smem > 48 * 1024)
-        CFX_CUDA(cudaFuncSetAttribute(k_mingru_fp32<TM, WM, WU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    constexpr int smem = ST * gru_stage_floats<TM, WM, WU>() * (int)sizeof(float);
+    int rc = allow_smem<k_mingru_fp32<TM, WM, WU, ST>>(smem);
+    if (rc) return rc;
     const dim3 grid((n + BM - 1) / BM, H / BU);
-    int rc;
     const int s_aligned = ((uintptr_t)a.state & 15) == 0;
     for (int l = 0; l < a.L; l++) {
         float* r = a.r_state ? reinterpret_cast<float*>(reinterpret_cast<char*>(a.r_state) +
                                                         (size_t)l * n * H * (a.r_state_bf16 ? 2 : 4))
                              : nullptr;
-        rc = launch_chained(k_mingru_fp32<TM, WM, WU>, grid, T, smem, st, a.scratch_h[l & 1],
+        rc = launch_chained(k_mingru_fp32<TM, WM, WU, ST>, grid, T, smem, st, a.scratch_h[l & 1],
                             a.gates_t + (size_t)l * 3 * H * H, a.state + (size_t)l * n * H, a.prev_terminals,
-                            a.scratch_h[(l + 1) & 1], r, a.r_state_bf16, n, H, s_aligned);
+                            a.scratch_h[(l + 1) & 1], r, a.r_state_bf16, n, H, s_aligned, early);
         if (rc) return rc;
     }
-    *cnt += a.L;
     return CFX_OK;
 }
 
-// Full strict forward.  scratch_h: two [H][n] fp32 buffers; logits_av [n][A+1].
+// Full strict forward.  scratch_h: two buffers of n H activations; logits_av [n][A+1].
 int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     const int H = a.H, L = a.L, A = a.A, n = a.n;
     const ArenaLayout o = ArenaLayout::make(H, L, A, a.game == CFX_GAME_CLASSIC ? kClassicObs : kObs);
-    int cnt = 0, rc;
+    int rc;
     const long long q = (long long)n * H / 1024;
+    const int tm = strict_tile(q), te = strict_encoder_tile(q);
+    // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own
+    // (512 envs, 64 blocks a layer: 88 us with it, 72 without)
+    const long long blocks = (te == 11 ? 2 * q : q / 2) + L * (tm == 1 ? 2 * q : q / 2) + n / 16;
+    const int early = (a.game == CFX_GAME_FULL && blocks <= 148 ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
     if (a.game == CFX_GAME_CLASSIC) {
         rc = launch_chained(k_classic_encoder_fp32, dim3(n), H, 0, st, a.records, a.params + o.w_enc, a.params + o.b_enc,
                             a.scratch_h[0], n, H);
     } else {
-        const int te = strict_encoder_tile(q);
-        if (te == 11) rc = strict_encoder<1, 1>(a, o, st);
-        else if (te == 41 || H % 64 != 0) rc = strict_encoder<4, 1>(a, o, st);
-        else rc = te == 42 ? strict_encoder<4, 2>(a, o, st) : strict_encoder<8, 2>(a, o, st);
+        if (te == 11) rc = strict_encoder<1, 1>(a, o, early, st);
+        else if (te == 41 || H % 64 != 0) rc = strict_encoder<4, 1>(a, o, early, st);
+        else rc = te == 42 ? strict_encoder<4, 2>(a, o, early, st) : strict_encoder<8, 2>(a, o, early, st);
     }
     if (rc) return rc;
-    cnt++;
     // a hidden size that is an odd multiple of 32 has the warps of a block side by side along the envs
-    const int tm = strict_tile(q);
     if (H % 64 == 0)
-        rc = tm == 8 ? strict_layers<8, 2, 2>(a, o, st, &cnt) : tm == 4 ? strict_layers<4, 2, 2>(a, o, st, &cnt)
-                                                              : strict_layers<1, 2, 2>(a, o, st, &cnt);
+        rc = tm == 8 ? strict_layers<8, 2, 2, 2>(a, early, st) : tm == 1 ? strict_layers<1, 2, 2, 4>(a, early, st)
+             : q <= 592 ? strict_layers<4, 2, 2, 3>(a, early, st) : strict_layers<4, 2, 2, 2>(a, early, st);
     else
-        rc = tm == 8 ? strict_layers<8, 4, 1>(a, o, st, &cnt) : tm == 4 ? strict_layers<4, 4, 1>(a, o, st, &cnt)
-                                                              : strict_layers<1, 4, 1>(a, o, st, &cnt);
+        rc = tm == 8 ? strict_layers<8, 4, 1, 2>(a, early, st) : tm == 4 ? strict_layers<4, 4, 1, 2>(a, early, st)
+                                                                 : strict_layers<1, 4, 1, 4>(a, early, st);
     if (rc) return rc;
     const size_t hsmem = head_smem(H, A);
-    if (hsmem > 48 * 1024)
-        CFX_CUDA(cudaFuncSetAttribute(k_heads_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+    if ((rc = allow_smem<k_heads_fp32>((int)hsmem))) return rc;
     rc = launch_chained(k_heads_fp32, dim3(n / kHeadEnvs), head_threads(A), hsmem, st, a.scratch_h[L & 1],
-                        a.params + o.w_a, a.params + o.b_a, a.params + o.w_v, a.params + o.b_v, a.logits_av, n, H, A);
+                        a.params + o.w_a, a.params + o.b_a, a.params + o.w_v, a.params + o.b_v, a.logits_av, n, H, A, early);
     if (rc) return rc;
     rc = launch_sample(a.logits_av, A + 1, A, a.uniforms, a.seed, a.env_offset, a.step_ctr, a.bump_step, n,
-                       a.env_actions, a.actions, a.logprobs, a.values, st);
+                       a.env_actions, a.actions, a.logprobs, a.values, st, early);
     if (rc) return rc;
-    if (launches) *launches = cnt + 2;
+    if (launches) *launches = 1 + L + 2;
     return CFX_OK;
 }
 

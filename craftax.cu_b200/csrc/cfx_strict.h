@@ -9,12 +9,12 @@ struct StrictArgs {
     int n, H, L, A;
     int game = 0;           // CFX_GAME_FULL or CFX_GAME_CLASSIC (148-byte records, gather encoder)
     const float* params;    // fp32 arena
-    const float* gates_t;   // [L][H][3H] transposed gate matrices
+    const float* gates_t;   // [L] gate matrices as launch_transpose_gates writes them
     const uint8_t* records;
     const float* prev_terminals;
     const float* uniforms;
     float* state;           // [L][n][H]
-    float* scratch_h[2];    // [H][n] each, 16-byte aligned
+    float* scratch_h[2];    // n H activations each, 16-byte aligned
     float* logits_av;       // [n][A+1]
     float* r_state;
     int r_state_bf16 = 0;   // r_state holds bf16 instead of fp32
@@ -25,6 +25,7 @@ struct StrictArgs {
     uint64_t seed, env_offset;
     unsigned long long* step_ctr;   // {Philox offset, blocks finished (bump_step)}
     int bump_step = 0;      // raise the offset after the forward
+    int weights_ready = 0;  // nothing queued on the stream writes params or gates_t
 };
 
 int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches);
@@ -34,7 +35,7 @@ int launch_done_to_terminals(const int8_t* done, float* out, int n, cudaStream_t
 int launch_sample(const float* logits, int ld, int A, const float* u, uint64_t seed,
                   uint64_t env_offset, unsigned long long* step_ctr, int bump, int n,
                   float* env_actions, int32_t* actions, float* logprobs, float* values,
-                  cudaStream_t st);
+                  cudaStream_t st, int early = 0);
 int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, float* u, cudaStream_t st);
 // copies `bytes` (a multiple of 16) from page-locked host memory, both 16-byte aligned
 int launch_fetch(const void* host, void* dst, size_t bytes, cudaStream_t st);
