@@ -159,10 +159,11 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
 }
 
 // ------------------------------------------------------------------ MMA
-// One thread issues every MMA.  There is one tile, so every ring position is a compile-time constant and every
-// descriptor one addition away from two bases: an MMA whose descriptor is computed takes ~150 cycles to issue, and
-// 54 of them were two thirds of the encoder.  The barriers of the next step are probed before the
-// current step's MMAs (CFX_PROBE), so that a probe's round trip runs under their issue.
+// The whole warp walks through the steps and an elected lane issues: with the code uniform over the warp the compiler keeps
+// descriptors in uniform registers (one lane alone in a branch: 2 to 6 % slower a step).  There is one tile, so every ring
+// position is a compile-time constant and every descriptor one addition away from two bases: an MMA whose descriptor is
+// computed takes ~150 cycles to issue, and 54 of them were two thirds of the encoder.  The barriers of the next step are
+// probed before the current step's MMAs (CFX_PROBE), so that a probe's round trip runs under their issue.
 #define CFX_SPROBE(name, barid, parity) CFX_PROBE(name, sm.bar(barid), (uint32_t)(parity))
 #define CFX_SWAIT_PROBED(name, barid, parity)                                                               \
     {                                                                                                       \
@@ -197,13 +198,16 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + as, (kc / kASlots) & 1);
         if (kc + 1 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + (kc + 1) % kASlots, ((kc + 1) / kASlots) & 1);
         tc_fence_after_sync();
+        __syncwarp();
         const uint64_t bd = wdesc + (uint64_t)(((slot * kWSlot + blk % C::kEncPerItem * C::kEncTile) >> 4) + first);
         const uint32_t a = tmem + kColAexp + as * 32;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < ks; k++) mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
-        if (kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
-        if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
-        if (ends && ((blk + 1) % C::kEncPerItem == 0 || kc == kChunks - 1)) mma_commit(sm.bar(W_EMPTY + slot));
+            for (int k = 0; k < ks; k++) mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+            if (kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
+            if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
+            if (ends && ((blk + 1) % C::kEncPerItem == 0 || kc == kChunks - 1)) mma_commit(sm.bar(W_EMPTY + slot));
+        }
     }
     // ---- layers and heads (a loop over the layers: straight-line code for all of them would be fetched cold)
     uint32_t wpar = 0;   // parity bit of every ring slot
@@ -231,13 +235,16 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                 wpar ^= 1u << slot;
                 CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
                 tc_fence_after_sync();
+                __syncwarp();
                 const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 4; ks++)
-                    mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
-                if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL + j));
-                if (j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
-                mma_commit(sm.bar(W_EMPTY + slot));
+                    for (int ks = 0; ks < 4; ks++)
+                        mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
+                    if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL + j));
+                    if (j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
+                    mma_commit(sm.bar(W_EMPTY + slot));
+                }
             }
         }
     }
@@ -253,12 +260,15 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
             CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
         }
         tc_fence_after_sync();
+        __syncwarp();
         const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ks++)
-            mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+            for (int ks = 0; ks < 4; ks++)
+                mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+            if (kb == C::kKB - 1) mma_commit(sm.bar(H_FULL));
+        }
     }
-    mma_commit(sm.bar(H_FULL));
 }
 
 // ------------------------------------------------------------------ state
@@ -565,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     if (warp == 0) {
         if (lane == 0) role_weights<GAME, HID, S>(sm, P, rank);
     } else if (warp == 1) {
-        if (lane == 0) role_mma<T16, GAME, HID, S>(sm, P, tmem, rank);
+        role_mma<T16, GAME, HID, S>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
     } else if (warp == 2) {
         // the tile's records, 32 rows a copy
         wait_for_previous_kernel();
