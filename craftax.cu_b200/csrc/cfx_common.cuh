@@ -2,6 +2,7 @@
 // record / arena layout, the handle, error plumbing.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -60,7 +61,8 @@ struct DeviceGuard {
     bool ok = true;
     explicit DeviceGuard(int dev) {
         if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
-        if (prev != dev) ok = (cudaSetDevice(dev) == cudaSuccess);
+        if (prev == dev) prev = -1;   // nothing to put back
+        else ok = (cudaSetDevice(dev) == cudaSuccess);
     }
     ~DeviceGuard() {
         if (prev >= 0) cudaSetDevice(prev);
@@ -81,7 +83,8 @@ struct DeviceGuard {
 // under the kernel in front of it in the stream, and it waits here until the results of that kernel are in
 // memory.  Nothing that another kernel may have written is read before.  Only kernels of few blocks
 // let the next one start early (launch_next_kernel): the blocks of a larger one would fill the SMs that this
-// kernel's last blocks leave free and pile up there (fp32 forward, 4,096 envs: 227 us against 178).
+// kernel's last blocks leave free and pile up there (fp32 forward, 4,096 envs: 227 us against 178; classic record
+// write, 20,000 envs: 9.1 us against 4.2).
 #ifdef __CUDACC__
 __device__ __forceinline__ void launch_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -99,6 +102,20 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     CFX_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return CFX_OK;
+}
+
+// A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per device
+template <auto kernel>
+int allow_smem(int smem) {
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> done[kMaxDevices];   // the largest size allowed so far
+    int dev = 0;
+    CFX_CUDA(cudaGetDevice(&dev));
+    if (dev < kMaxDevices && done[dev].load(std::memory_order_relaxed) >= smem) return CFX_OK;
+    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (dev < kMaxDevices) done[dev].store(smem, std::memory_order_relaxed);
     return CFX_OK;
 }
 #endif

@@ -659,7 +659,7 @@ extern "C" int cfx_record_obs(int device, const cfx_env_view* view, uint8_t* rec
     P.n = n;
     P.skip = skip;
     const unsigned blocks = (unsigned)((n + record::kBlockEnvs - 1) / record::kBlockEnvs);
-    CFX_CUDA(cudaFuncSetAttribute(record::k_record_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(record::Shared)));
+    if ((rc = allow_smem<record::k_record_rows>((int)sizeof(record::Shared)))) return rc;
     return launch_chained(record::k_record_rows, dim3(blocks), record::kBlockThreads, sizeof(record::Shared), (cudaStream_t)stream, P);
 }
 

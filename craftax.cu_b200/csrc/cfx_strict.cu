@@ -734,20 +734,6 @@ static int strict_tile(long long q) { return q >= 1024 ? 8 : (q >= 96 ? 4 : 1); 
 // at hidden 256, q = 512: 102, 97 and 113 us a forward with the last three; 1,024 envs: 73, 80 and 94).
 static int strict_encoder_tile(long long q) { return q >= 640 ? 82 : (q >= 400 ? 42 : (q >= 96 ? 41 : 11)); }
 
-// A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per device
-template <auto kernel>
-static int allow_smem(int smem) {
-    constexpr int kMaxDevices = 64;
-    static std::atomic<int> done[kMaxDevices];   // the largest size allowed so far
-    int dev = 0;
-    CFX_CUDA(cudaGetDevice(&dev));
-    if (dev < kMaxDevices && done[dev].load(std::memory_order_relaxed) >= smem) return CFX_OK;
-    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    if (dev < kMaxDevices) done[dev].store(smem, std::memory_order_relaxed);
-    return CFX_OK;
-}
-
 template <int TM, int G>
 static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, int early, cudaStream_t st) {
     using E = Enc<TM, G>;
