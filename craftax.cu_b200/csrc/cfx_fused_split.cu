@@ -20,6 +20,10 @@
 //   heads     in every CTA, over all rows; the quadrants of rows are sampled in different CTAs
 // The cluster works on one tile and exits, so every barrier but those of the rings is used once or once a
 // layer.  The products of a row are accumulated in the order of cfx_fused.cu: same bits.
+// Tiles of 32 rows (ONE), the smallest batches: a quadrant of TMEM lanes belongs to one SM scheduler, so one
+// quadrant of rows would leave three schedulers idle.  The operand chunks go to shared memory instead, one of the sixteen
+// warps a chunk; and the layers' A operand is tensor memory again, where every quadrant gets a copy of the 32
+// rows: each quadrant's lanes then hold the gates of all rows, and its warps do a quarter of the units (@@).
 // The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
 // records.  The one input buffer is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
@@ -39,10 +43,14 @@ constexpr int kWorkerWarp0 = 4, kWorkerWarps = 16, kThreads = (kWorkerWarp0 + kW
 constexpr int kWarpUnits = 16;                       // units of a 64-unit slice that one worker warp handles
 constexpr int kABlock = kTile * 128;                 // K block of the layer input: [128 rows][64 K]
 constexpr int kWSlots = 4, kWSlot = kGateBlockBytes; // weight ring: one gate K block (24 KB) a slot
+constexpr int kMaxChunks = Gm<CFX_GAME_CLASSIC>::kEncChunks;
 constexpr int kASlots = 12;                          // operand chunks in tensor memory; a multiple of the warpgroups
 constexpr int kSSlots = 4, kSBox = kTile * 128, kQuadBox = 32 * 128;   // state ring: 128 rows x 32 units a slot, copied 32 rows at a time
 constexpr uint32_t kColAexp = 0, kColAcc = 384, kColHead = 448;
 __host__ __device__ constexpr uint32_t col_gate(int j) { return 192u * (uint32_t)j; }   // over the operand chunks, done by then
+
+constexpr int kQuadBlock = 32 * 128;                  // ONE: an operand chunk's block, [32 rows][64 K]
+constexpr uint32_t kColA = 192;                       // ONE: layer input, 32 columns a K block
 
 template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kKB = HID / 64;                        // K blocks of a layer's input
@@ -57,6 +65,10 @@ template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kBoxes = 2 * kNS;                      // state boxes of a layer
     static constexpr int kOffS = kKB * kABlock, kASBytes = kOffS + kSSlots * kSBox;   // layer input, state; first the records
     static constexpr int kOffW = (kASBytes > 4 * kQuadBytes ? kASBytes : 4 * kQuadBytes + 1023) / 1024 * 1024;
+    // ONE: operand chunks; an MMA reads 96 rows beyond a block's 32, which nobody looks at.  The classic game's 22 blocks
+    // reach from the records over the layer input, the full game's 14 lie where the state boxes are later
+    static constexpr int kOffX = GAME == CFX_GAME_FULL ? kOffS : 8192;
+    static_assert(kOffX + (Gm<GAME>::kEncBlocks + 3) * kQuadBlock <= kOffW + kWSlots * kWSlot && 32 * Gm<GAME>::kRecBytes <= kOffX, "operand chunks");
     static constexpr int kOffBias = kOffW + kWSlots * kWSlot;
     static constexpr int kOffBars = kOffBias + (kUnits + kHeadMax) * 4;
     static_assert(kNS >= 1 && kNS <= 2 && kUnits * S == HID && kEncTile * kEncPerItem <= kWSlot &&
@@ -66,10 +78,11 @@ template <int GAME, int HID, int S> struct Cfg {
 
 enum Bar {
     W_FULL = 0, W_EMPTY = W_FULL + kWSlots, REC_FULL = W_EMPTY + kWSlots, REC_FREE = REC_FULL + 4,
-    AEXP_FULL = REC_FREE + 1, AEXP_EMPTY = AEXP_FULL + kASlots, ACC_FULL = AEXP_EMPTY + kASlots,
+    AEXP_FULL = REC_FREE + 1, AEXP_EMPTY = AEXP_FULL + kMaxChunks, ACC_FULL = AEXP_EMPTY + kASlots,
     S_FULL = ACC_FULL + 1, ST_READY = S_FULL + kSSlots, MMA_DONE = ST_READY + kSSlots,
     QUAD = MMA_DONE + 1, G_FULL = QUAD + 8,   // QUAD: [slice][quadrant]
-    H_FULL = G_FULL + 2, A_KB = H_FULL + 1,   // A_KB: [layer input][K block]
+    H_FULL = G_FULL + 2, AT_KB = H_FULL + 1, A_KB = AT_KB + 4,   // AT_KB: ONE, K blocks of the layer input in tensor memory
+    // A_KB: [layer input][K block]
     NUM_BARS = A_KB + (kMaxLayers + 1) * 4
 };
 template <int GAME, int HID, int S> constexpr int smem_bytes() {
@@ -171,7 +184,7 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
         CFX_PROBE_READ(name, ready_);                                                                       \
         if (ready_ == 0 && !mbar_wait_spin(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return; \
     }
-template <typename T16, int GAME, int HID, int S>
+template <typename T16, int GAME, int HID, int S, bool ONE>
 __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32_t tmem, uint32_t rank) {
     using C = Cfg<GAME, HID, S>;
     constexpr uint32_t fmt = Op16<T16>::kFmt;
@@ -180,6 +193,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
     constexpr int kChunks = Gm<GAME>::kEncChunks, kGateItems = C::kNS * C::kKB;
     static_assert(kGateItems % kWSlots == 0 || kWSlots % kGateItems == 0, "a layer's first ring slot");
     const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
+    const uint64_t xdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffX));
     // ---- encoder
     CFX_SPROBE(cfx_p_b, W_FULL, 0);
     CFX_SPROBE(cfx_p_a, AEXP_FULL, 0);
@@ -190,21 +204,26 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         const int blk = full && kc >= 12 ? (kc < 14 ? 12 : 13) : kc, first = full && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0;
         const int ks = full ? full_ksteps(kc) : (kc == kChunks - 1 ? 1 : 4);
         const bool starts = !(full && (kc == 13 || kc == 15)), ends = !(full && (kc == 12 || kc == 14));
-        const int item = blk / C::kEncPerItem, slot = item % kWSlots, as = kc % kASlots;
+        const int item = blk / C::kEncPerItem, slot = item % kWSlots, as = ONE ? kc : kc % kASlots;
         if (starts && blk % C::kEncPerItem == 0) {
             CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, (item / kWSlots) & 1);
             CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
         }
-        CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + as, (kc / kASlots) & 1);
-        if (kc + 1 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + (kc + 1) % kASlots, ((kc + 1) / kASlots) & 1);
+        CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + as, ONE ? 0 : (kc / kASlots) & 1);
+        if (kc + 1 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + (ONE ? kc + 1 : (kc + 1) % kASlots), ONE ? 0 : ((kc + 1) / kASlots) & 1);
         tc_fence_after_sync();
         __syncwarp();
         const uint64_t bd = wdesc + (uint64_t)(((slot * kWSlot + blk % C::kEncPerItem * C::kEncTile) >> 4) + first);
         const uint32_t a = tmem + kColAexp + as * 32;
         if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < ks; k++) mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
-            if (kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
+            for (int k = 0; k < ks; k++) {
+                if constexpr (ONE)
+                    mma_f16_ss(tmem + kColAcc, xdesc + (uint64_t)(((blk * kQuadBlock) >> 4) + first + 2 * k), bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+                else
+                    mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+            }
+            if (!ONE && kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
             if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
             if (ends && ((blk + 1) % C::kEncPerItem == 0 || kc == kChunks - 1)) mma_commit(sm.bar(W_EMPTY + slot));
         }
@@ -218,18 +237,19 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 #pragma unroll 1
     for (int l = 0; l < P.L; l++) {
         const int slot0 = first_slot(l);
-        CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
+        if (!ONE) CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
         // this CTA's own K blocks first: the gate columns are free when its cells have read them
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) CFX_SWAIT_SPIN(A_KB + 4 * l + (int)rank * C::kNS + j, 0);
+        if (ONE) CFX_SPROBE(cfx_p_a, AT_KB, l & 1);
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) {
 #pragma unroll
             for (int kb = 0; kb < C::kKB; kb++) {
                 const int slot = (slot0 + j * C::kKB + kb) % kWSlots, slot1 = (slot + 1) % kWSlots;
                 if (j == 0) {
-                    CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * l + kb, 0);
-                    if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * l + kb + 1, 0);
+                    CFX_SWAIT_PROBED(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * l) + kb, ONE ? l & 1 : 0);
+                    if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * l) + kb + 1, ONE ? l & 1 : 0);
                 }
                 CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, wpar >> slot & 1u);
                 wpar ^= 1u << slot;
@@ -239,8 +259,12 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                 const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
                 if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 4; ks++)
-                        mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
+                    for (int ks = 0; ks < 4; ks++) {
+                        if constexpr (ONE)
+                            mma_f16_ts(tmem + col_gate(j), tmem + kColA + 32 * kb + 8 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
+                        else
+                            mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
+                    }
                     if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL + j));
                     if (j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
                     mma_commit(sm.bar(W_EMPTY + slot));
@@ -249,12 +273,12 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         }
     }
     const int slot0 = first_slot(P.L);
-    CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L, 0);
+    CFX_SPROBE(cfx_p_a, ONE ? (int)AT_KB : A_KB + 4 * P.L, ONE ? P.L & 1 : 0);
 #pragma unroll
     for (int kb = 0; kb < C::kKB; kb++) {
         const int slot = (slot0 + kb / 2) % kWSlots, slot1 = (slot + 1) % kWSlots;
-        CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * P.L + kb, 0);
-        if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L + kb + 1, 0);
+        CFX_SWAIT_PROBED(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * P.L) + kb, ONE ? P.L & 1 : 0);
+        if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * P.L) + kb + 1, ONE ? P.L & 1 : 0);
         if (kb % 2 == 0) {
             CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, wpar >> slot & 1u);
             CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
@@ -264,8 +288,12 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
         if (elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < 4; ks++)
-                mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+            for (int ks = 0; ks < 4; ks++) {
+                if constexpr (ONE)
+                    mma_f16_ts(tmem + kColHead, tmem + kColA + 32 * kb + 8 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+                else
+                    mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+            }
             if (kb == C::kKB - 1) mma_commit(sm.bar(H_FULL));
         }
     }
@@ -274,7 +302,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 // ------------------------------------------------------------------ state
 // One thread: box b of the tile (layer b / kBoxes, 32 units of all rows) uses slot b % kSSlots; a slot is loaded again when
 // the box before has been read out of it.
-template <int GAME, int HID, int S>
+template <int GAME, int HID, int S, bool ONE>
 __device__ __forceinline__ void role_state(const Smem& sm, const Params& P, int row0, uint32_t rank) {
     using C = Cfg<GAME, HID, S>;
     const int boxes = P.L * C::kBoxes;
@@ -287,6 +315,7 @@ __device__ __forceinline__ void role_state(const Smem& sm, const Params& P, int 
             tensor_g2s_2d(slot_at(b) + q * kQuadBox, &P.state_map[b / C::kBoxes], unit(b), row0 + 32 * q, sm.bar(S_FULL + b % kSSlots));
     };
     CFX_SWAIT(REC_FREE, 0);
+    if (ONE) CFX_SWAIT(ACC_FULL, 0);   // the operand chunks are used up
     for (int b = 0; b < kSSlots && b < boxes; b++) load(b);
     for (int b = 0; b < boxes; b++) {
         CFX_SWAIT(ST_READY + b % kSSlots, (b / kSSlots) & 1);
@@ -524,8 +553,216 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     }
 }
 
-// ------------------------------------------------------------------ kernel
+// ONE: warp (quadrant, wg) converts chunk 4 wg + quadrant (and the one 16 further), brings K block wg of every layer input
+// from shared memory to its quadrant's tensor memory, and handles units [16 wg + 4 quadrant, + 4) of the CTA's
+// slice; lane = row in all of it.
 template <typename T16, int GAME, int HID, int S>
+__device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
+                                                uint32_t rank) {
+    using Op = Op16<T16>;
+    using C = Cfg<GAME, HID, S>;
+    constexpr int kChunks = Gm<GAME>::kEncChunks, kA = Gm<GAME>::kA;
+    constexpr bool kFull = GAME == CFX_GAME_FULL;
+    const int quadrant = warp & 3, wg = (warp - kWorkerWarp0) >> 2, w = 4 * wg + quadrant, swz = lane & 7;
+    const uint32_t lane_base = tmem + ((uint32_t)(quadrant * 32) << 16);
+    const int env = row0 + lane;
+    const bool valid = env < P.n;   // all rows (n is a multiple of 32)
+    const float* bias = reinterpret_cast<const float*>(sm.base + C::kOffBias);
+    const bool draws = rank == 0 && w == 0;
+    const unsigned long long step0 = draws && P.uniforms == nullptr ? *P.step_ctr : 0ull;
+    const bool zero_state = valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
+    if (lane < 2 * P.L)   // two rows of the state, on their way to L2 while the records are expanded
+#pragma unroll
+        for (int r = w; r < 32; r += kWorkerWarps)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(P.state + ((size_t)(lane >> 1) * P.n + row0 + r) * HID + rank * kSliceUnits + 32 * (lane & 1)));
+    // 16-byte piece c of this lane's row of a 128-byte-swizzled block
+    auto piece = [&](uint32_t block, int c) { return sm.base + block + (lane >> 3) * 1024 + swz * 128 + ((c ^ swz) << 4); };
+
+    // ---- expand: K columns of a chunk go to the columns that its weight block has for them
+    CFX_SWAIT(REC_FULL, 0);
+    for (int kc = w; kc < kChunks; kc += kWorkerWarps) {
+        uint32_t regs[32];
+        const uint8_t* rec = sm.base + lane * C::kRowBytes;
+        if constexpr (kFull) expand_full<Op>(rec + 64 * kc, kc, regs);
+        else expand_classic<Op>(rec, kc, regs);
+        const int blk = kFull && kc >= 12 ? (kc < 14 ? 12 : 13) : kc;
+        const int first = kFull && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0, pieces = 2 * (kFull ? full_ksteps(kc) : 4);
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+            if (c < pieces)
+                *reinterpret_cast<uint4*>(piece(C::kOffX + blk * kQuadBlock, first + c)) = make_uint4(regs[4 * c], regs[4 * c + 1], regs[4 * c + 2], regs[4 * c + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + kc));
+    }
+    auto free_records = [&]() {
+        __syncwarp();
+        if (lane < S) mbar_arrive_cluster(map_to_cta(sm.bar(REC_FREE), (uint32_t)lane));
+    };
+    if (kFull) free_records();
+    float u = 0.0f;
+    if (draws) {   // (the counter: see role_worker)
+        u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
+        __syncwarp();
+        if (lane == 0 && P.bump_step) {
+            __threadfence();
+            if (atomicAdd(P.done_ctr, 1u) == P.done_blocks - 1) {
+                *P.step_ctr += 1ULL;
+                *P.done_ctr = 0u;
+            }
+        }
+    }
+
+    // Layer input l: the CTA's own K block is complete when all warps are here; then it goes to the other CTAs.
+    const uint32_t own = rank * kABlock;
+    auto send = [&](int l) {
+        tc_fence_before_sync();
+        fence_proxy_async_smem();
+        __syncwarp();
+        bool ok = true;
+        if (lane == 0) {
+            mbar_arrive(sm.bar(QUAD));
+            if (w == 0) {
+                ok = mbar_wait<false>(sm.bar(QUAD), l & 1, sm.abort_flag(), kSite + QUAD);
+                if (ok) {
+                    const uint32_t src = smem_u32(sm.base) + own, bar = sm.bar(A_KB + 4 * l + (int)rank);
+                    mbar_arrive(bar);
+#pragma unroll
+                    for (uint32_t d = 1; d < (uint32_t)S; d++) {
+                        const uint32_t peer = (rank + d) % (uint32_t)S;
+                        bulk_s2s(map_to_cta(src, peer), src, kABlock / 4, map_to_cta(bar, peer));
+                    }
+                }
+            }
+        }
+        return __all_sync(0xffffffffu, ok);
+    };
+    // K block wg of layer input l -> this quadrant's tensor memory
+    auto to_tmem = [&](int l) {
+        if (wg >= C::kKB) return true;
+        if (!mbar_wait<false>(sm.bar(A_KB + 4 * l + wg), 0, sm.abort_flag(), kSite + A_KB)) return false;
+        uint32_t lo[16], hi[16];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const uint4 a = *reinterpret_cast<const uint4*>(piece(wg * kABlock, c)), b = *reinterpret_cast<const uint4*>(piece(wg * kABlock, 4 + c));
+            lo[4 * c] = a.x; lo[4 * c + 1] = a.y; lo[4 * c + 2] = a.z; lo[4 * c + 3] = a.w;
+            hi[4 * c] = b.x; hi[4 * c + 1] = b.y; hi[4 * c + 2] = b.z; hi[4 * c + 3] = b.w;
+        }
+        tmem_st16(lane_base + kColA + 32 * wg, lo);
+        tmem_st16(lane_base + kColA + 32 * wg + 16, hi);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sm.bar(AT_KB + wg));
+        return true;
+    };
+
+    // ---- encoder output + bias -> layer-0 input (the first quadrant's lanes hold it)
+    CFX_SWAIT(ACC_FULL, 0);
+    tc_fence_after_sync();
+    if (!kFull) free_records();
+    CFX_SWAIT(REC_FREE, 0);
+    if (quadrant == 0) {
+        uint32_t acc[16];
+        tmem_ld16(lane_base + kColAcc + kWarpUnits * wg, acc);
+        tmem_wait_ld();
+        const float* b = bias + kWarpUnits * wg;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            uint32_t h[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int i = 8 * c + 2 * q;
+                h[q] = Op::pack(__uint_as_float(acc[i]) + b[i], __uint_as_float(acc[i + 1]) + b[i + 1]);
+            }
+            *reinterpret_cast<uint4*>(piece(own, 2 * wg + c)) = make_uint4(h[0], h[1], h[2], h[3]);
+        }
+    }
+    if (!send(0)) return;
+
+    // ---- layers: this thread's four units, bytes 8 (quadrant & 1) of piece 2 wg + quadrant / 2 of its row
+    uint2* xp = reinterpret_cast<uint2*>(piece(own, 2 * wg + (quadrant >> 1)) + 8 * (quadrant & 1));
+    const int unit = kWarpUnits * wg + 4 * quadrant;
+    for (int l = 0; l < P.L; l++) {
+        if (!to_tmem(l)) return;
+        CFX_SWAIT(A_KB + 4 * l + (int)rank, 0);
+        const uint2 x = *xp;
+        const int box = l * C::kBoxes + (wg >> 1), slot = box % kSSlots;
+        CFX_SWAIT(S_FULL + slot, (box / kSSlots) & 1);
+        float4* sp = reinterpret_cast<float4*>(piece(C::kOffS + slot * kSBox, 4 * (wg & 1) + quadrant));
+        float4 st = *sp;
+        if (zero_state) st = make_float4(0.f, 0.f, 0.f, 0.f);
+        // optional BPTT record of the post-zero input state (craftax_full.cu:9370-9375)
+        if (P.r_state != nullptr && valid) {
+            const size_t at = ((size_t)l * P.n + env) * HID + rank * kSliceUnits + unit;
+            if (P.r_state_bf16)
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(P.r_state) + at) =
+                    make_uint2(Op16<__nv_bfloat16>::pack(st.x, st.y), Op16<__nv_bfloat16>::pack(st.z, st.w));
+            else
+                *reinterpret_cast<float4*>(P.r_state + at) = st;
+        }
+        CFX_SWAIT(G_FULL, l & 1);
+        tc_fence_after_sync();
+        uint32_t zh[4], zg[4], zp[4];
+        tmem_ld4(lane_base + col_gate(0) + unit, zh);
+        tmem_ld4(lane_base + col_gate(0) + kSliceUnits + unit, zg);
+        tmem_ld4(lane_base + col_gate(0) + 2 * kSliceUnits + unit, zp);
+        tmem_wait_ld();
+        const float2 x01 = Op::unpack(x.x), x23 = Op::unpack(x.y);
+        float h0, h1, h2, h3;
+        mingru_cell_pair(__uint_as_float(zh[0]), __uint_as_float(zh[1]), __uint_as_float(zg[0]), __uint_as_float(zg[1]),
+                         __uint_as_float(zp[0]), __uint_as_float(zp[1]), st.x, st.y, x01.x, x01.y, st.x, st.y, h0, h1);
+        mingru_cell_pair(__uint_as_float(zh[2]), __uint_as_float(zh[3]), __uint_as_float(zg[2]), __uint_as_float(zg[3]),
+                         __uint_as_float(zp[2]), __uint_as_float(zp[3]), st.z, st.w, x23.x, x23.y, st.z, st.w, h2, h3);
+        *sp = st;
+        CFX_SWAIT(MMA_DONE, l & 1);
+        *xp = make_uint2(Op::pack(h0, h1), Op::pack(h2, h3));
+        if (!send(l + 1)) return;
+        if (lane == 0) mbar_arrive(sm.bar(ST_READY + slot));   // (send fenced the box as well)
+    }
+    if (!to_tmem(P.L)) return;
+
+    // ---- heads + sampler: every warp takes a sixteenth of the exponentials, the first one draws
+    if (rank == 0) {
+        constexpr int kHeadCols = (kA + 1 + 15) / 16 * 16, kPart = (kA + kWorkerWarps - 1) / kWorkerWarps;
+        CFX_SWAIT(H_FULL, 0);
+        tc_fence_after_sync();
+        uint32_t hv[kHeadCols];
+#pragma unroll
+        for (int b = 0; b < kHeadCols / 16; b++) {
+            uint32_t t[16];
+            tmem_ld16(lane_base + kColHead + 16 * b, t);
+#pragma unroll
+            for (int q = 0; q < 16; q++) hv[16 * b + q] = t[q];
+        }
+        tmem_wait_ld();
+        const float* hb = bias + C::kUnits;
+        float* p = reinterpret_cast<float*>(sm.base + C::kOffW) + lane;   // [action][row]: all weights are used up
+        float logits[kA];
+#pragma unroll
+        for (int a = 0; a < kA; a++) logits[a] = __uint_as_float(hv[a]) + hb[a];
+        const float value = __uint_as_float(hv[kA]) + hb[kA];
+        float m = logits[0];
+#pragma unroll
+        for (int a = 1; a < kA; a++) m = fmaxf(m, logits[a]);
+#pragma unroll
+        for (int a = 0; a < kA; a++)
+            if (a / kPart == w) p[a * 32] = expf(logits[a] - m);
+        if (w == kWorkerWarps - 1 && valid) write_logits<GAME>(P, env, logits, value);
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        if (w == 0 && valid) {
+            float pr[kA];
+#pragma unroll
+            for (int a = 0; a < kA; a++) pr[a] = p[a * 32];
+            float lp;
+            const int act = draw_action<kA>(logits, pr, m, u, &lp);
+            write_action(P, env, act, lp, value);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ kernel
+template <typename T16, int GAME, int HID, int S, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_constant__ Params P) {
     using C = Cfg<GAME, HID, S>;
     constexpr int kA = Gm<GAME>::kA;
@@ -542,12 +779,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     if (warp == 0) {   // a lane sets a barrier up
         for (int i = lane; i < NUM_BARS; i += 32) {
             uint32_t arrivals = 1, bytes = 0;
-            if (i == REC_FREE) arrivals = S * 4 * quads;
-            else if (i >= AEXP_FULL && i < AEXP_FULL + kASlots) arrivals = quads;
+            if (i == REC_FREE) arrivals = ONE ? S * kWorkerWarps : S * 4 * quads;
+            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? 1 : quads;
             else if (i == ACC_FULL) arrivals = 2;                          // the MMAs, and the biases are in place
-            else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = 2 * quads;
+            else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = ONE ? 8 : 2 * quads;
             else if (i == MMA_DONE) arrivals = S;
-            else if (i >= QUAD && i < QUAD + 8) arrivals = 4;
+            else if (i >= QUAD && i < QUAD + 8) arrivals = ONE ? kWorkerWarps : 4;
+            else if (i >= AT_KB && i < A_KB) arrivals = 4;
             else if (i >= A_KB) {
                 const int kb = (i - A_KB) % 4;
                 if (kb / C::kNS == (int)rank) arrivals = quads;
@@ -575,7 +813,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     if (warp == 0) {
         if (lane == 0) role_weights<GAME, HID, S>(sm, P, rank);
     } else if (warp == 1) {
-        role_mma<T16, GAME, HID, S>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
+        role_mma<T16, GAME, HID, S, ONE>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
     } else if (warp == 2) {
         // the tile's records, 32 rows a copy
         wait_for_previous_kernel();
@@ -593,10 +831,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         if (lane == 0) mbar_arrive(sm.bar(ACC_FULL));
     } else if (warp == 3) {
         wait_for_previous_kernel();
-        if (lane == 0) role_state<GAME, HID, S>(sm, P, row0, rank);
+        if (lane == 0) role_state<GAME, HID, S, ONE>(sm, P, row0, rank);
     } else {
         wait_for_previous_kernel();
-        role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
+        if constexpr (ONE) role_worker_one<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
+        else role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
     }
 
     // common exit, also after a timed-out wait: no CTA leaves while another may still copy to it
@@ -612,13 +851,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-static const void* kernel(int precision, int game, int H, int S, int* smem) {
+static const void* kernel(int precision, int game, int H, int S, bool one, int* smem) {
     const bool h = precision == CFX_PREC_F16;
 #define CFX_SPLIT(G, HID, SS)                                               \
     do {                                                                    \
         *smem = smem_bytes<G, HID, SS>();                                   \
-        return h ? (const void*)k_policy_split<__half, G, HID, SS>          \
-                 : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS>;  \
+        if constexpr (HID / 64 / SS == 1)                                   \
+            if (one)                                                        \
+                return h ? (const void*)k_policy_split<__half, G, HID, SS, true>          \
+                         : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS, true>;  \
+        return h ? (const void*)k_policy_split<__half, G, HID, SS, false>          \
+                 : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS, false>;  \
     } while (0)
     if (game == CFX_GAME_CLASSIC) {
         if (S == 4) CFX_SPLIT(CFX_GAME_CLASSIC, 256, 4);
@@ -651,7 +894,9 @@ int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_
     *max_clusters = 0;
     if (H / 64 / S < 1) return CFX_OK;
     int smem = 0;
-    const void* k = split::kernel(precision, game, H, S, &smem);
+    const void* k = split::kernel(precision, game, H, S, true, &smem);
+    CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k = split::kernel(precision, game, H, S, false, &smem);
     CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = split::config(at, sm_count / S * S, S, smem, nullptr);
@@ -664,7 +909,7 @@ int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_
 
 int split_launch(int precision, int game, int H, int S, int tiles, const Params& P, cudaStream_t st) {
     int smem = 0;
-    const void* k = split::kernel(precision, game, H, S, &smem);
+    const void* k = split::kernel(precision, game, H, S, P.tile_rows == 32, &smem);
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = split::config(at, tiles * S, S, smem, st);
     void* args[1] = {(void*)&P};
