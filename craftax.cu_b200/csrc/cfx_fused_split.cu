@@ -23,14 +23,14 @@
 // Tiles of 32 rows (ONE), the smallest batches: a quadrant of TMEM lanes belongs to one SM scheduler, so one
 // quadrant of rows would leave three schedulers idle.  The operand chunks go to shared memory instead, one of the sixteen
 // warps a chunk; and the layers' A operand is tensor memory again, where every quadrant gets a copy of the 32
-// rows: each quadrant's lanes then hold the gates of all rows, and its warps do a quarter of the units (@@).
+// rows: each quadrant's lanes then hold the gates of all rows, and its warps do a quarter of the units
+// (1,024 envs h256x2 15.5 -> 13.6 us).
 // The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
 // records.  The one input buffer is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
-// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 14.4, 1,024 25.7 -> 16.4,
-// 2,368 26 -> 19.9, 8,192 26.9 -> 22.8; classic h256x3, 1,024 envs 35.7 -> 23.4.  Bound by the chain: of 26,000 cycles
-// at 1,024 envs the records take 1,400, the encoder 7,000 (54 MMAs at the ~105 cycles one takes to issue), a layer 6,500 (exchange
-// 1,900, MMAs 1,800, cell 2,700: 48 tanh for each of the four warps of an SM scheduler), heads and sampler 4,500.
+// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 11.7, 1,024 25.7 -> 13.6,
+// 2,016 26 -> 16.5, 4,000 26 -> 19.2, 8,192 26.9 -> 21.6; classic h256x3, 1,024 envs 35.7 -> 16.6.  Bound by the chain of
+// dependent steps and the 3 us between one kernel's end and the next one's start.
 #include "cfx_fused_split.h"
 
 #include <type_traits>

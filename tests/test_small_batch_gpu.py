@@ -36,8 +36,8 @@ def _forward(cfx, n, H, L, prec, game, rec, params, state, prev_t, r_state, laun
     (2336, 256, 3, "bf16", "full", "bf16"), (2400, 256, 2, "f16", "full", None),    # the last one half empty; of 128
     (4704, 256, 4, "f16", "full", "fp32"), (4768, 256, 2, "f16", "full", "bf16"),   # clusters of four, of two
     (9472, 256, 3, "f16", "full", "fp32"), (9504, 256, 1, "f16", "full", None),     # the last of them; one CTA a tile
-    (64, 128, 2, "f16", "full", "bf16"), (2400, 128, 3, "bf16", "full", "fp32"), (9440, 128, 4, "f16", "full", None),
-    (160, 256, 3, "f16", "classic", None), (4736, 256, 2, "bf16", "classic", "fp32"),
+    (64, 128, 2, "f16", "full", "bf16"), (2368, 128, 1, "bf16", "full", "fp32"), (2400, 128, 3, "bf16", "full", "fp32"), (9440, 128, 4, "f16", "full", None),
+    (160, 256, 3, "f16", "classic", None), (1152, 256, 2, "bf16", "classic", "bf16"), (4736, 256, 2, "bf16", "classic", "fp32"),
     (9376, 256, 3, "f16", "classic", "bf16")])
 def test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, H, L, prec, game, r_state):
     from cfx import synth
