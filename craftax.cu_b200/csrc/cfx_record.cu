@@ -531,14 +531,17 @@ static_assert(offsetof(cfx_env_view, mob_type_id) - offsetof(cfx_env_view, playe
 // ------------------------------------------------------------------ classic game
 // record_obs_kernel (craftax_classic.cu:1884-1890) gives every env a thread that writes its 148
 // bytes one by one: 148 store instructions per warp, each touching 32 different records.  Here a
-// block gathers the records of 128 consecutive envs in shared memory, thread per env (the SoA
-// loads of a warp are contiguous), and writes the 18,944 contiguous bytes out as coalesced 16-byte
-// words.  The nine cells of a view row are nibbles of at most five bytes, so of two aligned words of the map: 14
-// loads a thread for the view, all in flight at once, where a load per cell made 63 (each touching
-// 32 sectors a warp), and the record's words are put together in registers (row length 37 words: no bank conflicts).
-// 262,144 envs: 103 -> 42 us.
+// block gathers the records of 64 consecutive envs, thread per env (the SoA loads of a warp are
+// contiguous, and all in flight at once), puts them together word by word in registers, and writes the 9,472
+// contiguous bytes out of shared memory as coalesced 16-byte words (row length 37 words: no bank conflicts).
+// The seven map rows of a view are 224 contiguous bytes: the warp copies those of two envs an
+// instruction to shared memory (whole rows: what is read from memory is 32-byte sectors anyway), where a
+// thread then takes the nine nibbles of a row from two words.  Loads of these words from the map
+// itself, 14 a thread, touch 32 cache lines an instruction: 20 of 41 us of a cache's time.  262,144 envs: a load per cell
+// 103 us, words from the map 41.5, rows through shared memory 27.3 (127 MB: 4.7 TB/s); 65,536 envs 12.4 -> 8.2 us.
 constexpr int kClRows = 7, kClCols = 9, kClCells = kClRows * kClCols, kClMap = 64, kClRowBytes = 32;
-constexpr int kClInv = 12, kClOutOfBounds = 1, kClBlockEnvs = 128, kClWords = kClassicRec / 4;
+constexpr int kClSpan = kClRows * kClRowBytes + 16;   // 60 words: as few bank conflicts as 16-byte pieces allow
+constexpr int kClInv = 12, kClOutOfBounds = 1, kClBlockEnvs = 64, kClWords = kClassicRec / 4;
 static_assert(2 * kClCells + kClInv + 6 + 4 == kClassicRec && kClassicRec % 4 == 0, "classic record layout");
 
 // bytes of a record put together in order, word by word; positions are compile-time constants once unrolled
@@ -552,87 +555,102 @@ struct ClassicWords {
 
 __global__ void __launch_bounds__(kClBlockEnvs) k_classic_record_rows(const __grid_constant__ cfx_classic_env_view V,
                                                                      uint8_t* __restrict__ records, int n_envs) {
-    __shared__ __align__(16) uint32_t srec[kClBlockEnvs * kClWords];
-    const int t = threadIdx.x;
-    const int e0 = blockIdx.x * kClBlockEnvs, e = e0 + t;
+    // the envs' map rows (the word before the first and the one after the last are read, and masked), then the records
+    __shared__ __align__(16) uint8_t smem[16 + kClBlockEnvs * kClSpan + 16];
+    static_assert(sizeof(smem) >= kClBlockEnvs * kClassicRec, "the records lie where the rows were");
+    const int t = threadIdx.x, lane = t & 31;
+    const int e0 = blockIdx.x * kClBlockEnvs, e = min(e0 + t, n_envs - 1);
     const int n = V.num_envs;
     wait_for_previous_kernel();
-    if (e < n_envs) {
-        const int pr = soa(V.player_r, 0, n, e), pc = soa(V.player_c, 0, n, e);
+    const int pr = soa(V.player_r, 0, n, e), pc = soa(V.player_c, 0, n, e);
+    int8_t inv[kClInv];
+#pragma unroll
+    for (int i = 0; i < kClInv; i++) inv[i] = soa(V.inv, i, n, e);
+    const int8_t intr[5] = {soa(V.health, 0, n, e), soa(V.food, 0, n, e), soa(V.drink, 0, n, e), soa(V.energy, 0, n, e),
+                            soa(V.player_dir, 0, n, e)};
+    const uint8_t sleeping = soa(V.is_sleeping, 0, n, e);
+    const float light = soa(V.light_level, 0, n, e);
+    constexpr int kMobsCl = 11;
+    const int16_t* const mob_r[4] = {V.zombie_r, V.cow_r, V.skel_r, V.arrow_r};
+    const int16_t* const mob_c[4] = {V.zombie_c, V.cow_c, V.skel_c, V.arrow_c};
+    const uint8_t* const mob_m[4] = {V.zombie_mask, V.cow_mask, V.skel_mask, V.arrow_mask};
+    constexpr int kKind[kMobsCl] = {0, 0, 0, 1, 1, 1, 2, 2, 3, 3, 3}, kSlot[kMobsCl] = {0, 1, 2, 0, 1, 2, 0, 1, 0, 1, 2};
+    int16_t mr[kMobsCl], mc[kMobsCl];
+    uint8_t on[kMobsCl];
+#pragma unroll
+    for (int i = 0; i < kMobsCl; i++) {
+        on[i] = soa(mob_m[kKind[i]], kSlot[i], n, e);
+        mr[i] = soa(mob_r[kKind[i]], kSlot[i], n, e);
+        mc[i] = soa(mob_c[kKind[i]], kSlot[i], n, e);
+    }
+    // view rows: blocks (a nibble per map column; 1 outside the map)  (:1061-1100)
+    // first byte and word of the view's columns in a map row (a view that is off the map is masked as a whole)
+    const int o = (pc - 4) >> 1, wi = min(max(o >> 2, -1), kClRowBytes / 4 - 1);
+    uint8_t* const span = smem + 16 + t * kClSpan;
+    const uintptr_t align = reinterpret_cast<uintptr_t>(V.map_packed) | V.map_stride;
+    if ((align & 15) == 0) {
+        const int j = lane & 15, half = lane >> 4;
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+            const int row = __shfl_sync(0xffffffffu, pr, i + half) - 3 + (j >> 1), env = __shfl_sync(0xffffffffu, e, i + half);
+            if (j < 2 * kClRows && row >= 0 && row < kClMap) {
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem + 16 + ((t & ~31) + i + half) * kClSpan + 16 * j);
+                const uint8_t* q = V.map_packed + (size_t)env * V.map_stride + row * kClRowBytes + 16 * (j & 1);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(q) : "memory");
+            }
+        }
+    } else {
         const uint8_t* map = V.map_packed + (size_t)e * V.map_stride;
-        // view rows: blocks (a nibble per map column; 1 outside the map)  (:1061-1100)
-        const int o = (pc - 4) >> 1, wi = o >> 2;   // first byte and word of the view's columns in a map row
-        const bool aligned = ((reinterpret_cast<uintptr_t>(V.map_packed) | V.map_stride) & 3) == 0;
-        auto word = [&](int mr, int i) -> uint32_t {
-            if (mr < 0 || mr >= kClMap || i < 0 || i >= kClRowBytes / 4) return 0u;
-            const uint8_t* q = map + mr * kClRowBytes + 4 * i;
-            if (aligned) return ld_now(reinterpret_cast<const uint32_t*>(q));
-            return ld_now(q) | (uint32_t)ld_now(q + 1) << 8 | (uint32_t)ld_now(q + 2) << 16 | (uint32_t)ld_now(q + 3) << 24;
-        };
-        uint32_t m0[kClRows], m1[kClRows];
-#pragma unroll
-        for (int r = 0; r < kClRows; r++) {
-            m0[r] = word(pr - 3 + r, wi);
-            m1[r] = word(pr - 3 + r, wi + 1);
+        for (int k = 0; k < 2 * kClRows; k++) {
+            const int row = pr - 3 + k / 2, i = wi + k % 2;
+            if (row < 0 || row >= kClMap || i < 0 || i >= kClRowBytes / 4) continue;
+            const uint8_t* q = map + row * kClRowBytes + 4 * i;
+            uint32_t w;
+            if ((align & 3) == 0) w = ld_now(reinterpret_cast<const uint32_t*>(q));
+            else w = ld_now(q) | (uint32_t)ld_now(q + 1) << 8 | (uint32_t)ld_now(q + 2) << 16 | (uint32_t)ld_now(q + 3) << 24;
+            *reinterpret_cast<uint32_t*>(span + k / 2 * kClRowBytes + 4 * i) = w;
         }
-        int8_t inv[kClInv];
+    }
+    ClassicWords R;
 #pragma unroll
-        for (int i = 0; i < kClInv; i++) inv[i] = soa(V.inv, i, n, e);
-        const int8_t intr[5] = {soa(V.health, 0, n, e), soa(V.food, 0, n, e), soa(V.drink, 0, n, e), soa(V.energy, 0, n, e),
-                                soa(V.player_dir, 0, n, e)};
-        const uint8_t sleeping = soa(V.is_sleeping, 0, n, e);
-        const float light = soa(V.light_level, 0, n, e);
-        constexpr int kMobsCl = 11;
-        const int16_t* const mob_r[4] = {V.zombie_r, V.cow_r, V.skel_r, V.arrow_r};
-        const int16_t* const mob_c[4] = {V.zombie_c, V.cow_c, V.skel_c, V.arrow_c};
-        const uint8_t* const mob_m[4] = {V.zombie_mask, V.cow_mask, V.skel_mask, V.arrow_mask};
-        constexpr int kKind[kMobsCl] = {0, 0, 0, 1, 1, 1, 2, 2, 3, 3, 3}, kSlot[kMobsCl] = {0, 1, 2, 0, 1, 2, 0, 1, 0, 1, 2};
-        int16_t mr[kMobsCl], mc[kMobsCl];
-        uint8_t on[kMobsCl];
+    for (int i = 0; i < kClWords; i++) R.w[i] = 0u;
+    // inventory, intrinsics, direction, sleeping, light  (:1590-1603)
+    constexpr int kTailPos = 2 * kClCells;
 #pragma unroll
-        for (int i = 0; i < kMobsCl; i++) {
-            on[i] = soa(mob_m[kKind[i]], kSlot[i], n, e);
-            mr[i] = soa(mob_r[kKind[i]], kSlot[i], n, e);
-            mc[i] = soa(mob_c[kKind[i]], kSlot[i], n, e);
-        }
-        ClassicWords R;
+    for (int i = 0; i < kClInv; i++) R.put(kTailPos + i, (uint8_t)inv[i], 1);
 #pragma unroll
-        for (int i = 0; i < kClWords; i++) R.w[i] = 0u;
-        // inventory, intrinsics, direction, sleeping, light  (:1590-1603)
-        constexpr int kTailPos = 2 * kClCells;
+    for (int i = 0; i < 5; i++) R.put(kTailPos + kClInv + i, (uint8_t)intr[i], 1);
+    R.put(kTailPos + kClInv + 5, sleeping ? 1u : 0u, 1);
+    R.put(kTailPos + kClInv + 6, __float_as_uint(light), 4);
+    // columns of the view that lie on the map, a nibble each
+    uint64_t in = 0;
 #pragma unroll
-        for (int i = 0; i < kClInv; i++) R.put(kTailPos + i, (uint8_t)inv[i], 1);
+    for (int c = 0; c < kClCols; c++)
+        if (pc - 4 + c >= 0 && pc - 4 + c < kClMap) in |= 15ull << (4 * c);
+    const int shift = 8 * (o & 3) + 4 * (pc & 1);
+    wait_spans();
 #pragma unroll
-        for (int i = 0; i < 5; i++) R.put(kTailPos + kClInv + i, (uint8_t)intr[i], 1);
-        R.put(kTailPos + kClInv + 5, sleeping ? 1u : 0u, 1);
-        R.put(kTailPos + kClInv + 6, __float_as_uint(light), 4);
-        // columns of the view that lie on the map, a nibble each
-        uint64_t in = 0;
+    for (int r = 0; r < kClRows; r++) {
+        const bool row_in = pr - 3 + r >= 0 && pr - 3 + r < kClMap;
+        const uint64_t keep = row_in ? in : 0ull;
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(span + r * kClRowBytes) + wi;
+        const uint64_t v = (((uint64_t)w[1] << 32 | w[0]) >> shift & keep) | (0x111111111ull * kClOutOfBounds & ~keep);
+        const uint32_t lo = (uint32_t)v, even = lo & 0x0F0F0F0Fu, odd = lo >> 4 & 0x0F0F0F0Fu;
+        R.put(r * kClCols, __byte_perm(even, odd, 0x5140), 4);
+        R.put(r * kClCols + 4, __byte_perm(even, odd, 0x7362), 4);
+        R.put(r * kClCols + 8, (uint32_t)(v >> 32) & 15u, 1);
+    }
+    __syncthreads();   // the rows of all warps are in registers
+    uint32_t* const srec = reinterpret_cast<uint32_t*>(smem);
 #pragma unroll
-        for (int c = 0; c < kClCols; c++)
-            if (pc - 4 + c >= 0 && pc - 4 + c < kClMap) in |= 15ull << (4 * c);
-        const int shift = 8 * (o & 3) + 4 * (pc & 1);
+    for (int i = 0; i < kClWords; i++) srec[t * kClWords + i] = R.w[i];
+    // mobs inside the view set their bit  (:1102-1125)
+    uint8_t* mobs = reinterpret_cast<uint8_t*>(srec + t * kClWords) + kClCells;
 #pragma unroll
-        for (int r = 0; r < kClRows; r++) {
-            const bool row_in = pr - 3 + r >= 0 && pr - 3 + r < kClMap;
-            const uint64_t keep = row_in ? in : 0ull;
-            const uint64_t v = (((uint64_t)m1[r] << 32 | m0[r]) >> shift & keep) |
-                               (0x111111111ull * kClOutOfBounds & ~keep);
-            const uint32_t lo = (uint32_t)v, even = lo & 0x0F0F0F0Fu, odd = lo >> 4 & 0x0F0F0F0Fu;
-            R.put(r * kClCols, __byte_perm(even, odd, 0x5140), 4);
-            R.put(r * kClCols + 4, __byte_perm(even, odd, 0x7362), 4);
-            R.put(r * kClCols + 8, (uint32_t)(v >> 32) & 15u, 1);
-        }
-#pragma unroll
-        for (int i = 0; i < kClWords; i++) srec[t * kClWords + i] = R.w[i];
-        // mobs inside the view set their bit  (:1102-1125)
-        uint8_t* mobs = reinterpret_cast<uint8_t*>(srec + t * kClWords) + kClCells;
-#pragma unroll
-        for (int i = 0; i < kMobsCl; i++) {
-            const int dr = mr[i] - pr + 3, dc = mc[i] - pc + 4;
-            if (on[i] != 0 && (unsigned)dr < (unsigned)kClRows && (unsigned)dc < (unsigned)kClCols)
-                mobs[dr * kClCols + dc] |= (uint8_t)(1 << kKind[i]);
-        }
+    for (int i = 0; i < kMobsCl; i++) {
+        const int dr = mr[i] - pr + 3, dc = mc[i] - pc + 4;
+        if (on[i] != 0 && (unsigned)dr < (unsigned)kClRows && (unsigned)dc < (unsigned)kClCols)
+            mobs[dr * kClCols + dc] |= (uint8_t)(1 << kKind[i]);
     }
     __syncthreads();
     // the block's records are contiguous in global memory: 37 words per env

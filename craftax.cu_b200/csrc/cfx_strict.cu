@@ -117,7 +117,7 @@ __host__ __device__ __forceinline__ size_t act_at(size_t e, int k, int H) { retu
 // stages over.  4,096 envs, hidden 256: 52 us, against 63 us with every warp doing both, and 78 us
 // with the features kept as bytes and converted by the lanes that multiply.  A small batch is bound by the latency of these
 // loads: record words are fetched three chunks ahead, W_enc rows S - 2 chunks, and the 51 raw floats of the tail are copied
-// at the start by the warps that multiply (32 envs: 25 us with one chunk ahead, @@ now).
+// at the start by the warps that multiply (32 envs, encoder by itself: 25 us with one chunk ahead, 17 so).
 constexpr int kEncK = 32, kEncAhead = 3;
 constexpr int kMapChunks = (kMap + kEncK - 1) / kEncK, kEncChunks = kMapChunks + (kTail + kEncK - 1) / kEncK;   // 25 of record bytes, 2 of the tail
 static_assert(kEncChunks % kEncAhead == 0, "the chunk loop is unrolled by the words in flight");

@@ -99,7 +99,8 @@ def _classic_records(f, maps):
     return rec
 
 
-@pytest.mark.parametrize("n,stride,rec_shift", [(1, 2048, 0), (127, 2052, 4), (128, 2049, 0), (259, 2048, 12)])
+@pytest.mark.parametrize("n,stride,rec_shift", [(1, 2048, 0), (127, 2052, 4), (128, 2049, 0), (259, 2048, 12),
+                                                (64, 2064, 0), (65, 2048, 0)])
 def test_classic_record_rows_at_edges(cfx, gpu, n, stride, rec_shift):
     rng = np.random.default_rng(n)
     maps = rng.integers(0, 256, (n, stride)).astype(np.uint8)
