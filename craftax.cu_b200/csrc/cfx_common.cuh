@@ -106,8 +106,9 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
 }
 
 // A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per device
+// (`static`: a process that has loaded two builds of the library sets them for the kernels of each)
 template <auto kernel>
-int allow_smem(int smem) {
+static int allow_smem(int smem) {
     constexpr int kMaxDevices = 64;
     static std::atomic<int> done[kMaxDevices];   // the largest size allowed so far
     int dev = 0;

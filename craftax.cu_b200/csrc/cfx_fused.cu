@@ -732,6 +732,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         const bool valid = env < P.n;
         const bool zero_state =
             valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
+        const uint32_t zero_rows = __ballot_sync(0xffffffffu, zero_state);
 
         // ---- expand: record bytes -> 16-bit operand rows in the TMEM chunk ring.
         // Full game: wg 1 converts chunks 0-2 and the even ones after them, wg 0 (which samples
@@ -853,6 +854,16 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             const uint32_t a_cur = tmem + lane_base + ((l & 1) ? kColA1 : kColA0);
             const uint32_t a_next = tmem + lane_base + ((l & 1) ? kColA0 : kColA1);
             for (int j = 0; j < kSlices; j++, gcnt++) {
+                const int box = 2 * j + wg;
+                const uint32_t scnt = (it * P.L + l) * kStateItems + box;
+                constexpr int kNS = C::kNS;
+                const int slot = scnt % kNS;
+                if (P.r_state != nullptr && valid) {   // under the slice's MMAs (of a warp's rows all or none are valid)
+                    CFX_WAITW(S_FULL + slot, (scnt / kNS) & 1, W_S_FULL);
+                    write_r_state<8, kH>(P, sm.s_slot(slot) + quarter * 4096, 0,
+                                         ((size_t)l * P.n + tile * kTile + quarter * 32) * kH + kSliceUnits * j + kHalfUnits * wg,
+                                         zero_rows, lane);
+                }
                 {
                     uint32_t g_ok;
                     CFX_PROBE_READ(cfx_p_g, g_ok);
@@ -860,10 +871,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 }
                 CFX_MARK(6);
                 tc_fence_after_sync();
-                const int box = 2 * j + wg;
-                const uint32_t scnt = (it * P.L + l) * kStateItems + box;
-                constexpr int kNS = C::kNS;
-                const int slot = scnt % kNS;
                 CFX_PROBE(cfx_p_s, sm.bar(S_FULL + slot), (scnt / kNS) & 1);
                 const uint32_t gcol = tmem + lane_base + kColG + kHalfUnits * wg;
                 uint8_t* rbase = sm.s_slot(slot) + (row >> 3) * 1024 + (row & 7) * 128;
@@ -907,21 +914,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                         float4* sp = reinterpret_cast<float4*>(rbase + (((4 * hf + q) ^ xr) << 4));
                         float4 st = *sp;
                         if (zero_state) st = make_float4(0.f, 0.f, 0.f, 0.f);
-                        // optional BPTT record of the post-zero input state (what the reference's
-                        // k_mingru_epi_fwd stores, craftax_full.cu:9370-9375): [L][n][256] fp32
-                        if (P.r_state != nullptr && valid) {
-                            const size_t o = ((size_t)l * P.n + env) * kH + kSliceUnits * j + kHalfUnits * wg + u;
-                            if (P.r_state_bf16) {
-                                __nv_bfloat162 lo2 = __floats2bfloat162_rn(st.x, st.y);
-                                __nv_bfloat162 hi2 = __floats2bfloat162_rn(st.z, st.w);
-                                uint2 v2;
-                                v2.x = *reinterpret_cast<uint32_t*>(&lo2);
-                                v2.y = *reinterpret_cast<uint32_t*>(&hi2);
-                                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(P.r_state) + o) = v2;
-                            } else {
-                                *reinterpret_cast<float4*>(P.r_state + o) = st;
-                            }
-                        }
                         const float2 x01 = Op::unpack(xin[u / 2]), x23 = Op::unpack(xin[u / 2 + 1]);
                         float4 out;
                         float h0, h1, h2, h3;

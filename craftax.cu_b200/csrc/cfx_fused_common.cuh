@@ -219,6 +219,36 @@ __device__ __forceinline__ void mingru_cell_pair(float hzh0, float hzh1, float h
     f2unpack(h, h0, h1);
 }
 
+// ---------------------------------------------------------------- BPTT record of the state
+// The optional record of the post-zero input state (what the reference's k_mingru_epi_fwd stores,
+// craftax_full.cu:9370-9375), [L][n][H] fp32 or bf16.  A warp writes its 32 rows x 4 PIECES units from
+// the state box (128-byte swizzled rows) before the cell updates it in place: PIECES lanes side by side take a row's
+// 16-byte pieces, so that a store instruction touches 32 / PIECES rows.  With every lane writing the row whose cell
+// it computes, it touched 32, and these stores kept the load/store unit busy for most of a slice: h256x2, 57,600 envs
+// 126.6 -> 112.9 us with a bf16 record, 139.3 -> 123.1 with fp32; 16,416 envs 35.0 -> 30.7 and 37.1 -> 33.8; 8,192 envs
+// (cfx_fused_split.cu) 25.9 -> 24.2 and 28.9 -> 25.2.
+// `box`: the row of lane 0 (a multiple of 8 rows into the box); `at`: element of that row and the first of the warp's units
+template <int PIECES, int HID>
+__device__ __forceinline__ void write_r_state(const Params& P, const uint8_t* box, int piece0, size_t at, uint32_t zero_rows,
+                                              int lane) {
+    const int piece = lane % PIECES, k = lane / PIECES;
+    // eight lanes in turn read shared memory without a bank conflict: rows that differ in bit 2 where they take two rows
+    const int r0 = PIECES == 4 ? (k >> 1) | (k & 1) << 2 : k;
+#pragma unroll
+    for (int i = 0; i < PIECES; i++) {
+        const int r = i * (32 / PIECES) + r0;
+        float4 st = *reinterpret_cast<const float4*>(box + (r >> 3) * 1024 + (r & 7) * 128 + (((piece0 + piece) ^ (r & 7)) << 4));
+        if (zero_rows >> r & 1u) st = make_float4(0.f, 0.f, 0.f, 0.f);
+        const size_t o = at + (size_t)r * HID + 4 * piece;
+        if (P.r_state_bf16)
+            *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(P.r_state) + o) =
+                make_uint2(Op16<__nv_bfloat16>::pack(st.x, st.y), Op16<__nv_bfloat16>::pack(st.z, st.w));
+        else
+            *reinterpret_cast<float4*>(P.r_state + o) = st;
+    }
+    __syncwarp();   // the cell's lanes overwrite the box
+}
+
 // ------------------------------------------------------------------ record expansion
 // One operand chunk (64 K columns, 32 packed pairs) of one env.
 // Full game: chunk kc = record bytes [64 kc, 64 kc + 64) at `src` (4-byte aligned): map bytes, then raw

@@ -347,6 +347,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     const bool samples = quadrant * min(S, quads) / quads == (int)rank;   // this CTA samples the quadrant's rows
     const unsigned long long step0 = samples && wg == 0 && P.uniforms == nullptr ? *P.step_ctr : 0ull;
     const bool zero_state = valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
+    const uint32_t zero_rows = __ballot_sync(0xffffffffu, zero_state);
     if (valid && lane < P.L * C::kNS) {   // this warp's rows of the state, on their way to L2 while the records are expanded
         const float* q = P.state + ((size_t)(lane / C::kNS) * P.n + env - lane) * HID + ((int)rank * C::kNS + lane % C::kNS) * kSliceUnits;
         for (int r = wg; r < 32; r += 4) {
@@ -460,6 +461,12 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     for (int l = 0; l < P.L; l++) {
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) {
+            const int box = l * C::kBoxes + 2 * j + (wg >> 1), slot = box % kSSlots;
+            CFX_SWAIT(S_FULL + slot, (box / kSSlots) & 1);
+            if (P.r_state != nullptr && valid)   // under the slice's MMAs
+                write_r_state<4, HID>(P, sm.base + C::kOffS + slot * kSBox + quadrant * 4096, 4 * (wg & 1),
+                                      ((size_t)l * P.n + row0 + 32 * quadrant) * HID + ((int)rank * C::kNS + j) * kSliceUnits + wg * kWarpUnits,
+                                      zero_rows, lane);
             CFX_SWAIT(G_FULL + j, l & 1);
             tc_fence_after_sync();
             uint32_t zh[16], zg[16], zp[16];
@@ -467,8 +474,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             tmem_ld16(lane_base + col_gate(j) + kSliceUnits + kWarpUnits * wg, zg);
             tmem_ld16(lane_base + col_gate(j) + 2 * kSliceUnits + kWarpUnits * wg, zp);
             tmem_wait_ld();
-            const int box = l * C::kBoxes + 2 * j + (wg >> 1), slot = box % kSSlots;
-            CFX_SWAIT(S_FULL + slot, (box / kSSlots) & 1);
             uint8_t* sp = sm.base + C::kOffS + slot * kSBox + (row >> 3) * 1024 + (row & 7) * 128;
             auto piece = [&](int q) { return reinterpret_cast<float4*>(sp + (((4 * (wg & 1) + q) ^ (row & 7)) << 4)); };
             float st[kWarpUnits];
@@ -477,23 +482,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 float4 v = *piece(q);
                 if (zero_state) v = make_float4(0.f, 0.f, 0.f, 0.f);
                 st[4 * q] = v.x; st[4 * q + 1] = v.y; st[4 * q + 2] = v.z; st[4 * q + 3] = v.w;
-            }
-            // optional BPTT record of the post-zero input state (craftax_full.cu:9370-9375)
-            if (P.r_state != nullptr && valid) {
-                const size_t at = ((size_t)l * P.n + env) * HID + ((int)rank * C::kNS + j) * kSliceUnits + wg * kWarpUnits;
-                if (P.r_state_bf16) {
-#pragma unroll
-                    for (int q = 0; q < kWarpUnits / 8; q++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int i = 0; i < 4; i++) w[i] = Op16<__nv_bfloat16>::pack(st[8 * q + 2 * i], st[8 * q + 2 * i + 1]);
-                        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(P.r_state) + at + 8 * q) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                } else {
-#pragma unroll
-                    for (int q = 0; q < kWarpUnits / 4; q++)
-                        *reinterpret_cast<float4*>(P.r_state + at + 4 * q) = make_float4(st[4 * q], st[4 * q + 1], st[4 * q + 2], st[4 * q + 3]);
-                }
             }
 #pragma unroll
             for (int q = 0; q < kWarpUnits / 4; q++) {
