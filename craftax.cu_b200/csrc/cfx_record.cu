@@ -4,20 +4,21 @@
 // The reference gives every env a warp and lets lane 0 walk the mob slots and compute the 51
 // tail scalars; every one of its ~110 scalar loads then fetches 4 bytes of a sector on its own,
 // one after the other.  Here a block of eight warps owns 32 consecutive envs:
-//   1. the view of an env is 9 rows of 11 bytes, 48 bytes apart: at most 410 contiguous bytes of each of
-//      three map planes.  Every warp starts asynchronous 16-byte copies of its four envs' spans to shared
-//      memory, all twelve in flight;
+//   1. the view of an env is 9 rows of 11 bytes in each of three map planes, a row in at most two 16-byte pieces.  A lane
+//      takes a row of a plane, and every warp starts asynchronous copies of its four envs' pieces to shared
+//      memory, all in flight;
 //   2. meanwhile, lane per env: the ~50 SoA fields and the 14 mob slots of the player's level are loaded
 //      by lane e for env e, so that a warp's loads of a field are one 128-byte line, each warp an eighth
 //      of them, all of a lane's in flight; they leave the 51 tail floats and the mobs (an earlier
 //      slot of a class that a later slot covers is dropped) in shared memory;
-//   3. warp per env: a lane makes four cells of a view row from the spans in registers, the four records
-//      are put together where the spans were, and go out as one bulk copy (1,992 blocks of 16 bytes a
+//   3. warp per env: a lane makes four cells of a view row from the pieces in registers, the four records
+//      are put together where the pieces were, and go out as one bulk copy (1,992 blocks of 16 bytes a
 //      block) or, where an env is skipped, as coalesced words.
 // Before: a byte load per cell and map, two half-used store instructions per 32 cells, the fields one DRAM
 // latency after the other (see ld_now), a read of the light map per mob behind them.  65,536 envs with 62 KB of maps
-// each: 54.7 -> 49 us (16,384 envs: 24.9 -> 14.9 us); 182 MB of DRAM traffic instead of 204, bound by
-// the scattered pieces: 3.7 TB/s whatever the mix, and the time adds up over writes, spans and fields.
+// each: 54.7 us; whole 410-byte spans of the planes copied, three a warp and env, 49.5; pieces of rows 46.6 (16,384 envs: 24.9
+// -> 14.9 us with spans).  About 180 MB of DRAM traffic, 3.9 TB/s: bound by the scattered pieces, the time adds up over
+// writes, map rows and fields, and five blocks an SM instead of four take 48.4 us.
 // The bytes are the reference's: the same predicates, the same "last slot of a class wins a
 // cell" order, the same float expressions (sqrtf(x) * 0.1f, x * 0.1f, x * 0.5f, x * 0.25f; no
 // fused multiply-add can form).
@@ -47,17 +48,18 @@ struct Params {
     const int* count_dev;
     int n;
 };
-constexpr int kSpan = 416, kPlanes = 3;   // 8 rows x 48 + 11 bytes, plus 15 to the boundary before: 410
+constexpr int kPlanes = 3, kRowSpan = 32;                // a view row: 11 bytes, so of at most two 16-byte pieces of a map row
+constexpr int kSpan = kRows * kRowSpan;                  // of a plane
 constexpr int kWarps = kBlockThreads / 32, kOwn = kBlockEnvs / kWarps;   // envs whose records a warp writes
 constexpr int kPlaneBytes = kMapSize * kMapSize, kRecWords = kRec / 4, kMapWords = kMap / 4;
 struct Shared {
     float tail[kBlockEnvs][kTail];       // odd row length: conflict-free thread-per-env writes
     uint32_t mobs[kBlockEnvs][kMobs];
-    // per warp the spans of its four envs (light, block, item; words before and after are read, and masked), and in their
-    // place, once they are in registers, its four records as they go out
-    __align__(16) uint8_t span[kWarps][kOwn][kPlanes][kSpan];
+    // per warp its four records as they go out, and before that, until they are in registers, the rows of its four
+    // envs' views (light, block, item)
+    __align__(16) uint8_t span[kWarps][kOwn * kRec];
 };
-static_assert(kOwn * kRec % 16 == 0 && kRec <= kPlanes * kSpan, "a warp's records are whole 16-byte words");
+static_assert(kOwn * kRec % 16 == 0 && kRec >= kPlanes * kSpan, "a warp's records are whole 16-byte words");
 
 // craftax_wg_jax_index (:1963-1975): negative indices wrap once, then clamp
 __device__ __forceinline__ int jax_index(int i, int size) {
@@ -154,7 +156,7 @@ __device__ __forceinline__ void gather_env(const cfx_env_view& V, int e, int t, 
     const int n = V.num_envs;
     float* o = S.tail[t];
     // mobs of the player's level inside the view and on the map (:9195-9236).  Whether the cell is lit is
-    // looked up in the span when the record is put together: two slots on one cell are both lit or
+    // looked up in the copied row when the record is put together: two slots on one cell are both lit or
     // both not, so the order of dropping does not depend on it.
     const int mob_level = jax_index(level, kLevels);
     auto mobs = [&](auto... c) { return (gather_mobs<decltype(c)::value>(V, e, mob_level, top, left, S.mobs[t]) | ...); };
@@ -227,53 +229,56 @@ __device__ __forceinline__ void gather_env(const cfx_env_view& V, int e, int t, 
     }
 }
 
-// What the copies and the assembly of one env need, two words: the rows and columns of the view that are on the map are
-// contiguous in a plane from `first` (aligned down to what the copies move at a time, `grain` bytes).
+// What the copies and the assembly of one env need, in a word: top and left of the view, plane of the level, and whether there
+// is such a level.
 struct View {
-    uint32_t where;   // first | (top + 32) << 12 | (left + 32) << 19 | level in [0, 9) << 26
-    uint32_t plane;   // bytes to copy | level's plane << 16
-    __device__ __forceinline__ int first() const { return where & 0xFFF; }
-    __device__ __forceinline__ int top() const { return (int)(where >> 12 & 127u) - 32; }
-    __device__ __forceinline__ int left() const { return (int)(where >> 19 & 127u) - 32; }
-    __device__ __forceinline__ bool level_ok() const { return where >> 26; }
-    __device__ __forceinline__ int bytes() const { return plane & 0xFFFF; }
-    __device__ __forceinline__ int level() const { return plane >> 16; }
+    uint32_t bits;   // (top + 32) | (left + 32) << 8 | plane << 16 | ok << 24
+    __device__ __forceinline__ int top() const { return (int)(bits & 255u) - 32; }
+    __device__ __forceinline__ int left() const { return (int)(bits >> 8 & 255u) - 32; }
+    __device__ __forceinline__ int level() const { return bits >> 16 & 255u; }
+    __device__ __forceinline__ bool level_ok() const { return bits >> 24; }
 };
-__device__ __forceinline__ View make_view(int level, int top, int left, int grain) {
+__device__ __forceinline__ View make_view(int level, int top, int left) {
     top = min(max(top, -32), 64);      // (a view that is off the map stays off it)
     left = min(max(left, -32), 64);
-    const int r0 = max(top, 0), r1 = min(top + kRows, kMapSize) - 1, c0 = max(left, 0), c1 = min(left + kCols, kMapSize) - 1;
-    int first = 0, bytes = 0;
-    if (r0 <= r1 && c0 <= c1) {
-        first = (r0 * kMapSize + c0) & ~(grain - 1);
-        bytes = r1 * kMapSize + c1 + 1 - first;
+    return {(uint32_t)(top + 32) | (uint32_t)(left + 32) << 8 | (uint32_t)jax_index(level, kLevels) << 16 |
+            ((unsigned)level < (unsigned)kLevels ? 1u << 24 : 0u)};
+}
+// Where byte `o` of a view row's 32 bytes lies: rows 4 to 7 have their halves swapped, so that a warp's reads of the nine rows
+// meet in a bank two at a time and not three
+__device__ __forceinline__ int row_byte(int dr, int o) { return dr * kRowSpan + (o ^ (dr & 4) << 2); }
+// The part of a lane in the copies of a view's rows (light, block, item): row `dr` of plane `plane`, `src` is the plane of env 0
+struct CopyLane {
+    const uint8_t* src;
+    int plane, dr;
+    __device__ __forceinline__ CopyLane(const cfx_env_view& V, int lane) {
+        plane = lane / kRows;
+        dr = lane % kRows;
+        src = V.state_base + (plane == 0 ? V.light_map_offset : plane == 1 ? V.map_offset : V.item_map_offset);
     }
-    View v;
-    v.where = (uint32_t)first | (uint32_t)(top + 32) << 12 | (uint32_t)(left + 32) << 19 |
-              ((unsigned)level < (unsigned)kLevels ? 1u << 26 : 0u);
-    v.plane = (uint32_t)bytes | (uint32_t)jax_index(level, kLevels) << 16;
-    return v;
-}
-// Starts the copies of one env's three spans (light, block, item) into `dst`.  A plane is 2,304 bytes, so 16-byte
-// pieces (4-byte pieces) stay inside it where the planes are aligned to 16 (4) bytes.
-__device__ __forceinline__ void copy_spans(const cfx_env_view& V, int e, View v, int grain, int lane, uint8_t (*dst)[kSpan]) {
-    const uint8_t* q = V.state_base + (size_t)e * V.state_stride + (v.level() * kPlaneBytes + v.first());
-    auto plane = [&](const uint8_t* src, uint8_t* d) {
-        const uint32_t ds = (uint32_t)__cvta_generic_to_shared(d);
+    // Starts the copies of env e's rows into `dst`.  A map row is 48 bytes, so 16-byte pieces (4-byte pieces) stay inside
+    // it where the planes are aligned to 16 (4) bytes.
+    __device__ __forceinline__ void start(const cfx_env_view& V, int e, View v, int grain, uint8_t* dst) const {
+        const int row = v.top() + dr, left = v.left(), c0 = left & ~15;
+        if (plane >= kPlanes || (unsigned)row >= (unsigned)kMapSize) return;
+        const uint8_t* q = src + (size_t)e * V.state_stride + (v.level() * kPlaneBytes + row * kMapSize + c0);
+        uint8_t* d = dst + plane * kSpan;
+        auto wanted = [&](int o, int bytes) { return c0 + o >= 0 && c0 + o < min(left + kCols, kMapSize) && c0 + o + bytes > left; };
         if (grain == 16) {
-            const int o = 16 * lane;
-            if (o < v.bytes()) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ds + o), "l"(src + o) : "memory");
+#pragma unroll
+            for (int o = 0; o < kRowSpan; o += 16)
+                if (wanted(o, 16))
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d + row_byte(dr, o))), "l"(q + o) : "memory");
         } else if (grain == 4) {
-            for (int o = 4 * lane; o < v.bytes(); o += 128)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(ds + o), "l"(src + o) : "memory");
+            for (int o = 0; o < kRowSpan; o += 4)
+                if (wanted(o, 4))
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(d + row_byte(dr, o))), "l"(q + o) : "memory");
         } else {
-            for (int o = lane; o < v.bytes(); o += 32) d[o] = ld_now(src + o);
+            for (int o = 0; o < kRowSpan; o++)
+                if (wanted(o, 1)) d[row_byte(dr, o)] = ld_now(q + o);
         }
-    };
-    plane(q + V.light_map_offset, dst[0]);
-    plane(q + V.map_offset, dst[1]);
-    plane(q + V.item_map_offset, dst[2]);
-}
+    }
+};
 __device__ __forceinline__ void wait_spans() {
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     __syncwarp();
@@ -283,11 +288,12 @@ __device__ __forceinline__ int copy_grain(const cfx_env_view& V) {
     return (a & 15) == 0 ? 16 : ((a & 3) == 0 ? 4 : 1);
 }
 
-// phase 3: the map cells of an env's record from its spans, 8 bytes each {block, item + 1, lit, five mob
-// classes} (:9241-9269).  A lane takes four cells of a row, bytes side by side in the spans.
-__device__ __forceinline__ uint32_t span_word(const uint8_t* span, int o) {   // bytes o .. o + 3
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(span + (o & ~3));
-    return __funnelshift_r(w[0], w[1], 8 * (o & 3));
+// phase 3: the map cells of an env's record from its view rows, 8 bytes each {block, item + 1, lit, five mob
+// classes} (:9241-9269).  A lane takes four cells of a row, bytes side by side.
+__device__ __forceinline__ uint32_t span_word(const uint8_t* span, int dr, int o) {   // bytes o .. o + 3 of a row
+    const uint32_t a = *reinterpret_cast<const uint32_t*>(span + row_byte(dr, o & ~3));
+    const uint32_t b = *reinterpret_cast<const uint32_t*>(span + row_byte(dr, (o & ~3) + 4));
+    return __funnelshift_r(a, b, 8 * (o & 3));
 }
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {   // (__byte_perm drops the sign bit of a selector)
     uint32_t r;
@@ -298,16 +304,16 @@ __device__ __forceinline__ uint32_t low_bytes(int k) { return k <= 0 ? 0u : (k >
 struct Cells { uint32_t w[4]; };   // first words of this lane's cells; the second ones hold mobs only
 constexpr int kGroups = (kCols + 3) / 4;
 static_assert(kRows * kGroups <= 32, "a lane a group");
-__device__ __forceinline__ Cells make_cells(View v, int lane, const uint8_t (*span)[kSpan]) {
+__device__ __forceinline__ Cells make_cells(View v, int lane, const uint8_t* span) {
     const int dr = lane / kGroups, g = lane % kGroups, row = v.top() + dr, col = v.left() + 4 * g;
     Cells c = {{0u, 0u, 0u, 0u}};
     // (a level outside [0, 9) never comes out of the env; the reference would read outside
     // its maps there, here such an env gets unlit cells)
-    if (dr >= kRows || (unsigned)row >= (unsigned)kMapSize || v.bytes() == 0 || !v.level_ok()) return c;
-    const int o = row * kMapSize + col - v.first();
+    if (dr >= kRows || (unsigned)row >= (unsigned)kMapSize || !v.level_ok()) return c;
+    const int o = (v.left() & 15) + 4 * g;   // at most 23
     const uint32_t in = low_bytes(min(kMapSize - col, kCols - 4 * g)) & ~low_bytes(-col);
-    const uint32_t lit = __vcmpgtu4(span_word(span[0], o), kLit * 0x01010101u) & in;
-    const uint32_t b = span_word(span[1], o) & lit, it = __vadd4(span_word(span[2], o), 0x01010101u) & lit;
+    const uint32_t lit = __vcmpgtu4(span_word(span, dr, o), kLit * 0x01010101u) & in;
+    const uint32_t b = span_word(span + kSpan, dr, o) & lit, it = __vadd4(span_word(span + 2 * kSpan, dr, o), 0x01010101u) & lit;
     const uint32_t one = lit & 0x01010101u, lo = __byte_perm(b, it, 0x5140), hi = __byte_perm(b, it, 0x7362);
     c.w[0] = prmt(lo, one, 0xC410);   // {block, item, lit, 0}: selector 8 + i repeats the sign of byte i, here 0
     c.w[1] = prmt(lo, one, 0xD532);
@@ -324,10 +330,10 @@ __device__ __forceinline__ void put_cells(const Cells& c, int lane, uint32_t* re
         if (4 * g + i < kCols) { d[2 * i] = c.w[i]; d[2 * i + 1] = 0u; }
 }
 // a mob whose cell is lit, or 0 (the mobs of a level are those of the light plane that was copied), and its byte
-__device__ __forceinline__ uint32_t lit_mob(View v, uint32_t pk, const uint8_t (*span)[kSpan]) {
+__device__ __forceinline__ uint32_t lit_mob(View v, uint32_t pk, const uint8_t* span) {
     if (!(pk & 0x80000000u)) return 0u;
     const int cell = (pk >> 8) & 0xFFu;
-    return span[0][(v.top() + cell / kCols) * kMapSize + v.left() + cell % kCols - v.first()] > kLit ? pk : 0u;
+    return span[row_byte(cell / kCols, (v.left() & 15) + cell % kCols)] > kLit ? pk : 0u;
 }
 __device__ __forceinline__ void put_mob(uint32_t pk, uint32_t* rec) {
     if (pk) reinterpret_cast<uint8_t*>(rec)[((pk >> 8) & 0xFFu) * 8 + ((pk >> 4) & 0xFu)] = (uint8_t)(pk & 0xFu);
@@ -352,14 +358,15 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
         top = soa(P.v.player_position, 0, n, e) - kRows / 2;
         left = soa(P.v.player_position, 1, n, e) - kCols / 2;
     }
-    const View mine = make_view(level, top, left, grain);
+    const View mine = make_view(level, top, left);
+    const CopyLane copy(P.v, lane);
+    uint8_t* const span = S.span[warp];
     const uint32_t todo = __ballot_sync(0xffffffffu, live) >> (kOwn * warp) & ((1u << kOwn) - 1u);
     View v[kOwn];   // of this warp's envs, kOwn * warp + k of the block
 #pragma unroll
     for (int k = 0; k < kOwn; k++) {
-        v[k].where = __shfl_sync(0xffffffffu, mine.where, kOwn * warp + k);
-        v[k].plane = __shfl_sync(0xffffffffu, mine.plane, kOwn * warp + k);
-        if (todo >> k & 1u) copy_spans(P.v, e0 + kOwn * warp + k, v[k], grain, lane, S.span[warp][k]);
+        v[k].bits = __shfl_sync(0xffffffffu, mine.bits, kOwn * warp + k);
+        if (todo >> k & 1u) copy.start(P.v, e0 + kOwn * warp + k, v[k], grain, span + k * kPlanes * kSpan);
     }
     if (live) gather_env(P.v, e, lane, warp, level, top, left, S);
     wait_spans();
@@ -367,16 +374,16 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
     Cells cells[kOwn];
     uint32_t mob[kOwn / 2];   // two envs at a time, 16 lanes each
 #pragma unroll
-    for (int k = 0; k < kOwn; k++) cells[k] = make_cells(v[k], lane, S.span[warp][k]);
+    for (int k = 0; k < kOwn; k++) cells[k] = make_cells(v[k], lane, span + k * kPlanes * kSpan);
 #pragma unroll
     for (int k = 0; k < kOwn; k += 2) {
         const int h = k + (lane >> 4);
         mob[k / 2] = 0u;
         if ((todo >> h & 1u) && (lane & 15) < kMobs)
-            mob[k / 2] = lit_mob(lane < 16 ? v[k] : v[k + 1], S.mobs[kOwn * warp + h][lane & 15], S.span[warp][h]);
+            mob[k / 2] = lit_mob(lane < 16 ? v[k] : v[k + 1], S.mobs[kOwn * warp + h][lane & 15], span + h * kPlanes * kSpan);
     }
-    __syncwarp();   // the spans are in registers
-    uint32_t* rec = reinterpret_cast<uint32_t*>(S.span[warp]);   // [kOwn][kRecWords]
+    __syncwarp();   // the rows are in registers
+    uint32_t* rec = reinterpret_cast<uint32_t*>(span);   // [kOwn][kRecWords]
 #pragma unroll
     for (int k = 0; k < kOwn; k++) {
         put_cells(cells[k], lane, rec + k * kRecWords);
@@ -404,7 +411,7 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
 // ------------------------------------------------------------------ list of envs
 // The envs named by a device-side list (first int32 of every entry): a few that are being reset, anywhere in
 // the batch, so what counts is the chain of dependent loads and not coalescing.  A warp takes an
-// env: entry -> every scalar, the level and the position, all lanes at once -> mobs and map spans -> record.  About 250
+// env: entry -> every scalar, the level and the position, all lanes at once -> mobs and map rows -> record.  About 250
 // entries of 65,536 envs: 26 us with a block for 32 entries, now 9.9.
 // The fields of the tail by position: which field pointer of the view, which element, how it is scaled.
 enum Scale : uint8_t { S_SQRT10, S_10, S_2, S_4, S_INT, S_F10, S_FLOAT, S_FLAG, S_DIR, S_KILLED, S_BOSS };
@@ -457,7 +464,7 @@ __device__ __forceinline__ float tail_value(const TailField& f, uint32_t raw, bo
 
 struct ListShared {
     uint32_t rec[kRecWords + 3];
-    __align__(16) uint8_t span[kPlanes][kSpan];
+    __align__(16) uint8_t span[kPlanes * kSpan];
 };
 static_assert(sizeof(ListShared) % 16 == 0, "alignment");
 constexpr int kListThreads = 128, kListWarps = kListThreads / 32;
@@ -467,6 +474,7 @@ __global__ void __launch_bounds__(kListThreads) k_record_rows_list(const __grid_
     const cfx_env_view& V = P.v;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = V.num_envs, grain = copy_grain(V);
     ListShared& S = LS[warp];
+    const CopyLane copy(V, lane);
     const TailField f0 = kTailFields[lane], f1 = kTailFields[min(lane + 32, kTail - 1)];
     wait_for_previous_kernel();
     const int count = *P.count_dev;
@@ -477,8 +485,8 @@ __global__ void __launch_bounds__(kListThreads) k_record_rows_list(const __grid_
         const int level = soa(V.player_level, 0, n, e);
         const int top = soa(V.player_position, 0, n, e) - kRows / 2, left = soa(V.player_position, 1, n, e) - kCols / 2;
         const uint32_t raw0 = tail_raw(V, f0, e), raw1 = lane + 32 < kTail ? tail_raw(V, f1, e) : 0u;
-        const View v = make_view(level, top, left, grain);
-        copy_spans(V, e, v, grain, lane, S.span);
+        const View v = make_view(level, top, left);
+        copy.start(V, e, v, grain, S.span);
         const bool killed = (unsigned)level < (unsigned)kLevels && soa(V.monsters_killed, level, n, e) >= kKilledToClear;
         // lane 3 c + i: slot i of mob class c
         const int c = lane / kSlots, slot = lane % kSlots;
