@@ -17,26 +17,26 @@ __device__ __forceinline__ float philox_uniform(uint64_t seed, uint64_t env, uin
 // cf_nn_sample_action (craftax_full.cu:9147-9165): running max, p = expf(l - m)
 // summed in ascending action order, first action whose running sum reaches
 // u * total (default A - 1), logprob = l - m - logf(total).  A is a template
-// parameter so that p[] stays in registers (draw_action takes the maximum and the exponentials as given).
-template <int A>
-__device__ __forceinline__ int draw_action(const float (&logits)[A], const float (&p)[A], float m, float u, float* logprob) {
-    float total = 0.0f;
-#pragma unroll
-    for (int a = 0; a < A; a++) total += p[a];
-    float target = u * total, cum = 0.0f;
-    int action = A - 1;
-    float la = logits[A - 1];
-    bool found = false;
+// parameter so that p[] stays in registers.
+// draw_action: p[] comes in as the exponentials.  The running sums replace them, and as they never fall, the action is the
+// number of those that the target is beyond; `at(a, beyond)` is told of every action but the last.
+template <int A, typename F>
+__device__ __forceinline__ int draw_action(float (&p)[A], float u, float* total, F&& at) {
+    float sum = 0.0f;
 #pragma unroll
     for (int a = 0; a < A; a++) {
-        cum += p[a];
-        if (!found && target <= cum) {
-            action = a;
-            la = logits[a];
-            found = true;
-        }
+        sum += p[a];
+        p[a] = sum;
     }
-    *logprob = la - m - logf(total);
+    const float target = u * sum;
+    int action = 0;
+#pragma unroll
+    for (int a = 0; a < A - 1; a++) {
+        const bool beyond = !(target <= p[a]);
+        action += beyond ? 1 : 0;
+        at(a, beyond);
+    }
+    *total = sum;
     return action;
 }
 template <int A>
@@ -47,7 +47,10 @@ __device__ __forceinline__ int sample_action(const float (&logits)[A], float u, 
     float p[A];
 #pragma unroll
     for (int a = 0; a < A; a++) p[a] = expf(logits[a] - m);
-    return draw_action<A>(logits, p, m, u, logprob);
+    float la = logits[0], total;
+    const int action = draw_action<A>(p, u, &total, [&](int a, bool beyond) { la = beyond ? logits[a + 1] : la; });
+    *logprob = la - m - logf(total);
+    return action;
 }
 
 }  // namespace cfx
