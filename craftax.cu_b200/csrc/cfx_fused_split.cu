@@ -69,6 +69,12 @@ template <int GAME, int HID, int S> struct Cfg {
     // reach from the records over the layer input, the full game's 14 lie where the state boxes are later
     static constexpr int kOffX = GAME == CFX_GAME_FULL ? kOffS : 8192;
     static_assert(kOffX + (Gm<GAME>::kEncBlocks + 3) * kQuadBlock <= kOffW + kWSlots * kWSlot && 32 * Gm<GAME>::kRecBytes <= kOffX, "operand chunks");
+    // ONE: layer input l, K block kb, [32 rows][64 K]: two buffers in turn, so that nobody waits for the multiplications of
+    // the layer before writing the next one's input; beside the records where there is room
+    static constexpr bool kOneBeside = GAME == CFX_GAME_FULL && kOffS >= 32768 + kKB * 2 * kQuadBlock;
+    static __device__ __forceinline__ uint32_t one_block(int l, int kb) {
+        return (kOneBeside ? 32768 + kb * 2 * kQuadBlock : kb * kABlock) + (l & 1) * kQuadBlock;
+    }
     static constexpr int kOffBias = kOffW + kWSlots * kWSlot;
     static constexpr int kOffBars = kOffBias + (kUnits + kHeadMax) * 4;
     static_assert(kNS >= 1 && kNS <= 2 && kUnits * S == HID && kEncTile * kEncPerItem <= kWSlot &&
@@ -266,7 +272,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                             mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
                     }
                     if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL + j));
-                    if (j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
+                    if (!ONE && j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
                     mma_commit(sm.bar(W_EMPTY + slot));
                 }
             }
@@ -314,7 +320,7 @@ __device__ __forceinline__ void role_state(const Smem& sm, const Params& P, int 
         for (int q = 0; q < quads; q++)
             tensor_g2s_2d(slot_at(b) + q * kQuadBox, &P.state_map[b / C::kBoxes], unit(b), row0 + 32 * q, sm.bar(S_FULL + b % kSSlots));
     };
-    CFX_SWAIT(REC_FREE, 0);
+    if (!(ONE && C::kOneBeside)) CFX_SWAIT(REC_FREE, 0);
     if (ONE) CFX_SWAIT(ACC_FULL, 0);   // the operand chunks are used up
     for (int b = 0; b < kSSlots && b < boxes; b++) load(b);
     for (int b = 0; b < boxes; b++) {
@@ -636,7 +642,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         __syncwarp();
         if (lane < S) mbar_arrive_cluster(map_to_cta(sm.bar(REC_FREE), (uint32_t)lane));
     };
-    if (kFull) free_records();
+    if (kFull && !C::kOneBeside) free_records();
     float u = 0.0f;
     if (draws) {   // (the counter: see role_worker)
         u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
@@ -651,7 +657,6 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     }
 
     // Layer input l: the CTA's own K block is complete when all warps are here; then it goes to the other CTAs.
-    const uint32_t own = rank * kABlock;
     auto send = [&](int l) {
         tc_fence_before_sync();
         fence_proxy_async_smem();
@@ -662,7 +667,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
             if (w == 0) {
                 ok = mbar_wait<false>(sm.bar(QUAD), l & 1, sm.abort_flag(), kSite + QUAD);
                 if (ok) {
-                    const uint32_t src = smem_u32(sm.base) + own, bar = sm.bar(A_KB + 4 * l + (int)rank);
+                    const uint32_t src = smem_u32(sm.base) + C::one_block(l, (int)rank), bar = sm.bar(A_KB + 4 * l + (int)rank);
                     mbar_arrive(bar);
 #pragma unroll
                     for (uint32_t d = 1; d < (uint32_t)S; d++) {
@@ -681,7 +686,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         uint32_t lo[16], hi[16];
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            const uint4 a = *reinterpret_cast<const uint4*>(piece(wg * kABlock, c)), b = *reinterpret_cast<const uint4*>(piece(wg * kABlock, 4 + c));
+            const uint4 a = *reinterpret_cast<const uint4*>(piece(C::one_block(l, wg), c)), b = *reinterpret_cast<const uint4*>(piece(C::one_block(l, wg), 4 + c));
             lo[4 * c] = a.x; lo[4 * c + 1] = a.y; lo[4 * c + 2] = a.z; lo[4 * c + 3] = a.w;
             hi[4 * c] = b.x; hi[4 * c + 1] = b.y; hi[4 * c + 2] = b.z; hi[4 * c + 3] = b.w;
         }
@@ -698,7 +703,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     CFX_SWAIT(ACC_FULL, 0);
     tc_fence_after_sync();
     if (!kFull) free_records();
-    CFX_SWAIT(REC_FREE, 0);
+    if (!C::kOneBeside) CFX_SWAIT(REC_FREE, 0);
     if (quadrant == 0) {
         uint32_t acc[16];
         tmem_ld16(lane_base + kColAcc + kWarpUnits * wg, acc);
@@ -712,18 +717,18 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
                 const int i = 8 * c + 2 * q;
                 h[q] = Op::pack(__uint_as_float(acc[i]) + b[i], __uint_as_float(acc[i + 1]) + b[i + 1]);
             }
-            *reinterpret_cast<uint4*>(piece(own, 2 * wg + c)) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(piece(C::one_block(0, (int)rank), 2 * wg + c)) = make_uint4(h[0], h[1], h[2], h[3]);
         }
     }
     if (!send(0)) return;
 
     // ---- layers: this thread's four units, bytes 8 (quadrant & 1) of piece 2 wg + quadrant / 2 of its row
-    uint2* xp = reinterpret_cast<uint2*>(piece(own, 2 * wg + (quadrant >> 1)) + 8 * (quadrant & 1));
+    auto xp = [&](int l) { return reinterpret_cast<uint2*>(piece(C::one_block(l, (int)rank), 2 * wg + (quadrant >> 1)) + 8 * (quadrant & 1)); };
     const int unit = kWarpUnits * wg + 4 * quadrant;
     for (int l = 0; l < P.L; l++) {
         if (!to_tmem(l)) return;
         CFX_SWAIT(A_KB + 4 * l + (int)rank, 0);
-        const uint2 x = *xp;
+        const uint2 x = *xp(l);
         const int box = l * C::kBoxes + (wg >> 1), slot = box % kSSlots;
         CFX_SWAIT(S_FULL + slot, (box / kSSlots) & 1);
         float4* sp = reinterpret_cast<float4*>(piece(C::kOffS + slot * kSBox, 4 * (wg & 1) + quadrant));
@@ -752,8 +757,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         mingru_cell_pair(__uint_as_float(zh[2]), __uint_as_float(zh[3]), __uint_as_float(zg[2]), __uint_as_float(zg[3]),
                          __uint_as_float(zp[2]), __uint_as_float(zp[3]), st.z, st.w, x23.x, x23.y, st.z, st.w, h2, h3);
         *sp = st;
-        CFX_SWAIT(MMA_DONE, l & 1);
-        *xp = make_uint2(Op::pack(h0, h1), Op::pack(h2, h3));
+        *xp(l + 1) = make_uint2(Op::pack(h0, h1), Op::pack(h2, h3));
         if (!send(l + 1)) return;
         if (lane == 0) mbar_arrive(sm.bar(ST_READY + slot));   // (send fenced the box as well)
     }
