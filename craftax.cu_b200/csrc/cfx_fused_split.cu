@@ -24,13 +24,13 @@
 // quadrant of rows would leave three schedulers idle.  The operand chunks go to shared memory instead, one of the sixteen
 // warps a chunk; and the layers' A operand is tensor memory again, where every quadrant gets a copy of the 32
 // rows: each quadrant's lanes then hold the gates of all rows, and its warps do a quarter of the units
-// (1,024 envs h256x2 15.5 -> 13.6 us).
+// (1,024 envs h256x2 15.5 -> 13.6 us).  The layer input has two buffers there, beside the records.
 // The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
-// records.  The one input buffer is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
+// records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
-// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 11.7, 1,024 25.7 -> 13.6,
-// 2,016 26 -> 16.5, 4,000 26 -> 19.2, 8,192 26.9 -> 21.6; classic h256x3, 1,024 envs 35.7 -> 16.6.  Bound by the chain of
-// dependent steps and the 3 us between one kernel's end and the next one's start.
+// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 11.6, 1,024 25.7 -> 13.0,
+// 2,016 26 -> 16.7, 4,000 26 -> 19.5, 8,192 26.9 -> 21.4; classic h256x3, 1,024 envs 35.7 -> 17.0.  Bound by the chain of
+// dependent steps and the 2.3 us between one kernel's end and the next one's start.
 #include "cfx_fused_split.h"
 
 #include <type_traits>
