@@ -120,11 +120,6 @@ __device__ __forceinline__ void bulk_s2s(uint32_t dst_cluster, uint32_t src, uin
         : "memory");
 }
 
-// the cluster barrier without memory ordering (with it the arrival waits for the stores of the outputs)
-__device__ __forceinline__ void cluster_sync_relaxed() {
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-}
 // arrives on the barrier in every CTA of the cluster when all MMAs issued so far are done
 template <int S>
 __device__ __forceinline__ void mma_commit_all(uint32_t bar) {
@@ -780,8 +775,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     const uint32_t rank = cluster_ctarank();
     const int row0 = P.tile_begin * kTile + (int)blockIdx.x / S * P.tile_rows, quads = P.tile_rows / 32;
     launch_next_kernel();
-    if (warp == 0) {   // a lane sets a barrier up
-        for (int i = lane; i < NUM_BARS; i += 32) {
+    // Set-up: a CTA that starts where one of the kernel in front has just ended has none of it under that kernel, so it counts
+    // (2,700 cycles with a few lanes setting all barriers up and everybody waiting for the cluster here).
+    // A thread sets a barrier up.
+    if (tid >= 32 * kWorkerWarp0) {
+        const int i = tid - 32 * kWorkerWarp0;
+        if (i < NUM_BARS) {
             uint32_t arrivals = 1, bytes = 0;
             if (i == REC_FREE) arrivals = ONE ? S * kWorkerWarps : S * 4 * quads;
             else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? 1 : quads;
@@ -799,16 +798,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
             fence_mbar_init();
             if (bytes) mbar_arrive_expect_tx(sm.bar(i), bytes);
         }
-        if (lane == 0) *sm.abort_flag() = 0;
-    }
-    if (warp == 3 && lane == 0)
-        for (int l = 0; l < P.L; l++) prefetch_tensormap(&P.state_map[l]);
-    if (warp == 1) {
+        static_assert(NUM_BARS < 32 * kWorkerWarps, "a thread each");
+        if (i == NUM_BARS) *sm.abort_flag() = 0;
+        __syncwarp();
+    } else if (warp == 1) {
         tmem_alloc(smem_u32(sm.tmem_base()), 512);
         tmem_relinquish();
+    } else if (warp == 3) {
+        if (lane == 0)
+            for (int l = 0; l < P.L; l++) prefetch_tensormap(&P.state_map[l]);
+        __syncwarp();
     }
+    cluster_arrive_relaxed();   // waited for below, before the first access to another CTA
     tc_fence_before_sync();
-    cluster_sync_all();   // the other CTAs' barriers are initialised before anybody copies to them
+    __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *sm.tmem_base();
 
@@ -816,7 +819,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     // read while the kernel in front still runs; everything else waits for it.
     if (warp == 0) {
         if (lane == 0) role_weights<GAME, HID, S>(sm, P, rank);
+        __syncwarp();
+        cluster_wait();
     } else if (warp == 1) {
+        cluster_wait();
         role_mma<T16, GAME, HID, S, ONE>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
     } else if (warp == 2) {
         // the tile's records, 32 rows a copy
@@ -833,11 +839,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(sm.bar(ACC_FULL));
+        __syncwarp();
+        cluster_wait();
     } else if (warp == 3) {
         wait_for_previous_kernel();
+        cluster_wait();
         if (lane == 0) role_state<GAME, HID, S, ONE>(sm, P, row0, rank);
     } else {
         wait_for_previous_kernel();
+        cluster_wait();
         if constexpr (ONE) role_worker_one<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
         else role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
     }
@@ -845,7 +855,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     // common exit, also after a timed-out wait: no CTA leaves while another may still copy to it
     __syncwarp();
     tc_fence_before_sync();
-    cluster_sync_relaxed();
+    cluster_arrive_relaxed();
+    cluster_wait();
     const uint32_t aborted = *sm.abort_flag();
     if (aborted != 0) {
         if (tid == 0) *reinterpret_cast<volatile uint32_t*>(P.status) = aborted | ((uint32_t)blockIdx.x << 8);
