@@ -732,7 +732,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         const bool valid = env < P.n;
         const bool zero_state =
             valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
-        const uint32_t zero_rows = __ballot_sync(0xffffffffu, zero_state);
 
         // ---- expand: record bytes -> 16-bit operand rows in the TMEM chunk ring.
         // Full game: wg 1 converts chunks 0-2 and the even ones after them, wg 0 (which samples
@@ -858,11 +857,13 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 const uint32_t scnt = (it * P.L + l) * kStateItems + box;
                 constexpr int kNS = C::kNS;
                 const int slot = scnt % kNS;
-                if (P.r_state != nullptr && valid) {   // under the slice's MMAs (of a warp's rows all or none are valid)
+                // under the slice's MMAs (of a warp's rows all or none are valid).  The ballot of the flags stands here and not at
+                // the tile's start, where it would wait for them: 65,536 envs h256x3 145.7 -> 142.8 us
+                if (P.r_state != nullptr && valid) {
                     CFX_WAITW(S_FULL + slot, (scnt / kNS) & 1, W_S_FULL);
                     write_r_state<8, kH>(P, sm.s_slot(slot) + quarter * 4096, 0,
                                          ((size_t)l * P.n + tile * kTile + quarter * 32) * kH + kSliceUnits * j + kHalfUnits * wg,
-                                         zero_rows, lane);
+                                         __ballot_sync(0xffffffffu, zero_state), lane);
                 }
                 {
                     uint32_t g_ok;

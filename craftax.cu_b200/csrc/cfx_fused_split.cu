@@ -357,6 +357,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     const bool samples = quadrant * min(S, quads) / quads == (int)rank;   // this CTA samples the quadrant's rows
     const unsigned long long step0 = samples && wg == 0 && P.uniforms == nullptr ? *P.step_ctr : 0ull;
     const bool zero_state = valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
+    // (the flags are waited for here, under the records' way: with the ballot at its use, 8,192 envs took 21.8 us instead of 21.3)
     const uint32_t zero_rows = __ballot_sync(0xffffffffu, zero_state);
     if (valid && lane < P.L * C::kNS) {   // this warp's rows of the state, on their way to L2 while the records are expanded
         const float* q = P.state + ((size_t)(lane / C::kNS) * P.n + env - lane) * HID + ((int)rank * C::kNS + lane % C::kNS) * kSliceUnits;
