@@ -730,8 +730,8 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         CFX_MARK(0);
         const int env = tile * kTile + row;
         const bool valid = env < P.n;
-        const bool zero_state =
-            valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
+        float terminal = 0.0f;
+        if (valid && P.prev_terminals != nullptr) terminal = P.prev_terminals[env];
 
         // ---- expand: record bytes -> 16-bit operand rows in the TMEM chunk ring.
         // Full game: wg 1 converts chunks 0-2 and the even ones after them, wg 0 (which samples
@@ -849,6 +849,8 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         // accumulator is read, the next accumulator (or the heads) while the cell's last stores
         // drain.
         CFX_PROBE_CLEAR(cfx_p_g);
+        asm volatile("" : "+f"(terminal));   // (not looked at before: the tile's start would wait for it)
+        const bool zero_state = terminal != 0.0f;
         for (int l = 0; l < P.L; l++) {
             const uint32_t a_cur = tmem + lane_base + ((l & 1) ? kColA1 : kColA0);
             const uint32_t a_next = tmem + lane_base + ((l & 1) ? kColA0 : kColA1);
