@@ -86,18 +86,10 @@ static int policy_ensure_fp32(cfx_policy* p) {
     return CFX_OK;
 }
 
-static int policy_ensure_fused(cfx_policy* p) {
-    if (p->precision == CFX_PREC_FP32) return policy_ensure_fp32(p);
-    if (!fused_supported(p->H, p->L, p->A, p->precision, p->game)) {
-        set_error("precision %d is not built for hidden=%d layers=%d actions=%d", p->precision,
-                  p->H, p->L, p->A);
-        return CFX_ERR_UNSUPPORTED;
-    }
-    if (p->fused) {
-        fused_destroy(p->fused);
-        p->fused = nullptr;
-    }
-    return fused_create(&p->fused, p->device, p->n, p->H, p->L, p->A, p->precision, p->state, p->game);
+static int require_fused(const cfx_policy* p, int precision) {
+    if (fused_supported(p->H, p->L, p->A, precision, p->game)) return CFX_OK;
+    set_error("precision %d is not built for hidden=%d layers=%d actions=%d", precision, p->H, p->L, p->A);
+    return CFX_ERR_UNSUPPORTED;
 }
 
 extern "C" {
@@ -190,7 +182,9 @@ static int policy_create(cfx_policy** out, int device, int num_envs, int hidden,
     if (e == cudaSuccess) e = cudaMemsetAsync(p->state, 0, (size_t)layers * hn * sizeof(float), p->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(p->step_ctr, 0, 2 * sizeof(unsigned long long), p->stream);
     if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__));
-    rc = policy_ensure_fused(p);
+    if (precision == CFX_PREC_FP32) rc = policy_ensure_fp32(p);
+    else if ((rc = require_fused(p, precision)) == CFX_OK)
+        rc = fused_create(&p->fused, device, num_envs, hidden, layers, num_actions, precision, p->state, game);
     if (rc) return fail(rc);
     rc = policy_refresh_mirrors(p, p->stream);
     if (rc) return fail(rc);
@@ -350,33 +344,31 @@ int cfx_policy_set_precision(cfx_policy* p, int precision) {
     if (precision == p->precision) return CFX_OK;
     CFX_GUARD(p->device);
     CFX_CUDA(cudaStreamSynchronize(p->stream));
-    const int old = p->precision;
-    p->precision = precision;
+    int rc;
+    if (precision != CFX_PREC_FP32 && (rc = require_fused(p, precision))) return rc;
+    // What the handle uses stays as it is until the new operands are complete: a refused switch leaves it untouched (a
+    // captured graph holds its pointers), and no forward reads operands that are still being written (the
+    // kernels read them before they wait for the work in front of them).
+    FusedPlan* plan = nullptr;
     if (precision == CFX_PREC_FP32) {
-        int rc = policy_ensure_fp32(p);
-        if (rc) {
-            p->precision = old;
-            return rc;
-        }
-        if (p->fused) {
-            fused_destroy(p->fused);
-            p->fused = nullptr;
-        }
-        rc = policy_refresh_mirrors(p, p->stream);
-        if (rc) return rc;
-        CFX_CUDA(cudaStreamSynchronize(p->stream));
-        return CFX_OK;
+        if ((rc = policy_ensure_fp32(p))) return rc;
+        const ArenaLayout o = ArenaLayout::make(p->H, p->L, p->A, p->obs);
+        rc = launch_transpose_gates(p->params + o.w_gru, p->gates_t, p->H, p->L, p->stream);
+    } else {
+        if ((rc = fused_create(&plan, p->device, p->n, p->H, p->L, p->A, precision, p->state, p->game))) return rc;
+        rc = fused_refresh(plan, p->params, p->stream);
     }
-    int rc = policy_ensure_fused(p);
+    if (rc == CFX_OK) {
+        const cudaError_t e = cudaStreamSynchronize(p->stream);
+        if (e != cudaSuccess) rc = cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__);
+    }
     if (rc) {
-        p->precision = old;
-        if (old != CFX_PREC_FP32) policy_ensure_fused(p);
-        if (p->fused) fused_refresh(p->fused, p->params, p->stream);
+        fused_destroy(plan);
         return rc;
     }
-    rc = fused_refresh(p->fused, p->params, p->stream);
-    if (rc) return rc;
-    CFX_CUDA(cudaStreamSynchronize(p->stream));
+    fused_destroy(p->fused);
+    p->fused = plan;
+    p->precision = precision;
     return CFX_OK;
 }
 

@@ -106,7 +106,8 @@ int cfx_policy_save_cfw1(cfx_policy* p, const char* path);
 int cfx_policy_load_cfw1(cfx_policy* p, const char* path);
 
 /* Switches the operand type (the reference's CF_GEMM_BF16 / math-mode
- * switches, craftax_full.cu:11306-11312, 12512-12514) and rebuilds mirrors. */
+ * switches, craftax_full.cu:11306-11312, 12512-12514) and rebuilds mirrors.  A
+ * switch that fails leaves the handle as it was. */
 int cfx_policy_set_precision(cfx_policy* p, int precision);
 int cfx_policy_get_precision(const cfx_policy* p);
 
