@@ -1124,9 +1124,10 @@ k_policy_fused(const __grid_constant__ Params P) {
     }
 }
 
-// Self-test of the bounded wait: one block waits on a barrier on which nothing ever arrives,
+// Self-test of the bounded wait: the first warp of a block waits on a barrier on which nothing ever arrives,
 // with a limit of a few milliseconds, gives up, and reports through the same status word
-// protocol as the forward kernel.  The kernel ends normally; the context stays usable.
+// protocol as the forward kernels.  The second warp is at the first of the two meetings it has with the first one by then,
+// and is let go.  The kernel ends normally; the context stays usable.
 constexpr uint32_t kSelftestCode = 0x7E;
 __global__ void k_selftest_wait_timeout(uint32_t* status, unsigned long long limit_ns) {
     __shared__ uint64_t bar;
@@ -1137,7 +1138,13 @@ __global__ void k_selftest_wait_timeout(uint32_t* status, unsigned long long lim
         fence_mbar_init();
     }
     __syncthreads();
-    mbar_wait(smem_u32(&bar), 0, &abort_flag, kSelftestCode, limit_ns);
+    Meetings meet;
+    if (threadIdx.x >= 32 || mbar_wait(smem_u32(&bar), 0, &abort_flag, kSelftestCode, limit_ns)) {
+        meet.sync(1, 64);
+        meet.sync(1, 64);
+    }
+    __syncwarp();
+    meet.leave(1, 64, 2);
     __syncthreads();
     if (threadIdx.x == 0 && abort_flag != 0) atomicCAS(status, 0u, abort_flag | ((uint32_t)blockIdx.x << 8));
 }

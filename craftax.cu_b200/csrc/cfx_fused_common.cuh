@@ -335,6 +335,25 @@ __device__ __forceinline__ void expand_classic(const uint8_t* rp, int kc, uint32
     }
 }
 
+// ------------------------------------------------------------------ meetings of worker warps
+// The named barriers at which a warp meets others of its block: id `first`, then the one after it, each once a launch.  A
+// named barrier has no limit, so a warp that gives up in a bounded wait before a meeting arrives there
+// on its way out (leave): nobody waits for a warp that has gone.  (Only `met` lives through the role.)
+struct Meetings {
+    int met = 0;
+    __device__ __forceinline__ void sync(int first, int threads) {
+        asm volatile("bar.sync %0, %1;" ::"r"(first + met), "r"(threads) : "memory");
+        met++;
+    }
+    __device__ __forceinline__ void arrive(int first, int threads) {
+        asm volatile("bar.arrive %0, %1;" ::"r"(first + met), "r"(threads) : "memory");
+        met++;
+    }
+    __device__ __forceinline__ void leave(int first, int threads, int meetings) {
+        while (met < meetings) arrive(first, threads);
+    }
+};
+
 // ------------------------------------------------------------------ outputs of an env
 template <int GAME, int A>
 __device__ __forceinline__ void write_logits(const Params& P, int env, const float (&logits)[A], float value) {

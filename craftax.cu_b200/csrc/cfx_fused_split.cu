@@ -339,12 +339,17 @@ __device__ __forceinline__ void hand_on(const Smem& sm, uint32_t offset, uint32_
     else bulk_s2s(map_to_cta(src, peer), src, bytes, map_to_cta(bar, peer));
 }
 
+// The CTA of rank `rank` samples the rows of quadrant `quadrant` < quads
+template <int S> __device__ __forceinline__ bool samples_rows(int quadrant, int quads, uint32_t rank) {
+    return quadrant * min(S, quads) / quads == (int)rank;
+}
+
 // ------------------------------------------------------------------ workers
 // Sixteen warps: warp (quadrant, wg) owns TMEM lanes [32 quadrant, + 32) = those rows of the tile, converts
 // chunks wg, wg + 4, ... and handles units [16 wg, 16 wg + 16) of every slice of the CTA.
 template <typename T16, int GAME, int HID, int S>
 __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
-                                            uint32_t rank) {
+                                            uint32_t rank, Meetings& meet) {
     using Op = Op16<T16>;
     using C = Cfg<GAME, HID, S>;
     constexpr int kChunks = Gm<GAME>::kEncChunks, kA = Gm<GAME>::kA;
@@ -354,7 +359,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     if (quadrant >= quads) return;   // (rows that nobody reads)
     const bool valid = env < P.n;   // of a quadrant all rows or none (n is a multiple of 32)
     const float* bias = reinterpret_cast<const float*>(sm.base + C::kOffBias);
-    const bool samples = quadrant * min(S, quads) / quads == (int)rank;   // this CTA samples the quadrant's rows
+    const bool samples = samples_rows<S>(quadrant, quads, rank);
     const unsigned long long step0 = samples && wg == 0 && P.uniforms == nullptr ? *P.step_ctr : 0ull;
     const bool zero_state = valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
     // (the flags are waited for here, under the records' way: with the ballot at its use, 8,192 envs took 21.8 us instead of 21.3)
@@ -533,7 +538,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         for (int a = 0; a < kA; a++)
             if (a / kPart == wg) p[a * kTile] = expf(logits[a] - m);
         if (wg == 1 && valid) write_logits<GAME>(P, env, logits, value);
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + quadrant) : "memory");
+        meet.sync(1 + quadrant, 128);
         if (wg == 0 && valid) {
             float pr[kA];
 #pragma unroll
@@ -551,7 +556,8 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
 // whole row, and a sixteenth of the exponentials, 1,024 envs took 14.3 us instead of 13.8.
 // `head`: tensor memory of this warp's lanes, `env`: of the lane; `u`: its uniform, in the first warp
 template <int GAME>
-__device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t head, const float* bias, int w, int lane, int env, float u) {
+__device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t head, const float* bias, int w, int lane, int env, float u,
+                                           Meetings& meet) {
     constexpr int kA = Gm<GAME>::kA, kCols = 4, kWith = (kA + kCols) / kCols, kPitch = 33, W = kWorkerWarps;
     static_assert(kWith <= W && ((kA + 1) * kPitch + (kA + kWith) * 32) * 4 <= kWSlots * kWSlot, "scratch");
     float* p = s + (kA + 1) * kPitch + lane;   // logits [kA + 1][33], exponentials [kA][32], maxima [kWith][32]
@@ -570,7 +576,7 @@ __device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t h
         }
         most[w * 32] = m;
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory");
+    meet.sync(1, 32 * W);
     if (w < kWith) {
 #pragma unroll
         for (int i = 0; i < kWith; i++) m = fmaxf(m, most[i * 32]);
@@ -579,13 +585,13 @@ __device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t h
             if (kCols * w + i < kA) p[(kCols * w + i) * 32] = expf(l[i] - m);
     }
     if (w != 0) {
-        asm volatile("bar.arrive 1, %0;" ::"n"(32 * W) : "memory");
+        meet.arrive(1, 32 * W);
         if (P.logits_av != nullptr) {   // 32 rows, contiguous
             float* dst = P.logits_av + (size_t)(env - lane) * (kA + 1);
             for (int i = 32 * (w - 1) + lane; i < 32 * (kA + 1); i += 32 * (W - 1)) dst[i] = s[i % (kA + 1) * kPitch + i / (kA + 1)];
         }
     } else {
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory");
+        meet.sync(1, 32 * W);
         float pr[kA], total;
 #pragma unroll
         for (int a = 0; a < kA; a++) pr[a] = p[a * 32];
@@ -599,7 +605,7 @@ __device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t h
 // slice; lane = row in all of it.
 template <typename T16, int GAME, int HID, int S>
 __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
-                                                uint32_t rank) {
+                                                uint32_t rank, Meetings& meet) {
     using Op = Op16<T16>;
     using C = Cfg<GAME, HID, S>;
     constexpr int kChunks = Gm<GAME>::kEncChunks, kA = Gm<GAME>::kA;
@@ -757,7 +763,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     if (rank == 0) {
         CFX_SWAIT(H_FULL, 0);
         tc_fence_after_sync();
-        if (valid) sample_one<GAME>(P, reinterpret_cast<float*>(sm.base + C::kOffW), lane_base + kColHead, bias + C::kUnits, w, lane, env, u);
+        if (valid) sample_one<GAME>(P, reinterpret_cast<float*>(sm.base + C::kOffW), lane_base + kColHead, bias + C::kUnits, w, lane, env, u, meet);
     }
 }
 
@@ -849,8 +855,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     } else {
         wait_for_previous_kernel();
         cluster_wait();
-        if constexpr (ONE) role_worker_one<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
-        else role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank);
+        Meetings meet;
+        if constexpr (ONE) role_worker_one<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank, meet);
+        else role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank, meet);
+        // (meetings are left over only where a wait gave up)
+        __syncwarp();
+        const int quadrant = warp & 3;
+        if constexpr (ONE) {
+            if (rank == 0 && row0 < P.n) meet.leave(1, 32 * kWorkerWarps, 2);
+        } else {
+            if (quadrant < quads && samples_rows<S>(quadrant, quads, rank)) meet.leave(1 + quadrant, 128, 1);
+        }
     }
 
     // common exit, also after a timed-out wait: no CTA leaves while another may still copy to it
