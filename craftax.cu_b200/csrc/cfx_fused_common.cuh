@@ -338,8 +338,10 @@ __device__ __forceinline__ void expand_classic(const uint8_t* rp, int kc, uint32
 // ------------------------------------------------------------------ meetings of worker warps
 // The named barriers at which a warp meets others of its block: id `first`, then the one after it, each once a launch.  A
 // named barrier has no limit, so a warp that gives up in a bounded wait before a meeting arrives there
-// on its way out (leave): nobody waits for a warp that has gone.  (Only `met` lives through the role.)
+// on its way out (leave): nobody waits for a warp that has gone.  (Only `met` lives through the role, and what a warp that
+// gave up still owes is worked out for such a warp alone: 4,000 envs 19.55 us so, 19.85 with every warp working it out.)
 struct Meetings {
+    static constexpr int kAll = 255;   // the role has come to its end
     int met = 0;
     __device__ __forceinline__ void sync(int first, int threads) {
         asm volatile("bar.sync %0, %1;" ::"r"(first + met), "r"(threads) : "memory");

@@ -17,7 +17,7 @@
 //   state     boxes of 128 rows x 32 units by tensor copies, updated in place and written back (a thread's own
 //             64 bytes of a row, read and written by the threads, kept the load/store unit busy for 4,000 cycles a
 //             layer and with it every barrier operation of the SM)
-//   heads     in every CTA, over all rows; the quadrants of rows are sampled in different CTAs
+//   heads     in the CTAs that sample, over all rows; the quadrants of rows are sampled in different CTAs
 // The cluster works on one tile and exits, so every barrier but those of the rings is used once or once a
 // layer.  The products of a row are accumulated in the order of cfx_fused.cu: same bits.
 // Tiles of 32 rows (ONE), the smallest batches: a quadrant of TMEM lanes belongs to one SM scheduler, so one
@@ -129,15 +129,27 @@ __device__ __forceinline__ void mma_commit_all(uint32_t bar) {
         : "memory");
 }
 
+// The first min(S, quads) CTAs sample, one or two quadrants of rows each.  The others multiply no heads: nobody there
+// would wait for the products, and a CTA must not leave while its multiplications run.
+template <int S> __device__ __forceinline__ bool samples_rows(int quadrant, int quads, uint32_t rank) {
+    return quadrant * min(S, quads) / quads == (int)rank;
+}
+template <int S, bool ONE> __device__ __forceinline__ bool has_heads(int quads, uint32_t rank) {
+    if constexpr (ONE) return rank == 0;
+    else if constexpr (S == 2) return true;   // a tile of more than 32 rows has two quadrants or more
+    else return (int)rank < min(S, quads);
+}
+
 // ------------------------------------------------------------------ weights
 // The operand image is the one the CTA pairs of cfx_fused.cu use: stages of two blocks, every block in two halves of
 // rows.  A CTA's rows of an encoder block are contiguous in it, a gate K block is two pieces.
-template <int GAME, int HID, int S>
+template <int GAME, int HID, int S, bool ONE>
 __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, uint32_t rank) {
     using C = Cfg<GAME, HID, S>;
     constexpr int kSlices = HID / 64, kHalf = HID / 2;
     constexpr size_t enc_b = enc_bytes<GAME, HID>();
-    const int gates = P.L * C::kNS * C::kKB, items = C::kEncItems + gates + C::kHeadItems;
+    const int gates = P.L * C::kNS * C::kKB;
+    const int items = C::kEncItems + gates + (has_heads<S, ONE>(P.tile_rows / 32, rank) ? C::kHeadItems : 0);
     const uint32_t ring = smem_u32(sm.base + C::kOffW);
     for (int i = 0; i < items; i++) {
         const int slot = i % kWSlots;
@@ -273,6 +285,14 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
             }
         }
     }
+    if (__builtin_expect(!has_heads<S, ONE>(P.tile_rows / 32, rank), 0)) {
+        // no heads here: what is on its way to this CTA (the last layer's output) or was issued by it is only waited for
+        for (int kb = 0; kb < C::kKB; kb++) CFX_SWAIT(A_KB + 4 * P.L + kb, 0);
+        __syncwarp();
+        if (elect_one()) mma_commit(sm.bar(H_FULL));
+        CFX_SWAIT(H_FULL, 0);
+        return;
+    }
     const int slot0 = first_slot(P.L);
     CFX_SPROBE(cfx_p_a, ONE ? (int)AT_KB : A_KB + 4 * P.L, ONE ? P.L & 1 : 0);
 #pragma unroll
@@ -339,11 +359,6 @@ __device__ __forceinline__ void hand_on(const Smem& sm, uint32_t offset, uint32_
     else bulk_s2s(map_to_cta(src, peer), src, bytes, map_to_cta(bar, peer));
 }
 
-// The CTA of rank `rank` samples the rows of quadrant `quadrant` < quads
-template <int S> __device__ __forceinline__ bool samples_rows(int quadrant, int quads, uint32_t rank) {
-    return quadrant * min(S, quads) / quads == (int)rank;
-}
-
 // ------------------------------------------------------------------ workers
 // Sixteen warps: warp (quadrant, wg) owns TMEM lanes [32 quadrant, + 32) = those rows of the tile, converts
 // chunks wg, wg + 4, ... and handles units [16 wg, 16 wg + 16) of every slice of the CTA.
@@ -356,7 +371,10 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     const int quadrant = warp & 3, wg = (warp - kWorkerWarp0) >> 2, row = quadrant * 32 + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(quadrant * 32) << 16);
     const int env = row0 + row, quads = P.tile_rows / 32;
-    if (quadrant >= quads) return;   // (rows that nobody reads)
+    if (quadrant >= quads) {   // (rows that nobody reads)
+        meet.met = Meetings::kAll;
+        return;
+    }
     const bool valid = env < P.n;   // of a quadrant all rows or none (n is a multiple of 32)
     const float* bias = reinterpret_cast<const float*>(sm.base + C::kOffBias);
     const bool samples = samples_rows<S>(quadrant, quads, rank);
@@ -548,6 +566,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             write_action(P, env, act, la - m - logf(total), value);
         }
     }
+    meet.met = Meetings::kAll;
 }
 
 // ONE: the sampler of 32 rows by all warps, lane = row in each: a warp brings four columns of the logits, their maximum and their
@@ -757,14 +776,15 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         if (!send(l + 1)) return;
         if (lane == 0) mbar_arrive(sm.bar(ST_READY + slot));   // (send fenced the box as well)
     }
-    if (!to_tmem(P.L)) return;
 
     // ---- heads + sampler: all warps, each with the rows in its quadrant
     if (rank == 0) {
+        if (!to_tmem(P.L)) return;
         CFX_SWAIT(H_FULL, 0);
         tc_fence_after_sync();
         if (valid) sample_one<GAME>(P, reinterpret_cast<float*>(sm.base + C::kOffW), lane_base + kColHead, bias + C::kUnits, w, lane, env, u, meet);
     }
+    meet.met = Meetings::kAll;
 }
 
 // ------------------------------------------------------------------ kernel
@@ -825,7 +845,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     // The operand image and the biases are only ever written by calls that wait for the device, so they may be
     // read while the kernel in front still runs; everything else waits for it.
     if (warp == 0) {
-        if (lane == 0) role_weights<GAME, HID, S>(sm, P, rank);
+        if (lane == 0) role_weights<GAME, HID, S, ONE>(sm, P, rank);
         __syncwarp();
         cluster_wait();
     } else if (warp == 1) {
@@ -858,13 +878,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         Meetings meet;
         if constexpr (ONE) role_worker_one<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank, meet);
         else role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank, meet);
-        // (meetings are left over only where a wait gave up)
         __syncwarp();
-        const int quadrant = warp & 3;
-        if constexpr (ONE) {
-            if (rank == 0 && row0 < P.n) meet.leave(1, 32 * kWorkerWarps, 2);
-        } else {
-            if (quadrant < quads && samples_rows<S>(quadrant, quads, rank)) meet.leave(1 + quadrant, 128, 1);
+        if (__builtin_expect(meet.met != Meetings::kAll, 0)) {   // a wait gave up
+            const int quadrant = warp & 3;
+            if constexpr (ONE) {
+                if (rank == 0 && row0 < P.n) meet.leave(1, 32 * kWorkerWarps, 2);
+            } else {
+                if (samples_rows<S>(quadrant, quads, rank)) meet.leave(1 + quadrant, 128, 1);
+            }
         }
     }
 
