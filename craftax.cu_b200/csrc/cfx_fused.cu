@@ -1112,24 +1112,17 @@ k_policy_fused(const __grid_constant__ Params P) {
         if (PAIR) tmem_dealloc_pair(tmem, 512);
         else tmem_dealloc(tmem, 512);
     }
-    // The reference bumps the sampler offset with a one-thread kernel after the step
-    // (k_bump_ctr, craftax_full.cu:12085).  Here the last block to finish does it: every block
-    // read the counter (in its sampler threads) before it got here.
-    if (tid == 0 && P.bump_step) {
-        __threadfence();
-        if (atomicAdd(P.done_ctr, 1u) == P.done_blocks - 1) {
-            *P.step_ctr += 1ULL;
-            *P.done_ctr = 0u;
-        }
-    }
+    // every block read the counter (in its sampler threads) before it got here
+    if (tid == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
 }
 
 // Self-test of the bounded wait: the first warp of a block waits on a barrier on which nothing ever arrives,
 // with a limit of a few milliseconds, gives up, and reports through the same status word
 // protocol as the forward kernels.  The second warp is at the first of the two meetings it has with the first one by then,
-// and is let go.  The kernel ends normally; the context stays usable.
+// and is let go; it alone has said that it is done with the step counter.  The kernel ends normally; the context stays
+// usable.
 constexpr uint32_t kSelftestCode = 0x7E;
-__global__ void k_selftest_wait_timeout(uint32_t* status, unsigned long long limit_ns) {
+__global__ void k_selftest_wait_timeout(uint32_t* status, uint32_t* done, unsigned long long limit_ns) {
     __shared__ uint64_t bar;
     __shared__ uint32_t abort_flag;
     if (threadIdx.x == 0) {
@@ -1140,31 +1133,64 @@ __global__ void k_selftest_wait_timeout(uint32_t* status, unsigned long long lim
     __syncthreads();
     Meetings meet;
     if (threadIdx.x >= 32 || mbar_wait(smem_u32(&bar), 0, &abort_flag, kSelftestCode, limit_ns)) {
+        if ((threadIdx.x & 31) == 0) done_with_step(nullptr, done, 2);
         meet.sync(1, 64);
         meet.sync(1, 64);
     }
     __syncwarp();
     meet.leave(1, 64, 2);
     __syncthreads();
-    if (threadIdx.x == 0 && abort_flag != 0) atomicCAS(status, 0u, abort_flag | ((uint32_t)blockIdx.x << 8));
+    if (threadIdx.x == 0 && abort_flag != 0) *reinterpret_cast<volatile uint32_t*>(status) = abort_flag | ((uint32_t)blockIdx.x << 8);
 }
 
 }  // namespace fused
 
+// What a wait that gave up leaves behind, and how the host takes note of it
+struct WaitStatus {
+    uint32_t* status = nullptr;    // status word, in page-locked host memory: the host reads it without a copy
+    uint32_t* done_ctr = nullptr;  // see done_with_step
+    cudaError_t create() {
+        cudaError_t e = cudaMalloc((void**)&done_ctr, sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMemset(done_ctr, 0, sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaHostAlloc((void**)&status, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+        if (e == cudaSuccess) *status = 0;
+        return e;
+    }
+    // The kernels in question have been waited for.  Their warps that gave up may not have counted.
+    unsigned take() {
+        volatile uint32_t* word = status;
+        const uint32_t v = *word;
+        if (v != 0) {
+            *word = 0;
+            if (cudaMemset(done_ctr, 0, sizeof(uint32_t)) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess)
+                cudaGetLastError();   // (a context that is gone; the caller reports the time-out)
+        }
+        return v;
+    }
+    void destroy() {
+        if (status) cudaFreeHost(status);
+        if (done_ctr) cudaFree(done_ctr);
+    }
+};
+
 int fused_selftest_wait_timeout(unsigned limit_ms, unsigned* status_out) {
-    uint32_t* d = nullptr;
-    CFX_CUDA(cudaMalloc((void**)&d, sizeof(uint32_t)));
-    cudaError_t e = cudaMemset(d, 0, sizeof(uint32_t));
+    WaitStatus w;
+    cudaError_t e = w.create();
     if (e == cudaSuccess) {
-        fused::k_selftest_wait_timeout<<<1, 64>>>(d, (unsigned long long)limit_ms * 1000000ull);
+        fused::k_selftest_wait_timeout<<<1, 64>>>(w.status, w.done_ctr, (unsigned long long)limit_ms * 1000000ull);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    uint32_t v = 0;
-    if (e == cudaSuccess) e = cudaMemcpy(&v, d, sizeof(v), cudaMemcpyDeviceToHost);
-    cudaFree(d);
+    uint32_t before = 0, after = 1;
+    if (e == cudaSuccess) e = cudaMemcpy(&before, w.done_ctr, sizeof(before), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) *status_out = w.take();
+    if (e == cudaSuccess) e = cudaMemcpy(&after, w.done_ctr, sizeof(after), cudaMemcpyDeviceToHost);
+    w.destroy();
     if (e != cudaSuccess) return cuda_fail(e, "selftest", __FILE__, __LINE__);
-    *status_out = v;
+    if (before != 1 || after != 0) {
+        set_error("self-test: the count of a launch that gave up is %u, and %u after the check (1 and 0 expected)", before, after);
+        return CFX_ERR_CUDA;
+    }
     return CFX_OK;
 }
 
@@ -1173,8 +1199,7 @@ struct FusedPlan {
     int device, n, H, L, A, precision;
     int game = CFX_GAME_FULL;
     uint8_t* image = nullptr;
-    uint32_t* status = nullptr;    // status word, in page-locked host memory: the host reads it without a copy
-    uint32_t* done_ctr = nullptr;  // finished-block counter
+    WaitStatus wait;
     float* state = nullptr;
     const float* params = nullptr;
     CUtensorMap state_map[fused::kMaxLayers];
@@ -1246,10 +1271,7 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
     p->state = state;
     p->sm_count = sm_count;
     cudaError_t e = cudaMalloc((void**)&p->image, fused_image_bytes(game, H, L));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&p->done_ctr, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(p->done_ctr, 0, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaHostAlloc((void**)&p->status, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped);
-    if (e == cudaSuccess) *p->status = 0;
+    if (e == cudaSuccess) e = p->wait.create();
     if (e != cudaSuccess) {
         fused_destroy(p);
         return cuda_fail(e, "fused_create alloc", __FILE__, __LINE__);
@@ -1384,8 +1406,8 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     P.r_state = a.r_state;
     P.r_state_bf16 = a.r_state_bf16;
     P.step_ctr = a.step_ctr;
-    P.status = p->status;
-    P.done_ctr = p->done_ctr;
+    P.status = p->wait.status;
+    P.done_ctr = p->wait.done_ctr;
     P.bump_step = a.bump_step;
     P.seed = a.seed;
     P.env_offset = a.env_offset;
@@ -1447,18 +1469,12 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     return CFX_OK;
 }
 
-unsigned fused_take_status(FusedPlan* p) {
-    volatile uint32_t* word = p->status;
-    const uint32_t v = *word;
-    if (v != 0) *word = 0;
-    return v;
-}
+unsigned fused_take_status(FusedPlan* p) { return p->wait.take(); }
 
 void fused_destroy(FusedPlan* p) {
     if (!p) return;
     if (p->image) cudaFree(p->image);
-    if (p->status) cudaFreeHost(p->status);
-    if (p->done_ctr) cudaFree(p->done_ctr);
+    p->wait.destroy();
     delete p;
 }
 

@@ -105,7 +105,7 @@ struct Params {
     int r_state_bf16;                    // the record holds bf16 instead of fp32
     unsigned long long* step_ctr;        // device step counter (Philox offset); see bump_step
     uint32_t* status;
-    uint32_t* done_ctr;                  // blocks that have finished this launch (bump_step)
+    uint32_t* done_ctr;                  // blocks that are done with the step counter (bump_step)
     uint32_t done_blocks;                // how many there are (small-batch form: warps that need the counter)
     int bump_step;
     uint64_t seed, env_offset;
@@ -332,6 +332,18 @@ __device__ __forceinline__ void expand_classic(const uint8_t* rp, int kc, uint32
         for (int q = 22; q < 32; q++) regs[q] = Op::pack(sc[2 * (q - 22) + 1], sc[2 * (q - 22) + 2]);
     } else if (kc == kEncChunks - 1) {   // feature 1344: sleeping
         regs[0] = rp[2 * kClassicCells + 17] != 0 ? Op::kOne : 0u;
+    }
+}
+
+// ------------------------------------------------------------------ step counter
+// The reference bumps the sampler offset with a one-thread kernel after the step (k_bump_ctr, craftax_full.cu:12085).  Here
+// the last of `readers` to say that it has read the counter raises it.  A launch in which one gave up before it came to that
+// leaves the count where it is: WaitStatus::take clears it.
+__device__ __forceinline__ void done_with_step(unsigned long long* step, uint32_t* done, uint32_t readers) {
+    __threadfence();
+    if (atomicAdd(done, 1u) == readers - 1) {
+        *step += 1ULL;
+        *done = 0u;
     }
 }
 

@@ -432,13 +432,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         if (valid)
             u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
         __syncwarp();
-        if (lane == 0 && P.bump_step) {
-            __threadfence();
-            if (atomicAdd(P.done_ctr, 1u) == P.done_blocks - 1) {
-                *P.step_ctr += 1ULL;
-                *P.done_ctr = 0u;
-            }
-        }
+        if (lane == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
     }
 
     // Hands this thread's 16 units of layer input l, slice j, on: into the own K block, and, once the quadrant's four
@@ -670,13 +664,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     if (draws) {   // (the counter: see role_worker)
         u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
         __syncwarp();
-        if (lane == 0 && P.bump_step) {
-            __threadfence();
-            if (atomicAdd(P.done_ctr, 1u) == P.done_blocks - 1) {
-                *P.step_ctr += 1ULL;
-                *P.done_ctr = 0u;
-            }
-        }
+        if (lane == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
     }
 
     // Layer input l: the CTA's own K block is complete when all warps are here; then it goes to the other CTAs.
