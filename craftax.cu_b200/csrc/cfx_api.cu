@@ -7,6 +7,7 @@
 #include "cfx_common.cuh"
 #include "cfx_fused.h"
 #include "cfx_strict.h"
+#include "cfx_tmap.h"
 
 namespace cfx {
 
@@ -520,14 +521,24 @@ static int check_status(cfx_policy* p) {
     return CFX_ERR_DEVICE_TIMEOUT;
 }
 
-// The device's address of page-locked host memory, or NULL.
-static void* device_address(const void* host) {
+// The device's address of [host, host + bytes) where all of it lies in one piece of page-locked memory (allocated, or
+// registered as a whole), or NULL: a kernel that went past the end of such a piece would fault.
+static void* device_address(const void* host, size_t bytes) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+    if (a.type != cudaMemoryTypeHost || a.devicePointer == nullptr) return nullptr;
+    typedef CUresult (*PFN_attribute)(void*, CUpointer_attribute, CUdeviceptr);
+    static const PFN_attribute attribute = (PFN_attribute)driver_entry("cuPointerGetAttribute");
+    const uintptr_t at = (uintptr_t)a.devicePointer;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (attribute == nullptr || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)at) != CUDA_SUCCESS ||
+        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)at) != CUDA_SUCCESS)
+        return nullptr;
+    return at >= start && at - start <= size && bytes <= size - (at - start) ? a.devicePointer : nullptr;
 }
 
 // Small batches, fused kernel: what such a step costs is calls and round trips, not bytes.  Flags, uniforms and the four
@@ -556,13 +567,13 @@ static int forward_host_small(cfx_policy* p, const cfx_forward_io* h, cfx_forwar
     d->actions = (int32_t*)part(3);
     d->logprobs = h->logprobs ? (float*)part(4) : nullptr;
     d->values = h->values ? (float*)part(5) : nullptr;
-    void* logits = h->logits_av && n <= kHostLogitsEnvs ? device_address(h->logits_av) : nullptr;
+    void* logits = h->logits_av && n <= kHostLogitsEnvs ? device_address(h->logits_av, n * row) : nullptr;
     if (logits && ((uintptr_t)logits & 15) != 0) logits = nullptr;
     const bool staged = h->logits_av && !logits && n <= kHostLogitsCopyEnvs;
     if (staged) logits = part(6);
     if (logits) d->logits_av = (float*)logits;
     const size_t bytes = n * (size_t)p->rec_bytes;
-    const void* rec = n <= kHostFetchEnvs ? device_address(h->records) : nullptr;
+    const void* rec = n <= kHostFetchEnvs ? device_address(h->records, bytes) : nullptr;
     int rc;
     if (rec && ((uintptr_t)rec & 15) == 0) {
         if ((rc = launch_fetch(rec, p->st_records, bytes, st))) return rc;

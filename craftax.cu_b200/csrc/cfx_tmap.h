@@ -1,5 +1,5 @@
-// Host-side construction of TMA tensor maps through the driver entry point
-// (no link-time dependency on libcuda).
+// Functions of the driver through their entry points (no link-time dependency on libcuda), and the
+// host-side construction of TMA tensor maps.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -12,15 +12,16 @@ typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_
                                     const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+// A function of the driver, or NULL
+inline void* driver_entry(const char* name) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? p : nullptr;
+}
+
 inline PFN_encodeTiled get_encode_tiled() {
     static PFN_encodeTiled fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (PFN_encodeTiled)p;
-    }
+    if (!fn) fn = (PFN_encodeTiled)driver_entry("cuTensorMapEncodeTiled");
     return fn;
 }
 
