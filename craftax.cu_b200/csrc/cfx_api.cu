@@ -139,8 +139,8 @@ static int policy_create(cfx_policy** out, int device, int num_envs, int hidden,
     *out = nullptr;
     CFX_REQUIRE(num_envs > 0 && num_envs % 32 == 0,
                 "cfx_policy_create: num_envs=%d must be a positive multiple of 32", num_envs);
-    CFX_REQUIRE(hidden >= 32 && hidden <= 512 && hidden % 32 == 0,
-                "cfx_policy_create: hidden=%d must be a multiple of 32 in [32,512]", hidden);
+    CFX_REQUIRE(hidden >= 32 && hidden <= kMaxHidden && hidden % 32 == 0,
+                "cfx_policy_create: hidden=%d must be a multiple of 32 in [32,%d]", hidden, kMaxHidden);
     CFX_REQUIRE(layers >= 1 && layers <= 8, "cfx_policy_create: layers=%d out of [1,8]", layers);
     CFX_REQUIRE(num_actions >= 2 && num_actions <= kMaxActions,
                 "cfx_policy_create: num_actions=%d out of [2,%d]", num_actions, kMaxActions);

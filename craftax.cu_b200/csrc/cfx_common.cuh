@@ -15,6 +15,7 @@ constexpr int kMap = CFX_OBS_MAP;        // 792 one-byte map features
 constexpr int kTail = CFX_OBS_TAIL;      // 51 raw fp32 tail features
 constexpr int kRec = CFX_RECORD_BYTES;   // 996-byte record
 constexpr int kMaxActions = 63;
+constexpr int kMaxHidden = 512;
 // classic game (reference craftax_classic.cu:38-59): 148-byte record, 1345 features
 constexpr int kClassicRec = CFX_CLASSIC_RECORD_BYTES, kClassicObs = CFX_CLASSIC_OBS_FEATURES;
 constexpr int kClassicCells = 63, kClassicBlocks = 17, kClassicInv = 12;
@@ -105,18 +106,20 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
     return CFX_OK;
 }
 
-// A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per device
+// A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per device.  kMost is the most
+// that the kernel is ever launched with, one value a kernel: host threads that come here at the same time with
+// different shapes all set the same.
 // (`static`: a process that has loaded two builds of the library sets them for the kernels of each)
-template <auto kernel>
-static int allow_smem(int smem) {
+template <auto kernel, int kMost>
+static int allow_smem() {
     constexpr int kMaxDevices = 64;
-    static std::atomic<int> done[kMaxDevices];   // the largest size allowed so far
+    static std::atomic<bool> done[kMaxDevices];
     int dev = 0;
     CFX_CUDA(cudaGetDevice(&dev));
-    if (dev < kMaxDevices && done[dev].load(std::memory_order_relaxed) >= smem) return CFX_OK;
-    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (dev < kMaxDevices && done[dev].load(std::memory_order_relaxed)) return CFX_OK;
+    CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
     CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    if (dev < kMaxDevices) done[dev].store(smem, std::memory_order_relaxed);
+    if (dev < kMaxDevices) done[dev].store(true, std::memory_order_relaxed);
     return CFX_OK;
 }
 #endif

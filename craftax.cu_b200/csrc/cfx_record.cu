@@ -685,7 +685,7 @@ extern "C" int cfx_record_obs(int device, const cfx_env_view* view, uint8_t* rec
     P.n = n;
     P.skip = skip;
     const unsigned blocks = (unsigned)((n + record::kBlockEnvs - 1) / record::kBlockEnvs);
-    if ((rc = allow_smem<record::k_record_rows>((int)sizeof(record::Shared)))) return rc;
+    if ((rc = allow_smem<record::k_record_rows, (int)sizeof(record::Shared)>())) return rc;
     return launch_chained(record::k_record_rows, dim3(blocks), record::kBlockThreads, sizeof(record::Shared), (cudaStream_t)stream, P);
 }
 

@@ -737,7 +737,7 @@ static int strict_encoder_tile(long long q) { return q >= 640 ? 82 : (q >= 400 ?
 template <int TM, int G>
 static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, int early, cudaStream_t st) {
     using E = Enc<TM, G>;
-    int rc = allow_smem<k_encoder_fp32<TM, G>>(E::kSmem);
+    int rc = allow_smem<k_encoder_fp32<TM, G>, E::kSmem>();
     if (rc) return rc;
     return launch_chained(k_encoder_fp32<TM, G>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
                           a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], a.n, a.H,
@@ -749,7 +749,7 @@ static int strict_layers(const StrictArgs& a, int early, cudaStream_t st) {
     const int H = a.H, n = a.n;
     constexpr int BM = 4 * TM * WM, BU = 32 * WU, T = 32 * WM * WU;
     constexpr int smem = ST * gru_stage_floats<TM, WM, WU>() * (int)sizeof(float);
-    int rc = allow_smem<k_mingru_fp32<TM, WM, WU, ST>>(smem);
+    int rc = allow_smem<k_mingru_fp32<TM, WM, WU, ST>, smem>();
     if (rc) return rc;
     const dim3 grid((n + BM - 1) / BM, H / BU);
     const int s_aligned = ((uintptr_t)a.state & 15) == 0;
@@ -794,7 +794,7 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
                                                                  : strict_layers<1, 4, 1, 4>(a, early, st);
     if (rc) return rc;
     const size_t hsmem = head_smem(H, A);
-    if ((rc = allow_smem<k_heads_fp32>((int)hsmem))) return rc;
+    if ((rc = allow_smem<k_heads_fp32, (int)head_smem(kMaxHidden, kMaxActions)>())) return rc;
     rc = launch_chained(k_heads_fp32, dim3(n / kHeadEnvs), head_threads(A), hsmem, st, a.scratch_h[L & 1],
                         a.params + o.w_a, a.params + o.b_a, a.params + o.w_v, a.params + o.b_v, a.logits_av, n, H, A, early);
     if (rc) return rc;
