@@ -25,6 +25,13 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
     return CFX_ERR_CUDA;
 }
 
+unsigned long long current_context_id() {
+    typedef CUresult (*PFN_id)(CUcontext, unsigned long long*);
+    static const PFN_id get = (PFN_id)driver_entry("cuCtxGetId");
+    unsigned long long id = 0;
+    return get != nullptr && get(nullptr, &id) == CUDA_SUCCESS ? id : 0ull;
+}
+
 }  // namespace cfx
 
 using namespace cfx;

@@ -80,6 +80,9 @@ struct DeviceGuard {
         }                                                                                \
     } while (0)
 
+// The current context's number, unique in the process, or 0 where it cannot be told (before the first use of a device).
+unsigned long long current_context_id();
+
 // Kernels launched with programmatic stream serialisation: the launch and the start-up of a kernel run
 // under the kernel in front of it in the stream, and it waits here until the results of that kernel are in
 // memory.  Nothing that another kernel may have written is read before.  Only kernels of few blocks
@@ -106,20 +109,18 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
     return CFX_OK;
 }
 
-// A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per device.  kMost is the most
-// that the kernel is ever launched with, one value a kernel: host threads that come here at the same time with
-// different shapes all set the same.
+// A kernel's dynamic shared memory limit and its preference for shared memory over L1, set once per context (they go with it: after
+// cudaDeviceReset they are set again).  kMost is the most that the kernel is ever launched with, one value a kernel: host
+// threads that come here at the same time with different shapes all set the same.
 // (`static`: a process that has loaded two builds of the library sets them for the kernels of each)
 template <auto kernel, int kMost>
 static int allow_smem() {
-    constexpr int kMaxDevices = 64;
-    static std::atomic<bool> done[kMaxDevices];
-    int dev = 0;
-    CFX_CUDA(cudaGetDevice(&dev));
-    if (dev < kMaxDevices && done[dev].load(std::memory_order_relaxed)) return CFX_OK;
+    static std::atomic<unsigned long long> done[64];   // ids of contexts, an id's place is id % 64
+    const unsigned long long id = current_context_id();
+    if (id != 0 && done[id % 64].load(std::memory_order_relaxed) == id) return CFX_OK;
     CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
     CFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    if (dev < kMaxDevices) done[dev].store(true, std::memory_order_relaxed);
+    if (id != 0) done[id % 64].store(id, std::memory_order_relaxed);
     return CFX_OK;
 }
 #endif

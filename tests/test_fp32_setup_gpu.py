@@ -1,5 +1,5 @@
 """The fp32 mode's one-time set-up (its kernels' shared-memory limits), in processes of their own: first calls with
-different shapes from several host threads at once."""
+different shapes from several host threads at once, and calls after the device was reset."""
 import os
 import subprocess
 import sys
@@ -53,4 +53,18 @@ threads = [threading.Thread(target=work, args=s) for s in shapes]
 for s in shapes:
     forward(*s)
 assert not failed, failed
+""")
+
+
+@pytest.mark.parametrize("H,A", [(32, 2), (512, 63)])
+def test_calls_after_a_device_reset(cfx, gpu, H, A):
+    """The limits go with the context: handles made after cudaDeviceReset set them again."""
+    _run(f"H, A = {H}, {A}\n" + """
+import ctypes, glob, os
+import nvidia
+runtime, = glob.glob(os.path.join(list(nvidia.__path__)[0], "cuda_runtime/lib/libcudart.so.1*"))
+before = forward(H, A)
+runtime = ctypes.CDLL(runtime)
+assert runtime.cudaSetDevice(0) == 0 and runtime.cudaDeviceReset() == 0
+assert np.array_equal(forward(H, A), before)
 """)
