@@ -52,9 +52,11 @@ constexpr int kPlanes = 3, kRowSpan = 32;                // a view row: 11 bytes
 constexpr int kSpan = kRows * kRowSpan;                  // of a plane
 constexpr int kWarps = kBlockThreads / 32, kOwn = kBlockEnvs / kWarps;   // envs whose records a warp writes
 constexpr int kPlaneBytes = kMapSize * kMapSize, kRecWords = kRec / 4, kMapWords = kMap / 4;
-struct Shared {
+struct Gathered {
     float tail[kBlockEnvs][kTail];       // odd row length: conflict-free thread-per-env writes
     uint32_t mobs[kBlockEnvs][kMobs];
+};
+struct Shared : Gathered {
     // per warp its four records as they go out, and before that, until they are in registers, the rows of its four
     // envs' views (light, block, item)
     __align__(16) uint8_t span[kWarps][kOwn * kRec];
@@ -152,7 +154,7 @@ __device__ __forceinline__ bool gather_mobs(const cfx_env_view& V, int e, int mo
 // block works on env t of the block; warp `part` takes an eighth of the loads.  The 51 scalars are in
 // the order of craftax_encode_scalar_observation_tail_at (:2429-2487).
 __device__ __forceinline__ void gather_env(const cfx_env_view& V, int e, int t, int part, int level, int top, int left,
-                                           Shared& S) {
+                                           Gathered& S) {
     const int n = V.num_envs;
     float* o = S.tail[t];
     // mobs of the player's level inside the view and on the map (:9195-9236).  Whether the cell is lit is
@@ -365,6 +367,34 @@ __device__ __forceinline__ void store_record(uint8_t* records, int e, int lane, 
     for (int w = lane; w < kRecWords; w += 32) dst[w] = rec[w];
 }
 
+// Turns the view rows of a warp's kOwn envs in `span` into their records, in the same place; first: the first of the envs in the
+// block, todo: those that there are
+__device__ __forceinline__ uint32_t* assemble(const Gathered& S, const View (&v)[kOwn], uint32_t todo, int first, int lane, uint8_t* span) {
+    Cells cells[kOwn];
+    uint32_t mob[kOwn / 2];   // two envs at a time, 16 lanes each
+#pragma unroll
+    for (int k = 0; k < kOwn; k++) cells[k] = make_cells(v[k], lane, span + k * kPlanes * kSpan);
+#pragma unroll
+    for (int k = 0; k < kOwn; k += 2) {
+        const int h = k + (lane >> 4);
+        mob[k / 2] = 0u;
+        if ((todo >> h & 1u) && (lane & 15) < kMobs)
+            mob[k / 2] = lit_mob(lane < 16 ? v[k] : v[k + 1], S.mobs[first + h][lane & 15], span + h * kPlanes * kSpan);
+    }
+    __syncwarp();   // the rows are in registers
+    uint32_t* rec = reinterpret_cast<uint32_t*>(span);   // [kOwn][kRecWords]
+#pragma unroll
+    for (int k = 0; k < kOwn; k++) {
+        put_cells(cells[k], lane, rec + k * kRecWords);
+        for (int j = lane; j < kTail; j += 32) rec[k * kRecWords + kMapWords + j] = __float_as_uint(S.tail[first + k][j]);
+    }
+    __syncwarp();   // the mob bytes land on cells other lanes have written
+#pragma unroll
+    for (int k = 0; k < kOwn; k += 2) put_mob(mob[k / 2], rec + (k + (lane >> 4)) * kRecWords);
+    __syncwarp();
+    return rec;
+}
+
 __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_constant__ Params P) {
     extern __shared__ __align__(16) uint8_t smem[];
     Shared& S = *reinterpret_cast<Shared*>(smem);
@@ -392,28 +422,7 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
     if (live) gather_env(P.v, e, lane, warp, level, top, left, S);
     wait_spans();
     __syncthreads();
-    Cells cells[kOwn];
-    uint32_t mob[kOwn / 2];   // two envs at a time, 16 lanes each
-#pragma unroll
-    for (int k = 0; k < kOwn; k++) cells[k] = make_cells(v[k], lane, span + k * kPlanes * kSpan);
-#pragma unroll
-    for (int k = 0; k < kOwn; k += 2) {
-        const int h = k + (lane >> 4);
-        mob[k / 2] = 0u;
-        if ((todo >> h & 1u) && (lane & 15) < kMobs)
-            mob[k / 2] = lit_mob(lane < 16 ? v[k] : v[k + 1], S.mobs[kOwn * warp + h][lane & 15], span + h * kPlanes * kSpan);
-    }
-    __syncwarp();   // the rows are in registers
-    uint32_t* rec = reinterpret_cast<uint32_t*>(span);   // [kOwn][kRecWords]
-#pragma unroll
-    for (int k = 0; k < kOwn; k++) {
-        put_cells(cells[k], lane, rec + k * kRecWords);
-        for (int j = lane; j < kTail; j += 32) rec[k * kRecWords + kMapWords + j] = __float_as_uint(S.tail[kOwn * warp + k][j]);
-    }
-    __syncwarp();   // the mob bytes land on cells other lanes have written
-#pragma unroll
-    for (int k = 0; k < kOwn; k += 2) put_mob(mob[k / 2], rec + (k + (lane >> 4)) * kRecWords);
-    __syncwarp();
+    const uint32_t* rec = assemble(S, v, todo, kOwn * warp, lane, span);
     if (todo == (1u << kOwn) - 1u && (reinterpret_cast<uintptr_t>(P.records) & 15) == 0) {
         // the warp's records in one bulk copy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -433,7 +442,8 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
 // The envs named by a device-side list (first int32 of every entry): a few that are being reset, anywhere in
 // the batch, so what counts is the chain of dependent loads and not coalescing.  A warp takes an
 // env: entry -> every scalar, the level and the position, all lanes at once -> mobs and map rows -> record.  About 250
-// entries of 65,536 envs: 26 us with a block for 32 entries, now 9.9.
+// entries of 65,536 envs: 26 us with a block for 32 entries, now 4.3 (by itself, its buffers in L2).  A long list is another
+// matter: there a block takes 32 entries at a time as k_record_rows does, see list_block.
 // The fields of the tail by position: which field pointer of the view, which element, how it is scaled.
 enum Scale : uint8_t { S_SQRT10, S_10, S_2, S_4, S_INT, S_F10, S_FLOAT, S_FLAG, S_DIR, S_KILLED, S_BOSS };
 struct TailField { uint8_t field, elem, scale; };
@@ -489,17 +499,82 @@ struct ListShared {
 };
 static_assert(sizeof(ListShared) % 16 == 0, "alignment");
 constexpr int kListThreads = 128, kListWarps = kListThreads / 32;
+struct ListBlock : Gathered {
+    __align__(16) uint8_t span[kListWarps][kOwn * kRec];
+};
+union ListMemory {
+    ListShared warp[kListWarps];
+    ListBlock block;
+};
+static_assert(sizeof(ListMemory) <= 48 * 1024, "static shared memory");
+// Lists of more entries than this for each warp of the grid go by blocks.  65,536 envs, 2,368 warps, us by warps / by blocks:
+// 2,368 entries 5.0 / 8.7, 4,736 8.0 / 9.2, 7,104 11.0 / 9.5, 16,384 29 / 13, all of them 135 / 53.
+constexpr int kListPerWarp = 2;
 
-__global__ void __launch_bounds__(kListThreads) k_record_rows_list(const __grid_constant__ Params P) {
-    __shared__ ListShared LS[kListWarps];
+// 32 entries of the list from `base` on, lane = entry in the loads of the fields, a warp four envs at a time in the rest
+__device__ __forceinline__ void list_block(const Params& P, ListBlock& S, const CopyLane& copy, int grain, int base, int count) {
+    const cfx_env_view& V = P.v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = V.num_envs;
+    int e = -1, level = 0, top = 0, left = 0;
+    if (base + lane < count) e = *reinterpret_cast<const int32_t*>(P.list + (size_t)(base + lane) * P.list_stride);
+    const bool live = e >= 0 && e < n;
+    if (live) {
+        level = soa(V.player_level, 0, n, e);
+        top = soa(V.player_position, 0, n, e) - kRows / 2;
+        left = soa(V.player_position, 1, n, e) - kCols / 2;
+    }
+    const View mine = make_view(level, top, left);
+    const uint32_t all = __ballot_sync(0xffffffffu, live);
+    uint8_t* const span = S.span[warp];
+    View v[kOwn];
+    auto copies = [&](int first) {
+#pragma unroll
+        for (int k = 0; k < kOwn; k++) {
+            v[k].bits = __shfl_sync(0xffffffffu, mine.bits, first + k);
+            const int env = __shfl_sync(0xffffffffu, e, first + k);
+            if (all >> (first + k) & 1u) copy.start(V, env, v[k], grain, span + k * kPlanes * kSpan);
+        }
+    };
+    constexpr int kWarpEnvs = kBlockEnvs / kListWarps;
+    copies(kWarpEnvs * warp);
+#pragma unroll 1
+    for (int part = warp; part < kWarps; part += kListWarps)
+        if (live) gather_env(V, e, lane, part, level, top, left, S);
+    wait_spans();
+    __syncthreads();
+#pragma unroll 1
+    for (int i = 0; i < kWarpEnvs; i += kOwn) {
+        const int first = kWarpEnvs * warp + i;
+        if (i > 0) {
+            copies(first);
+            wait_spans();
+        }
+        const uint32_t todo = all >> first & ((1u << kOwn) - 1u);
+        const uint32_t* rec = assemble(S, v, todo, first, lane, span);
+        for (int k = 0; k < kOwn; k++) {
+            const int env = __shfl_sync(0xffffffffu, e, first + k);
+            if (todo >> k & 1u) store_record(P.records, env, lane, rec + k * kRecWords);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kListThreads, 4) k_record_rows_list(const __grid_constant__ Params P) {
+    __shared__ ListMemory M;
     const cfx_env_view& V = P.v;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = V.num_envs, grain = copy_grain(V);
-    ListShared& S = LS[warp];
+    ListShared& S = M.warp[warp];
     const CopyLane copy(V, lane);
     const TailField f0 = kTailFields[lane], f1 = kTailFields[min(lane + 32, kTail - 1)];
     wait_for_previous_kernel();
     const int count = *P.count_dev;
     const int stride = (int)gridDim.x * kListWarps;
+    if (count > kListPerWarp * stride) {
+        for (int base = (int)blockIdx.x * kBlockEnvs; base < count; base += (int)gridDim.x * kBlockEnvs)
+            list_block(P, M.block, copy, grain, base, count);
+        return;
+    }
     for (int i = (int)blockIdx.x * kListWarps + warp; i < count; i += stride) {
         const int e = *reinterpret_cast<const int32_t*>(P.list + (size_t)i * P.list_stride);
         if (e < 0 || e >= n) continue;
