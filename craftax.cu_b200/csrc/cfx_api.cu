@@ -742,8 +742,7 @@ int cfx_sample_actions(int device, const float* logits, int ld, int num_actions,
     CFX_REQUIRE(num_actions >= 2 && num_actions <= kMaxActions && ld >= num_actions,
                 "cfx_sample_actions: num_actions=%d ld=%d", num_actions, ld);
     CFX_GUARD(device);
-    return launch_sample(logits, ld, num_actions, uniforms, 0, 0, nullptr, 0, n, nullptr, actions,
-                         logprobs, nullptr, (cudaStream_t)stream);
+    return launch_sample_logits(logits, ld, num_actions, uniforms, n, actions, logprobs, (cudaStream_t)stream);
 }
 
 int cfx_philox_uniforms(int device, uint64_t seed, uint64_t env_offset, uint64_t step, int n,

@@ -36,6 +36,9 @@ int launch_sample(const float* logits, int ld, int A, const float* u, uint64_t s
                   uint64_t env_offset, unsigned long long* step_ctr, int bump, int n,
                   float* env_actions, int32_t* actions, float* logprobs, float* values,
                   cudaStream_t st, int early = 0);
+// logits by themselves: [n][ld] and a uniform an env -> action and log-probability
+int launch_sample_logits(const float* logits, int ld, int A, const float* u, int n, int32_t* actions, float* logprobs,
+                         cudaStream_t st);
 int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, float* u, cudaStream_t st);
 // copies `bytes` (a multiple of 16) from page-locked host memory, both 16-byte aligned
 int launch_fetch(const void* host, void* dst, size_t bytes, cudaStream_t st);

@@ -1,8 +1,36 @@
-"""Calls that take another way for many envs, on both sides of where it changes: the record write of a long list."""
+"""Calls that take another kernel for many envs, on both sides of where it changes: the stand-alone sampler, and the
+record write of a long list of envs."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [65535, 65536, 65537, 131071, 131200])
+@pytest.mark.parametrize("A,pad", [(2, 0), (17, 0), (32, 1), (33, 0), (43, 1), (63, 0)])
+def test_sampler_rule(cfx, gpu, n, A, pad):
+    """The same arithmetic in the same order in both forms: a batch is sampled as its halves are."""
+    rng = np.random.default_rng(n + A)
+    logits = rng.normal(0, 2, (n, A + pad)).astype(np.float32)
+    logits[::97, 0] = -np.inf
+    logits[5::101, A - 1] = np.inf     # no action has a probability: the last one
+    logits[7::103, A // 2] = np.nan
+    u = rng.random(n, dtype=np.float32)
+    u[::11], u[1::11] = 0.0, np.float32(1.0)
+
+    def sample(lo, hi):
+        d_l, d_u = cfx.DeviceBuffer.from_host(logits[lo:hi]), cfx.DeviceBuffer.from_host(u[lo:hi])
+        a, lp = cfx.DeviceBuffer((hi - lo + 1,), np.int32), cfx.DeviceBuffer((hi - lo + 1,), np.float32)
+        a.fill(0xCD), lp.fill(0xCD)
+        cfx.check(cfx.lib().cfx_sample_actions(0, d_l.ptr, A + pad, A, d_u.ptr, hi - lo, a.ptr, lp.ptr, None))
+        cfx.check(cfx.lib().cfx_stream_sync(0, None))
+        a, lp = a.download(), lp.download()
+        assert a.view(np.uint32)[-1] == 0xCDCDCDCD and lp.view(np.uint32)[-1] == 0xCDCDCDCD
+        return a[:-1], lp[:-1]
+    parts = [sample(lo, min(lo + 50000, n)) for lo in range(0, n, 50000)]
+    a, lp = sample(0, n)
+    assert np.array_equal(a, np.concatenate([p[0] for p in parts]))
+    assert np.array_equal(lp, np.concatenate([p[1] for p in parts]), equal_nan=True)
 
 
 @pytest.mark.parametrize("entries,shift", [(2 * 2368, 0), (2 * 2368 + 1, 0), (6001, 4), (2 * 2368 + 33, 1)])
