@@ -39,3 +39,21 @@ def test_partly_registered_logits(cfx, gpu, oracle, n, pieces):
         for a, _ in spans:
             assert int(rt.cudaHostUnregister(first + a * PAGE)) == 0
         pol.close()
+
+
+@pytest.mark.parametrize("pageable", [None, "logits_av", "actions"])
+def test_slices_with_pageable_outputs(cfx, gpu, oracle, pageable):
+    """A sliced call reads its outputs back at the end where one of them is pageable: the same values."""
+    n = 65536 + 4128
+    rec = cfx.PinnedBuffer((n, 996), np.uint8)
+    rec.array[...] = oracle.synthetic_records(2048, seed=6)[np.arange(n) % 2048]
+    pol = cfx.Policy(n, H, L, A, "f16")
+    pol.set_weights(oracle.init_weights(H, L, A, seed=12))
+    want = pol.forward_host(np.array(rec.array), None, seed=3)
+    shapes = {k: cfx.PinnedBuffer(v.shape, v.dtype) for k, v in want.items()}
+    out = {k: np.full(b.shape, 7, b.dtype) if k == pageable else b.array for k, b in shapes.items()}
+    pol.reset_state()
+    pol.forward_host(rec.array, None, seed=3, out=out)
+    for k in want:
+        assert np.array_equal(out[k], want[k]), k
+    pol.close()
