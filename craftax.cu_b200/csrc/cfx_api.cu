@@ -591,12 +591,14 @@ static int forward_host_small(cfx_policy* p, const cfx_forward_io* h, cfx_forwar
     const size_t bytes = n * (size_t)p->rec_bytes;
     const void* rec = n <= kHostFetchEnvs ? device_address(h->records, bytes) : nullptr;
     int rc;
-    if (rec && ((uintptr_t)rec & 15) == 0) {
+    const bool fetch = rec && ((uintptr_t)rec & 15) == 0;
+    if (fetch) {
         if ((rc = launch_fetch(rec, p->st_records, bytes, st))) return rc;
     } else {
         CFX_CUDA(cudaMemcpyAsync(p->st_records, h->records, bytes, cudaMemcpyHostToDevice, st));
     }
     if ((rc = cfx_policy_forward(p, d, st))) return rc;
+    p->last_launches += fetch ? 1 : 0;
     if (h->logits_av && !logits)
         CFX_CUDA(cudaMemcpyAsync(h->logits_av, p->st_logits, n * row, cudaMemcpyDeviceToHost, st));
     if (h->r_state)

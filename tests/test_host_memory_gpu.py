@@ -41,6 +41,17 @@ def test_partly_registered_logits(cfx, gpu, oracle, n, pieces):
         pol.close()
 
 
+@pytest.mark.parametrize("n,pinned,launches", [(32, True, 2), (256, True, 2), (288, True, 1), (32, False, 1)])
+def test_launches_of_a_small_call(cfx, gpu, oracle, n, pinned, launches):
+    """Page-locked records of the smallest batches are fetched by a kernel of their own, which counts."""
+    buf = cfx.PinnedBuffer((n, 996), np.uint8)
+    buf.array[...] = oracle.synthetic_records(n, seed=3)
+    pol = cfx.Policy(n, H, L, A, "f16")
+    pol.forward_host(buf.array if pinned else np.array(buf.array), None, seed=5)
+    assert pol.last_launches == launches
+    pol.close()
+
+
 @pytest.mark.parametrize("pageable", [None, "logits_av", "actions"])
 def test_slices_with_pageable_outputs(cfx, gpu, oracle, pageable):
     """A sliced call reads its outputs back at the end where one of them is pageable: the same values."""
