@@ -72,10 +72,10 @@ __device__ __forceinline__ int jax_index(int i, int size) {
 // Loads that are issued where they stand.  A plain load through a pointer of the view may alias the shared memory
 // that is written in between, so the compiler keeps load, conversion and store of every field in order, one DRAM
 // latency a field; a read-only load it sinks to its use, with the same effect.  Every loop below
-// therefore loads all its fields first.
+// therefore loads all its fields first.  (ld.global.nc would be wrong besides: see wait_for_previous_kernel.)
 __device__ __forceinline__ uint32_t ld_bits(const uint32_t* p) {
     uint32_t v;
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ int32_t ld_now(const int32_t* p) { return (int32_t)ld_bits(reinterpret_cast<const uint32_t*>(p)); }
@@ -83,13 +83,13 @@ __device__ __forceinline__ uint32_t ld_now(const uint32_t* p) { return ld_bits(p
 __device__ __forceinline__ float ld_now(const float* p) { return __uint_as_float(ld_bits(reinterpret_cast<const uint32_t*>(p))); }
 __device__ __forceinline__ uint8_t ld_now(const uint8_t* p) {
     uint16_t v;
-    asm volatile("ld.global.nc.u8 %0, [%1];" : "=h"(v) : "l"(p));
+    asm volatile("ld.global.u8 %0, [%1];" : "=h"(v) : "l"(p));
     return (uint8_t)v;
 }
 __device__ __forceinline__ int8_t ld_now(const int8_t* p) { return (int8_t)ld_now(reinterpret_cast<const uint8_t*>(p)); }
 __device__ __forceinline__ int16_t ld_now(const int16_t* p) {
     int16_t v;
-    asm volatile("ld.global.nc.s16 %0, [%1];" : "=h"(v) : "l"(p));
+    asm volatile("ld.global.s16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
 template <typename T>

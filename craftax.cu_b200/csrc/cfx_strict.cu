@@ -132,7 +132,7 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("
 
 template <int TM, int G>
 __global__ void __launch_bounds__(256, 2)
-k_encoder_fp32(const uint8_t* __restrict__ rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc,
+k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc,
                float* __restrict__ h_out, int n, int H, int w_aligned, int early) {
     using E = Enc<TM, G>;
     constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = kEncK, S = E::S, D = S - 2;
@@ -300,7 +300,7 @@ __global__ void k_classic_expand(const uint8_t* __restrict__ rec, float* __restr
 // bias, then per cell the block column and the set mob bits, then the 22 scalar features, every
 // term as fmaf(x, W, acc).  One thread per (env, unit); the block's threads read a W_enc row
 // coalesced.  Block ids outside [0,16] (never written by the game) are skipped.
-__global__ void k_classic_encoder_fp32(const uint8_t* __restrict__ rec, const float* __restrict__ W_enc,
+__global__ void k_classic_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc,
                                        const float* __restrict__ b_enc, float* __restrict__ h_out,
                                        int n, int H) {
     __shared__ uint8_t rs[kClassicRec];
@@ -356,8 +356,8 @@ template <int TM, int WM, int WU> constexpr int gru_stage_floats() { return kGru
 
 template <int TM, int WM, int WU, int ST>
 __global__ void __launch_bounds__(32 * WM * WU, 3)
-k_mingru_fp32(const float* __restrict__ x_in, const float* __restrict__ Wt, float* __restrict__ state,
-              const float* __restrict__ prev_terminals, float* __restrict__ h_out, float* __restrict__ r_state,
+k_mingru_fp32(const float* x_in, const float* __restrict__ Wt, float* __restrict__ state,
+              const float* prev_terminals, float* __restrict__ h_out, float* __restrict__ r_state,
               int r_bf16, int n, int H, int s_aligned, int early) {
     constexpr int T = 32 * WM * WU, BM = 4 * TM * WM, BU = 32 * WU, kStage = gru_stage_floats<TM, WM, WU>();
     constexpr int EB = BM < 32 ? BM : 32;         // envs of an activation tile that a block takes
@@ -504,7 +504,7 @@ constexpr size_t head_smem(int H, int A) {
     return ((size_t)kHeadEnvs * H + (size_t)head_row_groups(A) * kHeadRows * (H + 4)) * sizeof(float);
 }
 
-__global__ void __launch_bounds__(384) k_heads_fp32(const float* __restrict__ h, const float* __restrict__ W_a,
+__global__ void __launch_bounds__(384) k_heads_fp32(const float* h, const float* __restrict__ W_a,
                                                     const float* __restrict__ b_a, const float* __restrict__ W_v,
                                                     const float* __restrict__ b_v, float* __restrict__ logits_av,
                                                     int n, int H, int A, int early) {
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(384) k_heads_fp32(const float* __restrict__ h,
 constexpr int kSampleEnvs = 32, kSampleThreads = 128;
 
 __global__ void __launch_bounds__(kSampleThreads)
-k_sample(const float* __restrict__ logits, int ld, int A, const float* __restrict__ uniforms, uint64_t seed,
+k_sample(const float* logits, int ld, int A, const float* uniforms, uint64_t seed,
          uint64_t env_offset, unsigned long long* ctr, int bump, int n, float* __restrict__ env_actions,
          int32_t* __restrict__ actions, float* __restrict__ logprobs, float* __restrict__ values, int early) {
     __shared__ float l[kSampleEnvs][kMaxActions + 2], p[kSampleEnvs + 1][kMaxActions + 2];   // odd row length
@@ -639,7 +639,7 @@ k_sample(const float* __restrict__ logits, int ld, int A, const float* __restric
 // 63; 65,536 envs 5.4 / 4.1, 8.0 / 6.8, 14.8 / 15.0, 18.6 / 20.4; 16,384 envs 3.4 / 4.1, 3.7 / 6.1, 6.1 / 13.6, 7.7 / 18.5.
 constexpr int kSampleRows = 128;
 __global__ void __launch_bounds__(kSampleRows)
-k_sample_rows(const float* __restrict__ logits, int ld, int A, const float* __restrict__ uniforms, int n,
+k_sample_rows(const float* logits, int ld, int A, const float* uniforms, int n,
               int32_t* __restrict__ actions, float* __restrict__ logprobs) {
     extern __shared__ float rows[];   // [kSampleRows][A | 1]: logits, then the running sums of the exponentials
     const int tid = threadIdx.x, e0 = blockIdx.x * kSampleRows, pitch = A | 1;
@@ -674,7 +674,7 @@ __global__ void k_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, in
     if (e < n) u[e] = philox_uniform(seed, env_offset + (uint64_t)e, step);
 }
 
-__global__ void k_fetch(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t count) {
+__global__ void k_fetch(const uint4* src, uint4* __restrict__ dst, size_t count) {
     wait_for_previous_kernel();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count) dst[i] = src[i];
