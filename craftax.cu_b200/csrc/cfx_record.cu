@@ -283,8 +283,9 @@ struct CopyLane {
     }
     // Starts the copies of env e's rows into `dst`.  A map row is 48 bytes, so 16-byte pieces (4-byte pieces) stay inside
     // it where the planes are aligned to 16 (4) bytes.
+    template <bool BYTES>
     __device__ __forceinline__ void start(const cfx_env_view& V, int e, View v, int grain, uint8_t* dst) const {
-        if (grain == 1) return bytes(V, e, v, dst);
+        if constexpr (BYTES) return bytes(V, e, v, dst);
         const int row = v.top() + dr, left = v.left(), c0 = left & ~15;
         if (plane >= kPlanes || (unsigned)row >= (unsigned)kMapSize) return;
         const uint8_t* q = src + (size_t)e * V.state_stride + (v.level() * kPlaneBytes + row * kMapSize + c0);
@@ -306,7 +307,7 @@ __device__ __forceinline__ void wait_spans() {
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     __syncwarp();
 }
-__device__ __forceinline__ int copy_grain(const cfx_env_view& V) {
+__host__ __device__ __forceinline__ int copy_grain(const cfx_env_view& V) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(V.state_base) | V.state_stride | V.map_offset | V.item_map_offset | V.light_map_offset;
     return (a & 15) == 0 ? 16 : ((a & 3) == 0 ? 4 : 1);
 }
@@ -395,6 +396,8 @@ __device__ __forceinline__ uint32_t* assemble(const Gathered& S, const View (&v)
     return rec;
 }
 
+// (BYTES: the planes are not aligned to words.  A kernel of its own: beside the copies its loads made 1,024 envs 3 % slower.)
+template <bool BYTES>
 __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_constant__ Params P) {
     extern __shared__ __align__(16) uint8_t smem[];
     Shared& S = *reinterpret_cast<Shared*>(smem);
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
 #pragma unroll
     for (int k = 0; k < kOwn; k++) {
         v[k].bits = __shfl_sync(0xffffffffu, mine.bits, kOwn * warp + k);
-        if (todo >> k & 1u) copy.start(P.v, e0 + kOwn * warp + k, v[k], grain, span + k * kPlanes * kSpan);
+        if (todo >> k & 1u) copy.start<BYTES>(P.v, e0 + kOwn * warp + k, v[k], grain, span + k * kPlanes * kSpan);
     }
     if (live) gather_env(P.v, e, lane, warp, level, top, left, S);
     wait_spans();
@@ -512,6 +515,7 @@ static_assert(sizeof(ListMemory) <= 48 * 1024, "static shared memory");
 constexpr int kListPerWarp = 2;
 
 // 32 entries of the list from `base` on, lane = entry in the loads of the fields, a warp four envs at a time in the rest
+template <bool BYTES>
 __device__ __forceinline__ void list_block(const Params& P, ListBlock& S, const CopyLane& copy, int grain, int base, int count) {
     const cfx_env_view& V = P.v;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = V.num_envs;
@@ -532,7 +536,7 @@ __device__ __forceinline__ void list_block(const Params& P, ListBlock& S, const 
         for (int k = 0; k < kOwn; k++) {
             v[k].bits = __shfl_sync(0xffffffffu, mine.bits, first + k);
             const int env = __shfl_sync(0xffffffffu, e, first + k);
-            if (all >> (first + k) & 1u) copy.start(V, env, v[k], grain, span + k * kPlanes * kSpan);
+            if (all >> (first + k) & 1u) copy.start<BYTES>(V, env, v[k], grain, span + k * kPlanes * kSpan);
         }
     };
     constexpr int kWarpEnvs = kBlockEnvs / kListWarps;
@@ -560,6 +564,7 @@ __device__ __forceinline__ void list_block(const Params& P, ListBlock& S, const 
     __syncthreads();
 }
 
+template <bool BYTES>
 __global__ void __launch_bounds__(kListThreads, 4) k_record_rows_list(const __grid_constant__ Params P) {
     __shared__ ListMemory M;
     const cfx_env_view& V = P.v;
@@ -572,7 +577,7 @@ __global__ void __launch_bounds__(kListThreads, 4) k_record_rows_list(const __gr
     const int stride = (int)gridDim.x * kListWarps;
     if (count > kListPerWarp * stride) {
         for (int base = (int)blockIdx.x * kBlockEnvs; base < count; base += (int)gridDim.x * kBlockEnvs)
-            list_block(P, M.block, copy, grain, base, count);
+            list_block<BYTES>(P, M.block, copy, grain, base, count);
         return;
     }
     for (int i = (int)blockIdx.x * kListWarps + warp; i < count; i += stride) {
@@ -582,7 +587,7 @@ __global__ void __launch_bounds__(kListThreads, 4) k_record_rows_list(const __gr
         const int top = soa(V.player_position, 0, n, e) - kRows / 2, left = soa(V.player_position, 1, n, e) - kCols / 2;
         const uint32_t raw0 = tail_raw(V, f0, e), raw1 = lane + 32 < kTail ? tail_raw(V, f1, e) : 0u;
         const View v = make_view(level, top, left);
-        copy.start(V, e, v, grain, S.span);
+        copy.start<BYTES>(V, e, v, grain, S.span);
         const bool killed = (unsigned)level < (unsigned)kLevels && soa(V.monsters_killed, level, n, e) >= kKilledToClear;
         // lane 3 c + i: slot i of mob class c
         const int c = lane / kSlots, slot = lane % kSlots;
@@ -781,8 +786,13 @@ extern "C" int cfx_record_obs(int device, const cfx_env_view* view, uint8_t* rec
     P.n = n;
     P.skip = skip;
     const unsigned blocks = (unsigned)((n + record::kBlockEnvs - 1) / record::kBlockEnvs);
-    if ((rc = allow_smem<record::k_record_rows, (int)sizeof(record::Shared)>())) return rc;
-    return launch_chained(record::k_record_rows, dim3(blocks), record::kBlockThreads, sizeof(record::Shared), (cudaStream_t)stream, P);
+    auto launch = [&](auto bytes) {
+        constexpr auto kernel = record::k_record_rows<decltype(bytes)::value>;
+        const int rc = allow_smem<kernel, (int)sizeof(record::Shared)>();
+        if (rc) return rc;
+        return launch_chained(kernel, dim3(blocks), record::kBlockThreads, sizeof(record::Shared), (cudaStream_t)stream, P);
+    };
+    return record::copy_grain(*view) == 1 ? launch(std::true_type()) : launch(std::false_type());
 }
 
 extern "C" int cfx_record_obs_list(int device, const cfx_env_view* view, uint8_t* records, const void* list,
@@ -800,7 +810,8 @@ extern "C" int cfx_record_obs_list(int device, const cfx_env_view* view, uint8_t
     // (the reference uses at most 128 blocks of 8 warps for its list pass, :11941)
     int blocks = (view->num_envs + record::kListWarps - 1) / record::kListWarps;
     if (blocks > 592) blocks = 592;
-    return launch_chained(record::k_record_rows_list, dim3((unsigned)blocks), record::kListThreads, 0, (cudaStream_t)stream, P);
+    return launch_chained(record::copy_grain(*view) == 1 ? record::k_record_rows_list<true> : record::k_record_rows_list<false>,
+                          dim3((unsigned)blocks), record::kListThreads, 0, (cudaStream_t)stream, P);
 }
 
 extern "C" int cfx_classic_record_obs(int device, const cfx_classic_env_view* view, uint8_t* records, int n,
