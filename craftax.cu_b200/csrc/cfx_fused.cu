@@ -270,7 +270,7 @@ __device__ __forceinline__ int rec_owner(int kc) { return (kc & 1) ^ 1; }
 // A CTA's first tile has no sampler before it, so warpgroup 0 starts with chunk 1 there: a launch of one tile per SM is 2 to 3 %
 // shorter (12,000 envs h256x1 20.5 -> 19.9 us, 16,384 envs h128x2 19.9 -> 19.4).  At hidden 128 a tile's MMAs are shorter than
 // the conversion and every tile is better off so (131,104 envs 122.8 -> 121.2); at 256 the later ones are not (262,144
-// envs 417 -> 425).
+// envs 417 -> 425).  (A loop over one set of buffers.)
 constexpr int kHeadStart = 3, kWgRSlots = 3;
 template <int HID> __device__ __forceinline__ int head_start(bool first_tile) { return HID == 128 || first_tile ? 1 : kHeadStart; }
 __device__ __forceinline__ int full_owner(int kc, int hs) { return kc < hs ? 1 : ((kc & 1) ^ 1); }
@@ -869,7 +869,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 constexpr int kNS = C::kNS;
                 const int slot = scnt % kNS;
                 // under the slice's MMAs (of a warp's rows all or none are valid).  The ballot of the flags stands here and not at
-                // the tile's start, where it would wait for them: 65,536 envs h256x3 145.7 -> 142.8 us
+                // the tile's start, where it would wait for them: 65,536 envs h256x3 145.7 -> 142.8 us, one set of buffers
                 if (P.r_state != nullptr && valid) {
                     CFX_WAITW(S_FULL + slot, (scnt / kNS) & 1, W_S_FULL);
                     write_r_state<8, kH>(P, sm.s_slot(slot) + quarter * 4096, 0,

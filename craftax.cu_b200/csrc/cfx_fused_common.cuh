@@ -224,7 +224,8 @@ __device__ __forceinline__ void mingru_cell_pair(float hzh0, float hzh1, float h
 // craftax_full.cu:9370-9375), [L][n][H] fp32 or bf16.  A warp writes its 32 rows x 4 PIECES units from
 // the state box (128-byte swizzled rows) before the cell updates it in place: PIECES lanes side by side take a row's
 // 16-byte pieces, so that a store instruction touches 32 / PIECES rows.  With every lane writing the row whose cell
-// it computes, it touched 32, and these stores kept the load/store unit busy for most of a slice: h256x2, 57,600 envs
+// it computes, it touched 32, and these stores kept the load/store unit busy for most of a slice (us in a loop over one set of
+// buffers; over several in turn a step takes 3 to 7 % more): h256x2, 57,600 envs
 // 126.6 -> 112.9 us with a bf16 record, 139.3 -> 123.1 with fp32; 16,416 envs 35.0 -> 30.7 and 37.1 -> 33.8; 8,192 envs
 // (cfx_fused_split.cu) 25.9 -> 24.2 and 28.9 -> 25.2.
 // `box`: the row of lane 0 (a multiple of 8 rows into the box); `at`: element of that row and the first of the warp's units

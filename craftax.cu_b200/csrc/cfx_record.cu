@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
 // The envs named by a device-side list (first int32 of every entry): a few that are being reset, anywhere in
 // the batch, so what counts is the chain of dependent loads and not coalescing.  A warp takes an
 // env: entry -> every scalar, the level and the position, all lanes at once -> mobs and map rows -> record.  About 250
-// entries of 65,536 envs: 26 us with a block for 32 entries, now 4.3 (by itself, its buffers in L2).  A long list is another
+// entries of 65,536 envs: 26 us with a block for 32 entries, now 4 (9.8 from cold caches).  A long list is another
 // matter: there a block takes 32 entries at a time as k_record_rows does, see list_block.
 // The fields of the tail by position: which field pointer of the view, which element, how it is scaled.
 enum Scale : uint8_t { S_SQRT10, S_10, S_2, S_4, S_INT, S_F10, S_FLOAT, S_FLAG, S_DIR, S_KILLED, S_BOSS };
@@ -647,7 +647,8 @@ static_assert(offsetof(cfx_env_view, mob_type_id) - offsetof(cfx_env_view, playe
 // instruction to shared memory (whole rows: what is read from memory is 32-byte sectors anyway), where a
 // thread then takes the nine nibbles of a row from two words.  Loads of these words from the map
 // itself, 14 a thread, touch 32 cache lines an instruction: 20 of 41 us of a cache's time.  262,144 envs: a load per cell
-// 103 us, words from the map 41.5, rows through shared memory 27.3 (127 MB: 4.7 TB/s); 65,536 envs 12.4 -> 8.2 us.
+// 103 us, words from the map 41.5, rows through shared memory 27.3 (102 MB read from DRAM, 39 MB written); 65,536
+// envs 12.4 -> 8.2 us.
 constexpr int kClRows = 7, kClCols = 9, kClCells = kClRows * kClCols, kClMap = 64, kClRowBytes = 32;
 constexpr int kClSpan = kClRows * kClRowBytes + 16;   // 60 words: as few bank conflicts as 16-byte pieces allow
 constexpr int kClInv = 12, kClOutOfBounds = 1, kClBlockEnvs = 64, kClWords = kClassicRec / 4;

@@ -347,7 +347,7 @@ __global__ void k_done_to_terminals(const int8_t* __restrict__ done, float* __re
 // Wt is the layer's gate matrix as k_transpose_gates lays it out, x_in and h_out activations.  K chunks of 32; ST buffers:
 // two where several blocks share an SM, more for small batches, which wait for the loads (chunks of 16 with three: 155 against
 // 152 us a forward at 4,096 envs, 970 against 944 us at 8,192 envs with hidden 512, depth 3); the k loop has to be unrolled
-// well (by 4: 170 us).  Bound by the FMA pipe: 66 % of its peak at hidden 512; one thread per unit with 16 envs, before, 20 %.
+// well (by 4: 170 us).  Bound by the FMA pipe: busy 80 % of the time at hidden 512; one thread per unit with 16 envs, before, 20 %.
 __device__ __forceinline__ float sigmoid_ref(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float mingru_g_ref(float x) { return x >= 0.0f ? x + 0.5f : sigmoid_ref(x); }
 

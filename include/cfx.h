@@ -187,8 +187,10 @@ int cfx_selftest_wait_timeout(int device, unsigned limit_ms);
  * cfx_policy_forward, copies every non-NULL output back and synchronises.
  * With the fused kernel and at least 65,536 envs the records go up in two to
  * eight slices (one per 32,768 envs) on a second stream, the kernel is launched
- * once per slice behind them and the slice's outputs go down on a third (same
- * results; cfx_policy_last_launches counts the launches). */
+ * once per slice behind them and the slice's outputs go down on a third, or at
+ * the end where one of them is pageable (same results; cfx_policy_last_launches
+ * counts the launches, for small batches that of the kernel that fetches
+ * page-locked records too). */
 int cfx_policy_forward_host(cfx_policy* p, const cfx_forward_io* host_io);
 
 /* Strict-fp32 forward for callers that cannot allocate device memory while they run -- a
