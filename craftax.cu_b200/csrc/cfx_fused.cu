@@ -1430,11 +1430,12 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     if (launches) *launches = 1;
     // Small batches: a tile is shared by four (two) CTAs as long as every tile then has its SMs at once, and is as
     // short as that allows (cfx_fused_split.cu).  us a step, h256x2: 1,600 envs 16.0 with four CTAs and 64 rows, 18.0 with
-    // two and 32; 1,024 envs 13.6 with 32 rows, 15.5 with 64, 17.4 with 128.  CTAs of two slices take tiles of 128 rows only: at
-    // their other sizes four CTAs a tile have their SMs.
+    // two and 32; 1,024 envs 13.6 with 32 rows, 15.5 with 64, 17.4 with 128.  CTAs of two slices take tiles of 64 and
+    // 128 rows; at 32 four CTAs a tile have their SMs.  With the 33 clusters of four and 74 of two that this part holds, four
+    // CTAs go to 1,056, 2,112 and 4,224 envs, and two to 4,736 with 64 rows (4,544 envs h256x3 23.4 us, with 128 rows 25.0).
     const int rows = std::min(p->n, P.num_tiles * fused::kTile) - P.tile_begin * fused::kTile;
     for (int i = 0; i < 2; i++)
-        for (int S = i == 0 ? 4 : 2, tr = p->H == 64 * S ? 32 : fused::kTile; tr <= fused::kTile; tr *= 2) {
+        for (int S = i == 0 ? 4 : 2, tr = p->H == 64 * S ? 32 : 64; tr <= fused::kTile; tr *= 2) {
             const int tiles = (rows + tr - 1) / tr;
             if (tiles > p->max_split[i]) continue;
             for (int l = 0; l < p->L; l++) P.state_map[l] = p->quad_map[l];

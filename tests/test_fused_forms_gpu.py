@@ -1,6 +1,6 @@
-"""The persistent kernel as CTA pairs, at sizes that the small-batch form does not take: bit for bit what one CTA per tile
-computes, both operand types, both record types, filler tiles and several tiles a CTA; and the record of the state
-inputs against what it is a copy of."""
+"""The persistent kernel as CTA pairs, at sizes that the small-batch form does not take, and that form where its
+clusters and tiles change: bit for bit what one CTA per tile computes, both operand types, both record types, filler
+tiles and several tiles a CTA; and the record of the state inputs against what it is a copy of."""
 import numpy as np
 import pytest
 
@@ -41,6 +41,11 @@ def _bf16(x):
     (19008, 256, 3, "bf16", "full", "fp32"),      # 149 tiles: one pair has two rounds
     (57600, 256, 1, "f16", "full", "fp32"),       # 450: three or four tiles a CTA
     (9600, 128, 4, "bf16", "full", "fp32"), (38016, 128, 2, "bf16", "full", None), (16416, 128, 2, "f16", "full", "bf16"),
+    # where 33 clusters of four and 74 of two are resident: the last tiles of 32, 64 and 128 rows for four CTAs, the first
+    # of 64 and 128 after them, the first, the last and a ragged one of 64 rows for two CTAs
+    (1056, 256, 2, "f16", "full", "bf16"), (1088, 256, 1, "bf16", "full", None), (2112, 256, 3, "bf16", "full", "fp32"),
+    (2144, 256, 2, "f16", "full", "bf16"), (4224, 256, 1, "f16", "full", "fp32"), (4256, 256, 2, "bf16", "full", "fp32"),
+    (4512, 256, 3, "f16", "full", "bf16"), (4736, 256, 4, "f16", "full", None), (4576, 256, 3, "f16", "classic", "bf16"),
     (9504, 256, 3, "bf16", "classic", "bf16"), (38048, 256, 2, "f16", "classic", "fp32")])
 def test_pairs_equal_one_cta_per_tile(cfx, gpu, monkeypatch, n, H, L, prec, game, r_state):
     from cfx import synth
