@@ -352,7 +352,8 @@ __device__ __forceinline__ void done_with_step(unsigned long long* step, uint32_
 // The named barriers at which a warp meets others of its block: id `first`, then the one after it, each once a launch.  A
 // named barrier has no limit, so a warp that gives up in a bounded wait before a meeting arrives there
 // on its way out (leave): nobody waits for a warp that has gone.  (Only `met` lives through the role, and what a warp that
-// gave up still owes is worked out for such a warp alone: 4,000 envs 19.55 us so, 19.85 with every warp working it out.)
+// gave up still owes is worked out for such a warp alone: 4,000 envs 19.5 us so, 19.85 with every warp working it out.  The
+// check itself costs the smallest batches 1 %, 1,024 envs 12.7 us instead of 12.6; where the waits give up instead: 12.8.)
 struct Meetings {
     static constexpr int kAll = 255;   // the role has come to its end
     int met = 0;
