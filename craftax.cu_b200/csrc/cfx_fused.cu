@@ -246,10 +246,8 @@ struct Smem {
 // the three copy-issuing threads (weights, loads, stores): no back-off between probes
 #define CFX_WAIT_FAST(barid, parity, code) \
     if (!mbar_wait<false>(sm.bar(barid), (parity), sm.abort_flag(), (code))) return
-// The MMA role runs on ONE thread; the other lanes of its warp go straight to the exit.  (A
-// converged warp with an elected lane, one shuffle per wait and a __syncwarp per stage, was
-// 10 % slower end to end.)  It polls with test_wait: it never suspends.  The first probe is
-// inline: almost every wait of this thread finds its barrier complete (5 failed probes in the
+// The MMA warp polls with test_wait: it never suspends.  The first probe is
+// inline: almost every wait of this warp finds its barrier complete (5 failed probes in the
 // 32 weight waits of a tile), and the bounded loop costs ~150 cycles more than one probe.
 #define CFX_WAIT_LEADER(barid, parity, code)                                          \
     if (!mbar_test_wait(sm.bar(barid), (parity)) &&                                   \
@@ -512,7 +510,12 @@ __device__ __forceinline__ void role_stores(const Smem& sm, const Params& P) {
 }
 
 // ------------------------------------------------------------------ MMA role
-// One thread issues every MMA of the CTA.  The tensor pipe queues about eight MMAs, so the
+// The whole warp walks through the steps, so that the compiler keeps descriptors and ring positions in uniform
+// registers, and an elected lane issues every MMA of the CTA (262,144 envs h256x2 421 -> 412 us against one lane walking
+// alone, 131,104 h128x2 bf16 123.1 -> 119.8, 65,536 h256x3 150.3 -> 148.5, classic 1,048,576 2,284 -> 2,236).  With every ring
+// position a compile-time constant, the encoder and the four slices unrolled, the code is no faster and larger (417,
+// 120.1, 148.8, 2,224).
+// The tensor pipe queues about eight MMAs, so the
 // issuer runs ahead of it as long as its own loop is short: descriptors are one add away from
 // a per-slot base and every K-step loop is fully unrolled (rebuilding descriptors per MMA
 // measured ~150 cycles per instruction on B200, against 45-50 for the bare instruction), and
@@ -545,7 +548,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
     const uint64_t bdesc0 = smem_desc_sw128(smem_u32(sm.b_ring()));
     uint32_t acnt = 0, akb_use = 0, gcnt = 0, tcnt = 0;
     // position in the weight ring of the stage being consumed: slot and phase parity, advanced
-    // incrementally (a division per stage on this thread would sit on the critical path)
+    // incrementally (a division per stage of this warp would sit on the critical path)
     int bslot = 0;
     uint32_t bpar = 0;
     auto b_advance = [&]() {
@@ -581,22 +584,26 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         // ---- encoder: N = kH units; one weight stage (two blocks of 64 K columns) per two
         // chunks, except the full game's last stage, which four short chunks consume
         // one operand chunk: wait for it, issue its K steps against the block at descriptor bd
-#define CFX_ENC_CHUNK(kc, bd, ksteps)                                                              \
+#define CFX_ENC_CHUNK(kc, bd, ksteps, last)                                                        \
         {                                                                                          \
             const int as = acnt % kAexpSlots;                                                      \
             CFX_WAIT_PROBED(cfx_p_a, AEXP_FULL + as, (acnt / kAexpSlots) & 1, W_AEXP_FULL);        \
             CFX_MARK(2);                                                                           \
-            tc_fence_after_sync();                                                                 \
             if ((kc) + 1 < kEncChunks) probe_a(acnt + 1);                                          \
+            tc_fence_after_sync();                                                                 \
+            __syncwarp();                                                                          \
             const uint32_t a_col = tmem + kColAexp + as * 32;                                      \
-            if ((kc) == 0) MMA_TS(tmem + kColAcc, a_col, (bd), idesc_enc, 0);                      \
-            else MMA_TS(tmem + kColAcc, a_col, (bd), idesc_enc, 1);                                \
-            if ((ksteps) > 1) {                                                                    \
-                MMA_TS(tmem + kColAcc, a_col + 8, (bd) + 2, idesc_enc, 1);                         \
-                MMA_TS(tmem + kColAcc, a_col + 16, (bd) + 4, idesc_enc, 1);                        \
+            if (elect_one()) {                                                                     \
+                MMA_TS(tmem + kColAcc, a_col, (bd), idesc_enc, (kc) == 0 ? 0u : 1u);               \
+                if ((ksteps) > 1) {                                                                \
+                    MMA_TS(tmem + kColAcc, a_col + 8, (bd) + 2, idesc_enc, 1);                     \
+                    MMA_TS(tmem + kColAcc, a_col + 16, (bd) + 4, idesc_enc, 1);                    \
+                }                                                                                  \
+                if ((ksteps) > 3) MMA_TS(tmem + kColAcc, a_col + 24, (bd) + 6, idesc_enc, 1);      \
+                MMA_COMMIT(sm.bar(AEXP_EMPTY + as));                                               \
+                if (last) MMA_COMMIT(sm.bar(B_EMPTY + slot));                                      \
+                if ((kc) == kEncChunks - 1) MMA_COMMIT(sm.bar(ACC_FULL));                          \
             }                                                                                      \
-            if ((ksteps) > 3) MMA_TS(tmem + kColAcc, a_col + 24, (bd) + 6, idesc_enc, 1);          \
-            MMA_COMMIT(sm.bar(AEXP_EMPTY + as));                                                   \
             acnt++;                                                                                \
             CFX_MARK(4);                                                                           \
         }
@@ -613,9 +620,8 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                 const int kc = kStageBlocks * kp + c2;
                 // the classic game's last chunk carries one feature (one K step)
                 const int ksteps = GAME == CFX_GAME_CLASSIC && kc == kEncChunks - 1 ? 1 : 4;
-                CFX_ENC_CHUNK(kc, bd0 + (uint64_t)(c2 * kEncBlkStep), ksteps);
+                CFX_ENC_CHUNK(kc, bd0 + (uint64_t)(c2 * kEncBlkStep), ksteps, c2 == kStageBlocks - 1);
             }
-            MMA_COMMIT(sm.bar(B_EMPTY + slot));
         }
         if constexpr (GAME == CFX_GAME_FULL) {
             // blocks 12 and 13: chunk 12 = K columns 0-47 of block 12 (three K steps), chunk 13
@@ -626,14 +632,12 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
             probe_b_next();
             b_advance();
             const uint64_t bd0 = bdesc0 + (uint64_t)(slot * (kBSlot >> 4));
-            CFX_ENC_CHUNK(12, bd0, 3);
-            CFX_ENC_CHUNK(13, bd0 + 6, 1);
-            CFX_ENC_CHUNK(14, bd0 + (uint64_t)kEncBlkStep, 1);
-            CFX_ENC_CHUNK(15, bd0 + (uint64_t)(kEncBlkStep + 2), 1);
-            MMA_COMMIT(sm.bar(B_EMPTY + slot));
+            CFX_ENC_CHUNK(12, bd0, 3, false);
+            CFX_ENC_CHUNK(13, bd0 + 6, 1, false);
+            CFX_ENC_CHUNK(14, bd0 + (uint64_t)kEncBlkStep, 1, false);
+            CFX_ENC_CHUNK(15, bd0 + (uint64_t)(kEncBlkStep + 2), 1, true);
         }
 #undef CFX_ENC_CHUNK
-        MMA_COMMIT(sm.bar(ACC_FULL));
 
         // ---- MinGRU layers: 4 slices of 64 units, one stage per two K blocks, N = 192 (zh|zg|zp)
         for (int l = 0; l < P.L; l++, akb_use++) {
@@ -667,16 +671,19 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                             CFX_MARK(9);
                         }
                         tc_fence_after_sync();
+                        __syncwarp();
+                        if (elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < 4; ks++)
-                            MMA_TS(tmem + kColG, a_cur + kb * 32 + ks * 8,
-                                   bd0 + (uint64_t)(c2 * kGateBlkStep + 2 * ks), idesc_gate,
-                                   (kb | ks) != 0 ? 1u : 0u);
+                            for (int ks = 0; ks < 4; ks++)
+                                MMA_TS(tmem + kColG, a_cur + kb * 32 + ks * 8,
+                                       bd0 + (uint64_t)(c2 * kGateBlkStep + 2 * ks), idesc_gate,
+                                       (kb | ks) != 0 ? 1u : 0u);
+                            if (c2 == kStageBlocks - 1) MMA_COMMIT(sm.bar(B_EMPTY + slot));
+                            if (kb == kKBlocks - 1) MMA_COMMIT(sm.bar(G_FULL));
+                        }
                     }
-                    MMA_COMMIT(sm.bar(B_EMPTY + slot));
                     CFX_MARK(7);
                 }
-                MMA_COMMIT(sm.bar(G_FULL));
             }
         }
         // ---- heads: N = 48 (64 in a pair), one stage with all K blocks
@@ -691,15 +698,20 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
             for (int kb = 0; kb < kKBlocks; kb++) {
                 CFX_WAIT_LEADER(A_KB + kb, akb_use & 1, W_A_KB);
                 tc_fence_after_sync();
+                __syncwarp();
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 4; ks++)
-                    MMA_TS(tmem + kColHead, a_cur + kb * 32 + ks * 8,
-                           bd + (uint64_t)((kb * C::kHeadKbBytes + ks * 32) >> 4), idesc_head,
-                           (kb | ks) != 0 ? 1u : 0u);
+                    for (int ks = 0; ks < 4; ks++)
+                        MMA_TS(tmem + kColHead, a_cur + kb * 32 + ks * 8,
+                               bd + (uint64_t)((kb * C::kHeadKbBytes + ks * 32) >> 4), idesc_head,
+                               (kb | ks) != 0 ? 1u : 0u);
+                    if (kb == kKBlocks - 1) {
+                        MMA_COMMIT(sm.bar(B_EMPTY + slot));
+                        MMA_COMMIT(sm.bar(H_FULL));
+                    }
+                }
             }
             akb_use++;
-            MMA_COMMIT(sm.bar(B_EMPTY + slot));
-            MMA_COMMIT(sm.bar(H_FULL));
             CFX_MARK(8);
         }
     }
@@ -1083,7 +1095,7 @@ k_policy_fused(const __grid_constant__ Params P) {
     if (warp == 0) {
         if (lane == 0) role_weight_loads<PAIR, GAME, HID>(sm, P, lane, rank, bar0_cta0);
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) role_mma<T16, PAIR, GAME, HID>(sm, P, tmem);
+        if (rank == 0) role_mma<T16, PAIR, GAME, HID>(sm, P, tmem);
     } else if (warp == 2) {
         wait_for_previous_kernel();
         if (lane == 0) role_loads<PAIR, GAME, HID>(sm, P);
