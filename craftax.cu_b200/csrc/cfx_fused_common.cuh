@@ -19,7 +19,7 @@ namespace fused {
 constexpr int kTile = 128;       // envs per tile
 constexpr int kMaxLayers = 4;
 constexpr int kSliceUnits = 64;  // hidden units per gate slice (N = 192: zh|zg|zp)
-constexpr int kHalfUnits = 32;   // units of a slice handled by one worker warpgroup
+constexpr int kHalfUnits = 32;   // units of half a slice, and of a state box
 constexpr int kHeadMax = 64;     // head accumulator columns reserved in tensor memory
 // Shapes that follow from the hidden size the kernel is instantiated for (256 or 128).
 template <int HID> struct Hd {
@@ -28,15 +28,14 @@ template <int HID> struct Hd {
     static constexpr int kSlices = HID / kSliceUnits;     // gate slices per layer (4 / 2)
     static constexpr int kStateItems = HID / kHalfUnits;  // state boxes (128 rows x 32 units) per layer (8 / 4)
     static constexpr int kKBlocks = HID / 64;             // K blocks of 64 per HID-wide operand (4 / 2)
-    static constexpr int kEncBlockBytes = HID * 128;      // one encoder chunk: [HID units][64 K] 16-bit
-    static constexpr int kEncCopyBytes = 2 * HID * 128;   // encoder stage: two chunks
+    static constexpr int kEncBlockBytes = HID * 128;      // one encoder block: [HID units][64 K] 16-bit
     static_assert((HID / 64) % 2 == 0, "a gate stage carries two K blocks");
 };
 // brings the shapes of Hd<HID> into a function body
 #define CFX_DIMS(HID)                                                                        \
     constexpr int kH = Hd<HID>::kH, kSlices = Hd<HID>::kSlices, kStateItems = Hd<HID>::kStateItems, \
-                  kKBlocks = Hd<HID>::kKBlocks, kEncCopyBytes = Hd<HID>::kEncCopyBytes;      \
-    (void)kH; (void)kSlices; (void)kStateItems; (void)kKBlocks; (void)kEncCopyBytes
+                  kKBlocks = Hd<HID>::kKBlocks;                                              \
+    (void)kH; (void)kSlices; (void)kStateItems; (void)kKBlocks
 
 // What differs between the two games the kernel is instantiated for.
 //  full game (craftax_full.cu): 996-byte record = 792 map bytes + 51 raw floats, 843 features.
@@ -59,23 +58,18 @@ template <> struct Gm<CFX_GAME_CLASSIC> {
     static constexpr int kHeadSingle = 32, kHeadPair = 32;
 };
 
-// record boxes in shared memory: 32 rows x 80 bytes, four per 64-byte chunk of the 128 records of a tile
-constexpr int kRBoxBytes = 32 * 80, kRSlot = 4 * kRBoxBytes;
-// Image blocks (one K block of 64 columns each) and the ring stages that carry them.  A stage
-// holds TWO blocks, so that the MMA thread waits, probes and commits once per eight MMAs:
-// encoder stage = two chunks of 256 units (2 x 32 KB); gate stage = two K blocks of one 64-unit
-// slice (2 x 192 rows, 2 x 24 KB); head stage = all K blocks.  One CTA per tile stages whole
-// stages, [block][rows][64 K]; in a CTA pair every CTA stages its half of the rows of both
-// blocks, laid out [half][block][rows / 2][64 K] so that a CTA's part is one contiguous copy.
-constexpr int kStageBlocks = 2;
+// Image: blocks of 64 K columns, each a K-major, 128-byte-swizzled operand tile.  Encoder [block][HID units]; gate layers
+// [layer][slice of 64 units][K block][192 rows], where the rows are zh|zg|zp of 16 units, the units that one worker warp
+// handles, and then of the next 16: half of a slice is the 96 columns of one accumulator in cfx_fused.cu; heads.
 constexpr int kGateBlockBytes = 3 * kSliceUnits * 128;               // block: [192 rows][64 K]
-constexpr int kGateStageBytes = kStageBlocks * kGateBlockBytes;
+constexpr int kWarpUnits = 16;                                       // units of a slice that one worker warp handles
+// row (accumulator column) of a gate (0 zh, 1 zg, 2 zp) of a slice's unit
+__host__ __device__ constexpr int gate_row(int gate, int unit) { return (unit / kWarpUnits * 3 + gate) * kWarpUnits + unit % kWarpUnits; }
 // head stage: one CTA per tile [K block][rows][64 K]; pairs [half][K block][rows / 2][64 K]
 template <int GAME, int HID> __host__ __device__ constexpr int head_bytes(bool pair) {
     return Hd<HID>::kKBlocks * (pair ? Gm<GAME>::kHeadPair : Gm<GAME>::kHeadSingle) * 128;
 }
 template <int GAME, int HID> __host__ __device__ constexpr size_t enc_bytes() {
-    static_assert(Gm<GAME>::kEncBlocks % 2 == 0, "an encoder stage carries two blocks");
     return (size_t)Gm<GAME>::kEncBlocks * Hd<HID>::kEncBlockBytes;
 }
 
@@ -85,12 +79,11 @@ template <int GAME, int HID> __host__ __device__ constexpr size_t image_bytes(in
 }
 
 struct Params {
-    CUtensorMap rec_map;                 // uint8 [n/4][3984], box 32 x 80
-    // pair mode: the operand image as [rows][64] 16-bit tensors, one map per region (encoder,
+    // pair mode: the operand image as [blocks][rows][64] 16-bit tensors, one map per region (encoder,
     // gate layers, heads); a box is the part of a stage that one CTA of the pair copies
     CUtensorMap w_map[3];
     CUtensorMap state_map[kMaxLayers];   // fp32 [n][256] per layer, box 128 x 32, SWIZZLE_128B
-    const uint8_t* records;              // [n][996], for the L2 prefetch of the next tile
+    const uint8_t* records;              // [n][996] (classic [n][148])
     const float* state;                  // [L][n][256]
     const uint8_t* image;                // pre-swizzled 16-bit weight stages in consumption order
     const float* params;                 // fp32 arena (biases are read from it)
@@ -112,7 +105,6 @@ struct Params {
     int n, L, num_tiles;  // num_tiles: end of the tile range of this launch (exclusive)
     int tile_begin;       // first tile of this launch (a launch may cover a slice of the envs)
     int tile_rows;        // small-batch form: rows of a tile
-    int rec_bytes;        // bytes of one record (996 full game, 148 classic)
     int num_tiles_loop;   // trip bound of the tile loops: num_tiles, rounded up to even for CTA pairs
     size_t off_b_enc, off_b_a, off_b_v;
 };
@@ -279,6 +271,26 @@ __device__ __forceinline__ void expand_full(const uint8_t* src, int kc, uint32_t
                 regs[q] = Op::pack(__uint_as_float(word(2 * q)), __uint_as_float(word(2 * q + 1)));
             regs[4] = Op::pack(__uint_as_float(word(8)), 0.0f);
         }
+    }
+}
+// Weight block kc of the full game whole, from a record (chunks 12 and 13, 14 and 15 share one)
+template <typename Op>
+__device__ __forceinline__ void expand_block(const uint8_t* rec, int kc, uint32_t (&regs)[32]) {
+    if (kc < 13) {
+        expand_full<Op>(rec + 64 * kc, kc, regs);
+        if (kc < 12) return;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 32; q++) regs[q] = 0u;
+    }
+    const float* f = reinterpret_cast<const float*>(rec + kMap);   // (4-byte aligned)
+    if (kc == 12) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) regs[24 + q] = Op::pack(f[10 + 2 * q], f[11 + 2 * q]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 12; q++) regs[q] = Op::pack(f[26 + 2 * q], f[27 + 2 * q]);
+        regs[12] = Op::pack(f[50], 0.0f);
     }
 }
 // K steps of 16 columns that chunk kc of the full game feeds

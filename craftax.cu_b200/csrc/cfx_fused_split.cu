@@ -40,7 +40,6 @@ namespace fused {
 namespace split {
 
 constexpr int kWorkerWarp0 = 4, kWorkerWarps = 16, kThreads = (kWorkerWarp0 + kWorkerWarps) * 32;
-constexpr int kWarpUnits = 16;                       // units of a 64-unit slice that one worker warp handles
 constexpr int kABlock = kTile * 128;                 // K block of the layer input: [128 rows][64 K]
 constexpr int kWSlots = 4, kWSlot = kGateBlockBytes; // weight ring: one gate K block (24 KB) a slot
 constexpr int kMaxChunks = Gm<CFX_GAME_CLASSIC>::kEncChunks;
@@ -48,6 +47,12 @@ constexpr int kASlots = 12;                          // operand chunks in tensor
 constexpr int kSSlots = 4, kSBox = kTile * 128, kQuadBox = 32 * 128;   // state ring: 128 rows x 32 units a slot, copied 32 rows at a time
 constexpr uint32_t kColAexp = 0, kColAcc = 384, kColHead = 448;
 __host__ __device__ constexpr uint32_t col_gate(int j) { return 192u * (uint32_t)j; }   // over the operand chunks, done by then
+
+// 96 registers a thread at launch, then 64 for the four warps that copy and multiply and 104 for the sixteen workers, whose
+// cells need no local memory with them where a CTA has two slices (8,192 envs 21.8 -> 21.0 us).  Not in tiles of 32 rows, which
+// need fewer, and not in cfx_fused.cu, whose MMA warp is slower with 64 (262,144 envs 406 -> 418).
+constexpr int kLaunchRegs = 96, kRoleRegs = 64, kWorkerRegs = 104;
+static_assert(kWorkerWarp0 * kRoleRegs + kWorkerWarps * kWorkerRegs <= (kWorkerWarp0 + kWorkerWarps) * kLaunchRegs, "registers");
 
 constexpr int kQuadBlock = 32 * 128;                  // ONE: an operand chunk's block, [32 rows][64 K]
 constexpr uint32_t kColA = 192;                       // ONE: layer input, 32 columns a K block
@@ -141,12 +146,12 @@ template <int S, bool ONE> __device__ __forceinline__ bool has_heads(int quads, 
 }
 
 // ------------------------------------------------------------------ weights
-// The operand image is the one the CTA pairs of cfx_fused.cu use: stages of two blocks, every block in two halves of
-// rows.  A CTA's rows of an encoder block are contiguous in it, a gate K block is two pieces.
+// The operand image is the one that cfx_fused.cu uses.  A CTA's rows of an encoder block are contiguous in it, and so is a
+// gate K block.
 template <int GAME, int HID, int S, bool ONE>
 __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, uint32_t rank) {
     using C = Cfg<GAME, HID, S>;
-    constexpr int kSlices = HID / 64, kHalf = HID / 2;
+    constexpr int kSlices = HID / 64;
     constexpr size_t enc_b = enc_bytes<GAME, HID>();
     const int gates = P.L * C::kNS * C::kKB;
     const int items = C::kEncItems + gates + (has_heads<S, ONE>(P.tile_rows / 32, rank) ? C::kHeadItems : 0);
@@ -160,17 +165,16 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
             mbar_arrive_expect_tx(full, blocks * C::kEncTile);
             for (int b = 0; b < blocks; b++) {
                 const int blk = i * C::kEncPerItem + b;
-                const size_t off = (size_t)(blk / 2) * Hd<HID>::kEncCopyBytes +
-                                   (size_t)((u0 / kHalf) * 2 + (blk & 1)) * (kHalf * 128) + (size_t)(u0 % kHalf) * 128;
+                const size_t off = (size_t)blk * Hd<HID>::kEncBlockBytes + (size_t)u0 * 128;
                 bulk_g2s(dst + b * C::kEncTile, P.image + off, C::kEncTile, full);
             }
         } else if (i < C::kEncItems + gates) {
             const int g = i - C::kEncItems, kb = g % C::kKB, j = g / C::kKB % C::kNS, l = g / (C::kKB * C::kNS);
-            const int stage = (l * kSlices + (int)rank * C::kNS + j) * (C::kKB / 2) + kb / 2;
-            const uint8_t* src = P.image + enc_b + (size_t)stage * kGateStageBytes + (size_t)(kb & 1) * (kGateBlockBytes / 2);
+            const int blk = (l * kSlices + (int)rank * C::kNS + j) * C::kKB + kb;
             mbar_arrive_expect_tx(full, kGateBlockBytes);
+            const uint8_t* src = P.image + enc_b + (size_t)blk * kGateBlockBytes;
             bulk_g2s(dst, src, kGateBlockBytes / 2, full);
-            bulk_g2s(dst + kGateBlockBytes / 2, src + kGateBlockBytes, kGateBlockBytes / 2, full);
+            bulk_g2s(dst + kGateBlockBytes / 2, src + kGateBlockBytes / 2, kGateBlockBytes / 2, full);
         } else {
             const int h = i - C::kEncItems - gates;
             const uint8_t* src = P.image + enc_b + (size_t)P.L * kSlices * C::kKB * kGateBlockBytes;
@@ -491,9 +495,9 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             CFX_SWAIT(G_FULL + j, l & 1);
             tc_fence_after_sync();
             uint32_t zh[16], zg[16], zp[16];
-            tmem_ld16(lane_base + col_gate(j) + kWarpUnits * wg, zh);
-            tmem_ld16(lane_base + col_gate(j) + kSliceUnits + kWarpUnits * wg, zg);
-            tmem_ld16(lane_base + col_gate(j) + 2 * kSliceUnits + kWarpUnits * wg, zp);
+            tmem_ld16(lane_base + col_gate(j) + gate_row(0, kWarpUnits * wg), zh);
+            tmem_ld16(lane_base + col_gate(j) + gate_row(1, kWarpUnits * wg), zg);
+            tmem_ld16(lane_base + col_gate(j) + gate_row(2, kWarpUnits * wg), zp);
             tmem_wait_ld();
             uint8_t* sp = sm.base + C::kOffS + slot * kSBox + (row >> 3) * 1024 + (row & 7) * 128;
             auto piece = [&](int q) { return reinterpret_cast<float4*>(sp + (((4 * (wg & 1) + q) ^ (row & 7)) << 4)); };
@@ -749,9 +753,9 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         CFX_SWAIT(G_FULL, l & 1);
         tc_fence_after_sync();
         uint32_t zh[4], zg[4], zp[4];
-        tmem_ld4(lane_base + col_gate(0) + unit, zh);
-        tmem_ld4(lane_base + col_gate(0) + kSliceUnits + unit, zg);
-        tmem_ld4(lane_base + col_gate(0) + 2 * kSliceUnits + unit, zp);
+        tmem_ld4(lane_base + col_gate(0) + gate_row(0, unit), zh);
+        tmem_ld4(lane_base + col_gate(0) + gate_row(1, unit), zg);
+        tmem_ld4(lane_base + col_gate(0) + gate_row(2, unit), zp);
         tmem_wait_ld();
         const float2 x01 = Op::unpack(x.x), x23 = Op::unpack(x.y);
         float h0, h1, h2, h3;
@@ -832,35 +836,39 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
 
     // The operand image and the biases are only ever written by calls that wait for the device, so they may be
     // read while the kernel in front still runs; everything else waits for it.
-    if (warp == 0) {
-        if (lane == 0) role_weights<GAME, HID, S, ONE>(sm, P, rank);
-        __syncwarp();
-        cluster_wait();
-    } else if (warp == 1) {
-        cluster_wait();
-        role_mma<T16, GAME, HID, S, ONE>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
-    } else if (warp == 2) {
-        // the tile's records, 32 rows a copy
-        wait_for_previous_kernel();
-        if (lane < quads && row0 + 32 * lane < P.n) {
-            mbar_arrive_expect_tx(sm.bar(REC_FULL + lane), C::kQuadBytes);
-            bulk_g2s(smem_u32(sm.base + lane * C::kQuadBytes), P.records + ((size_t)row0 + 32 * lane) * C::kRowBytes,
-                     C::kQuadBytes, sm.bar(REC_FULL + lane));
+    if (warp < kWorkerWarp0) {
+        if constexpr (!ONE) registers_dec<kRoleRegs>();
+        if (warp == 0) {
+            if (lane == 0) role_weights<GAME, HID, S, ONE>(sm, P, rank);
+            __syncwarp();
+            cluster_wait();
+        } else if (warp == 1) {
+            cluster_wait();
+            role_mma<T16, GAME, HID, S, ONE>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
+        } else if (warp == 2) {
+            // the tile's records, 32 rows a copy
+            wait_for_previous_kernel();
+            if (lane < quads && row0 + 32 * lane < P.n) {
+                mbar_arrive_expect_tx(sm.bar(REC_FULL + lane), C::kQuadBytes);
+                bulk_g2s(smem_u32(sm.base + lane * C::kQuadBytes), P.records + ((size_t)row0 + 32 * lane) * C::kRowBytes,
+                         C::kQuadBytes, sm.bar(REC_FULL + lane));
+            }
+            for (int i = lane; i < C::kUnits + kA + 1; i += 32) {
+                const int a = i - C::kUnits;
+                reinterpret_cast<float*>(sm.base + C::kOffBias)[i] =
+                    P.params[a < 0 ? P.off_b_enc + C::kUnits * rank + i : (a < kA ? P.off_b_a + a : P.off_b_v)];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sm.bar(ACC_FULL));
+            __syncwarp();
+            cluster_wait();
+        } else if (warp == 3) {
+            wait_for_previous_kernel();
+            cluster_wait();
+            if (lane == 0) role_state<GAME, HID, S, ONE>(sm, P, row0, rank);
         }
-        for (int i = lane; i < C::kUnits + kA + 1; i += 32) {
-            const int a = i - C::kUnits;
-            reinterpret_cast<float*>(sm.base + C::kOffBias)[i] =
-                P.params[a < 0 ? P.off_b_enc + C::kUnits * rank + i : (a < kA ? P.off_b_a + a : P.off_b_v)];
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(sm.bar(ACC_FULL));
-        __syncwarp();
-        cluster_wait();
-    } else if (warp == 3) {
-        wait_for_previous_kernel();
-        cluster_wait();
-        if (lane == 0) role_state<GAME, HID, S, ONE>(sm, P, row0, rank);
     } else {
+        if constexpr (!ONE) registers_inc<kWorkerRegs>();
         wait_for_previous_kernel();
         cluster_wait();
         Meetings meet;
@@ -938,6 +946,12 @@ int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_
     CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     k = split::kernel(precision, game, H, S, false, &smem);
     CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaFuncAttributes attr;
+    CFX_CUDA(cudaFuncGetAttributes(&attr, k));
+    if (attr.numRegs < split::kLaunchRegs) {   // (its warps would wait for registers that do not exist)
+        set_error("small-batch kernel: built with fewer registers than its warps share out");
+        return CFX_ERR_CUDA;
+    }
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = split::config(at, sm_count / S * S, S, smem, nullptr);
     cfg.numAttrs = 1;

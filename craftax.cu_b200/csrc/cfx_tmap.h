@@ -42,4 +42,17 @@ inline bool make_tmap_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_byte
     return r == CUDA_SUCCESS;
 }
 
+// Blocks of rows of 64 16-bit elements (128 bytes), all contiguous: [blocks][rows][64]; box = [box_blocks][box_rows][64].
+inline bool make_tmap_blocks(CUtensorMap* map, void* base, uint64_t blocks, uint64_t rows, uint32_t box_blocks, uint32_t box_rows) {
+    PFN_encodeTiled enc = get_encode_tiled();
+    if (!enc) return false;
+    cuuint64_t dims[3] = {64, rows, blocks};
+    cuuint64_t strides[2] = {128, rows * 128};
+    cuuint32_t box[3] = {64, box_rows, box_blocks};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS;
+}
+
 }  // namespace cfx

@@ -172,6 +172,12 @@ __device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity,
     }
 }
 
+// ------------------------------------------------------------------ registers
+// A warpgroup (four warps from a multiple of four on, all of them) gives registers back to the block, or takes
+// some of those: `inc` waits until they are there, so the shares must fit into what the block was launched with.
+template <int N> __device__ __forceinline__ void registers_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void registers_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ------------------------------------------------------------------ fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -211,15 +217,15 @@ __device__ __forceinline__ void tensor_g2s_2d(uint32_t dst_smem, const CUtensorM
         "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
-// The same copy issued by a CTA of a pair (cta_group::2): the data lands in the issuing CTA's
+// 3-D, issued by a CTA of a pair (cta_group::2): the data lands in the issuing CTA's
 // shared memory, the completion (complete_tx) may be counted on an mbarrier of EITHER CTA of
 // the pair; `cluster_bar` is a shared::cluster address (mapa).  No multicast.
-__device__ __forceinline__ void tensor_g2s_2d_pair(uint32_t dst_smem, const CUtensorMap* map, int x,
-                                                   int y, uint32_t cluster_bar) {
+__device__ __forceinline__ void tensor_g2s_3d_pair(uint32_t dst_smem, const CUtensorMap* map, int x,
+                                                   int y, int z, uint32_t cluster_bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
-        "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst_smem),
-        "l"(map), "r"(x), "r"(y), "r"(cluster_bar)
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst_smem),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(cluster_bar)
         : "memory");
 }
 // 2-D tiled tensor copy shared -> global (bulk async-group completion).
