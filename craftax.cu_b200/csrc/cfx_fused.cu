@@ -1025,6 +1025,7 @@ struct FusedPlan {
     CUtensorMap state_map[fused::kMaxLayers];
     CUtensorMap quad_map[fused::kMaxLayers];   // the same with boxes of 32 rows
     CUtensorMap w_map[3];          // pair mode: operand image regions (encoder, gates, heads)
+    CUtensorMap gate_map[2];       // tiles of 32 rows: see fused::Params
     int sm_count = 0;
     int pair = 0;        // 1: launch as clusters of two CTAs (cta_group::2 MMAs)
     int max_pairs = 0;   // co-resident clusters of two
@@ -1139,6 +1140,7 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
         }
     }
     memset(p->w_map, 0, sizeof(p->w_map));
+    memset(p->gate_map, 0, sizeof(p->gate_map));
     if (p->pair) {
         // The operand image seen as blocks of rows of 64 16-bit values (128 bytes), one tensor per region;
         // a box is what ONE CTA of a pair copies of a stage.  The image is already
@@ -1156,6 +1158,12 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
             if (!make_tmap_blocks(&p->w_map[r], base, blocks[r], rows[r], box_blocks[r], box_rows[r])) {
                 fused_destroy(p);
                 set_error("fused_create: cuTensorMapEncodeTiled failed for the operand image");
+                return CFX_ERR_CUDA;
+            }
+            if (r == 1 && !(make_tmap_parts(&p->gate_map[0], base, blocks[r] * (fused::kSliceUnits / fused::kWarpUnits), 3, fused::kWarpUnits, 4, 2) &&
+                            make_tmap_parts(&p->gate_map[1], base, blocks[r] * (fused::kSliceUnits / fused::kWarpUnits), 3, fused::kWarpUnits, 4, 1))) {
+                fused_destroy(p);
+                set_error("fused_create: cuTensorMapEncodeTiled failed for the gate blocks");
                 return CFX_ERR_CUDA;
             }
             base += blocks[r] * rows[r] * 128;
@@ -1202,6 +1210,7 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     }
     for (int l = 0; l < p->L; l++) P.state_map[l] = p->state_map[l];
     for (int r = 0; r < 3; r++) P.w_map[r] = p->w_map[r];
+    for (int r = 0; r < 2; r++) P.gate_map[r] = p->gate_map[r];
     const ArenaLayout o = ArenaLayout::make(p->H, p->L, p->A, classic ? kClassicObs : kObs);
     P.records = a.records;
     P.state = a.state;

@@ -82,6 +82,8 @@ struct Params {
     // pair mode: the operand image as [blocks][rows][64] 16-bit tensors, one map per region (encoder,
     // gate layers, heads); a box is the part of a stage that one CTA of the pair copies
     CUtensorMap w_map[3];
+    // small-batch form, tiles of 32 rows: the gate blocks as [16 units][gate][16 rows]; a box is zh and zg, or zp, of a slice
+    CUtensorMap gate_map[2];
     CUtensorMap state_map[kMaxLayers];   // fp32 [n][256] per layer, box 128 x 32, SWIZZLE_128B
     const uint8_t* records;              // [n][996] (classic [n][148])
     const float* state;                  // [L][n][256]

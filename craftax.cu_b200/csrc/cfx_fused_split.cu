@@ -22,9 +22,11 @@
 // layer.  The products of a row are accumulated in the order of cfx_fused.cu: same bits.
 // Tiles of 32 rows (ONE), the smallest batches: a quadrant of TMEM lanes belongs to one SM scheduler, so one
 // quadrant of rows would leave three schedulers idle.  The operand chunks go to shared memory instead, one of the sixteen
-// warps a chunk; and the layers' A operand is tensor memory again, where every quadrant gets a copy of the 32
-// rows: each quadrant's lanes then hold the gates of all rows, and its warps do a quarter of the units
-// (1,024 envs h256x2 15.5 -> 13.6 us).  The layer input has two buffers there, beside the records.
+// warps a chunk, and all multiplications are the weight-stationary ones of 32 rows: their columns are spread over the
+// quadrants, so every warp has four of a slice's units, and they are shorter (an encoder step 29 cycles instead of 49,
+// one of the gates 73 instead of 96).  A slice's zh and zg are one product of 128 columns and its zp one of 64; the weights' copies
+// put the units of a quadrant together (1,024 envs h256x2 12.7 -> 11.6 us, against products of 128 rows with a copy of the layer
+// input in every quadrant of tensor memory).  The layer input has two buffers there, beside the records.
 // The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
 // records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
@@ -55,7 +57,8 @@ constexpr int kLaunchRegs = 96, kRoleRegs = 64, kWorkerRegs = 104;
 static_assert(kWorkerWarp0 * kRoleRegs + kWorkerWarps * kWorkerRegs <= (kWorkerWarp0 + kWorkerWarps) * kLaunchRegs, "registers");
 
 constexpr int kQuadBlock = 32 * 128;                  // ONE: an operand chunk's block, [32 rows][64 K]
-constexpr uint32_t kColA = 192;                       // ONE: layer input, 32 columns a K block
+constexpr uint32_t kGateB = 4 * 2 * kWarpUnits * 128;   // ONE: zh and zg of a slice, behind them its zp
+constexpr uint32_t kColP = 32;                        // ONE: columns of zh and zg in a quadrant, behind them zp
 
 template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kKB = HID / 64;                        // K blocks of a layer's input
@@ -70,10 +73,10 @@ template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kBoxes = 2 * kNS;                      // state boxes of a layer
     static constexpr int kOffS = kKB * kABlock, kASBytes = kOffS + kSSlots * kSBox;   // layer input, state; first the records
     static constexpr int kOffW = (kASBytes > 4 * kQuadBytes ? kASBytes : 4 * kQuadBytes + 1023) / 1024 * 1024;
-    // ONE: operand chunks; an MMA reads 96 rows beyond a block's 32, which nobody looks at.  The classic game's 22 blocks
+    // ONE: operand chunks.  The classic game's 22 blocks
     // reach from the records over the layer input, the full game's 14 lie where the state boxes are later
     static constexpr int kOffX = GAME == CFX_GAME_FULL ? kOffS : 8192;
-    static_assert(kOffX + (Gm<GAME>::kEncBlocks + 3) * kQuadBlock <= kOffW + kWSlots * kWSlot && 32 * Gm<GAME>::kRecBytes <= kOffX, "operand chunks");
+    static_assert(kOffX + Gm<GAME>::kEncBlocks * kQuadBlock <= kOffW && 32 * Gm<GAME>::kRecBytes <= kOffX, "operand chunks");
     // ONE: layer input l, K block kb, [32 rows][64 K]: two buffers in turn, so that nobody waits for the multiplications of
     // the layer before writing the next one's input; beside the records where there is room
     static constexpr bool kOneBeside = GAME == CFX_GAME_FULL && kOffS >= 32768 + kKB * 2 * kQuadBlock;
@@ -92,7 +95,7 @@ enum Bar {
     AEXP_FULL = REC_FREE + 1, AEXP_EMPTY = AEXP_FULL + kMaxChunks, ACC_FULL = AEXP_EMPTY + kASlots,
     S_FULL = ACC_FULL + 1, ST_READY = S_FULL + kSSlots, MMA_DONE = ST_READY + kSSlots,
     QUAD = MMA_DONE + 1, G_FULL = QUAD + 8,   // QUAD: [slice][quadrant]
-    H_FULL = G_FULL + 2, AT_KB = H_FULL + 1, A_KB = AT_KB + 4,   // AT_KB: ONE, K blocks of the layer input in tensor memory
+    H_FULL = G_FULL + 2, A_KB = H_FULL + 1,
     // A_KB: [layer input][K block]
     NUM_BARS = A_KB + (kMaxLayers + 1) * 4
 };
@@ -173,8 +176,13 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
             const int blk = (l * kSlices + (int)rank * C::kNS + j) * C::kKB + kb;
             mbar_arrive_expect_tx(full, kGateBlockBytes);
             const uint8_t* src = P.image + enc_b + (size_t)blk * kGateBlockBytes;
-            bulk_g2s(dst, src, kGateBlockBytes / 2, full);
-            bulk_g2s(dst + kGateBlockBytes / 2, src + kGateBlockBytes / 2, kGateBlockBytes / 2, full);
+            if constexpr (ONE) {
+                tensor_g2s_4d(dst, &P.gate_map[0], 0, 0, 0, 4 * blk, full);
+                tensor_g2s_4d(dst + kGateB, &P.gate_map[1], 0, 0, 2, 4 * blk, full);
+            } else {
+                bulk_g2s(dst, src, kGateBlockBytes / 2, full);
+                bulk_g2s(dst + kGateBlockBytes / 2, src + kGateBlockBytes / 2, kGateBlockBytes / 2, full);
+            }
         } else {
             const int h = i - C::kEncItems - gates;
             const uint8_t* src = P.image + enc_b + (size_t)P.L * kSlices * C::kKB * kGateBlockBytes;
@@ -205,8 +213,10 @@ template <typename T16, int GAME, int HID, int S, bool ONE>
 __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32_t tmem, uint32_t rank) {
     using C = Cfg<GAME, HID, S>;
     constexpr uint32_t fmt = Op16<T16>::kFmt;
-    constexpr uint32_t idesc_enc = make_idesc(fmt, kTile, C::kUnits), idesc_gate = make_idesc(fmt, kTile, 3 * kSliceUnits),
-                       idesc_head = make_idesc(fmt, kTile, Gm<GAME>::kHeadSingle);
+    constexpr int kRows = ONE ? 32 : kTile;
+    constexpr uint32_t idesc_enc = make_idesc(fmt, kRows, C::kUnits), idesc_gate = make_idesc(fmt, kTile, 3 * kSliceUnits),
+                       idesc_hg = make_idesc(fmt, kRows, 2 * kSliceUnits), idesc_p = make_idesc(fmt, kRows, kSliceUnits),
+                       idesc_head = make_idesc(fmt, kRows, ONE ? 64 : Gm<GAME>::kHeadSingle);   // (M = 32 takes N = 64, 128 or 256)
     constexpr int kChunks = Gm<GAME>::kEncChunks, kGateItems = C::kNS * C::kKB;
     static_assert(kGateItems % kWSlots == 0 || kWSlots % kGateItems == 0, "a layer's first ring slot");
     const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
@@ -236,7 +246,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 #pragma unroll
             for (int k = 0; k < ks; k++) {
                 if constexpr (ONE)
-                    mma_f16_ss(tmem + kColAcc, xdesc + (uint64_t)(((blk * kQuadBlock) >> 4) + first + 2 * k), bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+                    mma_f16_ws_ss(tmem + kColAcc, xdesc + (uint64_t)(((blk * kQuadBlock) >> 4) + first + 2 * k), bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
                 else
                     mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
             }
@@ -254,32 +264,32 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 #pragma unroll 1
     for (int l = 0; l < P.L; l++) {
         const int slot0 = first_slot(l);
-        if (!ONE) CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
+        CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
         // this CTA's own K blocks first: the gate columns are free when its cells have read them
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) CFX_SWAIT_SPIN(A_KB + 4 * l + (int)rank * C::kNS + j, 0);
-        if (ONE) CFX_SPROBE(cfx_p_a, AT_KB, l & 1);
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) {
 #pragma unroll
             for (int kb = 0; kb < C::kKB; kb++) {
                 const int slot = (slot0 + j * C::kKB + kb) % kWSlots, slot1 = (slot + 1) % kWSlots;
                 if (j == 0) {
-                    CFX_SWAIT_PROBED(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * l) + kb, ONE ? l & 1 : 0);
-                    if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * l) + kb + 1, ONE ? l & 1 : 0);
+                    CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * l + kb, 0);
+                    if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * l + kb + 1, 0);
                 }
                 CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, wpar >> slot & 1u);
                 wpar ^= 1u << slot;
                 CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
                 tc_fence_after_sync();
                 __syncwarp();
-                const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
+                const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)((ONE ? C::one_block(l, kb) : (uint32_t)(kb * kABlock)) >> 4);
                 if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < 4; ks++) {
-                        if constexpr (ONE)
-                            mma_f16_ts(tmem + col_gate(j), tmem + kColA + 32 * kb + 8 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
-                        else
+                        if constexpr (ONE) {
+                            mma_f16_ws_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_hg, (kb | ks) != 0 ? 1u : 0u);
+                            mma_f16_ws_ss(tmem + col_gate(j) + kColP, ad + 2 * ks, bd + (uint64_t)(kGateB >> 4) + 2 * ks, idesc_p, (kb | ks) != 0 ? 1u : 0u);
+                        } else
                             mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
                     }
                     if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL + j));
@@ -298,24 +308,24 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         return;
     }
     const int slot0 = first_slot(P.L);
-    CFX_SPROBE(cfx_p_a, ONE ? (int)AT_KB : A_KB + 4 * P.L, ONE ? P.L & 1 : 0);
+    CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L, 0);
 #pragma unroll
     for (int kb = 0; kb < C::kKB; kb++) {
         const int slot = (slot0 + kb / 2) % kWSlots, slot1 = (slot + 1) % kWSlots;
-        CFX_SWAIT_PROBED(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * P.L) + kb, ONE ? P.L & 1 : 0);
-        if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, (ONE ? AT_KB : A_KB + 4 * P.L) + kb + 1, ONE ? P.L & 1 : 0);
+        CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * P.L + kb, 0);
+        if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L + kb + 1, 0);
         if (kb % 2 == 0) {
             CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, wpar >> slot & 1u);
             CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
         }
         tc_fence_after_sync();
         __syncwarp();
-        const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
+        const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)((ONE ? C::one_block(P.L, kb) : (uint32_t)(kb * kABlock)) >> 4);
         if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < 4; ks++) {
                 if constexpr (ONE)
-                    mma_f16_ts(tmem + kColHead, tmem + kColA + 32 * kb + 8 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+                    mma_f16_ws_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
                 else
                     mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
             }
@@ -582,7 +592,7 @@ __device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t h
     float l[kCols], m = -INFINITY;
     if (w < kWith) {
         uint32_t t[kCols];
-        tmem_ld4(head + kCols * w, t);
+        tmem_ld4(head, t);
         tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < kCols; i++) {
@@ -617,9 +627,8 @@ __device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t h
     }
 }
 
-// ONE: warp (quadrant, wg) converts chunk 4 wg + quadrant (and the one 16 further), brings K block wg of every layer input
-// from shared memory to its quadrant's tensor memory, and handles units [16 wg + 4 quadrant, + 4) of the CTA's
-// slice; lane = row in all of it.
+// ONE: warp w = (quadrant, wg) converts chunk w (and the one 16 further) and handles units [4 w, 4 w + 4) of the CTA's
+// slice, which are in its quadrant of tensor memory; lane = row in all of it.
 template <typename T16, int GAME, int HID, int S>
 __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
                                                 uint32_t rank, Meetings& meet) {
@@ -627,7 +636,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     using C = Cfg<GAME, HID, S>;
     constexpr int kChunks = Gm<GAME>::kEncChunks, kA = Gm<GAME>::kA;
     constexpr bool kFull = GAME == CFX_GAME_FULL;
-    const int quadrant = warp & 3, wg = (warp - kWorkerWarp0) >> 2, w = 4 * wg + quadrant, swz = lane & 7;
+    const int quadrant = warp & 3, wg = (warp - kWorkerWarp0) >> 2, w = 4 * quadrant + wg, unit = 4 * w, swz = lane & 7;
     const uint32_t lane_base = tmem + ((uint32_t)(quadrant * 32) << 16);
     const int env = row0 + lane;
     const bool valid = env < P.n;   // all rows (n is a multiple of 32)
@@ -686,59 +695,31 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         }
         return __all_sync(0xffffffffu, ok);
     };
-    // K block wg of layer input l -> this quadrant's tensor memory
-    auto to_tmem = [&](int l) {
-        if (wg >= C::kKB) return true;
-        if (!mbar_wait<false>(sm.bar(A_KB + 4 * l + wg), 0, sm.abort_flag(), kSite + A_KB)) return false;
-        uint32_t lo[16], hi[16];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const uint4 a = *reinterpret_cast<const uint4*>(piece(C::one_block(l, wg), c)), b = *reinterpret_cast<const uint4*>(piece(C::one_block(l, wg), 4 + c));
-            lo[4 * c] = a.x; lo[4 * c + 1] = a.y; lo[4 * c + 2] = a.z; lo[4 * c + 3] = a.w;
-            hi[4 * c] = b.x; hi[4 * c + 1] = b.y; hi[4 * c + 2] = b.z; hi[4 * c + 3] = b.w;
-        }
-        tmem_st16(lane_base + kColA + 32 * wg, lo);
-        tmem_st16(lane_base + kColA + 32 * wg + 16, hi);
-        tmem_wait_st();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(sm.bar(AT_KB + wg));
-        return true;
-    };
+    // this thread's four units, bytes 8 (w & 1) of piece w / 2 of its row of the CTA's block
+    auto xp = [&](int l) { return reinterpret_cast<uint2*>(piece(C::one_block(l, (int)rank), w >> 1) + 8 * (w & 1)); };
 
-    // ---- encoder output + bias -> layer-0 input (the first quadrant's lanes hold it)
+    // ---- encoder output + bias -> layer-0 input
     CFX_SWAIT(ACC_FULL, 0);
     tc_fence_after_sync();
     if (!kFull) free_records();
     if (!C::kOneBeside) CFX_SWAIT(REC_FREE, 0);
-    if (quadrant == 0) {
-        uint32_t acc[16];
-        tmem_ld16(lane_base + kColAcc + kWarpUnits * wg, acc);
+    uint2 x;   // this thread's units of the layer input, packed: operand and the cell's blend input
+    {
+        uint32_t acc[4];
+        tmem_ld4(lane_base + kColAcc + 4 * wg, acc);
         tmem_wait_ld();
-        const float* b = bias + kWarpUnits * wg;
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-            uint32_t h[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int i = 8 * c + 2 * q;
-                h[q] = Op::pack(__uint_as_float(acc[i]) + b[i], __uint_as_float(acc[i + 1]) + b[i + 1]);
-            }
-            *reinterpret_cast<uint4*>(piece(C::one_block(0, (int)rank), 2 * wg + c)) = make_uint4(h[0], h[1], h[2], h[3]);
-        }
+        const float* b = bias + unit;
+        x = make_uint2(Op::pack(__uint_as_float(acc[0]) + b[0], __uint_as_float(acc[1]) + b[1]),
+                       Op::pack(__uint_as_float(acc[2]) + b[2], __uint_as_float(acc[3]) + b[3]));
+        *xp(0) = x;
     }
     if (!send(0)) return;
 
-    // ---- layers: this thread's four units, bytes 8 (quadrant & 1) of piece 2 wg + quadrant / 2 of its row
-    auto xp = [&](int l) { return reinterpret_cast<uint2*>(piece(C::one_block(l, (int)rank), 2 * wg + (quadrant >> 1)) + 8 * (quadrant & 1)); };
-    const int unit = kWarpUnits * wg + 4 * quadrant;
+    // ---- layers
     for (int l = 0; l < P.L; l++) {
-        if (!to_tmem(l)) return;
-        CFX_SWAIT(A_KB + 4 * l + (int)rank, 0);
-        const uint2 x = *xp(l);
-        const int box = l * C::kBoxes + (wg >> 1), slot = box % kSSlots;
+        const int box = l * C::kBoxes + (w >> 3), slot = box % kSSlots;
         CFX_SWAIT(S_FULL + slot, (box / kSSlots) & 1);
-        float4* sp = reinterpret_cast<float4*>(piece(C::kOffS + slot * kSBox, 4 * (wg & 1) + quadrant));
+        float4* sp = reinterpret_cast<float4*>(piece(C::kOffS + slot * kSBox, w & 7));
         float4 st = *sp;
         if (zero_state) st = make_float4(0.f, 0.f, 0.f, 0.f);
         // optional BPTT record of the post-zero input state (craftax_full.cu:9370-9375)
@@ -753,9 +734,9 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         CFX_SWAIT(G_FULL, l & 1);
         tc_fence_after_sync();
         uint32_t zh[4], zg[4], zp[4];
-        tmem_ld4(lane_base + col_gate(0) + gate_row(0, unit), zh);
-        tmem_ld4(lane_base + col_gate(0) + gate_row(1, unit), zg);
-        tmem_ld4(lane_base + col_gate(0) + gate_row(2, unit), zp);
+        tmem_ld4(lane_base + col_gate(0) + 4 * wg, zh);
+        tmem_ld4(lane_base + col_gate(0) + kWarpUnits + 4 * wg, zg);
+        tmem_ld4(lane_base + col_gate(0) + kColP + 4 * wg, zp);
         tmem_wait_ld();
         const float2 x01 = Op::unpack(x.x), x23 = Op::unpack(x.y);
         float h0, h1, h2, h3;
@@ -764,17 +745,17 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         mingru_cell_pair(__uint_as_float(zh[2]), __uint_as_float(zh[3]), __uint_as_float(zg[2]), __uint_as_float(zg[3]),
                          __uint_as_float(zp[2]), __uint_as_float(zp[3]), st.z, st.w, x23.x, x23.y, st.z, st.w, h2, h3);
         *sp = st;
-        *xp(l + 1) = make_uint2(Op::pack(h0, h1), Op::pack(h2, h3));
+        x = make_uint2(Op::pack(h0, h1), Op::pack(h2, h3));
+        *xp(l + 1) = x;
         if (!send(l + 1)) return;
         if (lane == 0) mbar_arrive(sm.bar(ST_READY + slot));   // (send fenced the box as well)
     }
 
     // ---- heads + sampler: all warps, each with the rows in its quadrant
     if (rank == 0) {
-        if (!to_tmem(P.L)) return;
         CFX_SWAIT(H_FULL, 0);
         tc_fence_after_sync();
-        if (valid) sample_one<GAME>(P, reinterpret_cast<float*>(sm.base + C::kOffW), lane_base + kColHead, bias + C::kUnits, w, lane, env, u, meet);
+        if (valid) sample_one<GAME>(P, reinterpret_cast<float*>(sm.base + C::kOffW), lane_base + kColHead + 4 * wg, bias + C::kUnits, w, lane, env, u, meet);
     }
     meet.met = Meetings::kAll;
 }
@@ -807,7 +788,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
             else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = ONE ? 8 : 2 * quads;
             else if (i == MMA_DONE) arrivals = S;
             else if (i >= QUAD && i < QUAD + 8) arrivals = ONE ? kWorkerWarps : 4;
-            else if (i >= AT_KB && i < A_KB) arrivals = 4;
             else if (i >= A_KB) {
                 const int kb = (i - A_KB) % 4;
                 if (kb / C::kNS == (int)rank) arrivals = quads;

@@ -55,4 +55,19 @@ inline bool make_tmap_blocks(CUtensorMap* map, void* base, uint64_t blocks, uint
     return r == CUDA_SUCCESS;
 }
 
+// Groups of parts of rows of 64 16-bit elements (128 bytes), all contiguous: [groups][parts][rows][64]; box =
+// [box_groups][box_parts][rows][64].
+inline bool make_tmap_parts(CUtensorMap* map, void* base, uint64_t groups, uint64_t parts, uint64_t rows, uint32_t box_groups,
+                            uint32_t box_parts) {
+    PFN_encodeTiled enc = get_encode_tiled();
+    if (!enc) return false;
+    cuuint64_t dims[4] = {64, rows, parts, groups};
+    cuuint64_t strides[3] = {128, rows * 128, parts * rows * 128};
+    cuuint32_t box[4] = {64, (cuuint32_t)rows, box_parts, box_groups};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS;
+}
+
 }  // namespace cfx

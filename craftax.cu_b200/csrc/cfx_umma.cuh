@@ -228,6 +228,14 @@ __device__ __forceinline__ void tensor_g2s_3d_pair(uint32_t dst_smem, const CUte
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(cluster_bar)
         : "memory");
 }
+// 4-D, counted on a barrier of this CTA
+__device__ __forceinline__ void tensor_g2s_4d(uint32_t dst_smem, const CUtensorMap* map, int x, int y, int z, int w, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst_smem),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+        : "memory");
+}
 // 2-D tiled tensor copy shared -> global (bulk async-group completion).
 __device__ __forceinline__ void tensor_s2g_2d(const CUtensorMap* map, uint32_t src_smem, int x,
                                               int y) {
@@ -396,6 +404,17 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uin
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Weight-stationary form for few rows (M = 32): D's columns are spread over the quadrants of tensor memory, N / 4
+// each, so that quadrant q holds columns [q N / 4, (q + 1) N / 4) of all 32 rows.  12 + N / 4 cycles (N = 64: 28.6, 128: 44.6),
+// where 128 rows take N / 2, and at least 49 with A in shared memory.
+__device__ __forceinline__ void mma_f16_ws_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.ws.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
