@@ -67,6 +67,13 @@ template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kEncTile = kUnits * 128;               // its rows of one encoder weight block
     static constexpr int kEncPerItem = kNS == 1 ? 3 : 1;        // encoder blocks of one ring slot
     static constexpr int kEncItems = (Gm<GAME>::kEncBlocks + kEncPerItem - 1) / kEncPerItem;
+    // ONE: ring slots whose operand chunks the MMA warp waits for together: the full game's sixteen chunks, a warp each, are there
+    // at the same time (1,024 envs 10.8 us, 11.0 with a wait a slot, 11.6 with one a chunk); the classic game's 22 are not
+    // (13.3 with two waits for all of them, 13.1 with one a slot, 13.0 with one a chunk)
+    static constexpr int kGroupItems = GAME == CFX_GAME_FULL ? kEncItems : 1;
+    static __device__ __forceinline__ int group_chunks(int group) {
+        return GAME == CFX_GAME_FULL ? Gm<GAME>::kEncChunks : max(1, min(kEncPerItem, Gm<GAME>::kEncBlocks - group * kEncPerItem));
+    }
     static constexpr int kHeadHalf = Gm<GAME>::kHeadPair / 2 * 128;   // half of the head rows, one K block
     static constexpr int kHeadItems = kKB / 2;                  // two K blocks of the heads a slot
     static constexpr int kRowBytes = Gm<GAME>::kRecBytes, kQuadBytes = 32 * kRowBytes;
@@ -224,35 +231,60 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
     // ---- encoder
     CFX_SPROBE(cfx_p_b, W_FULL, 0);
     CFX_SPROBE(cfx_p_a, AEXP_FULL, 0);
+    if constexpr (ONE) {
+        // the warps convert a chunk each at the same time: one wait for many of them, and the steps of a ring slot in one run
 #pragma unroll
-    for (int kc = 0; kc < kChunks; kc++) {
-        // block of 64 K columns, first of its 16-byte K pieces, K steps (see expand_full), last chunk of its block
-        const bool full = GAME == CFX_GAME_FULL;
-        const int blk = full && kc >= 12 ? (kc < 14 ? 12 : 13) : kc, first = full && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0;
-        const int ks = full ? full_ksteps(kc) : (kc == kChunks - 1 ? 1 : 4);
-        const bool starts = !(full && (kc == 13 || kc == 15)), ends = !(full && (kc == 12 || kc == 14));
-        const int item = blk / C::kEncPerItem, slot = item % kWSlots, as = ONE ? kc : kc % kASlots;
-        if (starts && blk % C::kEncPerItem == 0) {
+        for (int item = 0; item < C::kEncItems; item++) {
+            const int slot = item % kWSlots, blk0 = item * C::kEncPerItem;
+            constexpr int kBlocks = Gm<GAME>::kEncBlocks;
             CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, (item / kWSlots) & 1);
             CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
-        }
-        CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + as, ONE ? 0 : (kc / kASlots) & 1);
-        if (kc + 1 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + (ONE ? kc + 1 : (kc + 1) % kASlots), ONE ? 0 : ((kc + 1) / kASlots) & 1);
-        tc_fence_after_sync();
-        __syncwarp();
-        const uint64_t bd = wdesc + (uint64_t)(((slot * kWSlot + blk % C::kEncPerItem * C::kEncTile) >> 4) + first);
-        const uint32_t a = tmem + kColAexp + as * 32;
-        if (elect_one()) {
+            if (item % C::kGroupItems == 0) CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + item / C::kGroupItems, 0);
+            if ((item + 1) % C::kGroupItems == 0 && item + 1 < C::kEncItems) CFX_SPROBE(cfx_p_a, AEXP_FULL + (item + 1) / C::kGroupItems, 0);
+            tc_fence_after_sync();
+            __syncwarp();
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < ks; k++) {
-                if constexpr (ONE)
-                    mma_f16_ws_ss(tmem + kColAcc, xdesc + (uint64_t)(((blk * kQuadBlock) >> 4) + first + 2 * k), bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
-                else
-                    mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+                for (int b = 0; b < C::kEncPerItem; b++) {
+                    const int blk = blk0 + b, last = kBlocks - 1;
+                    if (blk > last) break;
+                    const int ks = blk < last ? 4 : (GAME == CFX_GAME_FULL ? 2 : 1);
+#pragma unroll
+                    for (int k = 0; k < ks; k++)
+                        mma_f16_ws_ss(tmem + kColAcc, xdesc + (uint64_t)((blk * kQuadBlock) >> 4) + 2 * k,
+                                      wdesc + (uint64_t)((slot * kWSlot + b * C::kEncTile) >> 4) + 2 * k, idesc_enc, (blk | k) != 0 ? 1u : 0u);
+                }
+                if (item == C::kEncItems - 1) mma_commit(sm.bar(ACC_FULL));
+                mma_commit(sm.bar(W_EMPTY + slot));
             }
-            if (!ONE && kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
-            if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
-            if (ends && ((blk + 1) % C::kEncPerItem == 0 || kc == kChunks - 1)) mma_commit(sm.bar(W_EMPTY + slot));
+        }
+    } else {
+#pragma unroll
+        for (int kc = 0; kc < kChunks; kc++) {
+            // block of 64 K columns, first of its 16-byte K pieces, K steps (see expand_full), last chunk of its block
+            const bool full = GAME == CFX_GAME_FULL;
+            const int blk = full && kc >= 12 ? (kc < 14 ? 12 : 13) : kc, first = full && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0;
+            const int ks = full ? full_ksteps(kc) : (kc == kChunks - 1 ? 1 : 4);
+            const bool starts = !(full && (kc == 13 || kc == 15)), ends = !(full && (kc == 12 || kc == 14));
+            const int item = blk / C::kEncPerItem, slot = item % kWSlots, as = kc % kASlots;
+            if (starts && blk % C::kEncPerItem == 0) {
+                CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, (item / kWSlots) & 1);
+                CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
+            }
+            CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + as, (kc / kASlots) & 1);
+            if (kc + 1 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + (kc + 1) % kASlots, ((kc + 1) / kASlots) & 1);
+            tc_fence_after_sync();
+            __syncwarp();
+            const uint64_t bd = wdesc + (uint64_t)(((slot * kWSlot + blk % C::kEncPerItem * C::kEncTile) >> 4) + first);
+            const uint32_t a = tmem + kColAexp + as * 32;
+            if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < ks; k++)
+                    mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+                if (kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
+                if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
+                if (ends && ((blk + 1) % C::kEncPerItem == 0 || kc == kChunks - 1)) mma_commit(sm.bar(W_EMPTY + slot));
+            }
         }
     }
     // ---- layers and heads (a loop over the layers: straight-line code for all of them would be fetched cold)
@@ -264,16 +296,19 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 #pragma unroll 1
     for (int l = 0; l < P.L; l++) {
         const int slot0 = first_slot(l);
-        CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
+        if (!ONE) CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
         // this CTA's own K blocks first: the gate columns are free when its cells have read them
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) CFX_SWAIT_SPIN(A_KB + 4 * l + (int)rank * C::kNS + j, 0);
+        if (ONE)   // the blocks of the other CTAs come at about the same time
+#pragma unroll
+            for (int kb = 0; kb < C::kKB; kb++) CFX_SWAIT_SPIN(A_KB + 4 * l + kb, 0);
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) {
 #pragma unroll
             for (int kb = 0; kb < C::kKB; kb++) {
                 const int slot = (slot0 + j * C::kKB + kb) % kWSlots, slot1 = (slot + 1) % kWSlots;
-                if (j == 0) {
+                if (!ONE && j == 0) {
                     CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * l + kb, 0);
                     if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * l + kb + 1, 0);
                 }
@@ -666,7 +701,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
                 *reinterpret_cast<uint4*>(piece(C::kOffX + blk * kQuadBlock, first + c)) = make_uint4(regs[4 * c], regs[4 * c + 1], regs[4 * c + 2], regs[4 * c + 3]);
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + kc));
+        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + blk / C::kEncPerItem / C::kGroupItems));
     }
     auto free_records = [&]() {
         __syncwarp();
@@ -783,7 +818,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         if (i < NUM_BARS) {
             uint32_t arrivals = 1, bytes = 0;
             if (i == REC_FREE) arrivals = ONE ? S * kWorkerWarps : S * 4 * quads;
-            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? 1 : quads;
+            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::group_chunks(i - AEXP_FULL) : quads;
             else if (i == ACC_FULL) arrivals = 2;                          // the MMAs, and the biases are in place
             else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = ONE ? 8 : 2 * quads;
             else if (i == MMA_DONE) arrivals = S;
