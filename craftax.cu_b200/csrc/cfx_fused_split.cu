@@ -271,8 +271,11 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                 CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, (item / kWSlots) & 1);
                 CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
             }
-            CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + as, (kc / kASlots) & 1);
-            if (kc + 1 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + (kc + 1) % kASlots, ((kc + 1) / kASlots) & 1);
+            // (four chunks, one of each warpgroup, are there at the same time)
+            if (kc % 4 == 0) {
+                CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + kc / 4, 0);
+                if (kc + 4 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + kc / 4 + 1, 0);
+            }
             tc_fence_after_sync();
             __syncwarp();
             const uint64_t bd = wdesc + (uint64_t)(((slot * kWSlot + blk % C::kEncPerItem * C::kEncTile) >> 4) + first);
@@ -447,7 +450,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + kc % kASlots));
+        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + kc / 4));
     };
     for (int kc = wg; kc < kChunks; kc += 4) {
         const int as = kc % kASlots;
@@ -818,7 +821,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         if (i < NUM_BARS) {
             uint32_t arrivals = 1, bytes = 0;
             if (i == REC_FREE) arrivals = ONE ? S * kWorkerWarps : S * 4 * quads;
-            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::group_chunks(i - AEXP_FULL) : quads;
+            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::group_chunks(i - AEXP_FULL) : max(1, min(4, Gm<GAME>::kEncChunks - 4 * (i - AEXP_FULL))) * quads;
             else if (i == ACC_FULL) arrivals = 2;                          // the MMAs, and the biases are in place
             else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = ONE ? 8 : 2 * quads;
             else if (i == MMA_DONE) arrivals = S;
