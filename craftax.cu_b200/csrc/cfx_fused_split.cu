@@ -30,8 +30,8 @@
 // The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
 // records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
-// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 11.6, 1,024 25.7 -> 12.7,
-// 2,016 26 -> 15.7, 4,000 26 -> 19.5, 8,192 26.9 -> 21.4; classic h256x3, 1,024 envs 35.7 -> 16.1.  Bound by the chain of
+// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 9.9, 1,024 25.7 -> 10.8,
+// 2,048 26 -> 15.3, 4,000 26 -> 18.2, 8,192 26.9 -> 20.8; classic h256x3, 1,024 envs 35.7 -> 16.1 (before the products of 32 rows).  Bound by the chain of
 // dependent steps and the 1.3 us between one kernel's end and the next one's start.
 #include "cfx_fused_split.h"
 
