@@ -177,12 +177,13 @@ __global__ void k_pack_image(const float* __restrict__ params, uint8_t* __restri
 
 struct Smem {
     uint8_t* base;
-    int off_s, off_bias, off_bars, off_misc;
+    int off_s, off_bias, off_misc;
+    uint32_t bars;   // shared address of the barriers
     template <bool PAIR, int GAME, int HID> __device__ __forceinline__ void layout() {
         using C = Cfg<PAIR, GAME, HID>;
-        off_s = C::kOffS; off_bias = C::kOffBias; off_bars = C::kOffBars; off_misc = C::kOffMisc;
+        off_s = C::kOffS; off_bias = C::kOffBias; bars = smem_u32(base + C::kOffBars); off_misc = C::kOffMisc;
     }
-    __device__ __forceinline__ uint32_t bar(int i) const { return smem_u32(base + off_bars + i * 8); }
+    __device__ __forceinline__ uint32_t bar(int i) const { return bars + 8u * (uint32_t)i; }
     __device__ __forceinline__ uint8_t* b_ring() const { return base; }
     __device__ __forceinline__ uint8_t* s_slot(int s) const { return base + off_s + s * kSSlot; }
     __device__ __forceinline__ float* bias() const { return reinterpret_cast<float*>(base + off_bias); }
@@ -201,22 +202,19 @@ struct Smem {
 #endif
 
 // every role runs in its own function: a failed (timed-out) wait returns to the common exit
-// Copy threads and worker warps poll with try_wait (suspends while not ready).
+// Worker warps poll with try_wait (suspends while not ready).
 // Measured alternatives, all slower on B200: one polling lane per worker warp plus a shuffle
 // (+25 % kernel time), a test_wait probe in front of the loop (+6 %).
-#define CFX_WAIT(barid, parity, code) \
-    if (!mbar_wait(sm.bar(barid), (parity), sm.abort_flag(), (code))) return
-#define CFX_WAITW(barid, parity, code) CFX_WAIT(barid, parity, code)
-// the copy-issuing warps and threads (weights, loads, stores): no back-off between probes
+#define CFX_WAITW(barid, parity, code) \
+    if (!mbar_wait_warp(sm.bar(barid), (parity), sm.abort_flag(), (code))) return
+// the copy-issuing threads (one lane: loads, stores) and warp (weights): no back-off between probes
 #define CFX_WAIT_FAST(barid, parity, code) \
     if (!mbar_wait<false>(sm.bar(barid), (parity), sm.abort_flag(), (code))) return
-// The MMA warp polls with test_wait: it never suspends.  The first probe is
-// inline: almost every wait of this warp finds its barrier complete (5 failed probes in the
-// 32 weight waits of a tile), and the bounded loop costs ~150 cycles more than one probe.
-#define CFX_WAIT_LEADER(barid, parity, code)                                          \
-    if (!mbar_test_wait(sm.bar(barid), (parity)) &&                                   \
-        !mbar_wait_spin(sm.bar(barid), (parity), sm.abort_flag(), (code)))            \
-    return
+#define CFX_WAITW_FAST(barid, parity, code) \
+    if (!mbar_wait_warp<false>(sm.bar(barid), (parity), sm.abort_flag(), (code))) return
+// The MMA warp polls with test_wait: it never suspends.
+#define CFX_WAIT_LEADER(barid, parity, code) \
+    if (!mbar_wait_warp<false, true>(sm.bar(barid), (parity), sm.abort_flag(), (code))) return
 
 // Who converts which operand chunk (a weight block's 64 K columns).  Group 0 samples the previous tile's actions while the
 // other three convert: chunk kc is group 1 + kc % 3's.
@@ -254,8 +252,8 @@ __device__ __forceinline__ void role_weight_loads(const Smem& sm, const Params& 
             region = 2; row = 0; blk = (int)rank; bytes = head_bytes<GAME, HID>(PAIR);
         }
         uint32_t ready;
-        CFX_PROBE_READ(cfx_p_w, ready);
-        if (ready == 0) CFX_WAIT_FAST(B_EMPTY + slot, par, W_B_EMPTY);
+        CFX_PROBE_READ_ALL(cfx_p_w, ready);
+        if (ready == 0) CFX_WAITW_FAST(B_EMPTY + slot, par, W_B_EMPTY);
         const int slot1 = slot + 1 == C::kNB ? 0 : slot + 1;
         const uint32_t par1 = slot1 == 0 ? par ^ 1u : par;
         CFX_PROBE(cfx_p_w, sm.bar(B_EMPTY + slot1), par1);
@@ -448,8 +446,8 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 #define CFX_WAIT_PROBED(name, barid, parity, code)                                                  \
     {                                                                                               \
         uint32_t ready_;                                                                            \
-        CFX_PROBE_READ(name, ready_);                                                               \
-        if (ready_ == 0 && !mbar_wait_spin(sm.bar(barid), (parity), sm.abort_flag(), (code))) return; \
+        CFX_PROBE_READ_ALL(name, ready_);                                                               \
+        if (ready_ == 0) CFX_WAIT_LEADER(barid, parity, code);             \
     }
     CFX_PROBE(cfx_p_ge, sm.bar(G_EMPTY), 1);
     CFX_MARK_INIT(0);
@@ -626,7 +624,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             for (int kc = wg - 1; kc < kEncBlocks; kc += kExpGroups, acnt += kExpGroups) {
                 const int as = acnt % kAexpSlots;
                 uint32_t ae_ok;
-                CFX_PROBE_READ(cfx_p_ae, ae_ok);
+                CFX_PROBE_READ_ALL(cfx_p_ae, ae_ok);
                 if (ae_ok == 0) CFX_WAITW(AEXP_EMPTY + as, ((acnt / kAexpSlots) & 1) ^ 1, W_AEXP_EMPTY);
                 CFX_MARK(2);
                 tc_fence_after_sync();
@@ -718,7 +716,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 }
                 {
                     uint32_t g_ok;
-                    CFX_PROBE_READ(cfx_p_g, g_ok);
+                    CFX_PROBE_READ_ALL(cfx_p_g, g_ok);
                     if (g_ok == 0) CFX_WAITW(G_FULL + half, gcnt & 1, W_G_FULL);
                 }
                 CFX_MARK(6);
@@ -741,7 +739,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 CFX_MARK(7);
                 {
                     uint32_t s_ok;
-                    CFX_PROBE_READ(cfx_p_s, s_ok);
+                    CFX_PROBE_READ_ALL(cfx_p_s, s_ok);
                     if (s_ok == 0) CFX_WAITW(S_FULL + slot, sp_par, W_S_FULL);
                 }
                 CFX_MARK(8);
@@ -787,7 +785,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         // that their next-tile operand writes cannot overtake the last MMA)
         {
             uint32_t h_ok;
-            CFX_PROBE_READ(cfx_p_g, h_ok);
+            CFX_PROBE_READ_ALL(cfx_p_g, h_ok);
             if (h_ok == 0) CFX_WAITW(H_FULL, tcnt & 1, W_H_FULL);
         }
         CFX_MARK(10);
@@ -936,23 +934,31 @@ k_policy_fused(const __grid_constant__ Params P) {
     if (tid == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
 }
 
-// Self-test of the bounded wait: the first warp of a block waits on a barrier on which nothing ever arrives,
-// with a limit of a few milliseconds, gives up, and reports through the same status word
+// Self-test of the bounded wait: the first warp of a block waits with a limit of a few milliseconds, every other lane on a
+// phase that is complete, the rest on a barrier on which nothing ever arrives.  All of its lanes give up together (kSelftestParted
+// if some go on), and it reports through the same status word
 // protocol as the forward kernels.  The second warp is at the first of the two meetings it has with the first one by then,
 // and is let go; it alone has said that it is done with the step counter.  The kernel ends normally; the context stays
 // usable.
-constexpr uint32_t kSelftestCode = 0x7E;
+constexpr uint32_t kSelftestCode = 0x7E, kSelftestParted = 0x7F;
 __global__ void k_selftest_wait_timeout(uint32_t* status, uint32_t* done, unsigned long long limit_ns) {
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t abort_flag;
     if (threadIdx.x == 0) {
         abort_flag = 0;
-        mbar_init(smem_u32(&bar), 1);
+        mbar_init(smem_u32(&bar[0]), 1);
+        mbar_init(smem_u32(&bar[1]), 1);
         fence_mbar_init();
+        mbar_arrive(smem_u32(&bar[0]));
     }
     __syncthreads();
     Meetings meet;
-    if (threadIdx.x >= 32 || mbar_wait(smem_u32(&bar), 0, &abort_flag, kSelftestCode, limit_ns)) {
+    bool passed = true;
+    if (threadIdx.x < 32) {
+        passed = mbar_wait_warp(smem_u32(&bar[threadIdx.x & 1]), 0, &abort_flag, kSelftestCode, limit_ns);
+        if (__any_sync(0xffffffffu, passed)) abort_flag = kSelftestParted;
+    }
+    if (passed) {
         if ((threadIdx.x & 31) == 0) done_with_step(nullptr, done, 2);
         meet.sync(1, 64);
         meet.sync(1, 64);
@@ -1009,6 +1015,10 @@ int fused_selftest_wait_timeout(unsigned limit_ms, unsigned* status_out) {
     if (e != cudaSuccess) return cuda_fail(e, "selftest", __FILE__, __LINE__);
     if (before != 1 || after != 0) {
         set_error("self-test: the count of a launch that gave up is %u, and %u after the check (1 and 0 expected)", before, after);
+        return CFX_ERR_CUDA;
+    }
+    if ((*status_out & 0xFF) == fused::kSelftestParted) {
+        set_error("self-test: some lanes of a warp went on from a wait that the others gave up");
         return CFX_ERR_CUDA;
     }
     return CFX_OK;

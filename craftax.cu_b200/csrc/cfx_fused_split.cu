@@ -116,16 +116,18 @@ constexpr uint32_t kSite = 0x40;   // wait-site codes: kSite + barrier
 struct Smem {
     uint8_t* base;
     int off_bars;
-    __device__ __forceinline__ uint32_t bar(int i) const { return smem_u32(base + off_bars + i * 8); }
+    uint32_t bars;   // shared address of the barriers
+    __device__ __forceinline__ uint32_t bar(int i) const { return bars + 8u * (uint32_t)i; }
     __device__ __forceinline__ uint32_t* tmem_base() const { return reinterpret_cast<uint32_t*>(base + off_bars + NUM_BARS * 8); }
     __device__ __forceinline__ volatile uint32_t* abort_flag() const { return tmem_base() + 1; }
 };
-#define CFX_SWAIT(barid, parity) \
+// one lane waits (CFX_SWAIT1), or a whole warp (the MMA warp by polling alone)
+#define CFX_SWAIT1(barid, parity) \
     if (!mbar_wait<false>(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return
-#define CFX_SWAIT_SPIN(barid, parity)                                               \
-    if (!mbar_test_wait(sm.bar(barid), (parity)) &&                                 \
-        !mbar_wait_spin(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) \
-    return
+#define CFX_SWAIT(barid, parity) \
+    if (!mbar_wait_warp<false>(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return
+#define CFX_SWAIT_SPIN(barid, parity) \
+    if (!mbar_wait_warp<false, true>(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return
 
 // shared memory of this CTA -> shared memory of another CTA of the cluster, counted on a barrier there
 __device__ __forceinline__ void bulk_s2s(uint32_t dst_cluster, uint32_t src, uint32_t bytes, uint32_t bar_cluster) {
@@ -168,7 +170,7 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
     const uint32_t ring = smem_u32(sm.base + C::kOffW);
     for (int i = 0; i < items; i++) {
         const int slot = i % kWSlots;
-        if (i >= kWSlots) CFX_SWAIT(W_EMPTY + slot, ((i / kWSlots) - 1) & 1);
+        if (i >= kWSlots) CFX_SWAIT1(W_EMPTY + slot, ((i / kWSlots) - 1) & 1);
         const uint32_t dst = ring + slot * kWSlot, full = sm.bar(W_FULL + slot);
         if (i < C::kEncItems) {
             const int blocks = min(C::kEncPerItem, Gm<GAME>::kEncBlocks - i * C::kEncPerItem), u0 = C::kUnits * (int)rank;
@@ -210,11 +212,11 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
 // computed takes ~150 cycles to issue, and 54 of them were two thirds of the encoder.  The barriers of the next step are
 // probed before the current step's MMAs (CFX_PROBE), so that a probe's round trip runs under their issue.
 #define CFX_SPROBE(name, barid, parity) CFX_PROBE(name, sm.bar(barid), (uint32_t)(parity))
-#define CFX_SWAIT_PROBED(name, barid, parity)                                                               \
-    {                                                                                                       \
-        uint32_t ready_;                                                                                    \
-        CFX_PROBE_READ(name, ready_);                                                                       \
-        if (ready_ == 0 && !mbar_wait_spin(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return; \
+#define CFX_SWAIT_PROBED(name, barid, parity)                                      \
+    {                                                                              \
+        uint32_t ready_;                                                           \
+        CFX_PROBE_READ_ALL(name, ready_);                                              \
+        if (ready_ == 0) CFX_SWAIT_SPIN(barid, parity);  \
     }
 template <typename T16, int GAME, int HID, int S, bool ONE>
 __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32_t tmem, uint32_t rank) {
@@ -387,11 +389,11 @@ __device__ __forceinline__ void role_state(const Smem& sm, const Params& P, int 
         for (int q = 0; q < quads; q++)
             tensor_g2s_2d(slot_at(b) + q * kQuadBox, &P.state_map[b / C::kBoxes], unit(b), row0 + 32 * q, sm.bar(S_FULL + b % kSSlots));
     };
-    if (!(ONE && C::kOneBeside)) CFX_SWAIT(REC_FREE, 0);
-    if (ONE) CFX_SWAIT(ACC_FULL, 0);   // the operand chunks are used up
+    if (!(ONE && C::kOneBeside)) CFX_SWAIT1(REC_FREE, 0);
+    if (ONE) CFX_SWAIT1(ACC_FULL, 0);   // the operand chunks are used up
     for (int b = 0; b < kSSlots && b < boxes; b++) load(b);
     for (int b = 0; b < boxes; b++) {
-        CFX_SWAIT(ST_READY + b % kSSlots, (b / kSSlots) & 1);
+        CFX_SWAIT1(ST_READY + b % kSSlots, (b / kSSlots) & 1);
         for (int q = 0; q < quads; q++) tensor_s2g_2d(&P.state_map[b / C::kBoxes], slot_at(b) + q * kQuadBox, unit(b), row0 + 32 * q);
         bulk_commit_group();
         if (b + kSSlots < boxes) {
@@ -549,25 +551,28 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             tmem_wait_ld();
             uint8_t* sp = sm.base + C::kOffS + slot * kSBox + (row >> 3) * 1024 + (row & 7) * 128;
             auto piece = [&](int q) { return reinterpret_cast<float4*>(sp + (((4 * (wg & 1) + q) ^ (row & 7)) << 4)); };
-            float st[kWarpUnits];
+            // (half of the units at a time: with the state of all of them in registers, 22 words went through local memory, 43 with bf16)
 #pragma unroll
-            for (int q = 0; q < kWarpUnits / 4; q++) {
-                float4 v = *piece(q);
-                if (zero_state) v = make_float4(0.f, 0.f, 0.f, 0.f);
-                st[4 * q] = v.x; st[4 * q + 1] = v.y; st[4 * q + 2] = v.z; st[4 * q + 3] = v.w;
-            }
+            for (int h = 0; h < kWarpUnits / 4; h += 2) {
+                float4 st[2];
 #pragma unroll
-            for (int q = 0; q < kWarpUnits / 4; q++) {
-#pragma unroll
-                for (int i = 4 * q; i < 4 * q + 4; i += 2) {
-                    const float2 xv = Op::unpack(x[j][i / 2]);
-                    float o0, o1, h0, h1;
-                    mingru_cell_pair(__uint_as_float(zh[i]), __uint_as_float(zh[i + 1]), __uint_as_float(zg[i]), __uint_as_float(zg[i + 1]),
-                                     __uint_as_float(zp[i]), __uint_as_float(zp[i + 1]), st[i], st[i + 1], xv.x, xv.y, o0, o1, h0, h1);
-                    st[i] = o0; st[i + 1] = o1;
-                    x[j][i / 2] = Op::pack(h0, h1);
+                for (int q = 0; q < 2; q++) {
+                    st[q] = *piece(h + q);
+                    if (zero_state) st[q] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
-                *piece(q) = make_float4(st[4 * q], st[4 * q + 1], st[4 * q + 2], st[4 * q + 3]);
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const int i = 4 * (h + q);
+                    const float2 x01 = Op::unpack(x[j][i / 2]), x23 = Op::unpack(x[j][i / 2 + 1]);
+                    float h0, h1, h2, h3;
+                    mingru_cell_pair(__uint_as_float(zh[i]), __uint_as_float(zh[i + 1]), __uint_as_float(zg[i]), __uint_as_float(zg[i + 1]),
+                                     __uint_as_float(zp[i]), __uint_as_float(zp[i + 1]), st[q].x, st[q].y, x01.x, x01.y, st[q].x, st[q].y, h0, h1);
+                    mingru_cell_pair(__uint_as_float(zh[i + 2]), __uint_as_float(zh[i + 3]), __uint_as_float(zg[i + 2]), __uint_as_float(zg[i + 3]),
+                                     __uint_as_float(zp[i + 2]), __uint_as_float(zp[i + 3]), st[q].z, st[q].w, x23.x, x23.y, st[q].z, st[q].w, h2, h3);
+                    x[j][i / 2] = Op::pack(h0, h1);
+                    x[j][i / 2 + 1] = Op::pack(h2, h3);
+                    *piece(h + q) = st[q];
+                }
             }
             if (j == 0) CFX_SWAIT(MMA_DONE, l & 1);
             if (!send(l + 1, j, x[j])) return;
@@ -809,6 +814,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     Smem sm;
     sm.base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     sm.off_bars = C::kOffBars;
+    sm.bars = smem_u32(sm.base + C::kOffBars);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_ctarank();
     const int row0 = P.tile_begin * kTile + (int)blockIdx.x / S * P.tile_rows, quads = P.tile_rows / 32;

@@ -116,6 +116,10 @@ __device__ __forceinline__ void st_global_v8(float* p, const float (&v)[8]) {
                      "r"(bar), "r"(parity) : "memory")
 #define CFX_PROBE_CLEAR(name) asm volatile("setp.ne.u32 " #name ", 0, 0;")
 #define CFX_PROBE_READ(name, out) asm volatile("selp.u32 %0, 1, 0, " #name ";" : "=r"(out) : : "memory")
+// the same for a whole warp: 1 if every lane's probe found the phase complete (see mbar_wait_warp)
+#define CFX_PROBE_READ_ALL(name, out)                                                                                 \
+    asm volatile("{\n\t.reg .pred all;\n\tvote.sync.all.pred all, " #name ", 0xffffffff;\n\tselp.u32 %0, 1, 0, all;\n\t}" \
+                 : "=r"(out) : : "memory")
 
 // Bounded wait: spins on try_wait; after kWaitLimitNs without completion (or as soon as
 // another thread of the CTA has given up) it records `code` in *abort_flag (shared
@@ -151,20 +155,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
     }
 }
 
-// Same contract, but polls with test_wait only (never suspends): for the MMA-issuing thread,
-// whose wake-up latency is on the critical path of every tile.
-__device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity,
-                                               volatile uint32_t* abort_flag, uint32_t code) {
-    uint64_t t0 = 0;
-    uint32_t spins = 0;
+// The same for a whole warp, all 32 lanes together: either every lane has seen the phase complete, or all of them give up.
+// mbar_wait decides lane by lane, and a warp in which some lanes give up while others go on must not come to an instruction
+// that takes all of it (elect.sync, the tcgen05 loads and stores, an aligned barrier): it would wait there without a limit.
+// kSpin: polls with test_wait, which never suspends, for the MMA-issuing warp, whose wake-up latency is on the critical path
+// of every tile.
+template <bool kBackoff = true, bool kSpin = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t code,
+                                               uint64_t limit_ns = kWaitLimitNs) {
+    constexpr uint32_t kEvery = kSpin ? 16384 : 4096;   // failed polls between looks at the timer and the abort flag
+    auto now = [] { return (uint32_t)(global_timer_ns() >> 16); };   // (one register: 65.5 us a tick)
+    uint32_t t0 = 0, spins = 0;
     while (true) {
-        if (mbar_test_wait(bar, parity)) return true;
-        if ((++spins & 16383u) == 0) {
-            if (*abort_flag != 0) return false;
-            const uint64_t now = global_timer_ns();
-            if (t0 == 0) {
-                t0 = now;
-            } else if (now - t0 > kWaitLimitNs) {
+        if (__all_sync(0xffffffffu, kSpin ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity))) return true;
+        if (kBackoff && !kSpin) __nanosleep(100);
+        if ((++spins & (kEvery - 1)) == 0) {
+            if (spins == kEvery) t0 = now();
+            if (__any_sync(0xffffffffu, *abort_flag != 0 || now() - t0 > (uint32_t)(limit_ns >> 16))) {
                 atomicCAS((uint32_t*)abort_flag, 0u, code);
                 return false;
             }
