@@ -972,10 +972,9 @@ int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_
     CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaFuncAttributes attr;
     CFX_CUDA(cudaFuncGetAttributes(&attr, k));
-    if (attr.numRegs < split::kLaunchRegs) {   // (its warps would wait for registers that do not exist)
-        set_error("small-batch kernel: built with fewer registers than its warps share out");
-        return CFX_ERR_CUDA;
-    }
+    // Built with fewer registers than its warps share out, they would wait for some that do not exist: such a build does without
+    // this kernel, and cfx_fused.cu's takes every batch.
+    if (attr.numRegs < split::kLaunchRegs) return CFX_OK;
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = split::config(at, sm_count / S * S, S, smem, nullptr);
     cfg.numAttrs = 1;
