@@ -71,19 +71,28 @@ enum Bar {
 
 // Shared memory map (offsets from a 1024-byte aligned base) and the shapes that depend on the
 // launch mode.
-//  weight ring: four stages of 24 KB in a CTA pair (cta_group::2: every CTA stages half of the rows), two of 48 KB with one
-//    CTA per tile;
+//  weight ring, a CTA pair (cta_group::2: every CTA stages half of the rows): four stages of 24 KB, an encoder block of 256
+//    units or two of 128, or half a gate slice with all K blocks;
+//  weight ring, one CTA per tile: a gate stage has two K blocks of half a slice (24 KB).  Hidden 256: four stages of 24 KB, and the
+//    encoder blocks (32 KB), which lie one behind the other in the image, are cut every 192 rows.  Hidden 128: three of 32 KB.  us a
+//    step, 131,072 envs h256x1, h256x3, h128x3, with two stages of 48 KB 162, 321, 157, three of 32 KB 152, 320, 139, four
+//    of 24 KB with encoder blocks in halves 161, 308, 145, as it is 145, 294, 139: a stage's way from L2 takes about as long as the
+//    products of two, so it is the number of full stages that counts;
 //  data area: 8 x 16 KB.  First the tile's records, 16 rows a slot (the classic game's all in slots 0 and 1), then the state boxes
 //    of the layers.  A slot's records of the next tile are fetched as soon as the last layer's box has left it: REC_FREE and
 //    S_FREE order the two uses.
 template <bool PAIR, int GAME, int HID> struct Cfg {
     static constexpr int kH = HID, kStateItems = Hd<HID>::kStateItems;
-    static constexpr int kNB = PAIR ? 4 : 2;
-    static constexpr int kBSlot = PAIR ? 24576 : 49152;
-    static constexpr int kEncPer = 256 / HID;                // encoder blocks of a stage
+    static constexpr bool kCut = !PAIR && HID == 256;        // encoder stages of 192 rows: a block of 256 takes parts of two
+    static constexpr int kNB = PAIR || kCut ? 4 : 3;
+    static constexpr int kBSlot = PAIR || kCut ? 24576 : 32768;
+    static constexpr int kEncPer = 256 / HID;                // encoder blocks of a stage that holds whole ones
     static constexpr int kEncRows = PAIR ? HID / 2 : HID;    // rows of a block that a CTA stages
+    static constexpr int kCutRows = 192, kCutUnit = HID - kCutRows;   // three blocks are four stages
     static constexpr int kGateRows = PAIR ? kHalfRows / 2 : kHalfRows;
-    static constexpr int kEncStages = Gm<GAME>::kEncBlocks / kEncPer, kLayerStages = 2 * Hd<HID>::kSlices;
+    static constexpr int kGateKb = PAIR ? Hd<HID>::kKBlocks : 2;   // K blocks of a gate stage
+    static constexpr int kEncStages = kCut ? (Gm<GAME>::kEncBlocks * HID + kCutRows - 1) / kCutRows : Gm<GAME>::kEncBlocks / kEncPer;
+    static constexpr int kLayerStages = 2 * Hd<HID>::kSlices * (Hd<HID>::kKBlocks / kGateKb);
     static constexpr int kHeadRows = PAIR ? Gm<GAME>::kHeadPair : Gm<GAME>::kHeadSingle;   // N of the head MMA
     static constexpr int kHeadKbBytes = (PAIR ? kHeadRows / 2 : kHeadRows) * 128;   // one K block of the head rows a CTA stages
     static constexpr int kM = PAIR ? 256 : 128;
@@ -102,7 +111,7 @@ template <bool PAIR, int GAME, int HID> struct Cfg {
     static constexpr int kSmemBytes = kOffMisc + 16 + 1024;   // + alignment slack
     static_assert(kNB <= kNBMax && kSmemBytes <= 232448 && kHeadRows <= kHeadMax && kRecSlots <= kNS &&
                       64 + kRecRows * kRecBytes <= kRecSlots / kRecCopies * kSSlot && kRecRows * kRecBytes % 16 == 0 && kNS % kStateItems == 0 &&
-                      Gm<GAME>::kEncBlocks % kEncPer == 0 && kEncPer * kEncRows * 128 <= kBSlot && Hd<HID>::kKBlocks * kGateRows * 128 <= kBSlot &&
+                      Gm<GAME>::kEncBlocks % kEncPer == 0 && (kCut ? kCutRows : kEncPer * kEncRows) * 128 <= kBSlot && kGateKb * kGateRows * 128 <= kBSlot &&
                       Hd<HID>::kKBlocks * kHeadKbBytes <= kBSlot && kGateRows % 8 == 0, "layout");
 };
 
@@ -244,10 +253,13 @@ __device__ __forceinline__ void role_weight_loads(const Smem& sm, const Params& 
         int region, row, blk;   // rows [row, ...) of blocks blk, blk + 1, ...
         uint32_t bytes;
         if (s < C::kEncStages) {
-            region = 0; row = 0; blk = s * C::kEncPer; bytes = C::kEncPer * kEncBlockBytes;
+            region = 0; row = 0; blk = s * C::kEncPer;
+            bytes = C::kCut ? min(C::kBSlot, Gm<GAME>::kEncBlocks * kEncBlockBytes - s * C::kBSlot) : C::kEncPer * kEncBlockBytes;
         } else if (s < enc_gate) {
             const int g = s - C::kEncStages;
-            region = 1; row = kHalfRows * (g & 1); blk = g / 2 * kKBlocks; bytes = kKBlocks * kHalfRows * 128;
+            constexpr int kParts = kKBlocks / C::kGateKb;   // stages of half a slice
+            region = 1; row = kHalfRows * (g / kParts & 1); blk = g / (2 * kParts) * kKBlocks + g % kParts * C::kGateKb;
+            bytes = C::kGateKb * kHalfRows * 128;
         } else {
             region = 2; row = 0; blk = (int)rank; bytes = head_bytes<GAME, HID>(PAIR);
         }
@@ -274,10 +286,10 @@ __device__ __forceinline__ void role_weight_loads(const Smem& sm, const Params& 
             mbar_arrive_expect_tx(full, bytes);
             const uint8_t* gates = P.image + enc_bytes<GAME, HID>();
             if (region == 0) {
-                bulk_g2s(dst, P.image + (size_t)blk * kEncBlockBytes, bytes, full);
+                bulk_g2s(dst, P.image + (C::kCut ? (size_t)s * C::kBSlot : (size_t)blk * kEncBlockBytes), bytes, full);
             } else if (region == 1) {
 #pragma unroll
-                for (int b = 0; b < kKBlocks; b++)
+                for (int b = 0; b < C::kGateKb; b++)
                     bulk_g2s(dst + b * kHalfRows * 128, gates + (size_t)(blk + b) * kGateBlockBytes + row * 128, kHalfRows * 128, full);
             } else {
                 bulk_g2s(dst, gates + (size_t)P.L * kSlices * kKBlocks * kGateBlockBytes, bytes, full);
@@ -440,7 +452,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
     auto gate_mmas = [&](int h, int kb, uint32_t a_cur, uint64_t bd0) {
 #pragma unroll
         for (int ks = 0; ks < 4; ks++)
-            MMA_TS(tmem + kColG + h * kHalfRows, a_cur + kb * 32 + ks * 8, bd0 + (uint64_t)(kb * kGateBlkStep + 2 * ks), idesc_gate,
+            MMA_TS(tmem + kColG + h * kHalfRows, a_cur + kb * 32 + ks * 8, bd0 + (uint64_t)(kb % C::kGateKb * kGateBlkStep + 2 * ks), idesc_gate,
                    (kb | ks) != 0 ? 1u : 0u);
     };
 #define CFX_WAIT_PROBED(name, barid, parity, code)                                                  \
@@ -459,7 +471,55 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         probe_a(acnt);
         CFX_PROBE(cfx_p_b, sm.bar(B_FULL + bslot), bpar);
         // ---- encoder: N = kH units; a block of 64 K columns is one operand chunk
-        for (int kc = 0; kc < kEncBlocks; kc += C::kEncPer) {
+        // the K steps of a block against n units of it from `unit` on, at bd
+        auto enc_mmas = [&](uint32_t a_col, uint64_t bd, bool first, bool last, int unit, int n) {
+            const uint32_t d = tmem + kColAcc + unit, idesc = n == kH ? idesc_enc : make_idesc(fmt, C::kM, n);
+            // the last block has 25 features (full game: two K steps) or one (classic: one K step)
+            MMA_TS(d, a_col, bd, idesc, first ? 0u : 1u);
+            if (GAME == CFX_GAME_FULL || !last) MMA_TS(d, a_col + 8, bd + 2, idesc, 1);
+            if (!last) {
+                MMA_TS(d, a_col + 16, bd + 4, idesc, 1);
+                MMA_TS(d, a_col + 24, bd + 6, idesc, 1);
+            }
+        };
+        if constexpr (C::kCut) {   // a block is multiplied in two parts, from the stage that its first units are in and from the next one
+            int slot = 0;
+            for (int kc0 = 0; kc0 < kEncBlocks; kc0 += 3) {
+#pragma unroll
+                for (int q = 0; q < 3; q++, acnt++) {   // the first q kCutUnit rows of the stage were the block before's
+                    const int kc = kc0 + q, as = acnt % kAexpSlots, n0 = C::kCutRows - C::kCutUnit * q;
+                    if (kc >= kEncBlocks) break;
+                    const bool last = kc == kEncBlocks - 1;
+                    if (q == 0) {
+                        slot = bslot;
+                        CFX_WAIT_PROBED(cfx_p_b, B_FULL + slot, bpar, W_B_FULL);
+                        probe_b_next();
+                        b_advance();
+                    }
+                    CFX_WAIT_PROBED(cfx_p_a, AEXP_FULL + as, (acnt / kAexpSlots) & 1, W_AEXP_FULL);
+                    if (!last) probe_a(acnt + 1);
+                    tc_fence_after_sync();
+                    __syncwarp();
+                    const uint32_t a_col = tmem + kColAexp + as * 32;
+                    if (elect_one()) {
+                        enc_mmas(a_col, bdesc0 + (uint64_t)(slot * (kBSlot >> 4) + ((q * C::kCutUnit * 128) >> 4)), kc == 0, last, 0, n0);
+                        MMA_COMMIT(sm.bar(B_EMPTY + slot));
+                    }
+                    slot = bslot;
+                    CFX_WAIT_PROBED(cfx_p_b, B_FULL + slot, bpar, W_B_FULL);
+                    probe_b_next();
+                    b_advance();
+                    tc_fence_after_sync();
+                    __syncwarp();
+                    if (elect_one()) {
+                        enc_mmas(a_col, bdesc0 + (uint64_t)(slot * (kBSlot >> 4)), kc == 0, last, n0, kH - n0);
+                        MMA_COMMIT(sm.bar(AEXP_EMPTY + as));
+                        if (q == 2 || last) MMA_COMMIT(sm.bar(B_EMPTY + slot));
+                        if (last) MMA_COMMIT(sm.bar(ACC_FULL));
+                    }
+                }
+            }
+        } else for (int kc = 0; kc < kEncBlocks; kc += C::kEncPer) {
             const int slot = bslot;
             CFX_WAIT_PROBED(cfx_p_b, B_FULL + slot, bpar, W_B_FULL);
             CFX_MARK(3);
@@ -477,13 +537,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                 const uint32_t a_col = tmem + kColAexp + as * 32;
                 const uint64_t bd = bdesc0 + (uint64_t)(slot * (kBSlot >> 4) + c2 * kEncBlkStep);
                 if (elect_one()) {
-                    // the last block has 25 features (full game: two K steps) or one (classic: one K step)
-                    MMA_TS(tmem + kColAcc, a_col, bd, idesc_enc, c2 != 0 || kc != 0 ? 1u : 0u);
-                    if (GAME == CFX_GAME_FULL || !last) MMA_TS(tmem + kColAcc, a_col + 8, bd + 2, idesc_enc, 1);
-                    if (!last) {
-                        MMA_TS(tmem + kColAcc, a_col + 16, bd + 4, idesc_enc, 1);
-                        MMA_TS(tmem + kColAcc, a_col + 24, bd + 6, idesc_enc, 1);
-                    }
+                    enc_mmas(a_col, bd, c2 == 0 && kc == 0, last, 0, kH);
                     MMA_COMMIT(sm.bar(AEXP_EMPTY + as));
                     if (c2 == C::kEncPer - 1) MMA_COMMIT(sm.bar(B_EMPTY + slot));
                     if (last) MMA_COMMIT(sm.bar(ACC_FULL));
@@ -510,36 +564,40 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                         CFX_WAIT_LEADER(ACC_READ, tcnt & 1, W_ACC_READ);
                         CFX_MARK(9);
                     }
-                    const int slot = bslot;
-                    CFX_WAIT_PROBED(cfx_p_b, B_FULL + slot, bpar, W_B_FULL);
-                    CFX_MARK(6);
-                    probe_b_next();
-                    b_advance();
-                    const uint64_t bd0 = bdesc0 + (uint64_t)(slot * (kBSlot >> 4));
-                    if (h == 0 && j == 0) {   // the layer's input arrives K block by K block (slice kb of the previous layer)
-                        for (int kb = 0; kb < kKBlocks; kb++) {
-                            CFX_WAIT_LEADER(A_KB + kb, akb_use & 1, W_A_KB);
-                            CFX_MARK(9);
+#pragma unroll
+                    for (int kp = 0; kp < kKBlocks; kp += C::kGateKb) {
+                        const int slot = bslot;
+                        CFX_WAIT_PROBED(cfx_p_b, B_FULL + slot, bpar, W_B_FULL);
+                        CFX_MARK(6);
+                        probe_b_next();
+                        b_advance();
+                        const uint64_t bd0 = bdesc0 + (uint64_t)(slot * (kBSlot >> 4));
+                        if (h == 0 && j == 0) {   // the layer's input arrives K block by K block (slice kb of the previous layer)
+                            for (int kb = kp; kb < kp + C::kGateKb; kb++) {
+                                CFX_WAIT_LEADER(A_KB + kb, akb_use & 1, W_A_KB);
+                                CFX_MARK(9);
+                                tc_fence_after_sync();
+                                __syncwarp();
+                                if (elect_one()) gate_mmas(h, kb, a_cur, bd0);
+                            }
+                        } else {
                             tc_fence_after_sync();
                             __syncwarp();
-                            if (elect_one()) gate_mmas(h, kb, a_cur, bd0);
-                        }
-                    } else {
-                        tc_fence_after_sync();
-                        __syncwarp();
-                        if (elect_one()) {
+                            if (elect_one()) {
 #pragma unroll
-                            for (int kb = 0; kb < kKBlocks; kb++) gate_mmas(h, kb, a_cur, bd0);
+                                for (int kb = kp; kb < kp + C::kGateKb; kb++) gate_mmas(h, kb, a_cur, bd0);
+                            }
                         }
+                        __syncwarp();
+                        // (the other half's accumulator: handed back while this half is multiplied)
+                        const bool ends = kp + C::kGateKb == kKBlocks;
+                        if (ends) CFX_PROBE(cfx_p_ge, sm.bar(G_EMPTY + (h ^ 1)), ((gcnt + h) & 1) ^ 1);
+                        if (elect_one()) {
+                            if (ends) MMA_COMMIT(sm.bar(G_FULL + h));
+                            MMA_COMMIT(sm.bar(B_EMPTY + slot));
+                        }
+                        CFX_MARK(7);
                     }
-                    __syncwarp();
-                    // (the other half's accumulator: handed back while this half is multiplied)
-                    CFX_PROBE(cfx_p_ge, sm.bar(G_EMPTY + (h ^ 1)), ((gcnt + h) & 1) ^ 1);
-                    if (elect_one()) {
-                        MMA_COMMIT(sm.bar(G_FULL + h));
-                        MMA_COMMIT(sm.bar(B_EMPTY + slot));
-                    }
-                    CFX_MARK(7);
                 }
             }
         }
