@@ -129,14 +129,6 @@ struct Smem {
 #define CFX_SWAIT_SPIN(barid, parity) \
     if (!mbar_wait_warp<false, true>(sm.bar(barid), (parity), sm.abort_flag(), kSite + (barid))) return
 
-// shared memory of this CTA -> shared memory of another CTA of the cluster, counted on a barrier there
-__device__ __forceinline__ void bulk_s2s(uint32_t dst_cluster, uint32_t src, uint32_t bytes, uint32_t bar_cluster) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_cluster),
-        "r"(src), "r"(bytes), "r"(bar_cluster)
-        : "memory");
-}
-
 // arrives on the barrier in every CTA of the cluster when all MMAs issued so far are done
 template <int S>
 __device__ __forceinline__ void mma_commit_all(uint32_t bar) {

@@ -10,10 +10,11 @@
 namespace cfx {
 namespace umma {
 
-// Debug builds (-DCFX_CHECK): every wrapper verifies the alignment rules of its operands,
-// reports a violation with printf and SKIPS the operation (the kernel's bounded waits then
+// Debug builds (-DCFX_CHECK): the wrappers of barriers on this CTA's side and of asynchronous copies verify the alignment rules
+// of their operands, report a violation with printf and SKIP the operation (the kernel's bounded waits then
 // end it with a status code instead of a fault).
 #ifdef CFX_CHECK
+#include <cstdio>
 #define CFX_CHK(cond, what, a, b)                                                          \
     if (!(cond)) {                                                                         \
         printf("CFX_CHECK %s: block %d thread %d a=%llx b=%llx\n", what, (int)blockIdx.x,  \
@@ -207,11 +208,14 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void* src, uin
         ::"r"(dst_smem), "l"(src), "r"(bytes), "r"(bar)
         : "memory");
 }
-// 1-D bulk copy shared -> global (bulk async-group completion).
-__device__ __forceinline__ void bulk_s2g(void* dst, uint32_t src_smem, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-                 "r"(src_smem), "r"(bytes)
-                 : "memory");
+// Shared memory of this CTA -> shared memory of another CTA of the cluster, counted on a barrier there (addresses from map_to_cta;
+// 16-byte aligned, bytes a multiple of 16).
+__device__ __forceinline__ void bulk_s2s(uint32_t dst_cluster, uint32_t src, uint32_t bytes, uint32_t bar_cluster) {
+    CFX_CHK((dst_cluster & 15) == 0 && (src & 15) == 0 && (bytes & 15) == 0 && (bar_cluster & 7) == 0, "bulk_s2s", dst_cluster, src)
+    asm volatile(
+        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_cluster),
+        "r"(src), "r"(bytes), "r"(bar_cluster)
+        : "memory");
 }
 // 2-D tiled tensor copy global -> shared.  x = innermost coordinate (x * elemsize must be
 // a multiple of 16 bytes), y = outer coordinate.
@@ -229,6 +233,7 @@ __device__ __forceinline__ void tensor_g2s_2d(uint32_t dst_smem, const CUtensorM
 // the pair; `cluster_bar` is a shared::cluster address (mapa).  No multicast.
 __device__ __forceinline__ void tensor_g2s_3d_pair(uint32_t dst_smem, const CUtensorMap* map, int x,
                                                    int y, int z, uint32_t cluster_bar) {
+    CFX_CHK((dst_smem & 127) == 0 && ((uintptr_t)map & 63) == 0 && (cluster_bar & 7) == 0, "tensor_g2s_3d_pair", dst_smem, (uintptr_t)map)
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
         "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst_smem),
@@ -237,6 +242,7 @@ __device__ __forceinline__ void tensor_g2s_3d_pair(uint32_t dst_smem, const CUte
 }
 // 4-D, counted on a barrier of this CTA
 __device__ __forceinline__ void tensor_g2s_4d(uint32_t dst_smem, const CUtensorMap* map, int x, int y, int z, int w, uint32_t bar) {
+    CFX_CHK((dst_smem & 127) == 0 && ((uintptr_t)map & 63) == 0 && (bar & 7) == 0, "tensor_g2s_4d", dst_smem, (uintptr_t)map)
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
         "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst_smem),
@@ -266,6 +272,7 @@ __device__ __forceinline__ void bulk_wait_group() {
 // Asks the memory system to bring [src, src + bytes) into L2 (no completion tracking);
 // src 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
+    CFX_CHK(((uintptr_t)src & 15) == 0 && (bytes & 15) == 0, "bulk_prefetch_l2", (uintptr_t)src, bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
