@@ -33,6 +33,10 @@ namespace umma {
 #endif
 
 // ------------------------------------------------------------------ addresses
+// A barrier in this CTA's shared memory (227 KB and the first KB).  In a cluster the address of a CTA's own shared memory has its
+// rank from bit 24 on.
+__host__ __device__ constexpr bool own_barrier(uint32_t bar) { return (bar & 7) == 0 && (bar & 0xFFFFFFu) < 233472; }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -55,23 +59,23 @@ __device__ __forceinline__ bool elect_one() {
 
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    CFX_CHK((bar & 7) == 0 && bar < 233472, "mbar_init", bar, count)
+    CFX_CHK(own_barrier(bar), "mbar_init", bar, count)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    CFX_CHK((bar & 7) == 0 && bar < 233472, "mbar_arrive", bar, 0)
+    CFX_CHK(own_barrier(bar), "mbar_arrive", bar, 0)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    CFX_CHK((bar & 7) == 0 && bar < 233472, "mbar_expect_tx", bar, bytes)
+    CFX_CHK(own_barrier(bar), "mbar_expect_tx", bar, bytes)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    CFX_CHK_BOOL((bar & 7) == 0 && bar < 233472, "mbar_try_wait", bar, parity)
+    CFX_CHK_BOOL(own_barrier(bar), "mbar_try_wait", bar, parity)
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred P;\n\t"
@@ -87,7 +91,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // cycles against ~67 for try_wait; inside the fused kernel, however, putting a test_wait in
 // front of every worker wait made the kernel 6 % slower, so only the MMA warp polls with it.
 __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
-    CFX_CHK_BOOL((bar & 7) == 0 && bar < 233472, "mbar_test_wait", bar, parity)
+    CFX_CHK_BOOL(own_barrier(bar), "mbar_test_wait", bar, parity)
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred P;\n\t"
@@ -475,7 +479,7 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
 // Makes the mbarrier track completion of all MMAs this thread issued so far
 // (implies tcgen05.fence::before_thread_sync).
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
-    CFX_CHK((bar & 7) == 0 && bar < 233472, "mma_commit", bar, 0)
+    CFX_CHK(own_barrier(bar), "mma_commit", bar, 0)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
