@@ -6,6 +6,9 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#ifdef CFX_CHECK
+#include <cstdio>
+#endif
 
 namespace cfx {
 namespace umma {
@@ -14,7 +17,6 @@ namespace umma {
 // of their operands, report a violation with printf and SKIP the operation (the kernel's bounded waits then
 // end it with a status code instead of a fault).
 #ifdef CFX_CHECK
-#include <cstdio>
 #define CFX_CHK(cond, what, a, b)                                                          \
     if (!(cond)) {                                                                         \
         printf("CFX_CHECK %s: block %d thread %d a=%llx b=%llx\n", what, (int)blockIdx.x,  \
