@@ -321,7 +321,8 @@ __device__ __forceinline__ void role_loads(const Smem& sm, const Params& P) {
     const int boxes = P.L * kStateItems;
     uint32_t it = 0;
     uint32_t fpar = 0;      // slots: parity of the "free" phase to wait for
-    // rows [32 q, 32 q + 32) are a quadrant's (n is a multiple of 32): all of them are there or none, and then nobody looks at them
+    // rows [32 q, 32 q + 32) are a quadrant's (n is a multiple of 32): all of them are there or none, and then what lies in the slot
+    // is converted and multiplied like records, and the results of those rows are dropped
     auto load_records = [&](int tile, int i) {
         const int r = i * C::kRecRows, row0 = tile * kTile + r, rows = min(C::kRecRows, P.n - row0);
         const uint32_t full = sm.bar(REC_FULL + r / 32);
@@ -882,13 +883,12 @@ k_policy_fused(const __grid_constant__ Params P) {
     CFX_DIMS(HID);
     constexpr int kA = Gm<GAME>::kA;
     // predicates of the deferred probes: weight loads, MMA warp (gate accumulators, weights, operand chunks), workers (operand
-    // slot, records, state box, next accumulator)
+    // slot, state box, next accumulator)
     CFX_PROBE_DECL(cfx_p_b);
     CFX_PROBE_DECL(cfx_p_a);
     CFX_PROBE_DECL(cfx_p_w);
     CFX_PROBE_DECL(cfx_p_ge);
     CFX_PROBE_DECL(cfx_p_ae);
-    CFX_PROBE_DECL(cfx_p_r);
     CFX_PROBE_DECL(cfx_p_s);
     CFX_PROBE_DECL(cfx_p_g);
     extern __shared__ uint8_t smem_raw[];
@@ -1272,10 +1272,6 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     }
     fused::Params P;
     const bool classic = p->game == CFX_GAME_CLASSIC;
-    if (((uintptr_t)a.records & 15) != 0) {
-        set_error("fused forward: records must be 16-byte aligned");
-        return CFX_ERR_CUDA;
-    }
     for (int l = 0; l < p->L; l++) P.state_map[l] = p->state_map[l];
     for (int r = 0; r < 3; r++) P.w_map[r] = p->w_map[r];
     for (int r = 0; r < 2; r++) P.gate_map[r] = p->gate_map[r];

@@ -29,7 +29,7 @@ template <int HID> struct Hd {
     static constexpr int kStateItems = HID / kHalfUnits;  // state boxes (128 rows x 32 units) per layer (8 / 4)
     static constexpr int kKBlocks = HID / 64;             // K blocks of 64 per HID-wide operand (4 / 2)
     static constexpr int kEncBlockBytes = HID * 128;      // one encoder block: [HID units][64 K] 16-bit
-    static_assert((HID / 64) % 2 == 0, "a gate stage carries two K blocks");
+    static_assert((HID / 64) % 2 == 0, "a gate stage of one CTA per tile and a head slot of the small-batch form carry two K blocks");
 };
 // brings the shapes of Hd<HID> into a function body
 #define CFX_DIMS(HID)                                                                        \

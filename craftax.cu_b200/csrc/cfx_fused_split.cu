@@ -669,7 +669,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
                                                 uint32_t rank, Meetings& meet) {
     using Op = Op16<T16>;
     using C = Cfg<GAME, HID, S>;
-    constexpr int kChunks = Gm<GAME>::kEncChunks, kA = Gm<GAME>::kA;
+    constexpr int kChunks = Gm<GAME>::kEncChunks;
     constexpr bool kFull = GAME == CFX_GAME_FULL;
     const int quadrant = warp & 3, wg = (warp - kWorkerWarp0) >> 2, w = 4 * quadrant + wg, unit = 4 * w, swz = lane & 7;
     const uint32_t lane_base = tmem + ((uint32_t)(quadrant * 32) << 16);
