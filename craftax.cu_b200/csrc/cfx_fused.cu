@@ -25,10 +25,14 @@
 //                  tile; full game or classic game (GAME): see Cfg and Gm
 //   hidden size    256 (the figures in this comment) or 128 (HID): two gate slices of two K
 //                  blocks per layer, A0 / A1 of 64 columns, encoder accumulator N = 128: see Hd
-// What bounds it: in long runs the board's power limit (1,000 W: 262,144 envs h256x2 run at 1.35 GHz, and without the MMAs
-// take 283 us at 1,965 MHz instead of 405).  In cycles, per tile of h256x2, 33,700 (39,900 with eight worker warps, record boxes through
-// a ring and one gate accumulator, which took 415 us): encoder 11,800, of which 2,300 until the last records are there
-// and converted, 2,300 to the first gate accumulator, 2,300 a slice (1,540 of SFU and of tensor pipe), heads.  What mattered, all of it seen
+// What bounds it: in long runs the board's power limit (1,000 W).  262,144 envs h256x2, 14 tiles a CTA, by the SM's clock and the global
+// timer read in the kernel: in a long run 455,000 cycles in 394 us, 1.16 GHz (410 us a step; nvidia-smi reads 1.16 to 1.31 GHz
+// meanwhile), in a burst of 20 launches 467,000 in 338 us, 1.38 GHz (346 us a step).  A CTA's first tile takes 41,000 cycles, the
+// others 31,700, the last 30,800.  With eight worker warps, record boxes through a ring and one gate accumulator a tile took 39,900 and a
+// step 415 us: that was 1.35 GHz, so fewer cycles come back as time only in part.  Without the MMAs a step takes 283 us at 1,965 MHz.
+// Of a tile (33,700 cycles with the marks of a timeline): encoder 11,800, of which 2,300 until the last records are there
+// and converted, 2,300 to the first gate accumulator, 2,300 a slice (1,540 of SFU and of tensor pipe), heads.  96 registers a thread,
+// and 68 / 60 bytes of spill stores / loads (pairs, full game, hidden 256).  What mattered, all of it seen
 // in clock64 timelines and rates of single instructions:
 //   * a TMA store runs at 32 B a cycle, the SM's rate of writing, and copies queue behind it: 16 KB of state are 512
 //     cycles.  Written by the workers instead (8 rows x 64 B an instruction) they held up the cells (262,144 envs 359 against 346 us);
@@ -1316,10 +1320,13 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     P.off_b_v = o.b_v;
     if (launches) *launches = 1;
     // Small batches: a tile is shared by four (two) CTAs as long as every tile then has its SMs at once, and is as
-    // short as that allows (cfx_fused_split.cu).  us a step, h256x2: 1,600 envs 16.0 with four CTAs and 64 rows, 18.0 with
-    // two and 32; 1,024 envs 13.6 with 32 rows, 15.5 with 64, 17.4 with 128.  CTAs of two slices take tiles of 64 and
+    // short as that allows (cfx_fused_split.cu).  CTAs of two slices take tiles of 64 and
     // 128 rows; at 32 four CTAs a tile have their SMs.  With the 33 clusters of four and 74 of two that this part holds, four
-    // CTAs go to 1,056, 2,112 and 4,224 envs, and two to 4,736 with 64 rows (4,544 envs h256x3 23.4 us, with 128 rows 25.0).
+    // CTAs go to 1,056, 2,112 and 4,224 envs, and two to 4,736 with 64 rows and 9,472 with 128.  At each of these limits the next
+    // form is slower, and the kernel below slower than all of them.  us a step, h256x2, clusters of four with 32, 64, 128
+    // rows, of two with 64 and 128, the kernel below: 1,056 envs 10.6, 14.7, 16.8, 17.7, 19.2, 21.5; 2,112 -, 15.0, 16.7, 18.0, 19.4, 21.8; 4,224
+    // -, -, 17.7, 18.4, 19.7, 22.0; 4,736 -, -, -, 18.7, 19.6, 22.5; 9,472 -, -, -, -, 20.3, 22.6.  h128x2, of two with 32, 64, 128 rows:
+    // 2,368 envs 9.0, 12.6, 13.5, 15.6; 4,736 -, 13.1, 13.6, 15.7; 9,472 -, -, 14.2, 16.1.  (h256x3, 4,544: 22.9 with 64 rows, 24.5 with 128.)
     const int rows = std::min(p->n, P.num_tiles * fused::kTile) - P.tile_begin * fused::kTile;
     for (int i = 0; i < 2; i++)
         for (int S = i == 0 ? 4 : 2, tr = p->H == 64 * S ? 32 : 64; tr <= fused::kTile; tr *= 2) {

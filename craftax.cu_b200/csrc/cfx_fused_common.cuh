@@ -39,15 +39,14 @@ template <int HID> struct Hd {
 
 // What differs between the two games the kernel is instantiated for.
 //  full game (craftax_full.cu): 996-byte record = 792 map bytes + 51 raw floats, 843 features.
-//    The record goes through the record ring in 16 chunks of 64 RECORD bytes: chunks 0-11 are 64
+//    It is expanded by weight blocks (cfx_fused.cu) or in 16 chunks of 64 RECORD bytes (cfx_fused_split.cu): chunks 0-11 are 64
 //    map bytes each (four K steps), chunk 12 is 24 map bytes and floats 0-9 (three K steps),
 //    chunks 13 and 14 are 16 floats each and chunk 15 the last 9 floats (one K step each).  The
 //    weight image has 14 blocks of 64 K columns: blocks 0-11 belong to chunks 0-11, block 12 to
 //    chunks 12 and 13 (K columns 0-47 and 48-63), block 13 to chunks 14 and 15 (K columns 0-15
 //    and 16-31).  43 actions;
 //  classic game (craftax_classic.cu): 148-byte record, 1345 one-hot / scalar features in 22
-//    chunks (one weight block each), the whole tile's records (18.5 KB) fetched by one TMA box,
-//    17 actions.
+//    chunks (one weight block each), 17 actions.
 template <int GAME> struct Gm;
 template <> struct Gm<CFX_GAME_FULL> {
     static constexpr int kA = 43, kEncChunks = 16, kEncBlocks = 14, kRecBytes = kRec;
@@ -87,7 +86,7 @@ struct Params {
     CUtensorMap state_map[kMaxLayers];   // fp32 [n][256] per layer, box 128 x 32, SWIZZLE_128B
     const uint8_t* records;              // [n][996] (classic [n][148])
     const float* state;                  // [L][n][256]
-    const uint8_t* image;                // pre-swizzled 16-bit weight stages in consumption order
+    const uint8_t* image;                // pre-swizzled 16-bit weight blocks: see above
     const float* params;                 // fp32 arena (biases are read from it)
     const float* prev_terminals;
     const float* uniforms;
@@ -192,7 +191,7 @@ __device__ __forceinline__ float tanh_fast(float x) {
 }
 
 // Two units at once with the packed fp32 instructions: the cell phase is bound by instruction
-// issue and latency (two worker warps per scheduler), not by the FMA pipe.
+// issue and latency (four worker warps per scheduler), not by the FMA pipe.
 // hzh, hzg, hzp: zh/2, zg/2, zp/2 of two units
 __device__ __forceinline__ void mingru_cell_pair(float hzh0, float hzh1, float hzg0, float hzg1, float hzp0,
                                                  float hzp1, float st0, float st1, float x0, float x1,

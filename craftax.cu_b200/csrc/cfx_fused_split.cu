@@ -2,12 +2,11 @@
 // SMs) of its own: a tile is given to a cluster of S CTAs (2 or 4), each of which owns 1/S of the hidden
 // units.  What a small batch costs is one tile's chain of dependent steps; here the chain is
 // shorter: a CTA multiplies 64 NS instead of 256 encoder columns, one gate slice (NS = 1) instead of four a
-// layer, and sixteen worker warps share the expansion and the cell where the one-SM kernel
-// (cfx_fused.cu) has eight.
+// layer, and sixteen worker warps share the expansion and the cell of 1/S of the units.
 //
 //   records   the tile's records are contiguous: four bulk copies of 32 rows into shared memory.  A row is an odd
 //             number of words, so thread-per-row reads have no bank conflicts.  (Tensor boxes of 80 bytes a
-//             row, as in cfx_fused.cu, cost more than the rest of the encoder here.)  Every CTA of
+//             row cost more than the rest of the encoder.)  Every CTA of
 //             the cluster expands the whole record into tensor memory, chunk kc by warpgroup kc % 4
 //   encoder   A from tensor memory, N = 64 NS own units
 //   layers    A from shared memory: the layer's input as K blocks of 64 units (128-byte swizzled operand
@@ -30,9 +29,9 @@
 // The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
 // records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
-// Measured (us a step in a stream, h256x2, fp16; one CTA pair per two tiles -> here): 32 envs 25.7 -> 9.9, 1,024 25.7 -> 10.8,
-// 2,048 26 -> 15.3, 4,000 26 -> 18.2, 8,192 26.9 -> 20.8; classic h256x3, 1,024 envs 35.7 -> 16.1 (before the products of 32 rows).  Bound by the chain of
-// dependent steps and the 1.3 us between one kernel's end and the next one's start.
+// Measured (us a step in a stream, fp16; the persistent kernel, one CTA pair per two tiles -> here): h256x2, 32 envs 20.6 -> 9.5,
+// 256 21.6 -> 9.95, 1,024 21.5 -> 10.5, 2,048 21.7 -> 15.0, 4,000 22.2 -> 17.6, 8,192 22.6 -> 20.2; classic h256x3, 1,024 envs 28.9 -> 14.5, 4,000
+// 29.7 -> 25.3, 8,192 30.2 -> 28.7.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
 #include "cfx_fused_split.h"
 
 #include <type_traits>
@@ -68,8 +67,8 @@ template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kEncPerItem = kNS == 1 ? 3 : 1;        // encoder blocks of one ring slot
     static constexpr int kEncItems = (Gm<GAME>::kEncBlocks + kEncPerItem - 1) / kEncPerItem;
     // ONE: ring slots whose operand chunks the MMA warp waits for together: the full game's sixteen chunks, a warp each, are there
-    // at the same time (1,024 envs 10.8 us, 11.0 with a wait a slot, 11.6 with one a chunk); the classic game's 22 are not
-    // (13.3 with two waits for all of them, 13.1 with one a slot, 13.0 with one a chunk)
+    // at the same time (1,024 envs 10.8 us, 11.0 with a wait a slot, 11.6 with one a chunk); the classic game's 22 are not, and it
+    // makes no difference (13.3 with two waits for all of them, 13.1 with one a slot, 13.0 with one a chunk, runs 0.2 apart)
     static constexpr int kGroupItems = GAME == CFX_GAME_FULL ? kEncItems : 1;
     static __device__ __forceinline__ int group_chunks(int group) {
         return GAME == CFX_GAME_FULL ? Gm<GAME>::kEncChunks : max(1, min(kEncPerItem, Gm<GAME>::kEncBlocks - group * kEncPerItem));
