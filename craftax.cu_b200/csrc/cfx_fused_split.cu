@@ -49,11 +49,14 @@ constexpr int kSSlots = 4, kSBox = kTile * 128, kQuadBox = 32 * 128;   // state 
 constexpr uint32_t kColAexp = 0, kColAcc = 384, kColHead = 448;
 __host__ __device__ constexpr uint32_t col_gate(int j) { return 192u * (uint32_t)j; }   // over the operand chunks, done by then
 
-// 96 registers a thread at launch, then 64 for the four warps that copy and multiply and 104 for the sixteen workers, whose
-// cells need no local memory with them where a CTA has two slices (8,192 envs 21.8 -> 21.0 us).  Not in tiles of 32 rows, which
-// need fewer, and not in cfx_fused.cu, whose MMA warp is slower with 64 (262,144 envs 406 -> 418).
+// Clusters of four, tiles of more than 32 rows: 96 registers a thread at launch, then 64 for the four warps that copy and multiply and
+// 104 for the sixteen workers (us a step without and with that: 2,048 envs h256x2 15.04 and 14.86, 4,000 17.75 and 17.60, classic
+// h256x3 2,048 26.2 and 21.9).  Not in tiles of 32 rows, which need fewer, not in cfx_fused.cu, whose MMA warp is slower with 64 (262,144 envs 406 ->
+// 418), and not with two CTAs, whose workers have two slices each and then go through local memory more often (8,192 envs, the same pairs:
+// h256x2 20.05 and 20.21, with a bf16 record 21.89 and 22.34, h256x3 with an fp32 record 29.05 and 30.29, bf16 29.60 and 31.00; h128x2 13.92 and 13.95).
 constexpr int kLaunchRegs = 96, kRoleRegs = 64, kWorkerRegs = 104;
 static_assert(kWorkerWarp0 * kRoleRegs + kWorkerWarps * kWorkerRegs <= (kWorkerWarp0 + kWorkerWarps) * kLaunchRegs, "registers");
+template <int S, bool ONE> constexpr bool kShareRegs = S == 4 && !ONE;
 
 constexpr int kQuadBlock = 32 * 128;                  // ONE: an operand chunk's block, [32 rows][64 K]
 constexpr uint32_t kGateB = 4 * 2 * kWarpUnits * 128;   // ONE: zh and zg of a slice, behind them its zp
@@ -542,7 +545,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             tmem_wait_ld();
             uint8_t* sp = sm.base + C::kOffS + slot * kSBox + (row >> 3) * 1024 + (row & 7) * 128;
             auto piece = [&](int q) { return reinterpret_cast<float4*>(sp + (((4 * (wg & 1) + q) ^ (row & 7)) << 4)); };
-            // (half of the units at a time: with the state of all of them in registers, 22 words went through local memory, 43 with bf16)
+            // (half of the units at a time: with the state of all of them in registers a bf16 cell reads 22 words from local memory, so 4)
 #pragma unroll
             for (int h = 0; h < kWarpUnits / 4; h += 2) {
                 float4 st[2];
@@ -852,7 +855,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     // The operand image and the biases are only ever written by calls that wait for the device, so they may be
     // read while the kernel in front still runs; everything else waits for it.
     if (warp < kWorkerWarp0) {
-        if constexpr (!ONE) registers_dec<kRoleRegs>();
+        if constexpr (kShareRegs<S, ONE>) registers_dec<kRoleRegs>();
         if (warp == 0) {
             if (lane == 0) role_weights<GAME, HID, S, ONE>(sm, P, rank);
             __syncwarp();
@@ -883,7 +886,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
             if (lane == 0) role_state<GAME, HID, S, ONE>(sm, P, row0, rank);
         }
     } else {
-        if constexpr (!ONE) registers_inc<kWorkerRegs>();
+        if constexpr (kShareRegs<S, ONE>) registers_inc<kWorkerRegs>();
         wait_for_previous_kernel();
         cluster_wait();
         Meetings meet;
@@ -965,7 +968,7 @@ int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_
     CFX_CUDA(cudaFuncGetAttributes(&attr, k));
     // Built with fewer registers than its warps share out, they would wait for some that do not exist: such a build does without
     // this kernel, and cfx_fused.cu's takes every batch.
-    if (attr.numRegs < split::kLaunchRegs) return CFX_OK;
+    if (S == 4 && attr.numRegs < split::kLaunchRegs) return CFX_OK;
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = split::config(at, sm_count / S * S, S, smem, nullptr);
     cfg.numAttrs = 1;

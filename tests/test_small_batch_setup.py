@@ -36,7 +36,7 @@ cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunch
 int main(int, char** argv) {
     g_regs = atoi(argv[1]);
     int clusters = -1;
-    const int rc = cfx::fused::split_prepare(CFX_PREC_F16, CFX_GAME_FULL, 256, 4, 148, &clusters);
+    const int rc = cfx::fused::split_prepare(CFX_PREC_F16, CFX_GAME_FULL, 256, atoi(argv[2]), 148, &clusters);
     printf("%d %d\n", rc, clusters);
 }
 """
@@ -56,7 +56,8 @@ def program(cfx, tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("registers,clusters", [(96, 33), (102, 33), (95, 0), (88, 0)])
-def test_too_few_registers_leave_the_kernel_out(program, registers, clusters):
-    out = subprocess.run([program, str(registers)], capture_output=True, text=True, check=True).stdout.split()
+@pytest.mark.parametrize("registers,ctas,clusters", [(96, 4, 33), (102, 4, 33), (95, 4, 0), (88, 4, 0), (88, 2, 33)])
+def test_too_few_registers_leave_the_kernel_out(program, registers, ctas, clusters):
+    """(Two CTAs a tile keep the registers they were launched with.)"""
+    out = subprocess.run([program, str(registers), str(ctas)], capture_output=True, text=True, check=True).stdout.split()
     assert [int(x) for x in out] == [0, clusters]
