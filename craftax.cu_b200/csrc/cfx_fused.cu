@@ -1324,9 +1324,9 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     // 128 rows; at 32 four CTAs a tile have their SMs.  With the 33 clusters of four and 74 of two that this part holds, four
     // CTAs go to 1,056, 2,112 and 4,224 envs, and two to 4,736 with 64 rows and 9,472 with 128.  At each of these limits the next
     // form is slower, and the kernel below slower than all of them.  us a step, h256x2, clusters of four with 32, 64, 128
-    // rows, of two with 64 and 128, the kernel below: 1,056 envs 10.6, 14.7, 16.8, 17.7, 19.2, 21.5; 2,112 -, 15.0, 16.7, 18.0, 19.4, 21.8; 4,224
-    // -, -, 17.7, 18.4, 19.7, 22.0; 4,736 -, -, -, 18.7, 19.6, 22.5; 9,472 -, -, -, -, 20.3, 22.6.  h128x2, of two with 32, 64, 128 rows:
-    // 2,368 envs 9.0, 12.6, 13.5, 15.6; 4,736 -, 13.1, 13.6, 15.7; 9,472 -, -, 14.2, 16.1.  (h256x3, 4,544: 22.9 with 64 rows, 24.5 with 128.)
+    // rows, of two with 64 and 128, the kernel below: 1,056 envs 10.6, 14.6, 16.8, 17.6, 19.0, 21.5; 2,112 -, 15.0, 16.8, 17.9, 19.2, 21.8; 4,224
+    // -, -, 17.7, 18.3, 19.6, 22.1; 4,736 -, -, -, 18.5, 19.4, 22.4; 9,472 -, -, -, -, 20.2, 22.4.  h128x2, of two with 32, 64, 128 rows:
+    // 2,368 envs 9.0, 12.5, 13.5, 15.6; 4,736 -, 13.0, 13.6, 15.7; 9,472 -, -, 14.1, 16.0.  (h256x3, 4,544: 22.7 with 64 rows, 24.4 with 128.)
     const int rows = std::min(p->n, P.num_tiles * fused::kTile) - P.tile_begin * fused::kTile;
     for (int i = 0; i < 2; i++)
         for (int S = i == 0 ? 4 : 2, tr = p->H == 64 * S ? 32 : 64; tr <= fused::kTile; tr *= 2) {

@@ -30,7 +30,7 @@
 // records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
 // Measured (us a step in a stream, fp16; the persistent kernel, one CTA pair per two tiles -> here): h256x2, 32 envs 20.6 -> 9.5,
-// 256 21.6 -> 9.95, 1,024 21.5 -> 10.5, 2,048 21.7 -> 15.0, 4,000 22.2 -> 17.6, 8,192 22.6 -> 20.2; classic h256x3, 1,024 envs 28.9 -> 14.5, 4,000
+// 256 21.0 -> 10.0, 1,024 21.5 -> 10.5, 2,048 21.7 -> 14.9, 4,000 22.3 -> 17.6, 8,192 22.7 -> 20.1; classic h256x3, 1,024 envs 28.9 -> 14.5, 4,000
 // 29.7 -> 25.3, 8,192 30.2 -> 28.7.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
 #include "cfx_fused_split.h"
 
