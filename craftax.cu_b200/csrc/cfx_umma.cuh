@@ -15,7 +15,8 @@ namespace umma {
 
 // Debug builds (-DCFX_CHECK): the wrappers of barriers on this CTA's side and of asynchronous copies verify the alignment rules
 // of their operands, report a violation with printf and SKIP the operation (the kernel's bounded waits then
-// end it with a status code instead of a fault).
+// end it with a status code instead of a fault; a barrier whose set-up is skipped has no such end, so that check must hold
+// for every CTA: own_barrier).
 #ifdef CFX_CHECK
 #define CFX_CHK(cond, what, a, b)                                                          \
     if (!(cond)) {                                                                         \
@@ -122,8 +123,7 @@ __device__ __forceinline__ void st_global_v8(float* p, const float (&v)[8]) {
     asm volatile("mbarrier.test_wait.parity.shared::cta.b64 " #name ", [%0], %1;" ::   \
                      "r"(bar), "r"(parity) : "memory")
 #define CFX_PROBE_CLEAR(name) asm volatile("setp.ne.u32 " #name ", 0, 0;")
-#define CFX_PROBE_READ(name, out) asm volatile("selp.u32 %0, 1, 0, " #name ";" : "=r"(out) : : "memory")
-// the same for a whole warp: 1 if every lane's probe found the phase complete (see mbar_wait_warp)
+// read by a whole warp: 1 if every lane's probe found the phase complete (see mbar_wait_warp)
 #define CFX_PROBE_READ_ALL(name, out)                                                                                 \
     asm volatile("{\n\t.reg .pred all;\n\tvote.sync.all.pred all, " #name ", 0xffffffff;\n\tselp.u32 %0, 1, 0, all;\n\t}" \
                  : "=r"(out) : : "memory")
