@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "cfx_common.cuh"
 #include "cfx_f32x2.cuh"
@@ -45,47 +46,56 @@ __global__ void k_expand(const uint8_t* __restrict__ rec, float* __restrict__ ou
 // shared-memory reads instead (a cycle per operand register and warp, broadcast or not).  In a layer a lane
 // owns TM envs x 4 units, all three gates, a warp 4 TM envs x 32 units (lane = 8 groups of units x 4
 // groups of envs), and a block is WM x WU such warps.  Activations travel between the kernels in tiles of
-// 32 envs, [n / 32][H][32], and the gate matrices in tiles of 64 (32) units, so that a chunk of k steps is one contiguous
-// piece for the copies and both operands of a k step are contiguous in shared memory; two units at a time go
-// through the packed FMA (`fma.rn.f32x2`, the rounding of fmaf), which leaves issue slots for
-// the operand reads.
+// 32 envs, [n / 32][H][32], and the gate matrices in tiles of 64 (32) units, so that both operands of a k step are
+// contiguous in shared memory; two units at a time go through the packed FMA (`fma.rn.f32x2`, the rounding of fmaf), which leaves
+// issue slots for the operand reads.  (One env and unit at a time: 199 us against 147 at 4,096 envs, hidden 256, depth 2.  Pairs of envs
+// times pairs of units, straight and crossed, which need half as many register moves: 157.)
 // (The doubled input of a pair is made with register moves: stored doubled it costs 8 more operand
-// registers from shared memory a k step, and the layer kernel went from 52 to 59 us at 4,096 envs.)
-template <int TM> struct Frag {   // the TM inputs of a lane, each doubled for the packed FMA
+// registers from shared memory a k step, and the layer kernel went from 52 to 59 us at 4,096 envs.  From tensor memory, as it is or
+// doubled, a loop of nothing but the sums of a layer keeps the FMA pipe 88 and 78 % busy, from shared memory 89 %.)
+// The TM envs of a lane among the 4 TM of its warp: quads of the 16 envs that the four groups g of lanes have together, then
+// a pair of 8, then one of 4, so that a lane's envs are aligned words in shared memory for any TM.
+template <int TM> struct Envs {
+    static constexpr int kQuads = TM / 4, kPair = TM % 4 / 2, kOne = TM % 2, kParts = kQuads + kPair + kOne;
+    static __host__ __device__ constexpr int first(int part) { return part < kQuads ? 4 * part : 4 * kQuads + (part > kQuads ? 2 * kPair : 0); }
+    static __host__ __device__ constexpr int count(int part) { return part < kQuads ? 4 : (part == kQuads && kPair ? 2 : 1); }
+    static __device__ __forceinline__ int at(int part, int g) { return 4 * first(part) + count(part) * g; }   // first env of a part
+};
+// its inputs, each doubled for the packed FMA; x: those of the warp's first env
+template <int TM> struct Frag {
     uint64_t v[TM];
-    __device__ __forceinline__ void load(const float* x) {
-        if constexpr (TM >= 4) {
+    __device__ __forceinline__ void load(const float* x, int g) {
+        using E = Envs<TM>;
 #pragma unroll
-            for (int q = 0; q < TM / 4; q++) {
-                const float4 f = *reinterpret_cast<const float4*>(x + 4 * q);
-                v[4 * q] = f2pack(f.x, f.x); v[4 * q + 1] = f2pack(f.y, f.y);
-                v[4 * q + 2] = f2pack(f.z, f.z); v[4 * q + 3] = f2pack(f.w, f.w);
+        for (int p = 0; p < E::kParts; p++) {
+            const float* q = x + E::at(p, g);
+            uint64_t* d = v + E::first(p);
+            if (E::count(p) == 4) {
+                const float4 f = *reinterpret_cast<const float4*>(q);
+                d[0] = f2pack(f.x, f.x); d[1] = f2pack(f.y, f.y); d[2] = f2pack(f.z, f.z); d[3] = f2pack(f.w, f.w);
+            } else if (E::count(p) == 2) {
+                const float2 f = *reinterpret_cast<const float2*>(q);
+                d[0] = f2pack(f.x, f.x); d[1] = f2pack(f.y, f.y);
+            } else {
+                d[0] = f2pack(q[0], q[0]);
             }
-        } else {
-            v[0] = f2pack(x[0], x[0]);
         }
     }
 };
-// TM consecutive envs of a unit
-template <int TM> __device__ __forceinline__ void load_envs(const float* p, float (&v)[TM]) {
-    if constexpr (TM >= 4) {
-#pragma unroll
-        for (int q = 0; q < TM / 4; q++) {
-            const float4 f = *reinterpret_cast<const float4*>(p + 4 * q);
-            v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
-        }
-    } else {
-        v[0] = p[0];
-    }
+// Four floats by a load that is issued where it stands
+__device__ __forceinline__ void ld_now4(const float* p, float* v) {
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
 }
-template <int TM> __device__ __forceinline__ void store_envs(float* p, const float (&v)[TM]) {
-    if constexpr (TM >= 4) {
-#pragma unroll
-        for (int q = 0; q < TM / 4; q++)
-            *reinterpret_cast<float4*>(p + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-    } else {
-        p[0] = v[0];
-    }
+// N envs side by side of a unit
+template <int N> __device__ __forceinline__ void store_envs(float* p, const float (&v)[4]) {
+    if constexpr (N == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else if constexpr (N == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    else *p = v[0];
+}
+__device__ __forceinline__ void store_envs(float* p, const float (&v)[4], int count) {   // (count is a constant once unrolled)
+    if (count == 4) store_envs<4>(p, v);
+    else if (count == 2) store_envs<2>(p, v);
+    else store_envs<1>(p, v);
 }
 // 16 bytes global -> shared in flight (zeros where `on` is false); a source that is only 4-byte
 // aligned goes as four words
@@ -114,27 +124,32 @@ __host__ __device__ __forceinline__ size_t act_at(size_t e, int k, int H) { retu
 // units, the groups 32 units apart.  Few warps of such tiles fall to an SM scheduler (one at 4,096 envs,
 // hidden 256), so everything but the sums is taken out of them: four warps of a block fill the stages (record words ->
 // fp32, transposed; W_enc rows by asynchronous copies), four multiply, and named barriers hand the
-// stages over.  4,096 envs, hidden 256: 52 us, against 63 us with every warp doing both, and 78 us
-// with the features kept as bytes and converted by the lanes that multiply.  A small batch is bound by the latency of these
+// stages over.  (4,096 envs, hidden 256: 63 us with every warp doing both, and 78 us
+// with the features kept as bytes and converted by the lanes that multiply.)  A small batch is bound by the latency of these
 // loads: record words are fetched three chunks ahead, W_enc rows S - 2 chunks, and the 51 raw floats of the tail are copied
 // at the start by the warps that multiply (32 envs, encoder by itself: 25 us with one chunk ahead, 17 so).
+// What a forward of 4,096 envs, hidden 256, depth 2 gained with 7 envs a lane (on 147 of 148 SMs) instead of 8 (128): 6 us; with two of the
+// multiplying warps side by side along the units, so that a block converts half as many records: 1.7; with the copies of a
+// chunk and its k steps written out: 2.  The fills' work still slows the sums beside them: 82,000 cycles a block, 62,000 in a loop of the sums alone.
 constexpr int kEncK = 32, kEncAhead = 3;
 constexpr int kMapChunks = (kMap + kEncK - 1) / kEncK, kEncChunks = kMapChunks + (kTail + kEncK - 1) / kEncK;   // 25 of record bytes, 2 of the tail
 static_assert(kEncChunks % kEncAhead == 0, "the chunk loop is unrolled by the words in flight");
-template <int TM, int G> struct Enc {
-    static constexpr int BM = 16 * TM, BU = 32 * G, XS = BM + 4;       // envs, units, row stride of x
-    static constexpr int S = TM == 1 ? 6 : (TM == 4 ? 4 : 3);          // stages
-    static constexpr int kStage = kEncK * (XS + BU);                   // floats
+template <int TM, int G, int WU> struct Enc {   // WU of the four warps side by side along the units
+    static constexpr int WM = 4 / WU, BM = 4 * TM * WM, BU = 32 * G * WU;   // envs, units
+    static constexpr int XS = BM + (BM % 8 == 0 ? 4 : 0);               // row stride of x: four rows are 16 banks on
+    static constexpr int S = TM == 1 ? 6 : (G == 1 ? 4 : 3);      // stages
+    static constexpr int kStage = kEncK * (XS + BU);                    // floats
     static constexpr int kSmem = (S * kStage + kTail * XS) * (int)sizeof(float);
+    static_assert(XS % 8 == 4, "no bank conflicts between the words that a warp stores");
 };
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
-template <int TM, int G>
+template <int TM, int G, int WU>
 __global__ void __launch_bounds__(256, 2)
 k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc,
                float* __restrict__ h_out, int n, int H, int w_aligned, int early) {
-    using E = Enc<TM, G>;
+    using E = Enc<TM, G, WU>;
     constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = kEncK, S = E::S, D = S - 2;
     constexpr int FULL = 1, EMPTY = FULL + S, TAIL = 15;   // barrier ids
     extern __shared__ __align__(16) float sm[];   // per stage: x [K][XS], w [K][BU]; then the tail [kTail][XS]
@@ -144,14 +159,16 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
     if (early & kLaunchNext) launch_next_kernel();
     if (warp >= 4) {
         const int tid = threadIdx.x - 128;
-        // rows of W_enc that chunk c needs, and the first of them
+        // the rows of W_enc of chunk c, a piece of 16 bytes a thread at a time
+        constexpr int NW = K * BU / (4 * 128);
+        static_assert(NW * 4 * 128 == K * BU, "whole pieces");
         auto copy_w = [&](int c) {
-            const int f0 = c < kMapChunks ? c * K : kMap + (c - kMapChunks) * K;
-            const int rows = c < kMapChunks ? min(K, kMap - c * K) : min(K, kObs - f0);
+            const int f0 = c < kMapChunks ? c * K : kMap + (c - kMapChunks) * K, end = c < kMapChunks ? kMap : kObs;
             float* w = sm + (c % S) * E::kStage + K * XS;
-            for (int i = tid; i < rows * (BU / 4); i += 128) {
-                const int k = i / (BU / 4), col = 4 * (i % (BU / 4));
-                copy16(w + k * BU + col, W_enc + (size_t)(f0 + k) * H + u0 + col, true, w_aligned != 0);
+#pragma unroll
+            for (int i = 0; i < NW; i++) {
+                const int at = i * 128 + tid, k = at / (BU / 4), col = 4 * (at % (BU / 4));
+                if (f0 + k < end) copy16(w + 4 * at, W_enc + (size_t)(f0 + k) * H + u0 + col, true, w_aligned != 0);
             }
         };
         if (!(early & kWeightsReady)) wait_for_previous_kernel();
@@ -159,11 +176,12 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
         for (int c = 0; c < D; c++) { copy_w(c); copy_commit(); }
         wait_for_previous_kernel();
         // a task is one record word (four features of an env): lanes = 16 envs x 2 words
-        constexpr int TASKS = BM * (K / 4) / 128;
+        constexpr int BM16 = (BM + 15) / 16 * 16, TASKS = BM16 * (K / 4) / 128;
+        static_assert(TASKS * 128 == BM16 * (K / 4), "whole tasks");
         auto slot = [&](int i, int& e, int& w) {
             const int idx = i * 128 + tid;
-            e = idx % 16 + 16 * ((idx / 32) % (BM / 16));
-            w = (idx % 32) / 16 + 2 * (idx / (2 * BM));
+            e = idx % 16 + 16 * ((idx / 32) % (BM16 / 16));
+            w = (idx % 32) / 16 + 2 * (idx / (2 * BM16));
         };
         uint32_t raw[kEncAhead][TASKS];
         auto fetch = [&](int c, uint32_t (&r)[TASKS]) {
@@ -172,7 +190,7 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
                 int e, w;
                 slot(i, e, w);
                 const int f = c * K + 4 * w;   // (792 is a multiple of 4)
-                r[i] = f < kMap && e0 + e < n ? *reinterpret_cast<const uint32_t*>(rec + (size_t)(e0 + e) * kRec + f) : 0u;
+                r[i] = f < kMap && e < BM && e0 + e < n ? *reinterpret_cast<const uint32_t*>(rec + (size_t)(e0 + e) * kRec + f) : 0u;
             }
         };
 #pragma unroll
@@ -192,6 +210,7 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
                     for (int i = 0; i < TASKS; i++) {
                         int e, wd;
                         slot(i, e, wd);
+                        if (BM16 != BM && e >= BM) continue;
 #pragma unroll
                         for (int b = 0; b < 4; b++) x[(4 * wd + b) * XS + e] = (float)((raw[q][i] >> (8 * b)) & 0xFFu);
                     }
@@ -211,7 +230,7 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
                      "l"(rec + (size_t)(on ? e0 + e : e0) * kRec + kMap + 4 * j), "r"(on ? 4 : 0) : "memory");
     }
     copy_commit();
-    const int el = warp * 4 * TM + (lane >> 3) * TM, ul = (lane & 7) * 4;
+    const int el = warp % E::WM * 4 * TM, ul = warp / E::WM * 32 * G + (lane & 7) * 4, lg = lane >> 3;   // the warp's first env
     uint64_t z[G][TM][2];
 #pragma unroll
     for (int g = 0; g < G; g++) {
@@ -221,7 +240,7 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
     }
     auto step = [&](const float* xp, const float* wp) {
         Frag<TM> x;
-        x.load(xp);
+        x.load(xp, lg);
 #pragma unroll
         for (int g = 0; g < G; g++) {
             const float4 w = *reinterpret_cast<const float4*>(wp + 32 * g);
@@ -244,7 +263,7 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
         const int rows = c < kMapChunks ? min(K, kMap - c * K) : min(K, kTail - (c - kMapChunks) * K);
         bar_sync(FULL + s, 256);
         if (rows == K) {
-#pragma unroll 16
+#pragma unroll
             for (int k = 0; k < K; k++) step(xp + k * XS, wp + k * BU);
         } else {
             int k = 0;
@@ -255,18 +274,22 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
         }
         if (c + S < kEncChunks) bar_arrive(EMPTY + s, 256);
     }
-    if (e0 + el < n) {
+#pragma unroll
+    for (int p = 0; p < Envs<TM>::kParts; p++) {
+        const int env = e0 + el + Envs<TM>::at(p, lg);
+        if (env >= n) continue;
 #pragma unroll
         for (int i = 0; i < 4 * G; i++) {
             const int g = i >> 2, u = i & 3;
-            float h[TM];
+            float h[4];
 #pragma unroll
-            for (int e = 0; e < TM; e++) {
+            for (int e = 0; e < 4; e++) {
+                if (e >= Envs<TM>::count(p)) break;
                 float lo, hi;
-                f2unpack(z[g][e][u >> 1], lo, hi);
+                f2unpack(z[g][Envs<TM>::first(p) + e][u >> 1], lo, hi);
                 h[e] = (u & 1) ? hi : lo;
             }
-            store_envs<TM>(h_out + act_at(e0 + el, u0 + ul + 32 * g + u, H), h);
+            store_envs(h_out + act_at(env, u0 + ul + 32 * g + u, H), h, Envs<TM>::count(p));
         }
     }
 }
@@ -347,78 +370,109 @@ __global__ void k_done_to_terminals(const int8_t* __restrict__ done, float* __re
 // Wt is the layer's gate matrix as k_transpose_gates lays it out, x_in and h_out activations.  K chunks of 32; ST buffers:
 // two where several blocks share an SM, more for small batches, which wait for the loads (chunks of 16 with three: 155 against
 // 152 us a forward at 4,096 envs, 970 against 944 us at 8,192 envs with hidden 512, depth 3); the k loop has to be unrolled
-// well (by 4: 170 us).  Bound by the FMA pipe: busy 80 % of the time at hidden 512; one thread per unit with 16 envs, before, 20 %.
-__device__ __forceinline__ float sigmoid_ref(float x) { return 1.0f / (1.0f + expf(-x)); }
-__device__ __forceinline__ float mingru_g_ref(float x) { return x >= 0.0f ? x + 0.5f : sigmoid_ref(x); }
+// well (by 4: 170 us), but not whole (8,192 envs, hidden 512: 2 % slower).  Bound by the FMA pipe.  Two blocks an SM, so that blocks of five envs
+// a lane and more keep everything in registers (three: 160 bytes of spills, 142 against 136 us at 4,096 envs).  us a forward, before the cell's loads and
+// divisions were taken out of their chains and the heights followed the number of blocks, and now: 4,096 envs, hidden 256, depth 2 146.9 and 123.7;
+// 5,120 222.1 and 153.9; 1,024 66.1 and 58.8; 8,192 envs, hidden 512, depth 3 887 and 827.
+// N values 1 / (1 + exp(-z)) at once.  The compiler's correctly rounded division has a branch, so sigmoids written one by one run
+// one after the other, about 150 cycles each: the 96 of a lane took half as long as a lone block's sums at hidden 256.
+// Here the reciprocals are refined without a branch, by a Newton step with the remainder in one FMA (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): the same bits as 1.0f / d for each of the
+// 1.06e9 values d in [1, 2^126].  Beyond, the batch is divided.
+// (n is a constant once unrolled)
+template <int N> __device__ __forceinline__ void sigmoids_ref(float (&z)[N], int n) {
+    float d[N], most = 1.0f;
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (i < n) d[i] = 1.0f + expf(-z[i]);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        if (i >= n) break;
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d[i]));
+        z[i] = fmaf(r, fmaf(-d[i], r, 1.0f), r);
+        most = fmaxf(most, d[i]);
+    }
+    if (most > 0x1p126f)
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if (i < n) z[i] = 1.0f / d[i];
+}
 
 constexpr int kGruK = 32;
 template <int TM, int WM, int WU> constexpr int gru_stage_floats() { return kGruK * (4 * TM * WM + 3 * 32 * WU); }
 
 template <int TM, int WM, int WU, int ST>
-__global__ void __launch_bounds__(32 * WM * WU, 3)
+__global__ void __launch_bounds__(32 * WM * WU, TM > 4 ? 2 : 3)
 k_mingru_fp32(const float* x_in, const float* __restrict__ Wt, float* __restrict__ state,
               const float* prev_terminals, float* __restrict__ h_out, float* __restrict__ r_state,
               int r_bf16, int n, int H, int s_aligned, int early) {
     constexpr int T = 32 * WM * WU, BM = 4 * TM * WM, BU = 32 * WU, kStage = gru_stage_floats<TM, WM, WU>();
-    constexpr int EB = BM < 32 ? BM : 32;         // envs of an activation tile that a block takes
-    extern __shared__ __align__(16) float sm[];   // per stage: x [BM / EB][kGruK][EB], w [kGruK][3][BU]
+    using E = Envs<TM>;
+    extern __shared__ __align__(16) float sm[];   // per stage: x [kGruK][BM], w [kGruK][3][BU]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int e0 = blockIdx.x * BM, u0 = blockIdx.y * BU;
-    const int el = (warp % WM) * 4 * TM + (lane >> 3) * TM, ul = (warp / WM) * 32 + (lane & 7) * 4;
-    const bool live = e0 + el < n;
+    const int el = (warp % WM) * 4 * TM, ul = (warp / WM) * 32 + (lane & 7) * 4, lg = lane >> 3;   // the warp's first env
     const float* wsrc = Wt + (size_t)u0 * 3 * H;
-    auto copy_w = [&](int c) {
-        float* w = sm + (c % ST) * kStage + kGruK * BM;
-        const float* src = wsrc + (size_t)c * kGruK * 3 * BU;
-#pragma unroll 4
-        for (int i = 4 * tid; i < kGruK * 3 * BU; i += 4 * T) copy16(w + i, src + i, true, true);
+    // the copies of a chunk, in pieces of 16 bytes a thread
+    constexpr int NW = kGruK * 3 * BU / (4 * T), NX = (kGruK * (BM / 4) + T - 1) / T;
+    static_assert(NW * 4 * T == kGruK * 3 * BU, "whole pieces");
+    auto copy_w = [&](int c, int i) {
+        const int at = 4 * (i * T + tid);
+        copy16(sm + (c % ST) * kStage + kGruK * BM + at, wsrc + (size_t)c * kGruK * 3 * BU + at, true, true);
     };
-    auto copy_x = [&](int c) {
-        float* x = sm + (c % ST) * kStage;
-#pragma unroll
-        for (int t = 0; t < BM / EB; t++) {
-            const bool on = e0 + t * EB < n;
-            const float* src = x_in + act_at(on ? e0 + t * EB : e0, c * kGruK, H);
-            for (int i = tid; i < kGruK * (EB / 4); i += T)
-                copy16(x + t * kGruK * EB + 4 * i, src + (i / (EB / 4)) * 32 + 4 * (i % (EB / 4)), on, true);
-        }
+    auto copy_x = [&](int c, int i) {
+        const int at = i * T + tid;
+        if (NX * T != kGruK * (BM / 4) && at >= kGruK * (BM / 4)) return;
+        const int k = at / (BM / 4), env = e0 + 4 * (at % (BM / 4));
+        const bool on = env < n;   // (n is a multiple of 32)
+        copy16(sm + (c % ST) * kStage + 4 * at, x_in + act_at(on ? env : e0, c * kGruK + k, H), on, true);
     };
     if (early & kLaunchNext) launch_next_kernel();
     const int chunks = H / kGruK;
     if (!(early & kWeightsReady)) wait_for_previous_kernel();
 #pragma unroll
     for (int c = 0; c < ST - 1; c++)
-        if (c < chunks) copy_w(c);
+        if (c < chunks)
+#pragma unroll
+            for (int i = 0; i < NW; i++) copy_w(c, i);
     wait_for_previous_kernel();
 #pragma unroll
     for (int c = 0; c < ST - 1; c++) {
-        if (c < chunks) copy_x(c);
+        if (c < chunks)
+#pragma unroll
+            for (int i = 0; i < NX; i++) copy_x(c, i);
         copy_commit();
     }
-    if (live)   // this lane's states, on their way to L2 while the sums run
 #pragma unroll
-        for (int e = 0; e < TM; e++)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(state + (size_t)(e0 + el + e) * H + u0 + ul));
+    for (int p = 0; p < E::kParts; p++) {   // this lane's states, on their way to L2 while the sums run
+        const int env = e0 + el + E::at(p, lg);
+        if (env < n)
+#pragma unroll
+            for (int e = 0; e < E::count(p); e++)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(state + (size_t)(env + e) * H + u0 + ul));
+    }
     uint64_t z[3][TM][2];
 #pragma unroll
     for (int g = 0; g < 3; g++)
 #pragma unroll
         for (int e = 0; e < TM; e++) z[g][e][0] = z[g][e][1] = 0ull;
-    const float* xl = sm + (el / EB) * kGruK * EB + el % EB;
     for (int c = 0; c < chunks; c++) {
         copy_wait<ST - 2>();
         __syncthreads();   // chunk c is complete, and everybody is done with chunk c - 1
         if (c + ST - 1 < chunks) {
-            copy_w(c + ST - 1);
-            copy_x(c + ST - 1);
+#pragma unroll
+            for (int i = 0; i < NW; i++) copy_w(c + ST - 1, i);
+#pragma unroll
+            for (int i = 0; i < NX; i++) copy_x(c + ST - 1, i);
         }
         copy_commit();
-        const float* x = xl + (c % ST) * kStage;
+        const float* x = sm + (c % ST) * kStage + el;
         const float* w = sm + (c % ST) * kStage + kGruK * BM + ul;
 #pragma unroll 16
         for (int k = 0; k < kGruK; k++) {
             Frag<TM> xv;
-            xv.load(x + k * EB);
+            xv.load(x + k * BM, lg);
 #pragma unroll
             for (int g = 0; g < 3; g++) {
                 const float4 wv = *reinterpret_cast<const float4*>(w + (k * 3 + g) * BU);
@@ -431,63 +485,87 @@ k_mingru_fp32(const float* x_in, const float* __restrict__ Wt, float* __restrict
             }
         }
     }
-    if (!live) return;
-    // this lane's TM x 4 states and terminal flags
-    float st[TM][4];
+    // The cell, a part of the lane's envs at a time: their states, flags and the inputs of the lane's units are loaded before anything is
+    // done with them, those of the next part when half of the accumulators of this one are used up.
+    float st[2][4][4], x[2][4][4], ended[2][4];
+    auto fetch = [&](int p) {
+        const int b = p & 1, env = e0 + el + E::at(p, lg);
+        if (env >= n) return;
 #pragma unroll
-    for (int e = 0; e < TM; e++) {
-        const size_t o = (size_t)(e0 + el + e) * H + u0 + ul;
-        st[e][0] = st[e][1] = st[e][2] = st[e][3] = 0.0f;
-        if (!(prev_terminals != nullptr && prev_terminals[e0 + el + e] != 0.0f)) {
-            if (s_aligned) {
-                const float4 f = *reinterpret_cast<const float4*>(state + o);
-                st[e][0] = f.x; st[e][1] = f.y; st[e][2] = f.z; st[e][3] = f.w;
-            } else {
+        for (int e = 0; e < 4; e++) {
+            if (e >= E::count(p)) break;
+            const float* src = state + (size_t)(env + e) * H + u0 + ul;
+            if (s_aligned) ld_now4(src, st[b][e]);
+            else
 #pragma unroll
-                for (int u = 0; u < 4; u++) st[e][u] = state[o + u];
+                for (int u = 0; u < 4; u++) st[b][e][u] = src[u];
+            ended[b][e] = prev_terminals != nullptr ? prev_terminals[env + e] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float* src = x_in + act_at(env, u0 + ul + u, H);
+            if (E::count(p) == 4) ld_now4(src, x[b][u]);
+            else
+#pragma unroll
+                for (int e = 0; e < E::count(p); e++) x[b][u][e] = src[e];
+        }
+    };
+    fetch(0);
+#pragma unroll
+    for (int p = 0; p < E::kParts; p++) {
+        const int b = p & 1, env = e0 + el + E::at(p, lg), count = E::count(p);
+        if (env >= n) {
+            if (p + 1 < E::kParts) fetch(p + 1);
+            continue;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (e < count && ended[b][e] != 0.0f) st[b][e][0] = st[b][e][1] = st[b][e][2] = st[b][e][3] = 0.0f;
+        if (r_state != nullptr) {   // the post-zero state inputs
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                if (e >= count) break;
+                const size_t o = (size_t)(env + e) * H + u0 + ul;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o + u] = __float2bfloat16(st[b][e][u]);
+                    else r_state[o + u] = st[b][e][u];
+                }
             }
         }
-    }
-    if (r_state != nullptr) {   // the post-zero state inputs
 #pragma unroll
-        for (int e = 0; e < TM; e++) {
-            const size_t o = (size_t)(e0 + el + e) * H + u0 + ul;
+        for (int u = 0; u < 4; u++) {
+            if (u == 2 && p + 1 < E::kParts) fetch(p + 1);
+            float h[4], zh[4], s[12];   // s: sigmoids of zh, zg, zp
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o + u] = __float2bfloat16(st[e][u]);
-                else r_state[o + u] = st[e][u];
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+                for (int g = 0; g < 3; g++) {
+                    if (e >= count) break;
+                    float lo, hi;
+                    f2unpack(z[g][E::first(p) + e][u >> 1], lo, hi);
+                    s[3 * e + g] = (u & 1) ? hi : lo;
+                    if (g == 0) zh[e] = s[3 * e];
+                }
+            sigmoids_ref(s, 3 * count);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                if (e >= count) break;
+                const float gh = zh[e] >= 0.0f ? zh[e] + 0.5f : s[3 * e], p = s[3 * e + 2];
+                const float out = st[b][e][u] + s[3 * e + 1] * (gh - st[b][e][u]);
+                h[e] = p * out + (1.0f - p) * x[b][u][e];
+                st[b][e][u] = out;
             }
+            store_envs(h_out + act_at(env, u0 + ul + u, H), h, count);
         }
-    }
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-        float x[TM], h[TM];
-        load_envs<TM>(x_in + act_at(e0 + el, u0 + ul + u, H), x);
+        for (int e = 0; e < 4; e++) {
+            if (e >= count) break;
+            float* dst = state + (size_t)(env + e) * H + u0 + ul;
+            if (s_aligned) *reinterpret_cast<float4*>(dst) = make_float4(st[b][e][0], st[b][e][1], st[b][e][2], st[b][e][3]);
+            else
 #pragma unroll
-        for (int e = 0; e < TM; e++) {
-            float lo, hi;
-            f2unpack(z[0][e][u >> 1], lo, hi);
-            const float zh = (u & 1) ? hi : lo;
-            f2unpack(z[1][e][u >> 1], lo, hi);
-            const float zg = (u & 1) ? hi : lo;
-            f2unpack(z[2][e][u >> 1], lo, hi);
-            const float zp = (u & 1) ? hi : lo;
-            const float s = st[e][u];
-            const float out = s + sigmoid_ref(zg) * (mingru_g_ref(zh) - s);
-            const float p = sigmoid_ref(zp);
-            h[e] = p * out + (1.0f - p) * x[e];
-            st[e][u] = out;
-        }
-        store_envs<TM>(h_out + act_at(e0 + el, u0 + ul + u, H), h);
-    }
-#pragma unroll
-    for (int e = 0; e < TM; e++) {
-        const size_t o = (size_t)(e0 + el + e) * H + u0 + ul;
-        if (s_aligned) {
-            *reinterpret_cast<float4*>(state + o) = make_float4(st[e][0], st[e][1], st[e][2], st[e][3]);
-        } else {
-#pragma unroll
-            for (int u = 0; u < 4; u++) state[o + u] = st[e][u];
+                for (int u = 0; u < 4; u++) dst[u] = st[b][e][u];
         }
     }
 }
@@ -769,21 +847,53 @@ int launch_init_uniform(float* w, int count, float bound, uint64_t seed, int sub
     return CFX_OK;
 }
 
-// Tiles by the number q of warps that 8 envs x 4 units a lane would give (the GPU has 592 SM schedulers).
-// A layer takes 8 envs a lane from q = 1,024 (4,096 envs at hidden 256: 152 us a forward, 154 with 4; at 3,072 envs
-// 152 against 134), 4 below, and 1 under 96, where even the 4-env tiles leave schedulers without a warp
-// (256 envs: 55 against 71 us; 512 envs: 77 against 72).
-static int strict_tile(long long q) { return q >= 1024 ? 8 : (q >= 96 ? 4 : 1); }
-// The encoder has a third of a layer's units: envs x groups of 4 units a lane, 1 x 1, 4 x 1, 4 x 2 and 8 x 2 (2,048 envs
-// at hidden 256, q = 512: 102, 97 and 113 us a forward with the last three; 1,024 envs: 73, 80 and 94).
-static int strict_encoder_tile(long long q) { return q >= 640 ? 82 : (q >= 400 ? 42 : (q >= 96 ? 41 : 11)); }
+// The tiles.  What a forward costs is the number of blocks that the fullest SM has one after the other, so the envs of a lane, TM, are
+// those for which that number times the time of a block is the least; both are estimated from what blocks of each height take
+// alone and two to an SM.  (Before, 8 envs a lane from q = n H / 1024 = 1,024 warps on, else 4: at 4,096 envs and hidden 256 that left 40
+// SMs with half of the others' layers, and 24 with three times at 5,120.  The times of all heights were measured at 26 sizes from 512 envs
+// to 16,384, hidden 64 to 512: this choice is the best at all of them in the encoder, and within 1 % of it in the layers.)
+constexpr int kSMs = 148;
+static int sm_rounds(int n, int envs, int unit_tiles) { return ((n + envs - 1) / envs * unit_tiles + kSMs - 1) / kSMs; }
+// A layer.  1 env a lane under q = 96, where even tiles of 4 leave schedulers without a warp (256 envs: 55 against 71 us;
+// 512 envs: 77 against 72).  Blocks of 4 envs a lane take the same time alone and beside each other, those of more envs a little less beside one.
+// Narrow layers have as much to do around the sums as in them, and stay with 4 longer (4,096 envs, hidden 128: 52.9 us, 54.3 with 7; 8,192 78.5
+// and 77.5).
+static int strict_tile(int n, int H) {
+    const long long q = (long long)n * H / 1024;
+    if (q < 96) return 1;
+    if (H % 64 != 0) return q >= 1024 ? 8 : 4;
+    if (H < 256 && q < 1024) return 4;
+    constexpr float kAlone[10] = {0, 0, 0, 0, 5.4f, 7.4f, 8.1f, 10.0f, 10.7f, 12.5f};
+    int best = 0;
+    float least = 0.0f;
+    for (int tm = 4; tm <= 9; tm++) {
+        const int b = sm_rounds(n, 8 * tm, H / 64);
+        const float cost = kAlone[tm] * (tm == 4 ? (float)b : 1.83f * (b / 2) + b % 2);
+        if (best == 0 || cost < least) { best = tm; least = cost; }
+    }
+    return best;
+}
+// The encoder: TM envs x 8 units a lane, where a block takes TM + 2 units of time; 4 envs x 4 units as long as every block has an SM of its
+// own (hidden 256: 1,024 envs 45.8 us with the forward of one layer, 55.3 with 8 units a lane; 1,536 envs 67.4 and 63.6), 1 env x 4 units
+// under q = 96.
+struct EncoderTile { int tm, g; };
+static EncoderTile strict_encoder_tile(int n, int H) {
+    const long long q = (long long)n * H / 1024;
+    if (q < 96) return {1, 1};
+    if (H % 64 != 0 || sm_rounds(n, 64, H / 32) == 1) return {4, 1};
+    const int wu = H % 128 == 0 ? 2 : 1;
+    int best = 4;
+    for (int tm = 5; tm <= 9; tm++)
+        if (sm_rounds(n, 16 * tm / wu, H / (64 * wu)) * (tm + 2) < sm_rounds(n, 16 * best / wu, H / (64 * wu)) * (best + 2)) best = tm;
+    return {best, 2};
+}
 
-template <int TM, int G>
+template <int TM, int G, int WU>
 static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, int early, cudaStream_t st) {
-    using E = Enc<TM, G>;
-    int rc = allow_smem<k_encoder_fp32<TM, G>, E::kSmem>();
+    using E = Enc<TM, G, WU>;
+    int rc = allow_smem<k_encoder_fp32<TM, G, WU>, E::kSmem>();
     if (rc) return rc;
-    return launch_chained(k_encoder_fp32<TM, G>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
+    return launch_chained(k_encoder_fp32<TM, G, WU>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
                           a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], a.n, a.H,
                           ((uintptr_t)(a.params + o.w_enc) & 15) == 0, early);
 }
@@ -809,33 +919,43 @@ static int strict_layers(const StrictArgs& a, int early, cudaStream_t st) {
     return CFX_OK;
 }
 
+template <int N> using Int = std::integral_constant<int, N>;
 // Full strict forward.  scratch_h: two buffers of n H activations; logits_av [n][A+1].
 int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     const int H = a.H, L = a.L, A = a.A, n = a.n;
     const ArenaLayout o = ArenaLayout::make(H, L, A, a.game == CFX_GAME_CLASSIC ? kClassicObs : kObs);
     int rc;
     const long long q = (long long)n * H / 1024;
-    const int tm = strict_tile(q), te = strict_encoder_tile(q);
+    const int tm = strict_tile(n, H);
+    const EncoderTile te = strict_encoder_tile(n, H);
     // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own
     // (512 envs, 64 blocks a layer: 88 us with it, 72 without)
-    const long long blocks = (te == 11 ? 2 * q : q / 2) + L * (tm == 1 ? 2 * q : q / 2) + n / 16;
+    const long long blocks = (te.tm == 1 ? 2 * q : q / 2) + L * (tm == 1 ? 2 * q : q / 2) + n / 16;
     const int early = (a.game == CFX_GAME_FULL && blocks <= 148 ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
     if (a.game == CFX_GAME_CLASSIC) {
         rc = launch_chained(k_classic_encoder_fp32, dim3(n), H, 0, st, a.records, a.params + o.w_enc, a.params + o.b_enc,
                             a.scratch_h[0], n, H);
     } else {
-        if (te == 11) rc = strict_encoder<1, 1>(a, o, early, st);
-        else if (te == 41 || H % 64 != 0) rc = strict_encoder<4, 1>(a, o, early, st);
-        else rc = te == 42 ? strict_encoder<4, 2>(a, o, early, st) : strict_encoder<8, 2>(a, o, early, st);
+        // (two warps side by side along the units, where there are 128: half of the conversions are other warps' too)
+        auto encode = [&](auto tile) {
+            constexpr int TM = decltype(tile)::value;
+            return H % 128 == 0 ? strict_encoder<TM, 2, 2>(a, o, early, st) : strict_encoder<TM, 2, 1>(a, o, early, st);
+        };
+        if (te.tm == 1) rc = strict_encoder<1, 1, 1>(a, o, early, st);
+        else if (te.g == 1) rc = strict_encoder<4, 1, 1>(a, o, early, st);
+        else rc = te.tm == 4 ? encode(Int<4>()) : te.tm == 5 ? encode(Int<5>()) : te.tm == 6 ? encode(Int<6>())
+                  : te.tm == 7 ? encode(Int<7>()) : te.tm == 8 ? encode(Int<8>()) : encode(Int<9>());
     }
     if (rc) return rc;
     // a hidden size that is an odd multiple of 32 has the warps of a block side by side along the envs
-    if (H % 64 == 0)
-        rc = tm == 8 ? strict_layers<8, 2, 2, 2>(a, early, st) : tm == 1 ? strict_layers<1, 2, 2, 4>(a, early, st)
-             : q <= 592 ? strict_layers<4, 2, 2, 3>(a, early, st) : strict_layers<4, 2, 2, 2>(a, early, st);
-    else
+    if (H % 64 != 0)
         rc = tm == 8 ? strict_layers<8, 4, 1, 2>(a, early, st) : tm == 4 ? strict_layers<4, 4, 1, 2>(a, early, st)
-                                                                 : strict_layers<1, 4, 1, 4>(a, early, st);
+                                                                         : strict_layers<1, 4, 1, 4>(a, early, st);
+    else if (tm == 1) rc = strict_layers<1, 2, 2, 4>(a, early, st);
+    else if (tm == 4) rc = q <= 592 ? strict_layers<4, 2, 2, 3>(a, early, st) : strict_layers<4, 2, 2, 2>(a, early, st);
+    else rc = tm == 5 ? strict_layers<5, 2, 2, 2>(a, early, st) : tm == 6 ? strict_layers<6, 2, 2, 2>(a, early, st)
+              : tm == 7 ? strict_layers<7, 2, 2, 2>(a, early, st) : tm == 8 ? strict_layers<8, 2, 2, 2>(a, early, st)
+                                                                         : strict_layers<9, 2, 2, 2>(a, early, st);
     if (rc) return rc;
     const size_t hsmem = head_smem(H, A);
     if ((rc = allow_smem<k_heads_fp32, (int)head_smem(kMaxHidden, kMaxActions)>())) return rc;

@@ -64,3 +64,29 @@ def test_static_forward_takes_arrays_of_any_word_alignment(cfx, gpu, oracle):
     lav = oracle.forward(params, rec, prev_t, st, H, L, A)
     _close(d_lav.download(), lav)
     _close(d_st.download()[1:].reshape(st.shape), st)
+
+
+@pytest.mark.parametrize("n,H,L", [(1248, 256, 1), (1568, 256, 1), (2048, 256, 2), (2272, 256, 1), (2528, 256, 1),   # layers 5 to 9
+                                   (1248, 512, 1), (1504, 512, 1), (1760, 512, 1), (2272, 512, 1), (2528, 512, 1),   # encoder 5 to 9
+                                   (3872, 192, 1), (5408, 192, 1)])   # encoder 5 and 7, its warps along the envs
+def test_strict_heights_match_the_oracle(cfx, gpu, oracle, n, H, L):
+    """Heights that are no multiple of four envs a lane, and batches that end inside a block."""
+    test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L)
+
+
+@pytest.mark.parametrize("n,H", [(32, 32), (416, 256), (1248, 256)])
+def test_strict_saturated_gates(cfx, gpu, oracle, n, H):
+    """Pre-activations up to some thousands: 1 + exp(-z) overflows, where the quotients are 0."""
+    rec, params, state, prev_t, u = _inputs(oracle, n, H, 1)
+    gates = slice(844 * H, 844 * H + 3 * H * H)
+    params[gates] *= 200.0
+    pol = cfx.Policy(n, H, 1, A, "fp32")
+    pol.set_weights(params)
+    pol.set_state(state)
+    d = pol.forward_host(rec, prev_t, u)
+    st = state.copy()
+    lav = oracle.forward(params, rec, prev_t, st, H, 1, A)
+    assert np.isfinite(lav).all() and np.abs(st).max() > 200
+    _close(d["logits_av"], lav)
+    _close(pol.get_state(), st)
+    pol.close()
