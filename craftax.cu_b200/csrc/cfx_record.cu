@@ -4,21 +4,23 @@
 // The reference gives every env a warp and lets lane 0 walk the mob slots and compute the 51
 // tail scalars; every one of its ~110 scalar loads then fetches 4 bytes of a sector on its own,
 // one after the other.  Here a block of eight warps owns 32 consecutive envs:
-//   1. the view of an env is 9 rows of 11 bytes in each of three map planes, a row in at most two 16-byte pieces.  A lane
-//      takes a row of a plane, and every warp starts asynchronous copies of its four envs' pieces to shared
-//      memory, all in flight;
-//   2. meanwhile, lane per env: the ~50 SoA fields and the 14 mob slots of the player's level are loaded
-//      by lane e for env e, so that a warp's loads of a field are one 128-byte line, each warp an eighth
-//      of them, all of a lane's in flight; they leave the 51 tail floats and the mobs (an earlier
-//      slot of a class that a later slot covers is dropped) in shared memory;
-//   3. warp per env: a lane makes four cells of a view row from the pieces in registers, the four records
-//      are put together where the pieces were, and go out as one bulk copy (1,992 blocks of 16 bytes a
+//   1. lane per env: position, level and flag; then, all of a lane's in flight, the ~50 SoA fields and the 14 mob slots of
+//      the player's level, lane e for env e, so that a warp's loads of a field are one 128-byte line, each warp an eighth of
+//      them (Gather);
+//   2. under these loads, the copies of the views to shared memory: in each of three map planes 9 rows of 11 bytes, 48 bytes apart.
+//      A warp copies the 395 bytes from first to last row of a plane side by side, an instruction a plane and env, for its four envs;
+//      then the fields become the 51 tail floats, and the mobs (an earlier slot of a class that a later slot covers is dropped) go
+//      to shared memory;
+//   3. warp per env: a lane makes four cells of a view row from the spans in registers, the four records
+//      are put together where the spans were, and go out as one bulk copy (1,992 blocks of 16 bytes a
 //      block) or, where an env is skipped, as coalesced words.
-// Before: a byte load per cell and map, two half-used store instructions per 32 cells, the fields one DRAM
-// latency after the other (see ld_now), a read of the light map per mob behind them.  65,536 envs with 62 KB of maps
-// each: 54.7 us; whole 410-byte spans of the planes copied, three a warp and env, 49.5; pieces of rows 46.6 (16,384 envs: 24.9
-// -> 14.9 us with spans).  About 180 MB of DRAM traffic, 3.9 TB/s: bound by the scattered pieces, the time adds up over
-// writes, map rows and fields, and five blocks an SM instead of four take 48.4 us.
+// 65,536 envs with 62 KB of maps each, about 180 MB of DRAM traffic (us, by itself; with the list of 250 reset envs behind it):
+// copies behind the position, then the fields and the two mob classes of a warp one latency after the other 46.4 and 52.9; all loads that
+// wait for nothing in front of the copies 42.5 and 49.1; the copies by rows (27 lanes with a row each, at most two pieces
+// of it) replaced by whole spans 41.8 and 48.0; the fields in front of what depends on the level, and not behind, 39.9 and 46.2, 4.5 TB/s.
+// A block took 25,000 cycles, a third of them memory latencies one behind the other; in 17,000 they still are.  Five blocks an SM (48
+// registers; copies by rows): 41.6 and 48.2, and 4 % slower up to 8,192 envs.  The next kernel's start under this one, early or
+// late in a block: 49.4 to 50.4 instead of 49.1.
 // The bytes are the reference's: the same predicates, the same "last slot of a class wins a
 // cell" order, the same float expressions (sqrtf(x) * 0.1f, x * 0.1f, x * 0.5f, x * 0.25f; no
 // fused multiply-add can form).
@@ -48,8 +50,9 @@ struct Params {
     const int* count_dev;
     int n;
 };
-constexpr int kPlanes = 3, kRowSpan = 32;                // a view row: 11 bytes, so of at most two 16-byte pieces of a map row
-constexpr int kSpan = kRows * kRowSpan;                  // of a plane
+// The view in a plane: nine rows of eleven bytes, 48 apart, so 395 bytes from the first to the last, in 26 pieces of 16
+constexpr int kPlanes = 3, kSpan = kRows * kMapSize, kPieces = 26;
+static_assert(15 + (kRows - 1) * kMapSize + kCols <= 16 * kPieces && 16 * kPieces <= kSpan && kPieces <= 32, "a lane a piece");
 constexpr int kWarps = kBlockThreads / 32, kOwn = kBlockEnvs / kWarps;   // envs whose records a warp writes
 constexpr int kPlaneBytes = kMapSize * kMapSize, kRecWords = kRec / 4, kMapWords = kMap / 4;
 struct Gathered {
@@ -57,11 +60,11 @@ struct Gathered {
     uint32_t mobs[kBlockEnvs][kMobs];
 };
 struct Shared : Gathered {
-    // per warp its four records as they go out, and before that, until they are in registers, the rows of its four
+    // per warp its four records as they go out, and before that, until they are in registers, the spans of its four
     // envs' views (light, block, item)
-    __align__(16) uint8_t span[kWarps][kOwn * kRec];
+    __align__(16) uint8_t span[kWarps][kOwn * kPlanes * kSpan];
 };
-static_assert(kOwn * kRec % 16 == 0 && kRec >= kPlanes * kSpan, "a warp's records are whole 16-byte words");
+static_assert(kOwn * kRec % 16 == 0 && kRec <= kPlanes * kSpan && kSpan % 16 == 0, "a warp's records are whole 16-byte words");
 
 // craftax_wg_jax_index (:1963-1975): negative indices wrap once, then clamp
 __device__ __forceinline__ int jax_index(int i, int size) {
@@ -110,126 +113,148 @@ __device__ __forceinline__ bool same_cell(uint32_t a, uint32_t b) {
     return (a & b & 0x80000000u) && ((a ^ b) & 0xFF00u) == 0;
 }
 
-// the slots of mob class C; true if one of them is alive
-template <int C>
-__device__ __forceinline__ bool gather_mobs(const cfx_env_view& V, int e, int mob_level, int top, int left, uint32_t* mobs) {
-    constexpr int kN = C == 2 ? 2 : kSlots;   // slot 2 of class 2 is never used
-    const int n = V.num_envs;
-    int32_t type[kN], row[kN], col[kN];
+// The kN slots of a mob class c on a level: which are alive, then what and where those are, then the slots as they go into the record
+template <int kN> struct Mobs {
     uint8_t on[kN];
+    int32_t type[kN], row[kN], col[kN];
+    __device__ __forceinline__ void load_alive(const cfx_env_view& V, int e, int c, int mob_level) {
 #pragma unroll
-    for (int i = 0; i < kN; i++) on[i] = soa(V.mob_mask, mob_index(C, mob_level, i), n, e);
-    // the rest of a slot only where a mob is alive: an env on another level than its neighbours reads a
-    // 64-byte burst for every word
+        for (int i = 0; i < kN; i++) on[i] = soa(V.mob_mask, mob_index(c, mob_level, i), V.num_envs, e);
+    }
+    // only where a mob is alive: an env on another level than its neighbours reads a 64-byte burst for every word
+    __device__ __forceinline__ void load_slots(const cfx_env_view& V, int e, int c, int mob_level) {
 #pragma unroll
-    for (int i = 0; i < kN; i++) {
-        const int idx = mob_index(C, mob_level, i);
-        type[i] = row[i] = col[i] = -1;
-        if (on[i] != 0) {
-            type[i] = soa(V.mob_type_id, idx, n, e);
-            row[i] = soa(V.mob_position, idx * 2, n, e);
-            col[i] = soa(V.mob_position, idx * 2 + 1, n, e);
+        for (int i = 0; i < kN; i++) {
+            const int idx = mob_index(c, mob_level, i);
+            type[i] = row[i] = col[i] = -1;
+            if (on[i] != 0) {
+                type[i] = soa(V.mob_type_id, idx, V.num_envs, e);
+                row[i] = soa(V.mob_position, idx * 2, V.num_envs, e);
+                col[i] = soa(V.mob_position, idx * 2 + 1, V.num_envs, e);
+            }
         }
     }
-    bool alive = false;
-    uint32_t pk[kSlots] = {0, 0, 0};
+    __device__ __forceinline__ bool put(int c, int top, int left, uint32_t* mobs) const {   // true if one is alive
+        bool alive = false;
+        uint32_t pk[kSlots] = {0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < kN; i++) {
-        alive = alive || on[i] != 0;
-        pk[i] = pack_mob(C, type[i], on[i] != 0, row[i], col[i], top, left);
+        for (int i = 0; i < kN; i++) {
+            alive = alive || on[i] != 0;
+            pk[i] = pack_mob(c, type[i], on[i] != 0, row[i], col[i], top, left);
+        }
+        // "last slot wins": a later slot of the class on the same cell replaces an earlier one
+        // (:9222-9231); the earlier one is dropped here, so the stores of phase 3 need no order
+#pragma unroll
+        for (int i = 0; i < kN - 1; i++)
+#pragma unroll
+            for (int i2 = i + 1; i2 < kN; i2++)
+                if (same_cell(pk[i], pk[i2])) pk[i] = 0;
+#pragma unroll
+        for (int i = 0; i < kSlots; i++) mobs[c * kSlots + i] = pk[i];
+        return alive;
     }
-    // "last slot wins": a later slot of the class on the same cell replaces an earlier one
-    // (:9222-9231); the earlier one is dropped here, so the stores of phase 3 need no order
-#pragma unroll
-    for (int i = 0; i < kN - 1; i++)
-#pragma unroll
-        for (int i2 = i + 1; i2 < kN; i2++)
-            if (same_cell(pk[i], pk[i2])) pk[i] = 0;
-#pragma unroll
-    for (int i = 0; i < kSlots; i++) mobs[C * kSlots + i] = pk[i];
-    return alive;
-}
+};
 
-// phase 2: everything of env e that does not depend on the cell.  Lane t of EVERY warp of the
-// block works on env t of the block; warp `part` takes an eighth of the loads.  The 51 scalars are in
-// the order of craftax_encode_scalar_observation_tail_at (:2429-2487).
-__device__ __forceinline__ void gather_env(const cfx_env_view& V, int e, int t, int part, int level, int top, int left,
-                                           Gathered& S) {
-    const int n = V.num_envs;
-    float* o = S.tail[t];
+// phase 2: everything of env e that does not depend on the cell.  Lane t of EVERY warp of the block works on env t of
+// the block; warp `part` takes an eighth of the loads.  The 51 scalars are in the order of
+// craftax_encode_scalar_observation_tail_at (:2429-2487).  In three steps, each a memory latency: the fields, which wait for nothing; what depends on
+// the level; the mobs that are alive.  (All of it behind the copies of the map rows, and the two classes of part 4 one after the other,
+// made that warp the last of the block by 5,000 of its 25,000 cycles.)
+struct Gather {
+    uint32_t raw[13];
+    int32_t killed;
+    Mobs<kSlots> first;   // of class 0 in part 4, of classes 1, 3 and 4 in parts 5 to 7
+    Mobs<2> ranged;       // of class 2, whose third slot is never used, in part 4
+    __device__ __forceinline__ void load_fields(const cfx_env_view& V, int e, int part) {
+        const int n = V.num_envs;
+        auto word = [&](const auto* f, int elem) { return ld_bits(reinterpret_cast<const uint32_t*>(f) + ((size_t)elem * (size_t)n + (size_t)e)); };
+        if (part == 0) {
+            const int32_t* const f[12] = {V.inv_wood, V.inv_stone, V.inv_coal, V.inv_iron, V.inv_diamond, V.inv_sapphire,
+                                          V.inv_ruby, V.inv_sapling, V.inv_torches, V.inv_arrows, V.inv_books, V.inv_pickaxe};
+#pragma unroll
+            for (int i = 0; i < 12; i++) raw[i] = word(f[i], 0);
+        } else if (part == 1) {
+            const int32_t* const f[4] = {V.inv_sword, V.sword_enchantment, V.bow_enchantment, V.inv_bow};
+#pragma unroll
+            for (int i = 0; i < 4; i++) raw[i] = word(f[i], 0);
+#pragma unroll
+            for (int i = 0; i < 6; i++) raw[4 + i] = word(V.inv_potions, i);
+            raw[10] = word(V.player_health, 0);
+        } else if (part == 2) {
+            const int32_t* const f[9] = {V.player_food, V.player_drink, V.player_energy, V.player_mana, V.player_xp,
+                                         V.player_dexterity, V.player_strength, V.player_intelligence, V.player_direction};
+#pragma unroll
+            for (int i = 0; i < 9; i++) raw[i] = word(f[i], 0);
+#pragma unroll
+            for (int i = 0; i < 4; i++) raw[9 + i] = word(V.inv_armour, i);
+        } else if (part == 3) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) raw[i] = word(V.armour_enchantments, i);
+            raw[4] = word(V.light_level, 0);
+            raw[5] = soa(V.is_sleeping, 0, n, e);
+            raw[6] = soa(V.is_resting, 0, n, e);
+            raw[7] = soa(V.learned_spells, 0, n, e);
+            raw[8] = soa(V.learned_spells, 1, n, e);
+        } else if (part == 4) {
+            raw[0] = word(V.boss_timesteps_to_spawn_this_round, 0);
+        }
+    }
     // mobs of the player's level inside the view and on the map (:9195-9236).  Whether the cell is lit is
     // looked up in the copied row when the record is put together: two slots on one cell are both lit or
     // both not, so the order of dropping does not depend on it.
-    const int mob_level = jax_index(level, kLevels);
-    auto mobs = [&](auto... c) { return (gather_mobs<decltype(c)::value>(V, e, mob_level, top, left, S.mobs[t]) | ...); };
-    if (part == 0) {
-        const int32_t* const counts[10] = {V.inv_wood, V.inv_stone, V.inv_coal, V.inv_iron, V.inv_diamond, V.inv_sapphire,
-                                           V.inv_ruby, V.inv_sapling, V.inv_torches, V.inv_arrows};
-        int32_t a[10];
-#pragma unroll
-        for (int i = 0; i < 10; i++) a[i] = soa(counts[i], 0, n, e);
-        const int32_t books = soa(V.inv_books, 0, n, e), pickaxe = soa(V.inv_pickaxe, 0, n, e);
-#pragma unroll
-        for (int i = 0; i < 10; i++) o[i] = sqrtf((float)a[i]) * (1.0f / 10.0f);
-        o[10] = (float)books * (1.0f / 2.0f);
-        o[11] = (float)pickaxe * (1.0f / 4.0f);
-    } else if (part == 1) {
-        const int32_t sword = soa(V.inv_sword, 0, n, e);
-        const int32_t b[3] = {soa(V.sword_enchantment, 0, n, e), soa(V.bow_enchantment, 0, n, e), soa(V.inv_bow, 0, n, e)};
-        int32_t p[6];
-#pragma unroll
-        for (int i = 0; i < 6; i++) p[i] = soa(V.inv_potions, i, n, e);
-        const float health = soa(V.player_health, 0, n, e);
-        o[12] = (float)sword * (1.0f / 4.0f);
-#pragma unroll
-        for (int i = 0; i < 3; i++) o[13 + i] = (float)b[i];
-#pragma unroll
-        for (int i = 0; i < 6; i++) o[16 + i] = sqrtf((float)p[i]) * (1.0f / 10.0f);
-        o[22] = health * (1.0f / 10.0f);
-    } else if (part == 2) {
-        const int32_t* const tenths[8] = {V.player_food, V.player_drink, V.player_energy, V.player_mana, V.player_xp,
-                                          V.player_dexterity, V.player_strength, V.player_intelligence};
-        int32_t a[8], arm[4];
-#pragma unroll
-        for (int i = 0; i < 8; i++) a[i] = soa(tenths[i], 0, n, e);
-        const int direction_index = soa(V.player_direction, 0, n, e) - 1;
-#pragma unroll
-        for (int i = 0; i < 4; i++) arm[i] = soa(V.inv_armour, i, n, e);
-#pragma unroll
-        for (int i = 0; i < 8; i++) o[23 + i] = (float)a[i] * (1.0f / 10.0f);
-#pragma unroll
-        for (int i = 0; i < 4; i++) o[31 + i] = i == direction_index ? 1.0f : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 4; i++) o[35 + i] = (float)arm[i] * (1.0f / 2.0f);
-    } else if (part == 3) {
-        int32_t ench[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) ench[i] = soa(V.armour_enchantments, i, n, e);
-        const float light = soa(V.light_level, 0, n, e);
-        const uint8_t f[4] = {soa(V.is_sleeping, 0, n, e), soa(V.is_resting, 0, n, e), soa(V.learned_spells, 0, n, e),
-                              soa(V.learned_spells, 1, n, e)};
-        const bool level_ok = (unsigned)level < (unsigned)kLevels;
-        const int killed = soa(V.monsters_killed, level_ok ? level : 0, n, e);
-#pragma unroll
-        for (int i = 0; i < 4; i++) o[39 + i] = (float)ench[i];
-        o[43] = light;
-#pragma unroll
-        for (int i = 0; i < 4; i++) o[44 + i] = f[i] != 0 ? 1.0f : 0.0f;
-        o[48] = (float)level * (1.0f / 10.0f);
-        o[49] = level_ok && killed >= kKilledToClear ? 1.0f : 0.0f;
-    } else if (part == 4) {
-        const int32_t boss = soa(V.boss_timesteps_to_spawn_this_round, 0, n, e);
-        const bool melee_or_ranged = mobs(std::integral_constant<int, 0>(), std::integral_constant<int, 2>());
-        // craftax_wg_is_boss_vulnerable (:1988-2003): no melee and no ranged mob alive on the level
-        o[50] = !melee_or_ranged && boss <= 0 ? 1.0f : 0.0f;
-    } else if (part == 5) {
-        mobs(std::integral_constant<int, 1>());
-    } else if (part == 6) {
-        mobs(std::integral_constant<int, 3>());
-    } else {
-        mobs(std::integral_constant<int, 4>());
+    __device__ __forceinline__ void load_of_level(const cfx_env_view& V, int e, int part, int level) {
+        const int mob_level = jax_index(level, kLevels);
+        if (part == 3) {
+            killed = soa(V.monsters_killed, (unsigned)level < (unsigned)kLevels ? level : 0, V.num_envs, e);
+        } else if (part >= 4) {
+            first.load_alive(V, e, mob_class(part), mob_level);
+            if (part == 4) ranged.load_alive(V, e, 2, mob_level);
+        }
     }
-}
+    __device__ __forceinline__ void finish(const cfx_env_view& V, int e, int t, int part, int level, int top, int left, Gathered& S) {
+        const int mob_level = jax_index(level, kLevels);
+        float* o = S.tail[t];
+        auto whole = [&](int i) { return (float)(int32_t)raw[i]; };
+        if (part == 0) {
+#pragma unroll
+            for (int i = 0; i < 10; i++) o[i] = sqrtf(whole(i)) * (1.0f / 10.0f);
+            o[10] = whole(10) * (1.0f / 2.0f);
+            o[11] = whole(11) * (1.0f / 4.0f);
+        } else if (part == 1) {
+            o[12] = whole(0) * (1.0f / 4.0f);
+#pragma unroll
+            for (int i = 0; i < 3; i++) o[13 + i] = whole(1 + i);
+#pragma unroll
+            for (int i = 0; i < 6; i++) o[16 + i] = sqrtf(whole(4 + i)) * (1.0f / 10.0f);
+            o[22] = __uint_as_float(raw[10]) * (1.0f / 10.0f);
+        } else if (part == 2) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) o[23 + i] = whole(i) * (1.0f / 10.0f);
+            const int direction_index = (int)raw[8] - 1;
+#pragma unroll
+            for (int i = 0; i < 4; i++) o[31 + i] = i == direction_index ? 1.0f : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) o[35 + i] = whole(9 + i) * (1.0f / 2.0f);
+        } else if (part == 3) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) o[39 + i] = whole(i);
+            o[43] = __uint_as_float(raw[4]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) o[44 + i] = raw[5 + i] != 0 ? 1.0f : 0.0f;
+            o[48] = (float)level * (1.0f / 10.0f);
+            o[49] = (unsigned)level < (unsigned)kLevels && killed >= kKilledToClear ? 1.0f : 0.0f;
+        } else {
+            const int c = mob_class(part);
+            first.load_slots(V, e, c, mob_level);
+            if (part == 4) ranged.load_slots(V, e, 2, mob_level);
+            const bool alive = first.put(c, top, left, S.mobs[t]);
+            // craftax_wg_is_boss_vulnerable (:1988-2003): no melee and no ranged mob alive on the level
+            if (part == 4) o[50] = !ranged.put(2, top, left, S.mobs[t]) && !alive && (int32_t)raw[0] <= 0 ? 1.0f : 0.0f;
+        }
+    }
+private:
+    static __device__ __forceinline__ int mob_class(int part) { return part == 4 ? 0 : part == 5 ? 1 : part - 3; }
+};
 
 // What the copies and the assembly of one env need, in a word: top and left of the view, plane of the level, and whether there
 // is such a level.
@@ -246,19 +271,13 @@ __device__ __forceinline__ View make_view(int level, int top, int left) {
     return {(uint32_t)(top + 32) | (uint32_t)(left + 32) << 8 | (uint32_t)jax_index(level, kLevels) << 16 |
             ((unsigned)level < (unsigned)kLevels ? 1u << 24 : 0u)};
 }
-// Where byte `o` of a view row's 32 bytes lies: rows 4 to 7 have their halves swapped, so that a warp's reads of the nine rows
-// meet in a bank two at a time and not three
-__device__ __forceinline__ int row_byte(int dr, int o) { return dr * kRowSpan + (o ^ (dr & 4) << 2); }
-// The part of a lane in the copies of a view's rows (light, block, item): row `dr` of plane `plane`, `src` is the plane of env 0
+// Where byte `o` of view row dr lies in a span, counted from the 16-byte word of the view's first byte; the nine rows start in eight
+// different groups of four banks
+__device__ __forceinline__ int row_byte(int dr, int o) { return dr * kMapSize + o; }
+// The part of a lane in the copies of an env's view (light, block, item)
 struct CopyLane {
-    const uint8_t* src;
-    int plane, dr, lane;
-    __device__ __forceinline__ CopyLane(const cfx_env_view& V, int l) {
-        lane = l;
-        plane = lane / kRows;
-        dr = lane % kRows;
-        src = V.state_base + (plane == 0 ? V.light_map_offset : plane == 1 ? V.map_offset : V.item_map_offset);
-    }
+    int lane;
+    __device__ __forceinline__ explicit CopyLane(int l) : lane(l) {}
     // Planes that are not aligned to words: a lane takes every 32nd cell of the view, its bytes of the three planes all in flight
     // (65,536 envs 59 us with a byte load per cell and map and nothing else, 75 with the bytes of a row one after the other)
     __device__ __forceinline__ void bytes(const cfx_env_view& V, int e, View v, uint8_t* dst) const {
@@ -281,25 +300,28 @@ struct CopyLane {
             for (int p = 0; p < kPlanes; p++) dst[p * kSpan + row_byte(cell / kCols, (v.left() & 15) + cell % kCols)] = b[i][p];
         }
     }
-    // Starts the copies of env e's rows into `dst`.  A map row is 48 bytes, so 16-byte pieces (4-byte pieces) stay inside
-    // it where the planes are aligned to 16 (4) bytes.
+    // Starts the copies of env e's view into `dst`: where the planes are aligned to 16 bytes, the pieces of a plane's span side by
+    // side, an instruction a plane (what lies between the view's rows comes along: memory is read in bursts of 64 bytes anyway);
+    // else words, a lane a row of a plane.
     template <bool BYTES>
     __device__ __forceinline__ void start(const cfx_env_view& V, int e, View v, int grain, uint8_t* dst) const {
         if constexpr (BYTES) return bytes(V, e, v, dst);
-        const int row = v.top() + dr, left = v.left(), c0 = left & ~15;
-        if (plane >= kPlanes || (unsigned)row >= (unsigned)kMapSize) return;
-        const uint8_t* q = src + (size_t)e * V.state_stride + (v.level() * kPlaneBytes + row * kMapSize + c0);
-        uint8_t* d = dst + plane * kSpan;
-        auto wanted = [&](int o, int bytes) { return c0 + o >= 0 && c0 + o < min(left + kCols, kMapSize) && c0 + o + bytes > left; };
+        const uint64_t off[kPlanes] = {V.light_map_offset, V.map_offset, V.item_map_offset};
+        const uint8_t* const q = V.state_base + (size_t)e * V.state_stride + v.level() * kPlaneBytes;
+        const int left = v.left(), c0 = left & ~15;
         if (grain == 16) {
+            const int at = v.top() * kMapSize + c0 + 16 * lane;
+            if (lane >= kPieces || (unsigned)at >= (unsigned)kPlaneBytes) return;
 #pragma unroll
-            for (int o = 0; o < kRowSpan; o += 16)
-                if (wanted(o, 16))
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d + row_byte(dr, o))), "l"(q + o) : "memory");
+            for (int p = 0; p < kPlanes; p++)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + p * kSpan + 16 * lane)), "l"(q + off[p] + at) : "memory");
         } else {
-            for (int o = 0; o < kRowSpan; o += 4)
-                if (wanted(o, 4))
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(d + row_byte(dr, o))), "l"(q + o) : "memory");
+            const int plane = lane / kRows, dr = lane % kRows, row = v.top() + dr;
+            if (plane >= kPlanes || (unsigned)row >= (unsigned)kMapSize) return;
+            const uint8_t* src = q + (plane == 0 ? off[0] : plane == 1 ? off[1] : off[2]) + row * kMapSize + c0;
+            for (int o = 0; o < 32; o += 4)   // the view's columns, and only those on the map
+                if (c0 + o >= 0 && c0 + o < min(left + kCols, kMapSize) && c0 + o + 4 > left)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + plane * kSpan + row_byte(dr, o))), "l"(src + o) : "memory");
         }
     }
 };
@@ -405,24 +427,32 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_record_rows(const __grid_c
     const int e0 = blockIdx.x * kBlockEnvs, e = e0 + lane;
     const int n = P.v.num_envs, grain = copy_grain(P.v);
     wait_for_previous_kernel();
-    const bool live = e < P.n && (P.skip == nullptr || ld_now(P.skip + e) == 0);
+    bool live = e < P.n;
     int level = 0, top = 0, left = 0;
-    if (live) {
+    if (live) {   // the flag and the position on their way together
+        const uint8_t skipped = P.skip != nullptr ? ld_now(P.skip + e) : (uint8_t)0;
         level = soa(P.v.player_level, 0, n, e);
         top = soa(P.v.player_position, 0, n, e) - kRows / 2;
         left = soa(P.v.player_position, 1, n, e) - kCols / 2;
+        live = skipped == 0;
     }
     const View mine = make_view(level, top, left);
-    const CopyLane copy(P.v, lane);
+    const CopyLane copy(lane);
     uint8_t* const span = S.span[warp];
     const uint32_t todo = __ballot_sync(0xffffffffu, live) >> (kOwn * warp) & ((1u << kOwn) - 1u);
     View v[kOwn];   // of this warp's envs, kOwn * warp + k of the block
 #pragma unroll
+    for (int k = 0; k < kOwn; k++) v[k].bits = __shfl_sync(0xffffffffu, mine.bits, kOwn * warp + k);
+    Gather g;
+    if (live) {
+        g.load_fields(P.v, e, warp);
+        g.load_of_level(P.v, e, warp, level);
+    }
+#pragma unroll
     for (int k = 0; k < kOwn; k++) {
-        v[k].bits = __shfl_sync(0xffffffffu, mine.bits, kOwn * warp + k);
         if (todo >> k & 1u) copy.start<BYTES>(P.v, e0 + kOwn * warp + k, v[k], grain, span + k * kPlanes * kSpan);
     }
-    if (live) gather_env(P.v, e, lane, warp, level, top, left, S);
+    if (live) g.finish(P.v, e, lane, warp, level, top, left, S);
     wait_spans();
     __syncthreads();
     const uint32_t* rec = assemble(S, v, todo, kOwn * warp, lane, span);
@@ -503,7 +533,7 @@ struct ListShared {
 static_assert(sizeof(ListShared) % 16 == 0, "alignment");
 constexpr int kListThreads = 128, kListWarps = kListThreads / 32;
 struct ListBlock : Gathered {
-    __align__(16) uint8_t span[kListWarps][kOwn * kRec];
+    __align__(16) uint8_t span[kListWarps][kOwn * kPlanes * kSpan];
 };
 union ListMemory {
     ListShared warp[kListWarps];
@@ -543,7 +573,12 @@ __device__ __forceinline__ void list_block(const Params& P, ListBlock& S, const 
     copies(kWarpEnvs * warp);
 #pragma unroll 1
     for (int part = warp; part < kWarps; part += kListWarps)
-        if (live) gather_env(V, e, lane, part, level, top, left, S);
+        if (live) {
+            Gather g;
+            g.load_fields(V, e, part);
+            g.load_of_level(V, e, part, level);
+            g.finish(V, e, lane, part, level, top, left, S);
+        }
     wait_spans();
     __syncthreads();
 #pragma unroll 1
@@ -570,7 +605,7 @@ __global__ void __launch_bounds__(kListThreads, 4) k_record_rows_list(const __gr
     const cfx_env_view& V = P.v;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = V.num_envs, grain = copy_grain(V);
     ListShared& S = M.warp[warp];
-    const CopyLane copy(V, lane);
+    const CopyLane copy(lane);
     const TailField f0 = kTailFields[lane], f1 = kTailFields[min(lane + 32, kTail - 1)];
     wait_for_previous_kernel();
     const int count = *P.count_dev;
