@@ -32,8 +32,8 @@
 // records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
 // Measured (us a step in a stream, fp16; the persistent kernel, one CTA pair per two tiles -> here): h256x2, 32 envs 20.6 -> 9.5,
-// 256 21.0 -> 10.0, 1,024 21.5 -> 10.4, 2,048 21.7 -> 14.8, 4,000 22.3 -> 17.4, 8,192 22.7 -> 18.9; classic h256x3, 1,024 envs 28.9 -> 14.5, 4,000
-// 29.7 -> 25.0, 8,192 30.2 -> 26.6.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
+// 256 21.0 -> 10.0, 1,024 21.5 -> 10.4, 2,048 21.7 -> 14.8, 4,000 22.3 -> 16.9, 8,192 22.7 -> 18.9; classic h256x3, 1,024 envs 28.9 -> 14.3, 4,000
+// 29.7 -> 24.4, 8,192 30.2 -> 26.6.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
 // In clusters of two an encoder's weights are 14 pieces of 16 KB a CTA: with one lane issuing them, 500 cycles a slot, and one a
 // slot of 24 KB, the multiplications waited for them, 10,200 cycles to the encoder's end at 8,192 envs; now 8,700, with the MMA warp waiting for
 // the records' conversion.  8,192 envs h256x2: 20.00 us before, 19.94 with the slices in turn, 19.46 with the weight warp converged, 19.08 with the
