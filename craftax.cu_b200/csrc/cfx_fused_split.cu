@@ -32,8 +32,8 @@
 // records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
 // Measured (us a step in a stream, fp16; the persistent kernel, one CTA pair per two tiles -> here): h256x2, 32 envs 20.6 -> 9.5,
-// 256 21.0 -> 10.0, 1,024 21.5 -> 10.4, 2,048 21.7 -> 14.8, 4,000 22.3 -> 16.9, 8,192 22.7 -> 18.9; classic h256x3, 1,024 envs 28.9 -> 14.3, 4,000
-// 29.7 -> 24.4, 8,192 30.2 -> 26.6.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
+// 256 21.0 -> 10.0, 1,024 21.5 -> 10.4, 2,048 21.7 -> 14.6, 4,000 22.3 -> 16.9, 8,192 22.7 -> 18.9; classic h256x3, 1,024 envs 28.9 -> 14.3, 4,000
+// 29.7 -> 24.3, 8,192 30.2 -> 26.5.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
 // In clusters of two an encoder's weights are 14 pieces of 16 KB a CTA: with one lane issuing them, 500 cycles a slot, and one a
 // slot of 24 KB, the multiplications waited for them, 10,200 cycles to the encoder's end at 8,192 envs; now 8,700, with the MMA warp waiting for
 // the records' conversion.  8,192 envs h256x2: 20.00 us before, 19.94 with the slices in turn, 19.46 with the weight warp converged, 19.08 with the
@@ -499,11 +499,12 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     __syncwarp();
     if (lane < S) mbar_arrive_cluster(map_to_cta(sm.bar(REC_FREE), (uint32_t)lane));
     // The last of the warps that need the step counter raises it, once all have read it (here, where the encoder's MMAs are
-    // waited for; at the kernel's end it was a microsecond of the step)
-    float u = 0.0f;
-    if (samples && wg == 0) {
-        if (valid)
-            u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
+    // waited for; at the kernel's end it was a microsecond of the step).  The draw itself comes under the first layer's MMAs: with both
+    // here, 2,600 cycles, the warp was late for the encoder's output, and the cluster with it (h256x2, 1,600 envs 14.6 -> 14.35 us, 2,112 15.0 -> 14.7;
+    // h128x2, 4,736 12.9 -> 12.7).
+    const bool draws = samples && wg == 0;
+    if (draws) {
+        asm volatile("" ::"l"(step0));   // has been read
         __syncwarp();
         if (lane == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
     }
@@ -548,6 +549,9 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             x[j][q] = Op::pack(__uint_as_float(acc[2 * q]) + b[2 * q], __uint_as_float(acc[2 * q + 1]) + b[2 * q + 1]);
         if (!send(0, j, x[j])) return;
     }
+    float u = 0.0f;
+    if (draws && valid)
+        u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
 
     // ---- layers
     for (int l = 0; l < P.L; l++) {
@@ -733,9 +737,8 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         if (lane < S) mbar_arrive_cluster(map_to_cta(sm.bar(REC_FREE), (uint32_t)lane));
     };
     if (kFull && !C::kOneBeside) free_records();
-    float u = 0.0f;
-    if (draws) {   // (the counter: see role_worker)
-        u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
+    if (draws) {   // (see role_worker)
+        asm volatile("" ::"l"(step0));
         __syncwarp();
         if (lane == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
     }
@@ -774,6 +777,8 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         *xp(0) = x;
     }
     if (!send(0)) return;
+    float u = 0.0f;
+    if (draws) u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
 
     // ---- layers
     for (int l = 0; l < P.L; l++) {
