@@ -134,8 +134,8 @@ __host__ __device__ __forceinline__ size_t act_at(size_t e, int k, int H) { retu
 constexpr int kEncK = 32, kEncAhead = 3;
 constexpr int kMapChunks = (kMap + kEncK - 1) / kEncK, kEncChunks = kMapChunks + (kTail + kEncK - 1) / kEncK;   // 25 of record bytes, 2 of the tail
 static_assert(kEncChunks % kEncAhead == 0, "the chunk loop is unrolled by the words in flight");
-template <int TM, int G, int WU> struct Enc {   // WU of the four warps side by side along the units
-    static constexpr int WM = 4 / WU, BM = 4 * TM * WM, BU = 32 * G * WU;   // envs, units
+template <int TM, int G, int WU, int UL> struct Enc {   // WU of the four warps side by side along the units, UL units of a group a lane
+    static constexpr int WM = 4 / WU, BM = UL * TM * WM, BU = 32 * G * WU;   // envs, units
     static constexpr int XS = BM + (BM % 8 == 0 ? 4 : 0);               // row stride of x: four rows are 16 banks on
     static constexpr int S = TM == 1 ? 6 : (G == 1 ? 4 : 3);      // stages
     static constexpr int kStage = kEncK * (XS + BU);                    // floats
@@ -145,11 +145,12 @@ template <int TM, int G, int WU> struct Enc {   // WU of the four warps side by 
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
-template <int TM, int G, int WU>
+template <int TM, int G, int WU, int UL>
 __global__ void __launch_bounds__(256, 2)
 k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc,
                float* __restrict__ h_out, int n, int H, int w_aligned, int early) {
-    using E = Enc<TM, G, WU>;
+    using E = Enc<TM, G, WU, UL>;
+    static_assert(UL == 4 || (UL == 1 && TM == 1 && G == 1), "tiles");
     constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = kEncK, S = E::S, D = S - 2;
     constexpr int FULL = 1, EMPTY = FULL + S, TAIL = 15;   // barrier ids
     extern __shared__ __align__(16) float sm[];   // per stage: x [K][XS], w [K][BU]; then the tail [kTail][XS]
@@ -230,15 +231,21 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
                      "l"(rec + (size_t)(on ? e0 + e : e0) * kRec + kMap + 4 * j), "r"(on ? 4 : 0) : "memory");
     }
     copy_commit();
-    const int el = warp % E::WM * 4 * TM, ul = warp / E::WM * 32 * G + (lane & 7) * 4, lg = lane >> 3;   // the warp's first env
+    const int el = warp % E::WM * UL * TM, ul = warp / E::WM * 32 * G + lane % (32 / UL) * UL, lg = lane / (32 / UL);   // the warp's first env
+    float z1 = UL == 1 ? b_enc[u0 + ul] : 0.0f;   // the sum of a lane with one
     uint64_t z[G][TM][2];
 #pragma unroll
     for (int g = 0; g < G; g++) {
+        if (UL == 1) break;
         const float* b = b_enc + u0 + ul + 32 * g;
 #pragma unroll
         for (int e = 0; e < TM; e++) { z[g][e][0] = f2pack(b[0], b[1]); z[g][e][1] = f2pack(b[2], b[3]); }
     }
     auto step = [&](const float* xp, const float* wp) {
+        if constexpr (UL == 1) {
+            z1 = fmaf(*xp, *wp, z1);
+            return;
+        }
         Frag<TM> x;
         x.load(xp, lg);
 #pragma unroll
@@ -273,6 +280,10 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
             for (; k < rows; k++) step(xp + k * XS, wp + k * BU);
         }
         if (c + S < kEncChunks) bar_arrive(EMPTY + s, 256);
+    }
+    if constexpr (UL == 1) {
+        if (e0 + el < n) h_out[act_at(e0 + el, u0 + ul, H)] = z1;
+        return;
     }
 #pragma unroll
     for (int p = 0; p < Envs<TM>::kParts; p++) {
@@ -570,6 +581,75 @@ k_mingru_fp32(const float* x_in, const float* __restrict__ Wt, float* __restrict
     }
 }
 
+// The smallest batches: one env x one unit a lane, a warp 32 units of an env.  With 4 units a lane the reads of shared memory (13 a k
+// step and warp) are what a lone block waits for, 63 cycles a k step; here they are 4.  The sums are the same ones in the same
+// order.  A block takes 2 envs x 64 units.
+constexpr int kSmallEnvs = 2, kSmallUnits = 64, kSmallStages = 4, kSmallThreads = 128;
+constexpr int kSmallStage = kGruK * (kSmallEnvs + 3 * kSmallUnits);   // floats: x [kGruK][2], w [kGruK][3][64]
+__global__ void __launch_bounds__(kSmallThreads)
+k_mingru_small(const float* x_in, const float* __restrict__ Wt, float* __restrict__ state, const float* prev_terminals,
+               float* __restrict__ h_out, float* __restrict__ r_state, int r_bf16, int H, int early) {
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, e = tid / kSmallUnits, u = tid % kSmallUnits;
+    const int e0 = blockIdx.x * kSmallEnvs, u0 = blockIdx.y * kSmallUnits;   // (n is a multiple of 32)
+    const float* wsrc = Wt + (size_t)u0 * 3 * H;
+    constexpr int NW = kGruK * 3 * kSmallUnits / (4 * kSmallThreads);
+    auto copy_w = [&](int c) {
+        float* w = sm + (c % kSmallStages) * kSmallStage + kGruK * kSmallEnvs;
+#pragma unroll
+        for (int i = 0; i < NW; i++) {
+            const int at = 4 * (i * kSmallThreads + tid);
+            copy16(w + at, wsrc + (size_t)c * kGruK * 3 * kSmallUnits + at, true, true);
+        }
+    };
+    auto copy_x = [&](int c) {
+        if (tid < kGruK)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(sm + (c % kSmallStages) * kSmallStage + tid * kSmallEnvs)),
+                         "l"(x_in + act_at(e0, c * kGruK + tid, H)) : "memory");
+    };
+    if (early & kLaunchNext) launch_next_kernel();
+    const int chunks = H / kGruK;
+    if (!(early & kWeightsReady)) wait_for_previous_kernel();
+#pragma unroll
+    for (int c = 0; c < kSmallStages - 1; c++)
+        if (c < chunks) copy_w(c);
+    wait_for_previous_kernel();
+#pragma unroll
+    for (int c = 0; c < kSmallStages - 1; c++) {
+        if (c < chunks) copy_x(c);
+        copy_commit();
+    }
+    const size_t o = (size_t)(e0 + e) * H + u0 + u;
+    float st = state[o];
+    const float ended = prev_terminals != nullptr ? prev_terminals[e0 + e] : 0.0f, x_own = x_in[act_at(e0 + e, u0 + u, H)];
+    float z[3] = {0.0f, 0.0f, 0.0f};
+    for (int c = 0; c < chunks; c++) {
+        copy_wait<kSmallStages - 2>();
+        __syncthreads();   // chunk c is complete, and everybody is done with chunk c - 1
+        if (c + kSmallStages - 1 < chunks) {
+            copy_w(c + kSmallStages - 1);
+            copy_x(c + kSmallStages - 1);
+        }
+        copy_commit();
+        const float* x = sm + (c % kSmallStages) * kSmallStage + e;
+        const float* w = sm + (c % kSmallStages) * kSmallStage + kGruK * kSmallEnvs + u;
+#pragma unroll
+        for (int k = 0; k < kGruK; k++)
+#pragma unroll
+            for (int g = 0; g < 3; g++) z[g] = fmaf(w[(3 * k + g) * kSmallUnits], x[k * kSmallEnvs], z[g]);
+    }
+    if (ended != 0.0f) st = 0.0f;
+    if (r_state != nullptr) {   // the post-zero state input
+        if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o] = __float2bfloat16(st);
+        else r_state[o] = st;
+    }
+    const float zh = z[0];
+    sigmoids_ref(z, 3);
+    const float gh = zh >= 0.0f ? zh + 0.5f : z[0], out = st + z[1] * (gh - st);
+    h_out[act_at(e0 + e, u0 + u, H)] = z[2] * out + (1.0f - z[2]) * x_own;
+    state[o] = out;
+}
+
 // ---------------------------------------------------------------- heads
 // logits_av[e][a] = bias[a] + sum_j W_av[a][j] * h[j][e] (ascending j); row A is the value head.
 // Accumulator starts at the bias as in the scalar reference (craftax_full.cu:9838-9845).  A block
@@ -854,12 +934,17 @@ int launch_init_uniform(float* w, int count, float bound, uint64_t seed, int sub
 // to 16,384, hidden 64 to 512: this choice is the best at all of them in the encoder, and within 1 % of it in the layers.)
 constexpr int kSMs = 148;
 static int sm_rounds(int n, int envs, int unit_tiles) { return ((n + envs - 1) / envs * unit_tiles + kSMs - 1) / kSMs; }
+// Up to q = 32 a lane has one sum, or one of each gate (tile 0): us a forward of 32 envs, hidden 256, depth 2, with 4 units a lane in both kernels
+// 46.2, in the encoder 38.7, in neither 32.0; 64 envs 47.6, 43.7 and 34.2; 128 envs 49.1 and 44.1; 192 envs 48.7 and 63; 32 envs, hidden 512 73 and 46;
+// 256 envs, hidden 128 38.7 and 35.2; 512 envs, hidden 64 33.4 and 31.1.
+constexpr int kSmallest = 32;
 // A layer.  1 env a lane under q = 96, where even tiles of 4 leave schedulers without a warp (256 envs: 55 against 71 us;
 // 512 envs: 77 against 72).  Blocks of 4 envs a lane take the same time alone and beside each other, those of more envs a little less beside one.
 // Narrow layers have as much to do around the sums as in them, and stay with 4 longer (4,096 envs, hidden 128: 52.9 us, 54.3 with 7; 8,192 78.5
 // and 77.5).
 static int strict_tile(int n, int H) {
     const long long q = (long long)n * H / 1024;
+    if (q <= kSmallest && H % 64 == 0) return 0;
     if (q < 96) return 1;
     if (H % 64 != 0) return q >= 1024 ? 8 : 4;
     if (H < 256 && q < 1024) return 4;
@@ -879,6 +964,7 @@ static int strict_tile(int n, int H) {
 struct EncoderTile { int tm, g; };
 static EncoderTile strict_encoder_tile(int n, int H) {
     const long long q = (long long)n * H / 1024;
+    if (q <= kSmallest) return {0, 1};
     if (q < 96) return {1, 1};
     if (H % 64 != 0 || sm_rounds(n, 64, H / 32) == 1) return {4, 1};
     const int wu = H % 128 == 0 ? 2 : 1;
@@ -888,12 +974,12 @@ static EncoderTile strict_encoder_tile(int n, int H) {
     return {best, 2};
 }
 
-template <int TM, int G, int WU>
+template <int TM, int G, int WU, int UL = 4>
 static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, int early, cudaStream_t st) {
-    using E = Enc<TM, G, WU>;
-    int rc = allow_smem<k_encoder_fp32<TM, G, WU>, E::kSmem>();
+    using E = Enc<TM, G, WU, UL>;
+    int rc = allow_smem<k_encoder_fp32<TM, G, WU, UL>, E::kSmem>();
     if (rc) return rc;
-    return launch_chained(k_encoder_fp32<TM, G, WU>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
+    return launch_chained(k_encoder_fp32<TM, G, WU, UL>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
                           a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], a.n, a.H,
                           ((uintptr_t)(a.params + o.w_enc) & 15) == 0, early);
 }
@@ -919,6 +1005,20 @@ static int strict_layers(const StrictArgs& a, int early, cudaStream_t st) {
     return CFX_OK;
 }
 
+// (H a multiple of 64)
+static int strict_layers_small(const StrictArgs& a, int early, cudaStream_t st) {
+    constexpr int smem = kSmallStages * kSmallStage * (int)sizeof(float);
+    int rc = allow_smem<k_mingru_small, smem>();
+    for (int l = 0; l < a.L && rc == CFX_OK; l++) {
+        const size_t at = (size_t)l * a.n * a.H;
+        float* r = a.r_state ? reinterpret_cast<float*>(reinterpret_cast<char*>(a.r_state) + at * (a.r_state_bf16 ? 2 : 4)) : nullptr;
+        rc = launch_chained(k_mingru_small, dim3(a.n / kSmallEnvs, a.H / kSmallUnits), kSmallThreads, smem, st, a.scratch_h[l & 1],
+                            a.gates_t + (size_t)l * 3 * a.H * a.H, a.state + at, a.prev_terminals, a.scratch_h[(l + 1) & 1], r, a.r_state_bf16,
+                            a.H, early);
+    }
+    return rc;
+}
+
 template <int N> using Int = std::integral_constant<int, N>;
 // Full strict forward.  scratch_h: two buffers of n H activations; logits_av [n][A+1].
 int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
@@ -928,10 +1028,12 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     const long long q = (long long)n * H / 1024;
     const int tm = strict_tile(n, H);
     const EncoderTile te = strict_encoder_tile(n, H);
-    // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own
-    // (512 envs, 64 blocks a layer: 88 us with it, 72 without)
-    const long long blocks = (te.tm == 1 ? 2 * q : q / 2) + L * (tm == 1 ? 2 * q : q / 2) + n / 16;
-    const int early = (a.game == CFX_GAME_FULL && blocks <= 148 ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
+    // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own (512 envs, 64 blocks a layer: 88 us
+    // with it, 72 without), or two of the smallest have one (32 envs, hidden 256, depths 1, 2, 3, with and without: 26.1 and 27.8, 31.7 and 33.5, 43.1
+    // and 39.1 us)
+    auto count = [&](int tile) { return tile == 0 ? 8 * q : tile == 1 ? 2 * q : q / 2; };
+    const long long blocks = count(te.tm) + L * count(tm) + n / 16;
+    const int early = (a.game == CFX_GAME_FULL && blocks <= (tm == 0 ? 200 : kSMs) ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
     if (a.game == CFX_GAME_CLASSIC) {
         rc = launch_chained(k_classic_encoder_fp32, dim3(n), H, 0, st, a.records, a.params + o.w_enc, a.params + o.b_enc,
                             a.scratch_h[0], n, H);
@@ -941,7 +1043,8 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
             constexpr int TM = decltype(tile)::value;
             return H % 128 == 0 ? strict_encoder<TM, 2, 2>(a, o, early, st) : strict_encoder<TM, 2, 1>(a, o, early, st);
         };
-        if (te.tm == 1) rc = strict_encoder<1, 1, 1>(a, o, early, st);
+        if (te.tm == 0) rc = strict_encoder<1, 1, 1, 1>(a, o, early, st);
+        else if (te.tm == 1) rc = strict_encoder<1, 1, 1>(a, o, early, st);
         else if (te.g == 1) rc = strict_encoder<4, 1, 1>(a, o, early, st);
         else rc = te.tm == 4 ? encode(Int<4>()) : te.tm == 5 ? encode(Int<5>()) : te.tm == 6 ? encode(Int<6>())
                   : te.tm == 7 ? encode(Int<7>()) : te.tm == 8 ? encode(Int<8>()) : encode(Int<9>());
@@ -951,6 +1054,7 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     if (H % 64 != 0)
         rc = tm == 8 ? strict_layers<8, 4, 1, 2>(a, early, st) : tm == 4 ? strict_layers<4, 4, 1, 2>(a, early, st)
                                                                          : strict_layers<1, 4, 1, 4>(a, early, st);
+    else if (tm == 0) rc = strict_layers_small(a, early, st);
     else if (tm == 1) rc = strict_layers<1, 2, 2, 4>(a, early, st);
     else if (tm == 4) rc = q <= 592 ? strict_layers<4, 2, 2, 3>(a, early, st) : strict_layers<4, 2, 2, 2>(a, early, st);
     else rc = tm == 5 ? strict_layers<5, 2, 2, 2>(a, early, st) : tm == 6 ? strict_layers<6, 2, 2, 2>(a, early, st)

@@ -74,7 +74,13 @@ def test_strict_heights_match_the_oracle(cfx, gpu, oracle, n, H, L):
     test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L)
 
 
-@pytest.mark.parametrize("n,H", [(32, 32), (416, 256), (1248, 256)])
+@pytest.mark.parametrize("n,H,L", [(32, 64, 4), (64, 512, 1), (128, 256, 2), (160, 192, 1), (96, 96, 2), (160, 256, 1)])
+def test_smallest_strict_batches_match_the_oracle(cfx, gpu, oracle, n, H, L):
+    """One sum a lane, up to the last size that takes it, and hidden sizes for which only the encoder does."""
+    test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L)
+
+
+@pytest.mark.parametrize("n,H", [(32, 32), (32, 256), (416, 256), (1248, 256)])
 def test_strict_saturated_gates(cfx, gpu, oracle, n, H):
     """Pre-activations up to some thousands: 1 + exp(-z) overflows, where the quotients are 0."""
     rec, params, state, prev_t, u = _inputs(oracle, n, H, 1)
