@@ -581,21 +581,26 @@ k_mingru_fp32(const float* x_in, const float* __restrict__ Wt, float* __restrict
     }
 }
 
-// The smallest batches: one env x one unit a lane, a warp 32 units of an env.  With 4 units a lane the reads of shared memory (13 a k
-// step and warp) are what a lone block waits for, 63 cycles a k step; here they are 4.  The sums are the same ones in the same
-// order.  A block takes 2 envs x 64 units.
-constexpr int kSmallEnvs = 2, kSmallUnits = 64, kSmallStages = 4, kSmallThreads = 128;
-constexpr int kSmallStage = kGruK * (kSmallEnvs + 3 * kSmallUnits);   // floats: x [kGruK][2], w [kGruK][3][64]
+// Small batches: N envs x N units a lane, N 1 or 2.  With 1 env x 4 units a lane the reads of shared memory (13 a k
+// step and warp) are what a lone block waits for, 63 cycles a k step; here they are 4, or 8 for as many sums as those 13.  The sums are the same ones
+// in the same order.  A block takes 2 N^2 envs x 64 units.
+constexpr int kSmallUnits = 64, kSmallStages = 4, kSmallThreads = 128;
+template <int N> struct Small {
+    static constexpr int kEnvs = 2 * N * N, kStage = kGruK * (kEnvs + 3 * kSmallUnits);   // floats: x [kGruK][kEnvs], w [kGruK][3][64]
+};
+template <int N>
 __global__ void __launch_bounds__(kSmallThreads)
 k_mingru_small(const float* x_in, const float* __restrict__ Wt, float* __restrict__ state, const float* prev_terminals,
                float* __restrict__ h_out, float* __restrict__ r_state, int r_bf16, int H, int early) {
+    constexpr int kEnvs = Small<N>::kEnvs, kStage = Small<N>::kStage;
     extern __shared__ __align__(16) float sm[];
-    const int tid = threadIdx.x, e = tid / kSmallUnits, u = tid % kSmallUnits;
-    const int e0 = blockIdx.x * kSmallEnvs, u0 = blockIdx.y * kSmallUnits;   // (n is a multiple of 32)
+    const int tid = threadIdx.x, el = tid / (kSmallUnits / N) * N, u = tid % (kSmallUnits / N) * N;   // this lane's first env and unit
+    const int e0 = blockIdx.x * kEnvs, u0 = blockIdx.y * kSmallUnits;   // (n is a multiple of 32)
     const float* wsrc = Wt + (size_t)u0 * 3 * H;
-    constexpr int NW = kGruK * 3 * kSmallUnits / (4 * kSmallThreads);
+    constexpr int NW = kGruK * 3 * kSmallUnits / (4 * kSmallThreads), NX = kGruK * kEnvs / 2;   // pieces of 16 and of 8 bytes
+    static_assert(NX <= kSmallThreads && kEnvs <= 32, "a thread a piece");
     auto copy_w = [&](int c) {
-        float* w = sm + (c % kSmallStages) * kSmallStage + kGruK * kSmallEnvs;
+        float* w = sm + (c % kSmallStages) * kStage + kGruK * kEnvs;
 #pragma unroll
         for (int i = 0; i < NW; i++) {
             const int at = 4 * (i * kSmallThreads + tid);
@@ -603,9 +608,9 @@ k_mingru_small(const float* x_in, const float* __restrict__ Wt, float* __restric
         }
     };
     auto copy_x = [&](int c) {
-        if (tid < kGruK)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(sm + (c % kSmallStages) * kSmallStage + tid * kSmallEnvs)),
-                         "l"(x_in + act_at(e0, c * kGruK + tid, H)) : "memory");
+        if (tid < NX)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(sm + (c % kSmallStages) * kStage + 2 * tid)),
+                         "l"(x_in + act_at(e0 + 2 * tid % kEnvs, c * kGruK + 2 * tid / kEnvs, H)) : "memory");
     };
     if (early & kLaunchNext) launch_next_kernel();
     const int chunks = H / kGruK;
@@ -619,10 +624,16 @@ k_mingru_small(const float* x_in, const float* __restrict__ Wt, float* __restric
         if (c < chunks) copy_x(c);
         copy_commit();
     }
-    const size_t o = (size_t)(e0 + e) * H + u0 + u;
-    float st = state[o];
-    const float ended = prev_terminals != nullptr ? prev_terminals[e0 + e] : 0.0f, x_own = x_in[act_at(e0 + e, u0 + u, H)];
-    float z[3] = {0.0f, 0.0f, 0.0f};
+    float st[N][N], ended[N], x_own[N][N], z[N][N][3] = {};
+#pragma unroll
+    for (int e = 0; e < N; e++) {
+        ended[e] = prev_terminals != nullptr ? prev_terminals[e0 + el + e] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            st[e][i] = state[(size_t)(e0 + el + e) * H + u0 + u + i];
+            x_own[e][i] = x_in[act_at(e0 + el + e, u0 + u + i, H)];
+        }
+    }
     for (int c = 0; c < chunks; c++) {
         copy_wait<kSmallStages - 2>();
         __syncthreads();   // chunk c is complete, and everybody is done with chunk c - 1
@@ -631,23 +642,41 @@ k_mingru_small(const float* x_in, const float* __restrict__ Wt, float* __restric
             copy_x(c + kSmallStages - 1);
         }
         copy_commit();
-        const float* x = sm + (c % kSmallStages) * kSmallStage + e;
-        const float* w = sm + (c % kSmallStages) * kSmallStage + kGruK * kSmallEnvs + u;
+        const float* xs = sm + (c % kSmallStages) * kStage + el;
+        const float* ws = sm + (c % kSmallStages) * kStage + kGruK * kEnvs + u;
+        auto load = [](const float* p, float (&v)[N]) {
+            if constexpr (N == 2) { const float2 f = *reinterpret_cast<const float2*>(p); v[0] = f.x; v[1] = f.y; }
+            else v[0] = *p;
+        };
 #pragma unroll
-        for (int k = 0; k < kGruK; k++)
+        for (int k = 0; k < kGruK; k++) {
+            float x[N], w[N];
+            load(xs + k * kEnvs, x);
 #pragma unroll
-            for (int g = 0; g < 3; g++) z[g] = fmaf(w[(3 * k + g) * kSmallUnits], x[k * kSmallEnvs], z[g]);
+            for (int g = 0; g < 3; g++) {
+                load(ws + (3 * k + g) * kSmallUnits, w);
+#pragma unroll
+                for (int e = 0; e < N; e++)
+#pragma unroll
+                    for (int i = 0; i < N; i++) z[e][i][g] = fmaf(w[i], x[e], z[e][i][g]);
+            }
+        }
     }
-    if (ended != 0.0f) st = 0.0f;
-    if (r_state != nullptr) {   // the post-zero state input
-        if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o] = __float2bfloat16(st);
-        else r_state[o] = st;
-    }
-    const float zh = z[0];
-    sigmoids_ref(z, 3);
-    const float gh = zh >= 0.0f ? zh + 0.5f : z[0], out = st + z[1] * (gh - st);
-    h_out[act_at(e0 + e, u0 + u, H)] = z[2] * out + (1.0f - z[2]) * x_own;
-    state[o] = out;
+#pragma unroll
+    for (int e = 0; e < N; e++)
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const size_t o = (size_t)(e0 + el + e) * H + u0 + u + i;
+            const float s = ended[e] != 0.0f ? 0.0f : st[e][i], zh = z[e][i][0];
+            if (r_state != nullptr) {   // the post-zero state input
+                if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o] = __float2bfloat16(s);
+                else r_state[o] = s;
+            }
+            sigmoids_ref(z[e][i], 3);
+            const float gh = zh >= 0.0f ? zh + 0.5f : z[e][i][0], out = s + z[e][i][1] * (gh - s);
+            h_out[act_at(e0 + el + e, u0 + u + i, H)] = z[e][i][2] * out + (1.0f - z[e][i][2]) * x_own[e][i];
+            state[o] = out;
+        }
 }
 
 // ---------------------------------------------------------------- heads
@@ -938,10 +967,11 @@ static int sm_rounds(int n, int envs, int unit_tiles) { return ((n + envs - 1) /
 // 46.2, in the encoder 38.7, in neither 32.0; 64 envs 47.6, 43.7 and 34.2; 128 envs 49.1 and 44.1; 192 envs 48.7 and 63; 32 envs, hidden 512 73 and 46;
 // 256 envs, hidden 128 38.7 and 35.2; 512 envs, hidden 64 33.4 and 31.1.
 constexpr int kSmallest = 32;
-// A layer.  1 env a lane under q = 96, where even tiles of 4 leave schedulers without a warp (256 envs: 55 against 71 us;
-// 512 envs: 77 against 72).  Blocks of 4 envs a lane take the same time alone and beside each other, those of more envs a little less beside one.
-// Narrow layers have as much to do around the sums as in them, and stay with 4 longer (4,096 envs, hidden 128: 52.9 us, 54.3 with 7; 8,192 78.5
-// and 77.5).
+// A layer.  Tile 1 under q = 96, where even tiles of 4 envs leave schedulers without a warp: 2 envs x 2 units a lane (hidden sizes that are odd multiples
+// of 32: 1 env x 4 units; us a forward, that and 2 x 2: 160 envs, hidden 256 48.2 and 44.5, 256 48.4 and 45.0, 320 71.4 and 62.2, 160 envs, hidden 512
+// 106.3 and 86.7; from q = 96 to 592 2 x 2 and 4 x 4 take the same time).  Blocks of 4 envs a lane take the same time alone and beside each other, those
+// of more envs a little less beside one.  Narrow layers have as much to do around the sums as in them, and stay with 4 longer (4,096 envs, hidden 128:
+// 52.9 us, 54.3 with 7; 8,192 78.5 and 77.5).
 static int strict_tile(int n, int H) {
     const long long q = (long long)n * H / 1024;
     if (q <= kSmallest && H % 64 == 0) return 0;
@@ -1006,13 +1036,14 @@ static int strict_layers(const StrictArgs& a, int early, cudaStream_t st) {
 }
 
 // (H a multiple of 64)
+template <int N>
 static int strict_layers_small(const StrictArgs& a, int early, cudaStream_t st) {
-    constexpr int smem = kSmallStages * kSmallStage * (int)sizeof(float);
-    int rc = allow_smem<k_mingru_small, smem>();
+    constexpr int smem = kSmallStages * Small<N>::kStage * (int)sizeof(float);
+    int rc = allow_smem<k_mingru_small<N>, smem>();
     for (int l = 0; l < a.L && rc == CFX_OK; l++) {
         const size_t at = (size_t)l * a.n * a.H;
         float* r = a.r_state ? reinterpret_cast<float*>(reinterpret_cast<char*>(a.r_state) + at * (a.r_state_bf16 ? 2 : 4)) : nullptr;
-        rc = launch_chained(k_mingru_small, dim3(a.n / kSmallEnvs, a.H / kSmallUnits), kSmallThreads, smem, st, a.scratch_h[l & 1],
+        rc = launch_chained(k_mingru_small<N>, dim3(a.n / Small<N>::kEnvs, a.H / kSmallUnits), kSmallThreads, smem, st, a.scratch_h[l & 1],
                             a.gates_t + (size_t)l * 3 * a.H * a.H, a.state + at, a.prev_terminals, a.scratch_h[(l + 1) & 1], r, a.r_state_bf16,
                             a.H, early);
     }
@@ -1054,8 +1085,8 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     if (H % 64 != 0)
         rc = tm == 8 ? strict_layers<8, 4, 1, 2>(a, early, st) : tm == 4 ? strict_layers<4, 4, 1, 2>(a, early, st)
                                                                          : strict_layers<1, 4, 1, 4>(a, early, st);
-    else if (tm == 0) rc = strict_layers_small(a, early, st);
-    else if (tm == 1) rc = strict_layers<1, 2, 2, 4>(a, early, st);
+    else if (tm == 0) rc = strict_layers_small<1>(a, early, st);
+    else if (tm == 1) rc = strict_layers_small<2>(a, early, st);
     else if (tm == 4) rc = q <= 592 ? strict_layers<4, 2, 2, 3>(a, early, st) : strict_layers<4, 2, 2, 2>(a, early, st);
     else rc = tm == 5 ? strict_layers<5, 2, 2, 2>(a, early, st) : tm == 6 ? strict_layers<6, 2, 2, 2>(a, early, st)
               : tm == 7 ? strict_layers<7, 2, 2, 2>(a, early, st) : tm == 8 ? strict_layers<8, 2, 2, 2>(a, early, st)

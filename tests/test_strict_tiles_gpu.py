@@ -74,9 +74,10 @@ def test_strict_heights_match_the_oracle(cfx, gpu, oracle, n, H, L):
     test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L)
 
 
-@pytest.mark.parametrize("n,H,L", [(32, 64, 4), (64, 512, 1), (128, 256, 2), (160, 192, 1), (96, 96, 2), (160, 256, 1)])
+@pytest.mark.parametrize("n,H,L", [(32, 64, 4), (64, 512, 1), (128, 256, 2), (160, 192, 1), (96, 96, 2), (160, 256, 2), (352, 256, 1), (160, 512, 1)])
 def test_smallest_strict_batches_match_the_oracle(cfx, gpu, oracle, n, H, L):
-    """One sum a lane, up to the last size that takes it, and hidden sizes for which only the encoder does."""
+    """One sum a lane, then two envs x two units in the layers, up to the last sizes that take them, and hidden sizes for which only
+    the encoder does."""
     test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L)
 
 
