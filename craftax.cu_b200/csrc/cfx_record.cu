@@ -52,6 +52,7 @@ struct Params {
 };
 // The view in a plane: nine rows of eleven bytes, 48 apart, so 395 bytes from the first to the last, in 26 pieces of 16
 constexpr int kPlanes = 3, kSpan = kRows * kMapSize, kPieces = 26;
+constexpr int kRowWords = (3 + kCols + 3) / 4;   // that a view row lies in
 static_assert(15 + (kRows - 1) * kMapSize + kCols <= 16 * kPieces && 16 * kPieces <= kSpan && kPieces <= 32, "a lane a piece");
 constexpr int kWarps = kBlockThreads / 32, kOwn = kBlockEnvs / kWarps;   // envs whose records a warp writes
 constexpr int kPlaneBytes = kMapSize * kMapSize, kRecWords = kRec / 4, kMapWords = kMap / 4;
@@ -279,7 +280,7 @@ struct CopyLane {
     int lane;
     __device__ __forceinline__ explicit CopyLane(int l) : lane(l) {}
     // Planes that are not aligned to words: a lane takes every 32nd cell of the view, its bytes of the three planes all in flight
-    // (65,536 envs 59 us with a byte load per cell and map and nothing else, 75 with the bytes of a row one after the other)
+    // (65,536 envs 55 us; 75 with the bytes of a row one after the other)
     __device__ __forceinline__ void bytes(const cfx_env_view& V, int e, View v, uint8_t* dst) const {
         constexpr int kCells = kRows * kCols, kRounds = (kCells + 31) / 32;
         const uint64_t off[kPlanes] = {V.light_map_offset, V.map_offset, V.item_map_offset};
@@ -302,7 +303,8 @@ struct CopyLane {
     }
     // Starts the copies of env e's view into `dst`: where the planes are aligned to 16 bytes, the pieces of a plane's span side by
     // side, an instruction a plane (what lies between the view's rows comes along: memory is read in bursts of 64 bytes anyway);
-    // else words, a lane a row of a plane.
+    // else the words that the view's rows lie in, four lanes a row (eight rows are 32 banks).  Words, us: a lane a row, its words one instruction
+    // after the other, 65,536 envs 50.7, 1,000 5.51, a list of all envs 55.8; so 48.9, 5.37, 54.4.  Bytes: 55.1, 6.39, 74.2.
     template <bool BYTES>
     __device__ __forceinline__ void start(const cfx_env_view& V, int e, View v, int grain, uint8_t* dst) const {
         if constexpr (BYTES) return bytes(V, e, v, dst);
@@ -316,12 +318,16 @@ struct CopyLane {
             for (int p = 0; p < kPlanes; p++)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + p * kSpan + 16 * lane)), "l"(q + off[p] + at) : "memory");
         } else {
-            const int plane = lane / kRows, dr = lane % kRows, row = v.top() + dr;
-            if (plane >= kPlanes || (unsigned)row >= (unsigned)kMapSize) return;
-            const uint8_t* src = q + (plane == 0 ? off[0] : plane == 1 ? off[1] : off[2]) + row * kMapSize + c0;
-            for (int o = 0; o < 32; o += 4)   // the view's columns, and only those on the map
-                if (c0 + o >= 0 && c0 + o < min(left + kCols, kMapSize) && c0 + o + 4 > left)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + plane * kSpan + row_byte(dr, o))), "l"(src + o) : "memory");
+            static_assert(kRowWords == 4 && kRows == 9, "eight rows an instruction, and the last one of the three planes");
+            const int o = (left & 12) + 4 * (lane & 3), col = c0 + o, dr = lane >> 2, row = v.top() + dr, last = v.top() + 8;
+            if ((unsigned)col >= (unsigned)kMapSize || col >= left + kCols) return;
+            auto word = [&](int p, uint64_t plane, int r, int at) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + p * kSpan + row_byte(r, o))), "l"(q + plane + (at * kMapSize + col)) : "memory");
+            };
+            if ((unsigned)row < (unsigned)kMapSize)
+#pragma unroll
+                for (int p = 0; p < kPlanes; p++) word(p, off[p], dr, row);
+            if (dr < kPlanes && (unsigned)last < (unsigned)kMapSize) word(dr, dr == 0 ? off[0] : dr == 1 ? off[1] : off[2], 8, last);
         }
     }
 };
@@ -540,8 +546,8 @@ union ListMemory {
     ListBlock block;
 };
 static_assert(sizeof(ListMemory) <= 48 * 1024, "static shared memory");
-// Lists of more entries than this for each warp of the grid go by blocks.  65,536 envs, 2,368 warps, us by warps / by blocks:
-// 2,368 entries 5.0 / 8.7, 4,736 8.0 / 9.2, 7,104 11.0 / 9.5, 16,384 29 / 13, all of them 135 / 53.
+// Lists of more entries than this for each warp of the grid go by blocks.  65,536 envs, 2,368 warps, random lists in three sets of buffers, us by warps /
+// by blocks: 250 entries 4.1 / 8.0, 2,368 5.8 / 9.7, 4,736 11.8 / 11.8, 7,104 17.1 / 13.9, 16,384 33.4 / 18.6, all of them 119 / 52.
 constexpr int kListPerWarp = 2;
 
 // 32 entries of the list from `base` on, lane = entry in the loads of the fields, a warp four envs at a time in the rest

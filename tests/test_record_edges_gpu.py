@@ -60,6 +60,22 @@ def test_record_rows_at_edges(cfx, gpu, oracle, n, shift, pad, rec_shift):
     del keep
 
 
+@pytest.mark.parametrize("shift", [0, 4, 1])
+def test_record_rows_at_every_column(cfx, gpu, oracle, shift):
+    """Every column of the player, on, beside and off the map, so every alignment of a view's rows to words and to 16 bytes."""
+    rows, cols = np.meshgrid([-5, 0, 3, 24, 44, 47, 52], np.arange(-7, 56), indexing="ij")
+    n = rows.size
+    st = oracle.synthetic_env_state(n, seed=5)
+    st["player_position"][:] = np.stack([rows.ravel(), cols.ravel()])
+    st["mob_position"][:] = (st["player_position"][None] + np.random.default_rng(shift).integers(-6, 7, (135, 2, n))).reshape(270, n)
+    view, keep = _view(cfx, st, shift, 0)
+    rec = cfx.DeviceBuffer((n, 996), np.uint8)
+    cfx.record_obs(view, rec)
+    cfx.check(cfx.lib().cfx_stream_sync(0, None))
+    assert np.array_equal(rec.download(), oracle.record_from_state(st))
+    del keep
+
+
 CLASSIC_FIELDS = (("player_r", "i2", 1), ("player_c", "i2", 1), ("player_dir", "i1", 1), ("health", "i1", 1), ("food", "i1", 1),
                   ("drink", "i1", 1), ("energy", "i1", 1), ("is_sleeping", "u1", 1), ("inv", "i1", 12),
                   ("zombie_r", "i2", 3), ("zombie_c", "i2", 3), ("zombie_mask", "u1", 3), ("cow_r", "i2", 3),
