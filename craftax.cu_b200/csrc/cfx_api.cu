@@ -513,6 +513,13 @@ extern "C" int cfx_selftest_wait_timeout(int device, unsigned limit_ms) {
     return CFX_ERR_DEVICE_TIMEOUT;
 }
 
+extern "C" int cfx_selftest_reciprocals(int device, uint32_t first, uint32_t last, uint32_t far, uint64_t* differing) {
+    CFX_REQUIRE(differing, "cfx_selftest_reciprocals: NULL argument");
+    CFX_REQUIRE(first >= 0x3F800000u && first <= last && last <= 0x7FFFFFFFu, "cfx_selftest_reciprocals: bits %x .. %x", first, last);
+    CFX_GUARD(device);
+    return selftest_reciprocals(first, last, far, differing);
+}
+
 // ------------------------------------------------------------------ host-buffer forward
 template <typename T>
 static int ensure_staging(T** slot, size_t count) {

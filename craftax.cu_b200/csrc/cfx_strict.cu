@@ -19,6 +19,8 @@
 
 namespace cfx {
 
+constexpr int kSMs = 148;
+
 // ---------------------------------------------------------------- expand
 // features[e][f] = (float)rec[e][f] for f < 792, raw fp32 bits for the tail
 // (k_expand_obs, craftax_full.cu:10028-10053).  One thread per output element;
@@ -377,6 +379,59 @@ __global__ void k_done_to_terminals(const int8_t* __restrict__ done, float* __re
 }
 
 // ---------------------------------------------------------------- MinGRU layer
+// d[i] = 1.0f / d[i] for d >= 1, n values at once (n is a constant once unrolled).  The compiler's correctly rounded division has a branch, so
+// sigmoids written one by one run one after the other, about 150 cycles each: the 96 of a lane took half as long as a lone block's sums
+// at hidden 256.  Here the reciprocals are refined without a branch, by a Newton step with the remainder in one FMA (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).  That this rounds correctly depends on the
+// approximation that it starts from: k_selftest_reciprocals compares all values up to 2^126 with the division.  Beyond, and for infinity, where
+// the reciprocal is subnormal or zero, the batch is divided.
+constexpr int kReciprocals = 12;   // of a batch in the wide layers: three gates of four envs
+template <int N> __device__ __forceinline__ void reciprocals(float (&d)[N], int n) {
+    float r[N], most = 1.0f;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        if (i >= n) break;
+        float a;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(d[i]));
+        r[i] = fmaf(a, fmaf(-d[i], a, 1.0f), a);
+        most = fmaxf(most, d[i]);
+    }
+    if (most > 0x1p126f)
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if (i < n) r[i] = 1.0f / d[i];
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (i < n) d[i] = r[i];
+}
+// Denominators with the bits first .. last, in batches as the layers have them; where `far` is not zero it is the last of every batch.  Counts
+// those whose reciprocal is not 1.0f / d.
+__global__ void k_selftest_reciprocals(uint32_t first, uint32_t last, uint32_t far, unsigned long long* differing) {
+    const uint32_t own = far != 0u ? kReciprocals - 1 : kReciprocals, stride = gridDim.x * blockDim.x;
+    const uint32_t batches = (last - first) / own + 1;
+    unsigned long long bad = 0;
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < batches; b += stride) {
+        float d[kReciprocals], r[kReciprocals];
+#pragma unroll
+        for (uint32_t i = 0; i < kReciprocals; i++)
+            r[i] = d[i] = __uint_as_float(i < own ? min(first + b * own + i, last) : far);
+        reciprocals(r, kReciprocals);
+#pragma unroll
+        for (int i = 0; i < kReciprocals; i++) {
+            const float want = 1.0f / d[i];
+            if (__float_as_uint(r[i]) != __float_as_uint(want) && !(r[i] != r[i] && want != want)) bad++;
+        }
+    }
+    if (bad != 0) atomicAdd(differing, bad);
+}
+// N values 1 / (1 + exp(-z)) at once
+template <int N> __device__ __forceinline__ void sigmoids_ref(float (&z)[N], int n) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (i < n) z[i] = 1.0f + expf(-z[i]);
+    reciprocals(z, n);
+}
+
 // One layer: gate dots (ascending j, fmaf) + cell (k_mingru_epi_fwd, craftax_full.cu:9350-9395).
 // Wt is the layer's gate matrix as k_transpose_gates lays it out, x_in and h_out activations.  K chunks of 32; ST buffers:
 // two where several blocks share an SM, more for small batches, which wait for the loads (chunks of 16 with three: 155 against
@@ -385,31 +440,6 @@ __global__ void k_done_to_terminals(const int8_t* __restrict__ done, float* __re
 // a lane and more keep everything in registers (three: 160 bytes of spills, 142 against 136 us at 4,096 envs).  us a forward, before the cell's loads and
 // divisions were taken out of their chains and the heights followed the number of blocks, and now: 4,096 envs, hidden 256, depth 2 146.9 and 123.7;
 // 5,120 222.1 and 153.9; 1,024 66.1 and 58.8; 8,192 envs, hidden 512, depth 3 887 and 827.
-// N values 1 / (1 + exp(-z)) at once.  The compiler's correctly rounded division has a branch, so sigmoids written one by one run
-// one after the other, about 150 cycles each: the 96 of a lane took half as long as a lone block's sums at hidden 256.
-// Here the reciprocals are refined without a branch, by a Newton step with the remainder in one FMA (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): the same bits as 1.0f / d for each of the
-// 1.06e9 values d in [1, 2^126].  Beyond, the batch is divided.
-// (n is a constant once unrolled)
-template <int N> __device__ __forceinline__ void sigmoids_ref(float (&z)[N], int n) {
-    float d[N], most = 1.0f;
-#pragma unroll
-    for (int i = 0; i < N; i++)
-        if (i < n) d[i] = 1.0f + expf(-z[i]);
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        if (i >= n) break;
-        float r;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d[i]));
-        z[i] = fmaf(r, fmaf(-d[i], r, 1.0f), r);
-        most = fmaxf(most, d[i]);
-    }
-    if (most > 0x1p126f)
-#pragma unroll
-        for (int i = 0; i < N; i++)
-            if (i < n) z[i] = 1.0f / d[i];
-}
-
 constexpr int kGruK = 32;
 template <int TM, int WM, int WU> constexpr int gru_stage_floats() { return kGruK * (4 * TM * WM + 3 * 32 * WU); }
 
@@ -956,12 +986,25 @@ int launch_init_uniform(float* w, int count, float bound, uint64_t seed, int sub
     return CFX_OK;
 }
 
+int selftest_reciprocals(uint32_t first, uint32_t last, uint32_t far, uint64_t* differing) {
+    unsigned long long* count = nullptr;
+    CFX_CUDA(cudaMalloc((void**)&count, sizeof(*count)));
+    cudaError_t e = cudaMemset(count, 0, sizeof(*count));
+    if (e == cudaSuccess) {
+        k_selftest_reciprocals<<<8 * kSMs, 256>>>(first, last, far, count);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(differing, count, sizeof(*count), cudaMemcpyDeviceToHost);
+    cudaFree(count);
+    CFX_CUDA(e);
+    return CFX_OK;
+}
+
 // The tiles.  What a forward costs is the number of blocks that the fullest SM has one after the other, so the envs of a lane, TM, are
 // those for which that number times the time of a block is the least; both are estimated from what blocks of each height take
 // alone and two to an SM.  (Before, 8 envs a lane from q = n H / 1024 = 1,024 warps on, else 4: at 4,096 envs and hidden 256 that left 40
 // SMs with half of the others' layers, and 24 with three times at 5,120.  The times of all heights were measured at 26 sizes from 512 envs
 // to 16,384, hidden 64 to 512: this choice is the best at all of them in the encoder, and within 1 % of it in the layers.)
-constexpr int kSMs = 148;
 static int sm_rounds(int n, int envs, int unit_tiles) { return ((n + envs - 1) / envs * unit_tiles + kSMs - 1) / kSMs; }
 // Up to q = 32 a lane has one sum, or one of each gate (tile 0): us a forward of 32 envs, hidden 256, depth 2, with 4 units a lane in both kernels
 // 46.2, in the encoder 38.7, in neither 32.0; 64 envs 47.6, 43.7 and 34.2; 128 envs 49.1 and 44.1; 192 envs 48.7 and 63; 32 envs, hidden 512 73 and 46;

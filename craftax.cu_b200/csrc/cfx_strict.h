@@ -44,6 +44,8 @@ int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, fl
 int launch_fetch(const void* host, void* dst, size_t bytes, cudaStream_t st);
 int launch_bump(unsigned long long* ctr, cudaStream_t st);
 int launch_transpose_gates(const float* W, float* Wt, int H, int L, cudaStream_t st);
+// counts the batches' reciprocals that are not 1.0f / d (see k_selftest_reciprocals); waits for the device
+int selftest_reciprocals(uint32_t first, uint32_t last, uint32_t far, uint64_t* differing);
 int launch_init_uniform(float* w, int count, float bound, uint64_t seed, int subseq, cudaStream_t st);
 
 }  // namespace cfx

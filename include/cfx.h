@@ -182,6 +182,12 @@ int cfx_policy_check(cfx_policy* p, void* stream);
  * stays usable. */
 int cfx_selftest_wait_timeout(int device, unsigned limit_ms);
 
+/* Self-test of the fp32 mode's sigmoids (no reference counterpart): *differing is how many of the
+ * reciprocals of the floats with the bit patterns first .. last (not below 1.0f), taken in batches as
+ * the layers take them, are not what the division 1.0f / d gives; where `far` is not zero, the float
+ * with that pattern is in every batch. */
+int cfx_selftest_reciprocals(int device, uint32_t first, uint32_t last, uint32_t far, uint64_t* differing);
+
 /* Same forward with HOST buffers (pinned for full copy speed): copies
  * records/prev_terminals/uniforms to handle-owned device staging, runs
  * cfx_policy_forward, copies every non-NULL output back and synchronises.
