@@ -431,8 +431,15 @@ template <int N> __device__ __forceinline__ void sigmoids_ref(float (&z)[N], int
         if (i < n) z[i] = 1.0f + expf(-z[i]);
     reciprocals(z, n);
 }
+// The cell of an env and unit (k_mingru_epi_fwd, craftax_full.cu:9350-9395): zh is the first gate's sum, s[0 .. 2] the sigmoids of all three, x the layer's
+// input, state is replaced; returns the layer's output.  One place for all layer kernels, whose batches must give the same bits.
+__device__ __forceinline__ float cell(float zh, const float* s, float x, float& state) {
+    const float gh = zh >= 0.0f ? zh + 0.5f : s[0];
+    state = state + s[1] * (gh - state);
+    return s[2] * state + (1.0f - s[2]) * x;
+}
 
-// One layer: gate dots (ascending j, fmaf) + cell (k_mingru_epi_fwd, craftax_full.cu:9350-9395).
+// One layer: gate dots (ascending j, fmaf) + cell.
 // Wt is the layer's gate matrix as k_transpose_gates lays it out, x_in and h_out activations.  K chunks of 32; ST buffers:
 // two where several blocks share an SM, more for small batches, which wait for the loads (chunks of 16 with three: 155 against
 // 152 us a forward at 4,096 envs, 970 against 944 us at 8,192 envs with hidden 512, depth 3); the k loop has to be unrolled
@@ -592,10 +599,7 @@ k_mingru_fp32(const float* x_in, const float* __restrict__ Wt, float* __restrict
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 if (e >= count) break;
-                const float gh = zh[e] >= 0.0f ? zh[e] + 0.5f : s[3 * e], p = s[3 * e + 2];
-                const float out = st[b][e][u] + s[3 * e + 1] * (gh - st[b][e][u]);
-                h[e] = p * out + (1.0f - p) * x[b][u][e];
-                st[b][e][u] = out;
+                h[e] = cell(zh[e], s + 3 * e, x[b][u][e], st[b][e][u]);
             }
             store_envs(h_out + act_at(env, u0 + ul + u, H), h, count);
         }
@@ -697,15 +701,15 @@ k_mingru_small(const float* x_in, const float* __restrict__ Wt, float* __restric
 #pragma unroll
         for (int i = 0; i < N; i++) {
             const size_t o = (size_t)(e0 + el + e) * H + u0 + u + i;
-            const float s = ended[e] != 0.0f ? 0.0f : st[e][i], zh = z[e][i][0];
+            float s = ended[e] != 0.0f ? 0.0f : st[e][i];
+            const float zh = z[e][i][0];
             if (r_state != nullptr) {   // the post-zero state input
                 if (r_bf16) reinterpret_cast<__nv_bfloat16*>(r_state)[o] = __float2bfloat16(s);
                 else r_state[o] = s;
             }
             sigmoids_ref(z[e][i], 3);
-            const float gh = zh >= 0.0f ? zh + 0.5f : z[e][i][0], out = s + z[e][i][1] * (gh - s);
-            h_out[act_at(e0 + el + e, u0 + u + i, H)] = z[e][i][2] * out + (1.0f - z[e][i][2]) * x_own[e][i];
-            state[o] = out;
+            h_out[act_at(e0 + el + e, u0 + u + i, H)] = cell(zh, z[e][i], x_own[e][i], s);
+            state[o] = s;
         }
 }
 

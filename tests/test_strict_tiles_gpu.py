@@ -97,3 +97,22 @@ def test_strict_saturated_gates(cfx, gpu, oracle, n, H):
     _close(d["logits_av"], lav)
     _close(pol.get_state(), st)
     pol.close()
+
+
+@pytest.mark.parametrize("H", [256, 96])   # (96: the layers' warps along the envs)
+def test_batches_of_any_size_give_the_same_bits(cfx, gpu, oracle, H):
+    """An env's results do not depend on which tiles its batch takes."""
+    rec, params, state, prev_t, u = _inputs(oracle, 4128, H, 2)
+
+    def run(n):
+        pol = cfx.Policy(n, H, 2, A, "fp32")
+        pol.set_weights(params)
+        pol.set_state(np.ascontiguousarray(state[:, :n]))
+        d = dict(pol.forward_host(rec[:n], prev_t[:n], u[:n], want_r_state=True), state=pol.get_state())
+        pol.close()
+        return {k: v[:, :32] if k in ("state", "r_state") else v[:32] for k, v in d.items()}
+    want = run(4128)
+    for n in (32, 160, 416, 1248, 1568, 2592):
+        got = run(n)
+        for k in want:
+            assert np.array_equal(got[k], want[k]), (n, k)
