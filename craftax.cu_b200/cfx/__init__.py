@@ -84,6 +84,7 @@ _SIGS = {
     "cfx_policy_check": (C.c_int, [C.c_void_p, C.c_void_p]),
     "cfx_selftest_wait_timeout": (C.c_int, [C.c_int, C.c_uint]),
     "cfx_selftest_reciprocals": (C.c_int, [C.c_int, C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(C.c_uint64)]),
+    "cfx_selftest_strict_tiles": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_int32)]),
     "cfx_strict_forward_static": (C.c_int, [C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
                                             C.c_void_p, C.POINTER(ForwardIO), C.c_void_p, C.c_void_p]),
     "cfx_classic_param_count": (C.c_size_t, [C.c_int] * 3),

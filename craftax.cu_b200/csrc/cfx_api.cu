@@ -520,6 +520,13 @@ extern "C" int cfx_selftest_reciprocals(int device, uint32_t first, uint32_t las
     return selftest_reciprocals(first, last, far, differing);
 }
 
+extern "C" int cfx_selftest_strict_tiles(int num_envs, int hidden, int32_t* tiles) {
+    CFX_REQUIRE(tiles && num_envs > 0 && num_envs % 32 == 0 && hidden > 0 && hidden % 32 == 0 && hidden <= kMaxHidden,
+                "cfx_selftest_strict_tiles: %d envs, hidden %d", num_envs, hidden);
+    strict_tiles(num_envs, hidden, tiles, tiles + 1, tiles + 2, tiles + 3);
+    return CFX_OK;
+}
+
 // ------------------------------------------------------------------ host-buffer forward
 template <typename T>
 static int ensure_staging(T** slot, size_t count) {

@@ -1009,6 +1009,10 @@ int selftest_reciprocals(uint32_t first, uint32_t last, uint32_t far, uint64_t* 
 // alone and two to an SM.  (Before, 8 envs a lane from q = n H / 1024 = 1,024 warps on, else 4: at 4,096 envs and hidden 256 that left 40
 // SMs with half of the others' layers, and 24 with three times at 5,120.  The times of all heights were measured at 26 sizes from 512 envs
 // to 16,384, hidden 64 to 512: this choice is the best at all of them in the encoder, and within 1 % of it in the layers.)
+// What each height is for, us a forward with all of them and without it: layers, 5 (2,944 envs, hidden 256, depth 2) 98.7 and 103.9, 6 (1,760) 78.0 and 84.0,
+// 7 (4,096) 123.6 and 128.1, 8 (8,192, hidden 512, depth 3) 827 and 864, 9 (2,656, hidden 512) 222 and 249; encoder, depth 1, 5 (11,840, hidden 128) 102.7
+// and 107.9, 6 (14,208, hidden 192) 181.9 and 200.0, 7 (16,384, hidden 256) 291.7 and 303.3, 8 (9,472) 167.9 and 181.9, 9 (10,656, hidden 128) 94.1 and
+// 100.3, although with 9 a lane spills 28 or 36 bytes (128 registers, two blocks of 256 threads an SM).
 static int sm_rounds(int n, int envs, int unit_tiles) { return ((n + envs - 1) / envs * unit_tiles + kSMs - 1) / kSMs; }
 // Up to q = 32 a lane has one sum, or one of each gate (tile 0): us a forward of 32 envs, hidden 256, depth 2, with 4 units a lane in both kernels
 // 46.2, in the encoder 38.7, in neither 32.0; 64 envs 47.6, 43.7 and 34.2; 128 envs 49.1 and 44.1; 192 envs 48.7 and 63; 32 envs, hidden 512 73 and 46;
@@ -1049,6 +1053,16 @@ static EncoderTile strict_encoder_tile(int n, int H) {
     for (int tm = 5; tm <= 9; tm++)
         if (sm_rounds(n, 16 * tm / wu, H / (64 * wu)) * (tm + 2) < sm_rounds(n, 16 * best / wu, H / (64 * wu)) * (best + 2)) best = tm;
     return {best, 2};
+}
+
+// Layers with 4 envs a lane: three stages of weights where few blocks share an SM
+static bool strict_deep(int n, int H) { return (long long)n * H / 1024 <= 592; }
+void strict_tiles(int n, int H, int* layer, int* deep, int* encoder, int* groups) {
+    const EncoderTile te = strict_encoder_tile(n, H);
+    *layer = strict_tile(n, H);
+    *deep = *layer == 4 && H % 64 == 0 && strict_deep(n, H);
+    *encoder = te.tm;
+    *groups = te.g;
 }
 
 template <int TM, int G, int WU, int UL = 4>
@@ -1134,7 +1148,7 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
                                                                          : strict_layers<1, 4, 1, 4>(a, early, st);
     else if (tm == 0) rc = strict_layers_small<1>(a, early, st);
     else if (tm == 1) rc = strict_layers_small<2>(a, early, st);
-    else if (tm == 4) rc = q <= 592 ? strict_layers<4, 2, 2, 3>(a, early, st) : strict_layers<4, 2, 2, 2>(a, early, st);
+    else if (tm == 4) rc = strict_deep(n, H) ? strict_layers<4, 2, 2, 3>(a, early, st) : strict_layers<4, 2, 2, 2>(a, early, st);
     else rc = tm == 5 ? strict_layers<5, 2, 2, 2>(a, early, st) : tm == 6 ? strict_layers<6, 2, 2, 2>(a, early, st)
               : tm == 7 ? strict_layers<7, 2, 2, 2>(a, early, st) : tm == 8 ? strict_layers<8, 2, 2, 2>(a, early, st)
                                                                          : strict_layers<9, 2, 2, 2>(a, early, st);

@@ -28,6 +28,9 @@ struct StrictArgs {
     int weights_ready = 0;  // nothing queued on the stream writes params or gates_t
 };
 
+// what the rules choose for n envs: envs a lane of the layers (0: one sum a gate), three stages or two where that is 4; envs a lane
+// of the encoder (0: one sum) and its groups of four units
+void strict_tiles(int n, int H, int* layer, int* deep, int* encoder, int* groups);
 int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches);
 int launch_expand(const uint8_t* rec, float* out, int n, cudaStream_t st);
 int launch_classic_expand(const uint8_t* rec, float* out, int n, cudaStream_t st);

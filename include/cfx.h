@@ -188,6 +188,11 @@ int cfx_selftest_wait_timeout(int device, unsigned limit_ms);
  * with that pattern is in every batch. */
 int cfx_selftest_reciprocals(int device, uint32_t first, uint32_t last, uint32_t far, uint64_t* differing);
 
+/* Which tiles the fp32 mode takes for a batch (no GPU is needed), so that tests can tell whether they reach
+ * all of them: tiles[0] envs a lane in the layers (0: one sum of each gate), [1] whether layers with 4
+ * have three stages of weights, [2] envs a lane in the encoder (0: one sum), [3] groups of four units there. */
+int cfx_selftest_strict_tiles(int num_envs, int hidden, int32_t* tiles);
+
 /* Same forward with HOST buffers (pinned for full copy speed): copies
  * records/prev_terminals/uniforms to handle-owned device staging, runs
  * cfx_policy_forward, copies every non-NULL output back and synchronises.

@@ -1,5 +1,9 @@
-"""Every tile shape of the fp32 layer kernels against the CPU oracle, at batch sizes that end inside
-a tile, and the allocation-free variant on arrays that are only 4-byte aligned."""
+"""Every tile shape of the fp32 kernels against the CPU oracle, at batch sizes that end inside
+a tile, and the allocation-free variant on arrays that are only 4-byte aligned.
+
+The cases: (n, hidden, layers) and the tiles that the library takes for them, as cfx_selftest_strict_tiles gives them: envs
+a lane of the layers (0: one sum a gate), whether with 4 they have three stages; envs a lane of the encoder (0: one
+sum) and its groups of four units.  (tests/test_strict_tiles.py: that they are so, and that none is missing.)"""
 import ctypes as C
 
 import numpy as np
@@ -22,12 +26,25 @@ def _close(got, want):
     assert np.abs(got - want).max() < 3e-5 * max(1.0, np.abs(want).max())
 
 
-@pytest.mark.parametrize("n,H,L", [(32, 32, 1),       # 1 env a lane, one unit tile
-                                   (416, 256, 1),     # 4 envs a lane (warps of q = 104)
-                                   (1632, 256, 2),    # encoder 4 x 2
-                                   (2592, 256, 1),    # encoder 8 x 2, ragged
-                                   (4128, 256, 2),    # 8 envs a lane, ragged
-                                   (1056, 96, 2), (11040, 96, 1)])   # warps along the envs
+TILES = {
+    (32, 32, 1): (1, 0, 0, 1),                                      # one unit tile
+    (416, 256, 1): (4, 1, 4, 1), (1632, 256, 2): (6, 0, 4, 2),
+    (2592, 256, 1): (9, 0, 5, 2), (4128, 256, 2): (7, 0, 7, 2),     # the last blocks of the encoder are not full
+    (1056, 96, 2): (4, 0, 4, 1), (11040, 96, 1): (8, 0, 4, 1)}      # odd multiples of 32: the layers' warps along the envs
+HEIGHTS = {
+    (1248, 256, 1): (5, 0, 4, 2), (1568, 256, 1): (6, 0, 4, 2), (2048, 256, 2): (7, 0, 4, 2), (2272, 256, 1): (8, 0, 4, 2),
+    (2528, 256, 1): (9, 0, 5, 2),
+    (1248, 512, 1): (9, 0, 5, 2), (1504, 512, 1): (6, 0, 6, 2), (1760, 512, 1): (6, 0, 6, 2), (2272, 512, 1): (8, 0, 8, 2),
+    (2528, 512, 1): (9, 0, 9, 2),
+    # odd multiples of 64: the encoder's warps along the envs
+    (3872, 192, 1): (4, 0, 5, 2), (5408, 192, 1): (4, 0, 7, 2),
+    (4768, 64, 1): (4, 1, 4, 2), (11872, 64, 1): (4, 0, 6, 2), (5536, 192, 1): (8, 0, 8, 2), (6304, 192, 1): (4, 0, 9, 2)}
+SMALLEST = {
+    (32, 64, 4): (0, 0, 0, 1), (64, 512, 1): (0, 0, 0, 1), (128, 256, 2): (0, 0, 0, 1), (160, 192, 1): (0, 0, 0, 1),
+    (96, 96, 2): (1, 0, 0, 1), (160, 256, 2): (1, 0, 1, 1), (352, 256, 1): (1, 0, 1, 1), (160, 512, 1): (1, 0, 1, 1)}
+
+
+@pytest.mark.parametrize("n,H,L", TILES)
 def test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L):
     rec, params, state, prev_t, u = _inputs(oracle, n, H, L)
     pol = cfx.Policy(n, H, L, A, "fp32")
@@ -66,15 +83,13 @@ def test_static_forward_takes_arrays_of_any_word_alignment(cfx, gpu, oracle):
     _close(d_st.download()[1:].reshape(st.shape), st)
 
 
-@pytest.mark.parametrize("n,H,L", [(1248, 256, 1), (1568, 256, 1), (2048, 256, 2), (2272, 256, 1), (2528, 256, 1),   # layers 5 to 9
-                                   (1248, 512, 1), (1504, 512, 1), (1760, 512, 1), (2272, 512, 1), (2528, 512, 1),   # encoder 5 to 9
-                                   (3872, 192, 1), (5408, 192, 1)])   # encoder 5 and 7, its warps along the envs
+@pytest.mark.parametrize("n,H,L", HEIGHTS)
 def test_strict_heights_match_the_oracle(cfx, gpu, oracle, n, H, L):
     """Heights that are no multiple of four envs a lane, and batches that end inside a block."""
     test_strict_tiles_match_the_oracle(cfx, gpu, oracle, n, H, L)
 
 
-@pytest.mark.parametrize("n,H,L", [(32, 64, 4), (64, 512, 1), (128, 256, 2), (160, 192, 1), (96, 96, 2), (160, 256, 2), (352, 256, 1), (160, 512, 1)])
+@pytest.mark.parametrize("n,H,L", SMALLEST)
 def test_smallest_strict_batches_match_the_oracle(cfx, gpu, oracle, n, H, L):
     """One sum a lane, then two envs x two units in the layers, up to the last sizes that take them, and hidden sizes for which only
     the encoder does."""
