@@ -31,14 +31,22 @@ def _forward(cfx, n, H, L, prec, game, rec, params, state, prev_t, r_state, laun
 
 
 @pytest.mark.parametrize("n,H,L,prec,game,r_state", [
-    (32, 256, 1, "f16", "full", "fp32"), (96, 256, 4, "bf16", "full", "bf16"),      # tiles of 32 rows
-    (1184, 256, 2, "f16", "full", None), (1216, 256, 2, "f16", "full", "fp32"),     # 37 tiles of 32; then of 64
-    (2336, 256, 3, "bf16", "full", "bf16"), (2400, 256, 2, "f16", "full", None),    # the last one half empty; of 128
-    (4704, 256, 4, "f16", "full", "fp32"), (4768, 256, 2, "f16", "full", "bf16"),   # clusters of four, of two
-    (9472, 256, 3, "f16", "full", "fp32"), (9504, 256, 1, "f16", "full", None),     # the last of them; one CTA a tile
+    # four CTAs a tile: 32 rows to 1,056 envs, 64 to 2,112, and to 4,224 128 where the state is recorded
+    (32, 256, 1, "f16", "full", "fp32"), (96, 256, 4, "bf16", "full", "bf16"),
+    (1184, 256, 2, "f16", "full", None), (1216, 256, 2, "f16", "full", "fp32"),
+    (2336, 256, 3, "bf16", "full", "bf16"), (2400, 256, 2, "f16", "full", None),    # (the second: two CTAs, 64 rows)
+    # two CTAs a tile: 64 rows to 4,736, 128 to 9,472; then the persistent kernel
+    (4704, 256, 4, "f16", "full", "fp32"), (4768, 256, 2, "f16", "full", "bf16"),
+    (9472, 256, 3, "f16", "full", "fp32"), (9504, 256, 1, "f16", "full", None),
+    # hidden 128, two CTAs: 32 rows to 2,368, 64 to 4,736, 128 to 9,472
     (64, 128, 2, "f16", "full", "bf16"), (2368, 128, 1, "bf16", "full", "fp32"), (2400, 128, 3, "bf16", "full", "fp32"), (9440, 128, 4, "f16", "full", None),
+    # the classic game, as hidden 256: tiles of 32, 64, two CTAs with 64 and with 128
     (160, 256, 3, "f16", "classic", None), (1152, 256, 2, "bf16", "classic", "bf16"), (4736, 256, 2, "bf16", "classic", "fp32"),
-    (9376, 256, 3, "f16", "classic", "bf16")])
+    (9376, 256, 3, "f16", "classic", "bf16"),
+    # without a record, both sides of the limits between four CTAs and two, and of 64 and 128 rows
+    (2112, 256, 2, "f16", "full", None), (2144, 256, 3, "bf16", "full", None), (3232, 256, 1, "f16", "full", None), (4224, 256, 3, "f16", "full", None),
+    (4256, 256, 2, "bf16", "full", None), (4768, 256, 2, "f16", "full", None), (3200, 256, 3, "f16", "classic", None),
+    (2400, 256, 2, "f16", "full", "bf16")])   # the same batch with one: four CTAs, 128 rows
 def test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, H, L, prec, game, r_state):
     from cfx import synth
     classic = game == "classic"
