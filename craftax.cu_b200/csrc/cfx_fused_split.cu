@@ -504,7 +504,9 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     // h128x2, 4,736 12.9 -> 12.7).
     const bool draws = samples && wg == 0;
     if (draws) {
-        asm volatile("" ::"l"(step0));   // has been read
+        // (the counter's load has been issued in front of this, which does not wait for it: the __syncwarp and the fence in done_with_step
+        // order the loads of all lanes before lane 0's count)
+        asm volatile("" ::"l"(step0));
         __syncwarp();
         if (lane == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
     }
