@@ -546,7 +546,7 @@ union ListMemory {
     ListBlock block;
 };
 static_assert(sizeof(ListMemory) <= 48 * 1024, "static shared memory");
-// Lists of more entries than this for each warp of the grid go by blocks.  65,536 envs, 2,368 warps, random lists in three sets of buffers, us by warps /
+// Lists of more entries than this for each warp of the grid go by blocks.  65,536 envs, 2,368 warps, envs chosen at random, three sets of buffers, us by warps /
 // by blocks: 250 entries 4.1 / 8.0, 2,368 5.8 / 9.7, 4,736 11.8 / 11.8, 7,104 17.1 / 13.9, 16,384 33.4 / 18.6, all of them 119 / 52.
 constexpr int kListPerWarp = 2;
 
