@@ -102,12 +102,13 @@ template <bool PAIR, int GAME, int HID> struct Cfg {
     static constexpr int kM = PAIR ? 256 : 128;
     // State boxes that are loaded as soon as their slots are free of records.  The slots come free at about the same time, and copies
     // queue in order: with eight boxes (128 KB from memory) in front of them the last weight stages of the encoder came 2,500 cycles late.  The others
-    // are loaded when the encoder is done, unless the state is recorded, which is done ahead of the cells.  us a step in long runs, all boxes at once
-    // and so: h256x2 18,944 envs 29.4 and 29.5, 37,888 63.7 and 62.1, 131,104 210.7 and 207.5, 262,144 421.9 and 421.9; h256x1 37,888 40.4 and 40.8, 65,536
-    // 78.5 and 76.2; h256x3 65,536 147.3 and 146.0, 262,144 559.5 and 560.6; h128x2 131,104 112.6 and 111.1, 262,144 219.5 and 216.5; classic h256x3
-    // 1,048,576 2,211 and 2,214.  All, 1, 2 or 4 first: h256x2 37,888 envs 63.1, 61.4, 61.8, 62.3; h128x2 131,104 113.8, 115.5, 113.9,
-    // 112.7; h256x2 16,416 with a bf16 record 31.3, 31.4, 31.6, 31.6.  Only in the first tiles of a CTA, four or at hidden 128 eight: within 0.6 % either
-    // way at 37 sizes.
+    // are loaded when the encoder is done.  us a step in long runs, all boxes at once and so: h256x2 18,944 envs 29.4 and 29.5, 37,888 63.7 and 62.1, 131,104
+    // 210.7 and 207.5, 262,144 421.9 and 421.9; h256x1 37,888 40.4 and 40.8, 65,536 78.5 and 76.2; h256x3 65,536 147.3 and 146.0, 262,144 559.5 and 560.6;
+    // h128x2 131,104 112.6 and 111.1, 262,144 219.5 and 216.5.  All, 1, 2 or 4 first: h256x2 37,888 envs 63.1, 61.4, 61.8, 62.3; h128x2 131,104 113.8, 115.5,
+    // 113.9, 112.7; h256x2 16,416 with a bf16 record 31.3, 31.4, 31.6, 31.6.  Only in the first tiles of a CTA, four or at hidden 128 eight: within 0.6 %
+    // either way at 37 sizes.
+    // All at once where the state is recorded, which is done ahead of the cells, and in the classic game, whose records leave six of the slots alone
+    // (classic h256x3, at once and so: 9,504 envs 31.66 and 31.91, 37,888 81.4 and 80.6, 1,048,576 2,192 and 2,197; h256x1 14,400 20.44 and 20.64).
     static constexpr int kEarlyBoxes = HID == 256 ? 1 : 4;
     // records: rows of one copy, slots that hold them, where row r of the tile begins in the data area.  Full game: 16 rows a
     // slot, the odd slots 64 bytes on, so that a warp's 32 rows start in 32 banks
@@ -367,7 +368,7 @@ __device__ __forceinline__ void role_loads(const Smem& sm, const Params& P) {
         }
         for (int b = 0; b < boxes; b++) {
             const int slot = b % kNS, l = b / kStateItems, j = b % kStateItems;
-            if (b == C::kEarlyBoxes && P.r_state == nullptr) CFX_WAIT_FAST(ACC_FULL, it & 1, W_ACC_FULL);
+            if (GAME == CFX_GAME_FULL && b == C::kEarlyBoxes && P.r_state == nullptr) CFX_WAIT_FAST(ACC_FULL, it & 1, W_ACC_FULL);
             if (b < C::kRecSlots) {
                 if ((b & 1) == 0) CFX_WAIT_FAST(REC_FREE + b / 2, it & 1, W_REC_FREE);
             } else if (b >= kNS || it > 0) {
