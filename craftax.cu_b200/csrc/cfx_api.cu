@@ -81,12 +81,12 @@ static void free_dev(void* p) {
 static int policy_refresh_mirrors(cfx_policy* p, cudaStream_t st) {
     if (p->precision != CFX_PREC_FP32) return fused_refresh(p->fused, p->params, st);
     const ArenaLayout o = ArenaLayout::make(p->H, p->L, p->A, p->obs);
-    return launch_transpose_gates(p->params + o.w_gru, p->gates_t, p->H, p->L, st);
+    return launch_transpose_gates(p->params, o, p->gates_t, p->H, p->L, st);
 }
 
 // What only the fp32 mode needs: the transposed gate matrices, two activation buffers [H][n] and room for the logits.
 static int policy_ensure_fp32(cfx_policy* p) {
-    if (!p->gates_t) CFX_CUDA(cudaMalloc((void**)&p->gates_t, (size_t)p->L * 3 * p->H * p->H * sizeof(float)));
+    if (!p->gates_t) CFX_CUDA(cudaMalloc((void**)&p->gates_t, strict_gate_floats(p->H, p->L) * sizeof(float)));
     for (int i = 0; i < 2; i++)
         if (!p->scratch_h[i]) CFX_CUDA(cudaMalloc((void**)&p->scratch_h[i], (size_t)p->H * p->n * sizeof(float)));
     if (!p->logits_scratch)
@@ -361,7 +361,7 @@ int cfx_policy_set_precision(cfx_policy* p, int precision) {
     if (precision == CFX_PREC_FP32) {
         if ((rc = policy_ensure_fp32(p))) return rc;
         const ArenaLayout o = ArenaLayout::make(p->H, p->L, p->A, p->obs);
-        rc = launch_transpose_gates(p->params + o.w_gru, p->gates_t, p->H, p->L, p->stream);
+        rc = launch_transpose_gates(p->params, o, p->gates_t, p->H, p->L, p->stream);
     } else {
         if ((rc = fused_create(&plan, p->device, p->n, p->H, p->L, p->A, precision, p->state, p->game))) return rc;
         rc = fused_refresh(plan, p->params, p->stream);

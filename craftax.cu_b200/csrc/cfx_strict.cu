@@ -124,115 +124,173 @@ __host__ __device__ __forceinline__ size_t act_at(size_t e, int k, int H) { retu
 // ---------------------------------------------------------------- encoder
 // h_enc[k][e] = b_enc[k] + sum_f x[e][f] * W_enc[f][k], ascending f.  A lane owns TM envs x G groups of 4
 // units, the groups 32 units apart.  Few warps of such tiles fall to an SM scheduler (one at 4,096 envs,
-// hidden 256), so everything but the sums is taken out of them: four warps of a block fill the stages (record words ->
-// fp32, transposed; W_enc rows by asynchronous copies), four multiply, and named barriers hand the
-// stages over.  (4,096 envs, hidden 256: 63 us with every warp doing both, and 78 us
-// with the features kept as bytes and converted by the lanes that multiply.)  A small batch is bound by the latency of these
-// loads: record words are fetched three chunks ahead, W_enc rows S - 2 chunks, and the 51 raw floats of the tail are copied
-// at the start by the warps that multiply (32 envs, encoder by itself: 25 us with one chunk ahead, 17 so).
-// What a forward of 4,096 envs, hidden 256, depth 2 gained with 7 envs a lane (on 147 of 148 SMs) instead of 8 (128): 6 us; with two of the
-// multiplying warps side by side along the units, so that a block converts half as many records: 1.7; with the copies of a
-// chunk and its k steps written out: 2.  The fills' work still slows the sums beside them: 82,000 cycles a block, 62,000 in a loop of the sums alone.
-constexpr int kEncK = 32, kEncAhead = 3;
-constexpr int kMapChunks = (kMap + kEncK - 1) / kEncK, kEncChunks = kMapChunks + (kTail + kEncK - 1) / kEncK;   // 25 of record bytes, 2 of the tail
-static_assert(kEncChunks % kEncAhead == 0, "the chunk loop is unrolled by the words in flight");
+// hidden 256), so everything but the sums is taken out of them: four warps of a block fill the stages (record bytes ->
+// fp32; W_enc rows by asynchronous copies), four multiply, and named barriers hand the stages over.
+// A feature that is zero in all envs of a block is left out: its products change no sum (but the sign of one that is still -0).  Most bytes of a
+// record are zero, five of a cell's eight unless there is a mob: of the 843 features 410 are left in blocks of 56 envs of a game, 546 with a mob of each
+// class on every hundredth cell.  Zero times a weight that is infinite or not a number is not zero: with such weights (odd_weights, looked for when the
+// weights are laid out) nothing is left out.  The block copies its records' maps to shared memory, ORs them over the envs, and makes a list of the features
+// that are left, from which the stages are filled.  (Features taken 32 at a time as they come, the left ones packed by masks: 117.5 us a forward at 4,096
+// envs, hidden 256, depth 2, and 10 us slower than every feature at 32: what a warp does for a feature is a chain of 150 cycles.  So all that the list and the map
+// give for a stage is loaded before it is used: 114.)
+// Bound by the FMA pipe, the operands' reads of shared memory beside it, and 4,000 cycles until the first stage is there.  us a forward with every feature and now,
+// hidden 256, depth 2: 4,096 envs 123.4 and 113.7, 2,048 84.3 and 75.4, 65,536 1,529 and 1,386, 128 43.9 and 40.0, 32 31.7 and 31.7; 8,192 envs, hidden 512,
+// depth 3 828 and 788; 4,096, hidden 128 65.3 and 56.6.  Where no feature is zero it is slower: 4,096 envs 126.5, 32 envs 36.6.
+constexpr int kEncWarps = 8, kEncFill = 4;   // warps of a block, those of them that fill the stages
+constexpr int kMapRounds = (kMap / 4 + 31) / 32, kMapPitch = kMap + 4;   // rounds of a warp's lanes with a word of a record each; bytes from one env's map to the next's
+constexpr int kMapGroups = (kMap + 31) / 32, kGroups = kMapGroups + (kTail + 31) / 32;   // features by 32
+static_assert(kGroups < 32 && 4 * kMapRounds < 32 && kMap % 4 == 0 && kMapPitch % 8 == 4, "a lane a group; a lane an env without bank conflicts");
 template <int TM, int G, int WU, int UL> struct Enc {   // WU of the four warps side by side along the units, UL units of a group a lane
     static constexpr int WM = 4 / WU, BM = UL * TM * WM, BU = 32 * G * WU;   // envs, units
-    static constexpr int XS = BM + (BM % 8 == 0 ? 4 : 0);               // row stride of x: four rows are 16 banks on
-    static constexpr int S = TM == 1 ? 6 : (G == 1 ? 4 : 3);      // stages
-    static constexpr int kStage = kEncK * (XS + BU);                    // floats
-    static constexpr int kSmem = (S * kStage + kTail * XS) * (int)sizeof(float);
-    static_assert(XS % 8 == 4, "no bank conflicts between the words that a warp stores");
+    static constexpr int XS = BM + (BM % 8 == 0 ? 4 : 0);               // row stride of x
+    static constexpr int K = G == 1 ? 32 : 16, S = TM == 1 ? 6 : 4, R = S * K;   // rows of a stage, stages
+    static constexpr int kOffMap = R * (XS + BU) * 4, kOffList = kOffMap + BM * kMapPitch;
+    static constexpr int kSmem = kOffList + (kObs + K) * 2;
+    static_assert(XS % 4 == 0 && kOffList % 8 == 0, "alignment");
 };
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
 template <int TM, int G, int WU, int UL>
-__global__ void __launch_bounds__(256, 2)
-k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc,
+__global__ void __launch_bounds__(32 * kEncWarps, 2)
+k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc, const uint32_t* __restrict__ odd_weights,
                float* __restrict__ h_out, int n, int H, int w_aligned, int early) {
     using E = Enc<TM, G, WU, UL>;
     static_assert(UL == 4 || (UL == 1 && TM == 1 && G == 1), "tiles");
-    constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = kEncK, S = E::S, D = S - 2;
-    constexpr int FULL = 1, EMPTY = FULL + S, TAIL = 15;   // barrier ids
-    extern __shared__ __align__(16) float sm[];   // per stage: x [K][XS], w [K][BU]; then the tail [kTail][XS]
-    float* tail = sm + S * E::kStage;
+    constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = E::K, S = E::S, R = E::R, D = S - 2;
+    constexpr int FULL = 1, EMPTY = FULL + S;   // barrier ids
+    static_assert(EMPTY + S <= 16, "barriers");
+    extern __shared__ __align__(16) float sm[];   // x [R][XS], w [R][BU], the records' map bytes [BM][kMapPitch], the list of features
+    __shared__ uint32_t part[kEncWarps][4 * kMapRounds];
+    float* const xring = sm;
+    float* const wring = sm + R * XS;
+    uint8_t* const map = reinterpret_cast<uint8_t*>(sm) + E::kOffMap;
+    uint16_t* const list = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(sm) + E::kOffList);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e0 = blockIdx.x * BM, u0 = blockIdx.y * BU;
     if (early & kLaunchNext) launch_next_kernel();
-    if (warp >= 4) {
-        const int tid = threadIdx.x - 128;
-        // the rows of W_enc of chunk c, a piece of 16 bytes a thread at a time
-        constexpr int NW = K * BU / (4 * 128);
-        static_assert(NW * 4 * 128 == K * BU, "whole pieces");
-        auto copy_w = [&](int c) {
-            const int f0 = c < kMapChunks ? c * K : kMap + (c - kMapChunks) * K, end = c < kMapChunks ? kMap : kObs;
-            float* w = sm + (c % S) * E::kStage + K * XS;
+    wait_for_previous_kernel();
+    // The map bytes of the block's envs (where there are none, the last one's again, which changes nothing), and which of them are not
+    // zero in all envs: a bit a feature, 32 to a group
+    {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(map);
+#pragma unroll 2
+        for (int i = warp; i < BM; i += kEncWarps) {
+            const uint8_t* r = rec + (size_t)min(e0 + i, n - 1) * kRec;
 #pragma unroll
-            for (int i = 0; i < NW; i++) {
-                const int at = i * 128 + tid, k = at / (BU / 4), col = 4 * (at % (BU / 4));
-                if (f0 + k < end) copy16(w + 4 * at, W_enc + (size_t)(f0 + k) * H + u0 + col, true, w_aligned != 0);
-            }
-        };
-        if (!(early & kWeightsReady)) wait_for_previous_kernel();
+            for (int j = 0; j < kMapRounds; j++)
+                if (32 * j + lane < kMap / 4)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + i * kMapPitch + 4 * (32 * j + lane)), "l"(r + 4 * (32 * j + lane)) : "memory");
+        }
+        copy_commit();
+        const bool all = __any_sync(0xffffffffu, (odd_weights[lane] | odd_weights[lane + 32]) != 0);
+        copy_wait<0>();
+        uint32_t any[kMapRounds] = {};   // (a lane reads what it has copied)
+#pragma unroll 4
+        for (int i = warp; i < BM; i += kEncWarps)
 #pragma unroll
-        for (int c = 0; c < D; c++) { copy_w(c); copy_commit(); }
-        wait_for_previous_kernel();
-        // a task is one record word (four features of an env): lanes = 16 envs x 2 words
-        constexpr int BM16 = (BM + 15) / 16 * 16, TASKS = BM16 * (K / 4) / 128;
-        static_assert(TASKS * 128 == BM16 * (K / 4), "whole tasks");
-        auto slot = [&](int i, int& e, int& w) {
-            const int idx = i * 128 + tid;
-            e = idx % 16 + 16 * ((idx / 32) % (BM16 / 16));
-            w = (idx % 32) / 16 + 2 * (idx / (2 * BM16));
-        };
-        uint32_t raw[kEncAhead][TASKS];
-        auto fetch = [&](int c, uint32_t (&r)[TASKS]) {
+            for (int j = 0; j < kMapRounds; j++)
+                if (32 * j + lane < kMap / 4) any[j] |= *reinterpret_cast<const uint32_t*>(map + i * kMapPitch + 4 * (32 * j + lane));
 #pragma unroll
-            for (int i = 0; i < TASKS; i++) {
-                int e, w;
-                slot(i, e, w);
-                const int f = c * K + 4 * w;   // (792 is a multiple of 4)
-                r[i] = f < kMap && e < BM && e0 + e < n ? *reinterpret_cast<const uint32_t*>(rec + (size_t)(e0 + e) * kRec + f) : 0u;
-            }
-        };
+        for (int j = 0; j < kMapRounds; j++) {
+            // a byte's bit 0 to bit 28 + its number, then to its place in the group
+            uint32_t b = (((__vcmpne4(any[j], 0u) & 0x01010101u) * 0x10204080u) >> 28) << (4 * (lane & 7));
+            if (all) b = 0xFu << (4 * (lane & 7));
 #pragma unroll
-        for (int c = 0; c < kEncAhead; c++) fetch(c, raw[c]);
-        for (int c0 = 0; c0 < kEncChunks; c0 += kEncAhead) {
+            for (int d = 1; d < 8; d *= 2) b |= __shfl_xor_sync(0xffffffffu, b, d);
+            if ((lane & 7) == 0) part[warp][4 * j + (lane >> 3)] = b;
+        }
+    }
+    __syncthreads();
+    // the list: lane c counts group c, then every warp writes some groups
+    int total;
+    {
+        uint32_t rows = 0u;
+        if (lane < kMapGroups) {
 #pragma unroll
-            for (int q = 0; q < kEncAhead; q++) {
-                const int c = c0 + q, s = c % S;
-                if (c + D < kEncChunks) {
-                    if (c + D >= S) bar_sync(EMPTY + (c + D) % S, 256);
-                    copy_w(c + D);
+            for (int w = 0; w < kEncWarps; w++) rows |= part[w][lane];
+            if (lane == kMapGroups - 1) rows &= ~0u >> (kMapGroups * 32 - kMap);
+        } else if (lane < kGroups) {
+            rows = ~0u >> (lane == kGroups - 1 ? (kGroups - kMapGroups) * 32 - kTail : 0);
+        }
+        int pos = __popc(rows);
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const int before = __shfl_up_sync(0xffffffffu, pos, d);
+            if (lane >= d) pos += before;
+        }
+        total = __shfl_sync(0xffffffffu, pos, 31);
+        pos -= __popc(rows);
+        for (int c = warp; c < kGroups; c += kEncWarps) {
+            const uint32_t r = __shfl_sync(0xffffffffu, rows, c);
+            const int p = __shfl_sync(0xffffffffu, pos, c);
+            if (r >> lane & 1u) list[p + __popc(r & ((1u << lane) - 1u))] = (uint16_t)(c < kMapGroups ? 32 * c + lane : kMap + 32 * (c - kMapGroups) + lane);
+        }
+        if (warp == 0 && lane < K) list[total + lane] = 0;   // (a stage's end: copied, and not multiplied)
+    }
+    __syncthreads();
+    const int stages = (total + K - 1) / K;
+    if (warp >= kEncWarps - kEncFill) {
+        // a warp has KW rows of every stage
+        constexpr int KW = K / kEncFill, ENVS = (BM + 31) / 32;
+        static_assert(KW % 4 == 0 && BU <= 128, "a row of weights an instruction");
+        const int k0 = (warp - (kEncWarps - kEncFill)) * KW;
+        for (int i = 0; i < stages + D; i++) {
+            if (i < stages) {
+                const int s = i % S;
+                if (i >= S) bar_sync(EMPTY + s, 32 * kEncWarps);
+                float* const x = xring + (s * K + k0) * XS + lane;
+                float* const w = wring + (s * K + k0) * BU + 4 * lane;
+                int f[KW];   // (everything is loaded before it is used: row by row the latencies of shared memory add up, 150 cycles a row)
+#pragma unroll
+                for (int k = 0; k < KW; k += 4) {
+                    const uint2 v = *reinterpret_cast<const uint2*>(list + i * K + k0 + k);
+                    f[k] = v.x & 0xFFFFu; f[k + 1] = v.x >> 16; f[k + 2] = v.y & 0xFFFFu; f[k + 3] = v.y >> 16;
                 }
-                copy_commit();
-                if (c < kMapChunks) {
-                    float* x = sm + s * E::kStage;
+                const float* const wsrc = W_enc + u0 + 4 * lane;
+                if (BU == 128 || lane < BU / 4) {
+                    if (w_aligned)
 #pragma unroll
-                    for (int i = 0; i < TASKS; i++) {
-                        int e, wd;
-                        slot(i, e, wd);
-                        if (BM16 != BM && e >= BM) continue;
+                        for (int k = 0; k < KW; k++) copy16(w + k * BU, wsrc + (size_t)f[k] * H, true, true);
+                    else
 #pragma unroll
-                        for (int b = 0; b < 4; b++) x[(4 * wd + b) * XS + e] = (float)((raw[q][i] >> (8 * b)) & 0xFFu);
+                        for (int k = 0; k < KW; k++) copy16(w + k * BU, wsrc + (size_t)f[k] * H, true, false);
+                }
+                if ((i + 1) * K <= total - kTail) {
+                    uint32_t v[KW][ENVS];
+#pragma unroll
+                    for (int q = 0; q < ENVS; q++) {
+                        const uint8_t* m = map + (BM % 32 != 0 ? min(32 * q + lane, BM - 1) : 32 * q + lane) * kMapPitch;
+#pragma unroll
+                        for (int k = 0; k < KW; k++) v[k][q] = m[f[k]];
                     }
-                    fetch(c + kEncAhead, raw[q]);
+#pragma unroll
+                    for (int q = 0; q < ENVS; q++)
+                        if (BM % 32 == 0 || 32 * q + lane < BM)
+#pragma unroll
+                            for (int k = 0; k < KW; k++) x[k * XS + 32 * q] = (float)v[k][q];
+                } else {
+#pragma unroll
+                    for (int q = 0; q < ENVS; q++) {
+                        const int e = 32 * q + lane;
+                        if (BM % 32 != 0 && e >= BM) break;
+                        const uint8_t* const r = rec + (size_t)min(e0 + e, n - 1) * kRec + kMap;
+#pragma unroll
+                        for (int k = 0; k < KW; k++) {
+                            if (f[k] < kMap) x[k * XS + 32 * q] = (float)map[e * kMapPitch + f[k]];
+                            else
+                                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(x + k * XS + 32 * q)),
+                                             "l"(r + 4 * (f[k] - kMap)) : "memory");
+                        }
+                    }
                 }
-                copy_wait<D>();
-                bar_arrive(FULL + s, 256);
             }
+            copy_commit();
+            copy_wait<D>();   // stage i - D is complete
+            if (i >= D) bar_arrive(FULL + (i - D) % S, 32 * kEncWarps);
         }
         return;
     }
-    wait_for_previous_kernel();
-    for (int i = threadIdx.x; i < BM * kTail; i += 128) {
-        const int e = i / kTail, j = i % kTail;
-        const bool on = e0 + e < n;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(tail + j * XS + e)),
-                     "l"(rec + (size_t)(on ? e0 + e : e0) * kRec + kMap + 4 * j), "r"(on ? 4 : 0) : "memory");
-    }
-    copy_commit();
     const int el = warp % E::WM * UL * TM, ul = warp / E::WM * 32 * G + lane % (32 / UL) * UL, lg = lane / (32 / UL);   // the warp's first env
     float z1 = UL == 1 ? b_enc[u0 + ul] : 0.0f;   // the sum of a lane with one
     uint64_t z[G][TM][2];
@@ -261,27 +319,18 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
             }
         }
     };
-    for (int c = 0; c < kEncChunks; c++) {
-        const int s = c % S;
-        const float* wp = sm + s * E::kStage + K * XS + ul;
-        if (c == kMapChunks) {
-            copy_wait<0>();
-            bar_sync(TAIL, 128);
-        }
-        const float* xp = (c < kMapChunks ? sm + s * E::kStage : tail + (c - kMapChunks) * K * XS) + el;
-        const int rows = c < kMapChunks ? min(K, kMap - c * K) : min(K, kTail - (c - kMapChunks) * K);
-        bar_sync(FULL + s, 256);
-        if (rows == K) {
+    for (int i = 0; i < stages; i++) {
+        const int s = i % S, left = total - i * K;
+        const float* xp = xring + s * K * XS + el;
+        const float* wp = wring + s * K * BU + ul;
+        bar_sync(FULL + s, 32 * kEncWarps);
+        if (left >= K) {
 #pragma unroll
             for (int k = 0; k < K; k++) step(xp + k * XS, wp + k * BU);
         } else {
-            int k = 0;
-            for (; k + 8 <= rows; k += 8)
-#pragma unroll
-                for (int i = 0; i < 8; i++) step(xp + (k + i) * XS, wp + (k + i) * BU);
-            for (; k < rows; k++) step(xp + k * XS, wp + k * BU);
+            for (int k = 0; k < left; k++) step(xp + k * XS, wp + k * BU);
         }
-        if (c + S < kEncChunks) bar_arrive(EMPTY + s, 256);
+        if (i + S < stages) bar_arrive(EMPTY + s, 32 * kEncWarps);
     }
     if constexpr (UL == 1) {
         if (e0 + el < n) h_out[act_at(e0 + el, u0 + ul, H)] = z1;
@@ -904,10 +953,18 @@ __global__ void k_fetch(const uint4* src, uint4* __restrict__ dst, size_t count)
 __global__ void k_bump(unsigned long long* ctr) { *ctr += 1ULL; }
 
 // Gate matrices for the fp32 layer kernel: Wt[l][unit tile][j][gate][unit of the tile] = W[l][gate H + unit][j], tiles of 64
-// units, or of 32 where the hidden size is an odd multiple of it.
-__global__ void k_transpose_gates(const float* __restrict__ W, float* __restrict__ Wt, int H, int L) {
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t per = (size_t)3 * H * H;
+// units, or of 32 where the hidden size is an odd multiple of it.  The last kOddWords blocks look W_enc over, an equal share each,
+// and leave behind the gate matrices whether anything in it is infinite or not a number (k_encoder_fp32).
+__global__ void k_transpose_gates(const float* __restrict__ W, float* __restrict__ Wt, int H, int L, const float* __restrict__ W_enc, int enc) {
+    const size_t per = (size_t)3 * H * H, idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int share = (int)blockIdx.x - (int)(gridDim.x - kOddWords);
+    if (share >= 0) {
+        bool odd = false;
+        for (int i = share * (int)blockDim.x + threadIdx.x; i < enc; i += kOddWords * (int)blockDim.x) odd |= !(fabsf(W_enc[i]) < INFINITY);
+        odd = __syncthreads_or(odd);
+        if (threadIdx.x == 0) reinterpret_cast<uint32_t*>(Wt + per * L)[share] = odd ? 1u : 0u;
+        return;
+    }
     if (idx >= per * L) return;
     const size_t l = idx / per, r = (idx % per) / H, j = idx % H;
     const int U = H % 64 == 0 ? 64 : 32, g = (int)(r / H), u = (int)(r % H);
@@ -977,9 +1034,9 @@ int launch_bump(unsigned long long* ctr, cudaStream_t st) {
     return CFX_OK;
 }
 
-int launch_transpose_gates(const float* W, float* Wt, int H, int L, cudaStream_t st) {
+int launch_transpose_gates(const float* params, const ArenaLayout& o, float* Wt, int H, int L, cudaStream_t st) {
     size_t total = (size_t)L * 3 * H * H;
-    k_transpose_gates<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(W, Wt, H, L);
+    k_transpose_gates<<<(unsigned)((total + 255) / 256) + kOddWords, 256, 0, st>>>(params + o.w_gru, Wt, H, L, params + o.w_enc, (int)(o.b_enc - o.w_enc));
     CFX_CUDA(cudaGetLastError());
     return CFX_OK;
 }
@@ -1071,8 +1128,8 @@ static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, int early, 
     int rc = allow_smem<k_encoder_fp32<TM, G, WU, UL>, E::kSmem>();
     if (rc) return rc;
     return launch_chained(k_encoder_fp32<TM, G, WU, UL>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
-                          a.params + o.w_enc, a.params + o.b_enc, a.scratch_h[0], a.n, a.H,
-                          ((uintptr_t)(a.params + o.w_enc) & 15) == 0, early);
+                          a.params + o.w_enc, a.params + o.b_enc, reinterpret_cast<const uint32_t*>(a.gates_t + strict_gate_floats(a.H, a.L) - kOddWords),
+                          a.scratch_h[0], a.n, a.H, ((uintptr_t)(a.params + o.w_enc) & 15) == 0, early);
 }
 
 template <int TM, int WM, int WU, int ST>
@@ -1121,11 +1178,10 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     const int tm = strict_tile(n, H);
     const EncoderTile te = strict_encoder_tile(n, H);
     // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own (512 envs, 64 blocks a layer: 88 us
-    // with it, 72 without), or two of the smallest have one (32 envs, hidden 256, depths 1, 2, 3, with and without: 26.1 and 27.8, 31.7 and 33.5, 43.1
-    // and 39.1 us)
+    // with it, 72 without; 32 envs, hidden 256, depth 2, 194 blocks: 34.4 and 31.6)
     auto count = [&](int tile) { return tile == 0 ? 8 * q : tile == 1 ? 2 * q : q / 2; };
     const long long blocks = count(te.tm) + L * count(tm) + n / 16;
-    const int early = (a.game == CFX_GAME_FULL && blocks <= (tm == 0 ? 200 : kSMs) ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
+    const int early = (a.game == CFX_GAME_FULL && blocks <= kSMs ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
     if (a.game == CFX_GAME_CLASSIC) {
         rc = launch_chained(k_classic_encoder_fp32, dim3(n), H, 0, st, a.records, a.params + o.w_enc, a.params + o.b_enc,
                             a.scratch_h[0], n, H);
@@ -1183,7 +1239,7 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
 // each call before they are read, so stale contents of an earlier call are harmless.
 namespace cfx {
 constexpr int kStaticMaxEnvs = 1024, kStaticHidden = 256, kStaticMaxLayers = 4;
-constexpr size_t kStaticGates = (size_t)kStaticMaxLayers * 3 * kStaticHidden * kStaticHidden;
+constexpr size_t kStaticGates = strict_gate_floats(kStaticHidden, kStaticMaxLayers);
 constexpr size_t kStaticLayerBuf = (size_t)kStaticMaxEnvs * kStaticHidden;
 constexpr size_t kStaticLogits = (size_t)kStaticMaxEnvs * (kMaxActions + 1);
 constexpr size_t kStaticFloats = kStaticGates + 2 * kStaticLayerBuf + kStaticLogits;
@@ -1241,7 +1297,7 @@ extern "C" int cfx_strict_forward_static(int device, const float* params, int hi
     }
     float* base = g_static_scratch_addr[device].load(std::memory_order_acquire);
     const ArenaLayout o = ArenaLayout::make(hidden, layers, num_actions);
-    int rc = launch_transpose_gates(params + o.w_gru, base, hidden, layers, st);
+    int rc = launch_transpose_gates(params, o, base, hidden, layers, st);
     if (rc) return rc;
     StrictArgs a;
     a.n = num_envs; a.H = hidden; a.L = layers; a.A = num_actions;

@@ -3,13 +3,15 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "cfx_common.cuh"
+
 namespace cfx {
 
 struct StrictArgs {
     int n, H, L, A;
     int game = 0;           // CFX_GAME_FULL or CFX_GAME_CLASSIC (148-byte records, gather encoder)
     const float* params;    // fp32 arena
-    const float* gates_t;   // [L] gate matrices as launch_transpose_gates writes them
+    const float* gates_t;   // what launch_transpose_gates writes
     const uint8_t* records;
     const float* prev_terminals;
     const float* uniforms;
@@ -46,7 +48,10 @@ int launch_uniforms(uint64_t seed, uint64_t env_offset, uint64_t step, int n, fl
 // copies `bytes` (a multiple of 16) from page-locked host memory, both 16-byte aligned
 int launch_fetch(const void* host, void* dst, size_t bytes, cudaStream_t st);
 int launch_bump(unsigned long long* ctr, cudaStream_t st);
-int launch_transpose_gates(const float* W, float* Wt, int H, int L, cudaStream_t st);
+// The gate matrices as the layers read them, and whether W_enc has values that are not finite, strict_gate_floats(H, L) in all
+constexpr int kOddWords = 64;
+constexpr size_t strict_gate_floats(int H, int L) { return (size_t)L * 3 * H * H + kOddWords; }
+int launch_transpose_gates(const float* params, const ArenaLayout& o, float* Wt, int H, int L, cudaStream_t st);
 // counts the batches' reciprocals that are not 1.0f / d (see k_selftest_reciprocals); waits for the device
 int selftest_reciprocals(uint32_t first, uint32_t last, uint32_t far, uint64_t* differing);
 int launch_init_uniform(float* w, int count, float bound, uint64_t seed, int subseq, cudaStream_t st);
