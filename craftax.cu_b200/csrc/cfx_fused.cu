@@ -107,7 +107,7 @@ template <bool PAIR, int GAME, int HID> struct Cfg {
     // h128x2 131,104 112.6 and 111.1, 262,144 219.5 and 216.5.  All, 1, 2 or 4 first: h256x2 37,888 envs 63.1, 61.4, 61.8, 62.3; h128x2 131,104 113.8, 115.5,
     // 113.9, 112.7; h256x2 16,416 with a bf16 record 31.3, 31.4, 31.6, 31.6.  Only in the first tiles of a CTA, four or at hidden 128 eight: within 0.6 %
     // either way at 37 sizes.
-    // All at once where the state is recorded, which is done ahead of the cells, and in the classic game, whose records leave six of the slots alone
+    // All at once where the state is recorded ahead of the cells (not REC16: h256x2 16,416 envs 29.5 and 29.2, 57,600 110.6 and 107.9), and in the classic game, whose records leave six of the slots alone
     // (classic h256x3, at once and so: 9,504 envs 31.66 and 31.91, 37,888 81.4 and 80.6, 1,048,576 2,192 and 2,197; h256x1 14,400 20.44 and 20.64).
     static constexpr int kEarlyBoxes = HID == 256 ? 1 : 4;
     // records: rows of one copy, slots that hold them, where row r of the tile begins in the data area.  Full game: 16 rows a
@@ -328,7 +328,7 @@ __device__ __forceinline__ void role_weight_loads(const Smem& sm, const Params& 
 // next while the warp served the other lanes.)
 //   load thread:  per tile, the records, then the state boxes, each when what was in its slots before is done with;
 //   store thread: the state box stores; it reports a box that has been read out of its slot (S_FREE).
-template <bool PAIR, int GAME, int HID>
+template <bool PAIR, int GAME, int HID, bool REC16>
 __device__ __forceinline__ void role_loads(const Smem& sm, const Params& P) {
     using C = Cfg<PAIR, GAME, HID>;
     CFX_DIMS(HID);
@@ -368,7 +368,7 @@ __device__ __forceinline__ void role_loads(const Smem& sm, const Params& P) {
         }
         for (int b = 0; b < boxes; b++) {
             const int slot = b % kNS, l = b / kStateItems, j = b % kStateItems;
-            if (GAME == CFX_GAME_FULL && b == C::kEarlyBoxes && P.r_state == nullptr) CFX_WAIT_FAST(ACC_FULL, it & 1, W_ACC_FULL);
+            if (GAME == CFX_GAME_FULL && b == C::kEarlyBoxes && (REC16 || P.r_state == nullptr)) CFX_WAIT_FAST(ACC_FULL, it & 1, W_ACC_FULL);
             if (b < C::kRecSlots) {
                 if ((b & 1) == 0) CFX_WAIT_FAST(REC_FREE + b / 2, it & 1, W_REC_FREE);
             } else if (b >= kNS || it > 0) {
@@ -655,7 +655,7 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 // ------------------------------------------------------------------ worker role
 // Sixteen warps, four per TMEM lane quarter (groups wg 0 to 3); thread (quarter, lane) owns env row
 // quarter*32 + lane of the tile in every phase.
-template <typename T16, bool PAIR, int GAME, int HID>
+template <typename T16, bool PAIR, int GAME, int HID, bool REC16>
 __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uint32_t tmem,
                                             int warp, int lane, uint32_t bar0_cta0) {
     using Op = Op16<T16>;
@@ -785,7 +785,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 spar ^= 1u << slot;
                 // under the slice's MMAs (of a warp's rows all or none are valid).  The ballot of the flags stands here and not at
                 // the tile's start, where it would wait for them: 65,536 envs h256x3 145.7 -> 142.8 us, one set of buffers
-                if (P.r_state != nullptr && valid) {
+                if (!REC16 && P.r_state != nullptr && valid) {
                     CFX_WAITW(S_FULL + slot, sp_par, W_S_FULL);
                     write_r_state<4, kH>(P, sm.s_slot(slot) + quarter * 4096, 4 * (wg & 1),
                                          ((size_t)l * P.n + tile * kTile + quarter * 32) * kH + kSliceUnits * j + kWarpUnits * wg,
@@ -821,12 +821,19 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 }
                 CFX_MARK(8);
                 uint32_t hn[kWarpUnits / 2];
+                float rs[kWarpUnits / 2];   // REC16: the state record of this thread's units, packed
 #pragma unroll
                 for (int q = 0; q < kWarpUnits / 4; q++) {
                     const int u = 4 * q;  // first of four units
                     float4* sp = reinterpret_cast<float4*>(rbase + (((4 * (wg & 1) + q) ^ xr) << 4));
                     float4 st = *sp;
                     if (zero_state) st = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (REC16) {
+                        rs[2 * q] = __uint_as_float(Op16<__nv_bfloat16>::pack(st.x, st.y));
+                        rs[2 * q + 1] = __uint_as_float(Op16<__nv_bfloat16>::pack(st.z, st.w));
+                        if (q == kWarpUnits / 4 - 1 && valid)
+                            st_global_v8(reinterpret_cast<float*>(reinterpret_cast<__nv_bfloat16*>(P.r_state) + ((size_t)l * P.n + env) * kH + kSliceUnits * j + kWarpUnits * wg), rs);
+                    }
                     const float2 x01 = Op::unpack(xin[u / 2]), x23 = Op::unpack(xin[u / 2 + 1]);
                     float4 out;
                     float h0, h1, h2, h3;
@@ -894,7 +901,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
 // of a pair owns tile 2 c + r in every respect (records, state, expand, cell, sampler) except
 // that the MMA warp of the even CTA issues one 256-row MMA for both tiles and every CTA
 // stages only its half of the weight rows.
-template <typename T16, bool PAIR, int GAME, int HID>
+template <typename T16, bool PAIR, int GAME, int HID, bool REC16>
 __global__ void __launch_bounds__(kThreads, 1)
 k_policy_fused(const __grid_constant__ Params P) {
     using C = Cfg<PAIR, GAME, HID>;
@@ -980,13 +987,13 @@ k_policy_fused(const __grid_constant__ Params P) {
         } else {
             wait_for_previous_kernel();
             if (lane == 0) {
-                if (warp == 2) role_loads<PAIR, GAME, HID>(sm, P);
+                if (warp == 2) role_loads<PAIR, GAME, HID, REC16>(sm, P);
                 else role_stores<PAIR, GAME, HID>(sm, P);
             }
         }
     } else {
         wait_for_previous_kernel();
-        role_worker<T16, PAIR, GAME, HID>(sm, P, tmem, warp, lane, bar0_cta0);
+        role_worker<T16, PAIR, GAME, HID, REC16>(sm, P, tmem, warp, lane, bar0_cta0);
     }
 
     // common exit: every role ends here, also after a timed-out wait.  In a pair neither CTA
@@ -1127,12 +1134,14 @@ bool fused_supported(int H, int L, int A, int precision, int game) {
 }
 
 // kernel instantiation and its shared-memory size for (operand type, launch mode, game, hidden)
-static const void* fused_kernel(int precision, int pair, int game, int H, int* smem) {
+static const void* fused_kernel(int precision, int pair, int game, int H, bool rec16, int* smem) {
     const bool h = precision == CFX_PREC_F16;
 #define CFX_K(T, P, G, HID)                                         \
     do {                                                            \
         *smem = fused::Cfg<P, G, HID>::kSmemBytes;                  \
-        return (const void*)fused::k_policy_fused<T, P, G, HID>;    \
+        if constexpr (G == CFX_GAME_FULL)                           \
+            if (rec16) return (const void*)fused::k_policy_fused<T, P, G, HID, true>; \
+        return (const void*)fused::k_policy_fused<T, P, G, HID, false>; \
     } while (0)
 #define CFX_K2(P, G, HID)                          \
     do {                                           \
@@ -1196,8 +1205,10 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
     }
     for (int pr = 0; pr < 2 && e == cudaSuccess; pr++) {
         int smem = 0;
-        const void* k = fused_kernel(precision, pr, game, H, &smem);
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        for (int rec16 = 0; rec16 < 2 && e == cudaSuccess; rec16++) {
+            const void* k = fused_kernel(precision, pr, game, H, rec16 != 0, &smem);
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        }
     }
     if (e != cudaSuccess) {
         fused_destroy(p);
@@ -1211,7 +1222,7 @@ int fused_create(FusedPlan** out, int device, int n, int H, int L, int A, int pr
         cfg.gridDim = dim3(2 * (unsigned)(p->sm_count / 2));
         cfg.blockDim = dim3(fused::kThreads);
         int smem = 0;
-        const void* kpair = fused_kernel(precision, 1, game, H, &smem);
+        const void* kpair = fused_kernel(precision, 1, game, H, false, &smem);
         cfg.dynamicSmemBytes = smem;
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeClusterDimension;
@@ -1333,10 +1344,11 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     // Small batches: a tile is shared by four (two) CTAs as long as every tile then has its SMs at once, and is as
     // short as that allows (cfx_fused_split.cu).  CTAs of two slices take tiles of 64 and
     // 128 rows; at 32 four CTAs a tile have their SMs.  With the 33 clusters of four and 74 of two that this part holds, four
-    // CTAs go to 1,056 and 2,112 envs, with 32 and 64 rows, and two to 4,736 with 64 rows and 9,472 with 128; where the state is recorded, four take
+    // CTAs go to 1,056 and 2,112 envs, with 32 and 64 rows, and two to 4,736 with 64 rows and 9,472 with 128; where the state is recorded by write_r_state, four take
     // 128 rows up to 4,224.  At each of these limits the next form is slower, and the kernel below slower than all of them.  us a step, h256x2, clusters
     // of four with 32, 64, 128 rows, of two with 64 and 128, the kernel below: 1,056 envs 10.5, 14.6, 16.8, 16.2, 17.9, 21.5; 2,112 -, 14.8, 16.4, 16.5,
     // 18.2, 21.8; 2,144 -, -, 17.0, 16.5, 18.2, 21.8; 4,224 -, -, 17.5, 16.9, 18.4, 22.0; 4,736 -, -, -, 17.1, 18.3, 22.3; 9,472 -, -, -, -, 19.0, 22.5.
+    // (The same with a bf16 record that the cells write, see record_by_rows: 4,224 envs h256x2 18.8 and 18.3, h256x1 14.7 and 14.2, h256x3 23.3 and 22.5.)
     // Four CTAs with 128 rows and two with 64, 3,200 envs: h256x1 13.25 and 13.16, h256x3 21.4 and 20.9, classic h256x3 25.0 and 24.7; with a record in
     // bf16 h256x2 18.5 and 18.9, in fp32 h256x3 22.3 and 23.5.  h128x2, of two with 32, 64, 128 rows, the kernel below:
     // 2,368 envs 8.9, 12.5, 13.4, 15.7; 4,736 -, 12.9, 13.5, 15.7; 9,472 -, -, 14.0, 16.0.
@@ -1345,14 +1357,14 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
         for (int S = i == 0 ? 4 : 2, tr = p->H == 64 * S ? 32 : 64; tr <= fused::kTile; tr *= 2) {
             const int tiles = (rows + tr - 1) / tr;
             if (tiles > p->max_split[i]) continue;
-            if (S == 4 && tr == fused::kTile && a.r_state == nullptr && (rows + 63) / 64 <= p->max_split[1]) continue;
+            if (S == 4 && tr == fused::kTile && (a.r_state == nullptr || (!classic && fused::record_by_rows(P))) && (rows + 63) / 64 <= p->max_split[1]) continue;
             for (int l = 0; l < p->L; l++) P.state_map[l] = p->quad_map[l];
             P.tile_rows = tr;
             P.done_blocks = (uint32_t)(tiles * (tr / 32));
             return fused::split_launch(p->precision, p->game, p->H, S, tiles, P, st);
         }
     int smem = 0;
-    const void* kern = fused_kernel(p->precision, p->pair, p->game, p->H, &smem);
+    const void* kern = fused_kernel(p->precision, p->pair, p->game, p->H, fused::record_by_rows(P), &smem);
     void* kargs[1] = {(void*)&P};
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(fused::kThreads);

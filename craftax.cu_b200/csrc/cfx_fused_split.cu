@@ -435,7 +435,7 @@ __device__ __forceinline__ void hand_on(const Smem& sm, uint32_t offset, uint32_
 // ------------------------------------------------------------------ workers
 // Sixteen warps: warp (quadrant, wg) owns TMEM lanes [32 quadrant, + 32) = those rows of the tile, converts
 // chunks wg, wg + 4, ... and handles units [16 wg, 16 wg + 16) of every slice of the CTA.
-template <typename T16, int GAME, int HID, int S>
+template <typename T16, int GAME, int HID, int S, bool REC16>
 __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
                                             uint32_t rank, Meetings& meet) {
     using Op = Op16<T16>;
@@ -561,7 +561,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         for (int j = 0; j < C::kNS; j++) {
             const int box = l * C::kBoxes + 2 * j + (wg >> 1), slot = box % kSSlots;
             CFX_SWAIT(S_FULL + slot, (box / kSSlots) & 1);
-            if (P.r_state != nullptr && valid)   // under the slice's MMAs
+            if (!REC16 && P.r_state != nullptr && valid)   // under the slice's MMAs
                 write_r_state<4, HID>(P, sm.base + C::kOffS + slot * kSBox + quadrant * 4096, 4 * (wg & 1),
                                       ((size_t)l * P.n + row0 + 32 * quadrant) * HID + C::slice((int)rank, j) * kSliceUnits + wg * kWarpUnits,
                                       zero_rows, lane);
@@ -574,6 +574,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             tmem_wait_ld();
             uint8_t* sp = sm.base + C::kOffS + slot * kSBox + (row >> 3) * 1024 + (row & 7) * 128;
             auto piece = [&](int q) { return reinterpret_cast<float4*>(sp + (((4 * (wg & 1) + q) ^ (row & 7)) << 4)); };
+            float rs[kWarpUnits / 2];   // REC16: the state record of this thread's units, packed
             // (half of the units at a time: with the state of all of them in registers a bf16 cell reads 22 words from local memory, so 4)
 #pragma unroll
             for (int h = 0; h < kWarpUnits / 4; h += 2) {
@@ -582,7 +583,14 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 for (int q = 0; q < 2; q++) {
                     st[q] = *piece(h + q);
                     if (zero_state) st[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (REC16) {
+                        rs[2 * (h + q)] = __uint_as_float(Op16<__nv_bfloat16>::pack(st[q].x, st[q].y));
+                        rs[2 * (h + q) + 1] = __uint_as_float(Op16<__nv_bfloat16>::pack(st[q].z, st[q].w));
+                    }
                 }
+                if (REC16 && h > 0 && valid)
+                    st_global_v8(reinterpret_cast<float*>(reinterpret_cast<__nv_bfloat16*>(P.r_state) + ((size_t)l * P.n + env) * HID +
+                                                          C::slice((int)rank, j) * kSliceUnits + wg * kWarpUnits), rs);
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
                     const int i = 4 * (h + q);
@@ -828,7 +836,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
 }
 
 // ------------------------------------------------------------------ kernel
-template <typename T16, int GAME, int HID, int S, bool ONE>
+template <typename T16, int GAME, int HID, int S, bool ONE, bool REC16>
 __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_constant__ Params P) {
     using C = Cfg<GAME, HID, S>;
     constexpr int kA = Gm<GAME>::kA;
@@ -922,7 +930,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         cluster_wait();
         Meetings meet;
         if constexpr (ONE) role_worker_one<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank, meet);
-        else role_worker<T16, GAME, HID, S>(sm, P, tmem, warp, lane, row0, rank, meet);
+        else role_worker<T16, GAME, HID, S, REC16>(sm, P, tmem, warp, lane, row0, rank, meet);
         __syncwarp();
         if (__builtin_expect(meet.met != Meetings::kAll, 0)) {   // a wait gave up
             const int quadrant = warp & 3;
@@ -948,17 +956,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-static const void* kernel(int precision, int game, int H, int S, bool one, int* smem) {
+static const void* kernel(int precision, int game, int H, int S, bool one, bool rec16, int* smem) {
     const bool h = precision == CFX_PREC_F16;
 #define CFX_SPLIT(G, HID, SS)                                               \
     do {                                                                    \
         *smem = smem_bytes<G, HID, SS>();                                   \
         if constexpr (HID / 64 / SS == 1)                                   \
             if (one)                                                        \
-                return h ? (const void*)k_policy_split<__half, G, HID, SS, true>          \
-                         : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS, true>;  \
-        return h ? (const void*)k_policy_split<__half, G, HID, SS, false>          \
-                 : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS, false>;  \
+                return h ? (const void*)k_policy_split<__half, G, HID, SS, true, false>          \
+                         : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS, true, false>;  \
+        if constexpr (G == CFX_GAME_FULL && HID == 256)                     \
+            if (rec16)                                                      \
+                return h ? (const void*)k_policy_split<__half, G, HID, SS, false, true>          \
+                         : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS, false, true>;  \
+        return h ? (const void*)k_policy_split<__half, G, HID, SS, false, false>          \
+                 : (const void*)k_policy_split<__nv_bfloat16, G, HID, SS, false, false>;  \
     } while (0)
     if (game == CFX_GAME_CLASSIC) {
         if (S == 4) CFX_SPLIT(CFX_GAME_CLASSIC, 256, 4);
@@ -991,15 +1003,17 @@ int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_
     *max_clusters = 0;
     if (H / 64 / S < 1) return CFX_OK;
     int smem = 0;
-    const void* k = split::kernel(precision, game, H, S, true, &smem);
+    const void* k = split::kernel(precision, game, H, S, true, false, &smem);
     CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k = split::kernel(precision, game, H, S, false, &smem);
-    CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    cudaFuncAttributes attr;
-    CFX_CUDA(cudaFuncGetAttributes(&attr, k));
-    // Built with fewer registers than its warps share out, they would wait for some that do not exist: such a build does without
-    // this kernel, and cfx_fused.cu's takes every batch.
-    if (S == 4 && attr.numRegs < split::kLaunchRegs) return CFX_OK;
+    for (int rec16 = 1; rec16 >= 0; rec16--) {
+        k = split::kernel(precision, game, H, S, false, rec16 != 0, &smem);
+        CFX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        cudaFuncAttributes attr;
+        CFX_CUDA(cudaFuncGetAttributes(&attr, k));
+        // Built with fewer registers than its warps share out, they would wait for some that do not exist: such a build does without
+        // this kernel, and cfx_fused.cu's takes every batch.
+        if (S == 4 && attr.numRegs < split::kLaunchRegs) return CFX_OK;
+    }
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = split::config(at, sm_count / S * S, S, smem, nullptr);
     cfg.numAttrs = 1;
@@ -1011,7 +1025,7 @@ int split_prepare(int precision, int game, int H, int S, int sm_count, int* max_
 
 int split_launch(int precision, int game, int H, int S, int tiles, const Params& P, cudaStream_t st) {
     int smem = 0;
-    const void* k = split::kernel(precision, game, H, S, P.tile_rows == 32, &smem);
+    const void* k = split::kernel(precision, game, H, S, P.tile_rows == 32, record_by_rows(P), &smem);
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = split::config(at, tiles * S, S, smem, st);
     void* args[1] = {(void*)&P};
