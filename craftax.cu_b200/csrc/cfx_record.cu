@@ -17,7 +17,8 @@
 // 65,536 envs with 62 KB of maps each, about 180 MB of DRAM traffic (us, by itself; with the list of 250 reset envs behind it):
 // copies behind the position, then the fields and the two mob classes of a warp one latency after the other 46.4 and 52.9; all loads that
 // wait for nothing in front of the copies 42.5 and 49.1; the copies by rows (27 lanes with a row each, at most two pieces
-// of it) replaced by whole spans 41.8 and 48.0; the fields in front of what depends on the level, and not behind, 39.9 and 46.2, 4.5 TB/s.
+// of it) replaced by whole spans 41.8 and 48.0; the fields in front of what depends on the level, and not behind, 39.9 and 46.2; 64 bytes a
+// miss (ld_bits) 38.1 and 44.6.
 // A block took 25,000 cycles, a third of them memory latencies one behind the other; in 17,000 they still are.  Five blocks an SM (48
 // registers; copies by rows): 41.6 and 48.2, and 4 % slower up to 8,192 envs.  The next kernel's start under this one, early or
 // late in a block: 49.4 to 50.4 instead of 49.1.
@@ -77,9 +78,14 @@ __device__ __forceinline__ int jax_index(int i, int size) {
 // that is written in between, so the compiler keeps load, conversion and store of every field in order, one DRAM
 // latency a field; a read-only load it sinks to its use, with the same effect.  Every loop below
 // therefore loads all its fields first.  (ld.global.nc would be wrong besides: see wait_for_previous_kernel.)
+// What a miss brings into L2 is limited to 64 bytes, a burst of the memory, here and in the copies: an env on another level than its neighbours reads
+// scattered words, and a view's span ends anywhere.  By default more comes along (us, this kernel and its list; the classic game's): words 46.3 -> 45.6, the
+// copies too 44.8, the words past L1 44.6; classic 262,144 envs 27.2 -> 25.7, its reads from memory 102 -> 86 MB.  With 128 or 256 bytes as by
+// default.  Not for bytes and shorts, of whose burst the neighbouring blocks use the rest (classic 27.2 -> 27.5).  Spans that leave L2 first (evict_first): 18,944 envs
+// 19.9 -> 18.0, 65,536 44.6 -> 45.4, classic 131,072 14.6 -> 13.7, 20,000 3.54 -> 3.92, 262,144 25.7 -> 26.1: not taken.
 __device__ __forceinline__ uint32_t ld_bits(const uint32_t* p) {
     uint32_t v;
-    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.L2::64B.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ int32_t ld_now(const int32_t* p) { return (int32_t)ld_bits(reinterpret_cast<const uint32_t*>(p)); }
@@ -316,7 +322,7 @@ struct CopyLane {
             if (lane >= kPieces || (unsigned)at >= (unsigned)kPlaneBytes) return;
 #pragma unroll
             for (int p = 0; p < kPlanes; p++)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + p * kSpan + 16 * lane)), "l"(q + off[p] + at) : "memory");
+                asm volatile("cp.async.cg.shared.global.L2::64B [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + p * kSpan + 16 * lane)), "l"(q + off[p] + at) : "memory");
         } else {
             static_assert(kRowWords == 4 && kRows == 9, "eight rows an instruction, and the last one of the three planes");
             const int o = (left & 12) + 4 * (lane & 3), col = c0 + o, dr = lane >> 2, row = v.top() + dr, last = v.top() + 8;
@@ -688,8 +694,8 @@ static_assert(offsetof(cfx_env_view, mob_type_id) - offsetof(cfx_env_view, playe
 // instruction to shared memory (whole rows: what is read from memory is 32-byte sectors anyway), where a
 // thread then takes the nine nibbles of a row from two words.  Loads of these words from the map
 // itself, 14 a thread, touch 32 cache lines an instruction: 20 of 41 us of a cache's time.  262,144 envs: a load per cell
-// 103 us, words from the map 41.5, rows through shared memory 27.3 (102 MB read from DRAM, 39 MB written); 65,536
-// envs 12.4 -> 8.2 us.
+// 103 us, words from the map 41.5, rows through shared memory 27.3 (102 MB read from DRAM, 39 MB written), with 64 bytes a miss 25.7
+// (86 MB); 65,536 envs 12.4 -> 8.2 us.
 constexpr int kClRows = 7, kClCols = 9, kClCells = kClRows * kClCols, kClMap = 64, kClRowBytes = 32;
 constexpr int kClSpan = kClRows * kClRowBytes + 16;   // 60 words: as few bank conflicts as 16-byte pieces allow
 constexpr int kClInv = 12, kClOutOfBounds = 1, kClBlockEnvs = 64, kClWords = kClassicRec / 4;
@@ -747,7 +753,7 @@ __global__ void __launch_bounds__(kClBlockEnvs) k_classic_record_rows(const __gr
             if (j < 2 * kClRows && row >= 0 && row < kClMap) {
                 const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem + 16 + ((t & ~31) + i + half) * kClSpan + 16 * j);
                 const uint8_t* q = V.map_packed + (size_t)env * V.map_stride + row * kClRowBytes + 16 * (j & 1);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(q) : "memory");
+                asm volatile("cp.async.cg.shared.global.L2::64B [%0], [%1], 16;" ::"r"(d), "l"(q) : "memory");
             }
         }
     } else {
