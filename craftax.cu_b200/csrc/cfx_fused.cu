@@ -328,6 +328,22 @@ __device__ __forceinline__ void role_weight_loads(const Smem& sm, const Params& 
 // next while the warp served the other lanes.)
 //   load thread:  per tile, the records, then the state boxes, each when what was in its slots before is done with;
 //   store thread: the state box stores; it reports a box that has been read out of its slot (S_FREE).
+// The records of a CTA's first tile are loaded ahead of this by a lane a copy (see the kernel).
+// Copy i of a tile's records.  Rows [32 q, 32 q + 32) are a quadrant's (n is a multiple of 32): all of them are there or none, and then what lies
+// in the slot is converted and multiplied like records, and the results of those rows are dropped.
+template <bool PAIR, int GAME, int HID>
+__device__ __forceinline__ void load_records(const Smem& sm, const Params& P, int tile, int i) {
+    using C = Cfg<PAIR, GAME, HID>;
+    const int r = i * C::kRecRows, row0 = tile * kTile + r, rows = min(C::kRecRows, P.n - row0);
+    const uint32_t full = sm.bar(REC_FULL + r / 32);
+    if (rows > 0) {
+        mbar_arrive_expect_tx(full, (uint32_t)rows * C::kRecBytes);
+        bulk_g2s(smem_u32(sm.s_slot(0)) + C::rec_offset(r), P.records + (size_t)row0 * C::kRecBytes, (uint32_t)rows * C::kRecBytes, full);
+    } else {
+        mbar_arrive(full);
+    }
+}
+
 template <bool PAIR, int GAME, int HID, bool REC16>
 __device__ __forceinline__ void role_loads(const Smem& sm, const Params& P) {
     using C = Cfg<PAIR, GAME, HID>;
@@ -335,35 +351,21 @@ __device__ __forceinline__ void role_loads(const Smem& sm, const Params& P) {
     const int boxes = P.L * kStateItems;
     uint32_t it = 0;
     uint32_t fpar = 0;      // slots: parity of the "free" phase to wait for
-    // rows [32 q, 32 q + 32) are a quadrant's (n is a multiple of 32): all of them are there or none, and then what lies in the slot
-    // is converted and multiplied like records, and the results of those rows are dropped
-    auto load_records = [&](int tile, int i) {
-        const int r = i * C::kRecRows, row0 = tile * kTile + r, rows = min(C::kRecRows, P.n - row0);
-        const uint32_t full = sm.bar(REC_FULL + r / 32);
-        if (rows > 0) {
-            mbar_arrive_expect_tx(full, (uint32_t)rows * C::kRecBytes);
-            bulk_g2s(smem_u32(sm.s_slot(0)) + C::rec_offset(r), P.records + (size_t)row0 * C::kRecBytes, (uint32_t)rows * C::kRecBytes, full);
-        } else {
-            mbar_arrive(full);
-        }
-    };
     auto prefetch_records = [&](int tile, int i) {
         const int row0 = tile * kTile + 16 * i;
         if (tile < P.num_tiles && row0 < P.n) bulk_prefetch_l2(P.records + (size_t)row0 * C::kRecBytes, 16 * C::kRecBytes);
     };
     CFX_MARK_INIT(4);
     for (int tile = P.tile_begin + blockIdx.x; tile < P.num_tiles_loop; tile += gridDim.x, it++) {
-        for (int u = 0; u < C::kRecSlots; u++) {
-            if (it > 0) {
-                if (u >= boxes) {   // no state boxes here
-                    if ((u & 1) == 0) CFX_WAIT_FAST(REC_FREE + u / 2, (it - 1) & 1, W_REC_FREE);
-                } else {
-                    CFX_WAIT_FAST(S_FREE + u, (fpar >> u) & 1u, W_S_FREE);
-                    fpar ^= 1u << u;
-                }
+        for (int u = 0; u < C::kRecSlots && it > 0; u++) {   // (those of the first tile: see the kernel)
+            if (u >= boxes) {   // no state boxes here
+                if ((u & 1) == 0) CFX_WAIT_FAST(REC_FREE + u / 2, (it - 1) & 1, W_REC_FREE);
+            } else {
+                CFX_WAIT_FAST(S_FREE + u, (fpar >> u) & 1u, W_S_FREE);
+                fpar ^= 1u << u;
             }
-            if (GAME == CFX_GAME_FULL) load_records(tile, u);
-            else if (u == C::kRecSlots - 1) load_records(tile, 0);
+            if (GAME == CFX_GAME_FULL) load_records<PAIR, GAME, HID>(sm, P, tile, u);
+            else if (u == C::kRecSlots - 1) load_records<PAIR, GAME, HID>(sm, P, tile, 0);
             CFX_MARK(20 + u);
         }
         for (int b = 0; b < boxes; b++) {
@@ -985,7 +987,12 @@ k_policy_fused(const __grid_constant__ Params P) {
         } else if (warp == 1) {
             if (rank == 0) role_mma<T16, PAIR, GAME, HID>(sm, P, tmem);
         } else {
+            // The first tile's records, a lane a copy: issued one behind the other they were 500 cycles apart.  us a step, h256x2 9,504 envs 24.3 -> 24.0,
+            // 18,944 28.4 -> 27.9, h128x2 16,160 17.0 -> 16.6, 20,000 28.2 -> 27.5.
+            const int first = P.tile_begin + (int)blockIdx.x;
             wait_for_previous_kernel();
+            if (warp == 2 && lane < C::kRecCopies && first < P.num_tiles_loop) load_records<PAIR, GAME, HID>(sm, P, first, lane);
+            __syncwarp();
             if (lane == 0) {
                 if (warp == 2) role_loads<PAIR, GAME, HID, REC16>(sm, P);
                 else role_stores<PAIR, GAME, HID>(sm, P);
