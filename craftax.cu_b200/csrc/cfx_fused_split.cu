@@ -22,8 +22,8 @@
 // The cluster works on one tile and exits, so every barrier but those of the rings is used once or once a
 // layer.  The products of a row are accumulated in the order of cfx_fused.cu: same bits.
 // Tiles of 32 rows (ONE), the smallest batches: a quadrant of TMEM lanes belongs to one SM scheduler, so one
-// quadrant of rows would leave three schedulers idle.  The operand chunks go to shared memory instead, one of the sixteen
-// warps a chunk, and all multiplications are the weight-stationary ones of 32 rows: their columns are spread over the
+// quadrant of rows would leave three schedulers idle.  The operand chunks go to shared memory instead, all
+// sixteen warps at three of them at a time, and all multiplications are the weight-stationary ones of 32 rows: their columns are spread over the
 // quadrants, so every warp has four of a slice's units, and they are shorter (an encoder step 29 cycles instead of 49,
 // one of the gates 73 instead of 96).  A slice's zh and zg are one product of 128 columns and its zp one of 64; the weights' copies
 // put the units of a quadrant together (1,024 envs h256x2 12.7 -> 11.6 us, against products of 128 rows with a copy of the layer
@@ -69,6 +69,12 @@ constexpr int kQuadBlock = 32 * 128;                  // ONE: an operand chunk's
 constexpr uint32_t kGateB = 4 * 2 * kWarpUnits * 128;   // ONE: zh and zg of a slice, behind them its zp
 constexpr uint32_t kColP = 32;                        // ONE: columns of zh and zg in a quadrant, behind them zp
 
+// ONE, full game: the twelve chunks of map bytes are converted three at a time, which are the blocks of a ring slot, by twelve warps with a
+// quarter of a chunk each, the tail's four meanwhile by the other four, one to an SM scheduler.  The multiplications of a slot run under the
+// conversion of the next one.  (A chunk a warp, and the multiplications behind all of them: the last chunk was there 1,500 cycles after the records, and
+// the encoder done 2,400 later; now 3,200 after the records.  32 envs h256x2 9.42 -> 9.25 us, 512 10.0 -> 9.7, h128x2 8.65 -> 8.34.)
+constexpr int kMapItems = 4, kMapWarps = 12;
+
 template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kKB = HID / 64;                        // K blocks of a layer's input
     static constexpr int kNS = HID / 64 / S;                    // gate slices of a CTA
@@ -80,12 +86,10 @@ template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kEncPieces = kNS * Gm<GAME>::kEncBlocks, kEncPerItem = kWSlot / kSlicePiece;
     static constexpr int kEncItems = (kEncPieces + kEncPerItem - 1) / kEncPerItem;
     static_assert(kEncPerItem * kSlicePiece == kWSlot && kWSlots * kEncPerItem % kNS == 0, "a block's pieces do not wrap around the ring");
-    // ONE: ring slots whose operand chunks the MMA warp waits for together: the full game's sixteen chunks, a warp each, are there
-    // at the same time (1,024 envs 10.8 us, 11.0 with a wait a slot, 11.6 with one a chunk); the classic game's 22 are not, and it
-    // makes no difference (13.3 with two waits for all of them, 13.1 with one a slot, 13.0 with one a chunk, runs 0.2 apart)
-    static constexpr int kGroupItems = GAME == CFX_GAME_FULL ? kEncItems : 1;
-    static __device__ __forceinline__ int group_chunks(int group) {
-        return GAME == CFX_GAME_FULL ? Gm<GAME>::kEncChunks : max(1, min(kEncPerItem, Gm<GAME>::kEncBlocks - group * kEncPerItem));
+    // ONE: how many warps bring the operand chunks of a ring slot
+    static __device__ __forceinline__ int item_warps(int item) {
+        if (GAME == CFX_GAME_FULL) return item < kMapItems ? kMapWarps : kWorkerWarps - kMapWarps;
+        return max(1, min(kEncPerItem, Gm<GAME>::kEncBlocks - item * kEncPerItem));
     }
     static constexpr int kHeadHalf = Gm<GAME>::kHeadPair / 2 * 128;   // half of the head rows, one K block
     static constexpr int kHeadItems = kKB / 2;                  // two K blocks of the heads a slot
@@ -246,15 +250,15 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
     CFX_SPROBE(cfx_p_b, W_FULL, 0);
     CFX_SPROBE(cfx_p_a, AEXP_FULL, 0);
     if constexpr (ONE) {
-        // the warps convert a chunk each at the same time: one wait for many of them, and the steps of a ring slot in one run
+        // a wait for the operand chunks of a ring slot, and the steps of the slot in one run
 #pragma unroll
         for (int item = 0; item < C::kEncItems; item++) {
             const int slot = item % kWSlots, blk0 = item * C::kEncPerItem;
             constexpr int kBlocks = Gm<GAME>::kEncBlocks;
             CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, (item / kWSlots) & 1);
             CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
-            if (item % C::kGroupItems == 0) CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + item / C::kGroupItems, 0);
-            if ((item + 1) % C::kGroupItems == 0 && item + 1 < C::kEncItems) CFX_SPROBE(cfx_p_a, AEXP_FULL + (item + 1) / C::kGroupItems, 0);
+            CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + item, 0);
+            if (item + 1 < C::kEncItems) CFX_SPROBE(cfx_p_a, AEXP_FULL + item + 1, 0);
             tc_fence_after_sync();
             __syncwarp();
             if (elect_one()) {
@@ -701,8 +705,8 @@ __device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t h
     }
 }
 
-// ONE: warp w = (quadrant, wg) converts chunk w (and the one 16 further) and handles units [4 w, 4 w + 4) of the CTA's
-// slice, which are in its quadrant of tensor memory; lane = row in all of it.
+// ONE: warp w = (quadrant, wg) converts its part of the record (kMapItems; classic game: chunk w and the one 16 further) and handles units
+// [4 w, 4 w + 4) of the CTA's slice, which are in its quadrant of tensor memory; lane = row in all of it.
 template <typename T16, int GAME, int HID, int S>
 __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
                                                 uint32_t rank, Meetings& meet) {
@@ -727,20 +731,43 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
 
     // ---- expand: K columns of a chunk go to the columns that its weight block has for them
     CFX_SWAIT(REC_FULL, 0);
-    for (int kc = w; kc < kChunks; kc += kWorkerWarps) {
-        uint32_t regs[32];
-        const uint8_t* rec = sm.base + lane * C::kRowBytes;
-        if constexpr (kFull) expand_full<Op>(rec + 64 * kc, kc, regs);
-        else expand_classic<Op>(rec, kc, regs);
-        const int blk = kFull && kc >= 12 ? (kc < 14 ? 12 : 13) : kc;
-        const int first = kFull && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0, pieces = 2 * (kFull ? full_ksteps(kc) : 4);
-#pragma unroll
-        for (int c = 0; c < 8; c++)
-            if (c < pieces)
-                *reinterpret_cast<uint4*>(piece(C::kOffX + blk * kQuadBlock, first + c)) = make_uint4(regs[4 * c], regs[4 * c + 1], regs[4 * c + 2], regs[4 * c + 3]);
+    const uint8_t* rec = sm.base + lane * C::kRowBytes;
+    auto operand = [&](int blk, int c, const uint32_t* r) {   // 16-byte piece c of this row in a block
+        *reinterpret_cast<uint4*>(piece(C::kOffX + blk * kQuadBlock, c)) = make_uint4(r[0], r[1], r[2], r[3]);
+    };
+    auto converted = [&](int item) {
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + blk / C::kEncPerItem / C::kGroupItems));
+        if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + item));
+    };
+    if (kFull && wg < 3) {
+        static_assert(C::kEncPerItem == 3 && kMapWarps == 3 * 4 && kMapItems * 3 == 12, "a warp a quarter of a chunk");
+        uint32_t bytes[kMapItems][4];
+#pragma unroll
+        for (int i = 0; i < kMapItems; i++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) bytes[i][q] = *reinterpret_cast<const uint32_t*>(rec + 64 * (3 * i + wg) + 16 * quadrant + 4 * q);
+#pragma unroll
+        for (int i = 0; i < kMapItems; i++) {
+            uint32_t regs[8];
+#pragma unroll
+            for (int q = 0; q < 4; q++) Op::bytes4(bytes[i][q], regs[2 * q], regs[2 * q + 1]);
+            operand(3 * i + wg, 2 * quadrant, regs);
+            operand(3 * i + wg, 2 * quadrant + 1, regs + 4);
+            converted(i);
+        }
+    } else {
+        for (int kc = kFull ? 12 + quadrant : w; kc < kChunks; kc += kWorkerWarps) {
+            uint32_t regs[32];
+            if constexpr (kFull) expand_full<Op>(rec + 64 * kc, kc, regs);
+            else expand_classic<Op>(rec, kc, regs);
+            const int blk = kFull ? (kc < 14 ? 12 : 13) : kc;
+            const int first = kFull ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0, pieces = 2 * (kFull ? full_ksteps(kc) : 4);
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                if (c < pieces) operand(blk, first + c, regs + 4 * c);
+            converted(blk / C::kEncPerItem);
+        }
     }
     auto free_records = [&]() {
         __syncwarp();
@@ -860,7 +887,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         if (i < NUM_BARS) {
             uint32_t arrivals = 1, bytes = 0;
             if (i == REC_FREE) arrivals = ONE ? S * kWorkerWarps : S * 4 * quads;
-            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::group_chunks(i - AEXP_FULL) : max(1, min(4, Gm<GAME>::kEncChunks - 4 * (i - AEXP_FULL))) * quads;
+            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::item_warps(i - AEXP_FULL) : max(1, min(4, Gm<GAME>::kEncChunks - 4 * (i - AEXP_FULL))) * quads;
             else if (i == ACC_FULL) arrivals = 2;                          // the MMAs, and the biases are in place
             else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = ONE ? 8 : 2 * quads;
             else if (i == MMA_DONE) arrivals = S;
