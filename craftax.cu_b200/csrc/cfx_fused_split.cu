@@ -124,7 +124,7 @@ enum Bar {
     NUM_BARS = A_KB + (kMaxLayers + 1) * 4
 };
 template <int GAME, int HID, int S> constexpr int smem_bytes() {
-    return Cfg<GAME, HID, S>::kOffBars + NUM_BARS * 8 + 16 + 1024;   // misc, alignment slack
+    return Cfg<GAME, HID, S>::kOffBars + NUM_BARS * 8 + 16 + 128 + 1024;   // misc, uniforms, alignment slack
 }
 static_assert(smem_bytes<CFX_GAME_FULL, 256, 2>() <= 232448 && smem_bytes<CFX_GAME_FULL, 128, 2>() <= 232448, "shared memory");
 
@@ -136,6 +136,7 @@ struct Smem {
     uint32_t bars;   // shared address of the barriers
     __device__ __forceinline__ uint32_t bar(int i) const { return bars + 8u * (uint32_t)i; }
     __device__ __forceinline__ uint32_t* tmem_base() const { return reinterpret_cast<uint32_t*>(base + off_bars + NUM_BARS * 8); }
+    __device__ __forceinline__ float* uniforms() const { return reinterpret_cast<float*>(tmem_base() + 4); }   // ONE: of the tile's envs
     __device__ __forceinline__ volatile uint32_t* abort_flag() const { return tmem_base() + 1; }
 };
 // one lane waits (CFX_SWAIT1), or a whole warp (the MMA warp by polling alone)
@@ -659,9 +660,9 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
 // exponentials to shared memory, then the first one sums, searches and draws, and the others write the logits.  All of it by
 // one warp is the longest stretch of straight-line code in the chain of a step; with every warp taking the maximum of a
 // whole row, and a sixteenth of the exponentials, 1,024 envs took 14.3 us instead of 13.8.
-// `head`: tensor memory of this warp's lanes, `env`: of the lane; `u`: its uniform, in the first warp
+// `head`: tensor memory of this warp's lanes, `env`: of the lane; `uniforms`: of the rows
 template <int GAME>
-__device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t head, const float* bias, int w, int lane, int env, float u,
+__device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t head, const float* bias, int w, int lane, int env, const float* uniforms,
                                            Meetings& meet) {
     constexpr int kA = Gm<GAME>::kA, kCols = 4, kWith = (kA + kCols) / kCols, kPitch = 33, W = kWorkerWarps;
     static_assert(kWith <= W && ((kA + 1) * kPitch + (kA + kWith) * 32) * 4 <= kWSlots * kWSlot, "scratch");
@@ -700,7 +701,7 @@ __device__ __forceinline__ void sample_one(const Params& P, float* s, uint32_t h
         float pr[kA], total;
 #pragma unroll
         for (int a = 0; a < kA; a++) pr[a] = p[a * 32];
-        const int act = draw_action<kA>(pr, u, &total, [](int, bool) {});
+        const int act = draw_action<kA>(pr, uniforms[lane], &total, [](int, bool) {});
         write_action(P, env, act, s[act * kPitch + lane] - m - logf(total), s[kA * kPitch + lane]);
     }
 }
@@ -719,8 +720,6 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     const int env = row0 + lane;
     const bool valid = env < P.n;   // all rows (n is a multiple of 32)
     const float* bias = reinterpret_cast<const float*>(sm.base + C::kOffBias);
-    const bool draws = rank == 0 && w == 0;
-    const unsigned long long step0 = draws && P.uniforms == nullptr ? *P.step_ctr : 0ull;
     const bool zero_state = valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
     if (lane < 2 * P.L)   // two rows of the state, on their way to L2 while the records are expanded
 #pragma unroll
@@ -774,12 +773,6 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         if (lane < S) mbar_arrive_cluster(map_to_cta(sm.bar(REC_FREE), (uint32_t)lane));
     };
     if (kFull && !C::kOneBeside) free_records();
-    if (draws) {   // (see role_worker)
-        asm volatile("" ::"l"(step0));
-        __syncwarp();
-        if (lane == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
-    }
-
     // Layer input l: the CTA's own K block is complete when all warps are here; then it goes to the other CTAs.
     auto send = [&](int l) {
         tc_fence_before_sync();
@@ -814,8 +807,6 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
         *xp(0) = x;
     }
     if (!send(0)) return;
-    float u = 0.0f;
-    if (draws) u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
 
     // ---- layers
     for (int l = 0; l < P.L; l++) {
@@ -857,7 +848,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     if (rank == 0) {
         CFX_SWAIT(H_FULL, 0);
         tc_fence_after_sync();
-        if (valid) sample_one<GAME>(P, reinterpret_cast<float*>(sm.base + C::kOffW), lane_base + kColHead + 4 * wg, bias + C::kUnits, w, lane, env, u, meet);
+        if (valid) sample_one<GAME>(P, reinterpret_cast<float*>(sm.base + C::kOffW), lane_base + kColHead + 4 * wg, bias + C::kUnits, w, lane, env, sm.uniforms(), meet);
     }
     meet.met = Meetings::kAll;
 }
@@ -942,8 +933,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
                 reinterpret_cast<float*>(sm.base + C::kOffBias)[i] =
                     P.params[a < 0 ? P.off_b_enc + C::slice((int)rank, i / kSliceUnits) * kSliceUnits + i % kSliceUnits : (a < kA ? P.off_b_a + a : P.off_b_v)];
             }
+            // ONE: the uniforms of the tile's envs and the step counter, which the worker that samples raised under the encoder's products
+            // until those ended before it was done (512 envs h256x2 9.82 -> 9.72 us, h128x2 8.33 -> 8.17)
+            const bool draws = ONE && rank == 0;
+            if (draws) {
+                const int env = row0 + lane;   // (n is a multiple of 32)
+                sm.uniforms()[lane] = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, *P.step_ctr);
+            }
             __syncwarp();
-            if (lane == 0) mbar_arrive(sm.bar(ACC_FULL));
+            if (lane == 0) {
+                mbar_arrive(sm.bar(ACC_FULL));
+                if (draws && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
+            }
             __syncwarp();
             cluster_wait();
         } else if (warp == 3) {
