@@ -107,6 +107,14 @@ template <int GAME, int HID, int S> struct Cfg {
     static __device__ __forceinline__ uint32_t one_block(int l, int kb) {
         return (kOneBeside ? 32768 + kb * 2 * kQuadBlock : kb * kABlock) + (l & 1) * kQuadBlock;
     }
+    // ONE, full game: the encoder's last two blocks, which the ring has no slots for, lie behind the operand chunks and, where there is room for one
+    // alone, in the CTA's own blocks of the layer inputs, which it writes when the encoder is done
+    template <bool ONE> static constexpr int ring_items() { return ONE && GAME == CFX_GAME_FULL ? kWSlots : kEncItems; }
+    static_assert(kOffX + Gm<GAME>::kEncBlocks * kQuadBlock + (GAME == CFX_GAME_FULL ? kOneBeside ? 1 : 2 : 0) * kSlicePiece <= kOffW, "last blocks");
+    static __device__ __forceinline__ uint32_t last_block(int blk, uint32_t rank) {
+        constexpr uint32_t behind = kOffX + Gm<GAME>::kEncBlocks * kQuadBlock;
+        return blk == kWSlots * kEncPerItem ? behind : (kOneBeside ? one_block(0, (int)rank) : behind + kSlicePiece);
+    }
     static constexpr int kOffBias = kOffW + kWSlots * kWSlot;
     static constexpr int kOffBars = kOffBias + (kUnits + kHeadMax) * 4;
     static_assert(kNS >= 1 && kNS <= 2 && kUnits * S == HID &&
@@ -115,18 +123,19 @@ template <int GAME, int HID, int S> struct Cfg {
 };
 
 enum Bar {
-    W_FULL = 0, W_EMPTY = W_FULL + kWSlots, REC_FULL = W_EMPTY + kWSlots, REC_FREE = REC_FULL + 4,
+    W_FULL = 0, W_LAST = W_FULL + kWSlots, W_EMPTY = W_LAST + 1, REC_FULL = W_EMPTY + kWSlots, REC_FREE = REC_FULL + 4,
     AEXP_FULL = REC_FREE + 1, AEXP_EMPTY = AEXP_FULL + kMaxChunks, ACC_FULL = AEXP_EMPTY + kASlots,
     S_FULL = ACC_FULL + 1, ST_READY = S_FULL + kSSlots, MMA_DONE = ST_READY + kSSlots,
     QUAD = MMA_DONE + 1, G_FULL = QUAD + 8,   // QUAD: [slice][quadrant]
     H_FULL = G_FULL + 2, A_KB = H_FULL + 1,
-    // A_KB: [layer input][K block]
+    // A_KB: [layer input][K block]; ONE: [layer input][0] for all of its blocks, but not for those of the heads' input
     NUM_BARS = A_KB + (kMaxLayers + 1) * 4
 };
 template <int GAME, int HID, int S> constexpr int smem_bytes() {
     return Cfg<GAME, HID, S>::kOffBars + NUM_BARS * 8 + 16 + 128 + 1024;   // misc, uniforms, alignment slack
 }
-static_assert(smem_bytes<CFX_GAME_FULL, 256, 2>() <= 232448 && smem_bytes<CFX_GAME_FULL, 128, 2>() <= 232448, "shared memory");
+static_assert(smem_bytes<CFX_GAME_FULL, 256, 2>() <= 232448 && smem_bytes<CFX_GAME_FULL, 128, 2>() <= 232448 && smem_bytes<CFX_GAME_FULL, 256, 4>() <= 232448 &&
+                  smem_bytes<CFX_GAME_CLASSIC, 256, 4>() <= 232448, "shared memory");
 
 constexpr uint32_t kSite = 0x40;   // wait-site codes: kSite + barrier
 
@@ -184,7 +193,8 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
     constexpr int kSlices = HID / 64;
     constexpr size_t enc_b = enc_bytes<GAME, HID>();
     const int gates = P.L * C::kNS * C::kKB;
-    const int items = C::kEncItems + gates + (has_heads<S, ONE>(P.tile_rows / 32, rank) ? C::kHeadItems : 0);
+    constexpr int kEnc = C::template ring_items<ONE>();
+    const int items = kEnc + gates + (has_heads<S, ONE>(P.tile_rows / 32, rank) ? C::kHeadItems : 0);
     const uint32_t ring = smem_u32(sm.base + C::kOffW);
     for (int i = 0; i < items; i++) {
         const int slot = i % kWSlots, slot1 = (i + 1) % kWSlots;
@@ -197,15 +207,20 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
         __syncwarp();
         if (!elect_one()) continue;
         const uint32_t dst = ring + slot * kWSlot, full = sm.bar(W_FULL + slot);
-        if (i < C::kEncItems) {
+        if (i < kEnc) {
             const int pieces = min(C::kEncPerItem, C::kEncPieces - i * C::kEncPerItem);
             mbar_arrive_expect_tx(full, pieces * kSlicePiece);
             for (int q = 0; q < pieces; q++) {
                 const int p = i * C::kEncPerItem + q, blk = p / C::kNS, slice = C::slice((int)rank, p % C::kNS);
                 bulk_g2s(dst + q * kSlicePiece, P.image + (size_t)blk * Hd<HID>::kEncBlockBytes + (size_t)slice * kSlicePiece, kSlicePiece, full);
             }
-        } else if (i < C::kEncItems + gates) {
-            const int g = i - C::kEncItems, kb = g % C::kKB, j = g / C::kKB % C::kNS, l = g / (C::kKB * C::kNS);
+            if (kEnc < C::kEncItems && i == kEnc - 1) {
+                mbar_arrive_expect_tx(sm.bar(W_LAST), (C::kEncPieces - kEnc * C::kEncPerItem) * kSlicePiece);
+                for (int blk = kEnc * C::kEncPerItem; blk < C::kEncPieces; blk++)
+                    bulk_g2s(smem_u32(sm.base) + C::last_block(blk, rank), P.image + (size_t)blk * Hd<HID>::kEncBlockBytes + (size_t)rank * kSlicePiece, kSlicePiece, sm.bar(W_LAST));
+            }
+        } else if (i < kEnc + gates) {
+            const int g = i - kEnc, kb = g % C::kKB, j = g / C::kKB % C::kNS, l = g / (C::kKB * C::kNS);
             const int blk = (l * kSlices + C::slice((int)rank, j)) * C::kKB + kb;
             mbar_arrive_expect_tx(full, kGateBlockBytes);
             const uint8_t* src = P.image + enc_b + (size_t)blk * kGateBlockBytes;
@@ -217,7 +232,7 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
                 bulk_g2s(dst + kGateBlockBytes / 2, src + kGateBlockBytes / 2, kGateBlockBytes / 2, full);
             }
         } else {
-            const int h = i - C::kEncItems - gates;
+            const int h = i - kEnc - gates;
             const uint8_t* src = P.image + enc_b + (size_t)P.L * kSlices * C::kKB * kGateBlockBytes;
             mbar_arrive_expect_tx(full, 4 * C::kHeadHalf);
 #pragma unroll
@@ -235,85 +250,53 @@ __device__ __forceinline__ void role_weights(const Smem& sm, const Params& P, ui
 // position is a compile-time constant and every descriptor one addition away from two bases: an MMA whose descriptor is
 // computed takes ~150 cycles to issue, and 54 of them were two thirds of the encoder.  The barriers of the next step are
 // probed before the current step's MMAs (CFX_PROBE), so that a probe's round trip runs under their issue.
-template <typename T16, int GAME, int HID, int S, bool ONE>
+template <typename T16, int GAME, int HID, int S>
 __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32_t tmem, uint32_t rank) {
     using C = Cfg<GAME, HID, S>;
     constexpr uint32_t fmt = Op16<T16>::kFmt;
-    constexpr int kRows = ONE ? 32 : kTile;
-    constexpr uint32_t idesc_enc = make_idesc(fmt, kRows, C::kUnits), idesc_gate = make_idesc(fmt, kTile, 3 * kSliceUnits),
-                       idesc_hg = make_idesc(fmt, kRows, 2 * kSliceUnits), idesc_p = make_idesc(fmt, kRows, kSliceUnits),
-                       idesc_head = make_idesc(fmt, kRows, ONE ? 64 : Gm<GAME>::kHeadSingle);   // (M = 32 takes N = 64, 128 or 256)
+    constexpr uint32_t idesc_enc = make_idesc(fmt, kTile, C::kUnits), idesc_gate = make_idesc(fmt, kTile, 3 * kSliceUnits),
+                       idesc_head = make_idesc(fmt, kTile, Gm<GAME>::kHeadSingle);
     constexpr int kChunks = Gm<GAME>::kEncChunks, kGateItems = C::kNS * C::kKB;
     static_assert(kGateItems % kWSlots == 0 || kWSlots % kGateItems == 0, "a layer's first ring slot");
     const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
-    const uint64_t xdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffX));
     // ---- encoder
     CFX_SPROBE(cfx_p_b, W_FULL, 0);
     CFX_SPROBE(cfx_p_a, AEXP_FULL, 0);
-    if constexpr (ONE) {
-        // a wait for the operand chunks of a ring slot, and the steps of the slot in one run
 #pragma unroll
-        for (int item = 0; item < C::kEncItems; item++) {
-            const int slot = item % kWSlots, blk0 = item * C::kEncPerItem;
-            constexpr int kBlocks = Gm<GAME>::kEncBlocks;
-            CFX_SWAIT_PROBED(cfx_p_b, W_FULL + slot, (item / kWSlots) & 1);
-            CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
-            CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + item, 0);
-            if (item + 1 < C::kEncItems) CFX_SPROBE(cfx_p_a, AEXP_FULL + item + 1, 0);
-            tc_fence_after_sync();
-            __syncwarp();
-            if (elect_one()) {
+    for (int kc = 0; kc < kChunks; kc++) {
+        // block of 64 K columns, first of its 16-byte K pieces, K steps (see expand_full), last chunk of its block
+        const bool full = GAME == CFX_GAME_FULL;
+        const int blk = full && kc >= 12 ? (kc < 14 ? 12 : 13) : kc, first = full && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0;
+        const int ks = full ? full_ksteps(kc) : (kc == kChunks - 1 ? 1 : 4);
+        const bool starts = !(full && (kc == 13 || kc == 15)), ends = !(full && (kc == 12 || kc == 14));
+        const int as = kc % kASlots, piece = blk * C::kNS;
+        if (starts)
 #pragma unroll
-                for (int b = 0; b < C::kEncPerItem; b++) {
-                    const int blk = blk0 + b, last = kBlocks - 1;
-                    if (blk > last) break;
-                    const int ks = blk < last ? 4 : (GAME == CFX_GAME_FULL ? 2 : 1);
-#pragma unroll
-                    for (int k = 0; k < ks; k++)
-                        mma_f16_ws_ss(tmem + kColAcc, xdesc + (uint64_t)((blk * kQuadBlock) >> 4) + 2 * k,
-                                      wdesc + (uint64_t)((slot * kWSlot + b * kSlicePiece) >> 4) + 2 * k, idesc_enc, (blk | k) != 0 ? 1u : 0u);
-                }
-                if (item == C::kEncItems - 1) mma_commit(sm.bar(ACC_FULL));
-                mma_commit(sm.bar(W_EMPTY + slot));
+            for (int p = piece; p < piece + C::kNS; p++) {
+                const int item = p / C::kEncPerItem;
+                if (p % C::kEncPerItem != 0) continue;   // waited for with an earlier piece
+                CFX_SWAIT_PROBED(cfx_p_b, W_FULL + item % kWSlots, (item / kWSlots) & 1);
+                CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
             }
+        // (four chunks, one of each warpgroup, are there at the same time)
+        if (kc % 4 == 0) {
+            CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + kc / 4, 0);
+            if (kc + 4 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + kc / 4 + 1, 0);
         }
-    } else {
+        tc_fence_after_sync();
+        __syncwarp();
+        const uint64_t bd = wdesc + (uint64_t)((piece % (kWSlots * C::kEncPerItem) * kSlicePiece >> 4) + first);
+        const uint32_t a = tmem + kColAexp + as * 32;
+        if (elect_one()) {
 #pragma unroll
-        for (int kc = 0; kc < kChunks; kc++) {
-            // block of 64 K columns, first of its 16-byte K pieces, K steps (see expand_full), last chunk of its block
-            const bool full = GAME == CFX_GAME_FULL;
-            const int blk = full && kc >= 12 ? (kc < 14 ? 12 : 13) : kc, first = full && kc >= 12 ? (kc == 13 ? 6 : (kc == 15 ? 2 : 0)) : 0;
-            const int ks = full ? full_ksteps(kc) : (kc == kChunks - 1 ? 1 : 4);
-            const bool starts = !(full && (kc == 13 || kc == 15)), ends = !(full && (kc == 12 || kc == 14));
-            const int as = kc % kASlots, piece = blk * C::kNS;
-            if (starts)
+            for (int k = 0; k < ks; k++)
+                mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
+            if (kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
+            if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
+            if (ends)
 #pragma unroll
-                for (int p = piece; p < piece + C::kNS; p++) {
-                    const int item = p / C::kEncPerItem;
-                    if (p % C::kEncPerItem != 0) continue;   // waited for with an earlier piece
-                    CFX_SWAIT_PROBED(cfx_p_b, W_FULL + item % kWSlots, (item / kWSlots) & 1);
-                    CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
-                }
-            // (four chunks, one of each warpgroup, are there at the same time)
-            if (kc % 4 == 0) {
-                CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + kc / 4, 0);
-                if (kc + 4 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + kc / 4 + 1, 0);
-            }
-            tc_fence_after_sync();
-            __syncwarp();
-            const uint64_t bd = wdesc + (uint64_t)((piece % (kWSlots * C::kEncPerItem) * kSlicePiece >> 4) + first);
-            const uint32_t a = tmem + kColAexp + as * 32;
-            if (elect_one()) {
-#pragma unroll
-                for (int k = 0; k < ks; k++)
-                    mma_f16_ts(tmem + kColAcc, a + 8 * k, bd + 2 * k, idesc_enc, (kc | k) != 0 ? 1u : 0u);
-                if (kc + kASlots < kChunks) mma_commit(sm.bar(AEXP_EMPTY + as));
-                if (kc == kChunks - 1) mma_commit(sm.bar(ACC_FULL));
-                if (ends)
-#pragma unroll
-                    for (int p = piece; p < piece + C::kNS; p++)
-                        if ((p + 1) % C::kEncPerItem == 0 || p == C::kEncPieces - 1) mma_commit(sm.bar(W_EMPTY + p / C::kEncPerItem % kWSlots));
-            }
+                for (int p = piece; p < piece + C::kNS; p++)
+                    if ((p + 1) % C::kEncPerItem == 0 || p == C::kEncPieces - 1) mma_commit(sm.bar(W_EMPTY + p / C::kEncPerItem % kWSlots));
         }
     }
     // ---- layers and heads (a loop over the layers: straight-line code for all of them would be fetched cold)
@@ -325,19 +308,16 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
 #pragma unroll 1
     for (int l = 0; l < P.L; l++) {
         const int slot0 = first_slot(l);
-        if (!ONE) CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
+        CFX_SPROBE(cfx_p_a, A_KB + 4 * l, 0);
         // this CTA's own K block of slice 0 first: that slice's gate columns are free when its cells have read them (those of slice 1
         // when its own block is there, which is waited for with the others)
         CFX_SWAIT_SPIN(A_KB + 4 * l + C::slice((int)rank, 0), 0);
-        if (ONE)   // the blocks of the other CTAs come at about the same time
-#pragma unroll
-            for (int kb = 0; kb < C::kKB; kb++) CFX_SWAIT_SPIN(A_KB + 4 * l + kb, 0);
 #pragma unroll
         for (int j = 0; j < C::kNS; j++) {
 #pragma unroll
             for (int kb = 0; kb < C::kKB; kb++) {
                 const int slot = (slot0 + j * C::kKB + kb) % kWSlots, slot1 = (slot + 1) % kWSlots;
-                if (!ONE && j == 0) {
+                if (j == 0) {
                     CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * l + kb, 0);
                     if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * l + kb + 1, 0);
                 }
@@ -346,24 +326,18 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                 CFX_SPROBE(cfx_p_b, W_FULL + slot1, wpar >> slot1 & 1u);
                 tc_fence_after_sync();
                 __syncwarp();
-                const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)((ONE ? C::one_block(l, kb) : (uint32_t)(kb * kABlock)) >> 4);
+                const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
                 if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 4; ks++) {
-                        if constexpr (ONE) {
-                            mma_f16_ws_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_hg, (kb | ks) != 0 ? 1u : 0u);
-                            mma_f16_ws_ss(tmem + col_gate(j) + kColP, ad + 2 * ks, bd + (uint64_t)(kGateB >> 4) + 2 * ks, idesc_p, (kb | ks) != 0 ? 1u : 0u);
-                        } else
-                            mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
-                    }
+                    for (int ks = 0; ks < 4; ks++) mma_f16_ss(tmem + col_gate(j), ad + 2 * ks, bd + 2 * ks, idesc_gate, (kb | ks) != 0 ? 1u : 0u);
                     if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL + j));
-                    if (!ONE && j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
+                    if (j == C::kNS - 1 && kb == C::kKB - 1) mma_commit_all<S>(sm.bar(MMA_DONE));
                     mma_commit(sm.bar(W_EMPTY + slot));
                 }
             }
         }
     }
-    if (__builtin_expect(!has_heads<S, ONE>(P.tile_rows / 32, rank), 0)) {
+    if (__builtin_expect(!has_heads<S, false>(P.tile_rows / 32, rank), 0)) {
         // no heads here: what is on its way to this CTA (the last layer's output) or was issued by it is only waited for
         for (int kb = 0; kb < C::kKB; kb++) CFX_SWAIT(A_KB + 4 * P.L + kb, 0);
         __syncwarp();
@@ -384,15 +358,116 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
         }
         tc_fence_after_sync();
         __syncwarp();
-        const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)((ONE ? C::one_block(P.L, kb) : (uint32_t)(kb * kABlock)) >> 4);
+        const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)((kb * kABlock) >> 4);
         if (elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < 4; ks++) {
-                if constexpr (ONE)
-                    mma_f16_ws_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
-                else
-                    mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+            for (int ks = 0; ks < 4; ks++) mma_f16_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_head, (kb | ks) != 0 ? 1u : 0u);
+            if (kb == C::kKB - 1) mma_commit(sm.bar(H_FULL));
+        }
+    }
+}
+
+// ONE: a layer's weights are waited for while its input is on its way, and its input is one wait for all of its blocks, so that the 32 products of
+// a layer are one run, as long as the issue of its products takes (the blocks come at about the same time; with a wait for each, and the weights' waits between
+// them, 120 cycles a block).  The encoder's weights are waited for slot by slot: a CTA that starts where another one has ended has the first ones
+// 400 cycles before the last.  The heads take their input block by block, as the first one is their CTA's own and there 900 cycles before the others (in one
+// run 0.2 us slower).  us a step, h256x1 / x2 / x4 at 512 envs 7.92 / 9.76 / 13.45 -> 7.69 / 9.38 / 12.78, 32 envs h256x2 9.14 -> 8.74, 1,056 10.25 -> 9.97,
+// h128x2 512 8.17 -> 7.93, classic h256x3 512 13.98 -> 13.49; of that 0.1 to 0.15 by the encoder's last blocks beside the ring (last_block), without
+// which the first layer's last weights come late.
+template <typename T16, int GAME, int HID, int S>
+__device__ __forceinline__ void role_mma_one(const Smem& sm, const Params& P, uint32_t tmem, uint32_t rank) {
+    using C = Cfg<GAME, HID, S>;
+    constexpr uint32_t fmt = Op16<T16>::kFmt;
+    // (M = 32 takes N = 64, 128 or 256)
+    constexpr uint32_t idesc_64 = make_idesc(fmt, 32, kSliceUnits), idesc_hg = make_idesc(fmt, 32, 2 * kSliceUnits);
+    constexpr int kBlocks = Gm<GAME>::kEncBlocks, kEnc = C::template ring_items<true>();
+    static_assert(C::kUnits == kSliceUnits && C::kKB <= kWSlots && C::kHeadItems <= kWSlots, "a layer's weights are in the ring at once");
+    const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
+    const uint64_t xdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffX));
+    // ---- encoder
+    CFX_SPROBE(cfx_p_b, W_FULL, 0);
+    CFX_SPROBE(cfx_p_a, AEXP_FULL, 0);
+#pragma unroll
+    for (int item = 0; item < C::kEncItems; item++) {
+        const int slot = item % kWSlots;
+        CFX_SWAIT_PROBED(cfx_p_b, item < kEnc ? W_FULL + slot : W_LAST, item < kEnc ? (item / kWSlots) & 1 : 0);
+        if (item + 1 < C::kEncItems) CFX_SPROBE(cfx_p_b, item + 1 < kEnc ? W_FULL + (item + 1) % kWSlots : W_LAST, item + 1 < kEnc ? ((item + 1) / kWSlots) & 1 : 0);
+        CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + item, 0);
+        if (item + 1 < C::kEncItems) CFX_SPROBE(cfx_p_a, AEXP_FULL + item + 1, 0);
+        tc_fence_after_sync();
+        __syncwarp();
+        if (elect_one()) {
+#pragma unroll
+            for (int b = 0; b < C::kEncPerItem; b++) {
+                const int blk = item * C::kEncPerItem + b, last = kBlocks - 1;
+                if (blk > last) break;
+                const int ks = blk < last ? 4 : (GAME == CFX_GAME_FULL ? 2 : 1);
+                const uint64_t bd = item < kEnc ? wdesc + (uint64_t)((slot * kWSlot + b * kSlicePiece) >> 4) : adesc + (uint64_t)(C::last_block(blk, rank) >> 4);
+#pragma unroll
+                for (int k = 0; k < ks; k++)
+                    mma_f16_ws_ss(tmem + kColAcc, xdesc + (uint64_t)((blk * kQuadBlock) >> 4) + 2 * k, bd + 2 * k, idesc_64, (blk | k) != 0 ? 1u : 0u);
             }
+            if (item == C::kEncItems - 1) mma_commit(sm.bar(ACC_FULL));
+            if (item < kEnc) mma_commit(sm.bar(W_EMPTY + slot));
+        }
+    }
+    // ---- layers (a loop: straight-line code for all of them would be fetched cold)
+    uint32_t wpar = 0;   // parity bit of every ring slot
+#pragma unroll
+    for (int i = 0; i < kEnc; i++) wpar ^= 1u << (i % kWSlots);
+    // the ring slot of a layer's first item: the same for every layer where its items are whole rounds of the ring
+    auto first_slot = [&](int l) { return C::kKB % kWSlots == 0 ? kEnc % kWSlots : (kEnc + l * C::kKB) % kWSlots; };
+#pragma unroll 1
+    for (int l = 0; l < P.L; l++) {
+        const int slot0 = first_slot(l);
+#pragma unroll
+        for (int kb = 0; kb < C::kKB; kb++) {
+            const int slot = (slot0 + kb) % kWSlots;
+            CFX_SWAIT_SPIN(W_FULL + slot, wpar >> slot & 1u);
+            wpar ^= 1u << slot;
+        }
+        CFX_SWAIT_SPIN(A_KB + 4 * l, 0);
+        tc_fence_after_sync();
+        __syncwarp();
+        if (elect_one()) {
+#pragma unroll
+            for (int kb = 0; kb < C::kKB; kb++) {
+                const int slot = (slot0 + kb) % kWSlots;
+                const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot) >> 4), ad = adesc + (uint64_t)(C::one_block(l, kb) >> 4);
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++) {
+                    mma_f16_ws_ss(tmem + col_gate(0), ad + 2 * ks, bd + 2 * ks, idesc_hg, (kb | ks) != 0 ? 1u : 0u);
+                    mma_f16_ws_ss(tmem + col_gate(0) + kColP, ad + 2 * ks, bd + (uint64_t)(kGateB >> 4) + 2 * ks, idesc_64, (kb | ks) != 0 ? 1u : 0u);
+                }
+                if (kb == C::kKB - 1) mma_commit(sm.bar(G_FULL));
+                mma_commit(sm.bar(W_EMPTY + slot));
+            }
+        }
+    }
+    if (__builtin_expect(!has_heads<S, true>(1, rank), 0)) {
+        // no heads here: what is on its way to this CTA (the last layer's output) or was issued by it is only waited for
+        for (int kb = 0; kb < C::kKB; kb++) CFX_SWAIT(A_KB + 4 * P.L + kb, 0);
+        __syncwarp();
+        if (elect_one()) mma_commit(sm.bar(H_FULL));
+        CFX_SWAIT(H_FULL, 0);
+        return;
+    }
+    const int slot0 = first_slot(P.L);
+#pragma unroll
+    for (int i = 0; i < C::kHeadItems; i++) CFX_SWAIT_SPIN(W_FULL + (slot0 + i) % kWSlots, wpar >> (slot0 + i) % kWSlots & 1u);
+    // (a block at a time: the first one is this CTA's own, which is there before the others)
+    CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L, 0);
+#pragma unroll
+    for (int kb = 0; kb < C::kKB; kb++) {
+        CFX_SWAIT_PROBED(cfx_p_a, A_KB + 4 * P.L + kb, 0);
+        if (kb + 1 < C::kKB) CFX_SPROBE(cfx_p_a, A_KB + 4 * P.L + kb + 1, 0);
+        tc_fence_after_sync();
+        __syncwarp();
+        const int slot = (slot0 + kb / 2) % kWSlots;
+        const uint64_t bd = wdesc + (uint64_t)((slot * kWSlot + (kb & 1) * 2 * C::kHeadHalf) >> 4), ad = adesc + (uint64_t)(C::one_block(P.L, kb) >> 4);
+        if (elect_one()) {
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) mma_f16_ws_ss(tmem + kColHead, ad + 2 * ks, bd + 2 * ks, idesc_64, (kb | ks) != 0 ? 1u : 0u);
             if (kb == C::kKB - 1) mma_commit(sm.bar(H_FULL));
         }
     }
@@ -783,7 +858,7 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
             mbar_arrive(sm.bar(QUAD));
             if (w < S) {
                 ok = mbar_wait<false>(sm.bar(QUAD), l & 1, sm.abort_flag(), kSite + QUAD);
-                if (ok) hand_on<S>(sm, C::one_block(l, (int)rank), kQuadBlock, A_KB + 4 * l + (int)rank, rank, (uint32_t)w);
+                if (ok) hand_on<S>(sm, C::one_block(l, (int)rank), kQuadBlock, A_KB + 4 * l + (l == P.L ? (int)rank : 0), rank, (uint32_t)w);
             }
         }
         return __all_sync(0xffffffffu, ok);
@@ -885,7 +960,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
             else if (i >= QUAD && i < QUAD + 8) arrivals = ONE ? kWorkerWarps : 4;
             else if (i >= A_KB) {
                 const int kb = (i - A_KB) % 4;
-                if (kb < C::kKB && kb % S == (int)rank) arrivals = quads;
+                if (ONE && (i - A_KB) / 4 < P.L) {   // one barrier for all blocks of a layer input: its own, and the bytes of the others
+                    if (kb == 0) { arrivals = 2; bytes = (C::kKB - 1) * kQuadBlock; }
+                } else if (kb < C::kKB && kb % S == (int)rank) arrivals = quads;
                 else if (kb < C::kKB) bytes = quads * (kABlock / 4);       // a block of another CTA, counted by its bytes
             }
             mbar_init(sm.bar(i), arrivals);
@@ -919,7 +996,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
             cluster_wait();
         } else if (warp == 1) {
             cluster_wait();
-            role_mma<T16, GAME, HID, S, ONE>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
+            if constexpr (ONE) role_mma_one<T16, GAME, HID, S>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
+            else role_mma<T16, GAME, HID, S>(sm, P, __shfl_sync(0xffffffffu, tmem, 0), rank);
         } else if (warp == 2) {
             // the tile's records, 32 rows a copy
             wait_for_previous_kernel();
