@@ -816,14 +816,17 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
     };
     if (kFull && wg < 3) {
         static_assert(C::kEncPerItem == 3 && kMapWarps == 3 * 4 && kMapItems * 3 == 12, "a warp a quarter of a chunk");
+        // (a step's bytes are on their way while the one before is converted; all four steps' first: 0.05 to 0.1 us slower)
         uint32_t bytes[kMapItems][4];
-#pragma unroll
-        for (int i = 0; i < kMapItems; i++)
+        auto load = [&](int i) {
 #pragma unroll
             for (int q = 0; q < 4; q++) bytes[i][q] = *reinterpret_cast<const uint32_t*>(rec + 64 * (3 * i + wg) + 16 * quadrant + 4 * q);
+        };
+        load(0);
 #pragma unroll
         for (int i = 0; i < kMapItems; i++) {
             uint32_t regs[8];
+            if (i + 1 < kMapItems) load(i + 1);
 #pragma unroll
             for (int q = 0; q < 4; q++) Op::bytes4(bytes[i][q], regs[2 * q], regs[2 * q + 1]);
             operand(3 * i + wg, 2 * quadrant, regs);
