@@ -915,11 +915,13 @@ __device__ __forceinline__ void role_worker_one(const Smem& sm, const Params& P,
                          __uint_as_float(zp[0]), __uint_as_float(zp[1]), st.x, st.y, x01.x, x01.y, st.x, st.y, h0, h1);
         mingru_cell_pair(__uint_as_float(zh[2]), __uint_as_float(zh[3]), __uint_as_float(zg[2]), __uint_as_float(zg[3]),
                          __uint_as_float(zp[2]), __uint_as_float(zp[3]), st.z, st.w, x23.x, x23.y, st.z, st.w, h2, h3);
-        *sp = st;
         x = make_uint2(Op::pack(h0, h1), Op::pack(h2, h3));
         *xp(l + 1) = x;
         if (!send(l + 1)) return;
-        if (lane == 0) mbar_arrive(sm.bar(ST_READY + slot));   // (send fenced the box as well)
+        *sp = st;   // (behind what the next layer waits for: 512 envs h256x4 12.66 -> 12.56 us, 1,024 13.50 -> 13.39)
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sm.bar(ST_READY + slot));
     }
 
     // ---- heads + sampler: all warps, each with the rows in its quadrant
