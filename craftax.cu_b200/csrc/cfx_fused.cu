@@ -1385,7 +1385,7 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
             if (S == 4 && tr == fused::kTile && (a.r_state == nullptr || (!classic && fused::record_by_rows(P))) && (rows + 63) / 64 <= p->max_split[1]) continue;
             for (int l = 0; l < p->L; l++) P.state_map[l] = p->quad_map[l];
             P.tile_rows = tr;
-            P.done_blocks = (uint32_t)(tiles * (tr / 32));
+            P.done_blocks = (uint32_t)(tiles * std::min(S, tr / 32));
             return fused::split_launch(p->precision, p->game, p->H, S, tiles, P, st);
         }
     int smem = 0;

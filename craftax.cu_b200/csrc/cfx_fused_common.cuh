@@ -100,7 +100,7 @@ struct Params {
     unsigned long long* step_ctr;        // device step counter (Philox offset); see bump_step
     uint32_t* status;
     uint32_t* done_ctr;                  // blocks that are done with the step counter (bump_step)
-    uint32_t done_blocks;                // how many there are (small-batch form: warps that need the counter)
+    uint32_t done_blocks;                // how many there are (small-batch form: those that sample)
     int bump_step;
     uint64_t seed, env_offset;
     int n, L, num_tiles;  // num_tiles: end of the tile range of this launch (exclusive)

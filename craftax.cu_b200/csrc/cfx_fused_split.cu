@@ -132,7 +132,7 @@ enum Bar {
     NUM_BARS = A_KB + (kMaxLayers + 1) * 4
 };
 template <int GAME, int HID, int S> constexpr int smem_bytes() {
-    return Cfg<GAME, HID, S>::kOffBars + NUM_BARS * 8 + 16 + 128 + 1024;   // misc, uniforms, alignment slack
+    return Cfg<GAME, HID, S>::kOffBars + NUM_BARS * 8 + 16 + 4 * kTile + 1024;   // misc, uniforms, alignment slack
 }
 static_assert(smem_bytes<CFX_GAME_FULL, 256, 2>() <= 232448 && smem_bytes<CFX_GAME_FULL, 128, 2>() <= 232448 && smem_bytes<CFX_GAME_FULL, 256, 4>() <= 232448 &&
                   smem_bytes<CFX_GAME_CLASSIC, 256, 4>() <= 232448, "shared memory");
@@ -145,7 +145,7 @@ struct Smem {
     uint32_t bars;   // shared address of the barriers
     __device__ __forceinline__ uint32_t bar(int i) const { return bars + 8u * (uint32_t)i; }
     __device__ __forceinline__ uint32_t* tmem_base() const { return reinterpret_cast<uint32_t*>(base + off_bars + NUM_BARS * 8); }
-    __device__ __forceinline__ float* uniforms() const { return reinterpret_cast<float*>(tmem_base() + 4); }   // ONE: of the tile's envs
+    __device__ __forceinline__ float* uniforms() const { return reinterpret_cast<float*>(tmem_base() + 4); }   // of the rows that this CTA samples
     __device__ __forceinline__ volatile uint32_t* abort_flag() const { return tmem_base() + 1; }
 };
 // one lane waits (CFX_SWAIT1), or a whole warp (the MMA warp by polling alone)
@@ -531,7 +531,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     const bool valid = env < P.n;   // of a quadrant all rows or none (n is a multiple of 32)
     const float* bias = reinterpret_cast<const float*>(sm.base + C::kOffBias);
     const bool samples = samples_rows<S>(quadrant, quads, rank);
-    const unsigned long long step0 = samples && wg == 0 && P.uniforms == nullptr ? *P.step_ctr : 0ull;
     const bool zero_state = valid && P.prev_terminals != nullptr && P.prev_terminals[env] != 0.0f;
     // (the flags are waited for here, under the records' way: with the ballot at its use, 8,192 envs took 21.8 us instead of 21.3)
     const uint32_t zero_rows = __ballot_sync(0xffffffffu, zero_state);
@@ -578,19 +577,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     hand_over(wg + (kChunks - 1 - wg) / 4 * 4);
     __syncwarp();
     if (lane < S) mbar_arrive_cluster(map_to_cta(sm.bar(REC_FREE), (uint32_t)lane));
-    // The last of the warps that need the step counter raises it, once all have read it (here, where the encoder's MMAs are
-    // waited for; at the kernel's end it was a microsecond of the step).  The draw itself comes under the first layer's MMAs: with both
-    // here, 2,600 cycles, the warp was late for the encoder's output, and the cluster with it (h256x2, 1,600 envs 14.6 -> 14.35 us, 2,112 15.0 -> 14.7;
-    // h128x2, 4,736 12.9 -> 12.7).
-    const bool draws = samples && wg == 0;
-    if (draws) {
-        // (the counter's load has been issued in front of this, which does not wait for it: the __syncwarp and the fence in done_with_step
-        // order the loads of all lanes before lane 0's count)
-        asm volatile("" ::"l"(step0));
-        __syncwarp();
-        if (lane == 0 && P.bump_step) done_with_step(P.step_ctr, P.done_ctr, P.done_blocks);
-    }
-
     // Hands this thread's 16 units of layer input l, slice j, on: into the own K block, and, once the quadrant's four
     // warps have done so, to the other CTAs, a warp of the quadrant for each.
     // (A barrier a slice: a warp may be one slice ahead of another, but not one layer.)
@@ -631,10 +617,6 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             x[j][q] = Op::pack(__uint_as_float(acc[2 * q]) + b[2 * q], __uint_as_float(acc[2 * q + 1]) + b[2 * q + 1]);
         if (!send(0, j, x[j])) return;
     }
-    float u = 0.0f;
-    if (draws && valid)
-        u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
-
     // ---- layers
     for (int l = 0; l < P.L; l++) {
 #pragma unroll
@@ -724,7 +706,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
 #pragma unroll
             for (int a = 0; a < kA; a++) pr[a] = p[a * kTile];
             float la = logits[0], total;
-            const int act = draw_action<kA>(pr, u, &total, [&](int a, bool beyond) { la = beyond ? logits[a + 1] : la; });
+            const int act = draw_action<kA>(pr, sm.uniforms()[row], &total, [&](int a, bool beyond) { la = beyond ? logits[a + 1] : la; });
             write_action(P, env, act, la - m - logf(total), value);
         }
     }
@@ -1016,13 +998,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
                 reinterpret_cast<float*>(sm.base + C::kOffBias)[i] =
                     P.params[a < 0 ? P.off_b_enc + C::slice((int)rank, i / kSliceUnits) * kSliceUnits + i % kSliceUnits : (a < kA ? P.off_b_a + a : P.off_b_v)];
             }
-            // ONE: the uniforms of the tile's envs and the step counter, which the worker that samples raised under the encoder's products
-            // until those ended before it was done (512 envs h256x2 9.82 -> 9.72 us, h128x2 8.33 -> 8.17)
-            const bool draws = ONE && rank == 0;
-            if (draws) {
-                const int env = row0 + lane;   // (n is a multiple of 32)
-                sm.uniforms()[lane] = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, *P.step_ctr);
-            }
+            // The uniforms of the rows that this CTA samples, and the step counter, which the last CTA that has read it raises.  (By the workers that sample,
+            // under the encoder's products, they were late in tiles of 32 rows, 512 envs h256x2 9.82 -> 9.72 us, h128x2 8.33 -> 8.17; in taller ones they cost registers: 8,192 envs
+            // h256x2 18.82 -> 18.74, with a bf16 record 21.46 -> 20.99, classic h256x3 26.4 -> 25.9, 4,736 h128x2 12.7 -> 12.2, 2,048 h256x2 14.56 -> 14.38.)
+            bool draws = false;
+            const unsigned long long step0 = P.uniforms == nullptr && has_heads<S, ONE>(quads, rank) ? *P.step_ctr : 0ull;
+            for (int q = 0; q < quads; q++)
+                if (ONE ? rank == 0 : samples_rows<S>(q, quads, rank)) {
+                    const int env = row0 + 32 * q + lane;   // (n is a multiple of 32)
+                    draws = true;
+                    if (env < P.n) sm.uniforms()[32 * q + lane] = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, step0);
+                }
+            asm volatile("" ::"l"(step0));
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(sm.bar(ACC_FULL));
