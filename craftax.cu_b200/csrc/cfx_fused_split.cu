@@ -53,6 +53,7 @@ constexpr int kSlicePiece = kSliceUnits * 128;       // a slice's rows of an enc
 constexpr int kMaxChunks = Gm<CFX_GAME_CLASSIC>::kEncChunks;
 constexpr int kASlots = 12;                          // operand chunks in tensor memory; a multiple of the warpgroups
 constexpr int kSSlots = 4, kSBox = kTile * 128, kQuadBox = 32 * 128;   // state ring: 128 rows x 32 units a slot, copied 32 rows at a time
+constexpr int kFirstChunks = 4;   // see role_worker
 constexpr uint32_t kColAexp = 0, kColAcc = 384, kColHead = 448;
 __host__ __device__ constexpr uint32_t col_gate(int j) { return 192u * (uint32_t)j; }   // over the operand chunks, done by then
 
@@ -79,6 +80,7 @@ template <int GAME, int HID, int S> struct Cfg {
     static constexpr int kKB = HID / 64;                        // K blocks of a layer's input
     static constexpr int kNS = HID / 64 / S;                    // gate slices of a CTA
     static constexpr int kUnits = 64 * kNS;                     // hidden units of a CTA
+    static constexpr int kFirst = GAME == CFX_GAME_FULL && kNS == 1 ? kFirstChunks : 0;   // chunks that come one by one, in tiles of more than 32 rows
     // slice j of a CTA, which is also the K block that it makes of a layer's input
     static __host__ __device__ constexpr int slice(int rank, int j) { return rank + S * j; }
     // Its rows of an encoder weight block, one piece a slice.  A ring slot has three pieces, and the pieces lie one behind the other
@@ -128,6 +130,8 @@ enum Bar {
     S_FULL = ACC_FULL + 1, ST_READY = S_FULL + kSSlots, MMA_DONE = ST_READY + kSSlots,
     QUAD = MMA_DONE + 1, G_FULL = QUAD + 8,   // QUAD: [slice][quadrant]
     H_FULL = G_FULL + 2, A_KB = H_FULL + 1,
+    // AEXP_FULL: four chunks each (ONE: of a ring slot); the first ones by themselves, see Cfg::kFirst
+    AEXP_FIRST = AEXP_FULL + kMaxChunks - kFirstChunks,
     // A_KB: [layer input][K block]; ONE: [layer input][0] for all of its blocks, but not for those of the heads' input
     NUM_BARS = A_KB + (kMaxLayers + 1) * 4
 };
@@ -260,8 +264,9 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
     static_assert(kGateItems % kWSlots == 0 || kWSlots % kGateItems == 0, "a layer's first ring slot");
     const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
     // ---- encoder
+    auto aexp = [](int kc) { return kc < C::kFirst ? AEXP_FIRST + kc : AEXP_FULL + kc / 4; };
     CFX_SPROBE(cfx_p_b, W_FULL, 0);
-    CFX_SPROBE(cfx_p_a, AEXP_FULL, 0);
+    CFX_SPROBE(cfx_p_a, aexp(0), 0);
 #pragma unroll
     for (int kc = 0; kc < kChunks; kc++) {
         // block of 64 K columns, first of its 16-byte K pieces, K steps (see expand_full), last chunk of its block
@@ -279,9 +284,10 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
                 CFX_SPROBE(cfx_p_b, W_FULL + (item + 1) % kWSlots, ((item + 1) / kWSlots) & 1);
             }
         // (four chunks, one of each warpgroup, are there at the same time)
-        if (kc % 4 == 0) {
-            CFX_SWAIT_PROBED(cfx_p_a, AEXP_FULL + kc / 4, 0);
-            if (kc + 4 < kChunks) CFX_SPROBE(cfx_p_a, AEXP_FULL + kc / 4 + 1, 0);
+        if (kc % 4 == 0 || kc < C::kFirst) {
+            CFX_SWAIT_PROBED(cfx_p_a, aexp(kc), 0);
+            const int next = kc + 1 < C::kFirst ? kc + 1 : kc / 4 * 4 + 4;
+            if (next < kChunks) CFX_SPROBE(cfx_p_a, aexp(next), 0);
         }
         tc_fence_after_sync();
         __syncwarp();
@@ -552,7 +558,35 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         __syncwarp();
         if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + kc / 4));
     };
-    for (int kc = wg; kc < kChunks; kc += 4) {
+    // Full game, one slice a CTA: the first four chunks a quarter of each a warp, so that the encoder starts with the first one while the others are converted. (A chunk
+    // a warp, all four are there 1,100 cycles after the records.  us: 1,600 envs h256x2 with a bf16 record 15.40 -> 15.22, x4 21.86 -> 21.54, 2,048 h256x2 14.37 -> 14.27, 4,224 with an fp32
+    // record 18.50 -> 18.03, 8,192 h128x2 13.39 -> 13.21.  With two slices a CTA the encoder's weights come too slowly for that to count, 8,192 h256x2 18.75 -> 18.68, and
+    // with a bf16 record the cells keep more in local memory, 6,400 h256x4 30.9 -> 31.2.)
+    constexpr int kFirst = C::kFirst;
+    if constexpr (kFirst > 0) {
+        uint32_t bytes[4], regs[8];
+        auto load = [&](int kc) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) bytes[q] = valid ? *reinterpret_cast<const uint32_t*>(rec + 64 * kc + 16 * wg + 4 * q) : 0u;
+        };
+        auto there = [&](int kc) {
+            tmem_wait_st();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sm.bar(AEXP_FIRST + kc));
+        };
+        load(0);
+#pragma unroll
+        for (int kc = 0; kc < kFirst; kc++) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) Op::bytes4(bytes[q], regs[2 * q], regs[2 * q + 1]);
+            if (kc + 1 < kFirst) load(kc + 1);
+            if (kc > 0) there(kc - 1);
+            tmem_st8(lane_base + kColAexp + kc * 32 + 8 * wg, regs);
+        }
+        there(kFirst - 1);
+    }
+    for (int kc = kFirst + wg; kc < kChunks; kc += 4) {
         const int as = kc % kASlots;
         uint32_t regs[32];
         if (valid) {
@@ -940,7 +974,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         if (i < NUM_BARS) {
             uint32_t arrivals = 1, bytes = 0;
             if (i == REC_FREE) arrivals = ONE ? S * kWorkerWarps : S * 4 * quads;
-            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::item_warps(i - AEXP_FULL) : max(1, min(4, Gm<GAME>::kEncChunks - 4 * (i - AEXP_FULL))) * quads;
+            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::item_warps(i - AEXP_FULL) : i >= AEXP_FIRST && C::kFirst > 0 ? 4 * quads : max(1, min(4, Gm<GAME>::kEncChunks - 4 * (i - AEXP_FULL))) * quads;
             else if (i == ACC_FULL) arrivals = 2;                          // the MMAs, and the biases are in place
             else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = ONE ? 8 : 2 * quads;
             else if (i == MMA_DONE) arrivals = S;
