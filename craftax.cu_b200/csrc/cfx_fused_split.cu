@@ -31,9 +31,9 @@
 // The records lie where the layer input and the state boxes are later: REC_FREE is complete when every CTA has expanded its
 // records.  With one input buffer, it is overwritten when every CTA has done its multiplications of the layer (MMA_DONE,
 // which a CTA's commit signals in all of them).
-// Measured (us a step in a stream, fp16; the persistent kernel, one CTA pair per two tiles -> here): h256x2, 32 envs 20.6 -> 9.5,
-// 256 21.0 -> 10.0, 1,024 21.5 -> 10.4, 2,048 21.7 -> 14.6, 4,000 22.3 -> 16.9, 8,192 22.7 -> 18.9; classic h256x3, 1,024 envs 28.9 -> 14.3, 4,000
-// 29.7 -> 24.3, 8,192 30.2 -> 26.5.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
+// Measured (us a step in a stream, fp16; the persistent kernel, one CTA pair per two tiles -> here): h256x2, 32 envs 20.6 -> 8.7,
+// 256 21.0 -> 9.2, 1,024 21.5 -> 9.8, 2,048 21.7 -> 14.3, 4,000 22.3 -> 16.7, 8,192 22.7 -> 18.7; classic h256x3, 1,024 envs 28.9 -> 13.9, 4,000
+// 29.7 -> 23.8, 8,192 30.2 -> 26.0.  Bound by the chain of dependent steps and the 1.3 us between one kernel's end and the next one's start.
 // In clusters of two an encoder's weights are 14 pieces of 16 KB a CTA: with one lane issuing them, 500 cycles a slot, and one a
 // slot of 24 KB, the multiplications waited for them, 10,200 cycles to the encoder's end at 8,192 envs; now 8,700, with the MMA warp waiting for
 // the records' conversion.  8,192 envs h256x2: 20.00 us before, 19.94 with the slices in turn, 19.46 with the weight warp converged, 19.08 with the
