@@ -1369,20 +1369,23 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     // Small batches: a tile is shared by four (two) CTAs as long as every tile then has its SMs at once, and is as
     // short as that allows (cfx_fused_split.cu).  CTAs of two slices take tiles of 64 and
     // 128 rows; at 32 four CTAs a tile have their SMs.  With the 33 clusters of four and 74 of two that this part holds, four
-    // CTAs go to 1,056 and 2,112 envs, with 32 and 64 rows, and two to 4,736 with 64 rows and 9,472 with 128; where the state is recorded by write_r_state, four take
-    // 128 rows up to 4,224.  At each of these limits the next form is slower, and the kernel below slower than all of them.  us a step, h256x2, clusters
+    // CTAs go to 1,056 and 2,112 envs, with 32 and 64 rows, and two to 4,736 with 64 rows and 9,472 with 128; where the state is recorded in other ways than two_before_four
+    // names, four take 128 rows up to 4,224.  At each of these limits the next form is slower, and the kernel below slower than all of them.  us a step, h256x2, clusters
     // of four with 32, 64, 128 rows, of two with 64 and 128, the kernel below: 1,056 envs 10.5, 14.6, 16.8, 16.2, 17.9, 21.5; 2,112 -, 14.8, 16.4, 16.5,
     // 18.2, 21.8; 2,144 -, -, 17.0, 16.5, 18.2, 21.8; 4,224 -, -, 17.5, 16.9, 18.4, 22.0; 4,736 -, -, -, 17.1, 18.3, 22.3; 9,472 -, -, -, -, 19.0, 22.5.
-    // (The same with a bf16 record that the cells write, see record_by_rows: 4,224 envs h256x2 18.8 and 18.3, h256x1 14.7 and 14.2, h256x3 23.3 and 22.5.)
-    // Four CTAs with 128 rows and two with 64, 3,200 envs: h256x1 13.25 and 13.16, h256x3 21.4 and 20.9, classic h256x3 25.0 and 24.7; with a record in
-    // bf16 h256x2 18.5 and 18.9, in fp32 h256x3 22.3 and 23.5.  h128x2, of two with 32, 64, 128 rows, the kernel below:
+    // Four CTAs with 128 rows and two with 64, 4,224 envs: h256x1 13.4 and 12.9, x2 17.4 and 16.8, x3 21.5 and 20.7; with a bf16 record that the cells write (record_by_rows)
+    // x1 14.7 and 13.8, x2 18.9 and 17.9, x3 23.2 and 22.1; classic h256x3, 3,200 envs, 25.0 and 24.7.  h128x2, of two with 32, 64, 128 rows, the kernel below:
     // 2,368 envs 8.9, 12.5, 13.4, 15.7; 4,736 -, 12.9, 13.5, 15.7; 9,472 -, -, 14.0, 16.0.
+    // The classic game with a record, four CTAs with 128 rows and two with 64, us: in bf16 h256x1 2,144 envs 16.93 and 16.16, 4,224 17.24 and 16.38, x2 21.5 and 20.5, 21.7 and
+    // 20.8, x3 25.8 and 24.9, 26.0 and 25.4; in fp32 x1 17.2 and 16.3, 17.4 and 16.5, x2 21.7 and 21.0, 22.0 and 21.4, but x3 26.3 and 25.8, at 3,200 26.3 and 26.6.  The
+    // full game in fp32: x1 13.0 and 13.1, 14.5 and 14.1, x2 17.6 and 17.9, x3 22.0 and 22.7, x4 26.4 and 27.5.
+    const bool two_before_four = a.r_state == nullptr || (classic ? P.r_state_bf16 || p->L <= 2 : fused::record_by_rows(P));
     const int rows = std::min(p->n, P.num_tiles * fused::kTile) - P.tile_begin * fused::kTile;
     for (int i = 0; i < 2; i++)
         for (int S = i == 0 ? 4 : 2, tr = p->H == 64 * S ? 32 : 64; tr <= fused::kTile; tr *= 2) {
             const int tiles = (rows + tr - 1) / tr;
             if (tiles > p->max_split[i]) continue;
-            if (S == 4 && tr == fused::kTile && (a.r_state == nullptr || (!classic && fused::record_by_rows(P))) && (rows + 63) / 64 <= p->max_split[1]) continue;
+            if (S == 4 && tr == fused::kTile && two_before_four && (rows + 63) / 64 <= p->max_split[1]) continue;
             for (int l = 0; l < p->L; l++) P.state_map[l] = p->quad_map[l];
             P.tile_rows = tr;
             P.done_blocks = (uint32_t)(tiles * std::min(S, tr / 32));

@@ -62,3 +62,11 @@ def test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, H, L
     for g in got:
         for k in want:
             assert np.array_equal(g[k], want[k]), k
+
+
+@pytest.mark.parametrize("n,L,prec,r_state", [
+    (2112, 3, "f16", "bf16"),                                                         # four CTAs, 64 rows
+    (2144, 3, "bf16", "bf16"), (4224, 1, "f16", "bf16"), (3232, 2, "f16", "fp32"),    # two CTAs, 64 rows
+    (3200, 3, "f16", "fp32")])                                                        # four CTAs, 128 rows
+def test_classic_game_with_a_record(cfx, gpu, monkeypatch, n, L, prec, r_state):
+    test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, 256, L, prec, "classic", r_state)
