@@ -328,7 +328,7 @@ __device__ __forceinline__ void role_weight_loads(const Smem& sm, const Params& 
 // next while the warp served the other lanes.)
 //   load thread:  per tile, the records, then the state boxes, each when what was in its slots before is done with;
 //   store thread: the state box stores; it reports a box that has been read out of its slot (S_FREE).
-// The records of a CTA's first tile are loaded ahead of this by a lane a copy (see the kernel).
+// Full game: the records of a CTA's first tile are loaded ahead of this by a lane a copy (see the kernel; the classic game's are one copy, and so 0.2 % slower).
 // Copy i of a tile's records.  Rows [32 q, 32 q + 32) are a quadrant's (n is a multiple of 32): all of them are there or none, and then what lies
 // in the slot is converted and multiplied like records, and the results of those rows are dropped.
 template <bool PAIR, int GAME, int HID>
@@ -357,12 +357,14 @@ __device__ __forceinline__ void role_loads(const Smem& sm, const Params& P) {
     };
     CFX_MARK_INIT(4);
     for (int tile = P.tile_begin + blockIdx.x; tile < P.num_tiles_loop; tile += gridDim.x, it++) {
-        for (int u = 0; u < C::kRecSlots && it > 0; u++) {   // (those of the first tile: see the kernel)
-            if (u >= boxes) {   // no state boxes here
-                if ((u & 1) == 0) CFX_WAIT_FAST(REC_FREE + u / 2, (it - 1) & 1, W_REC_FREE);
-            } else {
-                CFX_WAIT_FAST(S_FREE + u, (fpar >> u) & 1u, W_S_FREE);
-                fpar ^= 1u << u;
+        for (int u = 0; u < C::kRecSlots && (it > 0 || GAME != CFX_GAME_FULL); u++) {   // (full game, first tile: see the kernel)
+            if (it > 0) {
+                if (u >= boxes) {   // no state boxes here
+                    if ((u & 1) == 0) CFX_WAIT_FAST(REC_FREE + u / 2, (it - 1) & 1, W_REC_FREE);
+                } else {
+                    CFX_WAIT_FAST(S_FREE + u, (fpar >> u) & 1u, W_S_FREE);
+                    fpar ^= 1u << u;
+                }
             }
             if (GAME == CFX_GAME_FULL) load_records<PAIR, GAME, HID>(sm, P, tile, u);
             else if (u == C::kRecSlots - 1) load_records<PAIR, GAME, HID>(sm, P, tile, 0);
@@ -679,6 +681,8 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
     const float* bias = sm.bias();
     uint32_t tcnt = 0, gcnt = 0, it = 0;
     uint32_t spar = 0;   // phase parity of every state slot, one bit per slot
+    // (classic game, whose kernel has the registers; read for every tile: 1,048,576 envs h256x3 2,207 and 2,209)
+    const unsigned long long step0 = GAME == CFX_GAME_CLASSIC && P.uniforms == nullptr ? *P.step_ctr : 0ull;
     CFX_MARK_INIT(1);
     for (int tile = P.tile_begin + blockIdx.x; tile < P.num_tiles_loop; tile += gridDim.x, it++, tcnt++) {
         CFX_MARK(0);
@@ -731,9 +735,9 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 CFX_MARK(4);
             }
         } else if (valid) {   // the uniform of this env is drawn while the others convert
-            // (The step counter is constant for the launch: it is raised when every block is done.  Read once and kept in registers through the tiles, us: h128x2 24,064 envs
+            // (The step counter is constant for the launch: it is raised when every block is done.  Full game: read once and kept in registers through the tiles, us: h128x2 24,064 envs
             // 27.9 and so 27.1, 57,600 53.5 and 52.7, with an fp32 record 12,832 19.3 and 18.7; h256x2 20,000 41.5 and 41.3.)
-            u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, *P.step_ctr);
+            u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, GAME == CFX_GAME_CLASSIC ? step0 : *P.step_ctr);
         }
 
         // ---- encoder epilogue: accumulator + bias -> layer-0 input A0.  Like in the gate
@@ -998,7 +1002,7 @@ k_policy_fused(const __grid_constant__ Params P) {
             // 18,944 28.4 -> 27.9, h128x2 16,160 17.0 -> 16.6, 20,000 28.2 -> 27.5.
             const int first = P.tile_begin + (int)blockIdx.x;
             wait_for_previous_kernel();
-            if (warp == 2 && lane < C::kRecCopies && first < P.num_tiles_loop) load_records<PAIR, GAME, HID>(sm, P, first, lane);
+            if (GAME == CFX_GAME_FULL && warp == 2 && lane < C::kRecCopies && first < P.num_tiles_loop) load_records<PAIR, GAME, HID>(sm, P, first, lane);
             __syncwarp();
             if (lane == 0) {
                 if (warp == 2) role_loads<PAIR, GAME, HID, REC16>(sm, P);
