@@ -84,7 +84,12 @@ template <int TM> struct Frag {
         }
     }
 };
-// Four floats by a load that is issued where it stands
+// Loads that are issued where they stand, and see what a kernel in front has written
+__device__ __forceinline__ uint32_t ld_now(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void ld_now4(const float* p, float* v) {
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
 }
@@ -153,7 +158,7 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("
 
 template <int TM, int G, int WU, int UL>
 __global__ void __launch_bounds__(32 * kEncWarps, 2)
-k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc, const uint32_t* __restrict__ odd_weights,
+k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float* __restrict__ b_enc, const uint32_t* odd_weights,
                float* __restrict__ h_out, int n, int H, int w_aligned, int early) {
     using E = Enc<TM, G, WU, UL>;
     static_assert(UL == 4 || (UL == 1 && TM == 1 && G == 1), "tiles");
@@ -183,7 +188,7 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + i * kMapPitch + 4 * (32 * j + lane)), "l"(r + 4 * (32 * j + lane)) : "memory");
         }
         copy_commit();
-        const bool all = __any_sync(0xffffffffu, (odd_weights[lane] | odd_weights[lane + 32]) != 0);
+        const bool all = __any_sync(0xffffffffu, (ld_now(odd_weights + lane) | ld_now(odd_weights + lane + 32)) != 0);
         copy_wait<0>();
         uint32_t any[kMapRounds] = {};   // (a lane reads what it has copied)
 #pragma unroll 4

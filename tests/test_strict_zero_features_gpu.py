@@ -1,5 +1,7 @@
 """fp32 encoder: features that are zero in all envs of a block are left out, which changes no bit of a result and nothing where a weight is
 not finite."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -67,3 +69,29 @@ def test_weights_that_are_not_finite_reach_every_env(cfx, gpu, oracle, n, H, val
         else:
             assert np.array_equal(lav, want) and np.isfinite(lav).all()
     pol.close()
+
+
+@pytest.mark.parametrize("n", [32, 416, 1024])
+def test_each_static_forward_looks_at_its_own_weights(cfx, gpu, oracle, n):
+    """Forwards of the allocation-free entry point one behind the other on a stream, with weights that are finite and that are not in turn: what
+    the kernel in front of the encoder finds in them is what the encoder goes by."""
+    H = 256
+    params = oracle.init_weights(H, L, A, seed=5, scheme="uniform")
+    rec = oracle.synthetic_records(n, seed=4)
+    rec[:, 700] = 0
+    bad = params.copy()
+    bad[700 * H + H - 1] = np.inf
+    weights = [cfx.DeviceBuffer.from_host(p) for p in (params, bad)]
+    d_rec, d_state = cfx.DeviceBuffer.from_host(rec), cfx.DeviceBuffer((L, n, H), np.float32)
+    d_u, d_act = cfx.DeviceBuffer.from_host(np.full(n, 0.5, np.float32)), cfx.DeviceBuffer((n,), np.int32)
+    ended = cfx.DeviceBuffer.from_host(np.ones(n, np.float32))   # every forward starts from a state of zeros
+    outs = [cfx.DeviceBuffer((n, A + 1), np.float32) for _ in range(40)]
+    for i, out in enumerate(outs):
+        io = cfx.ForwardIO(d_rec.ptr, ended.ptr, d_u.ptr, None, d_act.ptr, None, None, out.ptr, None, 0, 0, 0, 0)
+        cfx.check(cfx.lib().cfx_strict_forward_static(0, weights[i % 2].ptr, H, L, A, n, d_state.ptr, C.byref(io), None, None))
+    cfx.check(cfx.lib().cfx_stream_sync(0, None))
+    want = outs[0].download()
+    assert np.isfinite(want).all()
+    for i, out in enumerate(outs):
+        lav = out.download()
+        assert np.isnan(lav).all() if i % 2 else np.array_equal(lav, want), i
