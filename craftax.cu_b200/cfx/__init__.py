@@ -258,11 +258,14 @@ class Timer:
 
 def host_address(a):
     """Where an array's data lies.  By way of the buffer protocol, which needs a third of the time of `a.__array_interface__`: a
-    step from host buffers asks for seven (32 envs 37.0 -> 33.7 us a call, 1,024 58.9 -> 55.5).  Arrays that are read-only, empty or not contiguous have no such buffer."""
-    try:
-        return C.addressof(C.c_char.from_buffer(a))
-    except (TypeError, ValueError, BufferError):
-        return a.__array_interface__["data"][0]
+    step from host buffers asks for seven (32 envs 37.0 -> 33.7 us a call, 1,024 58.9 -> 55.5).  Arrays that are read-only, empty or not
+    contiguous have no such buffer; what has a buffer and is no array, such as a bytearray, has no type and shape and is refused."""
+    if isinstance(a, np.ndarray) and a.flags.carray:
+        try:
+            return C.addressof(C.c_char.from_buffer(a))
+        except (TypeError, ValueError, BufferError):
+            pass
+    return a.__array_interface__["data"][0]
 
 
 class Policy:
