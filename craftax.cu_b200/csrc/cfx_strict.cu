@@ -1182,11 +1182,12 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     const long long q = (long long)n * H / 1024;
     const int tm = strict_tile(n, H);
     const EncoderTile te = strict_encoder_tile(n, H);
-    // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own (512 envs, 64 blocks a layer: 88 us
-    // with it, 72 without; 32 envs, hidden 256, depth 2, 194 blocks: 34.4 and 31.6)
+    // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own (64 envs, hidden 64, depths 1 and 2:
+    // 17.5 us with it, 19.2 without; 20.1 and 21.8; 32 envs, hidden 256, depth 2, 194 blocks: 34.4 and 31.6), but not with four envs a lane in the encoder,
+    // whose blocks then share SMs in some runs (depth 1, 416 envs, hidden 256: 43.0 to 51.4 and 42.5; 512 envs, hidden 192: 39.2 to 46.2 and 39.2)
     auto count = [&](int tile) { return tile == 0 ? 8 * q : tile == 1 ? 2 * q : q / 2; };
     const long long blocks = count(te.tm) + L * count(tm) + n / 16;
-    const int early = (a.game == CFX_GAME_FULL && blocks <= kSMs ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
+    const int early = (a.game == CFX_GAME_FULL && te.tm <= 1 && blocks <= kSMs ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);
     if (a.game == CFX_GAME_CLASSIC) {
         rc = launch_chained(k_classic_encoder_fp32, dim3(n), H, 0, st, a.records, a.params + o.w_enc, a.params + o.b_enc,
                             a.scratch_h[0], n, H);
