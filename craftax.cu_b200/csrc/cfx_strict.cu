@@ -134,13 +134,14 @@ __host__ __device__ __forceinline__ size_t act_at(size_t e, int k, int H) { retu
 // A feature that is zero in all envs of a block is left out: its products change no sum (but the sign of one that is still -0).  Most bytes of a
 // record are zero, five of a cell's eight unless there is a mob: of the 843 features 410 are left in blocks of 56 envs of a game, 546 with a mob of each
 // class on every hundredth cell.  Zero times a weight that is infinite or not a number is not zero: with such weights (odd_weights, looked for when the
-// weights are laid out) nothing is left out.  The block copies its records' maps to shared memory, ORs them over the envs, and makes a list of the features
-// that are left, from which the stages are filled.  (Features taken 32 at a time as they come, the left ones packed by masks: 117.5 us a forward at 4,096
-// envs, hidden 256, depth 2, and 10 us slower than every feature at 32: what a warp does for a feature is a chain of 150 cycles.  So all that the list and the map
-// give for a stage is loaded before it is used: 114.)
-// Bound by the FMA pipe, the operands' reads of shared memory beside it, and 4,000 cycles until the first stage is there.  us a forward with every feature and now,
-// hidden 256, depth 2: 4,096 envs 123.4 and 113.7, 2,048 84.3 and 75.4, 65,536 1,529 and 1,386, 128 43.9 and 40.0, 32 31.7 and 31.7; 8,192 envs, hidden 512,
-// depth 3 828 and 788; 4,096, hidden 128 65.3 and 56.6.  Where no feature is zero it is slower: 4,096 envs 126.5, 32 envs 36.6.
+// weights are laid out) nothing is left out.  The block copies its records' maps to shared memory, ORs them over the envs on their way, and makes a list of
+// the features that are left, from which the stages are filled.  What the list and the map give for a stage is loaded before it is used: row by row the latencies
+// of shared memory add up.  Narrow tiles fill several rows an instruction; where nothing is left out a word of the map gives four features.  Stages of 32 rows:
+// with 16 the barriers cost 2 to 6 %.
+// Bound by the FMA pipe, the operands' reads of shared memory beside it, and some 3,000 cycles until the first stage is there.  us a forward with every feature,
+// without a list; now; and now with records that have no zeros, which no game writes.  Hidden 256, depth 2: 32 envs 32.7, 29.7, 33.6, 128 43.6, 37.6, 43.1, 1,024
+// 58.8, 55.5, 60.0, 2,048 84.4, 73.4, 83.8, 4,096 123.5, 111.7, 122.1; depth 1: 65,536 1,075, 911, 1,059; 4,096, hidden 128 53.3, 42.5, 52.8; 8,192, hidden
+// 512, depth 3 828, 780, 821.
 constexpr int kEncWarps = 8, kEncFill = 4;   // warps of a block, those of them that fill the stages
 constexpr int kMapRounds = (kMap / 4 + 31) / 32, kMapPitch = kMap + 4;   // rounds of a warp's lanes with a word of a record each; bytes from one env's map to the next's
 constexpr int kMapGroups = (kMap + 31) / 32, kGroups = kMapGroups + (kTail + 31) / 32;   // features by 32
@@ -148,7 +149,7 @@ static_assert(kGroups < 32 && 4 * kMapRounds < 32 && kMap % 4 == 0 && kMapPitch 
 template <int TM, int G, int WU, int UL> struct Enc {   // WU of the four warps side by side along the units, UL units of a group a lane
     static constexpr int WM = 4 / WU, BM = UL * TM * WM, BU = 32 * G * WU;   // envs, units
     static constexpr int XS = BM + (BM % 8 == 0 ? 4 : 0);               // row stride of x
-    static constexpr int K = G == 1 ? 32 : 16, S = TM == 1 ? 6 : 4, R = S * K;   // rows of a stage, stages
+    static constexpr int K = 32, S = TM == 1 ? 6 : G == 1 ? 4 : WU == 2 && TM <= 6 ? 3 : 2, R = S * K;   // rows of a stage, stages
     static constexpr int kOffMap = R * (XS + BU) * 4, kOffList = kOffMap + BM * kMapPitch;
     static constexpr int kSmem = kOffList + (kObs + K) * 2;
     static_assert(XS % 4 == 0 && kOffList % 8 == 0, "alignment");
@@ -162,7 +163,7 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
                float* __restrict__ h_out, int n, int H, int w_aligned, int early) {
     using E = Enc<TM, G, WU, UL>;
     static_assert(UL == 4 || (UL == 1 && TM == 1 && G == 1), "tiles");
-    constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = E::K, S = E::S, R = E::R, D = S - 2;
+    constexpr int BM = E::BM, BU = E::BU, XS = E::XS, K = E::K, S = E::S, R = E::R, D = G == 1 ? 2 : S == 3 ? 1 : 0;   // D: stages filled behind one before it is handed over
     constexpr int FULL = 1, EMPTY = FULL + S;   // barrier ids
     static_assert(EMPTY + S <= 16, "barriers");
     extern __shared__ __align__(16) float sm[];   // x [R][XS], w [R][BU], the records' map bytes [BM][kMapPitch], the list of features
@@ -178,24 +179,29 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
     // The map bytes of the block's envs (where there are none, the last one's again, which changes nothing), and which of them are not
     // zero in all envs: a bit a feature, 32 to a group
     {
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(map);
-#pragma unroll 2
-        for (int i = warp; i < BM; i += kEncWarps) {
-            const uint8_t* r = rec + (size_t)min(e0 + i, n - 1) * kRec;
+        constexpr int ROWS = (BM + kEncWarps - 1) / kEncWarps, AT_ONCE = ROWS <= 9 ? ROWS : (ROWS + 1) / 2;   // a warp's envs; of them loaded before the first is stored
+        uint32_t any[kMapRounds] = {};
+#pragma unroll 1
+        for (int i0 = warp; i0 < BM; i0 += AT_ONCE * kEncWarps) {
+            uint32_t v[AT_ONCE][kMapRounds];
 #pragma unroll
-            for (int j = 0; j < kMapRounds; j++)
-                if (32 * j + lane < kMap / 4)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + i * kMapPitch + 4 * (32 * j + lane)), "l"(r + 4 * (32 * j + lane)) : "memory");
+            for (int i = 0; i < AT_ONCE; i++) {
+                const uint32_t* r = reinterpret_cast<const uint32_t*>(rec + (size_t)min(e0 + i0 + i * kEncWarps, n - 1) * kRec) + lane;
+#pragma unroll
+                for (int j = 0; j < kMapRounds; j++) v[i][j] = 32 * j + lane < kMap / 4 ? ld_now(r + 32 * j) : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < AT_ONCE; i++) {
+                if (i0 + i * kEncWarps >= BM) break;
+                uint32_t* m = reinterpret_cast<uint32_t*>(map + (i0 + i * kEncWarps) * kMapPitch) + lane;
+#pragma unroll
+                for (int j = 0; j < kMapRounds; j++) {
+                    any[j] |= v[i][j];
+                    if (32 * j + lane < kMap / 4) m[32 * j] = v[i][j];
+                }
+            }
         }
-        copy_commit();
         const bool all = __any_sync(0xffffffffu, (ld_now(odd_weights + lane) | ld_now(odd_weights + lane + 32)) != 0);
-        copy_wait<0>();
-        uint32_t any[kMapRounds] = {};   // (a lane reads what it has copied)
-#pragma unroll 4
-        for (int i = warp; i < BM; i += kEncWarps)
-#pragma unroll
-            for (int j = 0; j < kMapRounds; j++)
-                if (32 * j + lane < kMap / 4) any[j] |= *reinterpret_cast<const uint32_t*>(map + i * kMapPitch + 4 * (32 * j + lane));
 #pragma unroll
         for (int j = 0; j < kMapRounds; j++) {
             // a byte's bit 0 to bit 28 + its number, then to its place in the group
@@ -226,7 +232,9 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
         }
         total = __shfl_sync(0xffffffffu, pos, 31);
         pos -= __popc(rows);
-        for (int c = warp; c < kGroups; c += kEncWarps) {
+#pragma unroll
+        for (int i = 0; i < (kGroups + kEncWarps - 1) / kEncWarps; i++) {   // (groups from kGroups on have no bits)
+            const int c = warp + i * kEncWarps;
             const uint32_t r = __shfl_sync(0xffffffffu, rows, c);
             const int p = __shfl_sync(0xffffffffu, pos, c);
             if (r >> lane & 1u) list[p + __popc(r & ((1u << lane) - 1u))] = (uint16_t)(c < kMapGroups ? 32 * c + lane : kMap + 32 * (c - kMapGroups) + lane);
@@ -236,56 +244,76 @@ k_encoder_fp32(const uint8_t* rec, const float* __restrict__ W_enc, const float*
     __syncthreads();
     const int stages = (total + K - 1) / K;
     if (warp >= kEncWarps - kEncFill) {
-        // a warp has KW rows of every stage
-        constexpr int KW = K / kEncFill, ENVS = (BM + 31) / 32;
-        static_assert(KW % 4 == 0 && BU <= 128, "a row of weights an instruction");
-        const int k0 = (warp - (kEncWarps - kEncFill)) * KW;
+        // a warp has KW rows of every stage: their weights WR rows an instruction, a lane 16 bytes, their features XR rows an instruction, a lane an env
+        constexpr int KW = K / kEncFill, WL = BU / 4, WR = 32 / WL, XL = BM < 32 ? BM : 32, XR = 32 / XL, ENVS = (BM + 31) / 32;
+        static_assert(KW % 4 == 0 && BU <= 128 && 32 % WL == 0 && 32 % XL == 0 && KW % WR == 0 && KW % XR == 0, "whole rows");
+        const int k0 = (warp - (kEncWarps - kEncFill)) * KW, xl = lane % XL;
+        const bool whole = total == kObs;   // the list is all features
+        const float* const wsrc = W_enc + u0 + 4 * (lane % WL);
         for (int i = 0; i < stages + D; i++) {
             if (i < stages) {
                 const int s = i % S;
                 if (i >= S) bar_sync(EMPTY + s, 32 * kEncWarps);
-                float* const x = xring + (s * K + k0) * XS + lane;
+                const uint16_t* const rows = list + i * K + k0;
+                float* const x = xring + (s * K + k0 + lane / XL) * XS + xl;
                 float* const w = wring + (s * K + k0) * BU + 4 * lane;
-                int f[KW];   // (everything is loaded before it is used: row by row the latencies of shared memory add up, 150 cycles a row)
+                int f[KW / WR], g[KW / XR];   // the features whose weights and whose values this lane brings
+                if constexpr (XR == 1) {
 #pragma unroll
-                for (int k = 0; k < KW; k += 4) {
-                    const uint2 v = *reinterpret_cast<const uint2*>(list + i * K + k0 + k);
-                    f[k] = v.x & 0xFFFFu; f[k + 1] = v.x >> 16; f[k + 2] = v.y & 0xFFFFu; f[k + 3] = v.y >> 16;
+                    for (int k = 0; k < KW; k += 4) {
+                        const uint2 v = *reinterpret_cast<const uint2*>(rows + k);
+                        g[k] = v.x & 0xFFFFu; g[k + 1] = v.x >> 16; g[k + 2] = v.y & 0xFFFFu; g[k + 3] = v.y >> 16;
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < KW / XR; k++) g[k] = rows[k * XR + lane / XL];
                 }
-                const float* const wsrc = W_enc + u0 + 4 * lane;
-                if (BU == 128 || lane < BU / 4) {
-                    if (w_aligned)
 #pragma unroll
-                        for (int k = 0; k < KW; k++) copy16(w + k * BU, wsrc + (size_t)f[k] * H, true, true);
-                    else
+                for (int k = 0; k < KW / WR; k++) f[k] = WR == XR ? g[k] : rows[k * WR + lane / WL];
+                if (w_aligned)
 #pragma unroll
-                        for (int k = 0; k < KW; k++) copy16(w + k * BU, wsrc + (size_t)f[k] * H, true, false);
-                }
-                if ((i + 1) * K <= total - kTail) {
-                    uint32_t v[KW][ENVS];
+                    for (int k = 0; k < KW / WR; k++) copy16(w + k * WR * BU, wsrc + (size_t)f[k] * H, true, true);
+                else
+#pragma unroll
+                    for (int k = 0; k < KW / WR; k++) copy16(w + k * WR * BU, wsrc + (size_t)f[k] * H, true, false);
+                const bool maps = (i + 1) * K <= total - kTail;
+                if (XR == 1 && whole && maps) {   // four features a word
+                    uint32_t v[KW / 4][ENVS];
 #pragma unroll
                     for (int q = 0; q < ENVS; q++) {
-                        const uint8_t* m = map + (BM % 32 != 0 ? min(32 * q + lane, BM - 1) : 32 * q + lane) * kMapPitch;
+                        const uint8_t* m = map + (BM % 32 != 0 ? min(32 * q + lane, BM - 1) : 32 * q + lane) * kMapPitch + i * K + k0;
 #pragma unroll
-                        for (int k = 0; k < KW; k++) v[k][q] = m[f[k]];
+                        for (int k = 0; k < KW / 4; k++) v[k][q] = *reinterpret_cast<const uint32_t*>(m + 4 * k);
                     }
 #pragma unroll
                     for (int q = 0; q < ENVS; q++)
                         if (BM % 32 == 0 || 32 * q + lane < BM)
 #pragma unroll
-                            for (int k = 0; k < KW; k++) x[k * XS + 32 * q] = (float)v[k][q];
+                            for (int k = 0; k < KW; k++) x[k * XS + 32 * q] = (float)(v[k / 4][q] >> (8 * (k % 4)) & 0xFFu);
+                } else if (maps) {
+                    uint32_t v[KW / XR][ENVS];
+#pragma unroll
+                    for (int q = 0; q < ENVS; q++) {
+                        const uint8_t* m = map + (BM > 32 && BM % 32 != 0 ? min(32 * q + lane, BM - 1) : 32 * q + xl) * kMapPitch;
+#pragma unroll
+                        for (int k = 0; k < KW / XR; k++) v[k][q] = m[g[k]];
+                    }
+#pragma unroll
+                    for (int q = 0; q < ENVS; q++)
+                        if (BM <= 32 || BM % 32 == 0 || 32 * q + lane < BM)
+#pragma unroll
+                            for (int k = 0; k < KW / XR; k++) x[k * XR * XS + 32 * q] = (float)v[k][q];
                 } else {
 #pragma unroll
                     for (int q = 0; q < ENVS; q++) {
-                        const int e = 32 * q + lane;
-                        if (BM % 32 != 0 && e >= BM) break;
+                        const int e = 32 * q + xl;
+                        if (BM > 32 && BM % 32 != 0 && e >= BM) break;
                         const uint8_t* const r = rec + (size_t)min(e0 + e, n - 1) * kRec + kMap;
 #pragma unroll
-                        for (int k = 0; k < KW; k++) {
-                            if (f[k] < kMap) x[k * XS + 32 * q] = (float)map[e * kMapPitch + f[k]];
-                            else
-                                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(x + k * XS + 32 * q)),
-                                             "l"(r + 4 * (f[k] - kMap)) : "memory");
+                        for (int k = 0; k < KW / XR; k++) {
+                            float* const to = x + k * XR * XS + 32 * q;
+                            if (g[k] < kMap) *to = (float)map[e * kMapPitch + g[k]];
+                            else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(r + 4 * (g[k] - kMap)) : "memory");
                         }
                     }
                 }
@@ -1182,9 +1210,8 @@ int strict_forward(const StrictArgs& a, cudaStream_t st, int* launches) {
     const long long q = (long long)n * H / 1024;
     const int tm = strict_tile(n, H);
     const EncoderTile te = strict_encoder_tile(n, H);
-    // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own (64 envs, hidden 64, depths 1 and 2:
-    // 17.5 us with it, 19.2 without; 20.1 and 21.8; 32 envs, hidden 256, depth 2, 194 blocks: 34.4 and 31.6), but not with four envs a lane in the encoder,
-    // whose blocks then share SMs in some runs (depth 1, 416 envs, hidden 256: 43.0 to 51.4 and 42.5; 512 envs, hidden 192: 39.2 to 46.2 and 39.2)
+    // every kernel of a small forward lets the next one start at once, where all their blocks have SMs of their own (512 envs, 64 blocks a layer: 88 us
+    // with it, 72 without; 32 envs, hidden 256, depth 2, 194 blocks: 34.4 and 31.6)
     auto count = [&](int tile) { return tile == 0 ? 8 * q : tile == 1 ? 2 * q : q / 2; };
     const long long blocks = count(te.tm) + L * count(tm) + n / 16;
     const int early = (a.game == CFX_GAME_FULL && te.tm <= 1 && blocks <= kSMs ? kLaunchNext : 0) | (a.weights_ready ? kWeightsReady : 0);

@@ -95,3 +95,19 @@ def test_each_static_forward_looks_at_its_own_weights(cfx, gpu, oracle, n):
     for i, out in enumerate(outs):
         lav = out.download()
         assert np.isnan(lav).all() if i % 2 else np.array_equal(lav, want), i
+
+
+@pytest.mark.parametrize("n,H", [(32, 256), (160, 256), (416, 256), (1632, 256), (2592, 256), (4128, 256), (2528, 512), (1056, 96), (4768, 64), (5408, 192)])
+def test_records_without_zeros_give_the_bits_of_a_list(cfx, gpu, oracle, n, H):
+    """Where nothing is left out the features are taken by words of the map: the same bits as where one is left out, whose weights are zero."""
+    params = oracle.init_weights(H, L, A, seed=5, scheme="uniform")
+    params[700 * H:701 * H] = 0
+    rec = oracle.synthetic_records(n, seed=4)
+    rec[:, :MAP] = np.maximum(rec[:, :MAP], 1)
+    got = _forward(cfx, params, rec, n, H)
+    lav = oracle.forward(params, rec, None, np.zeros((L, n, H), np.float32), H, L, A)
+    assert np.abs(got["logits"] - lav).max() < 3e-5 * max(1.0, np.abs(lav).max())
+    rec[:, 700] = 0
+    want = _forward(cfx, params, rec, n, H)
+    for k in got:
+        assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), k
