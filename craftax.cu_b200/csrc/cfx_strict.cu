@@ -1095,14 +1095,9 @@ int selftest_reciprocals(uint32_t first, uint32_t last, uint32_t far, uint64_t* 
 }
 
 // The tiles.  What a forward costs is the number of blocks that the fullest SM has one after the other, so the envs of a lane, TM, are
-// those for which that number times the time of a block is the least; both are estimated from what blocks of each height take
-// alone and two to an SM.  (Before, 8 envs a lane from q = n H / 1024 = 1,024 warps on, else 4: at 4,096 envs and hidden 256 that left 40
-// SMs with half of the others' layers, and 24 with three times at 5,120.  The times of all heights were measured at 26 sizes from 512 envs
-// to 16,384, hidden 64 to 512: this choice is the best at all of them in the encoder, and within 1 % of it in the layers.)
+// those for which that number times the time of a block is the least; both are estimated from what blocks of each height take alone and two to an SM.
 // What each height is for, us a forward with all of them and without it: layers, 5 (2,944 envs, hidden 256, depth 2) 98.7 and 103.9, 6 (1,760) 78.0 and 84.0,
-// 7 (4,096) 123.6 and 128.1, 8 (8,192, hidden 512, depth 3) 827 and 864, 9 (2,656, hidden 512) 222 and 249; encoder, depth 1, 5 (11,840, hidden 128) 102.7
-// and 107.9, 6 (14,208, hidden 192) 181.9 and 200.0, 7 (16,384, hidden 256) 291.7 and 303.3, 8 (9,472) 167.9 and 181.9, 9 (10,656, hidden 128) 94.1 and
-// 100.3, although with 9 a lane spills 28 or 36 bytes (128 registers, two blocks of 256 threads an SM).
+// 7 (4,096) 123.6 and 128.1, 8 (8,192, hidden 512, depth 3) 827 and 864, 9 (2,656, hidden 512) 222 and 249.
 static int sm_rounds(int n, int envs, int unit_tiles) { return ((n + envs - 1) / envs * unit_tiles + kSMs - 1) / kSMs; }
 // Up to q = 32 a lane has one sum, or one of each gate (tile 0): us a forward of 32 envs, hidden 256, depth 2, with 4 units a lane in both kernels
 // 46.2, in the encoder 38.7, in neither 32.0; 64 envs 47.6, 43.7 and 34.2; 128 envs 49.1 and 44.1; 192 envs 48.7 and 63; 32 envs, hidden 512 73 and 46;
@@ -1129,10 +1124,15 @@ static int strict_tile(int n, int H) {
     }
     return best;
 }
-// The encoder: TM envs x 8 units a lane, where a block takes TM + 2 units of time; 4 envs x 4 units as long as every block has an SM of its
-// own (hidden 256: 1,024 envs 45.8 us with the forward of one layer, 55.3 with 8 units a lane; 1,536 envs 67.4 and 63.6), 1 env x 4 units
-// under q = 96.
+// The encoder: TM envs x 8 units a lane, where a block takes TM + 2 units of time, or, past the first round, TM + 4 where an SM holds one block at a time, whose
+// first 3,000 cycles are then under no other's sums; 4 envs x 4 units as long as every block has an SM of its own (hidden 256, depth 1: 1,024 envs 42.9 us, 45.0
+// with 8 units a lane; 1,536 56.3 and 48.9), 1 env x 4 units under q = 96.  Of the heights at 66 sizes, records of a game, this choice is the fastest or within 1.5 %
+// of it, but for hidden 320 at 8,192 and 12,288 envs (2 and 4 %).  us with each of the heights 4 to 9, depth 1: 4,096 envs, hidden 256 78.0, 85.2, 91.3,
+// 77.3, 81.0, 86.3; 6,144 112, 120, 110, 117, 124, 135; 65,536 936, 934, 931, 919, 911, 955; 10,656, hidden 128 86.8, 78.8, 85.0, 91.8, 96.6, 79.8;
+// hidden 192, one round of blocks at 6,304 (9) 93.7, 91.5, 102.9, 113.7, 109.6, 92.1, several at 8,192 110, 121, 113, 124, 129, 141, 65,536 710, 704, 755, 761, 762, 782.
+// With 9 a lane spills 12 or 32 bytes (128 registers, two blocks of 256 threads an SM).
 struct EncoderTile { int tm, g; };
+constexpr bool two_blocks(int tm, int wu) { return wu == 2 || tm <= 5; }   // (see strict_encoder)
 static EncoderTile strict_encoder_tile(int n, int H) {
     const long long q = (long long)n * H / 1024;
     if (q <= kSmallest) return {0, 1};
@@ -1140,8 +1140,12 @@ static EncoderTile strict_encoder_tile(int n, int H) {
     if (H % 64 != 0 || sm_rounds(n, 64, H / 32) == 1) return {4, 1};
     const int wu = H % 128 == 0 ? 2 : 1;
     int best = 4;
+    auto cost = [&](int tm) {
+        const int rounds = sm_rounds(n, 16 * tm / wu, H / (64 * wu));
+        return rounds * (tm + (rounds > 1 && !two_blocks(tm, wu) ? 4 : 2));
+    };
     for (int tm = 5; tm <= 9; tm++)
-        if (sm_rounds(n, 16 * tm / wu, H / (64 * wu)) * (tm + 2) < sm_rounds(n, 16 * best / wu, H / (64 * wu)) * (best + 2)) best = tm;
+        if (cost(tm) < cost(best)) best = tm;
     return {best, 2};
 }
 
@@ -1158,6 +1162,7 @@ void strict_tiles(int n, int H, int* layer, int* deep, int* encoder, int* groups
 template <int TM, int G, int WU, int UL = 4>
 static int strict_encoder(const StrictArgs& a, const ArenaLayout& o, int early, cudaStream_t st) {
     using E = Enc<TM, G, WU, UL>;
+    static_assert(two_blocks(TM, WU) == (2 * (E::kSmem + 2048) <= 228 * 1024), "what the rule for the tiles goes by");
     int rc = allow_smem<k_encoder_fp32<TM, G, WU, UL>, E::kSmem>();
     if (rc) return rc;
     return launch_chained(k_encoder_fp32<TM, G, WU, UL>, dim3((a.n + E::BM - 1) / E::BM, a.H / E::BU), 256, E::kSmem, st, a.records,
