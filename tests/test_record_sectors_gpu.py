@@ -49,3 +49,9 @@ def test_sectors_hold_the_record(cfx, gpu, monkeypatch, n, H, L, prec, pair):
     for a, b in zip(*outs):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     pol.close()
+
+
+@pytest.mark.parametrize("n,L,prec", [(2400, 3, "bf16"), (4224, 4, "bf16"), (3232, 1, "f16")])
+def test_records_off_a_sector_of_four_ctas_a_tile(cfx, gpu, monkeypatch, n, L, prec):
+    """Where the record starts off a sector four CTAs have a tile of 128 rows, on one two have 64: the same bits."""
+    test_sectors_hold_the_record(cfx, gpu, monkeypatch, n, 256, L, prec, "1")

@@ -31,10 +31,11 @@ def _forward(cfx, n, H, L, prec, game, rec, params, state, prev_t, r_state, laun
 
 
 @pytest.mark.parametrize("n,H,L,prec,game,r_state", [
-    # four CTAs a tile: 32 rows to 1,056 envs, 64 to 2,112, and to 4,224 128 where the state is recorded
+    # four CTAs a tile: 32 rows to 1,056 envs, 64 to 2,112, and to 4,224 128 where the state is recorded in fp32; else (also in bf16 on a 32-byte
+    # boundary) two CTAs with 64 rows
     (32, 256, 1, "f16", "full", "fp32"), (96, 256, 4, "bf16", "full", "bf16"),
     (1184, 256, 2, "f16", "full", None), (1216, 256, 2, "f16", "full", "fp32"),
-    (2336, 256, 3, "bf16", "full", "bf16"), (2400, 256, 2, "f16", "full", None),    # (the second: two CTAs, 64 rows)
+    (2336, 256, 3, "bf16", "full", "bf16"), (2400, 256, 2, "f16", "full", None),    # (two CTAs, 64 rows)
     # two CTAs a tile: 64 rows to 4,736, 128 to 9,472; then the persistent kernel
     (4704, 256, 4, "f16", "full", "fp32"), (4768, 256, 2, "f16", "full", "bf16"),
     (9472, 256, 3, "f16", "full", "fp32"), (9504, 256, 1, "f16", "full", None),
@@ -46,7 +47,7 @@ def _forward(cfx, n, H, L, prec, game, rec, params, state, prev_t, r_state, laun
     # without a record, both sides of the limits between four CTAs and two, and of 64 and 128 rows
     (2112, 256, 2, "f16", "full", None), (2144, 256, 3, "bf16", "full", None), (3232, 256, 1, "f16", "full", None), (4224, 256, 3, "f16", "full", None),
     (4256, 256, 2, "bf16", "full", None), (4768, 256, 2, "f16", "full", None), (3200, 256, 3, "f16", "classic", None),
-    (2400, 256, 2, "f16", "full", "bf16")])   # the same batch with one: four CTAs, 128 rows
+    (2400, 256, 2, "f16", "full", "bf16")])   # the same batch with one that the cells write: two CTAs, 64 rows too
 def test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, H, L, prec, game, r_state):
     from cfx import synth
     classic = game == "classic"
@@ -70,3 +71,9 @@ def test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, H, L
     (3200, 3, "f16", "fp32")])                                                        # four CTAs, 128 rows
 def test_classic_game_with_a_record(cfx, gpu, monkeypatch, n, L, prec, r_state):
     test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, 256, L, prec, "classic", r_state)
+
+
+@pytest.mark.parametrize("n,L,prec", [(2144, 4, "f16"), (2336, 3, "bf16"), (3136, 2, "f16"), (3232, 1, "bf16"), (4192, 4, "bf16"), (4224, 3, "f16")])
+def test_four_ctas_a_tile_of_128_rows(cfx, gpu, monkeypatch, n, L, prec):
+    """With an fp32 record, from the first batch of this form to the last; the last tile has 32, 64, 96 or all of its rows."""
+    test_small_batch_form_equals_one_cta_per_tile(cfx, gpu, monkeypatch, n, 256, L, prec, "full", "fp32")
