@@ -7,7 +7,7 @@
 //   records   the tile's records are contiguous: four bulk copies of 32 rows into shared memory.  A row is an odd
 //             number of words, so thread-per-row reads have no bank conflicts.  (Tensor boxes of 80 bytes a
 //             row cost more than the rest of the encoder.)  Every CTA of
-//             the cluster expands the whole record into tensor memory, chunk kc by warpgroup kc % 4
+//             the cluster expands the whole record into tensor memory, chunk kc by warpgroup kc % 4 (but the first ones by all: Cfg::kFirst)
 //   encoder   A from tensor memory, N = 64 NS own units
 //   layers    A from shared memory: the layer's input as K blocks of 64 units (128-byte swizzled operand
 //             tiles, 16 KB).  A CTA writes its own K blocks and copies them to the other CTAs (bulk
@@ -130,7 +130,8 @@ enum Bar {
     S_FULL = ACC_FULL + 1, ST_READY = S_FULL + kSSlots, MMA_DONE = ST_READY + kSSlots,
     QUAD = MMA_DONE + 1, G_FULL = QUAD + 8,   // QUAD: [slice][quadrant]
     H_FULL = G_FULL + 2, A_KB = H_FULL + 1,
-    // AEXP_FULL: four chunks each (ONE: of a ring slot); the first ones by themselves, see Cfg::kFirst
+    // AEXP_FULL: four chunks each (ONE: of a ring slot).  Where the first kFirst chunks come by themselves (Cfg::kFirst) they have the last barriers of this
+    // range, and those of four chunks that they would be part of are not used
     AEXP_FIRST = AEXP_FULL + kMaxChunks - kFirstChunks,
     // A_KB: [layer input][K block]; ONE: [layer input][0] for all of its blocks, but not for those of the heads' input
     NUM_BARS = A_KB + (kMaxLayers + 1) * 4
@@ -265,6 +266,8 @@ __device__ __forceinline__ void role_mma(const Smem& sm, const Params& P, uint32
     const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
     // ---- encoder
     auto aexp = [](int kc) { return kc < C::kFirst ? AEXP_FIRST + kc : AEXP_FULL + kc / 4; };
+    static_assert(C::kFirst % 4 == 0 && C::kFirst <= kFirstChunks && (C::kFirst == 0 || AEXP_FULL + (kChunks + 3) / 4 <= AEXP_FIRST) && (kChunks + 3) / 4 <= kMaxChunks,
+                  "a barrier for either");
     CFX_SPROBE(cfx_p_b, W_FULL, 0);
     CFX_SPROBE(cfx_p_a, aexp(0), 0);
 #pragma unroll
@@ -387,6 +390,7 @@ __device__ __forceinline__ void role_mma_one(const Smem& sm, const Params& P, ui
     // (M = 32 takes N = 64, 128 or 256)
     constexpr uint32_t idesc_64 = make_idesc(fmt, 32, kSliceUnits), idesc_hg = make_idesc(fmt, 32, 2 * kSliceUnits);
     constexpr int kBlocks = Gm<GAME>::kEncBlocks, kEnc = C::template ring_items<true>();
+    static_assert(C::kEncItems <= kMaxChunks, "a barrier a ring slot");
     static_assert(C::kUnits == kSliceUnits && C::kKB <= kWSlots && C::kHeadItems <= kWSlots, "a layer's weights are in the ring at once");
     const uint64_t wdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffW)), adesc = smem_desc_sw128(smem_u32(sm.base));
     const uint64_t xdesc = smem_desc_sw128(smem_u32(sm.base + C::kOffX));
@@ -519,8 +523,8 @@ __device__ __forceinline__ void hand_on(const Smem& sm, uint32_t offset, uint32_
 }
 
 // ------------------------------------------------------------------ workers
-// Sixteen warps: warp (quadrant, wg) owns TMEM lanes [32 quadrant, + 32) = those rows of the tile, converts
-// chunks wg, wg + 4, ... and handles units [16 wg, 16 wg + 16) of every slice of the CTA.
+// Sixteen warps: warp (quadrant, wg) owns TMEM lanes [32 quadrant, + 32) = those rows of the tile, converts a quarter of each of the first
+// kFirst chunks, then chunks kFirst + wg, + 4, ..., and handles units [16 wg, 16 wg + 16) of every slice of the CTA.
 template <typename T16, int GAME, int HID, int S, bool REC16>
 __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uint32_t tmem, int warp, int lane, int row0,
                                             uint32_t rank, Meetings& meet) {
