@@ -80,12 +80,13 @@ __device__ __forceinline__ int jax_index(int i, int size) {
 // therefore loads all its fields first.  (ld.global.nc would be wrong besides: see wait_for_previous_kernel.)
 // What a miss brings into L2 is limited to 64 bytes, a burst of the memory, here and in the copies: an env on another level than its neighbours reads
 // scattered words, and a view's span ends anywhere.  By default more comes along (us, this kernel and its list; the classic game's): words 46.3 -> 45.6, the
-// copies too 44.8, the words past L1 44.6; classic 262,144 envs 27.2 -> 25.7, its reads from memory 102 -> 86 MB.  With 128 or 256 bytes as by
+// copies too 44.8; classic 262,144 envs 27.2 -> 25.7, its reads from memory 102 -> 86 MB.  With 128 or 256 bytes as by
 // default.  Not for bytes and shorts, of whose burst the neighbouring blocks use the rest (classic 27.2 -> 27.5).  Spans that leave L2 first (evict_first): 18,944 envs
-// 19.9 -> 18.0, 65,536 44.6 -> 45.4, classic 131,072 14.6 -> 13.7, 20,000 3.54 -> 3.92, 262,144 25.7 -> 26.1: not taken.
+// 19.9 -> 18.0, 65,536 44.6 -> 45.4, classic 131,072 14.6 -> 13.7, 20,000 3.54 -> 3.92, 262,144 25.7 -> 26.1: not taken.  The words past L1: 65,536 envs 0.4 %
+// faster, but lanes and warps read the same lines: 4,096 envs 8.6 -> 10.0, a list of 1,000 of 65,536 4.4 -> 5.9.
 __device__ __forceinline__ uint32_t ld_bits(const uint32_t* p) {
     uint32_t v;
-    asm volatile("ld.global.L1::no_allocate.L2::64B.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.L2::64B.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ int32_t ld_now(const int32_t* p) { return (int32_t)ld_bits(reinterpret_cast<const uint32_t*>(p)); }
