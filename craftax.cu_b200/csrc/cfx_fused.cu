@@ -1002,8 +1002,10 @@ k_policy_fused(const __grid_constant__ Params P) {
             // 18,944 28.4 -> 27.9, h128x2 16,160 17.0 -> 16.6, 20,000 28.2 -> 27.5.
             const int first = P.tile_begin + (int)blockIdx.x;
             wait_for_previous_kernel();
-            if (GAME == CFX_GAME_FULL && warp == 2 && lane < C::kRecCopies && first < P.num_tiles_loop) load_records<PAIR, GAME, HID>(sm, P, first, lane);
-            __syncwarp();
+            if constexpr (GAME == CFX_GAME_FULL) {
+                if (warp == 2 && lane < C::kRecCopies && first < P.num_tiles_loop) load_records<PAIR, GAME, HID>(sm, P, first, lane);
+                __syncwarp();
+            }
             if (lane == 0) {
                 if (warp == 2) role_loads<PAIR, GAME, HID, REC16>(sm, P);
                 else role_stores<PAIR, GAME, HID>(sm, P);

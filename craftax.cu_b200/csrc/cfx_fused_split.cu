@@ -655,6 +655,12 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
             x[j][q] = Op::pack(__uint_as_float(acc[2 * q]) + b[2 * q], __uint_as_float(acc[2 * q + 1]) + b[2 * q + 1]);
         if (!send(0, j, x[j])) return;
     }
+    // The uniform of this row, which is there since the biases are (ACC_FULL).  In the classic game's kernel with one slice a CTA it is read ahead of the layers: so its cells
+    // keep nothing in local memory (with an fp32 record, x3: 1,600 envs 22.4 -> 22.0 us, 3,200 26.4 -> 25.8).  In the others that costs registers (with a bf16
+    // record 6,400 h256x2 20.0 -> 23.0; without one 8,192 classic x1 17.1 -> 17.2)
+    constexpr bool kAhead = GAME == CFX_GAME_CLASSIC && C::kNS == 1;
+    float u = 0.0f;
+    if (kAhead && samples && wg == 0 && valid) u = *reinterpret_cast<volatile float*>(&sm.uniforms()[row]);
     // ---- layers
     for (int l = 0; l < P.L; l++) {
 #pragma unroll
@@ -744,7 +750,7 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
 #pragma unroll
             for (int a = 0; a < kA; a++) pr[a] = p[a * kTile];
             float la = logits[0], total;
-            const int act = draw_action<kA>(pr, sm.uniforms()[row], &total, [&](int a, bool beyond) { la = beyond ? logits[a + 1] : la; });
+            const int act = draw_action<kA>(pr, kAhead ? u : sm.uniforms()[row], &total, [&](int a, bool beyond) { la = beyond ? logits[a + 1] : la; });
             write_action(P, env, act, la - m - logf(total), value);
         }
     }
