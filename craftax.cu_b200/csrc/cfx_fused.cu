@@ -103,12 +103,9 @@ template <bool PAIR, int GAME, int HID> struct Cfg {
     // State boxes that are loaded as soon as their slots are free of records.  The slots come free at about the same time, and copies
     // queue in order: with eight boxes (128 KB from memory) in front of them the last weight stages of the encoder came 2,500 cycles late.  The others
     // are loaded when the encoder is done.  us a step in long runs, all boxes at once and so: h256x2 18,944 envs 29.4 and 29.5, 37,888 63.7 and 62.1, 131,104
-    // 210.7 and 207.5, 262,144 421.9 and 421.9; h256x1 37,888 40.4 and 40.8, 65,536 78.5 and 76.2; h256x3 65,536 147.3 and 146.0, 262,144 559.5 and 560.6;
-    // h128x2 131,104 112.6 and 111.1, 262,144 219.5 and 216.5.  All, 1, 2 or 4 first: h256x2 37,888 envs 63.1, 61.4, 61.8, 62.3; h128x2 131,104 113.8, 115.5,
-    // 113.9, 112.7; h256x2 16,416 with a bf16 record 31.3, 31.4, 31.6, 31.6.  Only in the first tiles of a CTA, four or at hidden 128 eight: within 0.6 %
-    // either way at 37 sizes.
-    // All at once where the state is recorded ahead of the cells (not REC16: h256x2 16,416 envs 29.5 and 29.2, 57,600 110.6 and 107.9), and in the classic game, whose records leave six of the slots alone
-    // (classic h256x3, at once and so: 9,504 envs 31.66 and 31.91, 37,888 81.4 and 80.6, 1,048,576 2,192 and 2,197; h256x1 14,400 20.44 and 20.64).
+    // 210.7 and 207.5; h256x3 65,536 147.3 and 146.0; h128x2 131,104 112.6 and 111.1; within 0.6 % of each other above.
+    // All at once where the state is recorded ahead of the cells (not REC16: h256x2 16,416 envs 29.5 and 29.2), and in the classic game, whose records
+    // leave six of the slots alone (classic h256x3, at once and so: 9,504 envs 31.66 and 31.91, 1,048,576 2,192 and 2,197).
     static constexpr int kEarlyBoxes = HID == 256 ? 1 : 4;
     // records: rows of one copy, slots that hold them, where row r of the tile begins in the data area.  Full game: 16 rows a
     // slot, the odd slots 64 bytes on, so that a warp's 32 rows start in 32 banks
@@ -735,8 +732,8 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
                 CFX_MARK(4);
             }
         } else if (valid) {   // the uniform of this env is drawn while the others convert
-            // (The step counter is constant for the launch: it is raised when every block is done.  Full game: read once and kept in registers through the tiles, us: h128x2 24,064 envs
-            // 27.9 and so 27.1, 57,600 53.5 and 52.7, with an fp32 record 12,832 19.3 and 18.7; h256x2 20,000 41.5 and 41.3.)
+            // (The step counter is constant for the launch: it is raised when every block is done.  Full game: read once and kept in registers
+            // through the tiles, and so, us: h128x2 24,064 envs 27.9 and 27.1, 57,600 53.5 and 52.7; h256x2 20,000 41.5 and 41.3.)
             u = P.uniforms != nullptr ? P.uniforms[env] : philox_uniform(P.seed, P.env_offset + (uint64_t)env, GAME == CFX_GAME_CLASSIC ? step0 : *P.step_ctr);
         }
 
@@ -1014,10 +1011,9 @@ k_policy_fused(const __grid_constant__ Params P) {
     } else {
         // A CTA that has an SM to itself before the kernel in front has ended, because the CTA there had a tile less, asks for its first tile's records
         // to be brought into L2 meanwhile (not a read: what that kernel may still write to them is seen).  us a step without and with it: h256x2 20,000 envs
-        // 41.7 and 40.8, 37,888 58.3 and 57.2, 65,536 104.8 and 102.4, 262,144 378.5 and 376.6; h256x3 65,536 136.7 and 134.8; h128x2 28,416 28.9 and 28.0, 131,104
-        // 102.2 and 100.3.  As bulk prefetches 0.5 % faster still in a stream, but the copies then wait for them where there is no kernel in front (a pass by
-        // itself, 20,480 envs: 51.6, so 51.8, bulk 52.6).  Where every CTA has one tile they end together, and it is slower (18,944 28.2 and 28.6, h128x2 17.3 and
-        // 17.7; small batches 1 to 3 %).  The state of the tile too: 37,888 62.6, 94,720 138 and 147.  The classic game's records are a seventh: no difference.
+        // 41.7 and 40.8, 37,888 58.3 and 57.2, 65,536 104.8 and 102.4, 262,144 378.5 and 376.6; h128x2 28,416 28.9 and 28.0, 131,104 102.2 and 100.3.  A pass by
+        // itself, with no kernel in front: h256x2 20,480 57.1 and 57.7, 37,888 60.9 and 61.0, 262,144 341.2 and 341.1; h128x2 131,104 109.9 and 109.8.  Where every
+        // CTA has one tile they end together, and it is slower (18,944 28.2 and 28.6, h128x2 17.3 and 17.7).  The classic game's records are a seventh: no difference.
         if (GAME == CFX_GAME_FULL && P.num_tiles_loop - P.tile_begin > (int)gridDim.x) {
             const int row0 = (P.tile_begin + (int)blockIdx.x) * kTile, bytes = min(kTile, P.n - row0) * C::kRecBytes;
             const uint8_t* const p = P.records + (size_t)row0 * C::kRecBytes;
@@ -1373,18 +1369,16 @@ int fused_forward(FusedPlan* p, const FusedArgs& a, cudaStream_t st, int* launch
     P.off_b_v = o.b_v;
     if (launches) *launches = 1;
     // Small batches: a tile is shared by four (two) CTAs as long as every tile then has its SMs at once, and is as
-    // short as that allows (cfx_fused_split.cu).  CTAs of two slices take tiles of 64 and
-    // 128 rows; at 32 four CTAs a tile have their SMs.  With the 33 clusters of four and 74 of two that this part holds, four
-    // CTAs go to 1,056 and 2,112 envs, with 32 and 64 rows, and two to 4,736 with 64 rows and 9,472 with 128; where the state is recorded in other ways than two_before_four
-    // names, four take 128 rows up to 4,224.  At each of these limits the next form is slower, and the kernel below slower than all of them.  us a step, h256x2, clusters
+    // short as that allows (cfx_fused_split.cu).  CTAs of two slices take tiles of 64 and 128 rows; at 32 four CTAs a tile have their SMs.  With the 33
+    // clusters of four and 74 of two that this part holds, four CTAs go to 1,056 and 2,112 envs, with 32 and 64 rows, and two to 4,736 with 64 rows and
+    // 9,472 with 128.  At each of these limits the next form is slower, and the kernel below slower than all of them.  us a step, h256x2, clusters
     // of four with 32, 64, 128 rows, of two with 64 and 128, the kernel below: 1,056 envs 10.5, 14.6, 16.8, 16.2, 17.9, 21.5; 2,112 -, 14.8, 16.4, 16.5,
-    // 18.2, 21.8; 2,144 -, -, 17.0, 16.5, 18.2, 21.8; 4,224 -, -, 17.5, 16.9, 18.4, 22.0; 4,736 -, -, -, 17.1, 18.3, 22.3; 9,472 -, -, -, -, 19.0, 22.5.
-    // Four CTAs with 128 rows and two with 64, 4,224 envs: h256x1 13.4 and 12.9, x2 17.4 and 16.8, x3 21.5 and 20.7; with a bf16 record that the cells write (record_by_rows)
-    // x1 14.7 and 13.8, x2 18.9 and 17.9, x3 23.2 and 22.1; classic h256x3, 3,200 envs, 25.0 and 24.7.  h128x2, of two with 32, 64, 128 rows, the kernel below:
-    // 2,368 envs 8.9, 12.5, 13.4, 15.7; 4,736 -, 12.9, 13.5, 15.7; 9,472 -, -, 14.0, 16.0.
-    // The classic game with a record, four CTAs with 128 rows and two with 64, us: in bf16 h256x1 2,144 envs 16.93 and 16.16, 4,224 17.24 and 16.38, x2 21.5 and 20.5, 21.7 and
-    // 20.8, x3 25.8 and 24.9, 26.0 and 25.4; in fp32 x1 17.2 and 16.3, 17.4 and 16.5, x2 21.7 and 21.0, 22.0 and 21.4, but x3 26.3 and 25.8, at 3,200 26.3 and 26.6.  The
-    // full game in fp32: x1 13.0 and 13.1, 14.5 and 14.1, x2 17.6 and 17.9, x3 22.0 and 22.7, x4 26.4 and 27.5.
+    // 18.2, 21.8; 4,224 -, -, 17.5, 16.9, 18.4, 22.0; 4,736 -, -, -, 17.1, 18.3, 22.3; 9,472 -, -, -, -, 19.0, 22.5.  h128x2, of two with 32, 64, 128 rows, the
+    // kernel below: 2,368 envs 8.9, 12.5, 13.4, 15.7; 4,736 -, 12.9, 13.5, 15.7; 9,472 -, -, 14.0, 16.0.
+    // From 2,113 to 4,224 envs four CTAs have 128 rows where write_r_state records the state in front of the cells, work that more CTAs share: the full game in fp32, or in
+    // bf16 off a sector (four and two, us: h256x2 17.6 and 17.9, x4 26.4 and 27.5), and the classic game in fp32 from depth 3 on (x3 26.3 and 26.6).  Else two have 64:
+    // without a record (4,224 envs h256x1 13.4 and 12.9, x3 21.5 and 20.7), with one that the cells write (x1 14.7 and 13.8, x3 23.2 and 22.1), in the classic
+    // game (in bf16 x1 17.2 and 16.4, x3 26.0 and 25.4, in fp32 x2 22.0 and 21.4).
     const bool two_before_four = a.r_state == nullptr || (classic ? P.r_state_bf16 || p->L <= 2 : fused::record_by_rows(P));
     const int rows = std::min(p->n, P.num_tiles * fused::kTile) - P.tile_begin * fused::kTile;
     for (int i = 0; i < 2; i++)

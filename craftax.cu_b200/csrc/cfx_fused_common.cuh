@@ -245,9 +245,9 @@ __device__ __forceinline__ void write_r_state(const Params& P, const uint8_t* bo
 
 // The full game's bf16 record goes another way where it starts on a 32-byte sector: a thread's 16 units of its row are one sector, packed from the
 // registers that the cell has its state in (REC16 kernels), so that nothing is read twice and no step of its own stands in front of the cell.  us a step,
-// written by write_r_state and so: h256x2 9,504 envs 26.6 and 24.7, 16,416 30.5 and 29.2, 37,888 70.6 and 65.8, 262,144 458 and 437; h128x2 16,416 19.0 and 17.7,
-// 131,104 127 and 114; small batches h256x2 2,112 15.9 and 15.5, 6,400 21.9 and 21.3.  Slower, and not done so: fp32, two sectors a thread (h256x2 16,416 31.4 and 32.2,
-// 262,144 439 and 462; h128 +-2 %); small batches of hidden 128 (9,472 15.0 and 15.5).  No difference in the classic game (262,144 598 and 599), which has no such kernels.
+// written by write_r_state and so: h256x2 9,504 envs 26.6 and 24.7, 37,888 70.6 and 65.8, 262,144 458 and 437; h128x2 16,416 19.0 and 17.7, 131,104 127 and 114;
+// small batches h256x2 2,112 15.9 and 15.5, 6,400 21.9 and 21.3.  Slower, and not done so: fp32, two sectors a thread (h256x2 16,416 31.4 and 32.2);
+// small batches of hidden 128 (9,472 15.0 and 15.5).  No difference in the classic game, which has no such kernels.
 inline bool record_by_rows(const Params& P) { return P.r_state != nullptr && P.r_state_bf16 && (reinterpret_cast<uintptr_t>(P.r_state) & 31) == 0; }
 
 // ------------------------------------------------------------------ record expansion

@@ -562,10 +562,10 @@ __device__ __forceinline__ void role_worker(const Smem& sm, const Params& P, uin
         __syncwarp();
         if (lane == 0) mbar_arrive(sm.bar(AEXP_FULL + kc / 4));
     };
-    // Full game, one slice a CTA: the first four chunks a quarter of each a warp, so that the encoder starts with the first one while the others are converted. (A chunk
-    // a warp, all four are there 1,100 cycles after the records.  us: 1,600 envs h256x2 with a bf16 record 15.40 -> 15.22, x4 21.86 -> 21.54, 2,048 h256x2 14.37 -> 14.27, 4,224 with an fp32
-    // record 18.50 -> 18.03, 8,192 h128x2 13.39 -> 13.21.  With two slices a CTA the encoder's weights come too slowly for that to count, 8,192 h256x2 18.75 -> 18.68, and
-    // with a bf16 record the cells keep more in local memory, 6,400 h256x4 30.9 -> 31.2.)
+    // Full game, one slice a CTA: the first four chunks a quarter of each a warp, so that the encoder starts with the first one while the others are
+    // converted.  (A chunk a warp, all four are there 1,100 cycles after the records.  us: 2,048 envs h256x2 14.37 -> 14.27, 4,224 with an fp32 record 18.50 -> 18.03,
+    // 8,192 h128x2 13.39 -> 13.21.  With two slices a CTA the encoder's weights come too slowly for that to count: 8,192 h256x2 18.75 -> 18.68, with a bf16
+    // record 6,400 h256x4 30.9 -> 31.2.)
     constexpr int kFirst = C::kFirst;
     if constexpr (kFirst > 0) {
         uint32_t bytes[4], regs[8];
@@ -984,7 +984,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
         if (i < NUM_BARS) {
             uint32_t arrivals = 1, bytes = 0;
             if (i == REC_FREE) arrivals = ONE ? S * kWorkerWarps : S * 4 * quads;
-            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks) arrivals = ONE ? C::item_warps(i - AEXP_FULL) : i >= AEXP_FIRST && C::kFirst > 0 ? 4 * quads : max(1, min(4, Gm<GAME>::kEncChunks - 4 * (i - AEXP_FULL))) * quads;
+            else if (i >= AEXP_FULL && i < AEXP_FULL + kMaxChunks)
+                arrivals = ONE ? C::item_warps(i - AEXP_FULL)
+                           : i >= AEXP_FIRST && C::kFirst > 0 ? 4 * quads : max(1, min(4, Gm<GAME>::kEncChunks - 4 * (i - AEXP_FULL))) * quads;
             else if (i == ACC_FULL) arrivals = 2;                          // the MMAs, and the biases are in place
             else if (i >= ST_READY && i < ST_READY + kSSlots) arrivals = ONE ? 8 : 2 * quads;
             else if (i == MMA_DONE) arrivals = S;
@@ -1042,9 +1044,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_policy_split(const __grid_const
                 reinterpret_cast<float*>(sm.base + C::kOffBias)[i] =
                     P.params[a < 0 ? P.off_b_enc + C::slice((int)rank, i / kSliceUnits) * kSliceUnits + i % kSliceUnits : (a < kA ? P.off_b_a + a : P.off_b_v)];
             }
-            // The uniforms of the rows that this CTA samples, and the step counter, which the last CTA that has read it raises.  (By the workers that sample,
-            // under the encoder's products, they were late in tiles of 32 rows, 512 envs h256x2 9.82 -> 9.72 us, h128x2 8.33 -> 8.17; in taller ones they cost registers: 8,192 envs
-            // h256x2 18.82 -> 18.74, with a bf16 record 21.46 -> 20.99, classic h256x3 26.4 -> 25.9, 4,736 h128x2 12.7 -> 12.2, 2,048 h256x2 14.56 -> 14.38.)
+            // The uniforms of the rows that this CTA samples, and the step counter, which the last CTA that has read it raises.  (By the workers that
+            // sample, under the encoder's products, they were late in tiles of 32 rows, 512 envs h256x2 9.82 -> 9.72 us; in taller ones they cost registers:
+            // 8,192 envs h256x2 with a bf16 record 21.46 -> 20.99, classic h256x3 26.4 -> 25.9, 4,736 h128x2 12.7 -> 12.2.)
             bool draws = false;
             const unsigned long long step0 = P.uniforms == nullptr && has_heads<S, ONE>(quads, rank) ? *P.step_ctr : 0ull;
             for (int q = 0; q < quads; q++)

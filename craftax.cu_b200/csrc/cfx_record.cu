@@ -14,14 +14,10 @@
 //   3. warp per env: a lane makes four cells of a view row from the spans in registers, the four records
 //      are put together where the spans were, and go out as one bulk copy (1,992 blocks of 16 bytes a
 //      block) or, where an env is skipped, as coalesced words.
-// 65,536 envs with 62 KB of maps each, about 180 MB of DRAM traffic (us, by itself; with the list of 250 reset envs behind it):
-// copies behind the position, then the fields and the two mob classes of a warp one latency after the other 46.4 and 52.9; all loads that
-// wait for nothing in front of the copies 42.5 and 49.1; the copies by rows (27 lanes with a row each, at most two pieces
-// of it) replaced by whole spans 41.8 and 48.0; the fields in front of what depends on the level, and not behind, 39.9 and 46.2; 64 bytes a
-// miss (ld_bits) 38.1 and 44.6.
-// A block took 25,000 cycles, a third of them memory latencies one behind the other; in 17,000 they still are.  Five blocks an SM (48
-// registers; copies by rows): 41.6 and 48.2, and 4 % slower up to 8,192 envs.  The next kernel's start under this one, early or
-// late in a block: 49.4 to 50.4 instead of 49.1.
+// 65,536 envs with 62 KB of maps each: 38.4 us, with the list of 250 reset envs behind it 44.6; 128 MB read from DRAM.  What it gained (us, by itself; with the
+// list): loads that wait for nothing in front of the copies 46.4 -> 42.5, 52.9 -> 49.1; whole spans for rows piece by piece 41.8, 48.0; the fields in front of
+// what depends on the level 39.9, 46.2; 64 bytes a miss (ld_bits) 38.4, 44.6.  A block took 25,000 cycles and takes 17,000; the memory latencies one behind
+// the other, 8,000 of them, are left.
 // The bytes are the reference's: the same predicates, the same "last slot of a class wins a
 // cell" order, the same float expressions (sqrtf(x) * 0.1f, x * 0.1f, x * 0.5f, x * 0.25f; no
 // fused multiply-add can form).
@@ -79,11 +75,9 @@ __device__ __forceinline__ int jax_index(int i, int size) {
 // latency a field; a read-only load it sinks to its use, with the same effect.  Every loop below
 // therefore loads all its fields first.  (ld.global.nc would be wrong besides: see wait_for_previous_kernel.)
 // What a miss brings into L2 is limited to 64 bytes, a burst of the memory, here and in the copies: an env on another level than its neighbours reads
-// scattered words, and a view's span ends anywhere.  By default more comes along (us, this kernel and its list; the classic game's): words 46.3 -> 45.6, the
-// copies too 44.8; classic 262,144 envs 27.2 -> 25.7, its reads from memory 102 -> 86 MB.  With 128 or 256 bytes as by
-// default.  Not for bytes and shorts, of whose burst the neighbouring blocks use the rest (classic 27.2 -> 27.5).  Spans that leave L2 first (evict_first): 18,944 envs
-// 19.9 -> 18.0, 65,536 44.6 -> 45.4, classic 131,072 14.6 -> 13.7, 20,000 3.54 -> 3.92, 262,144 25.7 -> 26.1: not taken.  The words past L1: 65,536 envs 0.4 %
-// faster, but lanes and warps read the same lines: 4,096 envs 8.6 -> 10.0, a list of 1,000 of 65,536 4.4 -> 5.9.
+// scattered words, and a view's span ends anywhere.  By default more comes along (us: this kernel and its list 46.1 -> 44.6; classic game, 262,144 envs 27.4 -> 25.8, its
+// reads from memory 102 -> 86 MB).  Not for bytes and shorts, of whose burst the neighbouring blocks use the rest (classic 27.2 -> 27.5).  The words past L1:
+// 65,536 envs 0.4 % faster, but lanes and warps read the same lines: 4,096 envs 8.6 -> 10.0, a list of 1,000 of 65,536 4.4 -> 5.9.
 __device__ __forceinline__ uint32_t ld_bits(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.global.L2::64B.b32 %0, [%1];" : "=r"(v) : "l"(p));
